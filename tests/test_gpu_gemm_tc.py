@@ -107,3 +107,16 @@ def test_tc_prefill_size_properties(nk):
     rows = rng.choice(m, size=64, replace=False)
     want = O.gemm_i32_fast(packed, q1[torch.from_numpy(rows).cuda()].cpu().numpy(), 0)
     assert np.array_equal(y1[torch.from_numpy(rows).cuda()].cpu().numpy(), want)       # oracle on a random sample of tokens
+
+
+@pytest.mark.parametrize("m,n", [(130, 384), (500, 200), (64, 100), (129, 128)])
+def test_tc_bf16_output_of_partial_tiles(m, n):
+    """bf16 results with one weight scale where the last tile has fewer than 64 tokens or fewer than 32 rows: bit-equal to the rounding sequence."""
+    from test_gpu_linear import ref_dequant
+    from wf_bitnet import ops
+    k = 512
+    packed, q, s, rs = make(n, k, m, m + n)
+    want = torch.from_numpy(ref_dequant(packed, q, rs, np.float32(1.7), s)).to(torch.bfloat16)
+    got = ops.ternary_linear(ops.i2s_to_tile(cu(packed)), n, k, cu(q), mode="linear", rowsum=cu(rs), act_scale=cu(s), w_scale=torch.tensor([1.7]).cuda(),
+                             out_dtype=torch.bfloat16, algo=3).cpu()
+    assert torch.equal(got, want)

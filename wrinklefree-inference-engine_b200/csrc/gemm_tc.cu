@@ -445,7 +445,8 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
                         if (j < mcnt) {
                             const float2 t = tok[c * 32 + j];
                             // the reference's rounding sequence (linear_value in linear_common.cuh)
-                            float y = __fmul_rn(__fsub_rn(__fmul_rn((float)(int)v[j], ws), __fmul_rn(ws, t.x)), t.y);
+                            // t.x already holds fl(w_s * Sigma a) where that was folded in at the staging
+                            float y = __fmul_rn(__fsub_rn(__fmul_rn((float)(int)v[j], ws), fold_ws ? t.x : __fmul_rn(ws, t.x)), t.y);
                             const size_t o = (size_t)(m0 + j) * p.ep.ldo + col;
                             if (relu2) {
                                 const float g = bf16_round(y);
