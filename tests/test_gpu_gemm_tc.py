@@ -120,3 +120,25 @@ def test_tc_bf16_output_of_partial_tiles(m, n):
     got = ops.ternary_linear(ops.i2s_to_tile(cu(packed)), n, k, cu(q), mode="linear", rowsum=cu(rs), act_scale=cu(s), w_scale=torch.tensor([1.7]).cuda(),
                              out_dtype=torch.bfloat16, algo=3).cpu()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("m", [17, 33, 63, 65, 128, 129])
+@pytest.mark.parametrize("nk", [(131, 1152), (2540, 2560), (96, 6912)])
+def test_tc_shared_k_range(m, nk):
+    """Few tokens: the K range of a tile shared by a cluster (unequal parts when K / 128 is no multiple of the cluster), every kind of output."""
+    from test_gpu_linear import ref_dequant
+    from wf_bitnet import ops
+    n, k = nk
+    packed, q, s, rs = make(n, k, m, n + k + m)
+    pi, acc = cu(packed), O.gemm_i32_fast(packed, q, 0)
+    want = acc.astype(np.float32) * np.float32(0.0123)
+    assert np.array_equal(ops.bitnet_gemm(pi, cu(q), 0.0123).cpu().numpy(), want)
+    kw = dict(layout="i2s", mode="linear", rowsum=cu(rs), act_scale=cu(s), algo=3)
+    got = ops.ternary_linear(pi, n, k, cu(q), w_scale=torch.tensor([0.9]).cuda(), out_dtype=torch.bfloat16, **kw).cpu()
+    assert torch.equal(got, torch.from_numpy(ref_dequant(packed, q, rs, np.float32(0.9), s)).to(torch.bfloat16))
+    if n % 32 == 0:
+        gu = ops.interleave_rows16(cu(packed[:n // 2]), cu(packed[n // 2:]))
+        g = torch.from_numpy(ref_dequant(packed[:n // 2], q, rs, np.float32(0.9), s)).to(torch.bfloat16)
+        u = torch.from_numpy(ref_dequant(packed[n // 2:], q, rs, np.float32(1.6), s)).to(torch.bfloat16)
+        got = ops.ternary_linear(gu, n, k, cu(q), w_scale=torch.tensor([0.9, 1.6]).cuda(), relu2_mul=True, out_dtype=torch.bfloat16, **kw).cpu()
+        assert torch.equal(got, torch.relu(g).square() * u)

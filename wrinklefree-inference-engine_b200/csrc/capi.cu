@@ -75,6 +75,15 @@ extern "C" size_t wf_linear_workspace_bytes(int M, int N, int K) {
     return gemm_mma_workspace_bytes(M, N, K);
 }
 
+// tcgen05 or mma.sync.  From 17 tokens the mma.sync kernel takes its 32- and 64-token tiles and is bound by the legacy int8 pipe: 14336 x 4096 with
+// 48 tokens 38.3 us against 16.5, 4096 x 14336 with 17 tokens 18 against 14.7, 6912 x 2560 with 1987 tokens 157 against 50.  Below, its weight
+// stream is as fast and its launch cheaper (2560 x 2560, 9 tokens: 8.4 us against 10.4).  The same holds for its 64-token tiles on short-K matrices
+// while they fit in about one wave (6912 x 2560, 33 tokens: 10.4 against 12.4; 2560 x 2560, 192 tokens: 12.5 against 14.5).
+static bool tc_is_faster(int M, int N, int K) {
+    if (M < 17) return false;
+    return !(M > 32 && K <= 2560 && (long long)M * N * K <= 1300000000LL);
+}
+
 extern "C" int wf_ternary_linear(const wf_linear_args* a, void* stream) {
     if (!a) { set_error("wf_ternary_linear: null args"); return WF_ERR_INVALID; }
     EpiParams ep;
@@ -85,8 +94,7 @@ extern "C" int wf_ternary_linear(const wf_linear_args* a, void* stream) {
     int algo = a->algo;
     if (algo == 0) {
         if (a->M <= 8 && a->w_layout == WF_W_TILE && a->workspace && gemv_stream_fits(a->M, a->K)) algo = 1;   // else (70B down at M = 8: 8 x 28672 int8 rows) the tiled GEMM
-        else if (a->M >= 128) algo = 3;   // a real dense contraction: tcgen05 int8
-        else algo = 2;
+        else algo = tc_is_faster(a->M, a->N, a->K) ? 3 : 2;
     }
     switch (algo) {
         case 1: return launch_gemv_stream(a, ep, s, false);
@@ -107,7 +115,6 @@ static int compat_call(const uint8_t* packed, const int8_t* x, float scale, int 
     a.out_mode = WF_OUT_COMPAT_F32;
     a.out = y; a.ldo = N;
     a.workspace = ws; a.workspace_bytes = ws_bytes;
-    a.algo = 2;
     return wf_ternary_linear(&a, stream);
 }
 

@@ -59,6 +59,9 @@ struct TcParams {
     // tile each, and the epilogue adds the raw accumulators into a global fp32 buffer (exact: integers < 2^24) instead
     // of storing a finished output — the consumer phase of the decode step applies scales / residual / norm.
     int splitk, KBs;
+    // few-token form (launch_tc_split): the ksplit CTAs of a thread-block cluster take one tile's K range in equal parts and add their
+    // int32 accumulators through distributed shared memory (exact, so the order does not matter)
+    int ksplit;
     int l2_ahead;   // decode form: L2 prefetch distance of the weight stream in items of an unpack group (0 = off)
     float* red_acc;
     int red_ld;
@@ -134,11 +137,14 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;   // 128B-swizzle atoms need 1024-B alignment
     const int crank = (CL > 1) ? (int)(blockIdx.x % CL) : 0;          // 1-D cluster: rank == blockIdx.x % CL
-    const int cluster_id = blockIdx.x / CL, n_clusters = gridDim.x / CL;
+    const int ksp = CL == 1 ? p.ksplit : 1;                           // cluster of K parts (one tile per cluster) instead of a cluster of tiles
+    const int krank = ksp > 1 ? (int)(blockIdx.x % ksp) : 0;
+    const int cluster_id = blockIdx.x / (CL * ksp), n_clusters = gridDim.x / (CL * ksp);
     const int ngroups = (p.tiles_n + CL - 1) / CL;                    // groups of CL weight-row tiles
     const int total_tiles = ngroups * p.tiles_m * p.splitk;           // cluster tiles (x K-splits in the decode form)
     const int my_tiles = (total_tiles - cluster_id + n_clusters - 1) / n_clusters;
-    const int KBs = p.KBs;                                            // k-blocks per tile (== KB unless split)
+    const int k_part0 = ksp > 1 ? krank * p.KB / ksp : 0;             // this CTA's first k-block
+    const int KBs = ksp > 1 ? (krank + 1) * p.KB / ksp - k_part0 : p.KBs;   // k-blocks per tile (== KB unless split)
     const int n_items = my_tiles * KBs;
     auto tile_coords = [&](int tl, int& m_blk, int& n_blk, int& ks) {
         const int ct0 = cluster_id + tl * n_clusters;
@@ -179,7 +185,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
                 int m_blk, n_blk, ks;
                 tile_coords(tl, m_blk, n_blk, ks);
                 for (int kb = 0; kb < KBs; ++kb, ++it) {
-                    const int kg = ks * KBs + kb;
+                    const int kg = ks * KBs + k_part0 + kb;
                     const int s = it % TC_STAGES;
                     mbar_wait(&empty_bar[s], (uint32_t)(((it / TC_STAGES) & 1) ^ 1));   // all CL CTAs retired this slot
                     if (CL == 1 && (p.dbg & 8)) { mbar_arrive(&full_bar[s]); continue; }  // timing experiment: no activation traffic
@@ -284,7 +290,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
             // b200_tile_v1: word (16*(r&7) + 4*(j&3) + 2*(j>>2) + (r>>3)) of tile (row/16, kb) holds packed bytes [4j,4j+4) of row r
             const uint8_t* rowbase = i2s ? p.w + (size_t)row * K4
                                          : p.w + (size_t)(row >> 4) * p.KB * WF_TILE_BYTES + (size_t)(16 * (row & 7) + ((row >> 3) & 1)) * 4;
-            l_src = rowbase + ((size_t)ks * KBs + l_kb) * kb_stride;   // this tile's K run, this group's first k-block in it
+            l_src = rowbase + ((size_t)ks * KBs + k_part0 + l_kb) * kb_stride;   // this tile's K run, this group's first k-block in it
             pf_off = i2s ? 0u : (uint32_t)(((row >> 3) & 1) * 28);
         };
         seek();
@@ -393,6 +399,19 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
             const bool fast = fast_mode && mw0 + TC_EP_TOKS <= p.M && n_blk * TC_BM + q * 32 + 32 <= p.N;   // warp-uniform
             mbar_wait(&tfull_bar[buf], (uint32_t)((tl >> 1) & 1));
             tc_fence_after();
+            if (ksp > 1) {
+                // the ring is free (every MMA of this CTA's only tile has read its stage): the accumulators go there as [token][row]
+#pragma unroll 1
+                for (int c = 0; c < TC_EP_TOKS / 32 && mw0 + c * 32 < p.M; ++c) {
+                    uint32_t v[32];
+                    TC_LD32(tmem + lane_base + th * TC_EP_TOKS + c * 32, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    const uint32_t at = ring + ((uint32_t)((th * TC_EP_TOKS + c * 32) * TC_BM + q * 32 + lane) << 2);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + (uint32_t)(j * TC_BM * 4)), "r"(v[j]) : "memory");
+                }
+                continue;
+            }
 #pragma unroll 1
             for (int c = 0; c < TC_EP_TOKS / 32; ++c) {
                 uint32_t v[32];
@@ -478,6 +497,46 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
             }
         }
     }
+    if (ksp > 1) {
+        // sum of the K parts: every CTA of the cluster finishes an equal share of the tile's tokens
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        int m_blk, n_blk, ks;
+        tile_coords(0, m_blk, n_blk, ks);
+        const int m0 = m_blk * TC_BN, mcnt = min(TC_BN, p.M - m0), per = (mcnt + ksp - 1) / ksp;
+        const int t0 = krank * per, cnt = max(0, min(mcnt, t0 + per) - t0);
+        const bool relu2 = p.ep.out_mode == WF_OUT_LINEAR && (p.ep.epi_flags & WF_EPI_RELU2_MUL);
+        auto total4 = [&](int tok, int row, int (&v)[4]) {                    // rows row .. row + 3 of one token
+            const uint32_t at = ring + ((uint32_t)(tok * TC_BM + row) << 2);
+            v[0] = v[1] = v[2] = v[3] = 0;
+#pragma unroll 4
+            for (int r = 0; r < ksp; ++r) {
+                uint32_t ra;
+                int x, y, z, w;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(at), "r"(r));
+                asm volatile("ld.shared::cluster.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(ra) : "memory");
+                v[0] += x; v[1] += y; v[2] += z; v[3] += w;
+            }
+        };
+        const int quads = relu2 ? TC_BM / 8 : TC_BM / 4;                      // groups of four output columns per token
+        for (int i = tid; i < cnt * quads; i += (int)blockDim.x) {
+            const int tok = t0 + i / quads, j = i % quads * 4;
+            const int row = relu2 ? (j >> 4) * 32 + (j & 15) : j, n = n_blk * TC_BM + row;
+            int v[4], u[4];
+            total4(tok, row, v);
+            if (relu2) {
+                total4(tok, row + 16, u);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) if (n + k < p.N) epilogue_store_relu2(p.ep, m0 + tok, n + k, v[k], u[k]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) if (n + k < p.N) epilogue_store(p.ep, m0 + tok, n + k, v[k]);
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // nobody leaves while a peer may still read its part
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
     tc_fence_before();
     __syncthreads();
     if (CL > 1) {   // nobody leaves while a peer may still multicast into this CTA's ring or signal its barriers
@@ -541,7 +600,7 @@ static int launch_tc_cl(const wf_linear_args* a, const EpiParams& ep, cudaStream
     p.tiles_n = (a->N + TC_BM - 1) / TC_BM;
     p.tiles_m = (a->M + TC_BN - 1) / TC_BN;
     p.ep = ep;
-    p.splitk = 1; p.KBs = p.KB; p.red_acc = nullptr; p.red_ld = 0; p.l2_ahead = 0;
+    p.splitk = 1; p.KBs = p.KB; p.ksplit = 1; p.red_acc = nullptr; p.red_ld = 0; p.l2_ahead = 0;
     { const char* d = getenv("WF_TC_DBG"); p.dbg = d ? atoi(d) : 0; }
     const int total = ((p.tiles_n + CL - 1) / CL) * p.tiles_m;
     cudaLaunchConfig_t cfg = {};
@@ -593,7 +652,7 @@ int launch_gemm_tc_red(const uint8_t* w_tile, int N, int K, const int8_t* q, int
     p.tiles_n = (N + TC_BM - 1) / TC_BM;
     p.tiles_m = 1;
     p.ep.M = M; p.ep.N = N; p.ep.out_mode = WF_OUT_I32_PLUS1; p.ep.nseg = 1; p.ep.ldo = acc_ld; p.ep.out = acc;
-    p.red_acc = acc; p.red_ld = acc_ld;
+    p.red_acc = acc; p.red_ld = acc_ld; p.ksplit = 1;
     // largest divisor of KB that still gives every SM at most one tile
     const int sms = sm_count();
     int split = 1;
@@ -615,9 +674,47 @@ int launch_gemm_tc_red(const uint8_t* w_tile, int N, int K, const int8_t* q, int
     return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<1, NU>, tmap, p), "ternary_gemm_tc(decode)");
 }
 
+// Few tokens: the tiles alone leave SMs idle and one CTA walks all of K, a latency chain of ~450 clk per k-block.  A cluster of ksplit CTAs shares
+// the tile's K range instead, as many as the SMs hold at once with at least four k-blocks (one unpack prefetch) each.  Measured without / with:
+// 4096 x 14336, 64 tokens 31.8 / 16.5 us; 2560 x 6912, 128 tokens 20.6 / 13.3 us; 2560 x 2560, 48 tokens 13.6 / 10.4 us.
+static int launch_tc_split(const wf_linear_args* a, const EpiParams& ep, int ksplit, cudaStream_t s) {
+    constexpr int NU = 2;
+    CUtensorMap tmap;
+    const cuuint64_t gdim[2] = {(cuuint64_t)a->K, (cuuint64_t)a->M};
+    const cuuint64_t gstride[1] = {(cuuint64_t)a->ldq};
+    const cuuint32_t box[2] = {TC_BK, TC_BN};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult cr = g_encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)a->q, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                 CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) { set_error("gemm_tc_split: cuTensorMapEncodeTiled failed (%d)", (int)cr); return WF_ERR_CUDA; }
+    TcParams p;
+    memset(&p, 0, sizeof p);
+    p.w = a->w; p.w_layout = a->w_layout;
+    p.M = a->M; p.N = a->N; p.K = a->K; p.KB = a->K / WF_QK;
+    p.tiles_n = (a->N + TC_BM - 1) / TC_BM;
+    p.tiles_m = (a->M + TC_BN - 1) / TC_BN;
+    p.ep = ep;
+    p.splitk = 1; p.KBs = p.KB; p.ksplit = ksplit;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.tiles_n * p.tiles_m * ksplit);
+    cfg.blockDim = dim3(tc_threads(NU));
+    cfg.dynamicSmemBytes = TC_SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ksplit; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<1, NU>, tmap, p), "ternary_gemm_tc(split)");
+}
+
 int launch_gemm_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s) {
     gemm_tc_init_attrs();
     if (!g_encode) { set_error("gemm_tc: tcgen05 path unavailable (driver entry point / smem attribute)"); return WF_ERR_CUDA; }
+    const int tiles = ((a->N + TC_BM - 1) / TC_BM) * ((a->M + TC_BN - 1) / TC_BN), sms = sm_count();
+    int ksplit = 1;
+    while (ksplit < 8 && tiles * ksplit * 2 <= sms && a->K / WF_QK >= ksplit * 2 * 4) ksplit *= 2;
+    if (ksplit > 1) return launch_tc_split(a, ep, ksplit, s);
     if (g_tc_cluster == 4) return launch_tc_cl<4, 2>(a, ep, s);
     if (g_tc_cluster == 2) return g_tc_nu == 2 ? launch_tc_cl<2, 2>(a, ep, s) : launch_tc_cl<2, 3>(a, ep, s);
     if (g_tc_nu == 1) return launch_tc_cl<1, 1>(a, ep, s);

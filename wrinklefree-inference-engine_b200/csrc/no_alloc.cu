@@ -68,6 +68,5 @@ extern "C" int wf_bitnet_gemm_static(const uint8_t* packed_i2s, const int8_t* x,
     a.out_mode = WF_OUT_COMPAT_F32;
     a.out = y; a.ldo = N;
     a.workspace = ws; a.workspace_bytes = (size_t)WF_STATIC_WS_BYTES;
-    a.algo = 2;                        // the kernel wf_bitnet_gemv / wf_bitnet_gemm run
     return wf_ternary_linear(&a, stream);
 }
