@@ -35,6 +35,7 @@ struct LayerState {
     void* wo = nullptr;       // [W, heads * vdim]
     // latent attention
     void *dkv_norm = nullptr, *uk = nullptr, *ukT = nullptr, *uv = nullptr;
+    void* kvx = nullptr;      // [keys | values of every head] from a cached row: launch_latent_expand_weight (prompt portions; null: sizes that form does not take)
     long long cache_off = 0;  // element offset of this layer inside a cache page
     // delta
     void *conv_w = nullptr, *A_log = nullptr, *dt_bias = nullptr, *onorm = nullptr;
@@ -123,7 +124,10 @@ struct wf_seq_engine {
     int32_t *ids = nullptr, *counts = nullptr, *plan_scratch = nullptr, *sorted_rows = nullptr, *pair_row = nullptr, *tile_group = nullptr;
     int P = 0;                        // padded expert-row bound
     int fuse_input = 1;               // norm + input convolution (+ state roll of single-token sequences) in one kernel (WF_SEQ_FUSE_INPUT=0: three kernels)
-    int attn_mma = 2;                 // latent attention on tensor cores where the sizes allow it: 2 keys-as-rows form first, 1 heads-as-rows form only, 0 plain kernel (WF_SEQ_ATTN_MMA)
+    int attn_mma = 3;                 // attention on tensor cores where the sizes allow it: 3 prompt portions on tcgen05; below that 2 latent attention with keys as rows first, 1 heads as rows only, 0 plain kernels (WF_SEQ_ATTN_MMA)
+    // latent attention of prompt portions: the cached rows of the step's sequences gathered, and the keys and values of every head made from them
+    void *lat_rows = nullptr, *kvx = nullptr;
+    int kvx_rows = 0;
     float* row_inv = nullptr;         // [max_step_tokens][norm groups] row statistics of the many-token input kernel
     int attn_waves = 4;               // decode attention: resident waves of CTAs the key splits aim at (WF_SEQ_ATTN_WAVES)
     float* gqa_ws = nullptr;          // partial results of key-split grouped-query attention: gqa_ws_rows (token, head, split) rows
@@ -363,6 +367,15 @@ int prepare_step(wf_seq_engine* e, int nseq, const int32_t* slots, const int32_t
         for (int k = 0; k < counts[i]; ++k) { m_tok[at_] = tokens ? tokens[at_] : 0; m_tseq[at_] = i; m_tpos[at_] = m_pos0[i] + k; ++at_; }
     }
     for (int j = 0; j < nwant; ++j) m_want[j] = want[j];
+    int32_t* m_key = m + 4 * T + 4 * S;
+    long long ctx = 0;
+    v->b.pairs = 0.;
+    for (int i = 0; i < nseq; ++i) {
+        m_key[i] = (int32_t)ctx;
+        ctx += m_pos0[i] + counts[i];
+        v->b.pairs += (double)counts[i] * (m_pos0[i] + 0.5 * (counts[i] + 1));
+    }
+    v->b.ctx_total = (int)ctx;                      // at most the pool's tokens
     if (cuda_check(cudaMemcpyAsync(e->d_meta, m, e->meta_ints * 4, cudaMemcpyHostToDevice, e->stream), "step metadata H2D")) return WF_ERR_CUDA;
     if (e->pt.dirty) {
         std::vector<int32_t> tmp(e->pt.table);
@@ -379,6 +392,7 @@ int prepare_step(wf_seq_engine* e, int nseq, const int32_t* slots, const int32_t
     v->b.tok_seq = d + T; v->b.tok_pos = d + 2 * T;
     v->b.seq_start = d + 3 * T; v->b.seq_len = d + 3 * T + S; v->b.seq_pos0 = d + 3 * T + 2 * S; v->b.seq_slot = d + 3 * T + 3 * S;
     v->want = d + 3 * T + 4 * S;
+    v->b.key_row = d + 4 * T + 4 * S;
     return WF_OK;
 }
 
@@ -425,6 +439,29 @@ int run_latent(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
         if ((rc = launch_gemm(e->dt, lin(e->cq, 0, c.q_rank, L.uq, c.q_rank, e->qfull, 1, nq, n, nq, c.q_rank), s))) return rc;
         mark(e, "latent.query_latent");
         qsrc = e->qfull; ldq = nq;
+    }
+    // Prompt portions: every position's latent expanded to the heads' keys and values once, then attention with per-head keys (tcgen05).  Per (query, key)
+    // pair and head that is 2 (d + r + 2 dv) operations instead of 2 (2 R + r) on mma.sync (measured about 3e14 against 1e14 a second), at the price
+    // of the expansion of all positions so far, 2 (R + r) (d + r + dv) operations each at about 6e14, and of three launches.
+    const double us_absorbed = b.pairs * H * 2. * (2 * c.kv_rank + c.rot_dim) * 1e-8;
+    const double us_expanded = 30. + b.pairs * H * 2. * (per + 2 * c.vdim) / 3e8 + (double)b.ctx_total * H * 2. * nkv * (per + c.vdim) / 6e8;
+    if (e->attn_mma >= 3 && L.kvx && n > b.nseq && b.ctx_total <= e->kvx_rows && L.cache_off % 8 == 0 && e->page_stride % 8 == 0 && us_expanded < us_absorbed) {
+        if ((rc = launch_latent_q_prep(e->dt, b, D, qsrc, ldq, e->qn, nullptr, s))) return rc;
+        if ((rc = launch_latent_kv_write(e->dt, b, D, e->proj + L.kv_col, L.np, L.dkv_norm, e->cfg.eps, pc, s))) return rc;
+        mark(e, "latent.q_prep+kv_write");
+        const int nx = H * (per + c.vdim);
+        if ((rc = launch_latent_gather(b, D, pc, b.key_row, b.ctx_total, e->lat_rows, s))) return rc;
+        if ((rc = launch_gemm(e->dt, lin(e->lat_rows, 0, nkv, L.kvx, nkv, e->kvx, 0, nx, b.ctx_total, nx, nkv), s))) return rc;
+        mark(e, "latent.expand_gemm");
+        GqaDims G{H, H, per, c.vdim, c.scale, 0.f, c.window, 0, 0};
+        G.sink = L.sink_f ? 2 : 0; G.sink_h = L.sink_f;
+        if ((rc = launch_attn_tc_dense(b, G, e->qn, nullptr, e->kvx, at(e, e->kvx, (size_t)H * per), nx, b.ctx_total, b.key_row, c.head_gate ? (void*)e->ov : e->og, c.head_gate, s))) return rc;
+        mark(e, "latent.attention");
+        if (c.head_gate && (rc = launch_gate_mul(e->dt, e->ov, nv, e->proj + L.kv_col + nkv, L.np, 0, n, nv, e->og, nv, s))) return rc;
+        if (c.head_gate) mark(e, "latent.gate");
+        rc = launch_gemm(e->dt, lin(e->og, 0, nv, L.wo, nv, out, 1, W, n, W, nv), s);
+        mark(e, "latent.out_gemm");
+        return rc;
     }
     if ((rc = launch_latent_q_prep(e->dt, b, D, qsrc, ldq, e->qn, e->qr, s))) return rc;
     if ((rc = launch_latent_kv_write(e->dt, b, D, e->proj + L.kv_col, L.np, L.dkv_norm, e->cfg.eps, pc, s))) return rc;
@@ -575,6 +612,8 @@ int run_gqa(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
             if (splits < 1) splits = 1;
         }
         if ((rc = launch_talk_attn_mma(b, D, e->qn, pc, e->og, e->gqa_ws, splits, s))) return rc;
+    } else if (e->dt == WF_BF16 && e->attn_mma >= 3 && n > b.nseq && attn_tc_usable(D, pc)) {
+        if ((rc = launch_attn_tc(b, D, e->qn, gate, pc, e->cfg.max_pages, e->og, s))) return rc;
     } else if (e->dt == WF_BF16 && e->attn_mma >= 1 && gqa_attn_mma_usable(D, pc) && gqa_attn_mma_takes(D)) {
         // decoding (one token per sequence): few CTAs with long key ranges, so the keys are cut until there are about four resident
         // waves of CTAs (two are resident per SM): the machine is covered and the last wave's tail stays short.
@@ -1105,7 +1144,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     if (c.tied_head) e->head = e->embed;
     else { TRY(dalloc_t(e, &e->head, (size_t)c.vocab * W)); add_tensor(e, "head", e->head, (size_t)c.vocab * W); }
     // maxima over layers for the shared workspaces
-    size_t max_np = 1, max_hd = 1, max_hr = 1, max_hrot = 1, max_hv = 1, max_C = 1, max_H = 1, max_N = 1, max_top = 1, max_E = 1, max_ff = 1, max_uff = 0, max_gqa_dv = 0;
+    size_t max_np = 1, max_hd = 1, max_hr = 1, max_hrot = 1, max_hv = 1, max_C = 1, max_H = 1, max_N = 1, max_top = 1, max_E = 1, max_ff = 1, max_uff = 0, max_gqa_dv = 0, max_kvx = 0, max_lat = 0;
     long long cache_elems = 0;
     size_t st = 0;
     e->layers.resize(c.n_layers + c.n_extra);
@@ -1208,9 +1247,17 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             TRYL(walloc(&L.uk, (size_t)l.heads * l.dim * l.kv_rank)); name(mp + "uk", L.uk, (size_t)l.heads * l.dim * l.kv_rank);
             TRYL(walloc(&L.ukT, (size_t)l.heads * l.dim * l.kv_rank));
             TRYL(walloc(&L.uv, nv * l.kv_rank)); name(mp + "uv", L.uv, nv * l.kv_rank);
+            {
+                const int per = l.dim + l.rot_dim;
+                const GqaDims X{l.heads, l.heads, per, l.vdim, l.scale, 0.f, l.window, 0, 0};
+                if (e->dt == WF_BF16 && e->attn_mma >= 3 && attn_tc_dense_usable(X) && nkv % 8 == 0) {
+                    TRYL(walloc(&L.kvx, (size_t)l.heads * (per + l.vdim) * nkv));
+                    max_kvx = std::max(max_kvx, (size_t)l.heads * (per + l.vdim)); max_lat = std::max(max_lat, (size_t)nkv);
+                }
+            }
             L.cache_off = cache_elems;
             cache_elems += (long long)c.page_size * nkv;
-            max_hd = std::max(max_hd, (size_t)l.heads * l.dim); max_hr = std::max(max_hr, (size_t)l.heads * l.kv_rank);
+            max_hd = std::max(max_hd, (size_t)l.heads * (l.dim + l.rot_dim)); max_hr = std::max(max_hr, (size_t)l.heads * l.kv_rank);
             max_hrot = std::max(max_hrot, (size_t)l.heads * std::max(l.rot_dim, 1));
         } else if (l.type == WF_SEQ_MINGRU) {
             // [z | x | g], all of the channel count; state: one float per channel
@@ -1426,7 +1473,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     e->pt.init(c.max_pages, c.page_size, c.slots, max_blocks);
     e->h_len.assign(c.slots, 0);
     TRY(dalloc_n(e, &e->d_block_table, (size_t)c.slots * max_blocks));
-    e->meta_ints = (size_t)4 * T + (size_t)4 * c.slots;
+    e->meta_ints = (size_t)4 * T + (size_t)5 * c.slots;
     TRY(dalloc_n(e, &e->d_meta, e->meta_ints));
     if (cuda_check(cudaMallocHost((void**)&e->h_meta, e->meta_ints * 4), "pinned metadata")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
     // workspaces
@@ -1438,6 +1485,10 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     TRY(dalloc_t(e, &e->olat, (size_t)T * max_hr)); TRY(dalloc_n(e, &e->ov, (size_t)T * max_hv)); TRY(dalloc_t(e, &e->og, (size_t)T * max_hv));
     e->attn_ws_rows = 4 * 148;
     if (e->dt == WF_BF16 && max_hr > 1) TRY(dalloc_bytes(e, (void**)&e->attn_ws, (size_t)e->attn_ws_rows * (max_hr + 2 * max_H) * sizeof(float)));
+    if (max_kvx) {                             // enough positions for sequences of several full steps; longer ones keep the form that reads the latents
+        e->kvx_rows = (int)std::min<long long>((long long)c.max_pages * c.page_size, 4LL * T);
+        TRY(dalloc_t(e, &e->lat_rows, (size_t)e->kvx_rows * max_lat)); TRY(dalloc_t(e, &e->kvx, (size_t)e->kvx_rows * max_kvx));
+    }
     TRY(dalloc_n(e, &e->gate, (size_t)T * std::max(max_H, max_gate)));
     if (c.n_extra > 0) TRY(dalloc_n(e, &e->y2, (size_t)T * W));
     if (parallel) TRY(dalloc_t(e, &e->h_t2, (size_t)T * W));
@@ -1529,7 +1580,11 @@ extern "C" int wf_seq_finalize(wf_seq_engine* e) {
         if (!t.loaded) { set_error("wf_seq_finalize: tensor '%s' was not loaded", t.name.c_str()); return WF_ERR_INVALID; }
     for (LayerState& L : e->layers)
         if (L.c.type == WF_SEQ_LATENT_ATTENTION)      // W_uk per head [dim, kv_rank] -> [kv_rank, dim]: the weight of q -> W_uk^T q
+        {
             if (int rc = launch_transpose_heads(e->dt, L.uk, L.c.heads, L.c.dim, L.c.kv_rank, L.ukT, e->stream)) return rc;
+            const LatentDims D{L.c.heads, L.c.dim, L.c.rot_dim, L.c.vdim, L.c.kv_rank, L.c.scale, L.c.rope_base, L.c.rope_dims, L.c.window};
+            if (L.kvx) if (int rc = launch_latent_expand_weight(e->dt, D, L.uk, L.uv, L.kvx, e->stream)) return rc;
+        }
     // attention bias tables: the loaded rows [rel_rows, heads] expanded to one row per distance 0 .. rel_far (later distances share the last).
     // The bucket of a distance is computed here, once, in double: exact below rel_rows / 2, then logarithmic steps up to rel_far.
     for (int li = 0; li < (int)e->layers.size(); ++li) {

@@ -251,6 +251,27 @@ bool gemm_tc_usable(const GemmArgs& g) {
     return true;
 }
 
+void* tensor_map_encoder() {
+    if (!g_encode) {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult qr;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qr) == cudaSuccess && qr == cudaDriverEntryPointSuccess)
+            g_encode = (EncodeTiledFn)fn;
+    }
+    return (void*)g_encode;
+}
+
+int* tc_error_word() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev > 63) dev = 0;
+    if (!g_err_dev[dev]) {
+        if (cuda_check(cudaMalloc((void**)&g_err_dev[dev], 4), "cudaMalloc")) { g_err_dev[dev] = nullptr; return nullptr; }
+        if (cuda_check(cudaMemset(g_err_dev[dev], 0, 4), "memset")) return nullptr;
+    }
+    return g_err_dev[dev];
+}
+
 int gemm_tc_error(cudaStream_t s) {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -264,20 +285,9 @@ int gemm_tc_error(cudaStream_t s) {
 // n_groups: number of stacked weight matrices (1 when dense)
 int launch_gemm_tc(const GemmArgs& g, int n_groups, cudaStream_t s) {
     if (g_attr.need()) cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
-    if (!g_encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qr) == cudaSuccess && qr == cudaDriverEntryPointSuccess)
-            g_encode = (EncodeTiledFn)fn;
-    }
-    if (!g_encode) { set_error("gemm_tc: cuTensorMapEncodeTiled unavailable"); return WF_ERR_CUDA; }
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev > 63) dev = 0;
-    if (!g_err_dev[dev]) {
-        if (cuda_check(cudaMalloc((void**)&g_err_dev[dev], 4), "cudaMalloc")) return WF_ERR_CUDA;
-        if (cuda_check(cudaMemset(g_err_dev[dev], 0, 4), "memset")) return WF_ERR_CUDA;
-    }
+    if (!tensor_map_encoder()) { set_error("gemm_tc: cuTensorMapEncodeTiled unavailable"); return WF_ERR_CUDA; }
+    int* err = tc_error_word();
+    if (!err) return WF_ERR_CUDA;
     CUtensorMap tw, ta;
     const int group_w_rows = g.tile_group ? (int)(g.group_stride / g.ldb) : 0;
     const uint64_t w_rows = g.tile_group ? (uint64_t)(n_groups - 1) * group_w_rows + g.N : (uint64_t)g.N;
@@ -289,7 +299,7 @@ int launch_gemm_tc(const GemmArgs& g, int n_groups, cudaStream_t s) {
     p.tiles = p.n_tiles * ((g.M + TC_TOK - 1) / TC_TOK);
     p.C = g.C; p.ldc = g.ldc; p.c_f32 = g.c_f32; p.ep = g.ep;
     p.tile_group = g.tile_group; p.group_w_rows = group_w_rows;
-    p.err = g_err_dev[dev];
+    p.err = err;
     const int sms = sm_count();
     gemm_tc_kernel<<<p.tiles < sms ? p.tiles : sms, TC_THREADS, TC_SMEM, s>>>(tw, ta, p);
     return launch_check(cudaGetLastError(), "gemm_tc");

@@ -122,6 +122,9 @@ int launch_gemm(int dt, const GemmArgs& g, cudaStream_t s);
 // tcgen05 form (seq_gemm_tc.cu): bf16 operands, dense A rows; launch_gemm picks it from WF_SEQ_TC_MIN (17) rows up
 bool gemm_tc_usable(const GemmArgs& g);
 int launch_gemm_tc(const GemmArgs& g, int n_groups, cudaStream_t s);
+// shared by the tcgen05 kernels: the driver's tensor-map encoder (null: unavailable) and the current device's error word (null: no memory)
+void* tensor_map_encoder();
+int* tc_error_word();
 int gemm_tc_error(cudaStream_t s);           // 0 = no bounded wait of the tcgen05 kernel ever ran out on this device
 // dst T [P, W] = src T [rows[i], :] (zero rows where rows[i] < 0)
 int launch_gather_rows(int dt, const void* src, int ld, const int32_t* rows, int P, int W, void* dst, cudaStream_t s);
@@ -135,13 +138,19 @@ int launch_gemv_pairs(int dt, const GemmArgs& g, const int32_t* pair_expert, int
 // frequencies, tabulated by the caller (null: rope_base^(-2i / rope_dims) in float); the angle pos * freq, its cosine and sine are then
 // formed in double and rounded once; mscale multiplies cosines and sines.  sink (device, float [H]): the softmax denominator carries
 // exp(sink[h]) (null: nothing).
+struct PagedCache { void* pool; long long page_stride; long long layer_off; int page_size; const int32_t* block_table; int max_blocks; };
 struct LatentDims { int H, d, r, dv, R; float scale, rope_base; int rope_dims, window;
                     int interleaved = 0; const double* freq = nullptr; float mscale = 1.f; const float* sink = nullptr; };
 // q float [n, H * (d + r)] (ldq): unrotated parts -> qn T [n, H, d]; rotated parts -> rotary at tok_pos -> qr float [n, H, r]
+// (qr null: both parts -> qn T [n, H, d + r])
 int launch_latent_q_prep(int dt, const Batch& b, const LatentDims& L, const float* q, int ldq, void* qn, float* qr, cudaStream_t s);
+// The latents expanded to per-head keys and values: out T [H * (d + r) + H * dv, R + r], the matrix that takes a cached row [latent | rotated part]
+// to every head's key [W_uk c | kr] and value W_uv c; and the cached rows of the step's sequences, positions 0 .. last, one sequence after
+// another (sequence i from row key_row[i]; `rows` in all) as a dense buffer.
+int launch_latent_expand_weight(int dt, const LatentDims& L, const void* uk, const void* uv, void* out, cudaStream_t s);
+int launch_latent_gather(const Batch& b, const LatentDims& L, const PagedCache& pc, const int32_t* key_row, int rows, void* out, cudaStream_t s);
 // dkv float [n, R + r] (ld): first R RMS-normed with weight w (plain), last r rotated; written as T into the paged cache row of
 // (sequence, position): cache + page * page_stride + layer_off + slot_in_page * (R + r)
-struct PagedCache { void* pool; long long page_stride; long long layer_off; int page_size; const int32_t* block_table; int max_blocks; };
 int launch_latent_kv_write(int dt, const Batch& b, const LatentDims& L, const float* dkv, int ld, const void* w, float eps, const PagedCache& pc,
                            cudaStream_t s);
 // per (token, head): softmax over positions j in (pos - window, pos] of (qa . c_j + qr . kr_j) * scale; out T [n, H, R] = sum p_j c_j.
@@ -196,6 +205,17 @@ int launch_gqa_prep(int dt, const Batch& b, const GqaDims& D, const float* proj,
 // out T [n, H * dv]: per (token, head) softmax over keys j in (pos - window, pos] (and j < keep_first) of q . k_j * scale - slope_h * (pos - j),
 // weighted value sum, times gate[n, H] (null: no gate).
 int launch_gqa_attn(int dt, const Batch& b, const GqaDims& D, const void* qn, const float* gate, const PagedCache& pc, void* out, cudaStream_t s);
+
+// Prompt portions on tcgen05 (bf16 storage; seq_attn_tc.cu): causal / window attention with penalty, gates and sink as above (no chunks, kept first
+// positions, caps, bias tables, logarithmic penalties, mixed heads or values that are keys), per-head sizes multiples of 8 up to 128, page sizes
+// that are powers of two from 8 up.
+bool attn_tc_usable(const GqaDims& D, const PagedCache& pc);
+int launch_attn_tc(const Batch& b, const GqaDims& D, const void* qn, const float* gate, const PagedCache& pc, int max_pages, void* out, cudaStream_t s);
+// The same with keys and values in a dense buffer instead of the cache: k and v point at row 0's first head, heads d / dv elements apart, rows
+// row_stride elements apart.  Key position j of sequence i is row key_row[i] + j (device array).
+bool attn_tc_dense_usable(const GqaDims& D);
+int launch_attn_tc_dense(const Batch& b, const GqaDims& D, const void* qn, const float* gate, const void* k, const void* v, int row_stride, int rows,
+                         const int32_t* key_row, void* out, int out_f32, cudaStream_t s);
 
 // Attention whose heads' weights are mixed (D.talk) has kernels of its own: a plain one behind launch_gqa_attn, and tensor-core forms
 // (bf16 storage; seq_attn_talk.cu).  When every sequence brings one token the key range can be cut over `splits` CTAs; that form needs a

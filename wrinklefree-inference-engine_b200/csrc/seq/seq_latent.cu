@@ -52,8 +52,10 @@ __global__ void latent_q_prep_kernel(Batch b, LatentDims L, const float* __restr
     for (int idx = blockIdx.y * blockDim.x + threadIdx.x; idx < L.H * per; idx += gridDim.y * blockDim.x) {
         const int h = idx / per, c = idx % per;
         const float* src = q + (size_t)i * ldq + (size_t)h * per;
-        if (c < L.d) { qn[((size_t)i * L.H + h) * L.d + c] = from_f<T>(src[c]); continue; }
-        qr[((size_t)i * L.H + h) * L.r + c - L.d] = rope_entry(L, src + L.d, c - L.d, cs, sn);
+        if (c < L.d) { qn[((size_t)i * L.H + h) * (qr ? L.d : per) + c] = from_f<T>(src[c]); continue; }
+        const float v = rope_entry(L, src + L.d, c - L.d, cs, sn);
+        if (qr) qr[((size_t)i * L.H + h) * L.r + c - L.d] = v;
+        else qn[((size_t)i * L.H + h) * per + c] = from_f<T>(v);
     }
 }
 
@@ -157,7 +159,49 @@ int check_dims(const LatentDims& L) {
     return WF_OK;
 }
 
+// rows of every head's key [W_uk | 0] and [0 | unit rows], then of every head's value [W_uv | 0]
+template <typename T>
+__global__ void latent_expand_weight_kernel(LatentDims L, const T* __restrict__ uk, const T* __restrict__ uv, T* __restrict__ out) {
+    const int width = L.R + L.r, per = L.d + L.r, row = blockIdx.x;
+    for (int c = threadIdx.x; c < width; c += blockDim.x) {
+        T v = from_f<T>(0.f);
+        if (row < L.H * per) {
+            const int h = row / per, e = row - h * per;
+            if (e < L.d) { if (c < L.R) v = uk[((size_t)h * L.d + e) * L.R + c]; }
+            else if (c == L.R + e - L.d) v = from_f<T>(1.f);
+        } else if (c < L.R) v = uv[(size_t)(row - L.H * per) * L.R + c];
+        out[(size_t)row * width + c] = v;
+    }
+}
+
+// a warp per cached row, 16 bytes per lane and copy
+__global__ void latent_gather_kernel(Batch b, LatentDims L, PagedCache pc, const int32_t* __restrict__ key_row, int rows, __nv_bfloat16* __restrict__ out) {
+    const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    int sq = 0;
+    while (sq + 1 < b.nseq && key_row[sq + 1] <= row) ++sq;
+    const int j = row - key_row[sq], width = L.R + L.r;
+    const int page = pc.block_table[(size_t)b.seq_slot[sq] * pc.max_blocks + j / pc.page_size];
+    const uint4* src = reinterpret_cast<const uint4*>((const __nv_bfloat16*)pc.pool + (size_t)page * pc.page_stride + pc.layer_off + (size_t)(j % pc.page_size) * width);
+    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)row * width);
+    for (int c = lane; c < width / 8; c += 32) dst[c] = src[c];
+}
+
 }  // namespace
+
+int launch_latent_expand_weight(int dt, const LatentDims& L, const void* uk, const void* uv, void* out, cudaStream_t s) {
+    const int rows = L.H * (L.d + L.r + L.dv);
+    if (dt == WF_BF16) latent_expand_weight_kernel<<<rows, 128, 0, s>>>(L, (const __nv_bfloat16*)uk, (const __nv_bfloat16*)uv, (__nv_bfloat16*)out);
+    else latent_expand_weight_kernel<<<rows, 128, 0, s>>>(L, (const float*)uk, (const float*)uv, (float*)out);
+    return launch_check(cudaGetLastError(), "latent_expand_weight");
+}
+
+int launch_latent_gather(const Batch& b, const LatentDims& L, const PagedCache& pc, const int32_t* key_row, int rows, void* out, cudaStream_t s) {
+    if (rows <= 0) return WF_OK;
+    if ((L.R + L.r) % 8 || pc.layer_off % 8 || pc.page_stride % 8) { set_error("latent gather: cached rows are not 16-byte aligned"); return WF_ERR_UNSUPPORTED; }
+    latent_gather_kernel<<<(rows + 7) / 8, 256, 0, s>>>(b, L, pc, key_row, rows, (__nv_bfloat16*)out);
+    return launch_check(cudaGetLastError(), "latent_gather");
+}
 
 int launch_latent_q_prep(int dt, const Batch& b, const LatentDims& L, const float* q, int ldq, void* qn, float* qr, cudaStream_t s) {
     if (b.n <= 0) return WF_OK;
