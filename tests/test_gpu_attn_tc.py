@@ -19,7 +19,7 @@ def build(cfg, weights, page_size, shapes=None):
     from wf_bitnet import registry
     cls = registry.resolve(cfg)
     extra = {"shapes": shapes} if getattr(cls, "reads_shapes", False) else {}
-    m = cls(cfg, dtype="bfloat16", max_tokens=2048, slots=4, page_size=page_size, max_step_tokens=640, **extra)
+    m = cls(cfg, dtype="bfloat16", max_tokens=2048, slots=4, page_size=page_size, max_step_tokens=700, **extra)
     m.load_weights((k, v.numpy(), "F32") for k, v in weights.items())
     return m
 
@@ -50,7 +50,8 @@ def d64(weights, prefix):
     return {k[len(prefix):]: v.double() for k, v in weights.items() if k.startswith(prefix)}
 
 
-CUTS = {"whole": ([300, 129], [[300, 129]]), "portions": ([300, 129], [[127, 2], [2, 0], [1, 126], [170, 1]]), "tiles": ([256, 128], [[128, 128], [128, 0]]), "one": ([2, 1], [[2, 1]])}
+# (the form takes steps in which some sequence reaches more than 256 keys)
+CUTS = {"whole": ([520, 129], [[520, 129]]), "portions": ([520, 129], [[300, 2], [2, 0], [82, 126], [136, 1]]), "tiles": ([512, 128], [[384, 128], [128, 0]]), "start": ([257, 1], [[257, 1]])}
 
 
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,page", [(4, 4, 128, 128, 16), (8, 2, 128, 64, 8), (5, 1, 72, 128, 256), (6, 2, 64, 40, 128), (16, 1, 8, 8, 16)])
@@ -69,7 +70,7 @@ def test_penalty_and_head_gates(heads, kv_heads, dim, vdim, page, cut):
     model.close()
 
 
-@pytest.mark.parametrize("window", [1, 100, 128, 129, 1000])
+@pytest.mark.parametrize("window", [257, 300, 384, 385, 1000])
 @pytest.mark.parametrize("cut", ["whole", "portions"])
 def test_window_rotation_and_element_gates(window, cut):
     W = 64

@@ -26,6 +26,7 @@ struct Batch {
     const int32_t* seq_slot;   // [nseq] state slot = block-table row
     int max_len = 0;           // longest portion of the step (known on the host; sizes grids that cut portions into chunks)
     const int32_t* key_row = nullptr;   // [nseq] first row of the sequence where all its positions so far lie one sequence after another
+    int max_ctx = 0;           // most positions that a sequence holds behind the step (known on the host)
     int ctx_total = 0;         // those rows: the sum over sequences of the positions behind the step (known on the host)
     double pairs = 0.;         // (query, earlier or own key) pairs of the step, windows aside (known on the host)
 };

@@ -370,8 +370,10 @@ int prepare_step(wf_seq_engine* e, int nseq, const int32_t* slots, const int32_t
     int32_t* m_key = m + 4 * T + 4 * S;
     long long ctx = 0;
     v->b.pairs = 0.;
+    v->b.max_ctx = 0;
     for (int i = 0; i < nseq; ++i) {
         m_key[i] = (int32_t)ctx;
+        v->b.max_ctx = std::max(v->b.max_ctx, (int)(m_pos0[i] + counts[i]));
         ctx += m_pos0[i] + counts[i];
         v->b.pairs += (double)counts[i] * (m_pos0[i] + 0.5 * (counts[i] + 1));
     }
@@ -612,7 +614,9 @@ int run_gqa(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
             if (splits < 1) splits = 1;
         }
         if ((rc = launch_talk_attn_mma(b, D, e->qn, pc, e->og, e->gqa_ws, splits, s))) return rc;
-    } else if (e->dt == WF_BF16 && e->attn_mma >= 3 && n > b.nseq && attn_tc_usable(D, pc)) {
+    } else if (e->dt == WF_BF16 && e->attn_mma >= 3 && n > b.nseq && std::min(c.window, b.max_ctx) > 256 && attn_tc_usable(D, pc)) {
+        // up to two of its key tiles the tcgen05 form has nothing to overlap, and the mma.sync form's smaller CTAs start sooner: steps of 64 / 256 tokens at
+        // position 0 took 10 / 5 us longer with it; 3 x 300 tokens were equal, 512 tokens 3 us shorter, 256 tokens behind 3000 72 us shorter (20 heads of 128)
         if ((rc = launch_attn_tc(b, D, e->qn, gate, pc, e->cfg.max_pages, e->og, s))) return rc;
     } else if (e->dt == WF_BF16 && e->attn_mma >= 1 && gqa_attn_mma_usable(D, pc) && gqa_attn_mma_takes(D)) {
         // decoding (one token per sequence): few CTAs with long key ranges, so the keys are cut until there are about four resident
