@@ -126,6 +126,11 @@ typedef struct wf_linear_args {
 
 size_t wf_linear_workspace_bytes(int M, int N, int K);
 int wf_ternary_linear(const wf_linear_args* args, void* stream);
+/* The same with the weight scales by value: w_scales points at args->nseg (1..4) host floats and args->w_scale is not read. */
+int wf_ternary_linear_scales(const wf_linear_args* args, const float* w_scales, void* stream);
+/* What wf_bitnet_gemv / wf_bitnet_gemm (and wf_ternary_linear with algo 0 beyond 8 rows) can use of a workspace for this shape: at most
+ * wf_linear_workspace_bytes, 0 where the kernel they choose needs none. */
+size_t wf_bitnet_gemm_workspace_bytes(int M, int N, int K);
 
 /* torch.ops.sgl_kernel.bitnet_gemv_cpu(packed_weights, activations, scale) -> f32[N]
  * (docs/research/sglang_optimization_plan.md:61-64; call sites bitnet_patch.py:69,

@@ -7,14 +7,14 @@
 
 namespace wf {
 
-int fill_epi(const wf_linear_args* a, EpiParams* p) {
+int fill_epi(const wf_linear_args* a, EpiParams* p, const float* w_scales_host) {
     memset(p, 0, sizeof *p);
     p->M = a->M;
     p->N = a->N;
     p->rowsum = a->rowsum;
     p->act_scale = a->act_scale;
     p->act_scale_per_token = a->act_scale_per_token;
-    p->w_scale = a->w_scale;
+    p->w_scale = w_scales_host ? nullptr : a->w_scale;
     p->nseg = a->nseg <= 0 ? 1 : a->nseg;
     for (int i = 0; i < 4; ++i) p->seg_end[i] = a->seg_end[i];
     p->host_scale = a->host_scale;
@@ -35,7 +35,7 @@ int fill_epi(const wf_linear_args* a, EpiParams* p) {
     if (a->out_mode < WF_OUT_I32_PLUS1 || a->out_mode > WF_OUT_LINEAR) { set_error("wf_ternary_linear: bad out_mode %d", a->out_mode); return WF_ERR_INVALID; }
     if ((a->out_mode == WF_OUT_I32 || a->out_mode == WF_OUT_LINEAR) && !a->rowsum) { set_error("wf_ternary_linear: rowsum required for this out_mode"); return WF_ERR_INVALID; }
     if (a->out_mode == WF_OUT_LINEAR) {
-        if (!a->act_scale || !a->w_scale) { set_error("wf_ternary_linear: act_scale and w_scale required for WF_OUT_LINEAR"); return WF_ERR_INVALID; }
+        if (!a->act_scale || !(a->w_scale || w_scales_host)) { set_error("wf_ternary_linear: act_scale and w_scale required for WF_OUT_LINEAR"); return WF_ERR_INVALID; }
         if (a->nseg < 1 || a->nseg > 4) { set_error("wf_ternary_linear: nseg must be 1..4"); return WF_ERR_INVALID; }
         if (a->out_dtype != WF_F32 && a->out_dtype != WF_BF16) { set_error("wf_ternary_linear: out_dtype must be f32 or bf16"); return WF_ERR_INVALID; }
         if ((a->epi_flags & WF_EPI_RESIDUAL) && !a->residual) { set_error("wf_ternary_linear: residual pointer missing"); return WF_ERR_INVALID; }
@@ -45,6 +45,7 @@ int fill_epi(const wf_linear_args* a, EpiParams* p) {
         set_error("wf_ternary_linear: epilogue flags need WF_OUT_LINEAR");
         return WF_ERR_INVALID;
     }
+    for (int i = 0; w_scales_host && i < p->nseg && i < 4; ++i) p->w_scale_host[i] = w_scales_host[i];
     const int out_cols = (a->epi_flags & WF_EPI_RELU2_MUL) ? a->N / 2 : a->N;
     if (a->ldo < out_cols) { set_error("wf_ternary_linear: ldo (%d) < output columns (%d)", a->ldo, out_cols); return WF_ERR_INVALID; }
     return WF_OK;
@@ -84,10 +85,10 @@ static bool tc_is_faster(int M, int N, int K) {
     return !(M > 32 && K <= 2560 && (long long)M * N * K <= 1300000000LL);
 }
 
-extern "C" int wf_ternary_linear(const wf_linear_args* a, void* stream) {
+static int ternary_linear(const wf_linear_args* a, const float* w_scales_host, void* stream) {
     if (!a) { set_error("wf_ternary_linear: null args"); return WF_ERR_INVALID; }
     EpiParams ep;
-    int rc = fill_epi(a, &ep);
+    int rc = fill_epi(a, &ep, w_scales_host);
     if (rc) return rc;
     if (a->M == 0) return WF_OK;
     cudaStream_t s = (cudaStream_t)stream;
@@ -103,6 +104,17 @@ extern "C" int wf_ternary_linear(const wf_linear_args* a, void* stream) {
     }
     set_error("wf_ternary_linear: unknown algo %d", a->algo);
     return WF_ERR_INVALID;
+}
+
+extern "C" int wf_ternary_linear(const wf_linear_args* a, void* stream) { return ternary_linear(a, nullptr, stream); }
+
+extern "C" int wf_ternary_linear_scales(const wf_linear_args* a, const float* w_scales, void* stream) {
+    if (!w_scales) { set_error("wf_ternary_linear_scales: null scales"); return WF_ERR_INVALID; }
+    return ternary_linear(a, w_scales, stream);
+}
+
+extern "C" size_t wf_bitnet_gemm_workspace_bytes(int M, int N, int K) {
+    return M > 0 && N > 0 && tc_is_faster(M, N, K) ? 0 : wf_linear_workspace_bytes(M, N, K);
 }
 
 static int compat_call(const uint8_t* packed, const int8_t* x, float scale, int M, int N, int K, float* y, void* ws,

@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
         const bool red = p.red_acc != nullptr;
         const bool fast_mode = !red && mode == WF_OUT_LINEAR && !relu2 && !resid && obf16 && !p.dbg;
         const bool fold_ws = fast_mode && p.ep.nseg <= 1;
-        const float ws_all = fold_ws ? p.ep.w_scale[0] : 1.f;
+        const float ws_all = fold_ws ? w_scale_of(p.ep, 0) : 1.f;
         if (red) pdl_wait_prior();   // the accumulator buffer was cleared by an earlier phase of the step
         for (int tl = 0; tl < my_tiles; ++tl) {
             int m_blk, n_blk, ks;
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
             const int col = relu2 ? (n >> 5) * 16 + (n & 15) : n;                  // its output column (gate lanes under relu^2*up)
             const bool store_lane = relu2 ? (lane < 16 && col < ncols) : (n < p.N);
             float ws = 1.f;
-            if (mode == WF_OUT_LINEAR) ws = relu2 ? p.ep.w_scale[(lane >= 16 && p.ep.nseg > 1) ? 1 : 0] : seg_scale(p.ep, min(n, p.N - 1));
+            if (mode == WF_OUT_LINEAR) ws = relu2 ? w_scale_of(p.ep, (lane >= 16 && p.ep.nseg > 1) ? 1 : 0) : seg_scale(p.ep, min(n, p.N - 1));
             const bool fast = fast_mode && mw0 + TC_EP_TOKS <= p.M && n_blk * TC_BM + q * 32 + 32 <= p.N;   // warp-uniform
             mbar_wait(&tfull_bar[buf], (uint32_t)((tl >> 1) & 1));
             tc_fence_after();

@@ -14,8 +14,8 @@ struct EpiParams {
     const int32_t* rowsum;
     const float* act_scale;
     int act_scale_per_token;
-    float w_scale_host[4];  // unused on device; kept for debugging
-    const float* w_scale;
+    const float* w_scale;   // [nseg] on the device, or null: w_scale_host holds them
+    float w_scale_host[4];
     int nseg;
     int seg_end[4];
     float host_scale;
@@ -25,12 +25,14 @@ struct EpiParams {
     const __nv_bfloat16* residual;
 };
 
+__device__ __forceinline__ float w_scale_of(const EpiParams& p, int s) { return p.w_scale ? p.w_scale[s] : p.w_scale_host[s]; }
+
 __device__ __forceinline__ float seg_scale(const EpiParams& p, int n) {
     int s = 0;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
         if (i + 1 < p.nseg && n >= p.seg_end[i]) s = i + 1;
-    return p.w_scale[s];
+    return w_scale_of(p, s);
 }
 
 // value of the (dequantised) linear output for accumulator S (= sum (w+1) a) at (m, n)
@@ -77,8 +79,8 @@ __device__ __forceinline__ void epilogue_store(const EpiParams& p, int m, int n,
 // -> out[m, j] with j = (n_g / 32) * 16 + (n_g % 16).  bf16 rounding after every torch op:
 //   torch.relu(gate).square() * up   (direct_inference_full.py:259)
 __device__ __forceinline__ void epilogue_store_relu2(const EpiParams& p, int m, int n_g, int Sg, int Su) {
-    const float g = bf16_round(linear_value(p, m, p.w_scale[0], Sg));
-    const float u = bf16_round(linear_value(p, m, p.w_scale[p.nseg > 1 ? 1 : 0], Su));
+    const float g = bf16_round(linear_value(p, m, w_scale_of(p, 0), Sg));
+    const float u = bf16_round(linear_value(p, m, w_scale_of(p, p.nseg > 1 ? 1 : 0), Su));
     const float r = fmaxf(g, 0.f);
     const float h = bf16_round(bf16_round(r * r) * u);
     const int j = (n_g >> 5) * 16 + (n_g & 15);
@@ -88,7 +90,7 @@ __device__ __forceinline__ void epilogue_store_relu2(const EpiParams& p, int m, 
         reinterpret_cast<float*>(p.out)[(size_t)m * p.ldo + j] = h;
 }
 
-int fill_epi(const wf_linear_args* a, EpiParams* p);  // validates + copies (host)
+int fill_epi(const wf_linear_args* a, EpiParams* p, const float* w_scales_host = nullptr);  // validates + copies (host); w_scales_host: the scales by value (null: a->w_scale)
 
 // launchers implemented in the kernel files
 int launch_gemm_mma(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s);

@@ -16,6 +16,7 @@ calling them with CPU tensors raises (no CPU fallback).  `*_cuda`-free aliases a
 """
 import torch
 
+from wf_bitnet import _native
 from wf_bitnet import ops as _wf
 
 _LIB = torch.library.Library("sgl_kernel", "FRAGMENT")
@@ -33,17 +34,8 @@ _DEFS = {
 }
 
 
-def _gemv(packed_weights, activations, scale):
-    return _wf.bitnet_gemv(packed_weights, activations, scale)
-
-
-def _gemm(packed_weights, activations, scale):
-    return _wf.bitnet_gemm(packed_weights, activations, scale)
-
-
-def _quant(activations):
-    q, scale, _ = _wf.quantize_activations(activations, per_token=False)
-    return q, scale
+def _not_built(*args, **kwargs):
+    return _native.ops()          # raises: libwf_torch.so holds these kernels
 
 
 def _fake_gemv(packed_weights, activations, scale):
@@ -106,13 +98,7 @@ def _mlp_forward(x, gate_w, up_w, down_w, gate_scale, up_scale, down_scale, ffn_
     tile, N2, K = _fused_tile("gu", (gate_w, up_w))
     if x2.shape[1] != K:
         raise ValueError("x.shape[-1] != in_features")
-    q8, s, rs = _wf.quantize_activations(x2, per_token=True)
-    ws = torch.tensor([gate_scale, up_scale], dtype=torch.float32, device=x.device)
-    h = _wf.ternary_linear(tile, N2, K, q8, mode="linear", rowsum=rs, act_scale=s, w_scale=ws, relu2_mul=True, out_dtype=torch.bfloat16)
-    q2, s2, rs2, _ = _wf.rmsnorm_quant(h, ffn_sub_norm.to(torch.bfloat16), eps)
-    wd = torch.tensor([down_scale], dtype=torch.float32, device=x.device)
-    y = _wf.ternary_linear(down_w.contiguous(), down_w.shape[0], down_w.shape[1] * 4, q2, layout="i2s", mode="linear", rowsum=rs2, act_scale=s2,
-                           w_scale=wd, out_dtype=torch.bfloat16)
+    y = _native.ops().mlp(x2, tile, N2, down_w, gate_scale, up_scale, down_scale, ffn_sub_norm.to(torch.bfloat16), eps)
     return y.reshape(*x.shape[:-1], down_w.shape[0]).to(x.dtype)
 
 
@@ -125,7 +111,8 @@ def _fake_mlp(x, gate_w, up_w, down_w, gate_scale, up_scale, down_scale, ffn_sub
     return torch.empty(*x.shape[:-1], down_w.shape[0], dtype=x.dtype, device=x.device)
 
 
-_IMPL = {"bitnet_gemv": (_gemv, _fake_gemv), "bitnet_gemm": (_gemm, _fake_gemm), "bitnet_quantize_activations": (_quant, _fake_quant),
+# None: the CUDA kernel is native (csrc/torch_ops.cpp)
+_IMPL = {"bitnet_gemv": (None, _fake_gemv), "bitnet_gemm": (None, _fake_gemm), "bitnet_quantize_activations": (None, _fake_quant),
          "bitnet_qkv_forward": (_qkv_forward, _fake_qkv), "bitnet_mlp_forward": (_mlp_forward, _fake_mlp)}
 
 _registered = False
@@ -137,8 +124,13 @@ def register():
         return
     for name, schema in _DEFS.items():
         _LIB.define(name + schema)
+    built = _native.TORCH_LIB_PATH.exists()
+    if built:
+        _native.ops()
+    for name in _DEFS:
         impl, fake = _IMPL[name.replace("_cpu", "")]
-        _LIB.impl(name, impl, "CUDA")
+        if impl is not None or not built:
+            _LIB.impl(name, impl or _not_built, "CUDA")
         torch.library.register_fake(f"sgl_kernel::{name}", fake, lib=_LIB)
     _registered = True
 

@@ -15,10 +15,14 @@ from typing import Tuple
 import torch
 
 import wf_bitnet
-from wf_bitnet import ops as _ops
 
 BITNET_BLOCK_SIZE = wf_bitnet.BITNET_BLOCK_SIZE  # 128 == QK_I2_S (extern/BitNet/src/ggml-bitnet-mad.cpp:9)
 QK_I2_S = BITNET_BLOCK_SIZE
+
+# the registered ops (sgl_kernel/_ops.py), resolved once
+_GEMV = torch.ops.sgl_kernel.bitnet_gemv_cpu.default
+_GEMM = torch.ops.sgl_kernel.bitnet_gemm_cpu.default
+_QUANT = torch.ops.sgl_kernel.bitnet_quantize_activations_cpu.default
 
 
 def bitnet_check_kernel_available() -> bool:
@@ -37,7 +41,7 @@ def auto_tune_tiles(*args, **kwargs) -> None:
 
 def bitnet_quantize_activations(activations: torch.Tensor) -> Tuple[torch.Tensor, float]:
     """Quantize FP32/BF16 activations to INT8 (per-tensor absmax). Returns (int8 like x, float scale)."""
-    q, scale = torch.ops.sgl_kernel.bitnet_quantize_activations_cpu(activations)
+    q, scale = _QUANT(activations)
     return q, float(scale.item())
 
 
@@ -62,7 +66,7 @@ def bitnet_gemv(packed_weights: torch.Tensor, activations: torch.Tensor, scale: 
     if activations.dtype != torch.int8:
         raise ValueError("activations must be int8")
     _check(packed_weights, activations.shape[0])
-    return torch.ops.sgl_kernel.bitnet_gemv_cpu(packed_weights, activations, float(scale))
+    return _GEMV(packed_weights, activations, float(scale))
 
 
 def bitnet_gemm(packed_weights: torch.Tensor, activations: torch.Tensor, scale: float) -> torch.Tensor:
@@ -72,4 +76,4 @@ def bitnet_gemm(packed_weights: torch.Tensor, activations: torch.Tensor, scale: 
     if activations.dtype != torch.int8:
         raise ValueError("activations must be int8")
     _check(packed_weights, activations.shape[1])
-    return torch.ops.sgl_kernel.bitnet_gemm_cpu(packed_weights, activations, float(scale))
+    return _GEMM(packed_weights, activations, float(scale))

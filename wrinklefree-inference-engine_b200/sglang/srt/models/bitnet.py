@@ -84,17 +84,12 @@ class BitNetLinear(nn.Module):
         return self
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        o = _ops()
+        from wf_bitnet import _native
         src = x.device
         xf = _dev(x).reshape(-1, self.in_features)
-        q, act_scale, rowsum = o.quantize_activations(xf, per_token=False)
-        if self._tile is not None:
-            w, layout = self._tile, "tile"
-        else:
-            w, layout = _dev(self.qweight.data).contiguous(), "i2s"
-        out = o.ternary_linear(w, self.out_features, self.in_features, q, layout=layout, mode="linear", rowsum=rowsum,
-                               act_scale=act_scale, w_scale=_dev(self.weight_scale.data).float().reshape(-1)[:1],
-                               out_dtype=torch.float32)
+        tile = self._tile is not None
+        out = _native.ops().linear(xf, self._tile if tile else _dev(self.qweight.data), tile, self.out_features, self.in_features,
+                                   _dev(self.weight_scale.data).float().reshape(-1)[:1])
         if self.bias is not None:
             out = out + _dev(self.bias.data)
         return out.view(*x.shape[:-1], self.out_features).to(src)

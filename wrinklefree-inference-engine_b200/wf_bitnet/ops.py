@@ -11,7 +11,7 @@ from typing import Optional, Sequence, Tuple
 
 import torch
 
-from . import _lib
+from . import _lib, _native
 from ._lib import (WF_BF16, WF_EPI_RELU2_MUL, WF_EPI_RESIDUAL, WF_F16, WF_F32, WF_I8, WF_OUT_COMPAT_F32, WF_OUT_I32,
                    WF_OUT_I32_PLUS1, WF_OUT_LINEAR, WF_W_I2S, WF_W_TILE, KvLayout, LinearArgs, check, lib)
 
@@ -289,26 +289,14 @@ def rope_kv_append(qkv: torch.Tensor, H: int, kv: PagedKV, layer: int, positions
     return q_out
 
 
-_attn_ws = {}
-
-
 def paged_decode_attn(q: torch.Tensor, kv: PagedKV, layer: int, block_table: torch.Tensor, seq_lens: torch.Tensor,
                       scale: Optional[float] = None, out_dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
-    _need_cuda(q, block_table, seq_lens)
-    B, H, D = q.shape
-    if scale is None:
-        scale = 1.0 / (D ** 0.5)
-    out = torch.empty(B, H, D, dtype=out_dtype, device=q.device)
-    max_seq = block_table.shape[1] * kv.page_size
-    nbytes = int(lib().wf_attn_workspace_bytes(B, H, D, max_seq))
-    key = (q.device.index, _stream())
-    ws = _attn_ws.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
-        _attn_ws[key] = ws
-    check(lib().wf_paged_decode_attn(q.contiguous().data_ptr(), kv.ref(), layer, block_table.data_ptr(), block_table.shape[1],
-                                     seq_lens.data_ptr(), B, H, float(scale), out.data_ptr(), _DT[out_dtype], ws.data_ptr(), ws.numel(), _stream()))
-    return out
+    if not (q.is_cuda and block_table.is_cuda and seq_lens.is_cuda):
+        _need_cuda(q, block_table, seq_lens)
+    _DT[out_dtype]
+    c = kv.c
+    return _native.ops().paged_decode_attn(q, kv.raw if kv.dtype == torch.int8 else kv.pool, c.max_pages, c.layers, c.kv_heads, c.page_size, c.head_dim, c.dtype, layer,
+                                           block_table, seq_lens, 1.0 / (q.shape[-1] ** 0.5) if scale is None else scale, out_dtype)
 
 
 # ----------------------------------------------------------------------------------------- glue

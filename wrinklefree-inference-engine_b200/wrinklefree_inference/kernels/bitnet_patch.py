@@ -57,15 +57,13 @@ class BitNetLinearNative(nn.Module):
             self.bias = None
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        from wf_bitnet import ops
+        from wf_bitnet import _native
         batch_shape = x.shape[:-1]
         x_flat = x.reshape(-1, self.in_features)
         if not x_flat.is_cuda:
             x_flat = x_flat.to(self.packed_weight.device)
         # per-tensor absmax like bitnet_quantize_activations(x_flat) (reference :62)
-        q, act_scale, rowsum = ops.quantize_activations(x_flat, per_token=False)
-        out = ops.ternary_linear(self.tile_weight, self.out_features, self.in_features, q, layout="tile", mode="linear",
-                                 rowsum=rowsum, act_scale=act_scale, w_scale=self.weight_scale, out_dtype=torch.float32)
+        out = _native.ops().linear(x_flat, self.tile_weight, True, self.out_features, self.in_features, self.weight_scale)
         if self.bias is not None:
             out = out + self.bias
         return out.view(*batch_shape, self.out_features)
