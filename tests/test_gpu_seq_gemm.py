@@ -1,0 +1,42 @@
+"""The sequence engine's matrix product on tensor cores: CTA pairs (token tiles that are no whole tile, rows that leave the second CTA empty, several rounds
+of tiles) and the few-row form (row tiles short of 16, K that is no multiple of its steps, each split of the work).
+
+Tolerance: float sums of K bf16 products in another order, a few times 2^-24 sqrt(K) of the operands' unit scale; 2e-5 covers K = 7000 on the tcgen05 sum."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def product(A, B, algo, c_f32=True):
+    from wf_bitnet._lib import seq_check, seq_lib
+    (M, K), N = A.shape, B.shape[0]
+    C = torch.full((M, N), float("nan"), dtype=torch.float32 if c_f32 else torch.bfloat16, device="cuda")
+    seq_check(seq_lib().wf_seq_op_gemm(1, A.data_ptr(), 0, K, B.data_ptr(), K, C.data_ptr(), 1 if c_f32 else 0, N, M, N, K, None, 0, 1, algo,
+                                       torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    return C
+
+
+def operands(M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M + 3 * N + 7 * K)
+    return torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16), (torch.randn(N, K, device="cuda", generator=g) / math.sqrt(K)).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 8, 8), (33, 129, 72), (255, 257, 64), (257, 255, 200), (1000, 130, 1032), (530, 2561, 320), (2049, 1024, 6912), (3000, 5000, 64)])
+def test_pair_product(M, N, K):
+    A, B = operands(M, N, K)
+    want = A.double() @ B.double().T
+    assert (product(A, B, 3).double() - want).abs().max() < 2e-5 * (1 + want.abs().max())
+    assert (product(A, B, 3, c_f32=False).double() - want).abs().max() < 2.0 ** -8 * (1 + want.abs().max())
+
+
+@pytest.mark.parametrize("M", [1, 3, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(1, 8), (15, 40), (17, 72), (1000, 2304), (2560, 6912), (4737, 264), (9473, 1000), (30000, 136)])
+def test_few_rows(M, N, K):
+    A, B = operands(M, N, K)
+    want = A.double() @ B.double().T
+    assert (product(A, B, 5).double() - want).abs().max() < 5e-6 * (1 + want.abs().max())
+    assert (product(A, B, 5, c_f32=False).double() - want).abs().max() < 2.0 ** -8 * (1 + want.abs().max())

@@ -323,6 +323,102 @@ void gemv_launch(const GemmArgs& g, const PairArgs& pa, int rows, int ny, cudaSt
     else gemv_dispatch<T, 8>(g, pa, grid, s);
 }
 
+// ---- few-row form on tensor cores (bf16 operands, decoding): 16 weight rows per warp as the M side of mma.sync.m16n8k16, the activation rows as its N
+// side, so that a loaded weight serves all rows in two MMAs per 32 k instead of being multiplied row by row.  A lane loads 16 consecutive bytes of a
+// row: the four lanes of a row hold k 8 t .. 8 t + 7, and weights and activations are permuted over k alike, so no shuffle is needed.  The WK
+// warps of a tile take 64-k steps in turn (a short, wide product has too few rows to cover the machine otherwise) and meet in shared memory.
+// Every warp keeps four sums apart and all partial sums are added in float, which holds the error at the fused-multiply-add kernel's (4e-7 to 1e-6).
+// Bound: the weight stream, by latency on small matrices.  Measured with 8 rows against gemv_rows_kernel: 1024 x 2304 23.1 -> 9.3 us, 2560 x 6912
+// 64.6 -> 12.5, 13824 x 2560 43.7 -> 14.8, 128256 x 2560 298 -> 102; with 16 rows against gemm_mma_kernel: 2560 x 6912 131 -> 12.6.
+constexpr int FR_WARPS = 8;
+
+// U: 32-k blocks in flight per warp; OCC: blocks per SM
+template <int NT, int WK, int U, int OCC, bool CF32>
+__global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g) {
+    constexpr int TILES = FR_WARPS / WK;                  // 16-row tiles per block
+    constexpr int C = 4;                                  // independent sums, added in float at the end
+    __shared__ float part[FR_WARPS][NT * 8][16 + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g4 = lane >> 2, t4 = lane & 3;
+    const int tile = warp / WK, kw = warp % WK;
+    const int n0 = (blockIdx.x * TILES + tile) * 16;
+    const __nv_bfloat16 *B = (const __nv_bfloat16*)g.B, *A = (const __nv_bfloat16*)g.A;
+    const int ra = min(n0 + g4, g.N - 1), rb = min(n0 + g4 + 8, g.N - 1);          // rows past N repeat the last one; they are not stored
+    const __nv_bfloat16 *wa = B + (size_t)ra * g.ldb + 8 * t4, *wb = B + (size_t)rb * g.ldb + 8 * t4;
+    const __nv_bfloat16* xa[NT];
+    bool x_ok[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) { const int m = j * 8 + g4; x_ok[j] = m < g.M; xa[j] = A + (size_t)(x_ok[j] ? m : 0) * g.lda + 8 * t4; }
+    float acc[C][NT][4];
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) acc[c][j][0] = acc[c][j][1] = acc[c][j][2] = acc[c][j][3] = 0.f;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    const int blocks = (g.K + 31) / 32;                   // block i of this warp: steps of 64 k (two blocks) dealt to the WK warps in turn
+    for (int i0 = 0; ; i0 += U) {
+        const int first = ((i0 >> 1) * WK + kw) * 2;
+        if (first >= blocks) break;
+        uint4 a[U], b[U], x[U][NT];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int blk = (((i0 + u) >> 1) * WK + kw) * 2 + ((i0 + u) & 1), k = blk * 32;
+            const bool ok = blk < blocks && k + 8 * t4 + 8 <= g.K;
+            a[u] = ok ? __ldg(reinterpret_cast<const uint4*>(wa + k)) : zero;
+            b[u] = ok ? __ldg(reinterpret_cast<const uint4*>(wb + k)) : zero;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) x[u][j] = ok && x_ok[j] ? *reinterpret_cast<const uint4*>(xa[j] + k) : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t f0[4] = {a[u].x, b[u].x, a[u].y, b[u].y}, f1[4] = {a[u].z, b[u].z, a[u].w, b[u].w};
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                const uint32_t x0[2] = {x[u][j].x, x[u][j].y}, x1[2] = {x[u][j].z, x[u][j].w};
+                mma_bf16_16816(acc[u % C][j], f0, x0);
+                mma_bf16_16816(acc[u % C][j], f1, x1);
+            }
+        }
+    }
+    // acc: rows g4 (0, 1) and g4 + 8 (2, 3), activation rows 2 t4 and 2 t4 + 1
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) part[warp][j * 8 + 2 * t4 + (e & 1)][g4 + 8 * (e >> 1)] = (acc[0][j][e] + acc[1][j][e]) + (acc[2][j][e] + acc[3][j][e]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < TILES * NT * 8 * 16; i += FR_WARPS * 32) {
+        const int r = i & 15, m = (i >> 4) % (NT * 8), t = (i >> 4) / (NT * 8);
+        const int n = (blockIdx.x * TILES + t) * 16 + r;
+        if (n >= g.N || m >= g.M) continue;
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < WK; ++w) v += part[t * WK + w][m][r];
+        v = epilogue_f(g.ep, v);
+        if (CF32) ((float*)g.C)[(size_t)m * g.ldc + n] = v;
+        else ((__nv_bfloat16*)g.C)[(size_t)m * g.ldc + n] = __float2bfloat16_rn(v);
+    }
+}
+
+template <int NT, int WK, int U, int OCC>
+void few_launch(const GemmArgs& g, cudaStream_t s) {
+    const int tiles = (g.N + 15) / 16, per = FR_WARPS / WK, blocks = (tiles + per - 1) / per;
+    if (g.c_f32) gemm_few_kernel<NT, WK, U, OCC, true><<<blocks, FR_WARPS * 32, 0, s>>>(g); else gemm_few_kernel<NT, WK, U, OCC, false><<<blocks, FR_WARPS * 32, 0, s>>>(g);
+}
+// Which split: a warp wants many loads in flight while there are fewer row tiles than SMs (2560 x 6912: 14.4 us, 15.7 with half as many), blocks of two
+// tiles fit one wave up to two per SM (12.4 us), and beyond that resident blocks cover the latency (13824 x 2560: 14.6 us against 22.7 / 18.6 with
+// the first two; 128256 x 2560: 99 against 162 / 128).  With 9 to 16 rows the registers hold half as much in flight and a second block stays resident.
+template <int NT>
+void few_dispatch(const GemmArgs& g, cudaStream_t s) {
+    const int tiles = (g.N + 15) / 16, sms = sm_count();
+    if (NT == 1) {
+        if (tiles <= sms) few_launch<1, 8, 8, 1>(g, s);
+        else if (tiles <= 2 * sms) few_launch<1, 4, 8, 1>(g, s);
+        else few_launch<1, 4, 4, 4>(g, s);
+    } else {
+        if (tiles <= 4 * sms) few_launch<2, 8, 4, 1>(g, s);
+        else few_launch<2, 2, 4, 2>(g, s);
+    }
+}
+
 template <typename T>
 void simt_dispatch(const GemmArgs& g, dim3 grid, cudaStream_t s) {
     if (g.a_f32) { if (g.c_f32) gemm_simt_kernel<T, true, true><<<grid, 256, 0, s>>>(g); else gemm_simt_kernel<T, true, false><<<grid, 256, 0, s>>>(g); }
@@ -339,6 +435,11 @@ int launch_gemm(int dt, const GemmArgs& g, cudaStream_t s) {
     if (g_tc_min < 0) { const char* e = getenv("WF_SEQ_TC_MIN"); g_tc_min = e ? atoi(e) : 17; }
     if (g_force_simt < 0) { const char* e = getenv("WF_SEQ_GEMM_SIMT"); g_force_simt = (e && atoi(e)) ? 1 : 0; }
     const bool few = g.batch == 1 && !g.tile_group && !g.a_rows && g.M <= 8;
+    if (g.batch == 1 && !g.tile_group && !g.a_rows && g.M <= 16 && dt == WF_BF16 && !g.a_f32 && !g_force_simt && (g.algo == 0 || g.algo == 5) && gemv_ok<__nv_bfloat16>(g)) {
+        if (g.M <= 8) few_dispatch<1>(g, s); else few_dispatch<2>(g, s);
+        return launch_check(cudaGetLastError(), "gemm_few");
+    }
+    if (g.algo == 5) { set_error("gemm: the few-row tensor-core form does not take this shape"); return WF_ERR_UNSUPPORTED; }
     if ((g.algo == 0 && few) || g.algo == 4) {      // decoding: stream the weights once
         const PairArgs none{nullptr, 0, 1};
         if (few && dt == WF_F32 && gemv_ok<float>(g)) { gemv_launch<float>(g, none, g.M, 1, s); return launch_check(cudaGetLastError(), "gemv_rows"); }

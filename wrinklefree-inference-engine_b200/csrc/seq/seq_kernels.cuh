@@ -115,7 +115,7 @@ struct GemmArgs {
     const int32_t* a_rows = nullptr;
     int n_groups = 1;                        // weight matrices stacked behind B (grouped form)
     int ep = EP_NONE;
-    int algo = 0;                            // 0 = choose; 1 plain FMA, 2 mma.sync, 3 tcgen05, 4 few-row streaming (tests and measurements)
+    int algo = 0;                            // 0 = choose; 1 plain FMA, 2 mma.sync, 3 tcgen05, 4 few-row streaming, 5 few rows on mma.sync (tests and measurements)
 };
 constexpr int GEMM_BM = 128;                 // row granule of the grouped form (the token tile of the tcgen05 kernel)
 int launch_gemm(int dt, const GemmArgs& g, cudaStream_t s);
