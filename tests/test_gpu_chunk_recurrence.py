@@ -1,0 +1,74 @@
+"""The 16-token form of the matrix-state recurrences against the oracles, in float32: every length around its chunks, long portions in parallel segments,
+portions behind carried states, several sequences side by side, key sizes that do not fill a thread's rows, value sizes that do not fill a block.
+
+Tolerance: float32 sums over at most a few hundred terms of order one in another order, relative to a row's RMS; the delta rule's correction solves
+a 16 x 16 triangular system per chunk, whose condition the unit-length keys and beta < 1 keep below a few tens: 2e-4, as for the token form."""
+import numpy as np
+import pytest
+import torch
+
+import fivedra_oracle as FO
+import nukezen_oracle as NO
+
+pytestmark = pytest.mark.gpu
+CUTS = [([70], [[70]]), ([33, 100], [[33, 100]]), ([90, 64], [[32, 0], [15, 47], [43, 16], [0, 1]]), ([47], [[47]]), ([545, 140], [[21, 0], [524, 140]])]
+EPS = 1e-5
+
+
+def check(cfg, weights, shapes, wants, lens, cuts, W):
+    from wf_bitnet import registry
+    cls = registry.resolve(cfg)
+    extra = {"shapes": shapes} if getattr(cls, "reads_shapes", False) else {}
+    m = cls(cfg, dtype="float32", max_tokens=800, slots=4, page_size=16, max_step_tokens=672, **extra)
+    m.load_weights((k, v.numpy(), "F32") for k, v in weights.items())
+    g = np.random.default_rng(sum(lens))
+    rows = [g.standard_normal((n, W)).astype(np.float32) for n in lens]
+    slots, fed = [m.admit() for _ in rows], [0] * len(rows)
+    want = [wants(torch.from_numpy(r).double()).numpy() for r in rows]
+    for step in cuts:
+        act = [i for i, c in enumerate(step) if c]
+        got = m.engine.run_part(0, 2, [slots[i] for i in act], [step[i] for i in act], np.concatenate([rows[i][fed[i]:fed[i] + step[i]] for i in act]))
+        w = np.concatenate([want[i][fed[i]:fed[i] + step[i]] for i in act])
+        err = np.sqrt(((got - w) ** 2).mean(-1)) / np.sqrt((w ** 2).mean(-1))
+        assert err.max() < 2e-4, (step, int(err.argmax()), err.max())
+        for i in act:
+            fed[i] += step[i]
+    m.close()
+
+
+def d64(w, p):
+    return {k[len(p):]: v.double() for k, v in w.items() if k.startswith(p)}
+
+
+@pytest.mark.parametrize("lens,cuts", CUTS)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(4, 2, 128, 128), (2, 2, 36, 20), (40, 20, 64, 96), (3, 1, 68, 33)])
+def test_delta_rule_with_a_decay_per_row(heads, kv_heads, dim, vdim, lens, cuts):
+    W = 40
+    m = {"heads": heads, "kv_heads": kv_heads, "dim": dim, "vdim": vdim, "conv": 4}
+    cfg = {"architecture": "Nukezen", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": EPS}, "layers": [{"type": "channel_delta", "mixer": m, "mlp": None}]}
+    w = NO.random_weights(cfg, 1, {0: {"rank_a": 8, "rank_g": 8}})
+    check(cfg, w, {"l0.mix.a1": (8, W), "l0.mix.g1": (8, W)}, lambda x: NO.channel_delta(x, d64(w, "l0.mix."), "", m, EPS), lens, cuts, W)
+
+
+@pytest.mark.parametrize("lens,cuts", CUTS)
+@pytest.mark.parametrize("heads,groups,state,vdim", [(4, 2, 128, 64), (6, 3, 20, 12), (80, 5, 64, 64)])
+def test_state_space(heads, groups, state, vdim, lens, cuts):
+    W = 40
+    left = {"heads": 2, "kv_heads": 1, "dim": 8, "vdim": 8, "scale": 0.3, "mask": {"size": 8}, "rot": {"dims": 8, "base": 10000.0}}
+    right = {"heads": heads, "vdim": vdim, "state": state, "groups": groups, "conv": 4, "norm_groups": groups}
+    cfg = {"architecture": "Nukezen", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": EPS},
+           "layers": [{"type": "parallel", "mixer": {"left": left, "left_scale": 0.0, "right": right, "right_scale": 1.0}, "mlp": None}]}
+    w = NO.random_weights(cfg, 2)
+    check(cfg, w, {}, lambda x: NO.state_space(x, d64(w, "l0.mix.right."), "", right, EPS), lens, cuts, W)
+
+
+@pytest.mark.parametrize("lens,cuts", CUTS)
+@pytest.mark.parametrize("heads,dim,vdim", [(4, 128, 128), (3, 24, 15)])
+def test_matrix_memory(heads, dim, vdim, lens, cuts):
+    W = 40
+    left = {"heads": 2, "kv_heads": 1, "dim": 8, "vdim": 8, "scale": 0.3, "mask": {"size": 8}, "bias_max": 16}
+    right = {"heads": heads, "dim": dim, "vdim": vdim, "gate_cap": 15.0}
+    cfg = {"architecture": "Fivedra", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": EPS},
+           "layers": [{"type": "parallel", "mixer": {"left": left, "left_scale": 0.0, "right": right, "right_scale": 1.0}, "mlp": None}]}
+    w = FO.random_weights(cfg, 3)
+    check(cfg, w, {"l0.mix.left.rel": (8, 2)}, lambda x: FO.matrix_memory(x, d64(w, "l0.mix.right."), "", right, EPS), lens, cuts, W)

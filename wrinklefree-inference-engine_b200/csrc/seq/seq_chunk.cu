@@ -1,0 +1,479 @@
+// The matrix-state recurrences of seq_delta.cu over prompt portions, 16 tokens at a time instead of one by one.  With S the state before a chunk, c_j the
+// product of the decays of tokens 1 .. j and D(i, j) that of tokens i + 1 .. j (diagonal over the key rows, or a number):
+//     R_j = S^T (c_j k_j),   A_ji = k_i^T D(i, j) k_j (i < j),   u_j = beta_j (v_j - R_j - sum_{i<j} A_ji u_i)      -> U = T (V - R),
+//     o_j = S^T (c_j q_j) + sum_{i<=j} B_ji u_i with B_ji = k_i^T D(i, j) q_j,   S <- c_16 S + sum_j (D(j, 16) k_j) u_j^T.
+// Without the correction (state-space, gated linear attention, matrix memory) U = beta V.
+//   * chunk_prep_kernel, a block per (chunk, head): T = (I + beta A)^-1 beta and B, and with a decay per key row the decayed k and q rows;
+//   * chunk_scan_kernel, a block per (sequence, head, 16 columns): walks the chunks in order, the next one's rows under way by cp.async.  All products run
+//     on mma.sync m16n8k8 with every operand as a sum of two tf32 numbers (hi hi + hi lo + lo hi, 22 to 24 bits of each product) and float sums; the
+//     state stays in float registers, as S^T in accumulator layout, which with the key rows of an 8-row tile taken in the order 0 2 4 6 1 3 5 7 is also
+//     the operand layout of S^T k, so it is never moved.  The four warps share the 16 columns and split the key rows; their partial R and S^T q meet in
+//     shared memory once per chunk.
+// What bounded the forms before: token by token, a chain of multiply-adds, shuffles and shared-memory reads of about 1000 clk per token; chunks on
+// the multiply-add units, shared-memory bandwidth (every thread of a column reads every key: 5 wavefronts per request, 450 us for the case below).
+// Measured at 2048 tokens: delta rule (20 heads, 128 x 128, two sequences) 569 -> 231 us (48 of them the preparation), state space (40 heads, 128 x 64, one
+// sequence) 307 -> 202 us (32); eight warps with half the rows each 287 and 257 us (both in one pass).  Left: the chain of a chunk, about 3000 clk of products, one exchange of
+// partial sums and two barriers.  Error against 64 bits in float32 layers up to 1500 tokens long: 3.6e-7 to 5.6e-7, as token by token.
+// A token whose key, query or value is infinite or NaN makes its whole chunk's read-out NaN, and the state, as before, for good.
+#include "seq_kernels.cuh"
+
+namespace wf {
+namespace seq {
+
+namespace {
+
+constexpr int CR = CHUNK_TOKENS, CR_WARPS = 4, CR_THREADS = 32 * CR_WARPS, CR_COLS = 16;
+static_assert(CR == 16, "a chunk is two 8-token tiles");
+
+__device__ __forceinline__ void cr_cp16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+struct ChunkView {
+    const float *qkv, *beta, *decay; int ld, q_off, k_off, v_off;
+    float* rec;
+    int nchunks;
+};
+
+// one of the two passes over segments of SCAN_CHUNK tokens in parallel (recurrences linear in the state): pass 1 leaves each segment's own end state (from a
+// zero one) and, with one decay per head, the product of its decays; pass 3 reads the segments' start states, chained by scan_prefix_kernel; 0: whole portions
+struct Segments { int pass = 0, n = 1; float *local = nullptr, *prod = nullptr; const float* start = nullptr; };
+
+// a record: [T 256][B 256] then, decay per row: [c_j q_j 16 DS][c_j k_j 16 DS][D(j, 16) k_j 16 DS][c_16 DS]; one decay: [c_j 16][D(j, 16) 16][c_16, padding]
+// (DS: the key rows, padded to 64 or 128)
+__host__ __device__ constexpr int cr_rec_floats(int DS, bool vec) { return vec ? 512 + (3 * CR + 1) * DS : 512 + 48; }
+
+// transposed sum over 16 lanes: v[t] of all of them -> the sum of t = p for lane p
+__device__ __forceinline__ float cr_reduce(float (&v)[CR], int p) {
+#pragma unroll
+    for (int w = 8; w >= 1; w >>= 1) {
+        const bool up = (p & w) != 0;
+#pragma unroll
+        for (int k = 0; k < w; ++k) {
+            const float send = up ? v[k] : v[w + k], keep = up ? v[w + k] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+        }
+    }
+    return v[0];
+}
+
+template <int DS, bool VEC, bool DELTA>
+__global__ void __launch_bounds__(CR_THREADS) chunk_prep_kernel(Batch b, DeltaDims D, ChunkView w) {
+    constexpr int Q4 = DS / 64;             // float4 per lane part
+    __shared__ __align__(16) float ks[CR][DS], qs[CR][DS], gs[VEC ? CR : 1][VEC ? DS : 4];
+    __shared__ float As[CR][CR + 1], Bs[CR][CR + 1], gsc[CR], bt[CR];
+    const int sq = blockIdx.x / w.nchunks, ch = blockIdx.x - sq * w.nchunks, h = blockIdx.y;
+    const int len = b.seq_len[sq], start = b.seq_start[sq] + ch * CR, left = min(CR, len - ch * CR);
+    if (left <= 0) return;
+    const int tid = threadIdx.x, kh = h / (D.H / D.Hk);
+    float* rec = w.rec + ((size_t)(b.seq_start[sq] / CR + sq + ch) * D.H + h) * cr_rec_floats(DS, VEC);
+    for (int i = tid; i < CR * (DS / 4); i += CR_THREADS) {
+        const int t = i / (DS / 4), c = (i - t * (DS / 4)) * 4;
+        float4 k = make_float4(0.f, 0.f, 0.f, 0.f), q = k, g = make_float4(1.f, 1.f, 1.f, 1.f);
+        if (t < left && c < D.d) {
+            const float* row = w.qkv + (size_t)(start + t) * w.ld;
+            k = *reinterpret_cast<const float4*>(row + w.k_off + kh * D.d + c);
+            q = *reinterpret_cast<const float4*>(row + w.q_off + kh * D.d + c);
+            if (VEC) g = *reinterpret_cast<const float4*>(w.decay + ((size_t)(start + t) * D.H + h) * D.d + c);
+        }
+        *reinterpret_cast<float4*>(&ks[t][c]) = k;
+        *reinterpret_cast<float4*>(&qs[t][c]) = q;
+        if (VEC) *reinterpret_cast<float4*>(&gs[t][c]) = g;
+    }
+    if (tid < CR) {
+        bt[tid] = tid < left ? (w.beta ? w.beta[(size_t)(start + tid) * D.H + h] : 1.f) : 0.f;
+        if (!VEC) gsc[tid] = tid < left ? w.decay[(size_t)(start + tid) * D.H + h] : 1.f;
+    }
+    __syncthreads();
+    // ---- A and B: a thread takes the earlier tokens i and 15 - i and a sixteenth of the key rows, and runs over the later tokens j with the decayed keys in hand
+    {
+        const int p = tid & 15, i0 = tid >> 4, i1 = CR - 1 - i0;      // i0 < i1
+        float a0[CR], a1[CR], b0[CR], b1[CR];
+#pragma unroll
+        for (int j = 0; j < CR; ++j) a0[j] = a1[j] = b0[j] = b1[j] = 0.f;
+#pragma unroll
+        for (int m = 0; m < Q4; ++m) {
+            const int c = (p + 16 * m) * 4;
+            float4 x = *reinterpret_cast<const float4*>(&ks[i0][c]), y = *reinterpret_cast<const float4*>(&ks[i1][c]);
+#pragma unroll
+            for (int j = 0; j < CR; ++j) {
+                if (j < i0) continue;
+                const float4 q = *reinterpret_cast<const float4*>(&qs[j][c]);
+                float4 g, k;
+                if (VEC) g = *reinterpret_cast<const float4*>(&gs[j][c]);
+                if (DELTA) k = *reinterpret_cast<const float4*>(&ks[j][c]);
+                if (j > i0) {
+                    if (VEC) { x.x *= g.x; x.y *= g.y; x.z *= g.z; x.w *= g.w; }
+                    if (DELTA) a0[j] = fmaf(x.x, k.x, fmaf(x.y, k.y, fmaf(x.z, k.z, fmaf(x.w, k.w, a0[j]))));
+                }
+                b0[j] = fmaf(x.x, q.x, fmaf(x.y, q.y, fmaf(x.z, q.z, fmaf(x.w, q.w, b0[j]))));
+                if (j < i1) continue;
+                if (j > i1) {
+                    if (VEC) { y.x *= g.x; y.y *= g.y; y.z *= g.z; y.w *= g.w; }
+                    if (DELTA) a1[j] = fmaf(y.x, k.x, fmaf(y.y, k.y, fmaf(y.z, k.z, fmaf(y.w, k.w, a1[j]))));
+                }
+                b1[j] = fmaf(y.x, q.x, fmaf(y.y, q.y, fmaf(y.z, q.z, fmaf(y.w, q.w, b1[j]))));
+            }
+        }
+        float s0 = DELTA ? cr_reduce(a0, p) : 0.f, s1 = DELTA ? cr_reduce(a1, p) : 0.f, t0 = cr_reduce(b0, p), t1 = cr_reduce(b1, p);   // token j = p
+        if (!VEC) {
+            float pr = 1.f;
+            for (int j = CR - 1; j > i0; --j) if (j <= p) pr *= gsc[j];
+            s0 *= pr; t0 *= pr;
+            pr = 1.f;
+            for (int j = CR - 1; j > i1; --j) if (j <= p) pr *= gsc[j];
+            s1 *= pr; t1 *= pr;
+        }
+        if (DELTA) { As[p][i0] = s0; As[p][i1] = s1; }
+        Bs[p][i0] = t0; Bs[p][i1] = t1;
+    }
+    __syncthreads();
+    if (DELTA && tid < CR) {                              // column tid of (I + beta A)^-1, by forward substitution, times beta
+        float x[CR];
+#pragma unroll
+        for (int j = 0; j < CR; ++j) {
+            float v = 0.f;
+#pragma unroll
+            for (int l = 0; l < j; ++l) v = fmaf(As[j][l], x[l], v);     // x[l] = 0 for l < tid
+            x[j] = j == tid ? 1.f : j > tid ? -bt[j] * v : 0.f;
+            rec[j * CR + tid] = x[j] * bt[tid];
+        }
+    }
+    for (int i = tid; i < CR * CR; i += CR_THREADS) rec[256 + i] = Bs[i >> 4][i & 15];
+    if (VEC) {
+        float *qt = rec + 512, *kt = qt + CR * DS, *kn = kt + CR * DS, *ge = kn + CR * DS;
+        for (int c = tid; c < DS; c += CR_THREADS) {
+            float cum = 1.f;
+#pragma unroll
+            for (int t = 0; t < CR; ++t) {
+                cum *= gs[t][c];
+                qt[t * DS + c] = qs[t][c] * cum;
+                if (DELTA) kt[t * DS + c] = ks[t][c] * cum;
+            }
+            ge[c] = cum;
+            float suf = 1.f;
+#pragma unroll
+            for (int t = CR - 1; t >= 0; --t) { kn[t * DS + c] = ks[t][c] * suf; suf *= gs[t][c]; }
+        }
+    } else if (tid < CR) {
+        float cum = 1.f, suf = 1.f;
+        for (int t = 0; t <= tid; ++t) cum *= gsc[t];
+        for (int t = tid + 1; t < CR; ++t) suf *= gsc[t];
+        rec[512 + tid] = cum; rec[528 + tid] = suf;
+        if (tid == CR - 1) rec[544] = cum;
+    }
+}
+
+__device__ __forceinline__ void cr_split(float x, uint32_t& hi, uint32_t& lo) {
+    // round to 10 stored bits by integer arithmetic (the conversion instruction runs at a fraction of its rate); the instruction drops the low 13 bits of lo
+    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
+}
+__device__ __forceinline__ void cr_mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+struct CrA { uint32_t h[4], l[4]; };
+struct CrB { uint32_t h[2], l[2]; };
+// an accumulator tile as the A operand: columns 2 t and 2 t + 1 become k = t and t + 4
+__device__ __forceinline__ CrA cr_a(const float (&c)[4]) {
+    CrA a;
+    cr_split(c[0], a.h[0], a.l[0]); cr_split(c[2], a.h[1], a.l[1]); cr_split(c[1], a.h[2], a.l[2]); cr_split(c[3], a.h[3], a.l[3]);
+    return a;
+}
+__device__ __forceinline__ CrB cr_b(float x, float y) {
+    CrB b;
+    cr_split(x, b.h[0], b.l[0]); cr_split(y, b.h[1], b.l[1]);
+    return b;
+}
+__device__ __forceinline__ CrB cr_b2(const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return cr_b(v.x, v.y); }
+__device__ __forceinline__ void cr_mma3(float (&d)[4], const CrA& a, const CrB& b) { cr_mma(d, a.l, b.h); cr_mma(d, a.h, b.l); cr_mma(d, a.h, b.h); }
+
+template <int DS, bool VEC, bool DELTA> struct CrStage {
+    static constexpr int QS = DS + 8, KS = DS + 4;        // row strides: pairs of rows 8 tokens apart, single rows 2 tokens apart, each without bank conflicts
+    static constexpr int TS = 24;                         // of T and B
+    static constexpr int T = 0, B = T + (DELTA ? CR * TS : 0), Q = B + CR * TS, K = Q + CR * QS, N = K + (DELTA ? CR * QS : 0), G = N + CR * KS,
+                         FLOATS = G + (VEC ? DS : 48);    // G: c_16 per row, or [c_j][D(j, 16)][c_16]
+};
+constexpr int CR_RS = 24;                                 // row stride of the partial sums [16 columns][16 tokens]
+
+template <int DS, bool VEC, bool DELTA>
+__global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
+    using L = CrStage<DS, VEC, DELTA>;
+    constexpr int REC = cr_rec_floats(DS, VEC), NT = DS / (8 * CR_WARPS), STEP = CR_THREADS / (DS / 4);
+    extern __shared__ __align__(16) float sm[];
+    float* red = sm + 2 * L::FLOATS;                      // [4 warps][S^T q | R][16 columns][CR_RS]
+    const int sq = blockIdx.x / sg.n, seg = blockIdx.x - sq * sg.n, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int col0 = blockIdx.z * CR_COLS, dvs = D.dv + D.ones_col, kh = h / (D.H / D.Hk);
+    const int first = seg * SCAN_CHUNK, seq0 = b.seq_start[sq], start = seq0 + first;
+    const int len = sg.pass ? min(SCAN_CHUNK, b.seq_len[sq] - first) : b.seq_len[sq], nch = (len + CR - 1) / CR;
+    if (len <= 0) return;                                 // this sequence has fewer segments
+    const size_t entry = ((size_t)(seq0 / SCAN_CHUNK + sq + seg) * D.H + h) * D.d * dvs;
+    const float* S0 = sg.pass == 3 ? sg.start + entry : state + (size_t)b.seq_slot[sq] * slot_stride + (size_t)h * D.d * dvs;
+    const float* rec0 = w.rec + ((size_t)(seq0 / CR + sq + first / CR) * D.H + h) * REC;
+    float prod = 1.f;
+    const int row0 = warp * 8 * NT;                       // this warp's key rows
+    // s[nt]: columns col0 + g (0, 1) and col0 + g + 8 (2, 3), rows row0 + 8 nt + 2 t (0, 2) and + 1 (1, 3)
+    float s[NT][4];
+    auto at_state = [&](int nt, int e, bool& ok) -> size_t {
+        const int r = row0 + 8 * nt + 2 * t + (e & 1), c = col0 + g + 8 * (e >> 1);
+        ok = r < D.d && c < dvs;
+        return (size_t)r * dvs + c;
+    };
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { bool ok; const size_t i = at_state(nt, e, ok); s[nt][e] = ok && sg.pass != 1 ? S0[i] : 0.f; }
+    auto stage = [&](int ch) {
+        float* dst = sm + (ch & 1) * L::FLOATS;
+        const float* src = rec0 + (size_t)ch * D.H * REC;
+        if (tid < 64) {
+            const int r = tid >> 2, c = (tid & 3) * 4;
+            if (DELTA) cr_cp16(dst + L::T + r * L::TS + c, src + r * CR + c);
+            cr_cp16(dst + L::B + r * L::TS + c, src + 256 + r * CR + c);
+        }
+        const int c = (tid % (DS / 4)) * 4, r0 = tid / (DS / 4);
+        if (VEC) {
+            const float* x = src + 512 + r0 * DS + c;
+#pragma unroll
+            for (int r = 0; r < CR; r += STEP, x += STEP * DS) {
+                if (sg.pass != 1) cr_cp16(dst + L::Q + (r0 + r) * L::QS + c, x);
+                if (DELTA) cr_cp16(dst + L::K + (r0 + r) * L::QS + c, x + CR * DS);
+                cr_cp16(dst + L::N + (r0 + r) * L::KS + c, x + 2 * CR * DS);
+            }
+            if (tid < DS / 4) cr_cp16(dst + L::G + tid * 4, src + 512 + 3 * CR * DS + tid * 4);
+        } else {
+            const float* row = w.qkv + (size_t)(start + ch * CR + r0) * w.ld + kh * D.d + c;
+            const int left = c < D.d ? len - ch * CR - r0 : 0;
+#pragma unroll
+            for (int r = 0; r < CR; r += STEP, row += (size_t)STEP * w.ld) {
+                float *qd = dst + L::Q + (r0 + r) * L::QS + c, *kd = dst + L::K + (r0 + r) * L::QS + c, *nd = dst + L::N + (r0 + r) * L::KS + c;
+                if (r < left) {
+                    if (sg.pass != 1) cr_cp16(qd, row + w.q_off);
+                    if (DELTA) cr_cp16(kd, row + w.k_off);
+                    cr_cp16(nd, row + w.k_off);
+                } else {
+                    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+                    *reinterpret_cast<float4*>(qd) = z;
+                    if (DELTA) *reinterpret_cast<float4*>(kd) = z;
+                    *reinterpret_cast<float4*>(nd) = z;
+                }
+            }
+            if (tid < 12) cr_cp16(dst + L::G + tid * 4, src + 512 + tid * 4);
+        }
+        cp_async_commit();
+    };
+    // a chunk's values (times beta without the correction), in accumulator layout: columns g and g + 8, tokens 8 n + 2 t and + 1
+    float vn[2][4], bn[2][2];
+    auto values = [&](int tok0) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int tk = tok0 + 8 * n + 2 * t + (e & 1), c = col0 + g + 8 * (e >> 1);
+                vn[n][e] = tk >= len || c >= dvs ? 0.f : c == D.dv ? 1.f : w.qkv[(size_t)(start + tk) * w.ld + w.v_off + h * D.dv + c];
+                if (!DELTA && e < 2) bn[n][e] = w.beta && tk < len ? w.beta[(size_t)(start + tk) * D.H + h] : 1.f;
+            }
+    };
+    stage(0);
+    values(0);
+    for (int ch = 0; ch < nch; ++ch) {
+        const int tok0 = ch * CR;
+        float v[2][4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[n][e] = DELTA ? vn[n][e] : vn[n][e] * bn[n][e & 1];
+        cp_async_wait<0>();
+        __syncthreads();                                  // chunk ch has landed; everyone is done with the other half and the partial sums
+        if (ch + 1 < nch) { stage(ch + 1); values(tok0 + CR); }
+        const float* st = sm + (ch & 1) * L::FLOATS;
+        if (DELTA || sg.pass != 1) {
+        // ---- this warp's rows' share of S^T q and R; the small terms in accumulators of their own, so that no product waits for the one before it
+        float oq[2][4], rk[2][4], oql[2][4], rkl[2][4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) oq[n][e] = rk[n][e] = oql[n][e] = rkl[n][e] = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            const CrA a = cr_a(s[nt]);
+            const int r = row0 + 8 * nt + 2 * t;
+            CrB q[2], k[2];
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                q[n] = cr_b2(st + L::Q + (8 * n + g) * L::QS + r);
+                if (DELTA) k[n] = cr_b2(st + L::K + (8 * n + g) * L::QS + r);
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n) { cr_mma(oql[n], a.l, q[n].h); if (DELTA) cr_mma(rkl[n], a.l, k[n].h); }
+#pragma unroll
+            for (int n = 0; n < 2; ++n) { cr_mma(oq[n], a.h, q[n].h); if (DELTA) cr_mma(rk[n], a.h, k[n].h); }
+#pragma unroll
+            for (int n = 0; n < 2; ++n) { cr_mma(oql[n], a.h, q[n].l); if (DELTA) cr_mma(rkl[n], a.h, k[n].l); }
+        }
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { oq[n][e] += oql[n][e]; if (DELTA) rk[n][e] += rkl[n][e]; }
+        float* mine = red + warp * 2 * CR_COLS * CR_RS;
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                *reinterpret_cast<float2*>(mine + (g + 8 * c) * CR_RS + 8 * n + 2 * t) = make_float2(oq[n][2 * c], oq[n][2 * c + 1]);
+                if (DELTA) *reinterpret_cast<float2*>(mine + (CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t) = make_float2(rk[n][2 * c], rk[n][2 * c + 1]);
+            }
+        }
+        if (DELTA || sg.pass != 1) __syncthreads();
+        auto total = [&](int part, int n, int c) {
+            const float* p = red + (part * CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t;
+            float2 x = *reinterpret_cast<const float2*>(p);
+#pragma unroll
+            for (int k = 1; k < CR_WARPS; ++k) { const float2 y = *reinterpret_cast<const float2*>(p + k * 2 * CR_COLS * CR_RS); x.x += y.x; x.y += y.y; }
+            return x;
+        };
+        float u[2][4];
+        if (DELTA) {                                      // every warp forms all of U: it is the update's operand
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    float2 r = total(1, n, c);
+                    if (!VEC) { r.x *= st[L::G + 8 * n + 2 * t]; r.y *= st[L::G + 8 * n + 2 * t + 1]; }
+                    v[n][2 * c] -= r.x; v[n][2 * c + 1] -= r.y;
+                }
+            const CrA w0 = cr_a(v[0]), w1 = cr_a(v[1]);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                u[n][0] = u[n][1] = u[n][2] = u[n][3] = 0.f;
+                const float* row = st + L::T + (8 * n + g) * L::TS + 2 * t;
+                cr_mma3(u[n], w0, cr_b2(row));
+                if (n) cr_mma3(u[n], w1, cr_b2(row + 8));   // T is lower triangular
+            }
+        } else {
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) u[n][e] = v[n][e];
+        }
+        if (warp < 2 && sg.pass != 1) {                                   // the read-out of 8 tokens each
+            const int n = warp;
+            float out[4], add[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float2 x = total(0, n, c);
+                if (!VEC) { x.x *= st[L::G + 8 * n + 2 * t]; x.y *= st[L::G + 8 * n + 2 * t + 1]; }
+                out[2 * c] = x.x; out[2 * c + 1] = x.y;
+            }
+            const float* row = st + L::B + (8 * n + g) * L::TS + 2 * t;
+            cr_mma3(add, cr_a(u[0]), cr_b2(row));
+            if (n) cr_mma3(add, cr_a(u[1]), cr_b2(row + 8));
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int tk = tok0 + 8 * n + 2 * t + (e & 1), c = col0 + g + 8 * (e >> 1);
+                if (tk < len && c < dvs) o[((size_t)(start + tk) * D.H + h) * dvs + c] = (out[e] + add[e]) * D.o_scale;
+            }
+        }
+        if (!VEC) prod *= st[L::G + 32];
+        // ---- state update: the chunk's own sum from zero, so that the state itself is only ever rounded to nearest (the matrix unit's sums are cut off)
+        if (!VEC) {
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                const float d0 = st[L::G + 16 + 8 * n + 2 * t], d1 = st[L::G + 16 + 8 * n + 2 * t + 1];
+                u[n][0] *= d0; u[n][1] *= d1; u[n][2] *= d0; u[n][3] *= d1;
+            }
+        }
+        const CrA u0 = cr_a(u[0]), u1 = cr_a(u[1]);
+        CrB k0[NT], k1[NT];
+        float ds[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            const float* kr = st + L::N + 2 * t * L::KS + row0 + 8 * nt + g;
+            k0[nt] = cr_b(kr[0], kr[L::KS]); k1[nt] = cr_b(kr[8 * L::KS], kr[9 * L::KS]);
+            ds[nt][0] = ds[nt][1] = ds[nt][2] = ds[nt][3] = 0.f;
+        }
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u0.l, k0[nt].h);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u0.h, k0[nt].l);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u1.l, k1[nt].h);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u1.h, k1[nt].l);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u0.h, k0[nt].h);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u1.h, k1[nt].h);
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+            float2 ge;
+            if (VEC) ge = *reinterpret_cast<const float2*>(st + L::G + row0 + 8 * nt + 2 * t);
+            else ge.x = ge.y = st[L::G + 32];
+            s[nt][0] = fmaf(s[nt][0], ge.x, ds[nt][0]); s[nt][1] = fmaf(s[nt][1], ge.y, ds[nt][1]);
+            s[nt][2] = fmaf(s[nt][2], ge.x, ds[nt][2]); s[nt][3] = fmaf(s[nt][3], ge.y, ds[nt][3]);
+        }
+    }
+    if (sg.pass == 3) return;                             // scan_prefix_kernel has left the end states
+    float* S1 = sg.pass ? sg.local + entry : state + (size_t)b.seq_slot[sq] * slot_stride + (size_t)h * D.d * dvs;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { bool ok; const size_t i = at_state(nt, e, ok); if (ok) S1[i] = s[nt][e]; }
+    if (!VEC && sg.pass && blockIdx.z == 0 && tid == 0) sg.prod[(size_t)(seq0 / SCAN_CHUNK + sq + seg) * D.H + h] = prod;
+}
+
+template <int DS, bool VEC, bool DELTA>
+int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const float* decay, float* state, size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan) {
+    chunk_prep_kernel<DS, VEC, DELTA><<<dim3(b.nseq * w.nchunks, D.H), CR_THREADS, 0, s>>>(b, D, w);
+    if (int rc = launch_check(cudaGetLastError(), "chunk_prep")) return rc;
+    constexpr size_t smem = (size_t)(2 * CrStage<DS, VEC, DELTA>::FLOATS + CR_WARPS * 2 * CR_COLS * CR_RS) * sizeof(float);
+    static DevOnce once;
+    if (once.need() && cuda_check(cudaFuncSetAttribute(chunk_scan_kernel<DS, VEC, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "chunk shared memory")) return WF_ERR_CUDA;
+    Segments sg;
+    const int cols = (D.dv + D.ones_col + CR_COLS - 1) / CR_COLS;
+    auto scan_pass = [&](int pass) {
+        sg.pass = pass;
+        chunk_scan_kernel<DS, VEC, DELTA><<<dim3(b.nseq * sg.n, D.H, cols), CR_THREADS, smem, s>>>(b, D, w, state, slot_stride, o, sg);
+        return launch_check(cudaGetLastError(), "chunk_scan");
+    };
+    // Segments in parallel where the recurrence is linear in the state, one portion is long and the chains of whole portions leave the machine idle: the two
+    // passes cost half as much work again.  us, whole -> segments: 4 heads 128 x 64, 1024 tokens 87 -> 40, 300 tokens 35 -> 36; 16 heads, 2048 tokens 168 -> 95;
+    // 40 heads (160 blocks) 224 -> 202; two sequences of 841 and 1207, 16 heads (128 blocks) 109 -> 102, 40 heads (320 blocks) 185 -> 206.
+    if (DELTA || !scan->local || b.max_len < 4 * SCAN_CHUNK || b.n / SCAN_CHUNK + b.nseq + 1 > scan->chunks || 2LL * b.nseq * D.H * cols >= 3LL * sm_count())
+        return scan_pass(0);
+    sg.n = (b.max_len + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    sg.local = scan->local; sg.start = scan->start; sg.prod = scan->prod;
+    if (int rc = scan_pass(1)) return rc;
+    if (int rc = launch_scan_prefix(b, D, decay, state, slot_stride, scan, sg.n, s)) return rc;
+    return scan_pass(3);
+}
+
+}  // namespace
+
+size_t chunk_workspace_floats(const DeltaDims& D, int max_step_tokens, int slots) {
+    if (D.d > 128) return 0;
+    const size_t rec = cr_rec_floats(D.d <= 64 ? 64 : 128, D.vec_decay != 0);
+    return (size_t)(max_step_tokens / CR + slots + 1) * D.H * rec;
+}
+
+bool chunk_usable(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const ScanWorkspace* scan) {
+    const int qo = D.q_off >= 0 ? D.q_off : 0, ko = D.k_off >= 0 ? D.k_off : D.Hk * D.d;
+    return scan && scan->rec && b.max_len >= 2 * CR && D.d <= 128 && D.d % 4 == 0 && ld % 4 == 0 && qo % 4 == 0 && ko % 4 == 0 && ((uintptr_t)qkv & 15) == 0 && D.H <= 65535 &&
+           chunk_workspace_floats(D, b.n, b.nseq) <= scan->rec_floats;
+}
+
+int launch_chunk_recurrence(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const float* beta, const float* decay, float* state, size_t slot_stride,
+                            float* o, cudaStream_t s, const ScanWorkspace* scan) {
+    ChunkView w;
+    w.qkv = qkv; w.beta = beta; w.decay = decay; w.ld = ld;
+    w.q_off = D.q_off >= 0 ? D.q_off : 0; w.k_off = D.k_off >= 0 ? D.k_off : D.Hk * D.d; w.v_off = D.v_off >= 0 ? D.v_off : 2 * D.Hk * D.d;
+    w.rec = scan->rec; w.nchunks = (b.max_len + CR - 1) / CR;
+#define CR_PICK(vec, delta) (D.d <= 64 ? cr_launch<64, vec, delta>(b, D, w, decay, state, slot_stride, o, s, scan) : cr_launch<128, vec, delta>(b, D, w, decay, state, slot_stride, o, s, scan))
+    if (D.no_delta) return D.vec_decay ? CR_PICK(true, false) : CR_PICK(false, false);
+    return D.vec_decay ? CR_PICK(true, true) : CR_PICK(false, true);
+#undef CR_PICK
+}
+
+}  // namespace seq
+}  // namespace wf

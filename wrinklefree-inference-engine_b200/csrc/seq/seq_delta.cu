@@ -490,11 +490,24 @@ int delta_rule_launch(const Batch& b, const DeltaDims& D, const float* qkv, int 
 }
 }  // namespace
 
+// between the passes of the parallel form: the chunks' start states from their own end states, and the portions' end states
+int launch_scan_prefix(const Batch& b, const DeltaDims& D, const float* decay, float* state, size_t slot_stride, const ScanWorkspace* scan, int nchunks, cudaStream_t s) {
+    if (D.vec_decay) {
+        const int nd = D.H * D.d;
+        scan_decay_prod_kernel<<<dim3(b.nseq * nchunks, (nd + 127) / 128), 128, 0, s>>>(b, nd, SCAN_CHUNK, nchunks, decay, scan->prod);
+        if (int rc = launch_check(cudaGetLastError(), "scan_decay_prod")) return rc;
+    }
+    const int dd = D.d * (D.dv + D.ones_col);
+    scan_prefix_kernel<<<dim3(b.nseq, D.H, (dd + 255) / 256), 256, 0, s>>>(b, D.H, dd, SCAN_CHUNK, state, slot_stride, scan->local, scan->start, scan->prod, D.vec_decay ? D.d : 0);
+    return launch_check(cudaGetLastError(), "scan_prefix");
+}
+
 int launch_delta_rule(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const float* beta, const float* decay, float* state,
                       size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan) {
     if (b.nseq <= 0) return WF_OK;
     if (D.Hk <= 0 || D.H % D.Hk) { set_error("delta: %d heads over %d key heads", D.H, D.Hk); return WF_ERR_INVALID; }
     if (D.ones_col && !D.no_delta) { set_error("delta: the all-ones column belongs to the plain recurrence"); return WF_ERR_UNSUPPORTED; }
+    if (b.n != b.nseq && chunk_usable(b, D, qkv, ld, scan)) return launch_chunk_recurrence(b, D, qkv, ld, beta, decay, state, slot_stride, o, s, scan);
     if (D.no_delta) {
         auto plain = [&](const ScanArgs& sa) {
             return D.vec_decay ? delta_rule_launch<true, false>(b, D, qkv, ld, beta, decay, state, slot_stride, o, s, sa)
@@ -507,14 +520,7 @@ int launch_delta_rule(const Batch& b, const DeltaDims& D, const float* qkv, int 
             sa.local = scan->local; sa.start = scan->start; sa.prod = scan->prod;
             sa.pass = 1;
             if (int rc = plain(sa)) return rc;
-            if (D.vec_decay) {
-                const int nd = D.H * D.d;
-                scan_decay_prod_kernel<<<dim3(b.nseq * sa.nchunks, (nd + 127) / 128), 128, 0, s>>>(b, nd, SCAN_CHUNK, sa.nchunks, decay, scan->prod);
-                if (int rc = launch_check(cudaGetLastError(), "scan_decay_prod")) return rc;
-            }
-            const int dd = D.d * (D.dv + D.ones_col);
-            scan_prefix_kernel<<<dim3(b.nseq, D.H, (dd + 255) / 256), 256, 0, s>>>(b, D.H, dd, SCAN_CHUNK, state, slot_stride, scan->local, scan->start, scan->prod, D.vec_decay ? D.d : 0);
-            if (int rc = launch_check(cudaGetLastError(), "scan_prefix")) return rc;
+            if (int rc = launch_scan_prefix(b, D, decay, state, slot_stride, scan, sa.nchunks, s)) return rc;
             sa.pass = 3;
             return plain(sa);
         }

@@ -537,7 +537,7 @@ int run_delta(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
     const float* b_raw = e->proj + L.b_col;
     if ((rc = launch_delta_prep(e->dt, D, n, e->qkvc, C, a_raw, lda, b_raw, L.np, L.A_log, L.dt_bias, e->beta, e->decay, s))) return rc;
     mark(e, "delta.conv+prep");
-    if ((rc = launch_delta_rule(b, D, e->qkvc, C, e->beta, e->decay, e->state + L.st_S, e->slot_stride, e->od, s))) return rc;
+    if ((rc = launch_delta_rule(b, D, e->qkvc, C, e->beta, e->decay, e->state + L.st_S, e->slot_stride, e->od, s, &e->scan))) return rc;
     mark(e, "delta.rule");
     if ((rc = launch_delta_post(e->dt, D, n, e->od, L.onorm, e->cfg.eps, g_raw, ldg, e->og, s, c.gate_act))) return rc;
     mark(e, "delta.post");
@@ -1148,7 +1148,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     if (c.tied_head) e->head = e->embed;
     else { TRY(dalloc_t(e, &e->head, (size_t)c.vocab * W)); add_tensor(e, "head", e->head, (size_t)c.vocab * W); }
     // maxima over layers for the shared workspaces
-    size_t max_np = 1, max_hd = 1, max_hr = 1, max_hrot = 1, max_hv = 1, max_C = 1, max_H = 1, max_N = 1, max_top = 1, max_E = 1, max_ff = 1, max_uff = 0, max_gqa_dv = 0, max_kvx = 0, max_lat = 0;
+    size_t max_np = 1, max_hd = 1, max_hr = 1, max_hrot = 1, max_hv = 1, max_C = 1, max_H = 1, max_N = 1, max_top = 1, max_E = 1, max_ff = 1, max_uff = 0, max_gqa_dv = 0, max_kvx = 0, max_lat = 0, max_rec = 0;
     long long cache_elems = 0;
     size_t st = 0;
     e->layers.resize(c.n_layers + c.n_extra);
@@ -1291,6 +1291,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             L.st_S = st; st += (size_t)l.heads * l.dim * (l.vdim + 1);
             L.st_m = st; st += l.heads;
             max_scan = std::max(max_scan, (size_t)l.heads * l.dim * (l.vdim + 1));
+            max_rec = std::max(max_rec, chunk_workspace_floats(DeltaDims{l.heads, l.heads, l.dim, l.vdim}, T, c.slots));
             max_hv = std::max(max_hv, (size_t)l.heads * (l.vdim + 1));
             any_mlstm = true;
         } else if (l.type == WF_SEQ_GLA) {
@@ -1311,6 +1312,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             L.st_S = st; st += nk * l.vdim;
             max_decay = std::max(max_decay, nk);
             max_scan = std::max(max_scan, nk * l.vdim);
+            max_rec = std::max(max_rec, chunk_workspace_floats(DeltaDims{l.heads, l.heads, l.dim, l.vdim, 1}, T, c.slots));
         } else if (l.type == WF_SEQ_SSD) {
             // [z | x | B | C | dt]: x, B and C are the convolved channels
             const size_t GN = (size_t)l.kv_heads * l.dim;
@@ -1327,11 +1329,13 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             L.st_S = st; st += (size_t)l.heads * l.dim * l.vdim;
             max_C = std::max(max_C, (size_t)L.C);
             max_scan = std::max(max_scan, (size_t)l.heads * l.dim * l.vdim);
+            max_rec = std::max(max_rec, chunk_workspace_floats(DeltaDims{l.heads, l.kv_heads, l.dim, l.vdim}, T, c.slots));
         } else {
             // [q | k | v | gate (or its first factor) | write strength | decay (or its first factor)]
             const size_t nqk = (size_t)l.kv_heads * l.dim;
             L.C = (int)(2 * nqk + nv);
             L.n_decay = l.decay_channels ? l.heads * l.dim : l.heads;
+            max_rec = std::max(max_rec, chunk_workspace_floats(DeltaDims{l.heads, l.kv_heads, l.dim, l.vdim, l.decay_channels ? 1 : 0}, T, c.slots));
             const size_t g_rows = l.gate_rank > 0 ? (size_t)l.gate_rank : nv, a_rows = l.decay_rank > 0 ? (size_t)l.decay_rank : (size_t)L.n_decay;
             L.g_col = L.C; L.b_col = (int)(L.C + g_rows); L.a_col = L.b_col + l.heads;
             L.np = (int)(L.a_col + a_rows);
@@ -1502,6 +1506,10 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
         e->scan.chunks = scan_chunks_needed(T, c.slots);
         TRY(dalloc_n(e, &e->scan.local, (size_t)e->scan.chunks * max_scan)); TRY(dalloc_n(e, &e->scan.start, (size_t)e->scan.chunks * max_scan));
         TRY(dalloc_n(e, &e->scan.prod, (size_t)e->scan.chunks * std::max(max_H, max_decay)));
+    }
+    if (max_rec && T >= 2 * CHUNK_TOKENS) {
+        TRY(dalloc_n(e, &e->scan.rec, max_rec));
+        e->scan.rec_floats = max_rec;
     }
     if (max_gfull) TRY(dalloc_n(e, &e->gfull, (size_t)T * max_gfull));
     if (max_afull) TRY(dalloc_n(e, &e->afull, (size_t)T * max_afull));

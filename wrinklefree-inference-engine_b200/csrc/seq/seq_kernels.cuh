@@ -250,13 +250,22 @@ int launch_delta_prep(int dt, const DeltaDims& D, int n, float* qkv, int ld, con
 // every chunk's own contribution from a zero state, a short pass that chains the chunks' start states (S_start[c + 1] = prod_c S_start[c]
 // + local_c, the recurrence being linear in the state), then every chunk again from its start state for the outputs.
 constexpr int SCAN_CHUNK = 128;
-struct ScanWorkspace { float* local = nullptr; float* start = nullptr; float* prod = nullptr; int chunks = 0; };   // chunks: entries of H * d * dv floats each; prod: H (vec_decay: H * d) floats per chunk
+struct ScanWorkspace { float* local = nullptr; float* start = nullptr; float* prod = nullptr; int chunks = 0;
+                       float* rec = nullptr; size_t rec_floats = 0; };   // rec: records of the 16-token form (chunk_workspace_floats); chunks: entries of H * d * dv floats each; prod: H (vec_decay: H * d) floats per chunk
 // gated linear attention: decay[i, c] = sigmoid(z)^(1 / tau), z = a2[c, :] . a1[i, :] + bias[c], c < nout; a1 float [n, rank] (ld), a2 T [nout, rank];
 // products, logarithm and exponential in float
 int launch_gla_decay(int dt, int n, int rank, int nout, const float* a1, int ld, const void* a2, const void* bias, float tau, float* decay, cudaStream_t s);
 inline int scan_chunks_needed(int max_step_tokens, int slots) { return max_step_tokens / SCAN_CHUNK + slots + 1; }
 int launch_delta_rule(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const float* beta, const float* decay, float* state,
                       size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan = nullptr);
+int launch_scan_prefix(const Batch& b, const DeltaDims& D, const float* decay, float* state, size_t slot_stride, const ScanWorkspace* scan, int nchunks, cudaStream_t s);
+// The same recurrences 16 tokens at a time (seq_chunk.cu): portions of at least 32 tokens, key sizes multiples of 4 up to 128, aligned rows.
+// launch_delta_rule takes it where it can; chunk_workspace_floats: what a step of at most max_step_tokens over `slots` sequences needs of ScanWorkspace::rec.
+constexpr int CHUNK_TOKENS = 16;
+size_t chunk_workspace_floats(const DeltaDims& D, int max_step_tokens, int slots);
+bool chunk_usable(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const ScanWorkspace* scan);
+int launch_chunk_recurrence(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const float* beta, const float* decay, float* state, size_t slot_stride,
+                            float* o, cudaStream_t s, const ScanWorkspace* scan);
 // y T [n, H * dv] = o / sqrt(mean_dv(o^2) + eps) * w[dv] * act(g float [n, H * dv] (ldg)); act 0 silu, 1 sigmoid
 int launch_delta_post(int dt, const DeltaDims& D, int n, const float* o, const void* w, float eps, const float* g, int ldg, void* y, cudaStream_t s, int act = 0);
 // state-space recurrence around launch_delta_rule (no_delta form).  prep: step[n, H] = softplus(dt_raw + dt_bias[h]) (no clamp),
