@@ -125,7 +125,8 @@ constexpr uint32_t tc_idesc(int m, int n) {
 // NU = unpack warp groups (4 warps each, one per TMEM lane quarter); group g expands the stages with item % NU == g.
 // One warp issues ~190 instructions per stage at IPC ~0.3, so a single group paces the kernel at ~850 clk per stage
 // (measured) against the 256-clk tensor floor; three groups bring the unpack under the floor.
-template <int CL, int NU>
+// SPLIT: the few-token form, a cluster of K parts.  An instance of its own: its branches in the batched-decode form cost that 2 % of a 64-sequence step.
+template <int CL, int NU, bool SPLIT = false>
 __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcParams p) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[TC_STAGES];    // TMA bytes + 4 unpack-warp arrivals
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;   // 128B-swizzle atoms need 1024-B alignment
     const int crank = (CL > 1) ? (int)(blockIdx.x % CL) : 0;          // 1-D cluster: rank == blockIdx.x % CL
-    const int ksp = CL == 1 ? p.ksplit : 1;                           // cluster of K parts (one tile per cluster) instead of a cluster of tiles
+    const int ksp = SPLIT ? p.ksplit : 1;                           // cluster of K parts (one tile per cluster) instead of a cluster of tiles
     const int krank = ksp > 1 ? (int)(blockIdx.x % ksp) : 0;
     const int cluster_id = blockIdx.x / (CL * ksp), n_clusters = gridDim.x / (CL * ksp);
     const int ngroups = (p.tiles_n + CL - 1) / CL;                    // groups of CL weight-row tiles
@@ -399,7 +400,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
             const bool fast = fast_mode && mw0 + TC_EP_TOKS <= p.M && n_blk * TC_BM + q * 32 + 32 <= p.N;   // warp-uniform
             mbar_wait(&tfull_bar[buf], (uint32_t)((tl >> 1) & 1));
             tc_fence_after();
-            if (ksp > 1) {
+            if (SPLIT) {
                 // the ring is free (every MMA of this CTA's only tile has read its stage): the accumulators go there as [token][row]
 #pragma unroll 1
                 for (int c = 0; c < TC_EP_TOKS / 32 && mw0 + c * 32 < p.M; ++c) {
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
             }
         }
     }
-    if (ksp > 1) {
+    if (SPLIT) {
         // sum of the K parts: every CTA of the cluster finishes an equal share of the tile's tokens
         __syncwarp();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -561,6 +562,7 @@ void gemm_tc_init_attrs() {
     if (g_tc_attr.need()) {
         bool ok = cudaFuncSetAttribute(ternary_gemm_tc_kernel<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
         ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<1, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
         ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<1, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
         ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
         ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
@@ -705,7 +707,7 @@ static int launch_tc_split(const wf_linear_args* a, const EpiParams& ep, int ksp
     at[0].val.clusterDim.x = ksplit; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<1, NU>, tmap, p), "ternary_gemm_tc(split)");
+    return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<1, NU, true>, tmap, p), "ternary_gemm_tc(split)");
 }
 
 int launch_gemm_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s) {
