@@ -370,8 +370,8 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
         const bool obf16 = (mode == WF_OUT_LINEAR) && p.ep.out_dtype == WF_BF16;
         const int ncols = relu2 ? p.N / 2 : p.N;
         const bool red = p.red_acc != nullptr;
-        const bool fast_mode = !red && mode == WF_OUT_LINEAR && !relu2 && !resid && obf16 && !p.dbg;
-        const bool fold_ws = fast_mode && p.ep.nseg <= 1;
+        const bool fast_mode = !red && (mode == WF_OUT_LINEAR || mode == WF_OUT_COMPAT_F32) && !relu2 && !resid && !p.dbg;
+        const bool fold_ws = fast_mode && mode == WF_OUT_LINEAR && p.ep.nseg <= 1;
         const float ws_all = fold_ws ? w_scale_of(p.ep, 0) : 1.f;
         if (red) pdl_wait_prior();   // the accumulator buffer was cleared by an earlier phase of the step
         for (int tl = 0; tl < my_tiles; ++tl) {
@@ -428,27 +428,22 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
                 if (p.dbg) continue;
                 const int m0 = mw0 + c * 32;
                 if (fast) {
-                    // full tile, bf16 linear output: ~9 issued instructions per token (LDS.64, I2F, 3 FMUL, FADD, F2F, pointer add, STG);
+                    // full tile, plain output: ~9 issued instructions per token (LDS.64, I2F, 3 FMUL, FADD, F2F for bf16, pointer add, STG);
                     // the reference's rounding sequence (linear_value in linear_common.cuh)
-                    __nv_bfloat16* op = reinterpret_cast<__nv_bfloat16*>(p.ep.out) + (size_t)m0 * p.ep.ldo + col;
                     const size_t ldo = (size_t)p.ep.ldo;
                     const float2* tk = tok + c * 32;
+                    auto each = [&](auto* op, auto value) {
+                        op += (size_t)m0 * ldo + col;
 #pragma unroll
-                    if (fold_ws) {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const float2 t = tk[j];
-                            *op = __float2bfloat16_rn(__fmul_rn(__fsub_rn(__fmul_rn((float)(int)v[j], ws), t.x), t.y));
-                            op += ldo;
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            const float2 t = tk[j];
-                            *op = __float2bfloat16_rn(__fmul_rn(__fsub_rn(__fmul_rn((float)(int)v[j], ws), __fmul_rn(ws, t.x)), t.y));
-                            op += ldo;
-                        }
-                    }
+                        for (int j = 0; j < 32; ++j) { *op = value(j); op += ldo; }
+                    };
+                    auto folded = [&](int j) { const float2 t = tk[j]; return __fmul_rn(__fsub_rn(__fmul_rn((float)(int)v[j], ws), t.x), t.y); };
+                    auto plain = [&](int j) { const float2 t = tk[j]; return __fmul_rn(__fsub_rn(__fmul_rn((float)(int)v[j], ws), __fmul_rn(ws, t.x)), t.y); };
+                    if (mode == WF_OUT_COMPAT_F32) each(reinterpret_cast<float*>(p.ep.out), [&](int j) { return __fmul_rn((float)(int)v[j], p.ep.host_scale); });
+                    else if (!obf16 && fold_ws) each(reinterpret_cast<float*>(p.ep.out), folded);
+                    else if (!obf16) each(reinterpret_cast<float*>(p.ep.out), plain);
+                    else if (fold_ws) each(reinterpret_cast<__nv_bfloat16*>(p.ep.out), [&](int j) { return __float2bfloat16_rn(folded(j)); });
+                    else each(reinterpret_cast<__nv_bfloat16*>(p.ep.out), [&](int j) { return __float2bfloat16_rn(plain(j)); });
                     continue;
                 }
                 const int mcnt = min(32, p.M - m0);                                // tokens of this chunk that exist (warp-uniform)
