@@ -248,18 +248,22 @@ __device__ __forceinline__ QDiv make_qdiv(float scale) {
     d.slow = ((__float_as_uint(scale) & 0x007fffffu) == 0x007fffffu) ? 1 : 0;
     return d;
 }
+__device__ __forceinline__ float quant_quotient(float x, const QDiv& d) {
+    if (d.slow) return __fdiv_rn(x, d.scale);
+    const float q0 = __fmul_rn(x, d.rcp);
+    return __fmaf_rn(__fmaf_rn(-d.scale, q0, x), d.rcp, q0);
+}
 __device__ __forceinline__ int quant_i8(float x, const QDiv& d) {
-    float q;
-    if (d.slow) {
-        q = __fdiv_rn(x, d.scale);
-    } else {
-        const float q0 = __fmul_rn(x, d.rcp);
-        const float e = __fmaf_rn(-d.scale, q0, x);
-        q = __fmaf_rn(e, d.rcp, q0);
-    }
-    float r = rintf(q);
+    float r = rintf(quant_quotient(x, d));
     r = fminf(fmaxf(r, -128.f), 127.f);
     return (int)r;
+}
+// The same four times, packed: adding 1.5 * 2^23 leaves the nearest even integer, as rintf gives it, in the low bits (two's complement), and clamping to
+// whole bounds before it is clamping after it; NaN becomes -128 in both.  For the passes over prompts, which the round and convert instructions (a quarter
+// of the rate of the add) held back; the decode step's row kernels lost 1 % with it and keep the form above.
+__device__ __forceinline__ uint32_t quant_i8x4(float a, float b, float c, float e, const QDiv& d) {
+    auto bits = [&](float x) { return __float_as_uint(__fadd_rn(fminf(fmaxf(quant_quotient(x, d), -128.f), 127.f), 12582912.f)); };
+    return __byte_perm(__byte_perm(bits(a), bits(b), 0x0040), __byte_perm(bits(c), bits(e), 0x0040), 0x5410);
 }
 
 }  // namespace wf
