@@ -72,3 +72,51 @@ def test_matrix_memory(heads, dim, vdim, lens, cuts):
            "layers": [{"type": "parallel", "mixer": {"left": left, "left_scale": 0.0, "right": right, "right_scale": 1.0}, "mlp": None}]}
     w = FO.random_weights(cfg, 3)
     check(cfg, w, {"l0.mix.left.rel": (8, 2)}, lambda x: FO.matrix_memory(x, d64(w, "l0.mix.right."), "", right, EPS), lens, cuts, W)
+
+
+# ---- numbers that are not finite: one long portion (the 16-token form) against the same rows in portions of 31 tokens (token by token)
+def nonfinite_layer(kind):
+    W = 40
+    if kind == "delta":
+        m = {"heads": 4, "kv_heads": 2, "dim": 64, "vdim": 32, "conv": 4}
+        cfg = {"architecture": "Nukezen", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": EPS}, "layers": [{"type": "channel_delta", "mixer": m, "mlp": None}]}
+        return cfg, NO.random_weights(cfg, 1, {0: {"rank_a": 8, "rank_g": 8}}), {"l0.mix.a1": (8, W), "l0.mix.g1": (8, W)}, W
+    left = {"heads": 2, "kv_heads": 1, "dim": 8, "vdim": 8, "scale": 0.3, "mask": {"size": 8}}
+    if kind == "state_space":
+        left["rot"] = {"dims": 8, "base": 10000.0}
+        right = {"heads": 4, "vdim": 32, "state": 64, "groups": 2, "conv": 4, "norm_groups": 2}
+        arch, make, shapes = "Nukezen", lambda c: NO.random_weights(c, 2), {}
+    else:
+        left["bias_max"] = 16
+        right = {"heads": 4, "dim": 64, "vdim": 32, "gate_cap": 15.0}
+        arch, make, shapes = "Fivedra", lambda c: FO.random_weights(c, 3), {"l0.mix.left.rel": (8, 2)}
+    cfg = {"architecture": arch, "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": EPS},
+           "layers": [{"type": "parallel", "mixer": {"left": left, "left_scale": 0.0, "right": right, "right_scale": 1.0}, "mlp": None}]}
+    return cfg, make(cfg), shapes, W
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("at", [0, 37, 131])
+@pytest.mark.parametrize("kind", ["delta", "state_space", "memory"])
+def test_numbers_that_are_not_finite(kind, at, bad):
+    """A token whose row holds a NaN or an infinity: the same output rows are finite as token by token, in the portion and in the next one."""
+    from wf_bitnet import registry
+    cfg, weights, shapes, W = nonfinite_layer(kind)
+    cls = registry.resolve(cfg)
+    extra = {"shapes": shapes} if getattr(cls, "reads_shapes", False) else {}
+    m = cls(cfg, dtype="bfloat16", max_tokens=800, slots=4, page_size=16, max_step_tokens=400, **extra)
+    m.load_weights((k, v.numpy(), "F32") for k, v in weights.items())
+    g = np.random.default_rng(7)
+    rows = torch.from_numpy(g.standard_normal((300, W)).astype(np.float32)).to(torch.bfloat16).float().numpy()
+    rows[at, 3] = bad
+    a, b = m.admit(), m.admit()
+    whole = np.concatenate([m.engine.run_part(0, 2, [a], [n], rows[t:t + n]) for t, n in ((0, 260), (260, 40))])
+    pieces = np.concatenate([m.engine.run_part(0, 2, [b], [min(31, 300 - t)], rows[t:t + 31]) for t in range(0, 300, 31)])
+    m.close()
+    ok, want = np.isfinite(whole).all(-1), np.isfinite(pieces).all(-1)
+    assert np.array_equal(ok, want), (np.flatnonzero(ok != want), ok.sum(), want.sum())
+    assert want[:at].all()
+    if want[:at].any():
+        x, y = whole[:at], pieces[:at]
+        err = np.sqrt(((x - y) ** 2).mean(-1)) / np.sqrt((y ** 2).mean(-1))
+        assert err.max() < 2e-2          # two bf16 roundings of the same float values, and the products around them

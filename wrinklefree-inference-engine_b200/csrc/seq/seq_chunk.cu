@@ -14,7 +14,10 @@
 // Measured at 2048 tokens: delta rule (20 heads, 128 x 128, two sequences) 569 -> 231 us (48 of them the preparation), state space (40 heads, 128 x 64, one
 // sequence) 307 -> 202 us (32); eight warps with half the rows each 287 and 257 us (both in one pass).  Left: the chain of a chunk, about 3000 clk of products, one exchange of
 // partial sums and two barriers.  Error against 64 bits in float32 layers up to 1500 tokens long: 3.6e-7 to 5.6e-7, as token by token.
-// A token whose key, query or value is infinite or NaN makes its whole chunk's read-out NaN, and the state, as before, for good.
+// Numbers that are not finite: in a product with the zeros of T and B, or as a sum of two tf32 numbers, an infinity or a NaN would reach tokens and rows
+// that never meet it (and the rounding of cr_split would take the bit pattern of a NaN past the exponent, to zero).  So chunk_prep_kernel marks a chunk in
+// which anything it reads or forms is not finite, the scan watches its state and U, and such a chunk is taken token by token, with the meaning that the
+// recurrence has there.  Decays are taken to be at most one, so that finite values do not overflow between the two watched places.
 #include "seq_kernels.cuh"
 
 namespace wf {
@@ -40,8 +43,12 @@ struct ChunkView {
 struct Segments { int pass = 0, n = 1; float *local = nullptr, *prod = nullptr; const float* start = nullptr; };
 
 // a record: [T 256][B 256] then, decay per row: [c_j q_j 16 DS][c_j k_j 16 DS][D(j, 16) k_j 16 DS][c_16 DS]; one decay: [c_j 16][D(j, 16) 16][c_16, padding]
-// (DS: the key rows, padded to 64 or 128)
-__host__ __device__ constexpr int cr_rec_floats(int DS, bool vec) { return vec ? 512 + (3 * CR + 1) * DS : 512 + 48; }
+// (DS: the key rows, padded to 64 or 128), and at cr_mark a number other than zero where the chunk is to be taken token by token
+__host__ __device__ constexpr int cr_rec_floats(int DS, bool vec) { return vec ? 512 + (3 * CR + 1) * DS + 4 : 512 + 48; }
+__host__ __device__ constexpr int cr_mark(int DS, bool vec) { return vec ? DS : 36; }      // within the last part of a record and of a stage (CrStage::G)
+
+// x * 0 summed up: zero while everything is finite, NaN from the first infinity or NaN on
+__device__ __forceinline__ void cr_watch(float& w, float x) { w = fmaf(x, 0.f, w); }
 
 // transposed sum over 16 lanes: v[t] of all of them -> the sum of t = p for lane p
 __device__ __forceinline__ float cr_reduce(float (&v)[CR], int p) {
@@ -66,6 +73,7 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_prep_kernel(Batch b, DeltaDi
     const int len = b.seq_len[sq], start = b.seq_start[sq] + ch * CR, left = min(CR, len - ch * CR);
     if (left <= 0) return;
     const int tid = threadIdx.x, kh = h / (D.H / D.Hk);
+    float watch = 0.f;
     float* rec = w.rec + ((size_t)(b.seq_start[sq] / CR + sq + ch) * D.H + h) * cr_rec_floats(DS, VEC);
     for (int i = tid; i < CR * (DS / 4); i += CR_THREADS) {
         const int t = i / (DS / 4), c = (i - t * (DS / 4)) * 4;
@@ -75,6 +83,10 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_prep_kernel(Batch b, DeltaDi
             k = *reinterpret_cast<const float4*>(row + w.k_off + kh * D.d + c);
             q = *reinterpret_cast<const float4*>(row + w.q_off + kh * D.d + c);
             if (VEC) g = *reinterpret_cast<const float4*>(w.decay + ((size_t)(start + t) * D.H + h) * D.d + c);
+            else {
+                cr_watch(watch, k.x); cr_watch(watch, k.y); cr_watch(watch, k.z); cr_watch(watch, k.w);
+                cr_watch(watch, q.x); cr_watch(watch, q.y); cr_watch(watch, q.z); cr_watch(watch, q.w);
+            }
         }
         *reinterpret_cast<float4*>(&ks[t][c]) = k;
         *reinterpret_cast<float4*>(&qs[t][c]) = q;
@@ -137,9 +149,10 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_prep_kernel(Batch b, DeltaDi
             for (int l = 0; l < j; ++l) v = fmaf(As[j][l], x[l], v);     // x[l] = 0 for l < tid
             x[j] = j == tid ? 1.f : j > tid ? -bt[j] * v : 0.f;
             rec[j * CR + tid] = x[j] * bt[tid];
+            cr_watch(watch, x[j] * bt[tid]);
         }
     }
-    for (int i = tid; i < CR * CR; i += CR_THREADS) rec[256 + i] = Bs[i >> 4][i & 15];
+    for (int i = tid; i < CR * CR; i += CR_THREADS) { rec[256 + i] = Bs[i >> 4][i & 15]; cr_watch(watch, Bs[i >> 4][i & 15]); }
     if (VEC) {
         float *qt = rec + 512, *kt = qt + CR * DS, *kn = kt + CR * DS, *ge = kn + CR * DS;
         for (int c = tid; c < DS; c += CR_THREADS) {
@@ -147,13 +160,16 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_prep_kernel(Batch b, DeltaDi
 #pragma unroll
             for (int t = 0; t < CR; ++t) {
                 cum *= gs[t][c];
-                qt[t * DS + c] = qs[t][c] * cum;
-                if (DELTA) kt[t * DS + c] = ks[t][c] * cum;
+                const float q = qs[t][c] * cum;
+                qt[t * DS + c] = q;
+                cr_watch(watch, q);
+                if (DELTA) { const float k = ks[t][c] * cum; kt[t * DS + c] = k; cr_watch(watch, k); }
             }
             ge[c] = cum;
+            cr_watch(watch, cum);
             float suf = 1.f;
 #pragma unroll
-            for (int t = CR - 1; t >= 0; --t) { kn[t * DS + c] = ks[t][c] * suf; suf *= gs[t][c]; }
+            for (int t = CR - 1; t >= 0; --t) { const float k = ks[t][c] * suf; kn[t * DS + c] = k; cr_watch(watch, k); suf *= gs[t][c]; }
         }
     } else if (tid < CR) {
         float cum = 1.f, suf = 1.f;
@@ -161,7 +177,10 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_prep_kernel(Batch b, DeltaDi
         for (int t = tid + 1; t < CR; ++t) suf *= gsc[t];
         rec[512 + tid] = cum; rec[528 + tid] = suf;
         if (tid == CR - 1) rec[544] = cum;
+        cr_watch(watch, cum); cr_watch(watch, suf);
     }
+    const int mark = __syncthreads_or(!(watch == 0.f));
+    if (tid == 0) rec[512 + (VEC ? 3 * CR * DS : 0) + cr_mark(DS, VEC)] = mark ? 1.f : 0.f;
 }
 
 __device__ __forceinline__ void cr_split(float x, uint32_t& hi, uint32_t& lo) {
@@ -193,9 +212,79 @@ template <int DS, bool VEC, bool DELTA> struct CrStage {
     static constexpr int QS = DS + 8, KS = DS + 4;        // row strides: pairs of rows 8 tokens apart, single rows 2 tokens apart, each without bank conflicts
     static constexpr int TS = 24;                         // of T and B
     static constexpr int T = 0, B = T + (DELTA ? CR * TS : 0), Q = B + CR * TS, K = Q + CR * QS, N = K + (DELTA ? CR * QS : 0), G = N + CR * KS,
-                         FLOATS = G + (VEC ? DS : 48);    // G: c_16 per row, or [c_j][D(j, 16)][c_16]
+                         FLOATS = G + (VEC ? DS + 4 : 48);    // G: c_16 per row, or [c_j][D(j, 16)][c_16]; the mark
 };
 constexpr int CR_RS = 24;                                 // row stride of the partial sums [16 columns][16 tokens]
+
+// A chunk's tokens one by one, as the recurrence states them, rows straight from memory.  sv: the thread's part of the state, laid out as in
+// chunk_scan_kernel.  Not inlined: its registers would come out of the scan's.
+struct CrTokens {
+    const float *row, *decay, *beta;      // of the chunk's first token: qkv row; this head's decay (row) and beta (null: 1)
+    float* o;                             // this head's output row, or null: only the state is wanted
+    int n, ld, k_at, q_at, v_at, H, d, dv, dvs, col0;
+    float o_scale;
+};
+template <int DS, bool VEC, bool DELTA>
+__device__ __noinline__ void cr_by_token(const CrTokens a, float* sv, float* red) {
+    constexpr int NT = DS / (8 * CR_WARPS);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, row0 = warp * 8 * NT, c0 = a.col0 + g;
+    float s[NT][4];
+#pragma unroll
+    for (int i = 0; i < NT * 4; ++i) s[i >> 2][i & 3] = sv[i];
+#pragma unroll 1
+    for (int tk = 0; tk < a.n; ++tk) {
+        const float *row = a.row + (size_t)tk * a.ld, *kr = row + a.k_at, *qr = row + a.q_at, *gr = a.decay + (size_t)tk * a.H * (VEC ? a.d : 1);
+        const float gg = VEC ? 1.f : gr[0], bt = a.beta ? a.beta[(size_t)tk * a.H] : 1.f;
+        float r0 = 0.f, r1 = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = row0 + 8 * nt + 2 * t + e;
+                if (r >= a.d) continue;
+                if (VEC) { s[nt][e] *= gr[r]; s[nt][2 + e] *= gr[r]; }
+                if (DELTA) { r0 = fmaf(s[nt][e], kr[r], r0); r1 = fmaf(s[nt][2 + e], kr[r], r1); }
+            }
+        if (DELTA) {
+            r0 += __shfl_xor_sync(0xffffffffu, r0, 1); r1 += __shfl_xor_sync(0xffffffffu, r1, 1);
+            r0 += __shfl_xor_sync(0xffffffffu, r0, 2); r1 += __shfl_xor_sync(0xffffffffu, r1, 2);
+            __syncthreads();                              // what lay there has been read
+            if (t == 0) { red[warp * CR_COLS + g] = r0; red[warp * CR_COLS + g + 8] = r1; }
+            __syncthreads();
+            r0 = r1 = 0.f;
+#pragma unroll
+            for (int k = 0; k < CR_WARPS; ++k) { r0 += red[k * CR_COLS + g]; r1 += red[k * CR_COLS + g + 8]; }
+        }
+        const float v0 = c0 >= a.dvs ? 0.f : c0 == a.dv ? 1.f : row[a.v_at + c0], v1 = c0 + 8 >= a.dvs ? 0.f : c0 + 8 == a.dv ? 1.f : row[a.v_at + c0 + 8];
+        const float u0 = bt * (v0 - gg * r0), u1 = bt * (v1 - gg * r1);
+        float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = row0 + 8 * nt + 2 * t + e;
+                if (r >= a.d) continue;
+                s[nt][e] = fmaf(kr[r], u0, gg * s[nt][e]);
+                s[nt][2 + e] = fmaf(kr[r], u1, gg * s[nt][2 + e]);
+                if (a.o) { o0 = fmaf(s[nt][e], qr[r], o0); o1 = fmaf(s[nt][2 + e], qr[r], o1); }
+            }
+        if (!a.o) continue;
+        o0 += __shfl_xor_sync(0xffffffffu, o0, 1); o1 += __shfl_xor_sync(0xffffffffu, o1, 1);
+        o0 += __shfl_xor_sync(0xffffffffu, o0, 2); o1 += __shfl_xor_sync(0xffffffffu, o1, 2);
+        float* ro = red + CR_WARPS * CR_COLS;
+        __syncthreads();
+        if (t == 0) { ro[warp * CR_COLS + g] = o0; ro[warp * CR_COLS + g + 8] = o1; }
+        __syncthreads();
+        if (tid < CR_COLS && a.col0 + tid < a.dvs) {
+            float x = 0.f;
+#pragma unroll
+            for (int k = 0; k < CR_WARPS; ++k) x += ro[k * CR_COLS + tid];
+            a.o[(size_t)tk * a.H * a.dvs + a.col0 + tid] = x * a.o_scale;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NT * 4; ++i) sv[i] = s[i >> 2][i & 3];
+}
 
 template <int DS, bool VEC, bool DELTA>
 __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
@@ -241,7 +330,7 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
                 if (DELTA) cr_cp16(dst + L::K + (r0 + r) * L::QS + c, x + CR * DS);
                 cr_cp16(dst + L::N + (r0 + r) * L::KS + c, x + 2 * CR * DS);
             }
-            if (tid < DS / 4) cr_cp16(dst + L::G + tid * 4, src + 512 + 3 * CR * DS + tid * 4);
+            if (tid < DS / 4 + 1) cr_cp16(dst + L::G + tid * 4, src + 512 + 3 * CR * DS + tid * 4);
         } else {
             const float* row = w.qkv + (size_t)(start + ch * CR + r0) * w.ld + kh * D.d + c;
             const int left = c < D.d ? len - ch * CR - r0 : 0;
@@ -275,6 +364,15 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
                 if (!DELTA && e < 2) bn[n][e] = w.beta && tk < len ? w.beta[(size_t)(start + tk) * D.H + h] : 1.f;
             }
     };
+    // whether this thread's part of the state has left the finite numbers
+    auto state_bad = [&]() {
+        float x = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) cr_watch(x, s[nt][e]);
+        return !(x == 0.f);
+    };
     stage(0);
     values(0);
     for (int ch = 0; ch < nch; ++ch) {
@@ -285,9 +383,20 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[n][e] = DELTA ? vn[n][e] : vn[n][e] * bn[n][e & 1];
         cp_async_wait<0>();
-        __syncthreads();                                  // chunk ch has landed; everyone is done with the other half and the partial sums
+        const bool lost = __syncthreads_or(state_bad());  // chunk ch has landed; everyone is done with the other half and the partial sums
         if (ch + 1 < nch) { stage(ch + 1); values(tok0 + CR); }
         const float* st = sm + (ch & 1) * L::FLOATS;
+        if (!VEC) prod *= st[L::G + 32];
+        bool plain = lost || st[L::G + cr_mark(DS, VEC)] != 0.f;
+        float u[2][4];
+        auto total = [&](int part, int n, int c) {
+            const float* p = red + (part * CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t;
+            float2 x = *reinterpret_cast<const float2*>(p);
+#pragma unroll
+            for (int k = 1; k < CR_WARPS; ++k) { const float2 y = *reinterpret_cast<const float2*>(p + k * 2 * CR_COLS * CR_RS); x.x += y.x; x.y += y.y; }
+            return x;
+        };
+        if (!plain) {
         if (DELTA || sg.pass != 1) {
         // ---- this warp's rows' share of S^T q and R; the small terms in accumulators of their own, so that no product waits for the one before it
         float oq[2][4], rk[2][4], oql[2][4], rkl[2][4];
@@ -326,14 +435,6 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
             }
         }
         if (DELTA || sg.pass != 1) __syncthreads();
-        auto total = [&](int part, int n, int c) {
-            const float* p = red + (part * CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t;
-            float2 x = *reinterpret_cast<const float2*>(p);
-#pragma unroll
-            for (int k = 1; k < CR_WARPS; ++k) { const float2 y = *reinterpret_cast<const float2*>(p + k * 2 * CR_COLS * CR_RS); x.x += y.x; x.y += y.y; }
-            return x;
-        };
-        float u[2][4];
         if (DELTA) {                                      // every warp forms all of U: it is the update's operand
 #pragma unroll
             for (int n = 0; n < 2; ++n)
@@ -357,6 +458,25 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
 #pragma unroll
                 for (int e = 0; e < 4; ++e) u[n][e] = v[n][e];
         }
+        float x = 0.f;                                    // every warp holds the same U and sees the same
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) cr_watch(x, u[n][e]);
+        plain = __any_sync(0xffffffffu, !(x == 0.f));
+        }
+        if (plain) {
+            const size_t at = (size_t)(start + tok0) * D.H + h;
+            const CrTokens a{w.qkv + (size_t)(start + tok0) * w.ld, w.decay + at * (VEC ? D.d : 1), w.beta ? w.beta + at : nullptr, sg.pass == 1 ? nullptr : o + at * dvs,
+                             min(CR, len - tok0), w.ld, w.k_off + kh * D.d, w.q_off + kh * D.d, w.v_off + h * D.dv, D.H, D.d, D.dv, dvs, col0, D.o_scale};
+            float sv[NT * 4];
+#pragma unroll
+            for (int i = 0; i < NT * 4; ++i) sv[i] = s[i >> 2][i & 3];
+            cr_by_token<DS, VEC, DELTA>(a, sv, red);
+#pragma unroll
+            for (int i = 0; i < NT * 4; ++i) s[i >> 2][i & 3] = sv[i];
+            continue;
+        }
         if (warp < 2 && sg.pass != 1) {                                   // the read-out of 8 tokens each
             const int n = warp;
             float out[4], add[4] = {0.f, 0.f, 0.f, 0.f};
@@ -375,7 +495,6 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
                 if (tk < len && c < dvs) o[((size_t)(start + tk) * D.H + h) * dvs + c] = (out[e] + add[e]) * D.o_scale;
             }
         }
-        if (!VEC) prod *= st[L::G + 32];
         // ---- state update: the chunk's own sum from zero, so that the state itself is only ever rounded to nearest (the matrix unit's sums are cut off)
         if (!VEC) {
 #pragma unroll
