@@ -119,14 +119,13 @@ constexpr uint32_t tc_idesc(int m, int n) {
                    "=r"(v[30]), "=r"(v[31])                                                                             \
                  : "r"(taddr) : "memory")
 
-// CL = thread-block-cluster size: the CL CTAs of a cluster work on the SAME 128 tokens and CL consecutive 128-row
-// weight tiles; each CTA TMA-loads 128/CL tokens of the activation stage and multicasts them to all CL CTAs, so the
-// L2 -> SM activation traffic (the limiter of this kernel: ~6300 B/clk chip-wide) drops by CL.
+// Every CTA loads its activation tiles itself: sharing them between the CTAs of a cluster by one load was worth 1 to 3 % on prompt shapes, but such a
+// load must not meet another GPU's memory, and tensor-parallel processes run this kernel too.
 // NU = unpack warp groups (4 warps each, one per TMEM lane quarter); group g expands the stages with item % NU == g.
 // One warp issues ~190 instructions per stage at IPC ~0.3, so a single group paces the kernel at ~850 clk per stage
 // (measured) against the 256-clk tensor floor; three groups bring the unpack under the floor.
 // SPLIT: the few-token form, a cluster of K parts.  An instance of its own: its branches in the batched-decode form cost that 2 % of a 64-sequence step.
-template <int CL, int NU, bool SPLIT = false>
+template <int NU, bool SPLIT = false>
 __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const TcParams p) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[TC_STAGES];    // TMA bytes + 4 unpack-warp arrivals
@@ -137,27 +136,25 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;   // 128B-swizzle atoms need 1024-B alignment
-    const int crank = (CL > 1) ? (int)(blockIdx.x % CL) : 0;          // 1-D cluster: rank == blockIdx.x % CL
-    const int ksp = SPLIT ? p.ksplit : 1;                           // cluster of K parts (one tile per cluster) instead of a cluster of tiles
+    const int ksp = SPLIT ? p.ksplit : 1;                           // the CTAs of a cluster take K parts of one tile
     const int krank = ksp > 1 ? (int)(blockIdx.x % ksp) : 0;
-    const int cluster_id = blockIdx.x / (CL * ksp), n_clusters = gridDim.x / (CL * ksp);
-    const int ngroups = (p.tiles_n + CL - 1) / CL;                    // groups of CL weight-row tiles
-    const int total_tiles = ngroups * p.tiles_m * p.splitk;           // cluster tiles (x K-splits in the decode form)
-    const int my_tiles = (total_tiles - cluster_id + n_clusters - 1) / n_clusters;
+    const int worker = blockIdx.x / ksp, workers = gridDim.x / ksp;
+    const int total_tiles = p.tiles_n * p.tiles_m * p.splitk;         // tiles (x K-splits in the decode form)
+    const int my_tiles = (total_tiles - worker + workers - 1) / workers;
     const int k_part0 = ksp > 1 ? krank * p.KB / ksp : 0;             // this CTA's first k-block
     const int KBs = ksp > 1 ? (krank + 1) * p.KB / ksp - k_part0 : p.KBs;   // k-blocks per tile (== KB unless split)
     const int n_items = my_tiles * KBs;
     auto tile_coords = [&](int tl, int& m_blk, int& n_blk, int& ks) {
-        const int ct0 = cluster_id + tl * n_clusters;
+        const int ct0 = worker + tl * workers;
         ks = ct0 % p.splitk;                                          // splits of one tile run side by side
         const int ct = ct0 / p.splitk;
-        m_blk = ct / ngroups;
-        n_blk = (ct - m_blk * ngroups) * CL + crank;                  // may be >= tiles_n (padding tile: epilogue masks it)
+        m_blk = ct / p.tiles_n;
+        n_blk = ct - m_blk * p.tiles_n;
     };
     pdl_launch_dependents();   // no-op unless launched with programmatic stream serialisation (decode step)
 
     if (tid == 0) {
-        for (int s = 0; s < TC_STAGES; ++s) { mbar_init(&full_bar[s], 5); mbar_init(&empty_bar[s], CL); }
+        for (int s = 0; s < TC_STAGES; ++s) { mbar_init(&full_bar[s], 5); mbar_init(&empty_bar[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], TC_EPW); }
         fence_mbar_init();
     }
@@ -168,10 +165,6 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
     }
     tc_fence_before();
     __syncthreads();
-    if (CL > 1) {   // peers must see initialised barriers before the first multicast / remote commit
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    }
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
 
@@ -181,24 +174,17 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
             asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_q) : "memory");
             pdl_wait_prior();   // the activations are the previous kernel's output (the weights are not: unpack warps run ahead)
             int it = 0;
-            constexpr int SLICE = TC_BN / CL;   // tokens this CTA fetches for the whole cluster
             for (int tl = 0; tl < my_tiles; ++tl) {
                 int m_blk, n_blk, ks;
                 tile_coords(tl, m_blk, n_blk, ks);
                 for (int kb = 0; kb < KBs; ++kb, ++it) {
                     const int kg = ks * KBs + k_part0 + kb;
                     const int s = it % TC_STAGES;
-                    mbar_wait(&empty_bar[s], (uint32_t)(((it / TC_STAGES) & 1) ^ 1));   // all CL CTAs retired this slot
-                    if (CL == 1 && (p.dbg & 8)) { mbar_arrive(&full_bar[s]); continue; }  // timing experiment: no activation traffic
-                    mbar_expect_tx(&full_bar[s], TC_STAGE_BYTES);                        // own barrier: all CL slices land here
-                    const uint32_t dst = ring + s * TC_STAGE_BYTES + crank * SLICE * TC_BK;
-                    if (CL == 1)
-                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                     ::"r"(dst), "l"(&tmap_q), "r"(kg * TC_BK), "r"(m_blk * TC_BN), "r"(smem_u32(&full_bar[s])) : "memory");
-                    else
-                        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, {%2, %3}], [%4], %5;"
-                                     ::"r"(dst), "l"(&tmap_q), "r"(kg * TC_BK), "r"(m_blk * TC_BN + crank * SLICE), "r"(smem_u32(&full_bar[s])),
-                                       "h"((uint16_t)((1u << CL) - 1)) : "memory");
+                    mbar_wait(&empty_bar[s], (uint32_t)(((it / TC_STAGES) & 1) ^ 1));   // the slot's products are done
+                    if (p.dbg & 8) { mbar_arrive(&full_bar[s]); continue; }  // timing experiment: no activation traffic
+                    mbar_expect_tx(&full_bar[s], TC_STAGE_BYTES);
+                    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                                 ::"r"(ring + s * TC_STAGE_BYTES), "l"(&tmap_q), "r"(kg * TC_BK), "r"(m_blk * TC_BN), "r"(smem_u32(&full_bar[s])) : "memory");
                 }
             }
         }
@@ -245,11 +231,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
                         tc_mma_i8_ts(d_tmem, at + 8, bd + 2, idesc, 1u);
                         tc_mma_i8_ts(d_tmem, at + 16, bd + 4, idesc, 1u);
                         tc_mma_i8_ts(d_tmem, at + 24, bd + 6, idesc, 1u);
-                        if (CL == 1)
-                            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(empty0 + s * 8) : "memory");
-                        else   // the slot is refilled by every CTA of the cluster: tell all of them
-                            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                                         ::"r"(empty0 + s * 8), "h"((uint16_t)((1u << CL) - 1)) : "memory");
+                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(empty0 + s * 8) : "memory");
                         if (++kb == KBs) {
                             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tfull0 + (tl & 1) * 8) : "memory");
                             kb = 0; ++tl;
@@ -535,10 +517,6 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
     }
     tc_fence_before();
     __syncthreads();
-    if (CL > 1) {   // nobody leaves while a peer may still multicast into this CTA's ring or signal its barriers
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    }
     if (warp == W_MMA) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TC_TMEM_COLS) : "memory");
@@ -551,17 +529,14 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static EncodeTiledFn g_encode = nullptr;
 static DevOnce g_tc_attr;
-static int g_tc_cluster = 0, g_tc_nu = 0;
+static int g_tc_nu = 0;
 
 void gemm_tc_init_attrs() {
     if (g_tc_attr.need()) {
-        bool ok = cudaFuncSetAttribute(ternary_gemm_tc_kernel<1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<1, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<1, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<2, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
-        ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
+        bool ok = cudaFuncSetAttribute(ternary_gemm_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
+        ok = ok && cudaFuncSetAttribute(ternary_gemm_tc_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM) == cudaSuccess;
         (void)ok;
     }
     if (!g_encode) {
@@ -570,23 +545,19 @@ void gemm_tc_init_attrs() {
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qr) == cudaSuccess && qr == cudaDriverEntryPointSuccess)
             g_encode = (EncodeTiledFn)fn;
     }
-    if (!g_tc_cluster) {
-        const char* e = getenv("WF_TC_CLUSTER");
-        // pairs of CTAs share one multicast activation tile: 2B prefill shape 2312 -> 2331 TOP/s, 8B 2146 -> 2221 (call r02ah); 4 is slower
-        g_tc_cluster = e ? atoi(e) : 2;
-        if (g_tc_cluster != 1 && g_tc_cluster != 2 && g_tc_cluster != 4) g_tc_cluster = 2;
+    if (!g_tc_nu) {
         const char* u = getenv("WF_TC_NU");
         g_tc_nu = u ? atoi(u) : 2;     // two unpack groups: 18 warps at 112 registers (three groups = 22 warps at 88 spill)
         if (g_tc_nu < 1 || g_tc_nu > 3) g_tc_nu = 2;
     }
 }
 
-template <int CL, int NU>
-static int launch_tc_cl(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s) {
+template <int NU>
+static int launch_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s) {
     CUtensorMap tmap;
     const cuuint64_t gdim[2] = {(cuuint64_t)a->K, (cuuint64_t)a->M};
     const cuuint64_t gstride[1] = {(cuuint64_t)a->ldq};
-    const cuuint32_t box[2] = {TC_BK, TC_BN / CL};
+    const cuuint32_t box[2] = {TC_BK, TC_BN};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult cr = g_encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)a->q, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -599,29 +570,13 @@ static int launch_tc_cl(const wf_linear_args* a, const EpiParams& ep, cudaStream
     p.ep = ep;
     p.splitk = 1; p.KBs = p.KB; p.ksplit = 1; p.red_acc = nullptr; p.red_ld = 0; p.l2_ahead = 0;
     { const char* d = getenv("WF_TC_DBG"); p.dbg = d ? atoi(d) : 0; }
-    const int total = ((p.tiles_n + CL - 1) / CL) * p.tiles_m;
+    const int total = p.tiles_n * p.tiles_m, sms = sm_count();
     cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(total < sms ? total : sms);
     cfg.blockDim = dim3(tc_threads(NU));
     cfg.dynamicSmemBytes = TC_SMEM;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = CL > 1 ? 1 : 0;
-    static int max_clusters = 0;   // per CL instantiation
-    if (!max_clusters) {
-        max_clusters = sm_count() / CL;
-        if (CL > 1) {
-            cfg.gridDim = dim3(sm_count() / CL * CL);
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, ternary_gemm_tc_kernel<CL, NU>, &cfg) == cudaSuccess && n > 0) max_clusters = n;
-            else cudaGetLastError();
-        }
-    }
-    const int clusters = total < max_clusters ? total : max_clusters;
-    cfg.gridDim = dim3(clusters * CL);
-    return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<CL, NU>, tmap, p), "ternary_gemm_tc");
+    return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<NU>, tmap, p), "ternary_gemm_tc");
 }
 
 // Batched-decode form (the engine's phase kernels, 32 < M <= 128): S[m][n] += sum over this launch's K columns, added into the
@@ -668,7 +623,7 @@ int launch_gemm_tc_red(const uint8_t* w_tile, int N, int K, const int8_t* q, int
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = pdl ? 1 : 0;
-    return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<1, NU>, tmap, p), "ternary_gemm_tc(decode)");
+    return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<NU>, tmap, p), "ternary_gemm_tc(decode)");
 }
 
 // Few tokens: the tiles alone leave SMs idle and one CTA walks all of K, a latency chain of ~450 clk per k-block.  A cluster of ksplit CTAs shares
@@ -702,7 +657,7 @@ static int launch_tc_split(const wf_linear_args* a, const EpiParams& ep, int ksp
     at[0].val.clusterDim.x = ksplit; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<1, NU, true>, tmap, p), "ternary_gemm_tc(split)");
+    return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<NU, true>, tmap, p), "ternary_gemm_tc(split)");
 }
 
 int launch_gemm_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s) {
@@ -712,10 +667,8 @@ int launch_gemm_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s)
     int ksplit = 1;
     while (ksplit < 8 && tiles * ksplit * 2 <= sms && a->K / WF_QK >= ksplit * 2 * 4) ksplit *= 2;
     if (ksplit > 1) return launch_tc_split(a, ep, ksplit, s);
-    if (g_tc_cluster == 4) return launch_tc_cl<4, 2>(a, ep, s);
-    if (g_tc_cluster == 2) return g_tc_nu == 2 ? launch_tc_cl<2, 2>(a, ep, s) : launch_tc_cl<2, 3>(a, ep, s);
-    if (g_tc_nu == 1) return launch_tc_cl<1, 1>(a, ep, s);
-    return g_tc_nu == 2 ? launch_tc_cl<1, 2>(a, ep, s) : launch_tc_cl<1, 3>(a, ep, s);
+    if (g_tc_nu == 1) return launch_tc<1>(a, ep, s);
+    return g_tc_nu == 2 ? launch_tc<2>(a, ep, s) : launch_tc<3>(a, ep, s);
 }
 
 }  // namespace wf
