@@ -8,6 +8,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <pybind11/pybind11.h>
 #include <torch/library.h>
 
 #include <map>
@@ -20,16 +21,27 @@ namespace {
 
 using at::Tensor;
 
+// wf_bitnet._lib.WfError, as the calls through ctypes raise it: callers tell a failed launch from a bad argument by its type
+[[noreturn]] void raise_wf_error(const std::string& msg) {
+    if (Py_IsInitialized()) {
+        pybind11::gil_scoped_acquire gil;
+        const pybind11::object type = pybind11::module_::import("wf_bitnet._lib").attr("WfError");
+        PyErr_SetString(type.ptr(), msg.c_str());
+        throw pybind11::error_already_set();
+    }
+    TORCH_CHECK(false, msg);
+}
+
 void check(int rc) {          // the Python side's mapping of the C status
     if (rc == 0) return;
     const char* msg = wf_last_error();
     TORCH_CHECK_VALUE(rc != -1, msg);
     TORCH_CHECK_NOT_IMPLEMENTED(rc != -2, msg);
-    TORCH_CHECK(false, msg);
+    raise_wf_error(msg);
 }
 
 void need_gpu(std::initializer_list<const Tensor*> ts) {
-    TORCH_CHECK(wf_bitnet_available(), "no compute-capability-10.x CUDA device visible; the BitNet kernels are sm_100a-only and there is no CPU fallback");
+    if (!wf_bitnet_available()) raise_wf_error("no compute-capability-10.x CUDA device visible; the BitNet kernels are sm_100a-only and there is no CPU fallback");
     for (const Tensor* t : ts) TORCH_CHECK_VALUE(t->is_cuda(), "expected a CUDA tensor (the B200 BitNet ops have no CPU path)");
 }
 
@@ -202,11 +214,15 @@ TORCH_LIBRARY(wf_native, m) {
     m.def("paged_decode_attn(Tensor q, Tensor pool, int max_pages, int layers, int kv_heads, int page_size, int head_dim, int kv_dtype, int layer, Tensor block_table, "
           "Tensor seq_lens, float scale, ScalarType out_dtype) -> Tensor");
 }
-TORCH_LIBRARY_IMPL(wf_native, CUDA, m) {
-    m.impl("linear", linear);
-    m.impl("mlp", mlp);
-    m.impl("paged_decode_attn", paged_decode_attn);
-}
+// CPU: the same functions, for their errors (a missing GPU, a tensor that is not on it).
+#define WF_NATIVE_IMPL(key)                    \
+    TORCH_LIBRARY_IMPL(wf_native, key, m) {    \
+        m.impl("linear", linear);              \
+        m.impl("mlp", mlp);                    \
+        m.impl("paged_decode_attn", paged_decode_attn); \
+    }
+WF_NATIVE_IMPL(CUDA)
+WF_NATIVE_IMPL(CPU)
 TORCH_LIBRARY_IMPL(sgl_kernel, CUDA, m) {
     m.impl("bitnet_gemv_cpu", bitnet_gemv);
     m.impl("bitnet_gemv", bitnet_gemv);
