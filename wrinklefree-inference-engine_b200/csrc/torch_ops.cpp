@@ -214,7 +214,8 @@ TORCH_LIBRARY(wf_native, m) {
     m.def("paged_decode_attn(Tensor q, Tensor pool, int max_pages, int layers, int kv_heads, int page_size, int head_dim, int kv_dtype, int layer, Tensor block_table, "
           "Tensor seq_lens, float scale, ScalarType out_dtype) -> Tensor");
 }
-// CPU: the same functions, for their errors (a missing GPU, a tensor that is not on it).
+// CPU: the same functions, for their errors (a missing GPU, a tensor that is not on it).  Autograd: passed through, so that the outputs are plain tensors
+// whatever the inputs require, as behind the calls through ctypes.
 #define WF_NATIVE_IMPL(key)                    \
     TORCH_LIBRARY_IMPL(wf_native, key, m) {    \
         m.impl("linear", linear);              \
@@ -223,6 +224,11 @@ TORCH_LIBRARY(wf_native, m) {
     }
 WF_NATIVE_IMPL(CUDA)
 WF_NATIVE_IMPL(CPU)
+TORCH_LIBRARY_IMPL(wf_native, Autograd, m) {
+    m.impl("linear", torch::CppFunction::makeFallthrough());
+    m.impl("mlp", torch::CppFunction::makeFallthrough());
+    m.impl("paged_decode_attn", torch::CppFunction::makeFallthrough());
+}
 TORCH_LIBRARY_IMPL(sgl_kernel, CUDA, m) {
     m.impl("bitnet_gemv_cpu", bitnet_gemv);
     m.impl("bitnet_gemv", bitnet_gemv);
