@@ -167,7 +167,7 @@ Tensor mlp(const Tensor& x, const Tensor& gate_up_tile, int64_t N2, const Tensor
     TORCH_CHECK_VALUE(dw.dim() == 2, "packed weights must be 2-D");
     const int M = (int)x2.size(0), K = (int)x2.size(1), F = (int)N2 / 2, D = (int)dw.size(0);
     TORCH_CHECK_VALUE(dw.size(1) * 4 == F, "activations.shape[-1] != in_features");
-    TORCH_CHECK_VALUE(g.scalar_type() == at::kBFloat16 && g.numel() == F, "ffn_sub_norm must have one weight per feed-forward row");
+    TORCH_CHECK_VALUE(g.scalar_type() == at::kBFloat16 && g.numel() >= F, "ffn_sub_norm must have one weight per feed-forward row");
     Quant q = quantize(x2, true);
     const auto bf = x2.options().dtype(at::kBFloat16);
     Tensor h = at::empty({M, F}, bf), ws, ws2;
