@@ -16,7 +16,7 @@ calling them with CPU tensors raises (no CPU fallback).  `*_cuda`-free aliases a
 """
 import torch
 
-from wf_bitnet import _native
+from wf_bitnet import _lib, _native
 from wf_bitnet import ops as _wf
 
 _LIB = torch.library.Library("sgl_kernel", "FRAGMENT")
@@ -34,8 +34,21 @@ _DEFS = {
 }
 
 
-def _not_built(*args, **kwargs):
-    return _native.ops()          # raises: libwf_torch.so holds these kernels
+def _gemv(packed_weights, activations, scale):
+    return _wf.bitnet_gemv(packed_weights, activations, scale)
+
+
+def _gemm(packed_weights, activations, scale):
+    return _wf.bitnet_gemm(packed_weights, activations, scale)
+
+
+def _quant(activations):
+    q, scale, _ = _wf.quantize_activations(activations, per_token=False)
+    return q, scale
+
+
+def _absent(*args, **kwargs):
+    return _native.ops()          # raises: no library has been built
 
 
 def _fake_gemv(packed_weights, activations, scale):
@@ -111,8 +124,8 @@ def _fake_mlp(x, gate_w, up_w, down_w, gate_scale, up_scale, down_scale, ffn_sub
     return torch.empty(*x.shape[:-1], down_w.shape[0], dtype=x.dtype, device=x.device)
 
 
-# None: the CUDA kernel is native (csrc/torch_ops.cpp)
-_IMPL = {"bitnet_gemv": (None, _fake_gemv), "bitnet_gemm": (None, _fake_gemm), "bitnet_quantize_activations": (None, _fake_quant),
+# the first three only where libwf_torch.so, which registers native ones, is absent or does not load
+_IMPL = {"bitnet_gemv": (_gemv, _fake_gemv), "bitnet_gemm": (_gemm, _fake_gemm), "bitnet_quantize_activations": (_quant, _fake_quant),
          "bitnet_qkv_forward": (_qkv_forward, _fake_qkv), "bitnet_mlp_forward": (_mlp_forward, _fake_mlp)}
 
 _registered = False
@@ -124,13 +137,12 @@ def register():
         return
     for name, schema in _DEFS.items():
         _LIB.define(name + schema)
-    built = _native.TORCH_LIB_PATH.exists()
-    if built:
-        _native.ops()
+    built = _lib.LIB_PATH.exists()
+    native = built and _native.is_native()
     for name in _DEFS:
         impl, fake = _IMPL[name.replace("_cpu", "")]
-        if impl is not None or not built:
-            _LIB.impl(name, impl or _not_built, "CUDA")
+        if not (native and impl in (_gemv, _gemm, _quant)):
+            _LIB.impl(name, impl if built else _absent, "CUDA")
         torch.library.register_fake(f"sgl_kernel::{name}", fake, lib=_LIB)
     _registered = True
 

@@ -289,6 +289,23 @@ def rope_kv_append(qkv: torch.Tensor, H: int, kv: PagedKV, layer: int, positions
     return q_out
 
 
+_attn_ws = {}
+
+
+def paged_decode_attn_ctypes(q, layout: KvLayout, layer: int, block_table, seq_lens, scale: float, out_dtype: torch.dtype) -> torch.Tensor:
+    _need_cuda(q, block_table, seq_lens)
+    B, H, D = q.shape
+    out = torch.empty(B, H, D, dtype=out_dtype, device=q.device)
+    nbytes = int(lib().wf_attn_workspace_bytes(B, H, D, block_table.shape[1] * layout.page_size))
+    key = (q.device.index, _stream())
+    ws = _attn_ws.get(key)
+    if ws is None or ws.numel() < nbytes:
+        ws = _attn_ws[key] = torch.empty(nbytes, dtype=torch.uint8, device=q.device)
+    check(lib().wf_paged_decode_attn(q.contiguous().data_ptr(), C.byref(layout), layer, block_table.data_ptr(), block_table.shape[1], seq_lens.data_ptr(), B, H, float(scale),
+                                     out.data_ptr(), _DT[out_dtype], ws.data_ptr(), ws.numel(), _stream()))
+    return out
+
+
 def paged_decode_attn(q: torch.Tensor, kv: PagedKV, layer: int, block_table: torch.Tensor, seq_lens: torch.Tensor,
                       scale: Optional[float] = None, out_dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
     if not (q.is_cuda and block_table.is_cuda and seq_lens.is_cuda):
