@@ -104,3 +104,33 @@ def test_latent_with_expanded_keys(heads, dim, rot, vdim, rank):
     check(model, rows, [[40, 600], [560, 0], [501, 0]], wants, W)
     check(model, rows, [[600, 0], [1, 599], [500, 1]], wants, W)
     model.close()
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("kind", ["grouped", "latent"])
+def test_rows_that_do_not_see_a_value_stay_finite(kind, bad):
+    """A token whose row holds a NaN or an infinity leaves the tokens before it as they are, also those that share its tile of keys or of rows."""
+    W, at, n = 64, 437, 520
+    if kind == "grouped":
+        m = {"heads": 4, "kv_heads": 2, "dim": 64, "vdim": 64, "scale": 0.125}
+        cfg = {"architecture": "Tutizen", "vocab": 31, "width": W, "norm": {"eps": 1e-5}, "residual_mult": 1.0, "layers": [{"type": "attention", "mixer": m, "mlp": None}]}
+        w = TO.random_weights(cfg, 5)
+        P = d64(w, "l0.mix.")
+        want = lambda x: TO.attention(x, P, m, 1e-5)[0]           # noqa: E731
+    else:
+        m = {"heads": 20, "dim": 96, "rot_dim": 32, "vdim": 128, "kv_rank": 512, "q_rank": 48, "scale": 128 ** -0.5,
+             "rot": {"dims": 32, "base": 10000.0, "scaling": {"factor": 4.0, "original": 256, "fast": 32.0, "slow": 1.0}}}
+        cfg = {"architecture": "Fivedra", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5},
+               "layers": [{"type": "latent_attention", "mixer": m, "mlp": None}]}
+        w = FO.random_weights(cfg, 6)
+        P = d64(w, "l0.mix.")
+        want = lambda x: FO.latent_attention(x, P, "", m, 1e-5)   # noqa: E731
+    row = inputs([n], W, 11)[0]
+    ref = want(torch.from_numpy(row).double()).numpy()
+    row[at, 5] = bad
+    model = build(cfg, w, 16, {})
+    got = model.engine.run_part(0, 2, [model.admit()], [n], row)
+    model.close()
+    assert np.isfinite(got[:at]).all() and not np.isfinite(got[at:]).all(-1).any()
+    err = np.sqrt(((got[:at] - ref[:at]) ** 2).mean(-1)) / np.sqrt((ref[:at] ** 2).mean(-1))
+    assert err.max() < TOL

@@ -16,6 +16,8 @@
 // into the exponent's multiply-add.  Measured, 2048 tokens causal, 20 heads of 128: grouped-query attention 181 -> 60 us (mma.sync kernel before),
 // latent attention 895 -> 58 us (one CTA per token before; plus 40 us for the expansion).
 // Every wait is bounded: one that runs out records an error word that the host checks, and the CTA drains and leaves.
+// A value that is infinite or NaN meets the zero weights of the rows of its key tile that do not see it, too: a row whose sum of weights is finite and
+// whose output is not is taken again by its warp, over the keys that it sees (at_row).
 #include "seq_attn_mma.cuh"
 #include <cuda.h>
 #include <math.h>
@@ -42,6 +44,8 @@ struct AtParams {
     const int32_t* key_row;        // dense keys: a sequence's first row in the buffer (null: paged)
     int rep, tq;                   // query heads per key/value head, tokens per row tile
     int box;                       // keys per TMA box
+    const __nv_bfloat16 *k, *v;    // what the tensor maps cover, and their strides in elements
+    long long k_row, k_head, v_row, v_head, page_stride;
     int* err;
 };
 
@@ -108,10 +112,61 @@ __device__ __forceinline__ uint64_t at_fma2(uint64_t a, uint64_t b, uint64_t c) 
 __device__ __forceinline__ uint64_t at_add2(uint64_t a, uint64_t b) { uint64_t v; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b)); return v; }
 __device__ __forceinline__ float at_ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }   // weights below 2^-126 are zero
 
+// One row of one head, key by key over what it sees, with a whole warp: a lane per key for the scores, then a lane per 4 output columns.  Not inlined: its
+// registers would come out of the kernel's.
+__device__ __noinline__ void at_row(const AtParams& p, const int32_t* bt, int row0, int kvh, int head, int tok, int pos) {
+    const GqaDims& D = p.D;
+    const int lane = threadIdx.x & 31;
+    const __nv_bfloat16* q = p.qn + ((size_t)tok * D.H + head) * D.d;
+    const float slope2 = D.dist_exp > 0.f ? exp2f(-D.dist_exp * (float)(head + 1) / (float)D.H) * LOG2E : 0.f, scale2 = D.scale * LOG2E;
+    float m = -INFINITY, l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+    auto place = [&](const __nv_bfloat16* base, long long row_stride, long long head_stride, int j) {
+        const int pg = bt ? j / p.page_size : 0;
+        return base + (bt ? (long long)bt[pg] * p.page_stride + (long long)(j - pg * p.page_size) * row_stride : (long long)(row0 + j) * row_stride) + kvh * head_stride;
+    };
+    for (int j0 = max(0, pos - D.window + 1); j0 <= pos; j0 += 32) {
+        const int j = j0 + lane;
+        float x = -INFINITY;
+        if (j <= pos) {
+            const __nv_bfloat16* kr = place(p.k, p.k_row, p.k_head, j);
+            float dot = 0.f;
+            for (int c = 0; c < D.d; ++c) dot = fmaf(__bfloat162float(q[c]), __bfloat162float(kr[c]), dot);
+            x = fmaf(dot, scale2, -slope2 * (float)(pos - j));
+        }
+        float top = x;
+#pragma unroll
+        for (int w = 16; w; w >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, w));
+        top = fmaxf(m, top);
+        const float f = top == -INFINITY ? 1.f : exp2f(m - top), e = x == -INFINITY ? 0.f : exp2f(x - top);
+        m = top;
+        l *= f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[k] *= f;
+        const int n = min(32, pos - j0 + 1);
+        for (int i = 0; i < n; ++i) {
+            const float w = __shfl_sync(0xffffffffu, e, i);
+            const __nv_bfloat16* vr = place(p.v, p.v_row, p.v_head, j0 + i);
+            l += w;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { const int c = lane + 32 * k; if (c < D.dv) acc[k] = fmaf(w, __bfloat162float(vr[c]), acc[k]); }
+        }
+    }
+    const float mul = (p.gate && !D.gate_elem ? p.gate[(size_t)tok * D.H + head] : 1.f) * am_inv_sum(D, head, m, l);
+    const size_t at = ((size_t)tok * D.H + head) * D.dv;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int c = lane + 32 * k;
+        if (c >= D.dv) continue;
+        float y = acc[k] * mul;
+        if (p.gate && D.gate_elem) y *= p.gate[at + c];
+        if (p.out_f32) ((float*)p.out)[at + c] = y; else ((__nv_bfloat16*)p.out)[at + c] = __float2bfloat16_rn(y);
+    }
+}
+
 // SPLIT: the weights as a two-term bf16 split (grouped-query attention); without it rounded to bf16 (latent attention)
 template <bool SPLIT>
 __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const Batch b,
-                                                                const AtParams p) {
+                                                                const __grid_constant__ AtParams p) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t q_full[2], k_full[2], k_empty[2], v_full[2], v_empty[2], v_fixed, s_full[2], p_full[2], o_full[2];
     __shared__ uint32_t tmem_base_s;
@@ -365,6 +420,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                 const float mul = r_ok ? (p.gate && !D.gate_elem ? p.gate[(size_t)tok * D.H + head] : 1.f) * am_inv_sum(D, head, m_ref, l) : 0.f;
                 const size_t at = ((size_t)(r_ok ? tok : 0) * D.H + head) * D.dv;
                 const float* ge = p.gate && D.gate_elem ? p.gate + at : nullptr;
+                float watch = 0.f;                         // times zero: NaN from the first sum that is not finite on
 #pragma unroll 1
                 for (int c = 0; c < D.dv; c += 32) {
                     uint32_t o[32];
@@ -377,7 +433,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                             if (c + k >= D.dv) break;
                             float v[8];
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(o[k + e]) * mul;
+                            for (int e = 0; e < 8; ++e) { watch = fmaf(__uint_as_float(o[k + e]), 0.f, watch); v[e] = __uint_as_float(o[k + e]) * mul; }
                             if (ge) {
                                 const float4 g0 = *reinterpret_cast<const float4*>(ge + c + k), g1 = *reinterpret_cast<const float4*>(ge + c + k + 4);
                                 v[0] *= g0.x; v[1] *= g0.y; v[2] *= g0.z; v[3] *= g0.w; v[4] *= g1.x; v[5] *= g1.y; v[6] *= g1.z; v[7] *= g1.w;
@@ -391,6 +447,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                             }
                         }
                     }
+                }
+                __syncwarp();
+                for (uint32_t redo = __ballot_sync(0xffffffffu, r_ok && !(watch == 0.f) && l * 0.f == 0.f); redo; redo &= redo - 1) {
+                    const int r = __ffs(redo) - 1;
+                    at_row(p, p.key_row ? nullptr : p.block_table + (size_t)b.seq_slot[sq] * p.max_blocks, p.key_row ? p.key_row[sq] : 0, kvh, __shfl_sync(0xffffffffu, head, r),
+                           __shfl_sync(0xffffffffu, tok, r), __shfl_sync(0xffffffffu, pos, r));
+                    __syncwarp();
                 }
             } else ok = false;
         }
@@ -460,8 +523,10 @@ int launch_attn_tc(const Batch& b, const GqaDims& D, const void* qn, const float
     CUtensorMap tk, tv;
     const __nv_bfloat16* k = (const __nv_bfloat16*)pc.pool + pc.layer_off;
     const uint64_t ps = pc.page_size;
-    if (int rc = at_encode(&tk, k, D.d, ps, D.d, D.G, ps * D.d, max_pages, pc.page_stride, p.box)) return rc;
-    if (int rc = at_encode(&tv, k + (size_t)D.G * ps * D.d, D.dv, ps, D.dv, D.G, ps * D.dv, max_pages, pc.page_stride, p.box)) return rc;
+    p.k = k; p.v = k + (size_t)D.G * ps * D.d;
+    p.k_row = D.d; p.k_head = (long long)ps * D.d; p.v_row = D.dv; p.v_head = (long long)ps * D.dv; p.page_stride = pc.page_stride;
+    if (int rc = at_encode(&tk, p.k, D.d, ps, p.k_row, D.G, p.k_head, max_pages, pc.page_stride, p.box)) return rc;
+    if (int rc = at_encode(&tv, p.v, D.dv, ps, p.v_row, D.G, p.v_head, max_pages, pc.page_stride, p.box)) return rc;
     return at_launch(b, p, true, tk, tv, s);
 }
 
@@ -480,6 +545,8 @@ int launch_attn_tc_dense(const Batch& b, const GqaDims& D, const void* qn, const
     p.err = tc_error_word();
     if (!p.err) return WF_ERR_CUDA;
     CUtensorMap tk, tv;
+    p.k = (const __nv_bfloat16*)k; p.v = (const __nv_bfloat16*)v;
+    p.k_row = p.v_row = row_stride; p.k_head = D.d; p.v_head = D.dv; p.page_stride = 0;
     if (int rc = at_encode(&tk, k, D.d, rows, row_stride, D.G, D.d, 1, (uint64_t)rows * row_stride, AT_KEYS)) return rc;
     if (int rc = at_encode(&tv, v, D.dv, rows, row_stride, D.G, D.dv, 1, (uint64_t)rows * row_stride, AT_KEYS)) return rc;
     return at_launch(b, p, false, tk, tv, s);
