@@ -168,7 +168,7 @@ template <bool SPLIT>
 __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const Batch b,
                                                                 const __grid_constant__ AtParams p) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t q_full[2], k_full[2], k_empty[2], v_full[2], v_empty[2], v_fixed, s_full[2], p_full[2], o_full[2];
+    __shared__ __align__(8) uint64_t q_full[2], k_full[2], k_empty[2], v_full[2], v_empty[2], v_fixed, s_full[2], p_full[2], o_full[2], drained;
     __shared__ uint32_t tmem_base_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const GqaDims& D = p.D;
@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 4); mbar_init(&o_full[i], 1);
         }
         mbar_init(&v_fixed, 1);
+        mbar_init(&drained, 1);
         fence_mbar_init();
     }
     if (warp == 9) {
@@ -222,6 +223,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         const int kh = D.d > 64 ? 2 : 1, vh = D.dv > 64 ? 2 : 1, nbox = AT_KEYS / p.box;
         const int row0 = p.key_row ? p.key_row[sq] : 0;
         bool ok = true;
+        int issued[2] = {0, 0};                           // tiles of keys and of values under way or landed
         for (int i = 0; i < nt && ok; ++i) {
             const int st = i & 1, u = lo + i, j = u * AT_KEYS + lane * p.box;
             const bool mine = lane < nbox && j <= pos_last;
@@ -243,6 +245,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                                      ::"r"(dst + h * AT_HALF), "l"(kv ? &tmap_v : &tmap_k), "r"(h * 64), "r"(slot), "r"(kvh), "r"(page), "r"(smem_u32(full)) : "memory");
                 }
                 __syncwarp();
+                issued[kv] = i + 1;
             }
             if (ok && u == hi && fix_row < AT_KEYS) {
                 if (!at_wait_warp(&v_full[st], (uint32_t)((i >> 1) & 1))) { ok = false; break; }
@@ -255,7 +258,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                 if (lane == 0) mbar_arrive(&v_fixed);
             }
         }
-        if (!ok && lane == 0) atomicExch(p.err, 4);
+        if (!ok) {                                        // the CTA leaves early, but not before its copies have landed
+            if (lane == 0) atomicExch(p.err, 4);
+            for (int kv = 0; kv < 2; ++kv)
+                for (int i = max(0, issued[kv] - 2); i < issued[kv]; ++i) at_wait_warp(kv ? &v_full[i & 1] : &k_full[i & 1], (uint32_t)((i >> 1) & 1));
+        }
     } else if (warp == 9) {
         // ------------------------------------------------------------ MMA issuer
         uint32_t elected;
@@ -305,6 +312,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                 if (i + 1 < nt) at_commit(&k_empty[st1]);
             }
             if (!ok) atomicExch(p.err, 5);
+            at_commit(&drained);                          // nor while a product still reads shared memory or TMEM
+            at_wait(&drained, 0);
         }
         __syncwarp();
     } else {

@@ -102,7 +102,7 @@ __device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity) {
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
                                                                 const TcParams p) {
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t full_bar[TC_STAGES], empty_bar[TC_STAGES], tfull_bar[2], tempty_bar[2];
+    __shared__ __align__(8) uint64_t full_bar[TC_STAGES], empty_bar[TC_STAGES], tfull_bar[2], tempty_bar[2], drained;
     __shared__ uint32_t tmem_base_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     if (tid == 0) {
         for (int s = 0; s < TC_STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * TC_EPW); }
+        mbar_init(&drained, 1);
         fence_mbar_init();
     }
     if (warp == TC_EPW + 1) {
@@ -157,7 +158,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
             }
             // the last stages' hand-backs come from the other CTA too: none may be under way when this CTA leaves
             for (int j = it > TC_STAGES ? it - TC_STAGES : 0; ok && j < it; ++j) ok = wait_bounded(smem_u32(&empty_bar[j % TC_STAGES]), (uint32_t)((j / TC_STAGES) & 1));
-            if (!ok) atomicExch(p.err, 1);
+            if (!ok) {                                                     // the pair leaves early, but not before its copies have landed (both CTAs' report to the first)
+                atomicExch(p.err, 1);
+                for (int j = it > TC_STAGES ? it - TC_STAGES : 0; rank == 0 && j < it; ++j) wait_bounded(smem_u32(&full_bar[j % TC_STAGES]), (uint32_t)((j / TC_STAGES) & 1));
+            }
         }
         __syncwarp();
     } else if (warp == TC_EPW + 1) {
@@ -194,7 +198,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
                 commit_pair(smem_u32(&tfull_bar[buf]));
                 ++done;
             }
-            if (!ok) atomicExch(p.err, 2);
+            if (!ok) {                                                     // nor while a product still reads shared memory
+                atomicExch(p.err, 2);
+                commit_pair(smem_u32(&drained));
+                wait_bounded(smem_u32(&drained), 0);
+            }
         }
         __syncwarp();
     } else {
