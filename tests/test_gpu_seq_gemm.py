@@ -40,3 +40,21 @@ def test_few_rows(M, N, K):
     want = A.double() @ B.double().T
     assert (product(A, B, 5).double() - want).abs().max() < 5e-6 * (1 + want.abs().max())
     assert (product(A, B, 5, c_f32=False).double() - want).abs().max() < 2.0 ** -8 * (1 + want.abs().max())
+
+
+def test_the_row_limit_of_the_tcgen05_form_holds_below_17(tmp_path):
+    """WF_SEQ_TC_MIN = 9: products of 9 to 16 rows are the tcgen05 form's, bit for bit; by default the few-row form's."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+    here = Path(__file__).resolve().parent
+    code = ("import torch, test_gpu_seq_gemm as t\n"
+            "for m, n, k in ((9, 300, 1000), (16, 2560, 2560)):\n"
+            "    A, B = t.operands(m, n, k)\n"
+            "    print(int(torch.equal(t.product(A, B, 0), t.product(A, B, 3))), int(torch.equal(t.product(A, B, 0), t.product(A, B, 5))))\n")
+    for limit, want in (("9", "1 0"), ("17", "0 1")):
+        env = dict(os.environ, WF_SEQ_TC_MIN=limit, PYTHONPATH=f"{here}:{here.parent / 'wrinklefree-inference-engine_b200'}")
+        r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stderr[-2000:]
+        assert r.stdout.split("\n")[:2] == [want, want], r.stdout

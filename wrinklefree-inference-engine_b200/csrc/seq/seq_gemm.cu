@@ -435,7 +435,9 @@ int launch_gemm(int dt, const GemmArgs& g, cudaStream_t s) {
     if (g_tc_min < 0) { const char* e = getenv("WF_SEQ_TC_MIN"); g_tc_min = e ? atoi(e) : 17; }
     if (g_force_simt < 0) { const char* e = getenv("WF_SEQ_GEMM_SIMT"); g_force_simt = (e && atoi(e)) ? 1 : 0; }
     const bool few = g.batch == 1 && !g.tile_group && !g.a_rows && g.M <= 8;
-    if (g.batch == 1 && !g.tile_group && !g.a_rows && g.M <= 16 && dt == WF_BF16 && !g.a_f32 && !g_force_simt && (g.algo == 0 || g.algo == 5) && gemv_ok<__nv_bfloat16>(g)) {
+    // (9 to 16 rows go to the tcgen05 form where WF_SEQ_TC_MIN asks for it)
+    const bool few_mma = g.algo == 5 || (g.algo == 0 && !g_force_simt && (g.M <= 8 || g.M < g_tc_min || !gemm_tc_usable(g)));
+    if (few_mma && g.batch == 1 && !g.tile_group && !g.a_rows && g.M <= 16 && dt == WF_BF16 && !g.a_f32 && gemv_ok<__nv_bfloat16>(g)) {
         if (g.M <= 8) few_dispatch<1>(g, s); else few_dispatch<2>(g, s);
         return launch_check(cudaGetLastError(), "gemm_few");
     }
