@@ -1,4 +1,4 @@
-"""The 16-token form of the matrix-state recurrences against the oracles, in float32: every length around its chunks, long portions in parallel segments,
+"""The 16-token form of the matrix-state recurrences against the oracles, in float32, where it has to be asked for: every length around its chunks, long portions in parallel segments,
 portions behind carried states, several sequences side by side, key sizes that do not fill a thread's rows, value sizes that do not fill a block.
 
 Tolerance: float32 sums over at most a few hundred terms of order one in another order, relative to a row's RMS; the delta rule's correction solves
@@ -11,6 +11,13 @@ import fivedra_oracle as FO
 import nukezen_oracle as NO
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def sixteen_token_form(monkeypatch):
+    monkeypatch.setenv("WF_SEQ_CHUNK", "1")        # float32 engines keep the token form by themselves
+
+
 CUTS = [([70], [[70]]), ([33, 100], [[33, 100]]), ([90, 64], [[32, 0], [15, 47], [43, 16], [0, 1]]), ([47], [[47]]), ([545, 140], [[21, 0], [524, 140]])]
 EPS = 1e-5
 
@@ -120,3 +127,23 @@ def test_numbers_that_are_not_finite(kind, at, bad):
         x, y = whole[:at], pieces[:at]
         err = np.sqrt(((x - y) ** 2).mean(-1)) / np.sqrt((y ** 2).mean(-1))
         assert err.max() < 2e-2          # two bf16 roundings of the same float values, and the products around them
+
+
+def test_float32_engines_keep_the_token_form(monkeypatch):
+    """By default a float32 engine gives the bits of plain multiply-adds token by token, a bf16 engine those of the 16-token form."""
+    from wf_bitnet import registry
+    cfg, weights, shapes, W = nonfinite_layer("delta")
+    rows = np.random.default_rng(1).standard_normal((200, W)).astype(np.float32)
+
+    def run(dtype, form):
+        monkeypatch.delenv("WF_SEQ_CHUNK") if form is None else monkeypatch.setenv("WF_SEQ_CHUNK", form)
+        cls = registry.resolve(cfg)
+        extra = {"shapes": shapes} if getattr(cls, "reads_shapes", False) else {}
+        m = cls(cfg, dtype=dtype, max_tokens=400, slots=2, page_size=16, max_step_tokens=256, **extra)
+        m.load_weights((k, v.numpy(), "F32") for k, v in weights.items())
+        out = m.engine.run_part(0, 2, [m.admit()], [200], rows)
+        m.close()
+        monkeypatch.setenv("WF_SEQ_CHUNK", "1")
+        return out
+    assert np.array_equal(run("float32", None), run("float32", "0")) and not np.array_equal(run("float32", "0"), run("float32", "1"))
+    assert np.array_equal(run("bfloat16", None), run("bfloat16", "1"))

@@ -125,6 +125,7 @@ struct wf_seq_engine {
     int P = 0;                        // padded expert-row bound
     int fuse_input = 1;               // norm + input convolution (+ state roll of single-token sequences) in one kernel (WF_SEQ_FUSE_INPUT=0: three kernels)
     int attn_mma = 3;                 // attention on tensor cores where the sizes allow it: 3 prompt portions on tcgen05; below that 2 latent attention with keys as rows first, 1 heads as rows only, 0 plain kernels (WF_SEQ_ATTN_MMA)
+    int chunk_rec = 0;                // matrix-state recurrences of prompt portions 16 tokens at a time on the matrix units: set in bf16 engines (WF_SEQ_CHUNK: 0 never, 1 always)
     // latent attention of prompt portions: the cached rows of the step's sequences gathered, and the keys and values of every head made from them
     void *lat_rows = nullptr, *kvx = nullptr;
     int kvx_rows = 0;
@@ -1124,6 +1125,9 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     if (const char* am = getenv("WF_SEQ_ATTN_MMA")) e->attn_mma = atoi(am);
     if (const char* gm = getenv("WF_SEQ_GRAPH_MAX")) e->graph_max = atoi(gm);
     if (const char* aw = getenv("WF_SEQ_ATTN_WAVES")) e->attn_waves = atoi(aw) > 0 ? atoi(aw) : 1;
+    // float32 engines keep to plain multiply-adds: the 16-token form's products are sums of tf32 pairs
+    const char* cr = getenv("WF_SEQ_CHUNK");
+    e->chunk_rec = cr ? atoi(cr) : e->dt == WF_BF16;
     if (const char* fi = getenv("WF_SEQ_FUSE_INPUT")) e->fuse_input = atoi(fi);
     const wf_seq_config& c = e->cfg;
     const int W = c.width, T = c.max_step_tokens, taps = c.canon_taps;
@@ -1507,7 +1511,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
         TRY(dalloc_n(e, &e->scan.local, (size_t)e->scan.chunks * max_scan)); TRY(dalloc_n(e, &e->scan.start, (size_t)e->scan.chunks * max_scan));
         TRY(dalloc_n(e, &e->scan.prod, (size_t)e->scan.chunks * std::max(max_H, max_decay)));
     }
-    if (max_rec && T >= 2 * CHUNK_TOKENS) {
+    if (e->chunk_rec && max_rec && T >= 2 * CHUNK_TOKENS) {
         TRY(dalloc_n(e, &e->scan.rec, max_rec));
         e->scan.rec_floats = max_rec;
     }
