@@ -134,3 +134,23 @@ def test_rows_that_do_not_see_a_value_stay_finite(kind, bad):
     assert np.isfinite(got[:at]).all() and not np.isfinite(got[at:]).all(-1).any()
     err = np.sqrt(((got[:at] - ref[:at]) ** 2).mean(-1)) / np.sqrt((ref[:at] ** 2).mean(-1))
     assert err.max() < TOL
+
+
+def latent_groups(model, behind, count):
+    """The launch groups of a step of `count` tokens behind `behind` cached positions."""
+    s = model.admit()
+    model.engine.set_length(s, behind)
+    out = set(model.engine.profile_step([s], [count], 1))
+    model.release(s)
+    return out
+
+
+def test_the_latent_choice_counts_the_keys_under_the_window():
+    """A short portion behind a long context expands the latents where it sees all of them and reads them as they are where a window hides most."""
+    import test_gpu_karusun as K
+    for window, expands in ((100000, True), (512, False)):
+        cfg = K.config([K.lat(heads=20, dim=96, rot_dim=32, vdim=128, kv_rank=512, window=window)], width=64, vocab=40, groups=1, taps=2)
+        model = K.build(cfg, K.make_weights(cfg, 3), "bfloat16", max_tokens=4096, page_size=16, max_step_tokens=1024)
+        assert ("latent.expand_gemm" in latent_groups(model, 3000, 64)) == expands
+        assert "latent.expand_gemm" in latent_groups(model, 0, 1000)
+        model.close()

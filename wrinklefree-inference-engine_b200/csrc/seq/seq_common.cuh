@@ -28,7 +28,6 @@ struct Batch {
     const int32_t* key_row = nullptr;   // [nseq] first row of the sequence where all its positions so far lie one sequence after another
     int max_ctx = 0;           // most positions that a sequence holds behind the step (known on the host)
     int ctx_total = 0;         // those rows: the sum over sequences of the positions behind the step (known on the host)
-    double pairs = 0.;         // (query, earlier or own key) pairs of the step, windows aside (known on the host)
 };
 
 __device__ __forceinline__ float warp_sum(float v) {

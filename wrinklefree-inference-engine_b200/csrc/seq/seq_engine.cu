@@ -370,13 +370,11 @@ int prepare_step(wf_seq_engine* e, int nseq, const int32_t* slots, const int32_t
     for (int j = 0; j < nwant; ++j) m_want[j] = want[j];
     int32_t* m_key = m + 4 * T + 4 * S;
     long long ctx = 0;
-    v->b.pairs = 0.;
     v->b.max_ctx = 0;
     for (int i = 0; i < nseq; ++i) {
         m_key[i] = (int32_t)ctx;
         v->b.max_ctx = std::max(v->b.max_ctx, (int)(m_pos0[i] + counts[i]));
         ctx += m_pos0[i] + counts[i];
-        v->b.pairs += (double)counts[i] * (m_pos0[i] + 0.5 * (counts[i] + 1));
     }
     v->b.ctx_total = (int)ctx;                      // at most the pool's tokens
     if (cuda_check(cudaMemcpyAsync(e->d_meta, m, e->meta_ints * 4, cudaMemcpyHostToDevice, e->stream), "step metadata H2D")) return WF_ERR_CUDA;
@@ -424,6 +422,17 @@ int in_proj(wf_seq_engine* e, const LayerState& L, const Batch& b, const float**
     return launch_gemm(e->dt, lin(e->h_t, 0, W, L.wp, W, e->proj, 1, L.np, b.n, L.np, W), e->stream);
 }
 
+// (query, key) pairs of the step whose arrays prepare_step left in h_meta, under a window
+double visible_pairs(const wf_seq_engine* e, int nseq, int window) {
+    const size_t T = e->cfg.max_step_tokens, S = e->cfg.slots;
+    const int32_t *len = e->h_meta + 3 * T + S, *pos0 = len + S;
+    const double w = window;
+    auto up_to = [w](double x) { return x <= w ? 0.5 * x * (x + 1.) : 0.5 * w * (w + 1.) + (x - w) * w; };      // of positions 0 .. x - 1
+    double sum = 0.;
+    for (int i = 0; i < nseq; ++i) sum += up_to((double)pos0[i] + len[i]) - up_to(pos0[i]);
+    return sum;
+}
+
 // h (post-convolution input, storage type [n, W]) -> y float [n, W]
 int run_latent(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
     const wf_seq_layer& c = L.c;
@@ -446,8 +455,9 @@ int run_latent(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
     // Prompt portions: every position's latent expanded to the heads' keys and values once, then attention with per-head keys (tcgen05).  Per (query, key)
     // pair and head that is 2 (d + r + 2 dv) operations instead of 2 (2 R + r) on mma.sync (measured about 3e14 against 1e14 a second), at the price
     // of the expansion of all positions so far, 2 (R + r) (d + r + dv) operations each at about 6e14, and of three launches.
-    const double us_absorbed = b.pairs * H * 2. * (2 * c.kv_rank + c.rot_dim) * 1e-8;
-    const double us_expanded = 30. + b.pairs * H * 2. * (per + 2 * c.vdim) / 3e8 + (double)b.ctx_total * H * 2. * nkv * (per + c.vdim) / 6e8;
+    const double pairs = visible_pairs(e, b.nseq, c.window);
+    const double us_absorbed = pairs * H * 2. * (2 * c.kv_rank + c.rot_dim) * 1e-8;
+    const double us_expanded = 30. + pairs * H * 2. * (per + 2 * c.vdim) / 3e8 + (double)b.ctx_total * H * 2. * nkv * (per + c.vdim) / 6e8;
     if (e->attn_mma >= 3 && L.kvx && n > b.nseq && b.ctx_total <= e->kvx_rows && L.cache_off % 8 == 0 && e->page_stride % 8 == 0 && us_expanded < us_absorbed) {
         if ((rc = launch_latent_q_prep(e->dt, b, D, qsrc, ldq, e->qn, nullptr, s))) return rc;
         if ((rc = launch_latent_kv_write(e->dt, b, D, e->proj + L.kv_col, L.np, L.dkv_norm, e->cfg.eps, pc, s))) return rc;
