@@ -90,7 +90,8 @@ def test_window_rotation_and_element_gates(window, cut):
 
 @pytest.mark.parametrize("heads,dim,rot,vdim,rank", [(20, 96, 32, 128, 512), (8, 64, 32, 64, 256), (3, 40, 8, 24, 64)])
 def test_latent_with_expanded_keys(heads, dim, rot, vdim, rank):
-    """Portions long enough that the latents are expanded, then one behind cached latents, and a step that mixes a long portion with a single token."""
+    """Portions of which the long ones are expanded at the largest sizes (the cost rule keeps the others on the form that reads the latents), then one behind
+    cached latents, and a step that mixes a long portion with a single token."""
     W = 64
     m = {"heads": heads, "dim": dim, "rot_dim": rot, "vdim": vdim, "kv_rank": rank, "q_rank": 48, "scale": (dim + rot) ** -0.5,
          "rot": {"dims": rot, "base": 10000.0, "scaling": {"factor": 4.0, "original": 256, "fast": 32.0, "slow": 1.0}}}
@@ -154,3 +155,23 @@ def test_the_latent_choice_counts_the_keys_under_the_window():
         assert ("latent.expand_gemm" in latent_groups(model, 3000, 64)) == expands
         assert "latent.expand_gemm" in latent_groups(model, 0, 1000)
         model.close()
+
+
+@pytest.mark.parametrize("heads,dim,rot,vdim,rank", [(8, 64, 32, 64, 256), (3, 40, 8, 24, 64), (5, 24, 0, 128, 80), (7, 120, 8, 8, 32)])
+def test_latent_form_with_expanded_keys_at_small_sizes(heads, dim, rot, vdim, rank, monkeypatch):
+    """The same where its cost rule would decide otherwise: odd head counts, heads below a swizzle block, sequences whose rows start between tiles."""
+    monkeypatch.setenv("WF_SEQ_ATTN_MMA", "4")
+    W = 64
+    m = {"heads": heads, "dim": dim, "rot_dim": rot, "vdim": vdim, "kv_rank": rank, "q_rank": 48, "scale": (dim + rot) ** -0.5,
+         "rot": {"dims": rot, "base": 10000.0, "scaling": {"factor": 4.0, "original": 256, "fast": 32.0, "slow": 1.0}}}
+    cfg = {"architecture": "Fivedra", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5},
+           "layers": [{"type": "latent_attention", "mixer": m, "mlp": None}]}
+    w = FO.random_weights(cfg, heads)
+    lens = [333, 70, 190]
+    rows = inputs(lens, W, 7)
+    P = d64(w, "l0.mix.")
+    wants = [FO.latent_attention(torch.from_numpy(r).double(), P, "", m, 1e-5).numpy() for r in rows]
+    model = build(cfg, w, 16, {})
+    assert "latent.expand_gemm" in latent_groups(model, 0, 40)
+    check(model, rows, [[200, 3, 129], [5, 66, 0], [128, 1, 61]], wants, W)
+    model.close()

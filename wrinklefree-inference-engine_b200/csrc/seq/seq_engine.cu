@@ -124,7 +124,7 @@ struct wf_seq_engine {
     int32_t *ids = nullptr, *counts = nullptr, *plan_scratch = nullptr, *sorted_rows = nullptr, *pair_row = nullptr, *tile_group = nullptr;
     int P = 0;                        // padded expert-row bound
     int fuse_input = 1;               // norm + input convolution (+ state roll of single-token sequences) in one kernel (WF_SEQ_FUSE_INPUT=0: three kernels)
-    int attn_mma = 3;                 // attention on tensor cores where the sizes allow it: 3 prompt portions on tcgen05; below that 2 latent attention with keys as rows first, 1 heads as rows only, 0 plain kernels (WF_SEQ_ATTN_MMA)
+    int attn_mma = 3;                 // attention on tensor cores where the sizes allow it: 3 prompt portions on tcgen05 where that is the faster form (4: wherever it takes the sizes); below that 2 latent attention with keys as rows first, 1 heads as rows only, 0 plain kernels (WF_SEQ_ATTN_MMA)
     int chunk_rec = 0;                // matrix-state recurrences of prompt portions 16 tokens at a time on the matrix units: set in bf16 engines (WF_SEQ_CHUNK: 0 never, 1 always)
     // latent attention of prompt portions: the cached rows of the step's sequences gathered, and the keys and values of every head made from them
     void *lat_rows = nullptr, *kvx = nullptr;
@@ -458,7 +458,7 @@ int run_latent(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
     const double pairs = visible_pairs(e, b.nseq, c.window);
     const double us_absorbed = pairs * H * 2. * (2 * c.kv_rank + c.rot_dim) * 1e-8;
     const double us_expanded = 30. + pairs * H * 2. * (per + 2 * c.vdim) / 3e8 + (double)b.ctx_total * H * 2. * nkv * (per + c.vdim) / 6e8;
-    if (e->attn_mma >= 3 && L.kvx && n > b.nseq && b.ctx_total <= e->kvx_rows && L.cache_off % 8 == 0 && e->page_stride % 8 == 0 && us_expanded < us_absorbed) {
+    if (e->attn_mma >= 3 && L.kvx && n > b.nseq && b.ctx_total <= e->kvx_rows && L.cache_off % 8 == 0 && e->page_stride % 8 == 0 && (e->attn_mma >= 4 || us_expanded < us_absorbed)) {
         if ((rc = launch_latent_q_prep(e->dt, b, D, qsrc, ldq, e->qn, nullptr, s))) return rc;
         if ((rc = launch_latent_kv_write(e->dt, b, D, e->proj + L.kv_col, L.np, L.dkv_norm, e->cfg.eps, pc, s))) return rc;
         mark(e, "latent.q_prep+kv_write");
@@ -625,7 +625,7 @@ int run_gqa(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
             if (splits < 1) splits = 1;
         }
         if ((rc = launch_talk_attn_mma(b, D, e->qn, pc, e->og, e->gqa_ws, splits, s))) return rc;
-    } else if (e->dt == WF_BF16 && e->attn_mma >= 3 && n > b.nseq && std::min(c.window, b.max_ctx) > 256 && attn_tc_usable(D, pc)) {
+    } else if (e->dt == WF_BF16 && e->attn_mma >= 3 && n > b.nseq && (e->attn_mma >= 4 || std::min(c.window, b.max_ctx) > 256) && attn_tc_usable(D, pc)) {
         // up to two of its key tiles the tcgen05 form has nothing to overlap, and the mma.sync form's smaller CTAs start sooner: steps of 64 / 256 tokens at
         // position 0 took 10 / 5 us longer with it; 3 x 300 tokens were equal, 512 tokens 3 us shorter, 256 tokens behind 3000 72 us shorter (20 heads of 128)
         if ((rc = launch_attn_tc(b, D, e->qn, gate, pc, e->cfg.max_pages, e->og, s))) return rc;
