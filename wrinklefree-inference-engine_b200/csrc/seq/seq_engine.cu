@@ -1268,7 +1268,9 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             {
                 const int per = l.dim + l.rot_dim;
                 const GqaDims X{l.heads, l.heads, per, l.vdim, l.scale, 0.f, l.window, 0, 0};
-                if (e->dt == WF_BF16 && e->attn_mma >= 3 && attn_tc_dense_usable(X) && nkv % 8 == 0) {
+                // (the sizes that no mma.sync form takes keep the plain kernel, whose queries and weights stay in float)
+                const LatentDims Y{l.heads, l.dim, l.rot_dim, l.vdim, l.kv_rank, l.scale, l.rope_base, l.rope_dims, l.window};
+                if (e->dt == WF_BF16 && e->attn_mma >= 3 && attn_tc_dense_usable(X) && nkv % 8 == 0 && (latent_attn_kt_usable(Y) || latent_attn_mma_usable(Y))) {
                     TRYL(walloc(&L.kvx, (size_t)l.heads * (per + l.vdim) * nkv));
                     max_kvx = std::max(max_kvx, (size_t)l.heads * (per + l.vdim)); max_lat = std::max(max_lat, (size_t)nkv);
                 }
