@@ -329,6 +329,15 @@ struct StepView {
     const int32_t* want;
 };
 
+// after a step's synchronisation: whether a bounded wait of the tcgen05 kernels ran out, and where
+int check_waits(wf_seq_engine* e, const char* who) {
+    const int code = e->dt == WF_BF16 ? gemm_tc_error(e->stream) : 0;
+    if (!code) return WF_OK;
+    if (code < 0) set_error("%s: the tcgen05 kernels' error word cannot be read", who);
+    else set_error("%s: a bounded wait of the tcgen05 %s ran out (%d)", who, code <= 3 ? "matrix product" : "attention", code);
+    return WF_ERR_CUDA;
+}
+
 // host bookkeeping + one H2D copy of a step's index arrays
 int prepare_step(wf_seq_engine* e, int nseq, const int32_t* slots, const int32_t* counts, const int32_t* tokens, int nwant, const int32_t* want,
                  StepView* v) {
@@ -1719,7 +1728,7 @@ extern "C" int wf_seq_step(wf_seq_engine* e, int nseq, const int32_t* slots, con
     if (logits_host && nwant > 0)
         if (cuda_check(cudaMemcpyAsync(logits_host, e->logits, (size_t)nwant * e->cfg.vocab * 4, cudaMemcpyDeviceToHost, e->stream), "logits D2H")) return WF_ERR_CUDA;
     if (cuda_check(cudaStreamSynchronize(e->stream), "wf_seq_step")) return WF_ERR_CUDA;
-    if (e->dt == WF_BF16 && gemm_tc_error(e->stream)) { set_error("wf_seq_step: a bounded wait of the tensor-core matrix product ran out"); return WF_ERR_CUDA; }
+    if ((rc = check_waits(e, "wf_seq_step"))) return rc;
     commit_lengths(e, nseq, slots, counts);
     return WF_OK;
 }
@@ -1803,6 +1812,7 @@ extern "C" int wf_seq_run_part(wf_seq_engine* e, int layer, int part, int nseq, 
     if (rc) return rc;
     if (cuda_check(cudaMemcpyAsync(out_host, result, bytes, cudaMemcpyDeviceToHost, s), "out")) return WF_ERR_CUDA;
     if (cuda_check(cudaStreamSynchronize(s), "wf_seq_run_part")) return WF_ERR_CUDA;
+    if ((rc = check_waits(e, "wf_seq_run_part"))) return rc;
     commit_lengths(e, nseq, slots, counts);
     return WF_OK;
 }
@@ -1878,6 +1888,7 @@ extern "C" int wf_seq_time_step(wf_seq_engine* e, int nseq, const int32_t* slots
     for (int i = 0; i < nseq; ++i) e->pt.truncate(slots[i], e->h_len[slots[i]]);   // the timed tokens are not kept
     if (rc) return rc;
     if (cuda_check(ce, "wf_seq_time_step")) return WF_ERR_CUDA;
+    if ((rc = check_waits(e, "wf_seq_time_step"))) return rc;
     *ms_out = ms / iters;
     return WF_OK;
 }
