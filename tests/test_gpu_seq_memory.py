@@ -1,0 +1,46 @@
+"""An engine on a device that is nearly full: what only the faster prompt forms need is left out, and the rest works as without them."""
+import numpy as np
+import pytest
+import torch
+
+import fivedra_oracle as FO
+
+pytestmark = pytest.mark.gpu
+
+
+def test_the_workspaces_of_the_faster_forms_are_not_required(monkeypatch):
+    from wf_bitnet import registry
+    W = 64
+    m = {"heads": 20, "dim": 96, "rot_dim": 32, "vdim": 128, "kv_rank": 512, "q_rank": 48, "scale": 128 ** -0.5,
+         "rot": {"dims": 32, "base": 10000.0, "scaling": {"factor": 4.0, "original": 256, "fast": 32.0, "slow": 1.0}}}
+    cfg = {"architecture": "Fivedra", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5},
+           "layers": [{"type": "latent_attention", "mixer": m, "mlp": None}]}
+    weights = FO.random_weights(cfg, 1)
+    rows = np.random.default_rng(2).standard_normal((900, W)).astype(np.float32)
+
+    def build():
+        cls = registry.resolve(cfg)
+        extra = {"shapes": {}} if getattr(cls, "reads_shapes", False) else {}
+        e = cls(cfg, dtype="bfloat16", max_tokens=32768, slots=2, page_size=16, max_step_tokens=8192, **extra)
+        e.load_weights((k, v.numpy(), "F32") for k, v in weights.items())
+        return e
+
+    def run(e):
+        out = e.engine.run_part(0, 2, [e.admit()], [900], rows)
+        size = e.engine.device_bytes()
+        e.close()
+        return out, size
+    monkeypatch.setenv("WF_SEQ_ATTN_MMA", "2")
+    plain, small = run(build())
+    monkeypatch.delenv("WF_SEQ_ATTN_MMA")
+    _, full = run(build())
+    assert full > small + (200 << 20)
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    held = torch.empty(free - small - (128 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        tight, size = run(build())
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert size == small and np.array_equal(tight, plain)

@@ -35,6 +35,7 @@ struct LayerState {
     void* wo = nullptr;       // [W, heads * vdim]
     // latent attention
     void *dkv_norm = nullptr, *uk = nullptr, *ukT = nullptr, *uv = nullptr;
+    int kvx_src = -1;         // the layer run whose kvx this one uses (its own, or its tie's)
     void* kvx = nullptr;      // [keys | values of every head] from a cached row: launch_latent_expand_weight (prompt portions; null: sizes that form does not take)
     long long cache_off = 0;  // element offset of this layer inside a cache page
     // delta
@@ -172,6 +173,18 @@ template <typename P>
 int dalloc_t(wf_seq_engine* e, P** p, size_t count) { return dalloc_bytes(e, (void**)p, count * e->esz); }   // storage-type elements
 template <typename P>
 int dalloc_n(wf_seq_engine* e, P** p, size_t count) { return dalloc_bytes(e, (void**)p, count * sizeof(P)); }
+
+// for a workspace that the engine can do without: at most a quarter of what the device has left, and no error where there is none
+bool dalloc_spare(wf_seq_engine* e, void** p, size_t bytes) {
+    size_t left = 0, all = 0;
+    void* q = nullptr;
+    bytes = (bytes + 255) / 256 * 256;
+    if (cudaMemGetInfo(&left, &all) != cudaSuccess || bytes > left / 4 || cudaMalloc(&q, bytes) != cudaSuccess) { cudaGetLastError(); return false; }
+    e->allocs.push_back(q);
+    e->dev_bytes += bytes;
+    *p = q;
+    return true;
+}
 
 void add_tensor(wf_seq_engine* e, const std::string& name, void* dst, size_t count) {
     TensorSlot t;
@@ -1280,7 +1293,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
                 // (the sizes that no mma.sync form takes keep the plain kernel, whose queries and weights stay in float)
                 const LatentDims Y{l.heads, l.dim, l.rot_dim, l.vdim, l.kv_rank, l.scale, l.rope_base, l.rope_dims, l.window};
                 if (e->dt == WF_BF16 && e->attn_mma >= 3 && attn_tc_dense_usable(X) && nkv % 8 == 0 && (latent_attn_kt_usable(Y) || latent_attn_mma_usable(Y))) {
-                    TRYL(walloc(&L.kvx, (size_t)l.heads * (per + l.vdim) * nkv));
+                    if (own) L.kvx_src = (int)(&L - e->layers.data());
                     max_kvx = std::max(max_kvx, (size_t)l.heads * (per + l.vdim)); max_lat = std::max(max_lat, (size_t)nkv);
                 }
             }
@@ -1518,10 +1531,6 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     TRY(dalloc_t(e, &e->olat, (size_t)T * max_hr)); TRY(dalloc_n(e, &e->ov, (size_t)T * max_hv)); TRY(dalloc_t(e, &e->og, (size_t)T * max_hv));
     e->attn_ws_rows = 4 * 148;
     if (e->dt == WF_BF16 && max_hr > 1) TRY(dalloc_bytes(e, (void**)&e->attn_ws, (size_t)e->attn_ws_rows * (max_hr + 2 * max_H) * sizeof(float)));
-    if (max_kvx) {                             // enough positions for sequences of several full steps; longer ones keep the form that reads the latents
-        e->kvx_rows = (int)std::min<long long>((long long)c.max_pages * c.page_size, 4LL * T);
-        TRY(dalloc_t(e, &e->lat_rows, (size_t)e->kvx_rows * max_lat)); TRY(dalloc_t(e, &e->kvx, (size_t)e->kvx_rows * max_kvx));
-    }
     TRY(dalloc_n(e, &e->gate, (size_t)T * std::max(max_H, max_gate)));
     if (c.n_extra > 0) TRY(dalloc_n(e, &e->y2, (size_t)T * W));
     if (parallel) TRY(dalloc_t(e, &e->h_t2, (size_t)T * W));
@@ -1531,10 +1540,6 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
         e->scan.chunks = scan_chunks_needed(T, c.slots);
         TRY(dalloc_n(e, &e->scan.local, (size_t)e->scan.chunks * max_scan)); TRY(dalloc_n(e, &e->scan.start, (size_t)e->scan.chunks * max_scan));
         TRY(dalloc_n(e, &e->scan.prod, (size_t)e->scan.chunks * std::max(max_H, max_decay)));
-    }
-    if (e->chunk_rec && max_rec && T >= 2 * CHUNK_TOKENS) {
-        TRY(dalloc_n(e, &e->scan.rec, max_rec));
-        e->scan.rec_floats = max_rec;
     }
     if (max_gfull) TRY(dalloc_n(e, &e->gfull, (size_t)T * max_gfull));
     if (max_afull) TRY(dalloc_n(e, &e->afull, (size_t)T * max_afull));
@@ -1553,6 +1558,26 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     TRY(dalloc_t(e, &e->hperm, P * W));
     TRY(dalloc_n(e, &e->gu, P * 2 * max_ff)); TRY(dalloc_t(e, &e->hmid, P * max_ff)); TRY(dalloc_n(e, &e->yexp, P * W));
 #undef TRY
+    // What only the faster forms of prompt portions need comes last, each form's part as a whole, and only where that leaves three quarters of what is free
+    // by then: an engine that fits without them still fits, and takes the forms that need none.
+    if (e->chunk_rec && max_rec && T >= 2 * CHUNK_TOKENS && dalloc_spare(e, (void**)&e->scan.rec, max_rec * sizeof(float))) e->scan.rec_floats = max_rec;
+    if (max_kvx) {                             // enough positions for sequences of several full steps; longer ones keep the form that reads the latents
+        const size_t rows = (size_t)std::min<long long>((long long)c.max_pages * c.page_size, 4LL * T);
+        auto place = [](size_t& off, size_t elems) { const size_t at_ = off; off += (elems + 127) / 128 * 128; return at_; };        // 256-byte aligned
+        size_t elems = 0;
+        const size_t at_lat = place(elems, rows * max_lat), at_kvx = place(elems, rows * max_kvx);
+        std::vector<size_t> at_w(e->layers.size());
+        for (size_t i = 0; i < e->layers.size(); ++i) {
+            const wf_seq_layer& l = e->layers[i].c;
+            if (e->layers[i].kvx_src == (int)i) at_w[i] = place(elems, (size_t)l.heads * (l.dim + l.rot_dim + l.vdim) * (l.kv_rank + l.rot_dim));
+        }
+        void* base = nullptr;
+        if (dalloc_spare(e, &base, elems * e->esz)) {
+            e->kvx_rows = (int)rows;
+            e->lat_rows = at(e, base, at_lat); e->kvx = at(e, base, at_kvx);
+            for (LayerState& L : e->layers) if (L.kvx_src >= 0) L.kvx = at(e, base, at_w[L.kvx_src]);
+        }
+    }
     if (cuda_check(cudaMemsetAsync(e->state, 0, e->slot_stride * c.slots * 4, e->stream), "state")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
     if (cuda_check(cudaMemsetAsync(e->pool, 0, (size_t)std::max<long long>(cache_elems, 1) * c.max_pages * e->esz, e->stream), "pool")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
     if (cuda_check(cudaStreamSynchronize(e->stream), "sync")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
