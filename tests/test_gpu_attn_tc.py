@@ -180,7 +180,7 @@ def test_latent_form_with_expanded_keys_at_small_sizes(heads, dim, rot, vdim, ra
 def test_latent_sizes_without_a_tensor_core_form_keep_the_plain_kernel(monkeypatch):
     """Ranks that no mma.sync form takes had float queries and weights: asked for or not, they are not expanded."""
     monkeypatch.setenv("WF_SEQ_ATTN_MMA", "4")
-    m = {"heads": 20, "dim": 96, "rot_dim": 32, "vdim": 128, "kv_rank": 520, "q_rank": 48, "scale": 128 ** -0.5, "rot": {"dims": 32, "base": 10000.0}}
+    m = {"heads": 20, "dim": 96, "rot_dim": 32, "vdim": 128, "kv_rank": 504, "q_rank": 48, "scale": 128 ** -0.5, "rot": {"dims": 32, "base": 10000.0}}
     cfg = {"architecture": "Fivedra", "vocab": 31, "width": 64, "embedding": {"scale": 1.0}, "norm": {"eps": 1e-5},
            "layers": [{"type": "latent_attention", "mixer": m, "mlp": None}]}
     model = build(cfg, FO.random_weights(cfg, 2), 16, {})
