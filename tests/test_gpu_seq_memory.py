@@ -37,7 +37,7 @@ def test_the_workspaces_of_the_faster_forms_are_not_required(monkeypatch):
     assert full > small + (200 << 20)
     torch.cuda.empty_cache()
     free = torch.cuda.mem_get_info()[0]
-    held = torch.empty(free - small - (128 << 20), dtype=torch.uint8, device="cuda")
+    held = torch.empty(free - small - (256 << 20), dtype=torch.uint8, device="cuda")
     try:
         tight, size = run(build())
     finally:
