@@ -10,10 +10,10 @@ A "step" is one decode step (one new token for every sequence of the batch) of t
 BitNet-2B-4T-shaped model: 30 layers x (rmsnorm+int8 quant, fused q|k|v ternary linear, RoPE + paged KV
 append, paged flash-decode attention, sub-norm+quant, o linear, rmsnorm+quant, fused gate|up linear with
 relu^2*up, sub-norm+quant, down linear) + final norm + tied bf16 LM head + greedy argmax.
-Default workload = BASELINE.json configs[1]: batch 64, every sequence holding 4096 tokens of paged KV.
+Default workload: batch 64, every sequence holding 4096 tokens of paged KV.
 Weights are random-init ternary (synthetic), KV contents random.
 
-N > 1: the 2B model has 5 KV heads and does not shard over 2/4/8 GPUs (SURVEY §8e) -> replicas only:
+N > 1: the 2B model has 5 KV heads and does not shard over 2/4/8 GPUs -> replicas only:
 every rank runs its own batch of 64 (weak scaling, no data-path collective).
 
 --impl reference: the reference's own CPU implementation of the same step (the unmodified AVX2 I2_S
@@ -53,18 +53,18 @@ def emit(obj) -> None:
 import numpy as np
 import torch
 
-# BitNet-2B-4T shape (SURVEY §8): hidden 2560, 30 layers, 20/5 heads x 128, ffn 6912, vocab 128256
+# BitNet-2B-4T shape: hidden 2560, 30 layers, 20/5 heads x 128, ffn 6912, vocab 128256
 SHAPE = dict(hidden=2560, layers=30, heads=20, kv_heads=5, head_dim=128, ffn=6912, vocab=128256)
-LAYER_WEIGHT_BYTES = 17_367_040          # packed ternary bytes per layer (SURVEY Appendix B)
+LAYER_WEIGHT_BYTES = 17_367_040          # packed ternary bytes per layer
 KV_BYTES_PER_TOKEN_LAYER = 2 * 5 * 128 * 2
 LM_HEAD_BYTES = 128256 * 2560 * 2
 METRIC = "decode tok/s, BitNet-2B-4T-shaped, batch 64, 4K paged KV, 1 B200 (replicas for N>1)"
 
-# tensor-parallel workloads: N GPUs = TP degree, strong scaling
+# tensor-parallel workloads (8B- and 70B-shaped): N GPUs = TP degree, strong scaling
 TP_WORKLOADS = {
-    "8b_bs1": dict(shape="llama3_8b", batch=1, ctx=512, name="BASELINE.json configs[3]: Llama-3-8B-shaped 1.58-bit model, random-init, batch=1 decode, 512-token context, TP = n_gpus"),
-    "8b_bs32": dict(shape="llama3_8b", batch=32, ctx=2048, name="BASELINE.json configs[3]: Llama-3-8B-shaped 1.58-bit model, random-init, batch=32 decode, 2K-token paged KV, TP = n_gpus"),
-    "70b_bs16": dict(shape="llama3_70b", batch=16, ctx=8192, name="BASELINE.json configs[4]: Llama-3-70B-shaped 1.58-bit model, random-init, batch=16 decode, 8K-token paged KV, TP = n_gpus"),
+    "8b_bs1": dict(shape="llama3_8b", batch=1, ctx=512, name="Llama-3-8B-shaped 1.58-bit model, random-init, batch=1 decode, 512-token context, TP = n_gpus"),
+    "8b_bs32": dict(shape="llama3_8b", batch=32, ctx=2048, name="Llama-3-8B-shaped 1.58-bit model, random-init, batch=32 decode, 2K-token paged KV, TP = n_gpus"),
+    "70b_bs16": dict(shape="llama3_70b", batch=16, ctx=8192, name="Llama-3-70B-shaped 1.58-bit model, random-init, batch=16 decode, 8K-token paged KV, TP = n_gpus"),
 }
 
 
@@ -266,7 +266,7 @@ def _tp_parity(rank, world, dist):
 
 
 def run_tp_suite(rank, world, dist, K, W, peak):
-    """BASELINE.json configs[3] / configs[4] in front of the driver: at N ranks, TP = N parity and timing of the
+    """The 8B- and 70B-shaped workloads: at N ranks, TP = N parity and timing of the
     8B bs1 / 8B bs32 / 70B bs16 workloads; rank 0 additionally times the TP = 1 engine and a single-GPU stand-in for one rank's
     shard (heads, KV heads, ffn and vocab divided by N: the rank's compute without the exchanges) on its own GPU, so every line
     carries speedup_vs_tp1 and the exchange cost measured on the same box in the same run."""
@@ -533,8 +533,8 @@ def run_reference(args):
 
 def workload_name(w):
     if w == "bs64":
-        return "BASELINE.json configs[1]: BitNet-2B-4T-shaped batched decode, batch=64, 4K-token paged KV cache, single B200"
-    return "BASELINE.json configs[0] shape on GPU: BitNet-2B-4T-shaped batch=1 decode at 512-token context"
+        return "BitNet-2B-4T-shaped batched decode, batch=64, 4K-token paged KV cache, single B200"
+    return "BitNet-2B-4T-shaped batch=1 decode at 512-token context"
 
 
 # ------------------------------------------------------------------------------------------- GPU arm
@@ -639,7 +639,7 @@ def run_gpu(args):
         breakdown["error"] = str(ex)
     eng.close()
 
-    # ---------------- batch-1 decode + GEMV roofline (the other half of BASELINE's metric), N = 1 only
+    # ---------------- batch-1 decode + GEMV roofline (the other half of the headline metric), N = 1 only
     aux = {}
     if args.workload == "bs64" and world == 1 and not args.no_aux:
         try:
@@ -700,7 +700,7 @@ def run_gpu(args):
         except Exception as ex:  # noqa: BLE001
             aux["int8_kv"] = {"error": str(ex)}
 
-    # ---------------- kernel-level GEMV bandwidth (the third part of BASELINE's metric): M = 1, > L2 worth of weight copies
+    # ---------------- kernel-level GEMV bandwidth (the third part of the headline metric): M = 1, > L2 worth of weight copies
     if world == 1 and not args.no_aux:
         try:
             import ctypes as C
@@ -723,17 +723,17 @@ def run_gpu(args):
     if world == 1 and not args.no_cpu:
         cpu_baseline, _ = cpu_baseline_block(batch, ctx, 2)
 
-    # ---------------- BASELINE configs[2]: prefill 8 x 2048 tokens through the tcgen05 int8 ternary GEMM (N = 1 only)
+    # ---------------- prefill 8 x 2048 tokens through the tcgen05 int8 ternary GEMM (N = 1 only)
     if args.workload == "bs64" and world == 1 and not args.no_aux:
         try:
             sys.path.insert(0, str(ROOT / "tools"))
             import bench_prefill
             aux["prefill"] = bench_prefill.measure(16384, 8, 3, "2b")
-            aux["prefill"]["workload"] = "BASELINE.json configs[2]: BitNet-2B-4T-shaped prefill, 8 x 2048-token prompts, the 4 fused ternary linears of a layer at M = 16384"
+            aux["prefill"]["workload"] = "BitNet-2B-4T-shaped prefill, 8 x 2048-token prompts, the 4 fused ternary linears of a layer at M = 16384"
         except Exception as ex:  # noqa: BLE001
             aux["prefill"] = {"error": str(ex)[:300]}
 
-    # ---------------- BASELINE configs[3] / [4]: tensor-parallel 8B / 70B-shaped decode at TP = N (every N, incl. the TP = 1 lines at N = 1)
+    # ---------------- tensor-parallel 8B / 70B-shaped decode at TP = N (every N, incl. the TP = 1 lines at N = 1)
     if args.workload == "bs64" and not args.no_aux and not args.no_tp:
         try:
             tp_aux = run_tp_suite(rank, world, dist, 20, 3, peak)

@@ -47,7 +47,7 @@ const char* wf_version(void);
 /* plain device-to-device copy on `stream` (debug taps of engine buffers) */
 int wf_copy_d2d(void* dst, const void* src, size_t bytes, void* stream);
 
-/* ---- weight formats (north-star item 1) ------------------------------ */
+/* ---- weight formats ------------------------------ */
 
 /* _pack_ternary_weights (src/wrinklefree_inference/cache/bitnet_converter.py:26-77;
  * == quantize_i2_s, extern/BitNet/src/ggml-bitnet-mad.cpp:46-92): fp32 [N,K] ternary-ish ->
@@ -63,7 +63,7 @@ int wf_hf_to_i2s(const uint8_t* hf, int N4, int K, uint8_t* i2s, void* stream);
 
 /* GPU tile layout "b200_tile_v1": [ceil(N/16)][K/128][512 B]; one 512-B tile = 16 rows x 128 k,
  * lane l of a warp owns bytes [16l,16l+16) = the four u32 A-fragment source words of
- * mma.m16n8k32 (see DESIGN.md).  Rows N..ceil16(N) are filled with code 1 (weight 0).
+ * mma.m16n8k32.  Rows N..ceil16(N) are filled with code 1 (weight 0).
  * K % 128 == 0. */
 size_t wf_tile_bytes(int N, int K);
 int wf_repack_i2s_to_tile(const uint8_t* i2s, int N, int K, uint8_t* tile, void* stream);
@@ -72,7 +72,7 @@ int wf_repack_tile_to_i2s(const uint8_t* tile, int N, int K, uint8_t* i2s, void*
  * (out rows 32i..32i+15 = a rows 16i.., out rows 32i+16..32i+31 = b rows 16i..). N % 16 == 0. */
 int wf_interleave_rows16(const uint8_t* a, const uint8_t* b, int N, int K4, uint8_t* out, void* stream);
 
-/* ---- activation quantisation (north-star item 2) -------------------------- */
+/* ---- activation quantisation -------------------------- */
 
 /* sgl_kernel.quantization.bitnet_quantize_activations / torch.ops.sgl_kernel.
  * bitnet_quantize_activations_cpu (docs/research/sglang_optimization_plan.md:72-74; arithmetic:
@@ -84,7 +84,7 @@ int wf_interleave_rows16(const uint8_t* a, const uint8_t* b, int N, int K4, uint
 int wf_act_quant_i8(const void* x, int x_dtype, int M, int K, int ldx, int per_token, int8_t* q, float* scale_out,
                     int32_t* rowsum_out, void* workspace, void* stream);
 
-/* ---- ternary linear (north-star items 3, 4) ---------------------------- */
+/* ---- ternary linear ---------------------------- */
 
 /* weight layouts */
 #define WF_W_I2S 0  /* reference layout u8 [N,K/4] (what sgl_kernel ops receive) */
@@ -155,7 +155,7 @@ size_t wf_static_workspace_max_bytes(void);
 int wf_bitnet_gemm_static(const uint8_t* packed_i2s, const int8_t* x, float scale, int M, int N, int K, float* y,
                           void* stream);
 
-/* ---- paged KV cache + decode attention (north-star item 5) ------------ */
+/* ---- paged KV cache + decode attention ------------ */
 
 /* Pool layout: [max_pages][L][2][Hkv][page_size][D] bf16 — one (page, layer, K|V, head) block is
  * page_size*D contiguous elements.  Token t of a sequence lives at page block_table[t / page_size],
@@ -193,7 +193,7 @@ int wf_paged_decode_attn(const void* q, const wf_kv_layout* kv, int layer, const
                          int max_blocks, const int32_t* seq_lens, int B, int H, float scale, void* out,
                          int out_dtype, void* workspace, size_t workspace_bytes, void* stream);
 
-/* ---- glue around the linears (SURVEY §8 a11) -------------------------------------------- */
+/* ---- glue around the linears -------------------------------------------- */
 
 /* rms_norm (direct_inference_full.py:181-184) with the reference's bf16 rounding points, fused
  * with the following per-token activation quantisation (…:196).  x bf16 [M,K]; gamma bf16 [K].
@@ -211,7 +211,7 @@ size_t wf_lm_head_workspace_bytes(int B, int V);
 int wf_lm_head_argmax(const void* h, const void* E, int B, int V, int K, float* logits_out, int32_t* next_out,
                       void* workspace, size_t workspace_bytes, void* stream);
 
-/* ---- decode engine (SURVEY §8 f2: the whole step of scripts/direct_inference_full.py:267-302) --- */
+/* ---- decode engine (the whole step of scripts/direct_inference_full.py:267-302) --- */
 
 typedef struct wf_model_config {
     int hidden, layers, heads, kv_heads, head_dim, ffn, vocab;
@@ -257,8 +257,8 @@ int wf_engine_decode(wf_engine* e, const int32_t* host_tokens, int B, int32_t* h
 int wf_engine_decode_device(wf_engine* e, int B, int use_graph);
 int wf_engine_sync(wf_engine* e);
 void* wf_engine_stream(wf_engine* e);
-/* Tensor parallel engines (cfg.tp_size > 1; one process per GPU, SURVEY §8e — the reference has no multi-GPU path,
- * this is the north star's "TP sharding of QKV/O/MLP with an all-reduce over NVLink").  Each rank creates its engine
+/* Tensor parallel engines (cfg.tp_size > 1; one process per GPU — the reference has no multi-GPU path,
+ * QKV / O / MLP are sharded, with an all-reduce over NVLink).  Each rank creates its engine
  * with its tp_rank, uploads ITS shard through wf_engine_set_linear (q,k,v,gate,up: this rank's output rows; o,down: this
  * rank's input columns; norms/embedding replicated), then the ranks exchange wf_engine_tp_export() handles (CUDA IPC,
  * wf_engine_tp_handle_bytes() each, e.g. with torch.distributed.all_gather) and call wf_engine_tp_attach with all

@@ -228,7 +228,7 @@ def gemm_i32(packed: np.ndarray, act: np.ndarray, mode: int = 0) -> np.ndarray:
 
 
 def gemm_i32_fast(packed: np.ndarray, act: np.ndarray, mode: int = 0) -> np.ndarray:
-    """Same integers as gemm_i32, for BASELINE-size matrices: unpack with the C oracle, then an exact
+    """Same integers as gemm_i32, for full-size matrices: unpack with the C oracle, then an exact
     float64 BLAS product (|sum| <= 2*128*28672 < 2^53, so every partial sum is an exact integer)."""
     act = _c(act, np.int8)
     if act.ndim == 1:

@@ -7,7 +7,7 @@ from ``oracle/wf_oracle.c`` or, when built, the reference's own SIMD kernel in
 paged KV manager semantics of ``tests/test_kv_cache_cpp.py:20-127``.
 
 Attention parity note: the reference holds no test that pins attention VALUES
- — the function itself, run in fp32/bf16 on CPU, is the oracle.
+— the function itself, run in fp32/bf16 on CPU, is the oracle.
 """
 from __future__ import annotations
 

@@ -204,7 +204,7 @@ void wfo_quantize_act_i8_rows(const float* x, int M, int K, int8_t* q, float* sc
  * sumi = sum_k code[k] * y[k] with code in {0,1,2} read from the blocked layout:
  * byte j of 128-block b carries k = b*128 + {j, 32+j, 64+j, 96+j} in bits 7-6, 5-4,
  * 3-2, 1-0.  Exact int64 here; the AVX2 kernel's int16 lane partials can wrap on
- * adversarial data (SURVEY.md H5) — wfo_vec_dot_i2_i8_avx2model models that. */
+ * adversarial data — wfo_vec_dot_i2_i8_avx2model models that. */
 int64_t wfo_vec_dot_i2_i8(int K, const uint8_t* x, const int8_t* y) {
     int64_t sum = 0;
     int nb = K / WFO_QK;

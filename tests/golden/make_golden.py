@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Generate the golden vectors under tests/golden/ by IMPORTING THE REFERENCE'S OWN PYTHON.
 
-Run in the build container only (needs /root/reference; the GPU box does not have it):
+Run where the reference's sources are at hand (/root/reference):
 
     python tests/golden/make_golden.py
 
@@ -104,7 +104,7 @@ def main():
         aq[f"x_{tag}"] = x.numpy()
         aq[f"q_{tag}"] = q.numpy()
         aq[f"s_{tag}"] = np.array(s, np.float64)
-    # native.py variant truncates instead of rounding (documented divergence, SURVEY H3)
+    # native.py variant truncates instead of rounding (documented divergence)
     xn = cases["vec"].numpy()
     qn, sn = native.quantize_activations(xn)
     aq["native_q_vec"] = qn
@@ -172,7 +172,7 @@ def main():
         at[f"v_{tag}"] = vs.numpy()
         at[f"q_{tag}"] = qs.numpy()
         at[f"out_{tag}"] = torch.stack(outs).numpy()
-    # head_dim 128 (the only head size of the BASELINE shapes; what the CUDA kernel implements), bf16 cache
+    # head_dim 128 (what the CUDA kernel implements), bf16 cache
     L, H, D, S = 2, 4, 128, 40
     cfg = kvmod.KVCacheConfig(max_seq_len=S, num_layers=L, num_heads=H, head_dim=D, dtype=kvmod.KVCacheDtype.BF16)
     cache = kvmod.KVCache(cfg)

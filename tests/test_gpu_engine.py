@@ -347,7 +347,7 @@ def test_streaming_decode_gemm_equals_default_kernels(shape, B, ctx, monkeypatch
 
 
 # ---------------------------------------------------------------------------------------------------------------------
-# the full BitNet-2B-4T shape (30 layers, hidden 2560, 20/5 heads, ffn 6912, vocab 128256),
+# The full BitNet-2B-4T shape (30 layers, hidden 2560, 20/5 heads, ffn 6912, vocab 128256),
 # batch 1, 512-token prompt, 128 greedy tokens -- the protocol of extern/BitNet/utils/e2e_benchmark.py:36-53 run through
 # the generate loop of scripts/direct_inference_full.py:328-371 -- GPU engine vs the reference CPU path (oracle forward on
 # the reference's own unmodified AVX2 kernel) on identical synthetic random-init ternary weights.
@@ -423,7 +423,7 @@ def _protocol(cfg, w, with_sensitivity):
     om32 = OM.OracleModel(oracle_cfg(cfg), w, use_ref=True, attn_fp32=True) if with_sensitivity else None
     eng = Engine(cfg)
     eng.load_weights(w)
-    prompt = np.random.default_rng(0).integers(0, cfg.vocab, size=CFG0_PROMPT)   # SURVEY 8(d) config 1: randint(0, 128256), seed 0
+    prompt = np.random.default_rng(0).integers(0, cfg.vocab, size=CFG0_PROMPT)   # randint(0, 128256), seed 0
     for pos, t in enumerate(prompt):       # the reference's generate() prefill is exactly this token-by-token loop (:343-347)
         om.forward(int(t), pos)
         eng.decode([int(t)])

@@ -1,5 +1,5 @@
 """GPU parity: the tcgen05 (kind::i8) prefill GEMM.  int32 accumulators bit-exact vs the oracle on sizes it
-finishes in seconds, fused epilogues identical to the mma.sync path, and at the BASELINE prefill size
+finishes in seconds, fused epilogues identical to the mma.sync path, and at the 2B prefill size
 (8 x 2048 tokens) size-independent properties: equality with the already-pinned mma.sync kernel on the same
 inputs, linearity in the activations and an oracle check of a random sample of rows."""
 import numpy as np
@@ -89,7 +89,7 @@ def test_tc_fused_epilogues_match_mma_path():
 
 @pytest.mark.parametrize("nk", [(3840, 2560), (2560, 6912)])
 def test_tc_prefill_size_properties(nk):
-    """BASELINE config 3 size: M = 8 x 2048 tokens."""
+    """A full prefill batch: M = 8 x 2048 tokens."""
     from wf_bitnet import ops
     n, k = nk
     m = 16384

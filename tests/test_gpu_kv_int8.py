@@ -1,4 +1,4 @@
-"""int8 KV option (SURVEY §8f rank 3; the reference's KVCacheDtype.INT8, kv_cache/kv_cache.py:198-228) on the GPU path:
+"""int8 KV option (the reference's KVCacheDtype.INT8, kv_cache/kv_cache.py:198-228) on the GPU path:
 codes / scales bit-exact against the oracle's restatement of the reference arithmetic (per (token, head) row), attention
 against the oracle attention on the DEQUANTISED cache (what KVCache.get hands to SDPA), engine logits against the oracle
 model with the same cache, fused phase path == per-op path."""

@@ -76,7 +76,7 @@ def test_gemv_large_shapes_every_slab_mode(nk, m):
 @pytest.mark.parametrize("nk", [(57344, 8192), (8192, 28672)])
 def test_gemv_70b_shapes(nk):
     """The 70B matrices wf_bench_gemv times and reports bandwidth on: gate|up (57344 x 8192, 117 MB packed) and down
-    (8192 x 28672, 224 k-blocks: the longest row dot of any BASELINE config, |acc| up to 7.3 M), M = 1 (dp4a), 2 and 8 (mma).
+    (8192 x 28672, 224 k-blocks: the longest row dot of any shape here, |acc| up to 7.3 M), M = 1 (dp4a), 2 and 8 (mma).
     The expected accumulators come straight from the ternary matrix in exact float64 row chunks (no unpack in between);
     the packed bytes are the C oracle's (quantize_i2_s restatement)."""
     from wf_bitnet import ops
@@ -137,7 +137,7 @@ def test_accumulators_bit_exact_batched(nk, m):
 
 def test_raw_int8_activations_extremes():
     """extern/BitNet/gpu/test.py:32-61 style: random int8 in [-128,127], exact equality; plus the adversarial
-    all-(+1) x 127 case where the reference's AVX2 int16 lanes wrap (SURVEY H5) — exact oracle only."""
+    all-(+1) x 127 case where the reference's AVX2 int16 lanes wrap — exact oracle only."""
     from wf_bitnet import ops
     rng = np.random.default_rng(0)
     n, k = 2560, 6912
@@ -197,7 +197,7 @@ def test_linear_mode_within_1e3(nk, m):
     got = ops.ternary_linear(tile, n, k, cu(q), mode="linear", rowsum=cu(rs), act_scale=cu(s),
                              w_scale=torch.tensor([ws], device="cuda"), out_dtype=torch.float32).cpu().numpy()
     rel = np.linalg.norm(got - want) / np.linalg.norm(want)
-    assert rel <= 1e-3, rel
+    assert rel <= 1e-3, rel            # the bar for dequantised outputs
     # the epilogue follows the reference's own rounding sequence fl32(fl32(fl32(S*s_w) - fl32(s_w*sum a)) * s_a), so the fp32
     # values are in fact IDENTICAL to the CPU path's, not merely close
     assert np.array_equal(got, want), np.abs(got - want).max()

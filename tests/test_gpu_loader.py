@@ -1,4 +1,4 @@
-"""GPU parity of the checkpoint loader + cache converter (SURVEY §8f rank 1): an HF-style snapshot with the projections stored
+"""GPU parity of the checkpoint loader + cache converter: an HF-style snapshot with the projections stored
 as HF-packed uint8 [N/4, K] (tests/test_bitnet_core.py:21-53), as ternary floats, and as a packed_bitnet_v1 / b200_tile_v1 cache
 entry written by convert_and_save_bitnet must all load into the engine to the SAME logits as the in-memory weights."""
 import json

@@ -66,7 +66,7 @@ def test_tile_layout_roundtrip_and_definition(shape):
     tile = ops.i2s_to_tile(cu(packed))
     assert tile.numel() == ((n + 15) // 16) * (k // 128) * 512
     assert np.array_equal(ops.tile_to_i2s(tile, n, k).cpu().numpy(), packed)
-    # definition check (DESIGN.md): lane l, word i <- row 16rb + (l>>2) + 8(i&1), bytes 4(l&3) + 16(i>>1) of block kb
+    # definition check: lane l, word i <- row 16rb + (l>>2) + 8(i&1), bytes 4(l&3) + 16(i>>1) of block kb
     t = tile.cpu().numpy().reshape((n + 15) // 16, k // 128, 32, 4, 4)
     rb, kb, l, i = (n - 1) // 16 // 2, (k // 128) - 1, 13, 2
     row = rb * 16 + (l >> 2) + 8 * (i & 1)

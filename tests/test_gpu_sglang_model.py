@@ -1,4 +1,4 @@
-"""`sglang.srt.models.bitnet` mirror (SURVEY §8f rank 4), written the way the reference's own tests for the fork's module read:
+"""`sglang.srt.models.bitnet` mirror, written the way the reference's own tests for the fork's module read:
 tests/test_bitnet_weight_loading.py:15-135, tests/test_bitnet_comparison.py:10-74, tests/test_vllm_cpu_stub.py:225-295.
 Tensors are handed in on the CPU like there; the work happens on the GPU through the C ABI."""
 import numpy as np
@@ -73,7 +73,7 @@ def test_bitnet_linear_vs_oracle_and_float_matmul(batch, finalized):
     acc = q.astype(np.int64) @ weight.numpy().astype(np.int64).T
     want = acc.astype(np.float64) * 1.7 * s_a
     err = np.linalg.norm(y.numpy().astype(np.float64) - want) / np.linalg.norm(want)
-    assert err <= 1e-3, err                                                               # north-star tolerance for dequantised outputs
+    assert err <= 1e-3, err                                                               # the tolerance for dequantised outputs
     ref = torch.matmul(x, weight.t()) * 1.7
     cos = torch.nn.functional.cosine_similarity(ref.flatten().unsqueeze(0), y.flatten().unsqueeze(0)).item()
     assert cos > 0.99, cos

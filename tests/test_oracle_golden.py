@@ -164,7 +164,7 @@ def test_ref_kernel_agrees_with_oracle(shape):
 
 @needs_ref
 def test_ref_int16_wrap_is_modelled_not_reproduced():
-    """the AVX2 kernel wraps on adversarial data; the oracle of record is exact."""
+    """The AVX2 kernel wraps on adversarial data; the oracle of record is exact."""
     k = 4096
     w = np.ones((1, k), np.float32)
     packed, _ = O.pack_ternary(w)

@@ -1,4 +1,4 @@
-// Paged KV cache + split-KV flash-decode attention (north-star item 5).
+// Paged KV cache + split-KV flash-decode attention.
 //
 // Replaces the reference's KV utilities:
 //   * KVCache.update / .get + attention_with_kv_cache  (src/wrinklefree_inference/kv_cache/kv_cache.py:230-369)
@@ -25,12 +25,12 @@ constexpr int AT_WARPS = 4;
 constexpr int AT_EVEN_MAXB = 128;   // even work split (fused decode form): the per-sequence block counts are scanned by one CTA-wide pass
 constexpr int AT_STAGES = 3;
 constexpr int AT_BLK = 16;                              // tokens per stage
-constexpr int AT_D = 128;                               // head_dim (all BASELINE shapes)
+constexpr int AT_D = 128;                               // head_dim (all supported shapes)
 constexpr int AT_ROW = AT_D * 2;                        // bytes per token row
 constexpr int AT_STAGE_BYTES = 2 * AT_BLK * AT_ROW;     // K + V
 constexpr int AT_SMEM = AT_WARPS * AT_STAGES * AT_STAGE_BYTES;   // 96 KB
 
-// ---- int8 KV option (SURVEY 8f rank 3; the reference's KVCacheDtype.INT8, kv_cache/kv_cache.py:198-228): K and V are int8
+// ---- int8 KV option (the reference's KVCacheDtype.INT8, kv_cache/kv_cache.py:198-228): K and V are int8
 // with one fp32 scale per (token, kv head).  Pool = int8 region [page][layer][K|V][head][slot][D] followed by the scale
 // region [page][layer][K|V][head][slot].  The streaming loop moves half the bytes: int8 rows go through the same cp.async
 // ring (6 stages of 4 KB + 128 B of scales), ldmatrix reads them as b16 pairs and ONE PRMT per f16x2 operand register turns
@@ -111,7 +111,7 @@ struct AttnParams {
     int cluster;                 // 1 (fused form, small grids): the chunks of a (sequence, kv head) pair are ONE thread-block cluster; their partials
                                  // meet in distributed shared memory (two cluster barriers) instead of global memory + fence + atomic + reload
     int two_short_first;         // two-class grid: dispatch the short CTAs before the whole pairs (WF_ATTN_TWO_ORDER=1; measured worse: 5.26 vs 5.10 ms
-                                 // at bs64/4K, 8.43 vs 8.09 at 8K, profiles/r02ag_summary.txt)
+                                 // at bs64/4K, 8.43 vs 8.09 at 8K)
     int two_pa, two_nb;          // two-class grid (fused form): the first two_pa pairs are ONE CTA each (no split, no merge), every later pair is
                                  // two_nb CTAs of chunk_blocks blocks; 1-D grid, long CTAs first (two_nb = 0: uniform grid)
     int chunk_major;             // legacy grid order: 1 = (kv head, sequence, chunk), 0 = (chunk, kv head, sequence)
@@ -293,7 +293,6 @@ __global__ void __launch_bounds__(AT_WARPS * 32, I8 ? 3 : 2) paged_decode_attn_k
 
     // page of this warp's block i, looked up THREE issues ahead (a 3-deep register queue): one issue = one block of compute (~0.3-0.5 us),
     // an L2 round trip under load is ~1 us — with a single entry ahead 13 % of the kernel's stall samples sat on this dependency
-    // (profiles/r02_full_attn_fused_bs64.summary.txt, attn.cu kv_block_offset)
     auto page_of = [&](int i) -> int {
         const int tokf = (blk0 + warp + AT_WARPS * i) * AT_BLK;
         const int pi = p.page_shift >= 0 ? (tokf >> p.page_shift) : tokf / p.page_size;
@@ -966,7 +965,7 @@ int launch_paged_decode_attn(AttnParams p, int max_seq_hint, void* workspace, si
     }
     const int max_blocks16 = (max_seq_hint + AT_BLK - 1) / AT_BLK;
     // Chunking of a sequence's KV stream over CTAs (large grids; small ones take the cluster form below).  Cost model, calibrated on
-    // forced chunk counts (profiles/r02ab_summary.txt, r02ac_summary.txt), in units of one 16-token block of a CTA:
+    // forced chunk counts, in units of one 16-token block of a CTA:
     //   * J = pairs * n CTAs of length L = chunk + C0 (prologue, ring fill, 4-warp merge) run in waves of `slots` resident CTAs;
     //   * the KV stream is bandwidth-bound long before every slot is busy: R ~ 3/8 of the slots saturate HBM, so a wave of m >= R
     //     CTAs takes m * L / R, a wave of fewer takes L (each CTA then runs at its own latency-bound rate);
@@ -995,7 +994,7 @@ int launch_paged_decode_attn(AttnParams p, int max_seq_hint, void* workspace, si
         chunk_blocks = old_cb; nchunks = old_n;
     } else {
         const long long slots = (long long)(p.kv_scales ? 3 : 2) * sm_count();
-        // the int8 form is issue-bound, not HBM-bound: it gains from every resident CTA (R = slots).  Forced counts, profiles/r02ak_summary.txt:
+        // the int8 form is issue-bound, not HBM-bound: it gains from every resident CTA (R = slots).  Forced counts:
         // 2B bs32/2K one chunk 2.81 ms, two 2.45; bs48/4K one 4.09, three 3.77; bs64/4K and bs64/2K one chunk (320 CTAs on 444 slots) best
         const long long R = p.kv_scales ? slots : slots * 3 / 8;
         auto model = [&](int nn, int cb) -> long long {
@@ -1029,7 +1028,7 @@ int launch_paged_decode_attn(AttnParams p, int max_seq_hint, void* workspace, si
     const char* cl_s = getenv("WF_ATTN_CLUSTER");
     p.cluster = 0;
     if (fused_q && (!cl_s || atoi(cl_s) != 0)) {
-        // measured (profiles/r02k_summary.txt, 2B): batch 1 / 512: 1.375 -> 1.278 ms, batch 1 / 4K: 1.499 -> 1.395, batch 16 / 2K: 2.40 ->
+        // measured (2B): batch 1 / 512: 1.375 -> 1.278 ms, batch 1 / 4K: 1.499 -> 1.395, batch 16 / 2K: 2.40 ->
         // 2.19; but batch 8 / 2K with 7-CTA clusters 1.87 -> 2.01 and batch 1 / 16K with 8 x 129-block chunks 1.84 -> 1.90: clusters
         // of <= 4 once the grid exceeds one CTA per SM, and only while a chunk stays short (more chunks than a cluster holds = the
         // global form, which can use every SM)
@@ -1045,7 +1044,7 @@ int launch_paged_decode_attn(AttnParams p, int max_seq_hint, void* workspace, si
         }
     }
     nchunks = (max_blocks16 + chunk_blocks - 1) / chunk_blocks;
-    if (fused_q && cl_s && atoi(cl_s) == 2) p.cluster = 1;   // WF_ATTN_CLUSTER=2: clusters on large grids too — measured slower (5.40 vs 5.31 ms at batch 64 / 4K, profiles/r02y_summary.txt)
+    if (fused_q && cl_s && atoi(cl_s) == 2) p.cluster = 1;   // WF_ATTN_CLUSTER=2: clusters on large grids too — measured slower (5.40 vs 5.31 ms at batch 64 / 4K)
     if (p.cluster && (nchunks < 2 || nchunks > 8)) p.cluster = 0;
     p.chunk_blocks = chunk_blocks;
     p.max_chunks = nchunks;
@@ -1056,7 +1055,7 @@ int launch_paged_decode_attn(AttnParams p, int max_seq_hint, void* workspace, si
     const bool fused_form = p.qkv_acc != nullptr && p.merge_cnt != nullptr;
     const bool i8_pool = p.kv_scales != nullptr;
     const char* even_s = getenv("WF_ATTN_EVEN");   // read per launch (launches are graph-captured): tests switch it inside one process
-    const int even_env = even_s ? atoi(even_s) : 0;   // opt-in: measured 5.65 vs 5.46 ms per bs64/4K step (profiles/r02i_*): the per-segment
+    const int even_env = even_s ? atoi(even_s) : 0;   // opt-in: measured 5.65 vs 5.46 ms per bs64/4K step: the per-segment
                                                        // prologue / merge of a CTA costs what the missing partial wave saves
     { const char* cm = getenv("WF_ATTN_CHUNK_MAJOR"); p.chunk_major = cm ? atoi(cm) : 0; }   // measured: chunk-major dispatch 5.71 vs 5.47 ms (bs64/4K)
     int even_ctas = 0;
@@ -1095,7 +1094,7 @@ int launch_paged_decode_attn(AttnParams p, int max_seq_hint, void* workspace, si
             }
         }
     }
-    {   // per-sequence chunking (WF_ATTN_ADAPT=0: fixed chunks of the hint, the round-2 parity twin); read per launch like WF_ATTN_TWO
+    {   // per-sequence chunking (WF_ATTN_ADAPT=0: fixed chunks of the hint, for comparison); read per launch like WF_ATTN_TWO
         const char* ad = getenv("WF_ATTN_ADAPT");
         p.min_cb = (ad && atoi(ad) == 0) ? 0 : (p.cluster ? 4 : 16);
     }

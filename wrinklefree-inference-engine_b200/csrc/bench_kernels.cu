@@ -1,4 +1,4 @@
-// Kernel-level measurement support (SURVEY §8d): times the ternary GEMV the way the reference's
+// Kernel-level measurement support: times the ternary GEMV the way the reference's
 // scripts/benchmark_kernels.py:28-66 does — a loop of calls, bytes = N*K/4 + M*K + out — except that the launches
 // rotate over enough independent weight copies to exceed the 126 MB L2, so the figure is an HBM figure.
 #include "kernels.cuh"

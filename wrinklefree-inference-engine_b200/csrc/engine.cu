@@ -76,17 +76,17 @@ struct wf_engine {
     int linear_algo = 0;
     int hx = 1;              // relu^2(gate)*up in its own small kernel instead of every down-proj CTA's prologue (WF_HX=0 to fold it back)
     int decode_tc = 1;       // batched decode linears (B >= decode_tc_min, single GPU) on tcgen05 split-K REDs (gemm_tc.cu launch_gemm_tc_red) instead of the mma.sync one-shot
-                             // GEMM: bit-identical; with the round-2 issue loop / epilogue 3.65 -> 3.23 ms at batch 40 / 2K, 5.48 -> 5.32 ms at batch 64 / 4K (WF_DECODE_TC=0: off)
+                             // GEMM: bit-identical; with the present issue loop and epilogue 3.65 -> 3.23 ms at batch 40 / 2K, 5.48 -> 5.32 ms at batch 64 / 4K (WF_DECODE_TC=0: off)
     int decode_tc_min = 33;  // WF_DECODE_TC_MIN
     int decode_stream = 1;   // WF_DECODE_STREAM: streaming batched GEMM (gemm_stream.cu); 0 off, 1 = batches up to decode_stream_max rows, 2 = every batch it takes (<= 32)
-    int decode_stream_mask = 15;  // WF_DECODE_STREAM_MASK: which linears may take it (1 q|k|v, 2 o, 4 gate|up, 8 down) — for bisecting the TP mismatch
-    int decode_stream_max = 16;   // WF_DECODE_STREAM_MAX.  Measured (profiles/r02ap_summary.txt), ms per step stream / default: 2B bs2 1.33 / 1.58, bs8 1.43 / 1.63,
+    int decode_stream_mask = 15;  // WF_DECODE_STREAM_MASK: which linears may take it (1 q|k|v, 2 o, 4 gate|up, 8 down) — for bisecting the mismatch under tensor parallelism
+    int decode_stream_max = 16;   // WF_DECODE_STREAM_MAX.  Measured, ms per step stream / default: 2B bs2 1.33 / 1.58, bs8 1.43 / 1.63,
                                   // bs16/2K 1.99 / 2.17; 8B bs4 1.97 / 3.00, bs8 2.26 / 3.24, bs16/2K 3.06 / 3.85; 70B bs16/8K 20.0 / 22.9; but 17..32 rows (four n-tiles,
                                   // one CTA per SM): 2B bs32/2K 2.74 / 2.56, 8B bs32/2K 4.55 / 4.20
-    int tail_batch = 0;      // WF_TAIL_BATCH=1: the same for 8 < B <= 64 (layer_tail_batch.cu).  Opt-in: measured 5.74 ms vs 5.44 ms per bs64/4K step for the phase path (profiles/r02d_*)
+    int tail_batch = 0;      // WF_TAIL_BATCH=1: the same for 8 < B <= 64 (layer_tail_batch.cu).  Opt-in: measured 5.74 ms vs 5.44 ms per bs64/4K step for the phase path
     int small_max = 1;       // WF_SMALL_MAX: largest batch on the GEMV-style kernels (linear_small / layer_tail: the row glue runs per CTA and per row,
                              // ~3 us x B x 4 phases per layer); above it the batched kernels (row glue once per row in its own CTA + batched GEMM).
-                             // Measured (profiles/r02j_summary.txt, 2B, 512 ctx): B = 2 / 4 / 8: 1.81 / 2.46 / 3.70 ms on the GEMV-style kernels, 1.72 / 1.74 / 1.75 ms batched
+                             // Measured (2B, 512 ctx): B = 2 / 4 / 8: 1.81 / 2.46 / 3.70 ms on the GEMV-style kernels, 1.72 / 1.74 / 1.75 ms batched
     int tail_lam = 1;        // WF_TAIL_LAM: batch-1 tail kernel hands its phases over flag-in-data (no grid barriers); 0 = grid barriers
     int tail = 1;            // 1: persistent layer-tail kernel (layer_tail.cu) for B <= 8 on single-GPU engines: 2 launches per layer (WF_TAIL=0: phase kernels)
     // grid-barrier arrival counters, one set per launch site, and the epoch (steps so far) of each kernel family:
@@ -331,7 +331,7 @@ int run_step_tail(wf_engine* e, int B, int feed_back) {
 // NEXT phase applies scales / residual / relu^2*up / norm / re-quantisation in its prologue.
 //   B <= 8 : 5 launches per layer (qkv, attention, o, gate|up, down), each linear = glue prologue + TMA-streamed GEMV
 //   B  > 8 : 9 launches per layer (glue_rows + gemm_oneshot per linear, fused attention)
-// Tensor parallel (tp.size = T > 1, SURVEY §8e): q|k|v and gate|up are split by output rows (whole heads), attention and
+// Tensor parallel (tp.size = T > 1): q|k|v and gate|up are split by output rows (whole heads), attention and
 // the KV pool by KV head, o and down by input columns.  The exchanges are fused into the producers (tp_comm.cuh):
 //   B  attention stores its heads into attn_full of every rank            (all-gather, flag 4l+0)
 //   C  o-proj REDs its exact partial sums into acc_o of every rank         (all-reduce, flag 4l+1)
@@ -382,11 +382,11 @@ int run_step_fused(wf_engine* e, int B, int feed_back) {
         if (r) return r;
         // a real dense contraction (33..64 tokens): tcgen05 int8 with split-K REDs; single-GPU engines only for now
         // tcgen05 split-K form (one owner per 128-row tile streams its whole K; the one-shot GEMM pays a RED round per 4 k-blocks): from 33
-        // tokens up; from 9 tokens for K >= 8192 (70B shapes); from 24 tokens for >= 16 MB matrices.  Measured in profiles/r02q_summary.txt:
+        // tokens up; from 9 tokens for K >= 8192 (70B shapes); from 24 tokens for >= 16 MB matrices.  Measured:
         // 70B bs16 32.2 -> 24.6 ms, 8B bs32 4.95 -> 4.84 ms, while 8B bs16 gate|up (29 MB, K = 4096) is faster on the one-shot GEMM.
         const size_t wbytes = (size_t)N * K / 4;
         // (17..24 rows: the two-pass form wins where the tcgen05 split-K form does not apply (K < 8192): 8B bs20/2K 4.19 -> 3.91 ms, bs24 4.35 -> 4.06;
-        //  at the 70B widths it loses, 70B bs20/4K 20.0 -> 22.3: profiles/r02bc_summary.txt)
+        //  at the 70B widths it loses, 70B bs20/4K 20.0 -> 22.3)
         const int stream_rows = e->decode_stream >= 2 ? 32 : (K < 8192 && e->decode_stream_max == 16 ? 24 : e->decode_stream_max);
         if (e->decode_stream && ((e->decode_stream_mask >> slot) & 1) && B <= stream_rows && gemm_stream_fits(B, N, K)) {
             OneshotArgs o;
@@ -595,7 +595,7 @@ extern "C" int wf_engine_create(const wf_model_config* cfg, wf_engine** out) {
     const int T = c.tp_size <= 0 ? 1 : c.tp_size;
     if (T > TP_MAX || c.tp_rank < 0 || c.tp_rank >= T) { set_error("engine: tp_size must be 1..%d and 0 <= tp_rank < tp_size", TP_MAX); return WF_ERR_INVALID; }
     if (c.heads % T || c.kv_heads % T || c.ffn % (16 * T) || (c.ffn / T) % 128) {
-        set_error("engine: heads (%d), kv_heads (%d) and ffn/128 (%d) must be divisible by tp_size %d (SURVEY §8e: the 2B shape only shards over 1 or 5 GPUs)",
+        set_error("engine: heads (%d), kv_heads (%d) and ffn/128 (%d) must be divisible by tp_size %d (the 2B shape only shards over 1 or 5 GPUs)",
                   c.heads, c.kv_heads, c.ffn / 128, T);
         return WF_ERR_UNSUPPORTED;
     }
@@ -640,12 +640,12 @@ extern "C" int wf_engine_create(const wf_model_config* cfg, wf_engine** out) {
     { const char* x = getenv("WF_DECODE_STREAM_MAX"); if (x) e->decode_stream_max = atoi(x) < 1 ? 1 : (atoi(x) > 32 ? 32 : atoi(x)); }
     if (e->fused && !env_pdl) e->pdl = true;   // the phase kernels are built around programmatic dependent launch
     // Tensor-parallel engines keep the one-shot / tcgen05 linears: with the streaming GEMM under the exchanges TP = 2 at the 8B layer shape, batch 16, was
-    // bit-identical to TP = 1 in 12 of 14 runs only (profiles/r02bf_summary.txt; 0 mismatches in 33 runs without it, 0 in 10 x 7 single-GPU runs) — a
+    // bit-identical to TP = 1 in 12 of 14 runs only (0 mismatches in 33 runs without it, 0 in 10 x 7 single-GPU runs) — a
     // rare ordering problem between its REDs into peer accumulators and the flag protocol that was not tracked down.  WF_DECODE_STREAM=1 forces it.
     if (T > 1 && !getenv("WF_DECODE_STREAM")) e->decode_stream = 0;
     // Batch 1 on shapes whose ffn row is too long for the hand-off form of the tail kernel (register glue: <= 9216 elements; the 8B / 70B widths)
-    // goes through the row glue + streaming batched GEMM instead of the grid-barrier tail kernel: 8B bs1 1.97 -> 1.86 ms, 70B bs1 9.32 -> 8.22 ms
-    // (profiles/r02az_summary.txt).  Single-GPU engines only: under tensor parallelism batch 1 keeps the all-RED exchange of the GEMV-style kernels.
+    // goes through the row glue + streaming batched GEMM instead of the grid-barrier tail kernel: 8B bs1 1.97 -> 1.86 ms, 70B bs1 9.32 -> 8.22 ms.
+    // Single-GPU engines only: under tensor parallelism batch 1 keeps the all-RED exchange of the GEMV-style kernels.
     if (!getenv("WF_SMALL_MAX") && T == 1 && e->decode_stream) {
         int maxK = e->hidden > e->attn_full ? e->hidden : e->attn_full;
         if (e->ffn_full > maxK) maxK = e->ffn_full;
@@ -914,7 +914,7 @@ extern "C" int wf_engine_init_synthetic(wf_engine* e, uint64_t seed) {
         if ((rc = launch_fill_ternary(L.o, wf_tile_bytes(e->hidden, e->attn_dim), sr + 2, s))) return rc;
         if ((rc = launch_fill_ternary(L.gu, wf_tile_bytes(2 * e->ffn, e->hidden), sr + 3, s))) return rc;
         if ((rc = launch_fill_ternary(L.down, wf_tile_bytes(e->hidden, e->ffn), sr + 4, s))) return rc;
-        // weight_scale ~ U(0.5, 2.5) (SURVEY §8d); deterministic LCG on the host
+        // weight_scale ~ U(0.5, 2.5); deterministic LCG on the host
         uint64_t st = sd ^ 0xD1B54A32D192ED03ull;
         for (int i = 0; i < 7; ++i) {
             st = st * 6364136223846793005ull + 1442695040888963407ull;

@@ -1,5 +1,4 @@
-// Streaming batched ternary GEMM for the decode step, 1..32 activation rows (the engine uses it up to 16 rows, 24 where K < 8192, and for batch 1 at the 8B / 70B widths) (bitnet_gemm at decode batch sizes; the
-// engine's linears on the 8B / 70B matrices, DESIGN 7 gap 3).
+// Streaming batched ternary GEMM for the decode step, 1..32 activation rows (the engine uses it up to 16 rows, 24 where K < 8192, and for batch 1 at the 8B / 70B widths).
 //
 //   acc[m, n] += sum_k code[n, k] * a[m, k]        exact integers in fp32 (|S| < 2^24), RED into the step's split-K accumulators
 //   (reference: one ggml_vec_dot_i2_i8_s per output element, extern/BitNet/src/ggml-bitnet-mad.cpp:94-186)
@@ -254,7 +253,7 @@ int launch_gemm_stream(const OneshotArgs& a, cudaStream_t s, bool pdl) {
     cfg.gridDim = dim3(grid);
     // 9..16 rows whose activation window leaves room for only one CTA per SM (K windows of >= 3.5K at 16 rows: the 8B / 70B widths): that CTA
     // brings 16 consumer warps instead of 8
-    static const int wide_env = getenv("WF_GS_WIDE") ? atoi(getenv("WF_GS_WIDE")) : 0;   // measured slower: 8B bs16 3.19 vs 3.05 ms, 70B bs16 20.3 vs 19.9 (profiles/r02au_summary.txt)
+    static const int wide_env = getenv("WF_GS_WIDE") ? atoi(getenv("WF_GS_WIDE")) : 0;   // measured slower: 8B bs16 3.19 vs 3.05 ms, 70B bs16 20.3 vs 19.9
     const bool wide = ntl == 2 && cps == 1 && wide_env;
     cfg.blockDim = dim3((ntl == 4 || wide) ? 17 * 32 : 9 * 32);
     cfg.dynamicSmemBytes = smem;

@@ -1,4 +1,4 @@
-// Prefill / large-batch ternary GEMM on the 5th-generation tensor cores (tcgen05, kind::i8) — north-star item 4.
+// Prefill / large-batch ternary GEMM on the 5th-generation tensor cores (tcgen05, kind::i8).
 //
 //   S[m,n] = sum_k code[n,k] * a[m,k],  code = w+1 in {0,1,2} (u8), a int8, exact int32 accumulation
 //   (what bitnet_gemm computes row by row with ggml_vec_dot_i2_i8_s, extern/BitNet/src/ggml-bitnet-mad.cpp:94-186;
@@ -21,9 +21,9 @@
 //     correction, scales, residual, relu^2*up) in registers -> one store per token: a warp's 32 lanes are 32 consecutive n,
 //     so every store instruction is a full coalesced line and nothing is transposed through shared memory.
 // Shared memory is the binding resource of the main loop: TMA write + MMA read of the activation tile = 128 B/clk at the
-// 256-clk/stage tensor floor, i.e. all of an SM's shared-memory bandwidth.  Round 2 measurements (profiles/r02_prefill_*):
-// with the epilogue's math and stores switched off the kernel runs 2.15 PTOP/s (374 clk per stage) — the round-1 epilogue
-// (smem transpose + dependent per-token global loads) cost 40 % on the short-K shapes.  The cta_group::2 form (each SM
+// 256-clk/stage tensor floor, i.e. all of an SM's shared-memory bandwidth.  Measured
+// with the epilogue's math and stores switched off the kernel runs 2.15 PTOP/s (374 clk per stage); an epilogue with a
+// shared-memory transpose and dependent per-token global loads cost 40 % on the short-K shapes.  The cta_group::2 form (each SM
 // holds half of the activation tile) is what would lift the 374-clk stage.
 #include "linear_common.cuh"
 #include "fused_common.cuh"
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
         // A thread owns one weight row n (TMEM lane) and receives 32 tokens per tcgen05.ld.  The output is token-major, so a
         // warp's store of ONE token covers 32 consecutive n: a full 128-byte line in fp32 (64 B in bf16) — coalesced as it
         // stands, no transpose through shared memory.  Two warps share a lane quarter and take 64 tokens each: with four warps
-        // and ~34 issued instructions per token the epilogue paced the short-K shapes (ncu r02_full_gemm_tc: the four warps
+        // and ~34 issued instructions per token the epilogue paced the short-K shapes (the four warps
         // never idle, the MMA warp 27 % of its time waiting for a drained accumulator).  gate|up tiles (relu^2*up): the 16 up
         // rows of a 32-row group sit in lanes 16..31 and are handed to the gate lanes with one shuffle.
         const int q = warp & 3, th = warp >> 2;                                    // lane quarter, token half

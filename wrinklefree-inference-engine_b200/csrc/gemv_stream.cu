@@ -1,4 +1,4 @@
-// Bandwidth-bound ternary GEMV for decode (M <= 8 activation rows) — north-star item 3.
+// Bandwidth-bound ternary GEMV for decode (M <= 8 activation rows).
 //
 //   S[m,n] = sum_k code[n,k] * a[m,k]   (exact int32; reference: ggml_vec_dot_i2_i8_s,
 //   extern/BitNet/src/ggml-bitnet-mad.cpp:94-186, one call per output row under OpenMP)

@@ -1,4 +1,4 @@
-// Glue kernels around the ternary linears (SURVEY §8 a11): embedding gather, tied bf16 LM head with
+// Glue kernels around the ternary linears: embedding gather, tied bf16 LM head with
 // greedy argmax, step bookkeeping, and on-device synthetic data generators for bench / smoke.
 //
 // Reference: scripts/direct_inference_full.py:290 (embedding row), :297-300 (F.linear(hidden, embed) in
@@ -22,7 +22,7 @@ __global__ void embed_kernel(const uint4* __restrict__ table, const int32_t* __r
 
 // ---------------------------------------------------------------------------------------------
 // LM head: logits[b, v] = sum_k h[b,k] * E[v,k]; E bf16 [V,K] streamed once from HBM (657 MB for the 2B
-// model — more bytes than all ternary layers together, SURVEY H7).  CTA = 8 warps x 16 vocab rows,
+// model — more bytes than all ternary layers together).  CTA = 8 warps x 16 vocab rows,
 // 64-wide k stages through a 4-stage cp.async ring, XOR-swizzled smem, ldmatrix + mma.m16n8k16 bf16.
 constexpr int LM_ROWS = 128;
 constexpr int LM_KC = 64;                       // k per stage (128 B per row)

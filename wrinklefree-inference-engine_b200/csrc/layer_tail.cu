@@ -19,7 +19,7 @@
 //     outputs are written once by their owner — no split-K, no atomics, no zeroing duty — and gate|up can apply
 //     relu(gate)^2 * up in its epilogue; the extra CTAs of a non-divisible phase are rotated so that the bytes a CTA streams
 //     over the whole tail stay balanced;
-//   * batch 1 (the north-star shape) goes one step further: NO grid barrier between the phases.  The accumulator / h rows are
+//   * batch 1 goes one step further: NO grid barrier between the phases.  The accumulator / h rows are
 //     hand-off buffers that hold a sentinel until their owner stores the data; the consumer's row glue polls the words it needs
 //     (one L2 hop instead of release fence + atomic arrival + acquire poll + load), every CTA keeps the residual row and the
 //     previous phase's activation scale / rowsum locally (it computed them itself), and owners re-arm the sentinels two phases
@@ -417,8 +417,8 @@ int launch_layer_tail(const TailArgs& a, cudaStream_t s, bool pdl) {
     p.sacc_rbs = max_rbs + 2;
     // flag-in-data form: batch 1, the whole tail, every row in the register form of the glue (K <= 9216: the 2B shape).  Extending it to
     // the 8B / 70B ffn rows through the scratch form of the glue was measured: 1.95 -> 1.92 ms (8B), 9.25 -> 9.59 ms (70B), and the extra
-    // code cost the 2B shape 8 % (profiles/r02v_summary.txt) — not kept.  Neither was an instantiation whose register glue holds the 8B ffn
-    // row in 5 granules per thread: 316 bytes of spills, 1.95 -> 2.69 ms (profiles/r02x_summary.txt).
+    // code cost the 2B shape 8 % — not kept.  Neither was an instantiation whose register glue holds the 8B ffn
+    // row in 5 granules per thread: 316 bytes of spills, 1.95 -> 2.69 ms.
     const bool lam_ok = a.lam && a.M == 1 && a.nph >= 3 && Kmax <= LT_CT * 8 * 3;
     p.lam = lam_ok ? 1 : 0;
     p.xs_elems = lam_ok ? a.ph[1].K : 0;

@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(GR_T) glue_rows_cluster_kernel(const GlueParam
 
 int launch_glue_rows(const GlueParams& g, cudaStream_t s, bool pdl) {
     if (g.M < 1 || g.K % 8) { set_error("glue_rows: bad shape"); return WF_ERR_INVALID; }
-    // clusters for long rows when the rows alone leave most SMs idle: OPT-IN (WF_GLUE_CLUSTER=1), measured (profiles/r02ax_summary.txt): 70B bs16/8K
+    // clusters for long rows when the rows alone leave most SMs idle: OPT-IN (WF_GLUE_CLUSTER=1), measured: 70B bs16/8K
     // 19.84 -> 19.73 ms, bs8/4K 10.74 -> 10.56; forced on shorter rows it loses — 2B bs64/4K 5.10 -> 5.39 ms, 8B bs16/2K 3.05 -> 3.27: a cluster
     // launch and its three cluster barriers cost more than the second half of a 4096..6912-element row
     static const int cl_env = getenv("WF_GLUE_CLUSTER") ? atoi(getenv("WF_GLUE_CLUSTER")) : 0;

@@ -5,7 +5,7 @@
 // E is the largest matrix of the step (657 MB for the 2B model: more bytes than all ternary layers together), read once:
 // the kernel is HBM-bound and everything here exists to keep the stream running.  The mma.sync kernel (glue.cu) reaches 93 % of
 // the HBM peak at batch 1 but 65 % at batch 64: every warp re-reads the whole 64-token activation tile through ldmatrix (80 KB of
-// shared-memory reads per 24 KB weight stage, profiles/r01c_full_lmhead_bs64).  Here the tensor core reads both operands straight
+// shared-memory reads per 24 KB weight stage).  Here the tensor core reads both operands straight
 // from shared memory and nothing else touches them:
 //   * persistent CTA per SM, 6 warps: 4 epilogue (one per TMEM lane quarter), 1 TMA producer, 1 MMA issuer;
 //   * a stage = 64 k of 128 vocab rows (16 KB) + 64 k of 64 tokens (8 KB), both by cp.async.bulk.tensor.2d with the 128-byte
@@ -266,7 +266,7 @@ void lm_head_tc_init_attrs() {
 
 bool lm_head_tc_usable(int B, int V, int K, const void* h, const void* E) {
     // from 17 tokens: measured 134.7 -> 108.1 us at batch 32 and 156.0 -> 117.4 us at batch 64 (2B: 657 MB), but 110.8 -> 118.0 us at batch 16,
-    // where the mma.sync kernel's 16-token tile is cheap enough (profiles/r02aa_summary.txt)
+    // where the mma.sync kernel's 16-token tile is cheap enough
     return B > 16 && B <= LT2_TOK && K % LT2_KC == 0 && ((uintptr_t)h & 15) == 0 && ((uintptr_t)E & 15) == 0 && V >= 1;
 }
 

@@ -1,4 +1,4 @@
-// Activation quantisation (north-star item 2) and the RMSNorm that precedes it.
+// Activation quantisation and the RMSNorm that precedes it.
 //
 // Reference arithmetic: quantize_activations_i8, tests/test_bitnet_core.py:139-146 (copy of the
 // missing sgl_kernel/quantization/bitnet.py); rms_norm, scripts/direct_inference_full.py:181-184.

@@ -1,4 +1,4 @@
-// Tensor-parallel exchange over NVLink peer memory (north-star item 6).
+// Tensor-parallel exchange over NVLink peer memory.
 //
 // One process per GPU.  Every rank owns one "comm" allocation (cudaMalloc, exported with cudaIpcGetMemHandle and
 // opened by the peers) that holds the buffers other ranks write INTO:

@@ -2,7 +2,7 @@
 reference module (its Python is preserved verbatim in the reference's tests/test_bitnet_core.py:139-167
 and legacy/benchmark/test_sglang_bitnet_kernel.py:44-101), executed by the sm_100a kernels.
 
-Semantics kept from the SIMD kernel the server uses (SURVEY.md H2):
+Semantics kept from the SIMD kernel the server uses:
   * packed weights are the BLOCKED I2_S layout u8 [N, K/4];
   * bitnet_gemv / bitnet_gemm return  scale * sum_k (w+1) * a  in fp32 — the caller subtracts
     scale * sum(a) (scripts/direct_inference_full.py:204-206);

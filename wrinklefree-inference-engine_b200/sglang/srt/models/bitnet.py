@@ -1,4 +1,4 @@
-"""`sglang.srt.models.bitnet` of the reference's fork on the B200 kernels (SURVEY §8f rank 4).
+"""`sglang.srt.models.bitnet` of the reference's fork on the B200 kernels.
 
 The fork's file is not in the scrape; its surface is pinned by the reference's own tests and scripts:
   * `_pack_ternary_weights(w) -> (u8 [N, K/4] blocked I2_S, scale[1])`      tests/test_vllm_cpu_stub.py:234-247

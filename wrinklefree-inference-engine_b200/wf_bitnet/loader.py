@@ -1,4 +1,4 @@
-"""Checkpoint loader for the decode engine (SURVEY §8f rank 1).
+"""Checkpoint loader for the decode engine.
 
 The reference loads one `model.safetensors` and repacks every projection with Python loops
 (`DirectBitNetInference._preprocess_weights`, scripts/direct_inference_full.py:116-163: HF `[N/4, K]` u8 ->

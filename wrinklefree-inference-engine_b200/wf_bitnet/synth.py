@@ -1,4 +1,4 @@
-"""Seeded synthetic BitNet models (random-init ternary weights), SURVEY.md §8(d).
+"""Seeded synthetic BitNet models (random-init ternary weights).
 
 weights: ternary uniform over {-1,0,1} (as scripts/benchmark_kernels.py:35, extern/BitNet/gpu/test.py:43),
 weight_scale ~ U(0.5, 2.5), norm gammas 1 + 0.1 N(0,1), embeddings N(0, 0.02) bf16.

@@ -1,4 +1,4 @@
-"""Tensor-parallel host layer (north-star item 6): weight sharding and the one-off IPC handle exchange.
+"""Tensor-parallel host layer: weight sharding and the one-off IPC handle exchange.
 
 One process per GPU (torchrun).  torch.distributed is plumbing only: it carries the 64-byte CUDA IPC handles of the
 ranks' exchange buffers once; the per-step all-gathers / all-reduces are peer-memory stores and REDs issued by the

@@ -5,7 +5,7 @@ shapes): `BitNetLinearNative` (:28-78), `pack_ternary_weights` (:81-112),
 `extract_packed_weight_and_scale` (:115-162), `patch_model_with_native_kernels` (:165-210),
 `benchmark_kernels` (:213-268).
 
-Differences that are deliberate (SURVEY.md §3C, H2, H9):
+Differences that are deliberate:
   * weights are packed in the kernel's BLOCKED I2_S layout (the reference file packs LSB-sequentially,
     which only its Python fallback understands) and kept resident in the b200_tile_v1 GPU layout;
   * the Sigma-a correction is applied (fused in the GEMV epilogue), so forward() returns the true
