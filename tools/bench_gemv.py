@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Kernel-level ternary GEMV bandwidth (BASELINE.json metric "ternary GEMV HBM GB/s vs peak"), in the style of the
+"""Kernel-level ternary GEMV bandwidth, in the style of the
 reference's scripts/benchmark_kernels.py:28-66: bytes = N*K/4 + M*K + out per call, but the calls rotate over > L2 worth
 of weight copies (wf_bench_gemv).  One JSON line per (shape, M, variant)."""
 import argparse, ctypes as C, json, sys
@@ -10,7 +10,7 @@ for p in (str(ROOT), str(ROOT / "wrinklefree-inference-engine_b200")):
 from wf_bitnet import _lib
 from wf_bitnet._lib import check, lib
 
-SHAPES = {   # SURVEY Appendix B; fused matrices as the engine stores them
+SHAPES = {   # fused matrices as the engine stores them
     "2b_qkv": (3840, 2560), "2b_o": (2560, 2560), "2b_gateup": (13824, 2560), "2b_down": (2560, 6912),
     "8b_qkv": (6144, 4096), "8b_gateup": (28672, 4096), "8b_down": (4096, 14336),
     "70b_qkv": (10240, 8192), "70b_gateup": (57344, 8192), "70b_down": (8192, 28672),

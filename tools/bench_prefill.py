@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""BASELINE config 3: BitNet-2B-4T-shaped prefill, 8 x 2048 tokens (M = 16384) through the ternary linears of one
+"""BitNet-2B-4T-shaped prefill, 8 x 2048 tokens (M = 16384) through the ternary linears of one
 layer on the tcgen05 int8 path.  Prints one JSON line: int8 TOP/s per linear and per layer, next to the int8
 tensor-pipe peak measured on the same box with torch._int_mm (cuBLASLt) at 8192^3."""
 import argparse

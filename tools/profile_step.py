@@ -2,7 +2,7 @@
 """One decode step of the BitNet-2B-4T-shaped engine bracketed by cudaProfilerStart/Stop, for ncu:
 
     ncu --profile-from-start off --metrics gpu__time_duration.sum --clock-control none --csv \
-        --log-file gpurun_out/launches_bs64.csv python tools/profile_step.py --batch 64 --ctx 4096
+        --log-file launches_bs64.csv python tools/profile_step.py --batch 64 --ctx 4096
 
 Without ncu it prints the CUDA-event time of the same step (ms), so the plain run doubles as the
 "exited 0 without ncu" gate of B200_PROFILING.md.
