@@ -54,7 +54,6 @@ struct TcParams {
     int w_layout;
     int M, N, K, KB;
     int tiles_n, tiles_m;
-    int dbg;   // timing experiments only (WF_TC_DBG, bit mask): 1 = epilogue skips math/stores, 2 = also the TMEM loads, 4 = unpack warps skip the TMEM stores, 8 = no activation TMA
     // batched-decode form (launch_gemm_tc_red): the K dimension is cut into `splitk` equal runs of KBs k-blocks, one CTA
     // tile each, and the epilogue adds the raw accumulators into a global fp32 buffer (exact: integers < 2^24) instead
     // of storing a finished output — the consumer phase of the decode step applies scales / residual / norm.
@@ -181,7 +180,6 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
                     const int kg = ks * KBs + k_part0 + kb;
                     const int s = it % TC_STAGES;
                     mbar_wait(&empty_bar[s], (uint32_t)(((it / TC_STAGES) & 1) ^ 1));   // the slot's products are done
-                    if (p.dbg & 8) { mbar_arrive(&full_bar[s]); continue; }  // timing experiment: no activation traffic
                     mbar_expect_tx(&full_bar[s], TC_STAGE_BYTES);
                     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                                  ::"r"(ring + s * TC_STAGE_BYTES), "l"(&tmap_q), "r"(kg * TC_BK), "r"(m_blk * TC_BN), "r"(smem_u32(&full_bar[s])) : "memory");
@@ -325,7 +323,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
                         } while (!ok);
                     }
                     tc_fence_after();
-                    if (!(p.dbg & 4)) TC_ST32(tbase + slot * TC_A_COLS, v);              // (dbg 4: timing experiment without the TMEM stores)
+                    TC_ST32(tbase + slot * TC_A_COLS, v);
                     pending = full0 + slot * 8;
                     slot += NU;
                     if (slot >= TC_STAGES) { slot -= TC_STAGES; par ^= 1u; }
@@ -352,7 +350,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
         const bool obf16 = (mode == WF_OUT_LINEAR) && p.ep.out_dtype == WF_BF16;
         const int ncols = relu2 ? p.N / 2 : p.N;
         const bool red = p.red_acc != nullptr;
-        const bool fast_mode = !red && (mode == WF_OUT_LINEAR || mode == WF_OUT_COMPAT_F32) && !relu2 && !resid && !p.dbg;
+        const bool fast_mode = !red && (mode == WF_OUT_LINEAR || mode == WF_OUT_COMPAT_F32) && !relu2 && !resid;
         const bool fold_ws = fast_mode && mode == WF_OUT_LINEAR && p.ep.nseg <= 1;
         const float ws_all = fold_ws ? w_scale_of(p.ep, 0) : 1.f;
         if (red) pdl_wait_prior();   // the accumulator buffer was cleared by an earlier phase of the step
@@ -398,16 +396,13 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
 #pragma unroll 1
             for (int c = 0; c < TC_EP_TOKS / 32; ++c) {
                 uint32_t v[32];
-                if (!(p.dbg & 2)) {
-                    TC_LD32(tmem + lane_base + buf * TC_BN + th * TC_EP_TOKS + c * 32, v);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                }
+                TC_LD32(tmem + lane_base + buf * TC_BN + th * TC_EP_TOKS + c * 32, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (c == TC_EP_TOKS / 32 - 1) {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&tempty_bar[buf]);
                 }
-                if (p.dbg) continue;
                 const int m0 = mw0 + c * 32;
                 if (fast) {
                     // full tile, plain output: ~9 issued instructions per token (LDS.64, I2F, 3 FMUL, FADD, F2F for bf16, pointer add, STG);
@@ -569,7 +564,6 @@ static int launch_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t 
     p.tiles_m = (a->M + TC_BN - 1) / TC_BN;
     p.ep = ep;
     p.splitk = 1; p.KBs = p.KB; p.ksplit = 1; p.red_acc = nullptr; p.red_ld = 0; p.l2_ahead = 0;
-    { const char* d = getenv("WF_TC_DBG"); p.dbg = d ? atoi(d) : 0; }
     const int total = p.tiles_n * p.tiles_m, sms = sm_count();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(total < sms ? total : sms);
