@@ -198,8 +198,8 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
         const uint32_t a_tmem0 = __shfl_sync(0xffffffffu, tmem, 0) + TC_A_COL0;
         const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
         const uint32_t tfull0 = smem_u32(&tfull_bar[0]);
-        // One ELECTED thread runs the whole loop (elect.sync, not `lane == 0`: ptxas then knows the region is single-threaded
-        // and issues the tcgen05 instructions straight from uniform registers instead of one ELECT waterfall loop each).
+        // One ELECTED thread runs the whole loop (elect.sync, not `lane == 0`, under which a stage's
+        // issue took about 500 clk).
         uint32_t elected;
         asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
         if (elected) {
