@@ -173,3 +173,12 @@ def test_loader_shards_like_tp_shard_weights():
         loader._shard(t, "o", 0, 2)          # 96 bytes do not split into two runs of whole 32-byte blocks
     with pytest.raises(ValueError):
         loader._shard(t, "q", 0, 5)
+
+
+@pytest.mark.parametrize("m,n,k,tcgen05", [(16, 2560, 2560, False), (17, 2560, 1024, False), (32, 6912, 1920, False), (17, 2560, 2048, True), (33, 2560, 4096, True),
+                                           (64, 6912, 2560, False), (96, 6912, 2560, True), (64, 2560, 2560, True), (192, 2560, 2560, False), (256, 2560, 2560, True),
+                                           (64, 2560, 2048, False), (128, 6912, 1024, False), (192, 6912, 1024, True), (192, 2560, 3968, False), (16384, 2560, 6912, True)])
+def test_which_product_kernel_a_shape_takes(m, n, k, tcgen05):
+    """Either side of the lines between the mma.sync and the tcgen05 ternary product (148 SMs); only the former asks for a workspace."""
+    from wf_bitnet import _lib
+    assert (_lib.lib().wf_bitnet_gemm_workspace_bytes(m, n, k) == 0) == tcgen05

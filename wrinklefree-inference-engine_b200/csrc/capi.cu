@@ -76,13 +76,20 @@ extern "C" size_t wf_linear_workspace_bytes(int M, int N, int K) {
     return gemm_mma_workspace_bytes(M, N, K);
 }
 
-// tcgen05 or mma.sync.  From 17 tokens the mma.sync kernel takes its 32- and 64-token tiles and is bound by the legacy int8 pipe: 14336 x 4096 with
-// 48 tokens 38.3 us against 16.5, 4096 x 14336 with 17 tokens 18 against 14.7, 6912 x 2560 with 1987 tokens 157 against 50.  Below, its weight
-// stream is as fast and its launch cheaper (2560 x 2560, 9 tokens: 8.4 us against 10.4).  The same holds for its 64-token tiles on short-K matrices
-// while they fit in about one wave (6912 x 2560, 33 tokens: 10.4 against 12.4; 2560 x 2560, 192 tokens: 12.5 against 14.5).
+// tcgen05 or mma.sync, by what was measured with weights from HBM over K 1024 .. 4096, N 1024 .. 13824, 17 .. 384 tokens (us, mma.sync / tcgen05):
+//   * below 17 tokens the mma.sync kernel's weight stream is as fast and its launch cheaper (2560 x 2560, 9 tokens 8.4 / 10.4);
+//   * up to 32 tokens its 32-token tiles split K from K = 2048 on and lose by that (2560 x 1024, 17 tokens 5.0 / 6.9; 2560 x 2048 10.0 / 7.2);
+//   * beyond, its 64 x 64 tiles split K from K = 4096 on (2560 x 4096, 64 tokens 16.7 / 9.7).  Below they take one round of the SMs after the other, at
+//     2 us + K / 350 for the first and more than half of that for the next: while one round does (two below K = 2048), they are faster than a tcgen05 tile
+//     whose K range too few CTAs share (6912 x 2560, 64 tokens 9.7 / 11.5; 2560 x 2560, 192 tokens 9.6 / 12.9; 6912 x 1024, 128 tokens 7.8 / 10.5), and
+//     slower where four or more do (2560 x 2560, 64 tokens 9.2 / 8.3) or where they need another round (6912 x 2560, 96 tokens 14.8 / 12.4).
 static bool tc_is_faster(int M, int N, int K) {
     if (M < 17) return false;
-    return !(M > 32 && K <= 2560 && (long long)M * N * K <= 1300000000LL);
+    if (M <= 32) return K >= 2048;
+    if (K >= 4096) return true;
+    const long long sms = sm_count(), small = (long long)((N + 63) / 64) * ((M + 63) / 64), large = (long long)((N + 127) / 128) * ((M + 127) / 128);
+    if (K < 2048) return small > 2 * sms;
+    return small > sms || (K >= 2560 && 4 * large <= sms);
 }
 
 static int ternary_linear(const wf_linear_args* a, const float* w_scales_host, void* stream) {

@@ -336,7 +336,6 @@ constexpr int FR_WARPS = 8;
 template <int NT, int WK, int U, int OCC, bool CF32>
 __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g) {
     constexpr int TILES = FR_WARPS / WK;                  // 16-row tiles per block
-    constexpr int C = 4;                                  // independent sums, added in float at the end
     __shared__ float part[FR_WARPS][NT * 8][16 + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g4 = lane >> 2, t4 = lane & 3;
     const int tile = warp / WK, kw = warp % WK;
@@ -348,11 +347,9 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
     bool x_ok[NT];
 #pragma unroll
     for (int j = 0; j < NT; ++j) { const int m = j * 8 + g4; x_ok[j] = m < g.M; xa[j] = A + (size_t)(x_ok[j] ? m : 0) * g.lda + 8 * t4; }
-    float acc[C][NT][4];
+    float acc[NT][4];
 #pragma unroll
-    for (int c = 0; c < C; ++c)
-#pragma unroll
-        for (int j = 0; j < NT; ++j) acc[c][j][0] = acc[c][j][1] = acc[c][j][2] = acc[c][j][3] = 0.f;
+    for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     const int blocks = (g.K + 31) / 32;                   // block i of this warp: steps of 64 k (two blocks) dealt to the WK warps in turn
     for (int i0 = 0; ; i0 += U) {
@@ -374,8 +371,11 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
                 const uint32_t x0[2] = {x[u][j].x, x[u][j].y}, x1[2] = {x[u][j].z, x[u][j].w};
-                mma_bf16_16816(acc[u % C][j], f0, x0);
-                mma_bf16_16816(acc[u % C][j], f1, x1);
+                float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_bf16_16816(s0, f0, x0);
+                mma_bf16_16816(s1, f1, x1);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[j][e] += s0[e] + s1[e];
             }
         }
     }
@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) part[warp][j * 8 + 2 * t4 + (e & 1)][g4 + 8 * (e >> 1)] = (acc[0][j][e] + acc[1][j][e]) + (acc[2][j][e] + acc[3][j][e]);
+        for (int e = 0; e < 4; ++e) part[warp][j * 8 + 2 * t4 + (e & 1)][g4 + 8 * (e >> 1)] = acc[j][e];
     __syncthreads();
     for (int i = threadIdx.x; i < TILES * NT * 8 * 16; i += FR_WARPS * 32) {
         const int r = i & 15, m = (i >> 4) % (NT * 8), t = (i >> 4) / (NT * 8);
