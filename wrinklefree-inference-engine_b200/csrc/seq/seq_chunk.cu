@@ -15,9 +15,10 @@
 // sequence) 307 -> 202 us (32); eight warps with half the rows each 287 and 257 us (both in one pass).  Left: the chain of a chunk, about 3000 clk of products, one exchange of
 // partial sums and two barriers.  Error against 64 bits in float32 layers up to 1500 tokens long: 3.6e-7 to 5.6e-7, as token by token.
 // Numbers that are not finite: in a product with the zeros of T and B, or as a sum of two tf32 numbers, an infinity or a NaN would reach tokens and rows
-// that never meet it (and the rounding of cr_split would take the bit pattern of a NaN past the exponent, to zero).  So chunk_prep_kernel marks a chunk in
-// which anything it reads or forms is not finite, the scan watches its state and U, and such a chunk is taken token by token, with the meaning that the
-// recurrence has there.  Decays are taken to be at most one, so that finite values do not overflow between the two watched places.
+// that never meet it (and the rounding of cr_split takes the bit pattern of a NaN past the exponent, to zero).  So the preparation marks the heads in which
+// anything that it reads or forms is not finite, the scan those in which U or the state is not, and chunk_redo_kernel takes the marked portions again from
+// their start, token by token as the recurrence is stated: a launch of blocks that leave at once where nothing is marked (about 2 us; deciding chunk by
+// chunk inside the scan cost it 15 to 30 %).
 #include "seq_kernels.cuh"
 
 namespace wf {
@@ -36,19 +37,19 @@ struct ChunkView {
     const float *qkv, *beta, *decay; int ld, q_off, k_off, v_off;
     float* rec;
     int nchunks;
+    int *redo, cols;               // [sequence][head][CR_COLS columns]: marked; zero between launches
 };
+
+// x * 0 summed up: zero while everything is finite, NaN from the first infinity or NaN on
+__device__ __forceinline__ void cr_watch(float& w, float x) { w = fmaf(x, 0.f, w); }
 
 // one of the two passes over segments of SCAN_CHUNK tokens in parallel (recurrences linear in the state): pass 1 leaves each segment's own end state (from a
 // zero one) and, with one decay per head, the product of its decays; pass 3 reads the segments' start states, chained by scan_prefix_kernel; 0: whole portions
 struct Segments { int pass = 0, n = 1; float *local = nullptr, *prod = nullptr; const float* start = nullptr; };
 
 // a record: [T 256][B 256] then, decay per row: [c_j q_j 16 DS][c_j k_j 16 DS][D(j, 16) k_j 16 DS][c_16 DS]; one decay: [c_j 16][D(j, 16) 16][c_16, padding]
-// (DS: the key rows, padded to 64 or 128), and at cr_mark a number other than zero where the chunk is to be taken token by token
-__host__ __device__ constexpr int cr_rec_floats(int DS, bool vec) { return vec ? 512 + (3 * CR + 1) * DS + 4 : 512 + 48; }
-__host__ __device__ constexpr int cr_mark(int DS, bool vec) { return vec ? DS : 36; }      // within the last part of a record and of a stage (CrStage::G)
-
-// x * 0 summed up: zero while everything is finite, NaN from the first infinity or NaN on
-__device__ __forceinline__ void cr_watch(float& w, float x) { w = fmaf(x, 0.f, w); }
+// (DS: the key rows, padded to 64 or 128)
+__host__ __device__ constexpr int cr_rec_floats(int DS, bool vec) { return vec ? 512 + (3 * CR + 1) * DS : 512 + 48; }
 
 // transposed sum over 16 lanes: v[t] of all of them -> the sum of t = p for lane p
 __device__ __forceinline__ float cr_reduce(float (&v)[CR], int p) {
@@ -179,8 +180,8 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_prep_kernel(Batch b, DeltaDi
         if (tid == CR - 1) rec[544] = cum;
         cr_watch(watch, cum); cr_watch(watch, suf);
     }
-    const int mark = __syncthreads_or(!(watch == 0.f));
-    if (tid == 0) rec[512 + (VEC ? 3 * CR * DS : 0) + cr_mark(DS, VEC)] = mark ? 1.f : 0.f;
+    if (!(watch == 0.f))
+        for (int z = 0; z < w.cols; ++z) w.redo[((size_t)sq * D.H + h) * w.cols + z] = 1;
 }
 
 __device__ __forceinline__ void cr_split(float x, uint32_t& hi, uint32_t& lo) {
@@ -212,79 +213,9 @@ template <int DS, bool VEC, bool DELTA> struct CrStage {
     static constexpr int QS = DS + 8, KS = DS + 4;        // row strides: pairs of rows 8 tokens apart, single rows 2 tokens apart, each without bank conflicts
     static constexpr int TS = 24;                         // of T and B
     static constexpr int T = 0, B = T + (DELTA ? CR * TS : 0), Q = B + CR * TS, K = Q + CR * QS, N = K + (DELTA ? CR * QS : 0), G = N + CR * KS,
-                         FLOATS = G + (VEC ? DS + 4 : 48);    // G: c_16 per row, or [c_j][D(j, 16)][c_16]; the mark
+                         FLOATS = G + (VEC ? DS : 48);    // G: c_16 per row, or [c_j][D(j, 16)][c_16]
 };
 constexpr int CR_RS = 24;                                 // row stride of the partial sums [16 columns][16 tokens]
-
-// A chunk's tokens one by one, as the recurrence states them, rows straight from memory.  sv: the thread's part of the state, laid out as in
-// chunk_scan_kernel.  Not inlined: its registers would come out of the scan's.
-struct CrTokens {
-    const float *row, *decay, *beta;      // of the chunk's first token: qkv row; this head's decay (row) and beta (null: 1)
-    float* o;                             // this head's output row, or null: only the state is wanted
-    int n, ld, k_at, q_at, v_at, H, d, dv, dvs, col0;
-    float o_scale;
-};
-template <int DS, bool VEC, bool DELTA>
-__device__ __noinline__ void cr_by_token(const CrTokens a, float* sv, float* red) {
-    constexpr int NT = DS / (8 * CR_WARPS);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, row0 = warp * 8 * NT, c0 = a.col0 + g;
-    float s[NT][4];
-#pragma unroll
-    for (int i = 0; i < NT * 4; ++i) s[i >> 2][i & 3] = sv[i];
-#pragma unroll 1
-    for (int tk = 0; tk < a.n; ++tk) {
-        const float *row = a.row + (size_t)tk * a.ld, *kr = row + a.k_at, *qr = row + a.q_at, *gr = a.decay + (size_t)tk * a.H * (VEC ? a.d : 1);
-        const float gg = VEC ? 1.f : gr[0], bt = a.beta ? a.beta[(size_t)tk * a.H] : 1.f;
-        float r0 = 0.f, r1 = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int r = row0 + 8 * nt + 2 * t + e;
-                if (r >= a.d) continue;
-                if (VEC) { s[nt][e] *= gr[r]; s[nt][2 + e] *= gr[r]; }
-                if (DELTA) { r0 = fmaf(s[nt][e], kr[r], r0); r1 = fmaf(s[nt][2 + e], kr[r], r1); }
-            }
-        if (DELTA) {
-            r0 += __shfl_xor_sync(0xffffffffu, r0, 1); r1 += __shfl_xor_sync(0xffffffffu, r1, 1);
-            r0 += __shfl_xor_sync(0xffffffffu, r0, 2); r1 += __shfl_xor_sync(0xffffffffu, r1, 2);
-            __syncthreads();                              // what lay there has been read
-            if (t == 0) { red[warp * CR_COLS + g] = r0; red[warp * CR_COLS + g + 8] = r1; }
-            __syncthreads();
-            r0 = r1 = 0.f;
-#pragma unroll
-            for (int k = 0; k < CR_WARPS; ++k) { r0 += red[k * CR_COLS + g]; r1 += red[k * CR_COLS + g + 8]; }
-        }
-        const float v0 = c0 >= a.dvs ? 0.f : c0 == a.dv ? 1.f : row[a.v_at + c0], v1 = c0 + 8 >= a.dvs ? 0.f : c0 + 8 == a.dv ? 1.f : row[a.v_at + c0 + 8];
-        const float u0 = bt * (v0 - gg * r0), u1 = bt * (v1 - gg * r1);
-        float o0 = 0.f, o1 = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int r = row0 + 8 * nt + 2 * t + e;
-                if (r >= a.d) continue;
-                s[nt][e] = fmaf(kr[r], u0, gg * s[nt][e]);
-                s[nt][2 + e] = fmaf(kr[r], u1, gg * s[nt][2 + e]);
-                if (a.o) { o0 = fmaf(s[nt][e], qr[r], o0); o1 = fmaf(s[nt][2 + e], qr[r], o1); }
-            }
-        if (!a.o) continue;
-        o0 += __shfl_xor_sync(0xffffffffu, o0, 1); o1 += __shfl_xor_sync(0xffffffffu, o1, 1);
-        o0 += __shfl_xor_sync(0xffffffffu, o0, 2); o1 += __shfl_xor_sync(0xffffffffu, o1, 2);
-        float* ro = red + CR_WARPS * CR_COLS;
-        __syncthreads();
-        if (t == 0) { ro[warp * CR_COLS + g] = o0; ro[warp * CR_COLS + g + 8] = o1; }
-        __syncthreads();
-        if (tid < CR_COLS && a.col0 + tid < a.dvs) {
-            float x = 0.f;
-#pragma unroll
-            for (int k = 0; k < CR_WARPS; ++k) x += ro[k * CR_COLS + tid];
-            a.o[(size_t)tk * a.H * a.dvs + a.col0 + tid] = x * a.o_scale;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < NT * 4; ++i) sv[i] = s[i >> 2][i & 3];
-}
 
 template <int DS, bool VEC, bool DELTA>
 __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
@@ -330,7 +261,7 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
                 if (DELTA) cr_cp16(dst + L::K + (r0 + r) * L::QS + c, x + CR * DS);
                 cr_cp16(dst + L::N + (r0 + r) * L::KS + c, x + 2 * CR * DS);
             }
-            if (tid < DS / 4 + 1) cr_cp16(dst + L::G + tid * 4, src + 512 + 3 * CR * DS + tid * 4);
+            if (tid < DS / 4) cr_cp16(dst + L::G + tid * 4, src + 512 + 3 * CR * DS + tid * 4);
         } else {
             const float* row = w.qkv + (size_t)(start + ch * CR + r0) * w.ld + kh * D.d + c;
             const int left = c < D.d ? len - ch * CR - r0 : 0;
@@ -364,15 +295,7 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
                 if (!DELTA && e < 2) bn[n][e] = w.beta && tk < len ? w.beta[(size_t)(start + tk) * D.H + h] : 1.f;
             }
     };
-    // whether this thread's part of the state has left the finite numbers
-    auto state_bad = [&]() {
-        float x = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) cr_watch(x, s[nt][e]);
-        return !(x == 0.f);
-    };
+    float watch[4] = {0.f, 0.f, 0.f, 0.f};
     stage(0);
     values(0);
     for (int ch = 0; ch < nch; ++ch) {
@@ -383,20 +306,9 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[n][e] = DELTA ? vn[n][e] : vn[n][e] * bn[n][e & 1];
         cp_async_wait<0>();
-        const bool lost = __syncthreads_or(state_bad());  // chunk ch has landed; everyone is done with the other half and the partial sums
+        __syncthreads();                                  // chunk ch has landed; everyone is done with the other half and the partial sums
         if (ch + 1 < nch) { stage(ch + 1); values(tok0 + CR); }
         const float* st = sm + (ch & 1) * L::FLOATS;
-        if (!VEC) prod *= st[L::G + 32];
-        bool plain = lost || st[L::G + cr_mark(DS, VEC)] != 0.f;
-        float u[2][4];
-        auto total = [&](int part, int n, int c) {
-            const float* p = red + (part * CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t;
-            float2 x = *reinterpret_cast<const float2*>(p);
-#pragma unroll
-            for (int k = 1; k < CR_WARPS; ++k) { const float2 y = *reinterpret_cast<const float2*>(p + k * 2 * CR_COLS * CR_RS); x.x += y.x; x.y += y.y; }
-            return x;
-        };
-        if (!plain) {
         if (DELTA || sg.pass != 1) {
         // ---- this warp's rows' share of S^T q and R; the small terms in accumulators of their own, so that no product waits for the one before it
         float oq[2][4], rk[2][4], oql[2][4], rkl[2][4];
@@ -435,6 +347,14 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
             }
         }
         if (DELTA || sg.pass != 1) __syncthreads();
+        auto total = [&](int part, int n, int c) {
+            const float* p = red + (part * CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t;
+            float2 x = *reinterpret_cast<const float2*>(p);
+#pragma unroll
+            for (int k = 1; k < CR_WARPS; ++k) { const float2 y = *reinterpret_cast<const float2*>(p + k * 2 * CR_COLS * CR_RS); x.x += y.x; x.y += y.y; }
+            return x;
+        };
+        float u[2][4];
         if (DELTA) {                                      // every warp forms all of U: it is the update's operand
 #pragma unroll
             for (int n = 0; n < 2; ++n)
@@ -458,25 +378,10 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
 #pragma unroll
                 for (int e = 0; e < 4; ++e) u[n][e] = v[n][e];
         }
-        float x = 0.f;                                    // every warp holds the same U and sees the same
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) cr_watch(x, u[n][e]);
-        plain = __any_sync(0xffffffffu, !(x == 0.f));
-        }
-        if (plain) {
-            const size_t at = (size_t)(start + tok0) * D.H + h;
-            const CrTokens a{w.qkv + (size_t)(start + tok0) * w.ld, w.decay + at * (VEC ? D.d : 1), w.beta ? w.beta + at : nullptr, sg.pass == 1 ? nullptr : o + at * dvs,
-                             min(CR, len - tok0), w.ld, w.k_off + kh * D.d, w.q_off + kh * D.d, w.v_off + h * D.dv, D.H, D.d, D.dv, dvs, col0, D.o_scale};
-            float sv[NT * 4];
-#pragma unroll
-            for (int i = 0; i < NT * 4; ++i) sv[i] = s[i >> 2][i & 3];
-            cr_by_token<DS, VEC, DELTA>(a, sv, red);
-#pragma unroll
-            for (int i = 0; i < NT * 4; ++i) s[i >> 2][i & 3] = sv[i];
-            continue;
-        }
+            for (int e = 0; e < 4; ++e) cr_watch(watch[2 * n + (e & 1)], u[n][e]);
         if (warp < 2 && sg.pass != 1) {                                   // the read-out of 8 tokens each
             const int n = warp;
             float out[4], add[4] = {0.f, 0.f, 0.f, 0.f};
@@ -495,6 +400,7 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
                 if (tk < len && c < dvs) o[((size_t)(start + tk) * D.H + h) * dvs + c] = (out[e] + add[e]) * D.o_scale;
             }
         }
+        if (!VEC) prod *= st[L::G + 32];
         // ---- state update: the chunk's own sum from zero, so that the state itself is only ever rounded to nearest (the matrix unit's sums are cut off)
         if (!VEC) {
 #pragma unroll
@@ -533,13 +439,99 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
             s[nt][2] = fmaf(s[nt][2], ge.x, ds[nt][2]); s[nt][3] = fmaf(s[nt][3], ge.y, ds[nt][3]);
         }
     }
+    // a state that has left the finite numbers does not come back: looked at once
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) cr_watch(watch[e], s[nt][e]);
+    const int lost = __syncthreads_or(!((watch[0] + watch[1]) + (watch[2] + watch[3]) == 0.f));
+    if (lost && tid == 0) w.redo[((size_t)sq * D.H + h) * w.cols + blockIdx.z] = 1;
     if (sg.pass == 3) return;                             // scan_prefix_kernel has left the end states
+    if (sg.pass == 0 && (lost || w.redo[((size_t)sq * D.H + h) * w.cols + blockIdx.z])) return;      // the slot keeps the start state for chunk_redo_kernel
     float* S1 = sg.pass ? sg.local + entry : state + (size_t)b.seq_slot[sq] * slot_stride + (size_t)h * D.d * dvs;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) { bool ok; const size_t i = at_state(nt, e, ok); if (ok) S1[i] = s[nt][e]; }
     if (!VEC && sg.pass && blockIdx.z == 0 && tid == 0) sg.prod[(size_t)(seq0 / SCAN_CHUNK + sq + seg) * D.H + h] = prod;
+}
+
+// The marked portions again, token by token (see above), a block per (sequence, head, 16 columns); their start state is still in the slot, or, with segments,
+// that of the first one.  A thread holds the part of the state that it holds in chunk_scan_kernel; rows come straight from memory.
+template <int DS, bool VEC, bool DELTA>
+__global__ void __launch_bounds__(CR_THREADS) chunk_redo_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
+    constexpr int NT = DS / (8 * CR_WARPS);
+    __shared__ float rs[CR_WARPS][CR_COLS], os[CR_WARPS][CR_COLS];
+    const int sq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, row0 = warp * 8 * NT;
+    int* mark = w.redo + ((size_t)sq * D.H + h) * w.cols + blockIdx.z;
+    if (!*mark) return;
+    const int col0 = blockIdx.z * CR_COLS, c0 = col0 + g, dvs = D.dv + D.ones_col, kh = h / (D.H / D.Hk), start = b.seq_start[sq], len = b.seq_len[sq];
+    float* S1 = state + (size_t)b.seq_slot[sq] * slot_stride + (size_t)h * D.d * dvs;
+    const float* S0 = sg.start ? sg.start + ((size_t)(start / SCAN_CHUNK + sq) * D.H + h) * D.d * dvs : S1;
+    float s[NT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = row0 + 8 * nt + 2 * t + (e & 1), c = c0 + 8 * (e >> 1);
+            s[nt][e] = r < D.d && c < dvs ? S0[(size_t)r * dvs + c] : 0.f;
+        }
+#pragma unroll 1
+    for (int tk = 0; tk < len; ++tk) {
+        const size_t at = (size_t)(start + tk) * D.H + h;
+        const float *row = w.qkv + (size_t)(start + tk) * w.ld, *kr = row + w.k_off + kh * D.d, *qr = row + w.q_off + kh * D.d, *vr = row + w.v_off + h * D.dv;
+        const float *gr = w.decay + at * (VEC ? D.d : 1), gg = VEC ? 1.f : gr[0], bt = w.beta ? w.beta[at] : 1.f;
+        float r0 = 0.f, r1 = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = row0 + 8 * nt + 2 * t + e;
+                if (r >= D.d) continue;
+                if (VEC) { s[nt][e] *= gr[r]; s[nt][2 + e] *= gr[r]; }
+                if (DELTA) { r0 = fmaf(s[nt][e], kr[r], r0); r1 = fmaf(s[nt][2 + e], kr[r], r1); }
+            }
+        if (DELTA) {
+            r0 += __shfl_xor_sync(0xffffffffu, r0, 1); r1 += __shfl_xor_sync(0xffffffffu, r1, 1);
+            r0 += __shfl_xor_sync(0xffffffffu, r0, 2); r1 += __shfl_xor_sync(0xffffffffu, r1, 2);
+            if (t == 0) { rs[warp][g] = r0; rs[warp][g + 8] = r1; }
+            __syncthreads();                              // (the next token writes rs behind this token's second barrier)
+            r0 = r1 = 0.f;
+#pragma unroll
+            for (int k = 0; k < CR_WARPS; ++k) { r0 += rs[k][g]; r1 += rs[k][g + 8]; }
+        }
+        const float v0 = c0 >= dvs ? 0.f : c0 == D.dv ? 1.f : vr[c0], v1 = c0 + 8 >= dvs ? 0.f : c0 + 8 == D.dv ? 1.f : vr[c0 + 8];
+        const float u0 = bt * (v0 - gg * r0), u1 = bt * (v1 - gg * r1);
+        float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = row0 + 8 * nt + 2 * t + e;
+                if (r >= D.d) continue;
+                s[nt][e] = fmaf(kr[r], u0, gg * s[nt][e]); o0 = fmaf(s[nt][e], qr[r], o0);
+                s[nt][2 + e] = fmaf(kr[r], u1, gg * s[nt][2 + e]); o1 = fmaf(s[nt][2 + e], qr[r], o1);
+            }
+        o0 += __shfl_xor_sync(0xffffffffu, o0, 1); o1 += __shfl_xor_sync(0xffffffffu, o1, 1);
+        o0 += __shfl_xor_sync(0xffffffffu, o0, 2); o1 += __shfl_xor_sync(0xffffffffu, o1, 2);
+        if (!DELTA) __syncthreads();                      // the token before has been written out
+        if (t == 0) { os[warp][g] = o0; os[warp][g + 8] = o1; }
+        __syncthreads();
+        if (tid < CR_COLS && col0 + tid < dvs) {
+            float x = 0.f;
+#pragma unroll
+            for (int k = 0; k < CR_WARPS; ++k) x += os[k][tid];
+            o[at * dvs + col0 + tid] = x * D.o_scale;
+        }
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = row0 + 8 * nt + 2 * t + (e & 1), c = c0 + 8 * (e >> 1);
+            if (r < D.d && c < dvs) S1[(size_t)r * dvs + c] = s[nt][e];
+        }
+    if (tid == 0) *mark = 0;
 }
 
 template <int DS, bool VEC, bool DELTA>
@@ -550,7 +542,11 @@ int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const floa
     static DevOnce once;
     if (once.need() && cuda_check(cudaFuncSetAttribute(chunk_scan_kernel<DS, VEC, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "chunk shared memory")) return WF_ERR_CUDA;
     Segments sg;
-    const int cols = (D.dv + D.ones_col + CR_COLS - 1) / CR_COLS;
+    const int cols = w.cols;
+    auto redo = [&]() {
+        chunk_redo_kernel<DS, VEC, DELTA><<<dim3(b.nseq, D.H, cols), CR_THREADS, 0, s>>>(b, D, w, state, slot_stride, o, sg);
+        return launch_check(cudaGetLastError(), "chunk_redo");
+    };
     auto scan_pass = [&](int pass) {
         sg.pass = pass;
         chunk_scan_kernel<DS, VEC, DELTA><<<dim3(b.nseq * sg.n, D.H, cols), CR_THREADS, smem, s>>>(b, D, w, state, slot_stride, o, sg);
@@ -560,12 +556,16 @@ int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const floa
     // passes cost half as much work again.  us, whole -> segments: 4 heads 128 x 64, 1024 tokens 87 -> 40, 300 tokens 35 -> 36; 16 heads, 2048 tokens 168 -> 95;
     // 40 heads (160 blocks) 224 -> 202; two sequences of 841 and 1207, 16 heads (128 blocks) 109 -> 102, 40 heads (320 blocks) 185 -> 206.
     if (DELTA || !scan->local || b.max_len < 4 * SCAN_CHUNK || b.n / SCAN_CHUNK + b.nseq + 1 > scan->chunks || 2LL * b.nseq * D.H * cols >= 3LL * sm_count())
-        return scan_pass(0);
+    {
+        if (int rc = scan_pass(0)) return rc;
+        return redo();
+    }
     sg.n = (b.max_len + SCAN_CHUNK - 1) / SCAN_CHUNK;
     sg.local = scan->local; sg.start = scan->start; sg.prod = scan->prod;
     if (int rc = scan_pass(1)) return rc;
     if (int rc = launch_scan_prefix(b, D, decay, state, slot_stride, scan, sg.n, s)) return rc;
-    return scan_pass(3);
+    if (int rc = scan_pass(3)) return rc;
+    return redo();
 }
 
 }  // namespace
@@ -576,10 +576,12 @@ size_t chunk_workspace_floats(const DeltaDims& D, int max_step_tokens, int slots
     return (size_t)(max_step_tokens / CR + slots + 1) * D.H * rec;
 }
 
+size_t chunk_redo_words(const DeltaDims& D, int slots) { return (size_t)slots * D.H * ((D.dv + 1 + CR_COLS - 1) / CR_COLS); }
+
 bool chunk_usable(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const ScanWorkspace* scan) {
     const int qo = D.q_off >= 0 ? D.q_off : 0, ko = D.k_off >= 0 ? D.k_off : D.Hk * D.d;
     return scan && scan->rec && b.max_len >= 2 * CR && D.d <= 128 && D.d % 4 == 0 && ld % 4 == 0 && qo % 4 == 0 && ko % 4 == 0 && ((uintptr_t)qkv & 15) == 0 && D.H <= 65535 &&
-           chunk_workspace_floats(D, b.n, b.nseq) <= scan->rec_floats;
+           chunk_workspace_floats(D, b.n, b.nseq) <= scan->rec_floats && chunk_redo_words(D, b.nseq) <= scan->redo_words;
 }
 
 int launch_chunk_recurrence(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const float* beta, const float* decay, float* state, size_t slot_stride,
@@ -587,6 +589,7 @@ int launch_chunk_recurrence(const Batch& b, const DeltaDims& D, const float* qkv
     ChunkView w;
     w.qkv = qkv; w.beta = beta; w.decay = decay; w.ld = ld;
     w.q_off = D.q_off >= 0 ? D.q_off : 0; w.k_off = D.k_off >= 0 ? D.k_off : D.Hk * D.d; w.v_off = D.v_off >= 0 ? D.v_off : 2 * D.Hk * D.d;
+    w.redo = scan->redo; w.cols = (D.dv + D.ones_col + CR_COLS - 1) / CR_COLS;
     w.rec = scan->rec; w.nchunks = (b.max_len + CR - 1) / CR;
 #define CR_PICK(vec, delta) (D.d <= 64 ? cr_launch<64, vec, delta>(b, D, w, decay, state, slot_stride, o, s, scan) : cr_launch<128, vec, delta>(b, D, w, decay, state, slot_stride, o, s, scan))
     if (D.no_delta) return D.vec_decay ? CR_PICK(true, false) : CR_PICK(false, false);

@@ -1191,6 +1191,8 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     size_t max_gate = 1, max_decay = 1, max_gfull = 0, max_afull = 0, max_scan = 0, max_qfull = 0, max_qrank = 0;
     size_t max_talk_ws = 0;          // mixed heads: one unsplit partial result for every sequence, and room for one per SM
     bool any_mlstm = false;
+    size_t max_redo = 0;
+    auto rec_for = [&](const DeltaDims& D) { max_rec = std::max(max_rec, chunk_workspace_floats(D, T, c.slots)); max_redo = std::max(max_redo, chunk_redo_words(D, c.slots)); };
     bool own = true;                 // false while a tied layer is laid out: it allocates and names nothing, its weights are its source's
     auto walloc = [&](void** ptr, size_t count) -> int { return own ? dalloc_t(e, ptr, count) : WF_OK; };
     auto name = [&](const std::string& n, void* dst, size_t count) { if (own) add_tensor(e, n, dst, count); };
@@ -1329,7 +1331,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             L.st_S = st; st += (size_t)l.heads * l.dim * (l.vdim + 1);
             L.st_m = st; st += l.heads;
             max_scan = std::max(max_scan, (size_t)l.heads * l.dim * (l.vdim + 1));
-            max_rec = std::max(max_rec, chunk_workspace_floats(DeltaDims{l.heads, l.heads, l.dim, l.vdim}, T, c.slots));
+            rec_for(DeltaDims{l.heads, l.heads, l.dim, l.vdim});
             max_hv = std::max(max_hv, (size_t)l.heads * (l.vdim + 1));
             any_mlstm = true;
         } else if (l.type == WF_SEQ_GLA) {
@@ -1350,7 +1352,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             L.st_S = st; st += nk * l.vdim;
             max_decay = std::max(max_decay, nk);
             max_scan = std::max(max_scan, nk * l.vdim);
-            max_rec = std::max(max_rec, chunk_workspace_floats(DeltaDims{l.heads, l.heads, l.dim, l.vdim, 1}, T, c.slots));
+            rec_for(DeltaDims{l.heads, l.heads, l.dim, l.vdim, 1});
         } else if (l.type == WF_SEQ_SSD) {
             // [z | x | B | C | dt]: x, B and C are the convolved channels
             const size_t GN = (size_t)l.kv_heads * l.dim;
@@ -1367,13 +1369,13 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             L.st_S = st; st += (size_t)l.heads * l.dim * l.vdim;
             max_C = std::max(max_C, (size_t)L.C);
             max_scan = std::max(max_scan, (size_t)l.heads * l.dim * l.vdim);
-            max_rec = std::max(max_rec, chunk_workspace_floats(DeltaDims{l.heads, l.kv_heads, l.dim, l.vdim}, T, c.slots));
+            rec_for(DeltaDims{l.heads, l.kv_heads, l.dim, l.vdim});
         } else {
             // [q | k | v | gate (or its first factor) | write strength | decay (or its first factor)]
             const size_t nqk = (size_t)l.kv_heads * l.dim;
             L.C = (int)(2 * nqk + nv);
             L.n_decay = l.decay_channels ? l.heads * l.dim : l.heads;
-            max_rec = std::max(max_rec, chunk_workspace_floats(DeltaDims{l.heads, l.kv_heads, l.dim, l.vdim, l.decay_channels ? 1 : 0}, T, c.slots));
+            rec_for(DeltaDims{l.heads, l.kv_heads, l.dim, l.vdim, l.decay_channels ? 1 : 0});
             const size_t g_rows = l.gate_rank > 0 ? (size_t)l.gate_rank : nv, a_rows = l.decay_rank > 0 ? (size_t)l.decay_rank : (size_t)L.n_decay;
             L.g_col = L.C; L.b_col = (int)(L.C + g_rows); L.a_col = L.b_col + l.heads;
             L.np = (int)(L.a_col + a_rows);
@@ -1560,7 +1562,11 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
 #undef TRY
     // What only the faster forms of prompt portions need comes last, each form's part as a whole, and only where that leaves three quarters of what is free
     // by then: an engine that fits without them still fits, and takes the forms that need none.
-    if (e->chunk_rec && max_rec && T >= 2 * CHUNK_TOKENS && dalloc_spare(e, (void**)&e->scan.rec, max_rec * sizeof(float))) e->scan.rec_floats = max_rec;
+    if (e->chunk_rec && max_rec && T >= 2 * CHUNK_TOKENS && dalloc_spare(e, (void**)&e->scan.rec, (max_rec + max_redo) * sizeof(float))) {
+        e->scan.rec_floats = max_rec;
+        e->scan.redo = (int*)(e->scan.rec + max_rec); e->scan.redo_words = max_redo;
+        if (cuda_check(cudaMemsetAsync(e->scan.redo, 0, max_redo * 4, e->stream), "marks")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
+    }
     if (max_kvx) {                             // enough positions for sequences of several full steps; longer ones keep the form that reads the latents
         const size_t rows = (size_t)std::min<long long>((long long)c.max_pages * c.page_size, 4LL * T);
         auto place = [](size_t& off, size_t elems) { const size_t at_ = off; off += (elems + 127) / 128 * 128; return at_; };        // 256-byte aligned

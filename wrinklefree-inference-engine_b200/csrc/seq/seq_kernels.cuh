@@ -251,7 +251,7 @@ int launch_delta_prep(int dt, const DeltaDims& D, int n, float* qkv, int ld, con
 // + local_c, the recurrence being linear in the state), then every chunk again from its start state for the outputs.
 constexpr int SCAN_CHUNK = 128;
 struct ScanWorkspace { float* local = nullptr; float* start = nullptr; float* prod = nullptr; int chunks = 0;
-                       float* rec = nullptr; size_t rec_floats = 0; };   // rec: records of the 16-token form (chunk_workspace_floats); chunks: entries of H * d * dv floats each; prod: H (vec_decay: H * d) floats per chunk
+                       float* rec = nullptr; size_t rec_floats = 0; int* redo = nullptr; size_t redo_words = 0; };   // rec, redo: records and marks of the 16-token form (chunk_workspace_floats, chunk_redo_words; the marks zero between launches); chunks: entries of H * d * dv floats each; prod: H (vec_decay: H * d) floats per chunk
 // gated linear attention: decay[i, c] = sigmoid(z)^(1 / tau), z = a2[c, :] . a1[i, :] + bias[c], c < nout; a1 float [n, rank] (ld), a2 T [nout, rank];
 // products, logarithm and exponential in float
 int launch_gla_decay(int dt, int n, int rank, int nout, const float* a1, int ld, const void* a2, const void* bias, float tau, float* decay, cudaStream_t s);
@@ -263,6 +263,7 @@ int launch_scan_prefix(const Batch& b, const DeltaDims& D, const float* decay, f
 // launch_delta_rule takes it where it can; chunk_workspace_floats: what a step of at most max_step_tokens over `slots` sequences needs of ScanWorkspace::rec.
 constexpr int CHUNK_TOKENS = 16;
 size_t chunk_workspace_floats(const DeltaDims& D, int max_step_tokens, int slots);
+size_t chunk_redo_words(const DeltaDims& D, int slots);
 bool chunk_usable(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const ScanWorkspace* scan);
 int launch_chunk_recurrence(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const float* beta, const float* decay, float* state, size_t slot_stride,
                             float* o, cudaStream_t s, const ScanWorkspace* scan);
