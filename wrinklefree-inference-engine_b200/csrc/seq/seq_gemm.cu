@@ -327,7 +327,10 @@ void gemv_launch(const GemmArgs& g, const PairArgs& pa, int rows, int ny, cudaSt
 // side, so that a loaded weight serves all rows in two MMAs per 32 k instead of being multiplied row by row.  A lane loads 16 consecutive bytes of a
 // row: the four lanes of a row hold k 8 t .. 8 t + 7, and weights and activations are permuted over k alike, so no shuffle is needed.  The WK
 // warps of a tile take 64-k steps in turn (a short, wide product has too few rows to cover the machine otherwise) and meet in shared memory.
-// Every warp keeps four sums apart and all partial sums are added in float, which holds the error at the fused-multiply-add kernel's (4e-7 to 1e-6).
+// The matrix unit cuts off what it adds.  Up to 8 rows (before: the multiply-add kernel) it therefore never adds more than 16 products: those sums meet
+// pairwise in float, the warps' in double, and the error against 64 bits stays below the multiply-add kernel's (2-norm, K = 1024 / 2560 / 6912 / 28672: 5.7e-8 / 6.6e-8 /
+// 7.5e-8 / 9.4e-8 against 7.0e-8 / 8.4e-8 / 1.2e-7 / 2.4e-7; at K = 64, where every order rounds once or twice, 4.4e-8 against 4.0e-8).  From 9 rows on (before: one
+// running sum in gemm_mma_kernel, 2.7e-6 at K = 2560) four running sums per warp are close enough: 1.1e-7.
 // Bound: the weight stream, by latency on small matrices.  Measured with 8 rows against gemv_rows_kernel: 1024 x 2304 23.1 -> 9.3 us, 2560 x 6912
 // 64.6 -> 12.5, 13824 x 2560 43.7 -> 14.8, 128256 x 2560 298 -> 102; with 16 rows against gemm_mma_kernel: 2560 x 6912 131 -> 12.6.
 constexpr int FR_WARPS = 8;
@@ -336,6 +339,7 @@ constexpr int FR_WARPS = 8;
 template <int NT, int WK, int U, int OCC, bool CF32>
 __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g) {
     constexpr int TILES = FR_WARPS / WK;                  // 16-row tiles per block
+    constexpr int C = NT == 1 ? 1 : 4;                    // running sums
     __shared__ float part[FR_WARPS][NT * 8][16 + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g4 = lane >> 2, t4 = lane & 3;
     const int tile = warp / WK, kw = warp % WK;
@@ -347,9 +351,11 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
     bool x_ok[NT];
 #pragma unroll
     for (int j = 0; j < NT; ++j) { const int m = j * 8 + g4; x_ok[j] = m < g.M; xa[j] = A + (size_t)(x_ok[j] ? m : 0) * g.lda + 8 * t4; }
-    float acc[NT][4];
+    float acc[C][NT][4];
 #pragma unroll
-    for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) acc[c][j][0] = acc[c][j][1] = acc[c][j][2] = acc[c][j][3] = 0.f;
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     const int blocks = (g.K + 31) / 32;                   // block i of this warp: steps of 64 k (two blocks) dealt to the WK warps in turn
     for (int i0 = 0; ; i0 += U) {
@@ -365,34 +371,50 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
 #pragma unroll
             for (int j = 0; j < NT; ++j) x[u][j] = ok && x_ok[j] ? *reinterpret_cast<const uint4*>(xa[j] + k) : zero;
         }
+        float sum[U][4];                                      // NT = 1
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint32_t f0[4] = {a[u].x, b[u].x, a[u].y, b[u].y}, f1[4] = {a[u].z, b[u].z, a[u].w, b[u].w};
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
                 const uint32_t x0[2] = {x[u][j].x, x[u][j].y}, x1[2] = {x[u][j].z, x[u][j].w};
+                if (NT > 1) {
+                    mma_bf16_16816(acc[u % C][j], f0, x0);
+                    mma_bf16_16816(acc[u % C][j], f1, x1);
+                    continue;
+                }
                 float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
                 mma_bf16_16816(s0, f0, x0);
                 mma_bf16_16816(s1, f1, x1);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[j][e] += s0[e] + s1[e];
+                for (int e = 0; e < 4; ++e) sum[u][e] = s0[e] + s1[e];
             }
+        }
+        if (NT == 1) {
+#pragma unroll
+            for (int half = U / 2; half >= 1; half /= 2)
+#pragma unroll
+                for (int u = 0; u < half; ++u)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) sum[u][e] += sum[u + half][e];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[0][0][e] += sum[0][e];
         }
     }
     // acc: rows g4 (0, 1) and g4 + 8 (2, 3), activation rows 2 t4 and 2 t4 + 1
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) part[warp][j * 8 + 2 * t4 + (e & 1)][g4 + 8 * (e >> 1)] = acc[j][e];
+        for (int e = 0; e < 4; ++e) part[warp][j * 8 + 2 * t4 + (e & 1)][g4 + 8 * (e >> 1)] = C == 1 ? acc[0][j][e] : (acc[0][j][e] + acc[C / 2][j][e]) + (acc[C / 4][j][e] + acc[C - 1][j][e]);
     __syncthreads();
     for (int i = threadIdx.x; i < TILES * NT * 8 * 16; i += FR_WARPS * 32) {
         const int r = i & 15, m = (i >> 4) % (NT * 8), t = (i >> 4) / (NT * 8);
         const int n = (blockIdx.x * TILES + t) * 16 + r;
         if (n >= g.N || m >= g.M) continue;
-        float v = 0.f;
+        double all = 0.;
 #pragma unroll
-        for (int w = 0; w < WK; ++w) v += part[t * WK + w][m][r];
-        v = epilogue_f(g.ep, v);
+        for (int w = 0; w < WK; ++w) all += part[t * WK + w][m][r];
+        const float v = epilogue_f(g.ep, (float)all);
         if (CF32) ((float*)g.C)[(size_t)m * g.ldc + n] = v;
         else ((__nv_bfloat16*)g.C)[(size_t)m * g.ldc + n] = __float2bfloat16_rn(v);
     }
