@@ -114,8 +114,10 @@ __device__ __forceinline__ float at_ex2(float x) { float y; asm("ex2.approx.ftz.
 
 // One row of one head, key by key over what it sees, with a whole warp: a lane per key for the scores, then a lane per 4 output columns.  Not inlined: its
 // registers would come out of the kernel's.
-__device__ __noinline__ void at_row(const AtParams& p, const int32_t* bt, int row0, int kvh, int head, int tok, int pos) {
+__device__ __noinline__ void at_row(const Batch& b, const AtParams& p, int head, int tok) {
     const GqaDims& D = p.D;
+    const int kvh = blockIdx.y, sq = b.tok_seq[tok], pos = b.tok_pos[tok], row0 = p.key_row ? p.key_row[sq] : 0;
+    const int32_t* bt = p.key_row ? nullptr : p.block_table + (size_t)b.seq_slot[sq] * p.max_blocks;
     const int lane = threadIdx.x & 31;
     const __nv_bfloat16* q = p.qn + ((size_t)tok * D.H + head) * D.d;
     const float slope2 = D.dist_exp > 0.f ? exp2f(-D.dist_exp * (float)(head + 1) / (float)D.H) * LOG2E : 0.f, scale2 = D.scale * LOG2E;
@@ -165,7 +167,7 @@ __device__ __noinline__ void at_row(const AtParams& p, const int32_t* bt, int ro
 
 // SPLIT: the weights as a two-term bf16 split (grouped-query attention); without it rounded to bf16 (latent attention)
 template <bool SPLIT>
-__global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const Batch b,
+__global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ Batch b,
                                                                 const __grid_constant__ AtParams p) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t q_full[2], k_full[2], k_empty[2], v_full[2], v_empty[2], v_fixed, s_full[2], p_full[2], o_full[2], drained;
@@ -460,8 +462,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
                 __syncwarp();
                 for (uint32_t redo = __ballot_sync(0xffffffffu, r_ok && !(watch == 0.f) && l * 0.f == 0.f); redo; redo &= redo - 1) {
                     const int r = __ffs(redo) - 1;
-                    at_row(p, p.key_row ? nullptr : p.block_table + (size_t)b.seq_slot[sq] * p.max_blocks, p.key_row ? p.key_row[sq] : 0, kvh, __shfl_sync(0xffffffffu, head, r),
-                           __shfl_sync(0xffffffffu, tok, r), __shfl_sync(0xffffffffu, pos, r));
+                    at_row(b, p, __shfl_sync(0xffffffffu, head, r), __shfl_sync(0xffffffffu, tok, r));
                     __syncwarp();
                 }
             } else ok = false;
