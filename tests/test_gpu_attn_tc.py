@@ -186,3 +186,18 @@ def test_latent_sizes_without_a_tensor_core_form_keep_the_plain_kernel(monkeypat
     model = build(cfg, FO.random_weights(cfg, 2), 16, {})
     assert "latent.expand_gemm" not in latent_groups(model, 0, 600)
     model.close()
+
+
+@pytest.mark.parametrize("window", [1, 130, 300])
+def test_windowed_latent_form_with_expanded_keys(window, monkeypatch):
+    import test_gpu_karusun as K
+    monkeypatch.setenv("WF_SEQ_ATTN_MMA", "4")
+    cfg = K.config([K.lat(heads=5, dim=40, rot_dim=16, vdim=24, kv_rank=80, window=window)], width=64, vocab=40, groups=1, taps=2)
+    w = K.make_weights(cfg, 8)
+    model = K.build(cfg, w, "bfloat16", max_tokens=1024, page_size=16, max_step_tokens=512)
+    assert "latent.expand_gemm" in latent_groups(model, 0, 40)
+    x = inputs([500], 64, 9)[0]
+    P = {k: torch.from_numpy(v).double() for k, v in K.O.sub(w, "l0.mix.").items()}
+    want = K.O.latent_attention(torch.from_numpy(x).double(), P, cfg["layers"][0]["mixer"], 1e-6).numpy()
+    check(model, [x], [[260], [3], [237]], [want], 64)
+    model.close()

@@ -90,3 +90,23 @@ def test_native_calls_equal_those_through_ctypes(tmp_path):
     theirs = np.load(tmp_path / "r.npz")
     for i, a in enumerate(mine):
         assert np.array_equal(a, theirs[f"arr_{i}"]), i
+
+
+@pytest.mark.gpu
+def test_calls_on_two_streams_keep_to_their_own_workspaces():
+    """Products whose K range is split meet in a workspace: calls side by side on two streams give the bits of calls one after another."""
+    native()
+    g = torch.Generator().manual_seed(5)
+    w = (torch.randint(0, 256, (2560, 640), generator=g, dtype=torch.uint8) & 0xAA).cuda()
+    xs = [torch.randint(-127, 128, (m, 2560), generator=g, dtype=torch.int8).cuda() for m in (1, 12)]
+    want = [torch.ops.sgl_kernel.bitnet_gemm(w, x, 0.01) for x in xs]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = [[], []]
+    for _ in range(50):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got[i].append(torch.ops.sgl_kernel.bitnet_gemm(w, xs[i], 0.01))
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert all(torch.equal(y, want[i]) for y in got[i])

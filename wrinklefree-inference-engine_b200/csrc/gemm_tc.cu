@@ -2,8 +2,8 @@
 //
 //   S[m,n] = sum_k code[n,k] * a[m,k],  code = w+1 in {0,1,2} (u8), a int8, exact int32 accumulation
 //   (what bitnet_gemm computes row by row with ggml_vec_dot_i2_i8_s, extern/BitNet/src/ggml-bitnet-mad.cpp:94-186;
-//    signature src/wrinklefree_inference/kernels/bitnet_patch.py:73).  Used where the shape is a real dense
-//   contraction (M >= 128 tokens: prefill, 8 x 2048 tokens => 6.8e13 int8 MACs for the 2B shape).
+//    signature src/wrinklefree_inference/kernels/bitnet_patch.py:73).  Used from 17 tokens on where it is the
+//   faster form (capi.cu); a prefill of 8 x 2048 tokens is 6.8e13 int8 MACs for the 2B shape.
 //
 // B200 mapping (one persistent CTA per SM, 4 + 4*NU + 2 warps, warp-specialised):
 //   * D tile = 128 weight rows (UMMA M = TMEM lanes) x 128 tokens (UMMA N), int32, double-buffered in TMEM

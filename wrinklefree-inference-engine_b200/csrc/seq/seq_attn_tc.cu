@@ -13,8 +13,8 @@
 // the scale was last fixed (exact: the sum carries the same scale).
 // What bounds it: per pair of 128 x 128 tiles the tensor cores take 6 x 128^3 multiply-adds (about 3060 clk, 2040 without the split) and the eight
 // softmax warps about 5 instructions per score (1280 issue slots of each SM quarter's share), hence the packed float pairs and the scale folded
-// into the exponent's multiply-add.  Measured, 2048 tokens causal, 20 heads of 128: grouped-query attention 181 -> 60 us (mma.sync kernel before),
-// latent attention 895 -> 58 us (one CTA per token before; plus 40 us for the expansion).
+// into the exponent's multiply-add.  Measured, 2048 tokens causal, 20 heads of 128: grouped-query attention 181 -> 67 us (mma.sync kernel before),
+// latent attention 895 -> 65 us (one CTA per token before; plus 24 us for the expansion).
 // Every wait is bounded: one that runs out records an error word that the host checks, and the CTA drains and leaves.
 // A value that is infinite or NaN meets the zero weights of the rows of its key tile that do not see it, too: a row whose sum of weights is finite and
 // whose output is not is taken again by its warp, over the keys that it sees (at_row).

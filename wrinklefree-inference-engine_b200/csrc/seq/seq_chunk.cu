@@ -11,9 +11,10 @@
 //     shared memory once per chunk.
 // What bounded the forms before: token by token, a chain of multiply-adds, shuffles and shared-memory reads of about 1000 clk per token; chunks on
 // the multiply-add units, shared-memory bandwidth (every thread of a column reads every key: 5 wavefronts per request, 450 us for the case below).
-// Measured at 2048 tokens: delta rule (20 heads, 128 x 128, two sequences) 569 -> 231 us (48 of them the preparation), state space (40 heads, 128 x 64, one
-// sequence) 307 -> 202 us (32); eight warps with half the rows each 287 and 257 us (both in one pass).  Left: the chain of a chunk, about 3000 clk of products, one exchange of
-// partial sums and two barriers.  Error against 64 bits in float32 layers up to 1500 tokens long: 3.6e-7 to 5.6e-7, as token by token.
+// Measured: delta rule (20 heads, 128 x 128, two sequences, 1801 tokens) 569 -> 236 us, state space (40 heads, 128 x 64, one sequence, 2048 tokens) 307 -> 213 us;
+// with eight warps of half the rows each 287 and 257 us (both in one pass).  Left: the chain of a chunk, about 3000 clk of products, one exchange of partial
+// sums and two barriers.  Error against 64 bits (2-norm of a mixer's output, up to 2048 tokens): in float32 engines 4.47e-7 against 4.36e-7 token by token (delta rule),
+// 3.35e-7 / 3.33e-7 (state space), 4.82e-7 / 4.94e-7 (matrix memory); float32 engines keep the token form all the same.  In bf16 engines both 2.05e-3, 1.67e-3, 1.66e-3.
 // Numbers that are not finite: in a product with the zeros of T and B, or as a sum of two tf32 numbers, an infinity or a NaN would reach tokens and rows
 // that never meet it (and the rounding of cr_split takes the bit pattern of a NaN past the exponent, to zero).  So the preparation marks the heads in which
 // anything that it reads or forms is not finite, the scan those in which U or the state is not, and chunk_redo_kernel takes the marked portions again from
