@@ -1,15 +1,20 @@
 """A bulk load that one CTA issues for a whole cluster must never meet another GPU's memory, and the kernels here also run in tensor-parallel processes:
-no source issues one (commits that signal several CTAs' barriers are another matter)."""
+every bulk copy in the sources is one of the forms that serve the issuing CTA (or pair) alone."""
 import re
 from pathlib import Path
 
 CSRC = Path(__file__).resolve().parents[1] / "wrinklefree-inference-engine_b200" / "csrc"
+QUALIFIERS = {"cp", "async", "bulk", "tensor", "1d", "2d", "3d", "4d", "5d", "prefetch", "L2", "global", "shared::cluster", "shared::cta", "mbarrier::complete_tx::bytes",
+              "cta_group::1", "cta_group::2", "commit_group", "wait_group", "read", "bulk_group"}
 
 
-def test_no_bulk_load_is_shared_by_a_cluster():
-    found = []
+def test_bulk_copies_serve_the_cta_that_issues_them():
+    found, seen = [], 0
     for p in sorted(CSRC.rglob("*.cu*")):
         for i, line in enumerate(p.read_text().splitlines(), 1):
-            if re.search(r"cp\.async\.bulk\S*multicast", line) or re.search(r"SM\d+_TMA_LOAD_MULTICAST", line):
-                found.append(f"{p.name}:{i}")
-    assert not found, found
+            for name in re.findall(r'"[^"]*?(cp\.async\.bulk[\w.:]*)', line):
+                seen += 1
+                extra = set(name.split(".")) - QUALIFIERS
+                if extra:
+                    found.append((f"{p.name}:{i}", extra))
+    assert seen and not found, found
