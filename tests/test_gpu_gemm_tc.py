@@ -142,3 +142,38 @@ def test_tc_shared_k_range(m, nk):
         u = torch.from_numpy(ref_dequant(packed[n // 2:], q, rs, np.float32(1.6), s)).to(torch.bfloat16)
         got = ops.ternary_linear(gu, n, k, cu(q), w_scale=torch.tensor([0.9, 1.6]).cuda(), relu2_mul=True, out_dtype=torch.bfloat16, **kw).cpu()
         assert torch.equal(got, torch.relu(g).square() * u)
+
+
+# 32 .. 256 tokens per tile of CTA pairs: one k-block, partial loads of four k-blocks, one and several rounds of tiles, rows and tokens that end inside a tile
+PAIR_SHAPES = [(256, 128, 40), (272, 640, 33), (131, 384, 190), (2560, 2560, 200), (6912, 2560, 75), (4090, 1152, 777), (6905, 2560, 1987), (2560, 6912, 1500),
+               (13824, 2560, 300)]
+
+
+@pytest.mark.parametrize("nkm", PAIR_SHAPES)
+def test_tc_pairs(nkm):
+    """Every kind of output on CTA pairs, both weight layouts, bit-equal to the mma.sync kernel; accumulators of a sample of rows equal to the oracle's."""
+    from wf_bitnet import ops
+    n, k, m = nkm
+    rng = np.random.default_rng(n + k + m)
+    q = torch.from_numpy(rng.integers(-128, 128, size=(m, k)).astype(np.int8)).cuda()
+    code = rng.integers(0, 3, size=(n, k // 128, 4, 32)).astype(np.uint8)
+    packed = (code[:, :, 0] << 6 | code[:, :, 1] << 4 | code[:, :, 2] << 2 | code[:, :, 3]).reshape(n, k // 4)
+    pi = cu(packed)
+    tile = ops.i2s_to_tile(pi)
+    rs, sc = q.int().sum(1).int(), torch.rand(m, device="cuda") + 0.5
+    rows = rng.choice(m, size=min(m, 24), replace=False)
+    want = O.gemm_i32_fast(packed, q.cpu().numpy()[rows], 0)
+    res = torch.randn(m, n, device="cuda").to(torch.bfloat16)
+    one, two = torch.tensor([0.3], device="cuda"), torch.tensor([0.3, 0.2], device="cuda")
+    lin = dict(mode="linear", rowsum=rs, act_scale=sc)
+    forms = [dict(mode="i32", rowsum=rs), dict(lin, w_scale=one, out_dtype=torch.float32), dict(lin, w_scale=one, out_dtype=torch.bfloat16),
+             dict(lin, w_scale=two, seg_end=[n // 2, n], out_dtype=torch.float32), dict(lin, w_scale=one, residual=res, out_dtype=torch.bfloat16)]
+    if n % 32 == 0:
+        forms += [dict(lin, w_scale=two, relu2_mul=True, out_dtype=torch.bfloat16), dict(lin, w_scale=two, relu2_mul=True, out_dtype=torch.float32)]
+    for layout, wt in (("i2s", pi), ("tile", tile)):
+        got = ops.ternary_linear(wt, n, k, q, layout=layout, mode="i32_plus1", algo=3).cpu().numpy()
+        assert np.array_equal(got[rows], want), layout
+        for f in forms:
+            a, b = (ops.ternary_linear(wt, n, k, q, layout=layout, algo=x, **f) for x in (3, 2))
+            assert torch.equal(a, b), (layout, list(f))
+    assert torch.equal(ops.bitnet_gemm(pi, q, 0.0123).cpu()[rows], torch.from_numpy(want.astype(np.float32) * np.float32(0.0123)))

@@ -3,7 +3,7 @@
 //   S[m,n] = sum_k code[n,k] * a[m,k],  code = w+1 in {0,1,2} (u8), a int8, exact int32 accumulation
 //   (what bitnet_gemm computes row by row with ggml_vec_dot_i2_i8_s, extern/BitNet/src/ggml-bitnet-mad.cpp:94-186;
 //    signature src/wrinklefree_inference/kernels/bitnet_patch.py:73).  Used from 17 tokens on where it is the
-//   faster form (capi.cu); a prefill of 8 x 2048 tokens is 6.8e13 int8 MACs for the 2B shape.
+//   faster form (capi.cu) for few tokens, which share a tile's K range over a cluster, for single rounds of whole tiles, and for the decode step.
 //
 // B200 mapping (one persistent CTA per SM, 4 + 4*NU + 2 warps, warp-specialised):
 //   * D tile = 128 weight rows (UMMA M = TMEM lanes) x 128 tokens (UMMA N), int32, double-buffered in TMEM
@@ -20,14 +20,11 @@
 //   * epilogue warps: tcgen05.ld 32x32b.x32 (lane = weight row, columns = tokens) -> the linear epilogue (Sigma-a
 //     correction, scales, residual, relu^2*up) in registers -> one store per token: a warp's 32 lanes are 32 consecutive n,
 //     so every store instruction is a full coalesced line and nothing is transposed through shared memory.
-// Shared memory is the binding resource of the main loop: TMA write + MMA read of the activation tile = 128 B/clk at the
-// 256-clk/stage tensor floor, i.e. all of an SM's shared-memory bandwidth.  Measured
-// with the epilogue's math and stores switched off the kernel runs 2.15 PTOP/s (374 clk per stage); an epilogue with a
-// shared-memory transpose and dependent per-token global loads cost 40 % on the short-K shapes.  The cta_group::2 form (each SM
-// holds half of the activation tile) is what would lift the 374-clk stage.
-#include "linear_common.cuh"
+// Measured with the epilogue's math and stores switched off the kernel runs 2.15 PTOP/s (374 clk per stage: an MMA of 128 x 128 x 32 takes 93 clk, 64 of
+// them work); an epilogue with a shared-memory transpose and dependent per-token global loads cost 40 % on the short-K shapes.  Wider tiles on CTA pairs
+// (gemm_tc_pair.cu) are the faster form wherever they fill the SMs; launch_gemm_tc chooses.
+#include "gemm_tc_common.cuh"
 #include "fused_common.cuh"
-#include <cuda.h>
 #include <stdlib.h>
 #include <string.h>
 
@@ -66,57 +63,6 @@ struct TcParams {
     int red_ld;
     EpiParams ep;
 };
-
-// ---- tcgen05 / TMA wrappers -------------------------------------------------------------------------------
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem desc]; u8 x s8 -> s32
-__device__ __forceinline__ void tc_mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(smem_u32(smem_dst)), "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar)) : "memory");
-}
-// K-major operand tile with 128-byte rows, 128B swizzle: 8-row groups are 1024 B apart
-__device__ __forceinline__ uint64_t tc_smem_desc_sw128(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3ffffu) >> 4);        // start address
-    d |= (uint64_t)1 << 16;                           // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                 // stride byte offset
-    d |= (uint64_t)1 << 46;                           // descriptor version (sm_100)
-    d |= (uint64_t)2 << 61;                           // SWIZZLE_128B
-    return d;
-}
-// instruction descriptor: D s32, A u8 (K-major), B s8 (K-major), N, M
-constexpr uint32_t tc_idesc(int m, int n) {
-    return (2u << 4) | (0u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-#define TC_ST32(taddr, v)                                                                                              \
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16," \
-                 "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"                                  \
-                 ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),   \
-                 "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),          \
-                 "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),        \
-                 "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory")
-
-#define TC_LD32(taddr, v)                                                                                              \
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"       \
-                 "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"                            \
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),      \
-                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), \
-                   "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]),           \
-                   "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),           \
-                   "=r"(v[30]), "=r"(v[31])                                                                             \
-                 : "r"(taddr) : "memory")
 
 // Every CTA loads its activation tiles itself: sharing them between the CTAs of a cluster by one load was worth 1 to 3 % on prompt shapes, but such a
 // load must not meet another GPU's memory, and tensor-parallel processes run this kernel too.
@@ -519,12 +465,10 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
 }
 
 // ---- host side --------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static EncodeTiledFn g_encode = nullptr;
 static DevOnce g_tc_attr;
 static int g_tc_nu = 0;
+EncodeTiledFn tc_encoder() { return g_encode; }
 
 void gemm_tc_init_attrs() {
     if (g_tc_attr.need()) {
@@ -654,12 +598,27 @@ static int launch_tc_split(const wf_linear_args* a, const EpiParams& ep, int ksp
     return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<NU, true>, tmap, p), "ternary_gemm_tc(split)");
 }
 
+// This file's forms against CTA pairs (gemm_tc_pair.cu), by what each is expected to take.  Measured over N 2560 .. 14336, K 2560 .. 14336, 20 .. 4000 tokens
+// (us, this file / pairs):
+//   * K shared by a cluster: 0.25 us a k-block, 0.1 us per token that a CTA finishes: 4096 x 14336, 48 tokens 15.7 / 27.8; 2560 x 6912, 128 tokens 13.6 / 17.1;
+//     but 6912 x 2560, 48 tokens 12.3 / 10.6;
+//   * one CTA a tile: 0.26 us a k-block and round of tiles, and 4.5 us for an epilogue with missing tokens: 2560 x 2560, 512 tokens 10.4 / 11.4;
+//     14336 x 4096, 128 tokens 13.3 / 13.9, 96 tokens 17.1 / 13.3; 2560 x 6912, 1024 tokens 31.2 / 20.9.
+// relu^2 * up without a cluster: its epilogue here takes 14 us a tile (13824 x 2560, 512 tokens 43 / 24).
+static double tile_time(int M, int KB, int tiles, int ksplit, int sms, bool relu2) {
+    if (ksplit > 1) return 6.7 + 0.25 * ((KB + ksplit - 1) / ksplit) + 0.1 * (M < TC_BN ? M : TC_BN) / ksplit;
+    const int rounds = (tiles + sms - 1) / sms;
+    return 4.7 + 0.26 * rounds * KB + (M % TC_EP_TOKS ? 4.5 : 0.) + (relu2 ? 10. * rounds : 0.);
+}
+
 int launch_gemm_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s) {
     gemm_tc_init_attrs();
     if (!g_encode) { set_error("gemm_tc: tcgen05 path unavailable (driver entry point / smem attribute)"); return WF_ERR_CUDA; }
     const int tiles = ((a->N + TC_BM - 1) / TC_BM) * ((a->M + TC_BN - 1) / TC_BN), sms = sm_count();
     int ksplit = 1;
     while (ksplit < 8 && tiles * ksplit * 2 <= sms && a->K / WF_QK >= ksplit * 2 * 4) ksplit *= 2;
+    const bool relu2 = ep.out_mode == WF_OUT_LINEAR && (ep.epi_flags & WF_EPI_RELU2_MUL);
+    if (gemm_tc_pair_time(a->M, a->N, a->K) < tile_time(a->M, a->K / WF_QK, tiles, ksplit, sms, relu2)) return launch_gemm_tc_pair(a, ep, s);
     if (ksplit > 1) return launch_tc_split(a, ep, ksplit, s);
     if (g_tc_nu == 1) return launch_tc<1>(a, ep, s);
     return g_tc_nu == 2 ? launch_tc<2>(a, ep, s) : launch_tc<3>(a, ep, s);
