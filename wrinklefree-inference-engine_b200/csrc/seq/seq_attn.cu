@@ -31,6 +31,7 @@ template <typename T, int MAXD>
 __global__ void __launch_bounds__(GP_MAXW * 32) gqa_prep_kernel(Batch b, GqaDims D, const float* __restrict__ proj, int ld, int k_off, int v_off, int g_off,
                                                                    const T* __restrict__ qb, const T* __restrict__ kb, const T* __restrict__ vb, float eps,
                                                                    PagedCache pc, T* __restrict__ qn, float* __restrict__ gate) {
+    pdl_enter();
     __shared__ float rot_c[GA_MAXROT], rot_s[GA_MAXROT];
     extern __shared__ float vec[];                        // [warps][32 * MAXD]
     __shared__ float scratch[33];
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(GP_MAXW * 32) gqa_prep_kernel(Batch b, GqaDims
 template <typename T>
 __global__ void __launch_bounds__(GA_WARPS * 32) gqa_attn_kernel(Batch b, GqaDims D, const T* __restrict__ qn, const float* __restrict__ gate, PagedCache pc,
                                                                    T* __restrict__ out) {
+    pdl_enter();
     extern __shared__ float sm[];   // [GA_WARPS][dv] partial sums, [GA_WARPS] m, [GA_WARPS] l
     const int i = blockIdx.x, h = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -206,6 +208,7 @@ constexpr int GT_KEYS = 32, GT_THREADS = 256;
 template <typename T>
 __global__ void __launch_bounds__(GT_THREADS) gqa_talk_attn_kernel(Batch b, GqaDims D, const T* __restrict__ qn, const float* __restrict__ gate, PagedCache pc,
                                                                    T* __restrict__ out) {
+    pdl_enter();
     extern __shared__ float sm[];
     float* sc = sm;                                   // [H][GT_KEYS] scores, then normalised weights
     float* mix = sc + D.H * GT_KEYS;                  // [H][GT_KEYS] mixed weights
@@ -311,7 +314,7 @@ int launch_gqa_prep(int dt, const Batch& b, const GqaDims& D, const float* proj,
     if (!D.v_is_k && (k_off >= 0) != (v_off >= 0)) { set_error("attention: keys and values are projected together or not at all"); return WF_ERR_INVALID; }
     const bool small = D.d <= 128 && D.dv <= 128;
     const int threads = 32 * (b.n <= sm_count() ? GP_MAXW : GA_WARPS);
-#define GP_LAUNCH(T, MD) gqa_prep_kernel<T, MD><<<b.n, threads, (size_t)threads * MD * sizeof(float), s>>>(b, D, proj, ld, k_off, v_off, g_off, (const T*)qb, (const T*)kb, (const T*)vb, eps, pc, (T*)qn, gate)
+#define GP_LAUNCH(T, MD) launch_pdl(gqa_prep_kernel<T, MD>, b.n, threads, (size_t)threads * MD * sizeof(float), s, b, D, proj, ld, k_off, v_off, g_off, (const T*)qb, (const T*)kb, (const T*)vb, eps, pc, (T*)qn, gate)
     if (dt == WF_BF16) { if (small) GP_LAUNCH(__nv_bfloat16, 4); else GP_LAUNCH(__nv_bfloat16, GA_MAXD); }
     else { if (small) GP_LAUNCH(float, 4); else GP_LAUNCH(float, GA_MAXD); }
 #undef GP_LAUNCH
@@ -330,14 +333,14 @@ int launch_gqa_attn(int dt, const Batch& b, const GqaDims& D, const void* qn, co
             cudaFuncSetAttribute(gqa_talk_attn_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
             cudaFuncSetAttribute(gqa_talk_attn_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         }
-        if (dt == WF_BF16) gqa_talk_attn_kernel<<<b.n, GT_THREADS, bytes, s>>>(b, D, (const __nv_bfloat16*)qn, gate, pc, (__nv_bfloat16*)out);
-        else gqa_talk_attn_kernel<<<b.n, GT_THREADS, bytes, s>>>(b, D, (const float*)qn, gate, pc, (float*)out);
+        if (dt == WF_BF16) launch_pdl(gqa_talk_attn_kernel<__nv_bfloat16>, b.n, GT_THREADS, bytes, s, b, D, (const __nv_bfloat16*)qn, gate, pc, (__nv_bfloat16*)out);
+        else launch_pdl(gqa_talk_attn_kernel<float>, b.n, GT_THREADS, bytes, s, b, D, (const float*)qn, gate, pc, (float*)out);
         return launch_check(cudaGetLastError(), "gqa_talk_attn");
     }
     dim3 grid(b.n, D.H);
     const size_t smem = ((size_t)GA_WARPS * D.dv + 2 * GA_WARPS) * sizeof(float);
-    if (dt == WF_BF16) gqa_attn_kernel<<<grid, GA_WARPS * 32, smem, s>>>(b, D, (const __nv_bfloat16*)qn, gate, pc, (__nv_bfloat16*)out);
-    else gqa_attn_kernel<<<grid, GA_WARPS * 32, smem, s>>>(b, D, (const float*)qn, gate, pc, (float*)out);
+    if (dt == WF_BF16) launch_pdl(gqa_attn_kernel<__nv_bfloat16>, grid, GA_WARPS * 32, smem, s, b, D, (const __nv_bfloat16*)qn, gate, pc, (__nv_bfloat16*)out);
+    else launch_pdl(gqa_attn_kernel<float>, grid, GA_WARPS * 32, smem, s, b, D, (const float*)qn, gate, pc, (float*)out);
     return launch_check(cudaGetLastError(), "gqa_attn");
 }
 

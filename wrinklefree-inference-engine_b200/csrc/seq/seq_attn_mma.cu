@@ -38,6 +38,7 @@ struct AmParams {
 template <int DKP, int DVP, bool DECODE, int NSTAGE, bool EXT>
 __global__ void __launch_bounds__(AM_THREADS, 3) gqa_attn_mma_kernel(Batch b, GqaDims D, const __nv_bfloat16* __restrict__ qn, const float* __restrict__ gate,
                                                                     PagedCache pc, __nv_bfloat16* __restrict__ out, AmParams ap) {
+    pdl_enter();
     constexpr int KS = DKP + 8, VS = DVP + 8;              // shared-memory row strides in elements
     constexpr int NKS = DKP / 16;                          // k-steps of the score product
     constexpr int NVT = DVP / 8;                           // n-tiles of the value product
@@ -373,6 +374,7 @@ __global__ void __launch_bounds__(AM_THREADS, 3) gqa_attn_mma_kernel(Batch b, Gq
 
 // one warp per (token, head): merge the key splits' partial results (maxima in units of log 2), apply the gate
 __global__ void gqa_attn_merge_kernel(GqaDims D, int rows, int splits, const float* __restrict__ part, const float* __restrict__ gate, __nv_bfloat16* __restrict__ out) {
+    pdl_enter();
     const int dv = D.dv, gate_elem = D.gate_elem;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
@@ -400,7 +402,7 @@ int am_launch(const Batch& b, const GqaDims& D, const void* qn, const float* gat
         attr_set = true;
     }
     dim3 grid(tiles, D.G, DECODE ? ap.splits : 1);
-    gqa_attn_mma_kernel<DKP, DVP, DECODE, NSTAGE, EXT><<<grid, AM_THREADS, smem, s>>>(b, D, (const __nv_bfloat16*)qn, gate, pc, (__nv_bfloat16*)out, ap);
+    launch_pdl(gqa_attn_mma_kernel<DKP, DVP, DECODE, NSTAGE, EXT>, grid, AM_THREADS, smem, s, b, D, (const __nv_bfloat16*)qn, gate, pc, (__nv_bfloat16*)out, ap);
     return launch_check(cudaGetLastError(), "gqa_attn_mma");
 }
 
@@ -454,7 +456,7 @@ int launch_gqa_attn_mma(const Batch& b, const GqaDims& D, const void* qn, const 
                      : (g_decode_stages == 3 ? am_dispatch<true, 3>(b, D, qn, gate, pc, out, ap, tiles, s) : am_dispatch<true, 2>(b, D, qn, gate, pc, out, ap, tiles, s));
     if (rc || ap.splits == 1) return rc;
     const int rows = b.n * D.H;
-    gqa_attn_merge_kernel<<<(rows + 3) / 4, 128, 0, s>>>(D, rows, ap.splits, workspace, gate, (__nv_bfloat16*)out);
+    launch_pdl(gqa_attn_merge_kernel, (rows + 3) / 4, 128, 0, s, D, rows, ap.splits, workspace, gate, (__nv_bfloat16*)out);
     return launch_check(cudaGetLastError(), "gqa_attn_merge");
 }
 

@@ -96,6 +96,7 @@ struct TalkPromptShared {
 template <int DKP, int DVP, int KT>
 __global__ void __launch_bounds__(TP_THREADS, 1) __cluster_dims__(TP_CLUSTER, 1, 1)
     talk_prompt_kernel(Batch b, GqaDims D, const __nv_bfloat16* __restrict__ qn, PagedCache pc, __nv_bfloat16* __restrict__ out, TalkParams tp) {
+    pdl_enter();
     using SH = TalkPromptShared<DKP, DVP, KT>;
     constexpr int KS = SH::KS, VS = SH::VS, PS = SH::PS, WS = SH::WS, NKS = DKP / 16, NVT = DVP / 8, NST = KT / 8;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -372,6 +373,7 @@ struct TalkDecodeShared {
 // MT: 16-row tiles of heads; IT: (key/value head, 16 value columns) items per warp
 template <int MT, int IT>
 __global__ void __launch_bounds__(TK_THREADS, MT * IT <= 10 ? 2 : 1) talk_decode_kernel(Batch b, GqaDims D, const __nv_bfloat16* __restrict__ qn, PagedCache pc, TalkParams tp) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
     const TalkDecodeShared sh(D, tp.kt);
     const int KT = tp.kt, KS = sh.kp + 8, VS = sh.vp + 8, SS = KT + 4, WS = KT + 8, nks = sh.kp / 16, rep = D.H / D.G;
@@ -552,6 +554,7 @@ __global__ void __launch_bounds__(TK_THREADS, MT * IT <= 10 ? 2 : 1) talk_decode
 // read once.  blockDim = (values rounded up to 32, slices of the sum)
 constexpr int TM_HEADS = 4;
 __global__ void talk_merge_kernel(Batch b, GqaDims D, int splits, const float* __restrict__ parts, __nv_bfloat16* __restrict__ out) {
+    pdl_enter();
     extern __shared__ __align__(16) float cf[];            // [splits][H][TM_HEADS] factors, then [slices][TM_HEADS][dv] partial sums
     const int sq = blockIdx.x, kv = blockIdx.y, rep = D.H / D.G, h0 = kv * rep + blockIdx.z * TM_HEADS, tok = b.seq_start[sq];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x, cnt = min(TM_HEADS, kv * rep + rep - h0);
@@ -619,7 +622,7 @@ int prompt_launch(const Batch& b, const GqaDims& D, const void* qn, const PagedC
     static DevOnce once;
     if (once.need() && cuda_check(cudaFuncSetAttribute(talk_prompt_kernel<DKP, DVP, KT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TK_SMEM), "attention shared memory")) return WF_ERR_CUDA;
     // every sequence's tokens are cut into tiles of tq; n / tq + nseq bounds their number (clusters beyond the last tile return at once)
-    talk_prompt_kernel<DKP, DVP, KT><<<TP_CLUSTER * (b.n / tp.tq + b.nseq), TP_THREADS, prompt_bytes<KT>(D), s>>>(b, D, (const __nv_bfloat16*)qn, pc, (__nv_bfloat16*)out, tp);
+    launch_pdl(talk_prompt_kernel<DKP, DVP, KT>, TP_CLUSTER * (b.n / tp.tq + b.nseq), TP_THREADS, prompt_bytes<KT>(D), s, b, D, (const __nv_bfloat16*)qn, pc, (__nv_bfloat16*)out, tp);
     return launch_check(cudaGetLastError(), "talk_prompt");
 }
 
@@ -645,7 +648,7 @@ template <int MT, int IT>
 int decode_launch(const Batch& b, const GqaDims& D, const void* qn, const PagedCache& pc, const TalkParams& tp, cudaStream_t s) {
     static DevOnce once;
     if (once.need() && cuda_check(cudaFuncSetAttribute(talk_decode_kernel<MT, IT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TK_SMEM), "attention shared memory")) return WF_ERR_CUDA;
-    talk_decode_kernel<MT, IT><<<dim3(b.nseq, tp.splits), TK_THREADS, TalkDecodeShared(D, tp.kt).bytes(D, tp.nst), s>>>(b, D, (const __nv_bfloat16*)qn, pc, tp);
+    launch_pdl(talk_decode_kernel<MT, IT>, dim3(b.nseq, tp.splits), TK_THREADS, TalkDecodeShared(D, tp.kt).bytes(D, tp.nst), s, b, D, (const __nv_bfloat16*)qn, pc, tp);
     return launch_check(cudaGetLastError(), "talk_decode");
 }
 
@@ -675,7 +678,7 @@ int launch_talk_attn_mma(const Batch& b, const GqaDims& D, const void* qn, const
         if (rc) return rc;
         const int rep = D.H / D.G;
         const dim3 block((D.dv + 31) / 32 * 32, 8);
-        talk_merge_kernel<<<dim3(b.nseq, D.G, (rep + TM_HEADS - 1) / TM_HEADS), block, ((size_t)tp.splits * D.H + (size_t)block.y * D.dv) * TM_HEADS * sizeof(float), s>>>(
+        launch_pdl(talk_merge_kernel, dim3(b.nseq, D.G, (rep + TM_HEADS - 1) / TM_HEADS), block, ((size_t)tp.splits * D.H + (size_t)block.y * D.dv) * TM_HEADS * sizeof(float), s, 
             b, D, tp.splits, workspace, (__nv_bfloat16*)out);
         return launch_check(cudaGetLastError(), "talk_merge");
     }

@@ -169,6 +169,7 @@ __device__ __noinline__ void at_row(const Batch& b, const AtParams& p, int head,
 template <bool SPLIT>
 __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ Batch b,
                                                                 const __grid_constant__ AtParams p) {
+    pdl_enter();
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t q_full[2], k_full[2], k_empty[2], v_full[2], v_empty[2], v_fixed, s_full[2], p_full[2], o_full[2], drained;
     __shared__ uint32_t tmem_base_s;
@@ -502,8 +503,8 @@ int at_launch(const Batch& b, const AtParams& p, bool split, const CUtensorMap& 
                              cuda_check(cudaFuncSetAttribute(attn_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM), "attention shared memory"))) return WF_ERR_CUDA;
     // every sequence's tokens are cut into units of 2 tq; n / (2 tq) + nseq bounds their number (CTAs beyond the last unit return at once)
     const dim3 grid(b.n / (2 * p.tq) + b.nseq, p.D.G);
-    if (split) attn_tc_kernel<true><<<grid, AT_THREADS, AT_SMEM, s>>>(tk, tv, b, p);
-    else attn_tc_kernel<false><<<grid, AT_THREADS, AT_SMEM, s>>>(tk, tv, b, p);
+    if (split) launch_pdl(attn_tc_kernel<true>, grid, AT_THREADS, AT_SMEM, s, tk, tv, b, p);
+    else launch_pdl(attn_tc_kernel<false>, grid, AT_THREADS, AT_SMEM, s, tk, tv, b, p);
     return launch_check(cudaGetLastError(), "attn_tc");
 }
 

@@ -68,6 +68,7 @@ __device__ __forceinline__ float cr_reduce(float (&v)[CR], int p) {
 
 template <int DS, bool VEC, bool DELTA>
 __global__ void __launch_bounds__(CR_THREADS) chunk_prep_kernel(Batch b, DeltaDims D, ChunkView w) {
+    pdl_enter();
     constexpr int Q4 = DS / 64;             // float4 per lane part
     __shared__ __align__(16) float ks[CR][DS], qs[CR][DS], gs[VEC ? CR : 1][VEC ? DS : 4];
     __shared__ float As[CR][CR + 1], Bs[CR][CR + 1], gsc[CR], bt[CR];
@@ -220,6 +221,7 @@ constexpr int CR_RS = 24;                                 // row stride of the p
 
 template <int DS, bool VEC, bool DELTA>
 __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
+    pdl_enter();
     using L = CrStage<DS, VEC, DELTA>;
     constexpr int REC = cr_rec_floats(DS, VEC), NT = DS / (8 * CR_WARPS), STEP = CR_THREADS / (DS / 4);
     extern __shared__ __align__(16) float sm[];
@@ -461,6 +463,7 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
 // that of the first one.  A thread holds the part of the state that it holds in chunk_scan_kernel; rows come straight from memory.
 template <int DS, bool VEC, bool DELTA>
 __global__ void __launch_bounds__(CR_THREADS) chunk_redo_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
+    pdl_enter();
     constexpr int NT = DS / (8 * CR_WARPS);
     __shared__ float rs[CR_WARPS][CR_COLS], os[CR_WARPS][CR_COLS];
     const int sq = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, row0 = warp * 8 * NT;
@@ -537,7 +540,7 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_redo_kernel(Batch b, DeltaDi
 
 template <int DS, bool VEC, bool DELTA>
 int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const float* decay, float* state, size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan) {
-    chunk_prep_kernel<DS, VEC, DELTA><<<dim3(b.nseq * w.nchunks, D.H), CR_THREADS, 0, s>>>(b, D, w);
+    launch_pdl(chunk_prep_kernel<DS, VEC, DELTA>, dim3(b.nseq * w.nchunks, D.H), CR_THREADS, 0, s, b, D, w);
     if (int rc = launch_check(cudaGetLastError(), "chunk_prep")) return rc;
     constexpr size_t smem = (size_t)(2 * CrStage<DS, VEC, DELTA>::FLOATS + CR_WARPS * 2 * CR_COLS * CR_RS) * sizeof(float);
     static DevOnce once;
@@ -545,12 +548,12 @@ int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const floa
     Segments sg;
     const int cols = w.cols;
     auto redo = [&]() {
-        chunk_redo_kernel<DS, VEC, DELTA><<<dim3(b.nseq, D.H, cols), CR_THREADS, 0, s>>>(b, D, w, state, slot_stride, o, sg);
+        launch_pdl(chunk_redo_kernel<DS, VEC, DELTA>, dim3(b.nseq, D.H, cols), CR_THREADS, 0, s, b, D, w, state, slot_stride, o, sg);
         return launch_check(cudaGetLastError(), "chunk_redo");
     };
     auto scan_pass = [&](int pass) {
         sg.pass = pass;
-        chunk_scan_kernel<DS, VEC, DELTA><<<dim3(b.nseq * sg.n, D.H, cols), CR_THREADS, smem, s>>>(b, D, w, state, slot_stride, o, sg);
+        launch_pdl(chunk_scan_kernel<DS, VEC, DELTA>, dim3(b.nseq * sg.n, D.H, cols), CR_THREADS, smem, s, b, D, w, state, slot_stride, o, sg);
         return launch_check(cudaGetLastError(), "chunk_scan");
     };
     // Segments in parallel where the recurrence is linear in the state, one portion is long and the chains of whole portions leave the machine idle: the two

@@ -14,6 +14,7 @@ namespace {
 template <typename T>
 __global__ void delta_prep_kernel(DeltaDims D, float* __restrict__ qkv, int ld, const float* __restrict__ a_raw, int lda, const float* __restrict__ b_raw,
                                   int ldb, const T* __restrict__ A_log, const T* __restrict__ dt_bias, float* __restrict__ beta, float* __restrict__ decay) {
+    pdl_enter();
     const int i = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     float* row = qkv + (size_t)i * ld;
@@ -39,6 +40,7 @@ __global__ void delta_prep_kernel(DeltaDims D, float* __restrict__ qkv, int ld, 
 template <typename T>
 __global__ void ssd_prep_kernel(int n, int H, const float* __restrict__ dt_raw, int ld, const T* __restrict__ A_log, const T* __restrict__ dt_bias,
                                 float* __restrict__ step, float* __restrict__ decay) {
+    pdl_enter();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n * H) return;
     const int i = k / H, h = k - i * H;
@@ -52,6 +54,7 @@ __global__ void ssd_prep_kernel(int n, int H, const float* __restrict__ dt_raw, 
 template <typename T>
 __global__ void ssd_post_kernel(int H, int dv, int groups, const float* __restrict__ o, const float* __restrict__ x, int ldx, const float* __restrict__ z, int ldz,
                                 const T* __restrict__ Dskip, const T* __restrict__ w, float eps, T* __restrict__ y) {
+    pdl_enter();
     __shared__ float scratch[33];
     const int i = blockIdx.x, g = blockIdx.y;
     const int inner = H * dv, gw = inner / groups;
@@ -99,6 +102,7 @@ template <int DPT, int DR_PARTS, bool VEC, bool DELTA, int NC>
 __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(Batch b, DeltaDims D, const float* __restrict__ qkv, int ld,
                                                                          const float* __restrict__ beta, const float* __restrict__ decay,
                                                                          float* __restrict__ state, size_t slot_stride, float* __restrict__ o, ScanArgs sa) {
+    pdl_enter();
     constexpr int DR_COLS = DR_THREADS / DR_PARTS * NC;
     extern __shared__ __align__(16) float sm[];
     // A thread owns DPT consecutive key rows; a token's k / q / decay rows lie in shared memory with 4 floats of padding after every DPT, so
@@ -294,6 +298,7 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(Batch b, DeltaDi
 // prod has one entry per (chunk, head), or (d > 0) one per (chunk, head, key row) of dd / d state columns each
 __global__ void scan_prefix_kernel(Batch b, int H, int dd, int chunk, float* __restrict__ state, size_t slot_stride, const float* __restrict__ local,
                                    float* __restrict__ startws, const float* __restrict__ prod, int d) {
+    pdl_enter();
     const int sq = blockIdx.x, h = blockIdx.y, e = blockIdx.z * blockDim.x + threadIdx.x;
     if (e >= dd) return;
     const int len = b.seq_len[sq], nc = (len + chunk - 1) / chunk, base = b.seq_start[sq] / chunk + sq;
@@ -309,6 +314,7 @@ __global__ void scan_prefix_kernel(Batch b, int H, int dd, int chunk, float* __r
 
 // thread per (sequence and chunk, head and key row): the product of the chunk's decays
 __global__ void scan_decay_prod_kernel(Batch b, int nd, int chunk, int nchunks, const float* __restrict__ decay, float* __restrict__ prod) {
+    pdl_enter();
     const int sq = blockIdx.x / nchunks, c = blockIdx.x - sq * nchunks, k = blockIdx.y * blockDim.x + threadIdx.x;
     const int len = b.seq_len[sq], start = b.seq_start[sq];
     if (k >= nd || c * chunk >= len) return;
@@ -329,6 +335,7 @@ __device__ __forceinline__ float gla_decay_of(float z, float inv_tau) {        /
 constexpr int GM_TOK = 64, GM_CH = 64;
 __global__ void __launch_bounds__(128) gla_decay_mma_kernel(int n, int rank, int rp, int nout, const float* __restrict__ a1, int ld, const __nv_bfloat16* __restrict__ a2,
                                                             const __nv_bfloat16* __restrict__ bias, float inv_tau, float* __restrict__ decay) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char gm_raw[];
     __shared__ float zb[GM_CH];
     const int S = rp + 8, i0 = blockIdx.x * GM_TOK, c0 = blockIdx.y * GM_CH;
@@ -401,6 +408,7 @@ constexpr int GD_TOK = 8, GD_THREADS = 128;
 template <typename T>
 __global__ void __launch_bounds__(GD_THREADS) gla_decay_kernel(int n, int rank, int nout, const float* __restrict__ a1, int ld, const T* __restrict__ a2,
                                                                const T* __restrict__ bias, float inv_tau, float* __restrict__ decay) {
+    pdl_enter();
     extern __shared__ float rows[];                  // [rank][GD_TOK]
     const int i0 = blockIdx.x * GD_TOK, c = blockIdx.y * GD_THREADS + threadIdx.x;
     for (int idx = threadIdx.x; idx < rank * GD_TOK; idx += GD_THREADS) {
@@ -428,6 +436,7 @@ __global__ void __launch_bounds__(GD_THREADS) gla_decay_kernel(int n, int rank, 
 template <typename T>
 __global__ void delta_post_kernel(DeltaDims D, const float* __restrict__ o, const T* __restrict__ w, float eps, const float* __restrict__ g, int ldg,
                                   T* __restrict__ y, int act) {
+    pdl_enter();
     const int i = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int h = blockIdx.y * nw + warp; h < D.H; h += gridDim.y * nw) {
@@ -449,8 +458,8 @@ int launch_delta_prep(int dt, const DeltaDims& D, int n, float* qkv, int ld, con
                       const void* A_log, const void* dt_bias, float* beta, float* decay, cudaStream_t s) {
     if (n <= 0) return WF_OK;
     if (D.Hk <= 0 || D.H % D.Hk) { set_error("delta: %d heads over %d key heads", D.H, D.Hk); return WF_ERR_INVALID; }
-    if (dt == WF_BF16) delta_prep_kernel<<<n, 128, 0, s>>>(D, qkv, ld, a_raw, lda, b_raw, ldb_, (const __nv_bfloat16*)A_log, (const __nv_bfloat16*)dt_bias, beta, decay);
-    else delta_prep_kernel<<<n, 128, 0, s>>>(D, qkv, ld, a_raw, lda, b_raw, ldb_, (const float*)A_log, (const float*)dt_bias, beta, decay);
+    if (dt == WF_BF16) launch_pdl(delta_prep_kernel<__nv_bfloat16>, n, 128, 0, s, D, qkv, ld, a_raw, lda, b_raw, ldb_, (const __nv_bfloat16*)A_log, (const __nv_bfloat16*)dt_bias, beta, decay);
+    else launch_pdl(delta_prep_kernel<float>, n, 128, 0, s, D, qkv, ld, a_raw, lda, b_raw, ldb_, (const float*)A_log, (const float*)dt_bias, beta, decay);
     return launch_check(cudaGetLastError(), "delta_prep");
 }
 
@@ -480,7 +489,7 @@ int delta_rule_launch(const Batch& b, const DeltaDims& D, const float* qkv, int 
         const int qo = D.q_off >= 0 ? D.q_off : 0, ko = D.k_off >= 0 ? D.k_off : D.Hk * D.d, vo = D.v_off >= 0 ? D.v_off : 2 * D.Hk * D.d;
         sa.v4 = D.d % 4 == 0 && D.dv % 4 == 0 && ld % 4 == 0 && qo % 4 == 0 && ko % 4 == 0 && vo % 4 == 0 && ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)decay & 15) == 0;
     }
-#define DR_LAUNCH(dp, pa, nc) delta_rule_kernel<dp, pa, VEC, DELTA, nc><<<grid, DR_THREADS, smem, s>>>(b, D, qkv, ld, beta, decay, state, slot_stride, o, sa)
+#define DR_LAUNCH(dp, pa, nc) launch_pdl(delta_rule_kernel<dp, pa, VEC, DELTA, nc>, grid, DR_THREADS, smem, s, b, D, qkv, ld, beta, decay, state, slot_stride, o, sa)
     if (D.d > 256 || smem > 160 * 1024) { set_error("delta: key dimension %d above the supported 256", D.d); return WF_ERR_UNSUPPORTED; }
     if (wide) { if (dpt <= 8) DR_LAUNCH(8, 8, (DELTA ? 1 : 2)); else DR_LAUNCH(16, 8, (DELTA ? 1 : 2)); }
     else if (decode) { if (dpt <= 8) DR_LAUNCH(8, 4, 1); else if (dpt <= 16) DR_LAUNCH(16, 4, 1); else if (dpt <= 32) DR_LAUNCH(32, 4, 1); else DR_LAUNCH(64, 4, 1); }
@@ -494,11 +503,11 @@ int delta_rule_launch(const Batch& b, const DeltaDims& D, const float* qkv, int 
 int launch_scan_prefix(const Batch& b, const DeltaDims& D, const float* decay, float* state, size_t slot_stride, const ScanWorkspace* scan, int nchunks, cudaStream_t s) {
     if (D.vec_decay) {
         const int nd = D.H * D.d;
-        scan_decay_prod_kernel<<<dim3(b.nseq * nchunks, (nd + 127) / 128), 128, 0, s>>>(b, nd, SCAN_CHUNK, nchunks, decay, scan->prod);
+        launch_pdl(scan_decay_prod_kernel, dim3(b.nseq * nchunks, (nd + 127) / 128), 128, 0, s, b, nd, SCAN_CHUNK, nchunks, decay, scan->prod);
         if (int rc = launch_check(cudaGetLastError(), "scan_decay_prod")) return rc;
     }
     const int dd = D.d * (D.dv + D.ones_col);
-    scan_prefix_kernel<<<dim3(b.nseq, D.H, (dd + 255) / 256), 256, 0, s>>>(b, D.H, dd, SCAN_CHUNK, state, slot_stride, scan->local, scan->start, scan->prod, D.vec_decay ? D.d : 0);
+    launch_pdl(scan_prefix_kernel, dim3(b.nseq, D.H, (dd + 255) / 256), 256, 0, s, b, D.H, dd, SCAN_CHUNK, state, slot_stride, scan->local, scan->start, scan->prod, D.vec_decay ? D.d : 0);
     return launch_check(cudaGetLastError(), "scan_prefix");
 }
 
@@ -533,8 +542,8 @@ int launch_delta_rule(const Batch& b, const DeltaDims& D, const float* qkv, int 
 int launch_delta_post(int dt, const DeltaDims& D, int n, const float* o, const void* w, float eps, const float* g, int ldg, void* y, cudaStream_t s, int act) {
     if (n <= 0) return WF_OK;
     const dim3 grid(n, n < 64 ? (D.H + 3) / 4 : 1);
-    if (dt == WF_BF16) delta_post_kernel<<<grid, 128, 0, s>>>(D, o, (const __nv_bfloat16*)w, eps, g, ldg, (__nv_bfloat16*)y, act);
-    else delta_post_kernel<<<grid, 128, 0, s>>>(D, o, (const float*)w, eps, g, ldg, (float*)y, act);
+    if (dt == WF_BF16) launch_pdl(delta_post_kernel<__nv_bfloat16>, grid, 128, 0, s, D, o, (const __nv_bfloat16*)w, eps, g, ldg, (__nv_bfloat16*)y, act);
+    else launch_pdl(delta_post_kernel<float>, grid, 128, 0, s, D, o, (const float*)w, eps, g, ldg, (float*)y, act);
     return launch_check(cudaGetLastError(), "delta_post");
 }
 
@@ -545,23 +554,23 @@ int launch_gla_decay(int dt, int n, int rank, int nout, const float* a1, int ld,
     if (dt == WF_BF16 && rank > 0 && tau > 0.f && rank % 8 == 0 && mma_smem <= 160 * 1024) {
         static DevOnce once;
         if (once.need()) cudaFuncSetAttribute(gla_decay_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        gla_decay_mma_kernel<<<dim3((n + GM_TOK - 1) / GM_TOK, (nout + GM_CH - 1) / GM_CH), 128, mma_smem, s>>>(n, rank, rp, nout, a1, ld, (const __nv_bfloat16*)a2,
+        launch_pdl(gla_decay_mma_kernel, dim3((n + GM_TOK - 1) / GM_TOK, (nout + GM_CH - 1) / GM_CH), 128, mma_smem, s, n, rank, rp, nout, a1, ld, (const __nv_bfloat16*)a2,
                                                                                                               (const __nv_bfloat16*)bias, 1.f / tau, decay);
         return launch_check(cudaGetLastError(), "gla_decay_mma");
     }
     const size_t smem = (size_t)rank * GD_TOK * sizeof(float);
     if (rank <= 0 || !(tau > 0.f) || smem > 48 * 1024) { set_error("gla: decay projection of rank %d, tau %g", rank, tau); return WF_ERR_UNSUPPORTED; }
     const dim3 grid((n + GD_TOK - 1) / GD_TOK, (nout + GD_THREADS - 1) / GD_THREADS);
-    if (dt == WF_BF16) gla_decay_kernel<<<grid, GD_THREADS, smem, s>>>(n, rank, nout, a1, ld, (const __nv_bfloat16*)a2, (const __nv_bfloat16*)bias, 1.f / tau, decay);
-    else gla_decay_kernel<<<grid, GD_THREADS, smem, s>>>(n, rank, nout, a1, ld, (const float*)a2, (const float*)bias, 1.f / tau, decay);
+    if (dt == WF_BF16) launch_pdl(gla_decay_kernel<__nv_bfloat16>, grid, GD_THREADS, smem, s, n, rank, nout, a1, ld, (const __nv_bfloat16*)a2, (const __nv_bfloat16*)bias, 1.f / tau, decay);
+    else launch_pdl(gla_decay_kernel<float>, grid, GD_THREADS, smem, s, n, rank, nout, a1, ld, (const float*)a2, (const float*)bias, 1.f / tau, decay);
     return launch_check(cudaGetLastError(), "gla_decay");
 }
 
 int launch_ssd_prep(int dt, int n, int H, const float* dt_raw, int ld, const void* A_log, const void* dt_bias, float* step, float* decay, cudaStream_t s) {
     if (n <= 0) return WF_OK;
     const int blocks = (n * H + 127) / 128;
-    if (dt == WF_BF16) ssd_prep_kernel<<<blocks, 128, 0, s>>>(n, H, dt_raw, ld, (const __nv_bfloat16*)A_log, (const __nv_bfloat16*)dt_bias, step, decay);
-    else ssd_prep_kernel<<<blocks, 128, 0, s>>>(n, H, dt_raw, ld, (const float*)A_log, (const float*)dt_bias, step, decay);
+    if (dt == WF_BF16) launch_pdl(ssd_prep_kernel<__nv_bfloat16>, blocks, 128, 0, s, n, H, dt_raw, ld, (const __nv_bfloat16*)A_log, (const __nv_bfloat16*)dt_bias, step, decay);
+    else launch_pdl(ssd_prep_kernel<float>, blocks, 128, 0, s, n, H, dt_raw, ld, (const float*)A_log, (const float*)dt_bias, step, decay);
     return launch_check(cudaGetLastError(), "ssd_prep");
 }
 
@@ -572,8 +581,8 @@ int launch_ssd_post(int dt, int n, int H, int dv, int groups, const float* o, co
     const int gw = H * dv / groups;
     const int threads = gw >= 1024 ? 256 : (gw >= 256 ? 128 : 64);
     const dim3 grid(n, groups);
-    if (dt == WF_BF16) ssd_post_kernel<<<grid, threads, 0, s>>>(H, dv, groups, o, x, ldx, z, ldz, (const __nv_bfloat16*)Dskip, (const __nv_bfloat16*)w, eps, (__nv_bfloat16*)y);
-    else ssd_post_kernel<<<grid, threads, 0, s>>>(H, dv, groups, o, x, ldx, z, ldz, (const float*)Dskip, (const float*)w, eps, (float*)y);
+    if (dt == WF_BF16) launch_pdl(ssd_post_kernel<__nv_bfloat16>, grid, threads, 0, s, H, dv, groups, o, x, ldx, z, ldz, (const __nv_bfloat16*)Dskip, (const __nv_bfloat16*)w, eps, (__nv_bfloat16*)y);
+    else launch_pdl(ssd_post_kernel<float>, grid, threads, 0, s, H, dv, groups, o, x, ldx, z, ldz, (const float*)Dskip, (const float*)w, eps, (float*)y);
     return launch_check(cudaGetLastError(), "ssd_post");
 }
 

@@ -26,6 +26,7 @@ template <typename T>
 __global__ void __launch_bounds__(32 * MG_MAXW) mingru_kernel(Batch b, int C, int ch, const float* __restrict__ proj, int ld, int z_off, int x_off, int g_off,
                                                                 const T* __restrict__ zb, const T* __restrict__ xb, float* __restrict__ state,
                                                                 size_t slot_stride, T* __restrict__ out) {
+    pdl_enter();
     __shared__ float sA[32 * MG_MAXW], sB[32 * MG_MAXW];       // [slice][ch]
     const int sq = blockIdx.x, cl = threadIdx.x % ch, w = threadIdx.x / ch, nw = blockDim.x / ch;      // w: this thread's time slice of nw
     const int c = blockIdx.y * ch + cl;
@@ -92,6 +93,7 @@ template <typename T>
 __global__ void __launch_bounds__(32 * ML_MAXW) mlstm_gates_kernel(Batch b, int H, const float* __restrict__ proj, int ld, int i_off, int f_off,
                                                                      const T* __restrict__ ib, const T* __restrict__ fb, float cap, float* __restrict__ mstate,
                                                                      size_t slot_stride, float* __restrict__ keep, float* __restrict__ put, float* __restrict__ mrun) {
+    pdl_enter();
     __shared__ float totF[ML_MAXW], totI[ML_MAXW];
     const int sq = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int start = b.seq_start[sq], len = b.seq_len[sq];
@@ -142,6 +144,7 @@ __global__ void __launch_bounds__(32 * ML_MAXW) mlstm_gates_kernel(Batch b, int 
 template <typename T>
 __global__ void mlstm_post_kernel(int n, int H, int dv, const float* __restrict__ o, const float* __restrict__ mrun, float qscale, const T* __restrict__ w,
                                   float eps, const float* __restrict__ g, int ldg, T* __restrict__ y) {
+    pdl_enter();
     const int lane = threadIdx.x & 31;
     const long long unit = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (unit >= (long long)n * H) return;
@@ -171,8 +174,8 @@ int launch_mingru(int dt, const Batch& b, int C, const float* proj, int ld, int 
     int nw = b.max_len / (8 * (32 / ch));
     nw = nw < 1 ? 1 : (nw > MG_MAXW ? MG_MAXW : nw);
     const dim3 grid(b.nseq, (C + ch - 1) / ch);
-    if (dt == WF_BF16) mingru_kernel<<<grid, 32 * nw, 0, s>>>(b, C, ch, proj, ld, z_off, x_off, g_off, (const __nv_bfloat16*)zb, (const __nv_bfloat16*)xb, state, slot_stride, (__nv_bfloat16*)out);
-    else mingru_kernel<<<grid, 32 * nw, 0, s>>>(b, C, ch, proj, ld, z_off, x_off, g_off, (const float*)zb, (const float*)xb, state, slot_stride, (float*)out);
+    if (dt == WF_BF16) launch_pdl(mingru_kernel<__nv_bfloat16>, grid, 32 * nw, 0, s, b, C, ch, proj, ld, z_off, x_off, g_off, (const __nv_bfloat16*)zb, (const __nv_bfloat16*)xb, state, slot_stride, (__nv_bfloat16*)out);
+    else launch_pdl(mingru_kernel<float>, grid, 32 * nw, 0, s, b, C, ch, proj, ld, z_off, x_off, g_off, (const float*)zb, (const float*)xb, state, slot_stride, (float*)out);
     return launch_check(cudaGetLastError(), "mingru");
 }
 
@@ -182,8 +185,8 @@ int launch_mlstm_gates(int dt, const Batch& b, int H, const float* proj, int ld,
     int nw = (b.max_len + 31) / 32;
     nw = nw < 1 ? 1 : (nw > ML_MAXW ? ML_MAXW : nw);
     const dim3 grid(b.nseq, H);
-    if (dt == WF_BF16) mlstm_gates_kernel<<<grid, 32 * nw, 0, s>>>(b, H, proj, ld, i_off, f_off, (const __nv_bfloat16*)ib, (const __nv_bfloat16*)fb, cap, mstate, slot_stride, keep, put, mrun);
-    else mlstm_gates_kernel<<<grid, 32 * nw, 0, s>>>(b, H, proj, ld, i_off, f_off, (const float*)ib, (const float*)fb, cap, mstate, slot_stride, keep, put, mrun);
+    if (dt == WF_BF16) launch_pdl(mlstm_gates_kernel<__nv_bfloat16>, grid, 32 * nw, 0, s, b, H, proj, ld, i_off, f_off, (const __nv_bfloat16*)ib, (const __nv_bfloat16*)fb, cap, mstate, slot_stride, keep, put, mrun);
+    else launch_pdl(mlstm_gates_kernel<float>, grid, 32 * nw, 0, s, b, H, proj, ld, i_off, f_off, (const float*)ib, (const float*)fb, cap, mstate, slot_stride, keep, put, mrun);
     return launch_check(cudaGetLastError(), "mlstm_gates");
 }
 
@@ -192,8 +195,8 @@ int launch_mlstm_post(int dt, int n, int H, int dv, const float* o, const float*
     if (n <= 0) return WF_OK;
     const long long units = (long long)n * H;
     const int blocks = (int)((units + 3) / 4);
-    if (dt == WF_BF16) mlstm_post_kernel<<<blocks, 128, 0, s>>>(n, H, dv, o, mrun, qscale, (const __nv_bfloat16*)w, eps, g, ldg, (__nv_bfloat16*)y);
-    else mlstm_post_kernel<<<blocks, 128, 0, s>>>(n, H, dv, o, mrun, qscale, (const float*)w, eps, g, ldg, (float*)y);
+    if (dt == WF_BF16) launch_pdl(mlstm_post_kernel<__nv_bfloat16>, blocks, 128, 0, s, n, H, dv, o, mrun, qscale, (const __nv_bfloat16*)w, eps, g, ldg, (__nv_bfloat16*)y);
+    else launch_pdl(mlstm_post_kernel<float>, blocks, 128, 0, s, n, H, dv, o, mrun, qscale, (const float*)w, eps, g, ldg, (float*)y);
     return launch_check(cudaGetLastError(), "mlstm_post");
 }
 

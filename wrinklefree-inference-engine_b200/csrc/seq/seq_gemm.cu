@@ -15,6 +15,7 @@ constexpr int BM = 64, BN = 64, BK = 16;       // kernel tile; GEMM_BM (the grou
 
 template <typename T, bool AF32, bool CF32>
 __global__ void __launch_bounds__(256) gemm_simt_kernel(GemmArgs g) {
+    pdl_enter();
     __shared__ float As[BK][BM + 4];
     __shared__ float Bs[BK][BN + 4];
     const int tile_m = blockIdx.y, tile_n = blockIdx.x, z = blockIdx.z;
@@ -101,6 +102,7 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
 
 template <bool AF32, bool CF32>
 __global__ void __launch_bounds__(128) gemm_mma_kernel(GemmArgs g) {
+    pdl_enter();
     __shared__ __align__(16) __nv_bfloat16 As[2][BM][MK + MPAD];
     __shared__ __align__(16) __nv_bfloat16 Bs[2][BN][MK + MPAD];
     const int tile_m = blockIdx.y, tile_n = blockIdx.x, z = blockIdx.z;
@@ -241,6 +243,7 @@ struct PairArgs { const int32_t* pair_expert; int n_experts; int pair_div; };
 
 template <typename T, int MR, bool AF32, bool CF32>
 __global__ void __launch_bounds__(GV_WARPS * 32) gemv_rows_kernel(GemmArgs g, PairArgs pa) {
+    pdl_enter();
     constexpr int VN = Vec16<T>::N;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const T* B = (const T*)g.B;
@@ -302,8 +305,8 @@ __global__ void __launch_bounds__(GV_WARPS * 32) gemv_rows_kernel(GemmArgs g, Pa
 
 template <typename T, int MR>
 void gemv_dispatch(const GemmArgs& g, const PairArgs& pa, dim3 grid, cudaStream_t s) {
-    if (g.a_f32) { if (g.c_f32) gemv_rows_kernel<T, MR, true, true><<<grid, GV_WARPS * 32, 0, s>>>(g, pa); else gemv_rows_kernel<T, MR, true, false><<<grid, GV_WARPS * 32, 0, s>>>(g, pa); }
-    else { if (g.c_f32) gemv_rows_kernel<T, MR, false, true><<<grid, GV_WARPS * 32, 0, s>>>(g, pa); else gemv_rows_kernel<T, MR, false, false><<<grid, GV_WARPS * 32, 0, s>>>(g, pa); }
+    if (g.a_f32) { if (g.c_f32) launch_pdl(gemv_rows_kernel<T, MR, true, true>, grid, GV_WARPS * 32, 0, s, g, pa); else launch_pdl(gemv_rows_kernel<T, MR, true, false>, grid, GV_WARPS * 32, 0, s, g, pa); }
+    else { if (g.c_f32) launch_pdl(gemv_rows_kernel<T, MR, false, true>, grid, GV_WARPS * 32, 0, s, g, pa); else launch_pdl(gemv_rows_kernel<T, MR, false, false>, grid, GV_WARPS * 32, 0, s, g, pa); }
 }
 
 template <typename T>
@@ -338,6 +341,7 @@ constexpr int FR_WARPS = 8;
 // U: 32-k blocks in flight per warp; OCC: blocks per SM
 template <int NT, int WK, int U, int OCC, bool CF32>
 __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g) {
+    pdl_enter();
     constexpr int TILES = FR_WARPS / WK;                  // 16-row tiles per block
     constexpr int C = NT == 1 ? 1 : 4;                    // running sums
     __shared__ float part[FR_WARPS][NT * 8][16 + 1];
@@ -423,7 +427,7 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
 template <int NT, int WK, int U, int OCC>
 void few_launch(const GemmArgs& g, cudaStream_t s) {
     const int tiles = (g.N + 15) / 16, per = FR_WARPS / WK, blocks = (tiles + per - 1) / per;
-    if (g.c_f32) gemm_few_kernel<NT, WK, U, OCC, true><<<blocks, FR_WARPS * 32, 0, s>>>(g); else gemm_few_kernel<NT, WK, U, OCC, false><<<blocks, FR_WARPS * 32, 0, s>>>(g);
+    if (g.c_f32) launch_pdl(gemm_few_kernel<NT, WK, U, OCC, true>, blocks, FR_WARPS * 32, 0, s, g); else launch_pdl(gemm_few_kernel<NT, WK, U, OCC, false>, blocks, FR_WARPS * 32, 0, s, g);
 }
 // Which split: a warp wants many loads in flight while there are fewer row tiles than SMs (2560 x 6912: 14.4 us, 15.7 with half as many), blocks of two
 // tiles fit one wave up to two per SM (12.4 us), and beyond that resident blocks cover the latency (13824 x 2560: 14.6 us against 22.7 / 18.6 with
@@ -443,8 +447,8 @@ void few_dispatch(const GemmArgs& g, cudaStream_t s) {
 
 template <typename T>
 void simt_dispatch(const GemmArgs& g, dim3 grid, cudaStream_t s) {
-    if (g.a_f32) { if (g.c_f32) gemm_simt_kernel<T, true, true><<<grid, 256, 0, s>>>(g); else gemm_simt_kernel<T, true, false><<<grid, 256, 0, s>>>(g); }
-    else { if (g.c_f32) gemm_simt_kernel<T, false, true><<<grid, 256, 0, s>>>(g); else gemm_simt_kernel<T, false, false><<<grid, 256, 0, s>>>(g); }
+    if (g.a_f32) { if (g.c_f32) launch_pdl(gemm_simt_kernel<T, true, true>, grid, 256, 0, s, g); else launch_pdl(gemm_simt_kernel<T, true, false>, grid, 256, 0, s, g); }
+    else { if (g.c_f32) launch_pdl(gemm_simt_kernel<T, false, true>, grid, 256, 0, s, g); else launch_pdl(gemm_simt_kernel<T, false, false>, grid, 256, 0, s, g); }
 }
 
 int g_force_simt = -1, g_tc_min = -1;
@@ -477,8 +481,8 @@ int launch_gemm(int dt, const GemmArgs& g, cudaStream_t s) {
     else if (g.algo == 1 || (g.algo == 0 && g_force_simt)) simt_dispatch<__nv_bfloat16>(g, grid, s);
     else if (g.algo == 3 || (g.algo == 0 && g.M >= g_tc_min && gemm_tc_usable(g))) return launch_gemm_tc(g, g.n_groups, s);
     else {
-        if (g.a_f32) { if (g.c_f32) gemm_mma_kernel<true, true><<<grid, 128, 0, s>>>(g); else gemm_mma_kernel<true, false><<<grid, 128, 0, s>>>(g); }
-        else { if (g.c_f32) gemm_mma_kernel<false, true><<<grid, 128, 0, s>>>(g); else gemm_mma_kernel<false, false><<<grid, 128, 0, s>>>(g); }
+        if (g.a_f32) { if (g.c_f32) launch_pdl(gemm_mma_kernel<true, true>, grid, 128, 0, s, g); else launch_pdl(gemm_mma_kernel<true, false>, grid, 128, 0, s, g); }
+        else { if (g.c_f32) launch_pdl(gemm_mma_kernel<false, true>, grid, 128, 0, s, g); else launch_pdl(gemm_mma_kernel<false, false>, grid, 128, 0, s, g); }
     }
     return launch_check(cudaGetLastError(), "gemm");
 }

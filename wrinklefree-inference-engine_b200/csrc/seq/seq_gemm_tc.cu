@@ -126,6 +126,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_s;
+    pdl_enter();                                       // barriers, TMEM and the pair's meeting above overlap the kernel before
 
     // every role of both CTAs walks the same list of tiles and skips the same ones; `it` counts ring items, `done` counts tiles that were computed
     if (warp == TC_EPW) {
@@ -365,11 +366,13 @@ int launch_gemm_tc(const GemmArgs& g, int n_groups, cudaStream_t s) {
     cfg.blockDim = dim3(TC_THREADS);
     cfg.dynamicSmemBytes = TC_SMEM;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return launch_check(cudaLaunchKernelEx(&cfg, gemm_tc_kernel, tw, ta, p), "gemm_tc");
 }
 

@@ -43,6 +43,7 @@ __device__ __forceinline__ float rope_entry(const LatentDims& L, const float* __
 
 template <typename T>
 __global__ void latent_q_prep_kernel(Batch b, LatentDims L, const float* __restrict__ q, int ldq, T* __restrict__ qn, float* __restrict__ qr) {
+    pdl_enter();
     __shared__ float cs[LA_MAXPAIRS], sn[LA_MAXPAIRS];
     const int i = blockIdx.x;
     const int pos = b.tok_pos[i];
@@ -62,6 +63,7 @@ __global__ void latent_q_prep_kernel(Batch b, LatentDims L, const float* __restr
 // one block per token: latent RMS norm + rotary of the shared key part, stored as T in the token's cache row
 template <typename T>
 __global__ void latent_kv_write_kernel(Batch b, LatentDims L, const float* __restrict__ dkv, int ld, const T* __restrict__ w, float eps, PagedCache pc) {
+    pdl_enter();
     __shared__ float scratch[33];
     __shared__ float cs[LA_MAXPAIRS], sn[LA_MAXPAIRS];
     const int i = blockIdx.x;
@@ -89,6 +91,7 @@ constexpr int LA_MAXr = 8;     // rotated size up to 32 * 8
 template <typename T>
 __global__ void __launch_bounds__(LA_WARPS * 32) latent_attn_kernel(Batch b, LatentDims L, const float* __restrict__ qa, const float* __restrict__ qr,
                                                                       PagedCache pc, T* __restrict__ out) {
+    pdl_enter();
     extern __shared__ float sm[];   // [LA_WARPS][R] partial sums, then [LA_WARPS] m, [LA_WARPS] l
     const int i = blockIdx.x, h = blockIdx.y;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -162,6 +165,7 @@ int check_dims(const LatentDims& L) {
 // rows of every head's key [W_uk | 0] and [0 | unit rows], then of every head's value [W_uv | 0]
 template <typename T>
 __global__ void latent_expand_weight_kernel(LatentDims L, const T* __restrict__ uk, const T* __restrict__ uv, T* __restrict__ out) {
+    pdl_enter();
     const int width = L.R + L.r, per = L.d + L.r, row = blockIdx.x;
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
         T v = from_f<T>(0.f);
@@ -176,6 +180,7 @@ __global__ void latent_expand_weight_kernel(LatentDims L, const T* __restrict__ 
 
 // a warp per cached row, 16 bytes per lane and copy
 __global__ void latent_gather_kernel(Batch b, LatentDims L, PagedCache pc, const int32_t* __restrict__ key_row, int rows, __nv_bfloat16* __restrict__ out) {
+    pdl_enter();
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
     int sq = 0;
@@ -191,15 +196,15 @@ __global__ void latent_gather_kernel(Batch b, LatentDims L, PagedCache pc, const
 
 int launch_latent_expand_weight(int dt, const LatentDims& L, const void* uk, const void* uv, void* out, cudaStream_t s) {
     const int rows = L.H * (L.d + L.r + L.dv);
-    if (dt == WF_BF16) latent_expand_weight_kernel<<<rows, 128, 0, s>>>(L, (const __nv_bfloat16*)uk, (const __nv_bfloat16*)uv, (__nv_bfloat16*)out);
-    else latent_expand_weight_kernel<<<rows, 128, 0, s>>>(L, (const float*)uk, (const float*)uv, (float*)out);
+    if (dt == WF_BF16) launch_pdl(latent_expand_weight_kernel<__nv_bfloat16>, rows, 128, 0, s, L, (const __nv_bfloat16*)uk, (const __nv_bfloat16*)uv, (__nv_bfloat16*)out);
+    else launch_pdl(latent_expand_weight_kernel<float>, rows, 128, 0, s, L, (const float*)uk, (const float*)uv, (float*)out);
     return launch_check(cudaGetLastError(), "latent_expand_weight");
 }
 
 int launch_latent_gather(const Batch& b, const LatentDims& L, const PagedCache& pc, const int32_t* key_row, int rows, void* out, cudaStream_t s) {
     if (rows <= 0) return WF_OK;
     if ((L.R + L.r) % 8 || pc.layer_off % 8 || pc.page_stride % 8) { set_error("latent gather: cached rows are not 16-byte aligned"); return WF_ERR_UNSUPPORTED; }
-    latent_gather_kernel<<<(rows + 7) / 8, 256, 0, s>>>(b, L, pc, key_row, rows, (__nv_bfloat16*)out);
+    launch_pdl(latent_gather_kernel, (rows + 7) / 8, 256, 0, s, b, L, pc, key_row, rows, (__nv_bfloat16*)out);
     return launch_check(cudaGetLastError(), "latent_gather");
 }
 
@@ -207,8 +212,8 @@ int launch_latent_q_prep(int dt, const Batch& b, const LatentDims& L, const floa
     if (b.n <= 0) return WF_OK;
     if (int rc = check_dims(L)) return rc;
     const dim3 grid(b.n, b.n < 64 ? (L.H * (L.d + L.r) + 255) / 256 : 1);
-    if (dt == WF_BF16) latent_q_prep_kernel<<<grid, 256, 0, s>>>(b, L, q, ldq, (__nv_bfloat16*)qn, qr);
-    else latent_q_prep_kernel<<<grid, 256, 0, s>>>(b, L, q, ldq, (float*)qn, qr);
+    if (dt == WF_BF16) launch_pdl(latent_q_prep_kernel<__nv_bfloat16>, grid, 256, 0, s, b, L, q, ldq, (__nv_bfloat16*)qn, qr);
+    else launch_pdl(latent_q_prep_kernel<float>, grid, 256, 0, s, b, L, q, ldq, (float*)qn, qr);
     return launch_check(cudaGetLastError(), "latent_q_prep");
 }
 
@@ -216,8 +221,8 @@ int launch_latent_kv_write(int dt, const Batch& b, const LatentDims& L, const fl
                            cudaStream_t s) {
     if (b.n <= 0) return WF_OK;
     if (int rc = check_dims(L)) return rc;
-    if (dt == WF_BF16) latent_kv_write_kernel<<<b.n, 128, 0, s>>>(b, L, dkv, ld, (const __nv_bfloat16*)w, eps, pc);
-    else latent_kv_write_kernel<<<b.n, 128, 0, s>>>(b, L, dkv, ld, (const float*)w, eps, pc);
+    if (dt == WF_BF16) launch_pdl(latent_kv_write_kernel<__nv_bfloat16>, b.n, 128, 0, s, b, L, dkv, ld, (const __nv_bfloat16*)w, eps, pc);
+    else launch_pdl(latent_kv_write_kernel<float>, b.n, 128, 0, s, b, L, dkv, ld, (const float*)w, eps, pc);
     return launch_check(cudaGetLastError(), "latent_kv_write");
 }
 
@@ -227,8 +232,8 @@ int launch_latent_attn(int dt, const Batch& b, const LatentDims& L, const float*
     if (L.H > 65535) { set_error("latent attention: too many heads"); return WF_ERR_UNSUPPORTED; }
     dim3 grid(b.n, L.H);
     const size_t smem = ((size_t)LA_WARPS * L.R + 2 * LA_WARPS) * sizeof(float);
-    if (dt == WF_BF16) latent_attn_kernel<<<grid, LA_WARPS * 32, smem, s>>>(b, L, qa, qr, pc, (__nv_bfloat16*)out);
-    else latent_attn_kernel<<<grid, LA_WARPS * 32, smem, s>>>(b, L, qa, qr, pc, (float*)out);
+    if (dt == WF_BF16) launch_pdl(latent_attn_kernel<__nv_bfloat16>, grid, LA_WARPS * 32, smem, s, b, L, qa, qr, pc, (__nv_bfloat16*)out);
+    else launch_pdl(latent_attn_kernel<float>, grid, LA_WARPS * 32, smem, s, b, L, qa, qr, pc, (float*)out);
     return launch_check(cudaGetLastError(), "latent_attn");
 }
 

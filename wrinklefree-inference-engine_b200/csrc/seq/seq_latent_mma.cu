@@ -43,6 +43,7 @@ struct MmaParams {
 template <int NT>
 __global__ void latent_attn_mma_kernel(Batch b, LatentDims L, const float* __restrict__ qa, const float* __restrict__ qr, PagedCache pc,
                                        __nv_bfloat16* __restrict__ out, MmaParams mp) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
     const int HT = (L.H + 15) / 16, rows = HT * 16;
     const int stride = mp.stride, width = L.R + L.r;
@@ -218,6 +219,7 @@ __global__ void latent_attn_mma_kernel(Batch b, LatentDims L, const float* __res
 
 // one block per (token, head): out = sum_s exp(m_s - m) O_s / sum_s exp(m_s - m) l_s
 __global__ void latent_attn_merge_kernel(int H, int R, int splits, const float* __restrict__ part, __nv_bfloat16* __restrict__ out, const float* __restrict__ sink) {
+    pdl_enter();
     const int i = blockIdx.x, h = blockIdx.y;
     const float* p0 = part + (((size_t)i * splits) * H + h) * (R + 2);
     const size_t sstride = (size_t)H * (R + 2);
@@ -259,6 +261,7 @@ __host__ __device__ constexpr int kt_pt_stride(int NH) { return (NH & 1) ? NH * 
 template <int NH, int MTW>
 __global__ void __launch_bounds__(256) latent_attn_kt_kernel(Batch b, LatentDims L, const float* __restrict__ qa, const float* __restrict__ qr, PagedCache pc,
                                                              __nv_bfloat16* __restrict__ out, MmaParams mp) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int HP = NH * 8, PS = HP + 1, PT = kt_pt_stride(NH);
     const int stride = mp.stride, width = L.R + L.r;
@@ -478,7 +481,7 @@ int launch_kt(const Batch& b, const LatentDims& L, const float* qa, const float*
     static DevOnce once;
     if (once.need()) cudaFuncSetAttribute(latent_attn_kt_kernel<NH, MTW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     dim3 grid(b.n, mp.splits);
-    latent_attn_kt_kernel<NH, MTW><<<grid, 256, kt_smem(NH, L), s>>>(b, L, qa, qr, pc, (__nv_bfloat16*)out, mp);
+    launch_pdl(latent_attn_kt_kernel<NH, MTW>, grid, 256, kt_smem(NH, L), s, b, L, qa, qr, pc, (__nv_bfloat16*)out, mp);
     return launch_check(cudaGetLastError(), "latent_attn_kt");
 }
 
@@ -489,7 +492,7 @@ int launch_nt(const Batch& b, const LatentDims& L, const float* qa, const float*
     if (once.need()) cudaFuncSetAttribute(latent_attn_mma_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     const int HT = (L.H + 15) / 16;
     dim3 grid(b.n, mp.splits);
-    latent_attn_mma_kernel<NT><<<grid, HT * 128, smem, s>>>(b, L, qa, qr, pc, (__nv_bfloat16*)out, mp);
+    launch_pdl(latent_attn_mma_kernel<NT>, grid, HT * 128, smem, s, b, L, qa, qr, pc, (__nv_bfloat16*)out, mp);
     return launch_check(cudaGetLastError(), "latent_attn_mma");
 }
 
@@ -529,7 +532,7 @@ int launch_latent_attn_kt(const Batch& b, const LatentDims& L, const float* qa, 
     if (rc) return rc;
     if (mp.splits > 1) {
         dim3 grid(b.n, L.H);
-        latent_attn_merge_kernel<<<grid, 128, 0, s>>>(L.H, L.R, mp.splits, workspace, (__nv_bfloat16*)out, L.sink);
+        launch_pdl(latent_attn_merge_kernel, grid, 128, 0, s, L.H, L.R, mp.splits, workspace, (__nv_bfloat16*)out, L.sink);
         return launch_check(cudaGetLastError(), "latent_attn_merge");
     }
     return WF_OK;
@@ -579,7 +582,7 @@ int launch_latent_attn_mma(const Batch& b, const LatentDims& L, const float* qa,
     if (rc) return rc;
     if (mp.splits > 1) {
         dim3 grid(b.n, L.H);
-        latent_attn_merge_kernel<<<grid, 128, 0, s>>>(L.H, L.R, mp.splits, workspace, (__nv_bfloat16*)out, L.sink);
+        launch_pdl(latent_attn_merge_kernel, grid, 128, 0, s, L.H, L.R, mp.splits, workspace, (__nv_bfloat16*)out, L.sink);
         return launch_check(cudaGetLastError(), "latent_attn_merge");
     }
     return WF_OK;

@@ -97,6 +97,7 @@ __device__ void route_token(const RouterDims& R, const float* zr, const T* __res
 template <typename T>
 __global__ void moe_route_kernel(RouterDims R, const float* __restrict__ z, int ldz, const T* __restrict__ correction, int32_t* __restrict__ ids,
                                  float* __restrict__ wts, int32_t* __restrict__ counts) {
+    pdl_enter();
     extern __shared__ float sm[];
     route_token(R, z + (size_t)blockIdx.x * ldz, correction, ids, wts, counts, sm, blockIdx.x, threadIdx.x);
 }
@@ -113,6 +114,7 @@ template <typename T, bool VEC, int NT>
 __global__ void __launch_bounds__(NT) router_fused_kernel(RouterDims R, int n, int tb, const float* __restrict__ x, int ldx, const T* __restrict__ w, int NZ, int W,
                                                                   float* __restrict__ z, int ldz, const T* __restrict__ correction, int32_t* __restrict__ ids,
                                                                   float* __restrict__ wts, int32_t* __restrict__ counts) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int Wp = (W + 3) / 4 * 4, N = R.E + R.I, per = 2 * N + R.groups;
     float* xs = sm;                                  // [tb][Wp]
@@ -169,6 +171,7 @@ __global__ void __launch_bounds__(NT) router_fused_kernel(RouterDims R, int n, i
 // single block.  scratch: off[E + 1], cursor[E]
 __global__ void moe_plan_kernel(RouterDims R, int n, const int32_t* __restrict__ ids, const int32_t* __restrict__ counts, int32_t* __restrict__ scratch,
                                 int32_t* __restrict__ sorted_rows, int32_t* __restrict__ pair_row, int32_t* __restrict__ tile_group, int P) {
+    pdl_enter();
     int32_t* off = scratch;
     int32_t* cursor = scratch + R.E + 1;
     if (threadIdx.x == 0) {
@@ -193,6 +196,7 @@ __global__ void moe_plan_kernel(RouterDims R, int n, const int32_t* __restrict__
 // VEC = 4: ff a multiple of 4 (16-byte loads of the gate and up halves)
 template <typename T, int VEC>
 __global__ void silu_mul_kernel(const float* __restrict__ gu, int ff, const int32_t* __restrict__ tile_group, T* __restrict__ hmid, int act, float limit) {
+    pdl_enter();
     const int r = blockIdx.x;
     if (tile_group && tile_group[r / GEMM_BM] < 0) return;
     const float* row = gu + (size_t)r * (act == 3 ? 1 : 2) * ff;
@@ -228,6 +232,7 @@ template <typename T, int VEC>
 __global__ void moe_combine_kernel(RouterDims R, int W, const int32_t* __restrict__ ids, const float* __restrict__ wts, const int32_t* __restrict__ pair_row,
                                    const float* __restrict__ y, const T* __restrict__ h, float* __restrict__ out, const float* __restrict__ shared_y,
                                    const float* __restrict__ shared_gate, int ld_gate) {
+    pdl_enter();
     const int i = blockIdx.x;
     const float sg = shared_y ? (shared_gate ? sigmoid_f(shared_gate[(size_t)i * ld_gate]) : 1.f) : 0.f;
     for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC; c < W; c += gridDim.y * blockDim.x * VEC) {
@@ -271,8 +276,8 @@ int launch_moe_route(int dt, const RouterDims& R, int n, const float* z, int ldz
     }
     const size_t smem = (size_t)(2 * N + R.groups) * sizeof(float);
     if (smem > 48 * 1024) { set_error("router: %d outputs do not fit in shared memory", N); return WF_ERR_UNSUPPORTED; }
-    if (dt == WF_BF16) moe_route_kernel<<<n, 32, smem, s>>>(R, z, ldz, (const __nv_bfloat16*)correction, ids, wts, counts);
-    else moe_route_kernel<<<n, 32, smem, s>>>(R, z, ldz, (const float*)correction, ids, wts, counts);
+    if (dt == WF_BF16) launch_pdl(moe_route_kernel<__nv_bfloat16>, n, 32, smem, s, R, z, ldz, (const __nv_bfloat16*)correction, ids, wts, counts);
+    else launch_pdl(moe_route_kernel<float>, n, 32, smem, s, R, z, ldz, (const float*)correction, ids, wts, counts);
     return launch_check(cudaGetLastError(), "moe_route");
 }
 
@@ -299,7 +304,7 @@ int launch_router_fused(int dt, const RouterDims& R, int n, const float* x, int 
     const bool vec = (W * esz) % 16 == 0 && (((uintptr_t)w) & 15) == 0;
     const int blocks = (n + tb - 1) / tb;
     const bool few = n <= sm_count();
-#define RF_LAUNCH(T, VEC, NT) router_fused_kernel<T, VEC, NT><<<blocks, NT, smem, s>>>(R, n, tb, x, ldx, (const T*)w, NZ, W, z, ldz, (const T*)correction, ids, wts, counts)
+#define RF_LAUNCH(T, VEC, NT) launch_pdl(router_fused_kernel<T, VEC, NT>, blocks, NT, smem, s, R, n, tb, x, ldx, (const T*)w, NZ, W, z, ldz, (const T*)correction, ids, wts, counts)
 #define RF_PICK(T) do { if (vec) { if (few) RF_LAUNCH(T, true, RF_THREADS_FEW); else RF_LAUNCH(T, true, RF_THREADS); } \
                         else { if (few) RF_LAUNCH(T, false, RF_THREADS_FEW); else RF_LAUNCH(T, false, RF_THREADS); } } while (0)
     if (dt == WF_BF16) RF_PICK(__nv_bfloat16); else RF_PICK(float);
@@ -312,7 +317,7 @@ int launch_moe_plan(const RouterDims& R, int n, const int32_t* ids, const int32_
                     int32_t* pair_row, int32_t* tile_group, int P, cudaStream_t s) {
     if (n <= 0) return WF_OK;
     if (P % GEMM_BM) { set_error("moe_plan: row bound %d is not a multiple of the row tile", P); return WF_ERR_INVALID; }
-    moe_plan_kernel<<<1, 512, 0, s>>>(R, n, ids, counts, scratch, sorted_rows, pair_row, tile_group, P);
+    launch_pdl(moe_plan_kernel, 1, 512, 0, s, R, n, ids, counts, scratch, sorted_rows, pair_row, tile_group, P);
     return launch_check(cudaGetLastError(), "moe_plan");
 }
 
@@ -321,8 +326,8 @@ int launch_silu_mul(int dt, const float* gu, int P, int ff, const int32_t* tile_
     const bool vec = ff % 4 == 0 && (((uintptr_t)gu) & 15) == 0;
     const int per = 128 * (vec ? 4 : 1);
     const dim3 grid(P, P < 256 ? (ff + per - 1) / per : 1);
-    if (dt == WF_BF16) { if (vec) silu_mul_kernel<__nv_bfloat16, 4><<<grid, 128, 0, s>>>(gu, ff, tile_group, (__nv_bfloat16*)hmid, act, limit); else silu_mul_kernel<__nv_bfloat16, 1><<<grid, 128, 0, s>>>(gu, ff, tile_group, (__nv_bfloat16*)hmid, act, limit); }
-    else { if (vec) silu_mul_kernel<float, 4><<<grid, 128, 0, s>>>(gu, ff, tile_group, (float*)hmid, act, limit); else silu_mul_kernel<float, 1><<<grid, 128, 0, s>>>(gu, ff, tile_group, (float*)hmid, act, limit); }
+    if (dt == WF_BF16) { if (vec) launch_pdl(silu_mul_kernel<__nv_bfloat16, 4>, grid, 128, 0, s, gu, ff, tile_group, (__nv_bfloat16*)hmid, act, limit); else launch_pdl(silu_mul_kernel<__nv_bfloat16, 1>, grid, 128, 0, s, gu, ff, tile_group, (__nv_bfloat16*)hmid, act, limit); }
+    else { if (vec) launch_pdl(silu_mul_kernel<float, 4>, grid, 128, 0, s, gu, ff, tile_group, (float*)hmid, act, limit); else launch_pdl(silu_mul_kernel<float, 1>, grid, 128, 0, s, gu, ff, tile_group, (float*)hmid, act, limit); }
     return launch_check(cudaGetLastError(), "silu_mul");
 }
 
@@ -332,8 +337,8 @@ int launch_moe_combine(int dt, const RouterDims& R, int n, int W, const int32_t*
     const bool vec = W % 4 == 0 && (((uintptr_t)y) & 15) == 0 && (((uintptr_t)out) & 15) == 0;
     const int per = 256 * (vec ? 4 : 1);
     const dim3 grid(n, n < 64 ? (W + per - 1) / per : 1);       // few tokens: spread a row over several blocks
-    if (dt == WF_BF16) { if (vec) moe_combine_kernel<__nv_bfloat16, 4><<<grid, 256, 0, s>>>(R, W, ids, wts, pair_row, y, (const __nv_bfloat16*)h, out, shared_y, shared_gate, ld_gate); else moe_combine_kernel<__nv_bfloat16, 1><<<grid, 256, 0, s>>>(R, W, ids, wts, pair_row, y, (const __nv_bfloat16*)h, out, shared_y, shared_gate, ld_gate); }
-    else { if (vec) moe_combine_kernel<float, 4><<<grid, 256, 0, s>>>(R, W, ids, wts, pair_row, y, (const float*)h, out, shared_y, shared_gate, ld_gate); else moe_combine_kernel<float, 1><<<grid, 256, 0, s>>>(R, W, ids, wts, pair_row, y, (const float*)h, out, shared_y, shared_gate, ld_gate); }
+    if (dt == WF_BF16) { if (vec) launch_pdl(moe_combine_kernel<__nv_bfloat16, 4>, grid, 256, 0, s, R, W, ids, wts, pair_row, y, (const __nv_bfloat16*)h, out, shared_y, shared_gate, ld_gate); else launch_pdl(moe_combine_kernel<__nv_bfloat16, 1>, grid, 256, 0, s, R, W, ids, wts, pair_row, y, (const __nv_bfloat16*)h, out, shared_y, shared_gate, ld_gate); }
+    else { if (vec) launch_pdl(moe_combine_kernel<float, 4>, grid, 256, 0, s, R, W, ids, wts, pair_row, y, (const float*)h, out, shared_y, shared_gate, ld_gate); else launch_pdl(moe_combine_kernel<float, 1>, grid, 256, 0, s, R, W, ids, wts, pair_row, y, (const float*)h, out, shared_y, shared_gate, ld_gate); }
     return launch_check(cudaGetLastError(), "moe_combine");
 }
 
@@ -349,6 +354,7 @@ __device__ float block_reduce_sum(float v, float* scratch) { return block_sum(v,
 // the draw walks the kept entries in index order.
 __global__ void __launch_bounds__(SM_THREADS) sample_kernel(const float* __restrict__ logits, int V, float temperature, int top_k, float top_p,
                                                              const float* __restrict__ u, int32_t* __restrict__ next) {
+    pdl_enter();
     __shared__ float scratch[33];
     __shared__ float sv[SM_THREADS / 32];
     __shared__ int si[SM_THREADS / 32];
@@ -427,7 +433,7 @@ __global__ void __launch_bounds__(SM_THREADS) sample_kernel(const float* __restr
 int launch_sample(const float* logits, int m, int V, float temperature, int top_k, float top_p, const float* u, int32_t* next, cudaStream_t s) {
     if (m <= 0) return WF_OK;
     if (temperature > 0.f && !u) { set_error("sample: uniforms required when temperature > 0"); return WF_ERR_INVALID; }
-    sample_kernel<<<m, SM_THREADS, 0, s>>>(logits, V, temperature, top_k, top_p, u, next);
+    launch_pdl(sample_kernel, m, SM_THREADS, 0, s, logits, V, temperature, top_k, top_p, u, next);
     return launch_check(cudaGetLastError(), "sample");
 }
 

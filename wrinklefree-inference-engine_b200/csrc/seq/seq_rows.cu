@@ -8,6 +8,7 @@ namespace seq {
 template <typename T>
 __global__ void embed_f32_kernel(const T* __restrict__ table, const int32_t* __restrict__ tokens, int W, float* __restrict__ x, float scale, T* __restrict__ x_t,
                                  const T* __restrict__ pos_table, const int32_t* __restrict__ tok_pos) {
+    pdl_enter();
     const int i = blockIdx.x;
     const T* row = table + (size_t)tokens[i] * W;
     const T* prow = pos_table ? pos_table + (size_t)tok_pos[i] * W : nullptr;
@@ -22,19 +23,20 @@ __global__ void embed_f32_kernel(const T* __restrict__ table, const int32_t* __r
 int launch_embed_f32(int dt, const void* table, const int32_t* tokens, int n, int W, float* x, cudaStream_t s, float scale, void* x_t,
                      const void* pos_table, const int32_t* tok_pos) {
     if (n <= 0) return WF_OK;
-    if (dt == WF_BF16) embed_f32_kernel<<<n, 256, 0, s>>>((const __nv_bfloat16*)table, tokens, W, x, scale, (__nv_bfloat16*)x_t, (const __nv_bfloat16*)pos_table, tok_pos);
-    else embed_f32_kernel<<<n, 256, 0, s>>>((const float*)table, tokens, W, x, scale, (float*)x_t, (const float*)pos_table, tok_pos);
+    if (dt == WF_BF16) launch_pdl(embed_f32_kernel<__nv_bfloat16>, n, 256, 0, s, (const __nv_bfloat16*)table, tokens, W, x, scale, (__nv_bfloat16*)x_t, (const __nv_bfloat16*)pos_table, tok_pos);
+    else launch_pdl(embed_f32_kernel<float>, n, 256, 0, s, (const float*)table, tokens, W, x, scale, (float*)x_t, (const float*)pos_table, tok_pos);
     return launch_check(cudaGetLastError(), "embed_f32");
 }
 
 __global__ void axpby_kernel(float* __restrict__ y, float a, const float* __restrict__ y2, float b, size_t count) {
+    pdl_enter();
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x) y[k] = a * y[k] + b * y2[k];
 }
 
 int launch_axpby(float* y, float a, const float* y2, float b, size_t count, cudaStream_t s) {
     if (count == 0) return WF_OK;
     const int blocks = (int)((count + 255) / 256 > 4096 ? 4096 : (count + 255) / 256);
-    axpby_kernel<<<blocks, 256, 0, s>>>(y, a, y2, b, count);
+    launch_pdl(axpby_kernel, blocks, 256, 0, s, y, a, y2, b, count);
     return launch_check(cudaGetLastError(), "axpby");
 }
 
@@ -43,6 +45,7 @@ int launch_axpby(float* y, float a, const float* y2, float b, size_t count, cuda
 template <typename T>
 __global__ void embed_pos_kernel(const T* __restrict__ table, const int32_t* __restrict__ tokens, const int32_t* __restrict__ tok_pos, int W, float base,
                                  float* __restrict__ x, T* __restrict__ x_t) {
+    pdl_enter();
     const int i = blockIdx.x;
     const T* row = table + (size_t)tokens[i] * W;
     const double pos = (double)tok_pos[i], lb = log2((double)base);
@@ -56,14 +59,15 @@ __global__ void embed_pos_kernel(const T* __restrict__ table, const int32_t* __r
 
 int launch_embed_pos(int dt, const void* table, const int32_t* tokens, const int32_t* tok_pos, int n, int W, float base, float* x, void* x_t, cudaStream_t s) {
     if (n <= 0) return WF_OK;
-    if (dt == WF_BF16) embed_pos_kernel<<<n, 256, 0, s>>>((const __nv_bfloat16*)table, tokens, tok_pos, W, base, x, (__nv_bfloat16*)x_t);
-    else embed_pos_kernel<<<n, 256, 0, s>>>((const float*)table, tokens, tok_pos, W, base, x, (float*)x_t);
+    if (dt == WF_BF16) launch_pdl(embed_pos_kernel<__nv_bfloat16>, n, 256, 0, s, (const __nv_bfloat16*)table, tokens, tok_pos, W, base, x, (__nv_bfloat16*)x_t);
+    else launch_pdl(embed_pos_kernel<float>, n, 256, 0, s, (const float*)table, tokens, tok_pos, W, base, x, (float*)x_t);
     return launch_check(cudaGetLastError(), "embed_pos");
 }
 
 // x_t[i, :] = T(x[i, :])
 template <typename T>
 __global__ void round_rows_kernel(const float* __restrict__ x, size_t count, T* __restrict__ x_t) {
+    pdl_enter();
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x) x_t[k] = from_f<T>(x[k]);
 }
 
@@ -71,8 +75,8 @@ int launch_round_rows(int dt, const float* x, int n, int W, void* x_t, cudaStrea
     if (n <= 0) return WF_OK;
     const size_t count = (size_t)n * W;
     const int blocks = (int)((count + 255) / 256 > 4096 ? 4096 : (count + 255) / 256);
-    if (dt == WF_BF16) round_rows_kernel<<<blocks, 256, 0, s>>>(x, count, (__nv_bfloat16*)x_t);
-    else round_rows_kernel<<<blocks, 256, 0, s>>>(x, count, (float*)x_t);
+    if (dt == WF_BF16) launch_pdl(round_rows_kernel<__nv_bfloat16>, blocks, 256, 0, s, x, count, (__nv_bfloat16*)x_t);
+    else launch_pdl(round_rows_kernel<float>, blocks, 256, 0, s, x, count, (float*)x_t);
     return launch_check(cudaGetLastError(), "round_rows");
 }
 
@@ -83,6 +87,7 @@ template <typename T>
 __global__ void __launch_bounds__(SN_THREADS) scalar_rmsnorm_kernel(const float* __restrict__ y, int ldy, const T* __restrict__ bias, const T* __restrict__ gain, float mult,
                                                                     float eps, int W, const float* res, float* out, int ldo, T* __restrict__ out_t, int ldt,
                                                                     const int32_t* __restrict__ rows) {
+    pdl_enter();
     __shared__ float scratch[33];
     const int i = blockIdx.x;
     const int src = rows ? rows[i] : i;
@@ -120,21 +125,22 @@ int launch_scalar_rmsnorm(int dt, const float* y, int ldy, const void* bias, con
                           int ldo, void* out_t, int ldt, const int32_t* rows, cudaStream_t s) {
     if (n <= 0) return WF_OK;
     if (res && rows && out == res) { set_error("scalar_rmsnorm: gathered rows cannot be added in place"); return WF_ERR_INVALID; }
-    if (dt == WF_BF16) scalar_rmsnorm_kernel<<<n, SN_THREADS, 0, s>>>(y, ldy, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)gain, mult, eps, W, res, out, ldo, (__nv_bfloat16*)out_t, ldt, rows);
-    else scalar_rmsnorm_kernel<<<n, SN_THREADS, 0, s>>>(y, ldy, (const float*)bias, (const float*)gain, mult, eps, W, res, out, ldo, (float*)out_t, ldt, rows);
+    if (dt == WF_BF16) launch_pdl(scalar_rmsnorm_kernel<__nv_bfloat16>, n, SN_THREADS, 0, s, y, ldy, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)gain, mult, eps, W, res, out, ldo, (__nv_bfloat16*)out_t, ldt, rows);
+    else launch_pdl(scalar_rmsnorm_kernel<float>, n, SN_THREADS, 0, s, y, ldy, (const float*)bias, (const float*)gain, mult, eps, W, res, out, ldo, (float*)out_t, ldt, rows);
     return launch_check(cudaGetLastError(), "scalar_rmsnorm");
 }
 
 // y[i, :] += bias
 template <typename T>
 __global__ void add_bias_kernel(float* __restrict__ y, int ld, const T* __restrict__ bias, int W) {
+    pdl_enter();
     for (int c = threadIdx.x; c < W; c += blockDim.x) y[(size_t)blockIdx.x * ld + c] += to_f(bias[c]);
 }
 
 int launch_add_bias(int dt, float* y, int ld, const void* bias, int n, int W, cudaStream_t s) {
     if (n <= 0 || !bias) return WF_OK;
-    if (dt == WF_BF16) add_bias_kernel<<<n, 256, 0, s>>>(y, ld, (const __nv_bfloat16*)bias, W);
-    else add_bias_kernel<<<n, 256, 0, s>>>(y, ld, (const float*)bias, W);
+    if (dt == WF_BF16) launch_pdl(add_bias_kernel<__nv_bfloat16>, n, 256, 0, s, y, ld, (const __nv_bfloat16*)bias, W);
+    else launch_pdl(add_bias_kernel<float>, n, 256, 0, s, y, ld, (const float*)bias, W);
     return launch_check(cudaGetLastError(), "add_bias");
 }
 
@@ -143,6 +149,7 @@ template <typename T>
 __global__ void group_rmsnorm_kernel(const float* __restrict__ x, int ldx, const T* __restrict__ w, int gw, float eps, const float* res,
                                      float* y, int ldy, T* __restrict__ y_t, int ldt, const int32_t* __restrict__ rows, const float* __restrict__ x2, float a,
                                      float b, float w_offset) {
+    pdl_enter();
     __shared__ float scratch[33];
     const int i = blockIdx.x, g = blockIdx.y;
     const int src = rows ? rows[i] : i;
@@ -168,8 +175,8 @@ int launch_group_rmsnorm(int dt, const float* x, int ldx, const void* w, int gro
     const int gw = W / groups;
     const int threads = gw >= 2048 ? 512 : (gw >= 1024 ? 256 : (gw >= 256 ? 128 : 64));
     dim3 grid(n, groups);
-    if (dt == WF_BF16) group_rmsnorm_kernel<<<grid, threads, 0, s>>>(x, ldx, (const __nv_bfloat16*)w, gw, eps, res, y, ldy, (__nv_bfloat16*)y_t, ldt, rows, x2, a, b, w_offset);
-    else group_rmsnorm_kernel<<<grid, threads, 0, s>>>(x, ldx, (const float*)w, gw, eps, res, y, ldy, (float*)y_t, ldt, rows, x2, a, b, w_offset);
+    if (dt == WF_BF16) launch_pdl(group_rmsnorm_kernel<__nv_bfloat16>, grid, threads, 0, s, x, ldx, (const __nv_bfloat16*)w, gw, eps, res, y, ldy, (__nv_bfloat16*)y_t, ldt, rows, x2, a, b, w_offset);
+    else launch_pdl(group_rmsnorm_kernel<float>, grid, threads, 0, s, x, ldx, (const float*)w, gw, eps, res, y, ldy, (float*)y_t, ldt, rows, x2, a, b, w_offset);
     return launch_check(cudaGetLastError(), "group_rmsnorm");
 }
 
@@ -180,6 +187,7 @@ template <typename T>
 __global__ void __launch_bounds__(AD_THREADS) add_dual_norm_kernel(float* __restrict__ x, const float* __restrict__ y1, float a1, const float* __restrict__ y2, float a2,
                                                                      const float* __restrict__ y3, const T* __restrict__ w1, const T* __restrict__ w2, float w_offset,
                                                                      float eps, int W, T* __restrict__ h1, T* __restrict__ h2) {
+    pdl_enter();
     __shared__ float scratch[33];
     const size_t base = (size_t)blockIdx.x * W;
     const bool adds = y1 || y2 || y3;
@@ -213,8 +221,8 @@ __global__ void __launch_bounds__(AD_THREADS) add_dual_norm_kernel(float* __rest
 int launch_add_dual_norm(int dt, float* x, const float* y1, float a1, const float* y2, float a2, const float* y3, const void* w1, const void* w2,
                          float w_offset, float eps, int n, int W, void* h1, void* h2, cudaStream_t s) {
     if (n <= 0) return WF_OK;
-    if (dt == WF_BF16) add_dual_norm_kernel<<<n, AD_THREADS, 0, s>>>(x, y1, a1, y2, a2, y3, (const __nv_bfloat16*)w1, (const __nv_bfloat16*)w2, w_offset, eps, W, (__nv_bfloat16*)h1, (__nv_bfloat16*)h2);
-    else add_dual_norm_kernel<<<n, AD_THREADS, 0, s>>>(x, y1, a1, y2, a2, y3, (const float*)w1, (const float*)w2, w_offset, eps, W, (float*)h1, (float*)h2);
+    if (dt == WF_BF16) launch_pdl(add_dual_norm_kernel<__nv_bfloat16>, n, AD_THREADS, 0, s, x, y1, a1, y2, a2, y3, (const __nv_bfloat16*)w1, (const __nv_bfloat16*)w2, w_offset, eps, W, (__nv_bfloat16*)h1, (__nv_bfloat16*)h2);
+    else launch_pdl(add_dual_norm_kernel<float>, n, AD_THREADS, 0, s, x, y1, a1, y2, a2, y3, (const float*)w1, (const float*)w2, w_offset, eps, W, (float*)h1, (float*)h2);
     return launch_check(cudaGetLastError(), "add_dual_norm");
 }
 
@@ -236,6 +244,7 @@ constexpr int LN_PER = 8;
 template <typename T>
 __global__ void __launch_bounds__(512) layer_norm_kernel(const float* __restrict__ x, int ldx, const T* __restrict__ w, const T* __restrict__ b, float eps, int W,
                                                          float* __restrict__ y, int ldy, T* __restrict__ y_t, int ldt, const int32_t* __restrict__ rows) {
+    pdl_enter();
     __shared__ float scratch[33];
     const int i = blockIdx.x;
     const float* row = x + (size_t)(rows ? rows[i] : i) * ldx;
@@ -269,8 +278,8 @@ int row_threads(int W) { return W > 1024 ? 512 : (W > 256 ? 256 : 128); }
 int launch_layer_norm(int dt, const float* x, int ldx, const void* w, const void* b, float eps, int n, int W, float* y, int ldy, void* y_t, int ldt,
                       const int32_t* rows, cudaStream_t s) {
     if (n <= 0) return WF_OK;
-    if (dt == WF_BF16) layer_norm_kernel<<<n, row_threads(W), 0, s>>>(x, ldx, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b, eps, W, y, ldy, (__nv_bfloat16*)y_t, ldt, rows);
-    else layer_norm_kernel<<<n, row_threads(W), 0, s>>>(x, ldx, (const float*)w, (const float*)b, eps, W, y, ldy, (float*)y_t, ldt, rows);
+    if (dt == WF_BF16) launch_pdl(layer_norm_kernel<__nv_bfloat16>, n, row_threads(W), 0, s, x, ldx, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b, eps, W, y, ldy, (__nv_bfloat16*)y_t, ldt, rows);
+    else launch_pdl(layer_norm_kernel<float>, n, row_threads(W), 0, s, x, ldx, (const float*)w, (const float*)b, eps, W, y, ldy, (float*)y_t, ldt, rows);
     return launch_check(cudaGetLastError(), "layer_norm");
 }
 
@@ -278,6 +287,7 @@ int launch_layer_norm(int dt, const float* x, int ldx, const void* w, const void
 template <typename T>
 __global__ void __launch_bounds__(512) branch_add_norm_kernel(float* __restrict__ x, BranchSum bs, const T* __restrict__ w, const T* __restrict__ b, float w_offset, float eps,
                                                               int W, T* __restrict__ h) {
+    pdl_enter();
     __shared__ float scratch[33];
     const size_t base = (size_t)blockIdx.x * W;
     float* row = x + base;
@@ -351,6 +361,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
 template <typename T, int NV>
 __global__ void __launch_bounds__(1024) branch_add_norm_vec_kernel(float* __restrict__ x, BranchSum bs, const T* __restrict__ w, const T* __restrict__ b, float w_offset, float eps,
                                                                    int W, T* __restrict__ h) {
+    pdl_enter();
     __shared__ float scratch[33];
     const size_t base = (size_t)blockIdx.x * W;
     const float* gate = bs.gate ? bs.gate + (size_t)blockIdx.x * bs.ldg : nullptr;
@@ -427,14 +438,14 @@ int launch_branch_add_norm(int dt, float* x, const BranchSum& bs, const void* w,
     // rows of up to 8192 elements that start 16-byte aligned stay in registers, four elements per load
     if (W % 4 == 0 && W <= 8192 && bs.ldg % 4 == 0 && ((uintptr_t)bs.gate & 15) == 0) {
         const int nv = W <= 1024 ? 1 : 2, threads = (W / 4 + nv * 32 - 1) / (nv * 32) * 32;
-#define BA_LAUNCH(T, NV) branch_add_norm_vec_kernel<T, NV><<<n, threads, 0, s>>>(x, bs, (const T*)w, (const T*)b, w_offset, eps, W, (T*)h)
+#define BA_LAUNCH(T, NV) launch_pdl(branch_add_norm_vec_kernel<T, NV>, n, threads, 0, s, x, bs, (const T*)w, (const T*)b, w_offset, eps, W, (T*)h)
         if (dt == WF_BF16) { if (nv == 1) BA_LAUNCH(__nv_bfloat16, 1); else BA_LAUNCH(__nv_bfloat16, 2); }
         else { if (nv == 1) BA_LAUNCH(float, 1); else BA_LAUNCH(float, 2); }
 #undef BA_LAUNCH
         return launch_check(cudaGetLastError(), "branch_add_norm_vec");
     }
-    if (dt == WF_BF16) branch_add_norm_kernel<<<n, row_threads(W), 0, s>>>(x, bs, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b, w_offset, eps, W, (__nv_bfloat16*)h);
-    else branch_add_norm_kernel<<<n, row_threads(W), 0, s>>>(x, bs, (const float*)w, (const float*)b, w_offset, eps, W, (float*)h);
+    if (dt == WF_BF16) launch_pdl(branch_add_norm_kernel<__nv_bfloat16>, n, row_threads(W), 0, s, x, bs, (const __nv_bfloat16*)w, (const __nv_bfloat16*)b, w_offset, eps, W, (__nv_bfloat16*)h);
+    else launch_pdl(branch_add_norm_kernel<float>, n, row_threads(W), 0, s, x, bs, (const float*)w, (const float*)b, w_offset, eps, W, (float*)h);
     return launch_check(cudaGetLastError(), "branch_add_norm");
 }
 
@@ -442,6 +453,7 @@ int launch_branch_add_norm(int dt, float* x, const BranchSum& bs, const void* w,
 template <typename T>
 __global__ void dyn_tanh_kernel(const float* __restrict__ x, int ldx, const T* __restrict__ w, const T* __restrict__ b, const T* __restrict__ alpha, int W,
                                 float* __restrict__ y, T* __restrict__ y_t, const int32_t* __restrict__ rows) {
+    pdl_enter();
     const int i = blockIdx.x;
     const float* xr = x + (size_t)(rows ? rows[i] : i) * ldx;
     const float al = to_f(alpha[0]);
@@ -456,8 +468,8 @@ int launch_dyn_tanh(int dt, const float* x, int ldx, const DynNorm& nm, int n, i
     if (n <= 0) return WF_OK;
     if (!nm.w || !nm.b || !nm.alpha) { set_error("dyn_tanh: weight, bias and alpha are needed"); return WF_ERR_INVALID; }
     const dim3 grid(n, n < 256 ? (W + 255) / 256 : 1);
-    if (dt == WF_BF16) dyn_tanh_kernel<<<grid, 256, 0, s>>>(x, ldx, (const __nv_bfloat16*)nm.w, (const __nv_bfloat16*)nm.b, (const __nv_bfloat16*)nm.alpha, W, y, (__nv_bfloat16*)y_t, rows);
-    else dyn_tanh_kernel<<<grid, 256, 0, s>>>(x, ldx, (const float*)nm.w, (const float*)nm.b, (const float*)nm.alpha, W, y, (float*)y_t, rows);
+    if (dt == WF_BF16) launch_pdl(dyn_tanh_kernel<__nv_bfloat16>, grid, 256, 0, s, x, ldx, (const __nv_bfloat16*)nm.w, (const __nv_bfloat16*)nm.b, (const __nv_bfloat16*)nm.alpha, W, y, (__nv_bfloat16*)y_t, rows);
+    else launch_pdl(dyn_tanh_kernel<float>, grid, 256, 0, s, x, ldx, (const float*)nm.w, (const float*)nm.b, (const float*)nm.alpha, W, y, (float*)y_t, rows);
     return launch_check(cudaGetLastError(), "dyn_tanh");
 }
 
@@ -480,6 +492,7 @@ __device__ __forceinline__ void dyn_apply(const DynNorm& nm, int c, const float 
 // grid (tokens, channel blocks).  VEC = 4: W a multiple of 4 (rows 16-byte aligned)
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) stream_step_kernel(float* __restrict__ x, StreamStep st, int W) {
+    pdl_enter();
     const int i = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * VEC;
     if (c >= W) return;
     const size_t at = (size_t)i * W + c;
@@ -541,19 +554,20 @@ int launch_stream_step(int dt, float* x, const StreamStep& st, int n, int W, cud
     const int vec = W % 4 == 0 ? 4 : 1, per = W / vec;
     const int threads = per >= 256 && n >= sm_count() ? 256 : (per > 64 ? 128 : 64);      // few tokens: more, smaller blocks
     const dim3 grid(n, (per + threads - 1) / threads);
-    if (dt == WF_BF16) { if (vec == 4) stream_step_kernel<__nv_bfloat16, 4><<<grid, threads, 0, s>>>(x, st, W); else stream_step_kernel<__nv_bfloat16, 1><<<grid, threads, 0, s>>>(x, st, W); }
-    else { if (vec == 4) stream_step_kernel<float, 4><<<grid, threads, 0, s>>>(x, st, W); else stream_step_kernel<float, 1><<<grid, threads, 0, s>>>(x, st, W); }
+    if (dt == WF_BF16) { if (vec == 4) launch_pdl(stream_step_kernel<__nv_bfloat16, 4>, grid, threads, 0, s, x, st, W); else launch_pdl(stream_step_kernel<__nv_bfloat16, 1>, grid, threads, 0, s, x, st, W); }
+    else { if (vec == 4) launch_pdl(stream_step_kernel<float, 4>, grid, threads, 0, s, x, st, W); else launch_pdl(stream_step_kernel<float, 1>, grid, threads, 0, s, x, st, W); }
     return launch_check(cudaGetLastError(), "stream_step");
 }
 
 __global__ void softcap_kernel(float* __restrict__ z, size_t count, float cap) {
+    pdl_enter();
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x) z[k] = cap * tanhf(z[k] / cap);
 }
 
 int launch_softcap(float* z, size_t count, float cap, cudaStream_t s) {
     if (count == 0) return WF_OK;
     const int blocks = (int)((count + 255) / 256 > 4096 ? 4096 : (count + 255) / 256);
-    softcap_kernel<<<blocks, 256, 0, s>>>(z, count, cap);
+    launch_pdl(softcap_kernel, blocks, 256, 0, s, z, count, cap);
     return launch_check(cudaGetLastError(), "softcap");
 }
 
@@ -562,6 +576,7 @@ template <typename T>
 __global__ void causal_taps_kernel(Batch b, const float* __restrict__ in, int ld_in, const T* __restrict__ w, int taps, int C,
                                    const float* __restrict__ state, size_t slot_stride, int identity, int silu, T* __restrict__ out_t, int ld_t,
                                    float* __restrict__ out_f, int ld_f, const T* __restrict__ bias) {
+    pdl_enter();
     const int i = blockIdx.x;
     const int sq = b.tok_seq[i];
     const int li = i - b.seq_start[sq];                    // index inside this step's portion
@@ -585,8 +600,8 @@ int launch_causal_taps(int dt, const Batch& b, const float* in, int ld_in, const
     if (b.n <= 0) return WF_OK;
     if (taps < 1) { set_error("causal_taps: taps %d", taps); return WF_ERR_INVALID; }
     dim3 grid(b.n, (C + 255) / 256 > 8 ? 8 : (C + 255) / 256);
-    if (dt == WF_BF16) causal_taps_kernel<<<grid, 256, 0, s>>>(b, in, ld_in, (const __nv_bfloat16*)w, taps, C, state, slot_stride, identity, silu, (__nv_bfloat16*)out_t, ld_t, out_f, ld_f, (const __nv_bfloat16*)bias);
-    else causal_taps_kernel<<<grid, 256, 0, s>>>(b, in, ld_in, (const float*)w, taps, C, state, slot_stride, identity, silu, (float*)out_t, ld_t, out_f, ld_f, (const float*)bias);
+    if (dt == WF_BF16) launch_pdl(causal_taps_kernel<__nv_bfloat16>, grid, 256, 0, s, b, in, ld_in, (const __nv_bfloat16*)w, taps, C, state, slot_stride, identity, silu, (__nv_bfloat16*)out_t, ld_t, out_f, ld_f, (const __nv_bfloat16*)bias);
+    else launch_pdl(causal_taps_kernel<float>, grid, 256, 0, s, b, in, ld_in, (const float*)w, taps, C, state, slot_stride, identity, silu, (float*)out_t, ld_t, out_f, ld_f, (const float*)bias);
     return launch_check(cudaGetLastError(), "causal_taps");
 }
 
@@ -594,6 +609,7 @@ int launch_causal_taps(int dt, const Batch& b, const float* in, int ld_in, const
 // Ascending k is safe in place: entry k reads old entry len + k > k.
 __global__ void taps_state_kernel(Batch b, const float* __restrict__ in, int ld_in, int taps, int C, float* __restrict__ state, size_t slot_stride,
                                   int skip_single) {
+    pdl_enter();
     const int sq = blockIdx.x;
     const int len = b.seq_len[sq], start = b.seq_start[sq];
     if (skip_single && len == 1) return;                 // rolled by the fused norm + taps kernel
@@ -609,7 +625,7 @@ __global__ void taps_state_kernel(Batch b, const float* __restrict__ in, int ld_
 int launch_taps_state(const Batch& b, const float* in, int ld_in, int taps, int C, float* state, size_t slot_stride, cudaStream_t s, int skip_single) {
     if (b.nseq <= 0 || taps <= 1) return WF_OK;
     dim3 grid(b.nseq, (C + 255) / 256 > 8 ? 8 : (C + 255) / 256);
-    taps_state_kernel<<<grid, 256, 0, s>>>(b, in, ld_in, taps, C, state, slot_stride, skip_single);
+    launch_pdl(taps_state_kernel, grid, 256, 0, s, b, in, ld_in, taps, C, state, slot_stride, skip_single);
     return launch_check(cudaGetLastError(), "taps_state");
 }
 
@@ -622,6 +638,7 @@ constexpr int NTAPS_MAX = 8;
 template <typename T>
 __global__ void norm_taps_kernel(Batch b, const float* __restrict__ x, int ldx, const T* __restrict__ nw, int groups, float eps, const T* __restrict__ cw,
                                  int taps, int W, float* __restrict__ state, size_t slot_stride, T* __restrict__ out_t, int ld_t, float* __restrict__ hn) {
+    pdl_enter();
     __shared__ float red[NTAPS_MAX][33];
     __shared__ float inv[NTAPS_MAX * 32];            // [tap][group]
     const int i = blockIdx.x;
@@ -684,14 +701,15 @@ int launch_norm_taps(int dt, const Batch& b, const float* x, int ldx, const void
     if (b.n <= 0) return WF_OK;
     if (!norm_taps_usable(groups, taps, W)) { set_error("norm_taps: %d groups / %d taps are beyond the fused kernel", groups, taps); return WF_ERR_UNSUPPORTED; }
     const int threads = W >= 2048 ? 512 : (W >= 512 ? 256 : 128);
-    if (dt == WF_BF16) norm_taps_kernel<<<b.n, threads, 0, s>>>(b, x, ldx, (const __nv_bfloat16*)nw, groups, eps, (const __nv_bfloat16*)cw, taps, W, state, slot_stride, (__nv_bfloat16*)out_t, ld_t, hn);
-    else norm_taps_kernel<<<b.n, threads, 0, s>>>(b, x, ldx, (const float*)nw, groups, eps, (const float*)cw, taps, W, state, slot_stride, (float*)out_t, ld_t, hn);
+    if (dt == WF_BF16) launch_pdl(norm_taps_kernel<__nv_bfloat16>, b.n, threads, 0, s, b, x, ldx, (const __nv_bfloat16*)nw, groups, eps, (const __nv_bfloat16*)cw, taps, W, state, slot_stride, (__nv_bfloat16*)out_t, ld_t, hn);
+    else launch_pdl(norm_taps_kernel<float>, b.n, threads, 0, s, b, x, ldx, (const float*)nw, groups, eps, (const float*)cw, taps, W, state, slot_stride, (float*)out_t, ld_t, hn);
     return launch_check(cudaGetLastError(), "norm_taps");
 }
 
 // ---- the same for many tokens: statistics once per row, then a fully parallel apply ------------------------------------------------
 // inv[row][group] = 1 / sqrt(mean_group(x^2) + eps): one warp per (row, group)
 __global__ void row_group_inv_rms_kernel(const float* __restrict__ x, int ldx, int n, int groups, int gw, float eps, float* __restrict__ inv) {
+    pdl_enter();
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (wid >= n * groups) return;
     const int row = wid / groups, g = wid - row * groups;
@@ -708,6 +726,7 @@ template <typename T, int VEC>
 __global__ void norm_taps_apply_kernel(Batch b, const float* __restrict__ x, int ldx, const float* __restrict__ inv, const T* __restrict__ nw, int groups,
                                        const T* __restrict__ cw, int taps, int W, const float* __restrict__ state, size_t slot_stride, T* __restrict__ out_t,
                                        int ld_t, float* __restrict__ hn) {
+    pdl_enter();
     const int i = blockIdx.x;
     const int sq = b.tok_seq[i];
     const int li = i - b.seq_start[sq], len = b.seq_len[sq];
@@ -750,22 +769,23 @@ int launch_norm_taps_rows(int dt, const Batch& b, const float* x, int ldx, const
     if (b.n <= 0) return WF_OK;
     if (groups < 1 || W % groups || taps < 1) { set_error("norm_taps_rows: %d groups / %d taps", groups, taps); return WF_ERR_INVALID; }
     const int warps = b.n * groups;
-    row_group_inv_rms_kernel<<<(warps + 7) / 8, 256, 0, s>>>(x, ldx, b.n, groups, W / groups, eps, inv);
+    launch_pdl(row_group_inv_rms_kernel, (warps + 7) / 8, 256, 0, s, x, ldx, b.n, groups, W / groups, eps, inv);
     if (int rc = launch_check(cudaGetLastError(), "row_group_inv_rms")) return rc;
     const bool vec = W % 4 == 0 && (W / groups) % 4 == 0 && ldx % 4 == 0 && (((uintptr_t)x) & 15) == 0;
     dim3 grid(b.n, vec ? (W + 1023) / 1024 : (W + 255) / 256);
     if (dt == WF_BF16) {
-        if (vec) norm_taps_apply_kernel<__nv_bfloat16, 4><<<grid, 256, 0, s>>>(b, x, ldx, inv, (const __nv_bfloat16*)nw, groups, (const __nv_bfloat16*)cw, taps, W, state, slot_stride, (__nv_bfloat16*)out_t, ld_t, hn);
-        else norm_taps_apply_kernel<__nv_bfloat16, 1><<<grid, 256, 0, s>>>(b, x, ldx, inv, (const __nv_bfloat16*)nw, groups, (const __nv_bfloat16*)cw, taps, W, state, slot_stride, (__nv_bfloat16*)out_t, ld_t, hn);
+        if (vec) launch_pdl(norm_taps_apply_kernel<__nv_bfloat16, 4>, grid, 256, 0, s, b, x, ldx, inv, (const __nv_bfloat16*)nw, groups, (const __nv_bfloat16*)cw, taps, W, state, slot_stride, (__nv_bfloat16*)out_t, ld_t, hn);
+        else launch_pdl(norm_taps_apply_kernel<__nv_bfloat16, 1>, grid, 256, 0, s, b, x, ldx, inv, (const __nv_bfloat16*)nw, groups, (const __nv_bfloat16*)cw, taps, W, state, slot_stride, (__nv_bfloat16*)out_t, ld_t, hn);
     } else {
-        if (vec) norm_taps_apply_kernel<float, 4><<<grid, 256, 0, s>>>(b, x, ldx, inv, (const float*)nw, groups, (const float*)cw, taps, W, state, slot_stride, (float*)out_t, ld_t, hn);
-        else norm_taps_apply_kernel<float, 1><<<grid, 256, 0, s>>>(b, x, ldx, inv, (const float*)nw, groups, (const float*)cw, taps, W, state, slot_stride, (float*)out_t, ld_t, hn);
+        if (vec) launch_pdl(norm_taps_apply_kernel<float, 4>, grid, 256, 0, s, b, x, ldx, inv, (const float*)nw, groups, (const float*)cw, taps, W, state, slot_stride, (float*)out_t, ld_t, hn);
+        else launch_pdl(norm_taps_apply_kernel<float, 1>, grid, 256, 0, s, b, x, ldx, inv, (const float*)nw, groups, (const float*)cw, taps, W, state, slot_stride, (float*)out_t, ld_t, hn);
     }
     return launch_check(cudaGetLastError(), "norm_taps_apply");
 }
 
 template <typename T>
 __global__ void gate_mul_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ g, int ldg, int act, int C, T* __restrict__ y, int ldy) {
+    pdl_enter();
     const int i = blockIdx.x;
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < C; c += gridDim.y * blockDim.x) {
         const float z = g[(size_t)i * ldg + c];
@@ -776,26 +796,28 @@ __global__ void gate_mul_kernel(const float* __restrict__ x, int ldx, const floa
 int launch_gate_mul(int dt, const float* x, int ldx, const float* g, int ldg, int act, int n, int C, void* y, int ldy, cudaStream_t s) {
     if (n <= 0) return WF_OK;
     const dim3 grid(n, n < 64 ? (C + 255) / 256 : 1);
-    if (dt == WF_BF16) gate_mul_kernel<<<grid, 256, 0, s>>>(x, ldx, g, ldg, act, C, (__nv_bfloat16*)y, ldy);
-    else gate_mul_kernel<<<grid, 256, 0, s>>>(x, ldx, g, ldg, act, C, (float*)y, ldy);
+    if (dt == WF_BF16) launch_pdl(gate_mul_kernel<__nv_bfloat16>, grid, 256, 0, s, x, ldx, g, ldg, act, C, (__nv_bfloat16*)y, ldy);
+    else launch_pdl(gate_mul_kernel<float>, grid, 256, 0, s, x, ldx, g, ldg, act, C, (float*)y, ldy);
     return launch_check(cudaGetLastError(), "gate_mul");
 }
 
 template <typename T>
 __global__ void gather_rows_kernel(const T* __restrict__ src, int ld, const int32_t* __restrict__ rows, int W, T* __restrict__ dst) {
+    pdl_enter();
     const int i = blockIdx.x, r = rows[i];
     for (int c = threadIdx.x; c < W; c += blockDim.x) dst[(size_t)i * W + c] = r >= 0 ? src[(size_t)r * ld + c] : from_f<T>(0.f);
 }
 
 int launch_gather_rows(int dt, const void* src, int ld, const int32_t* rows, int P, int W, void* dst, cudaStream_t s) {
     if (P <= 0) return WF_OK;
-    if (dt == WF_BF16) gather_rows_kernel<<<P, 256, 0, s>>>((const __nv_bfloat16*)src, ld, rows, W, (__nv_bfloat16*)dst);
-    else gather_rows_kernel<<<P, 256, 0, s>>>((const float*)src, ld, rows, W, (float*)dst);
+    if (dt == WF_BF16) launch_pdl(gather_rows_kernel<__nv_bfloat16>, P, 256, 0, s, (const __nv_bfloat16*)src, ld, rows, W, (__nv_bfloat16*)dst);
+    else launch_pdl(gather_rows_kernel<float>, P, 256, 0, s, (const float*)src, ld, rows, W, (float*)dst);
     return launch_check(cudaGetLastError(), "gather_rows");
 }
 
 template <typename T>
 __global__ void transpose_heads_kernel(const T* __restrict__ in, int R, int C, T* __restrict__ out) {
+    pdl_enter();
     const size_t h = blockIdx.y;
     for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < R * C; idx += gridDim.x * blockDim.x) {
         const int r = idx / C, c = idx % C;
@@ -805,8 +827,8 @@ __global__ void transpose_heads_kernel(const T* __restrict__ in, int R, int C, T
 
 int launch_transpose_heads(int dt, const void* in, int H, int R, int C, void* out, cudaStream_t s) {
     dim3 grid((R * C + 255) / 256 > 1024 ? 1024 : (R * C + 255) / 256, H);
-    if (dt == WF_BF16) transpose_heads_kernel<<<grid, 256, 0, s>>>((const __nv_bfloat16*)in, R, C, (__nv_bfloat16*)out);
-    else transpose_heads_kernel<<<grid, 256, 0, s>>>((const float*)in, R, C, (float*)out);
+    if (dt == WF_BF16) launch_pdl(transpose_heads_kernel<__nv_bfloat16>, grid, 256, 0, s, (const __nv_bfloat16*)in, R, C, (__nv_bfloat16*)out);
+    else launch_pdl(transpose_heads_kernel<float>, grid, 256, 0, s, (const float*)in, R, C, (float*)out);
     return launch_check(cudaGetLastError(), "transpose_heads");
 }
 
