@@ -44,3 +44,26 @@ def test_the_workspaces_of_the_faster_forms_are_not_required(monkeypatch):
         del held
         torch.cuda.empty_cache()
     assert size == small and np.array_equal(tight, plain)
+
+
+@pytest.mark.parametrize("vocab,wants", [(4099, (1, 64, 65, 130)), (65536, (1, 4, 5, 9))])
+def test_logits_reach_pageable_memory_as_they_reach_pinned(vocab, wants):
+    """One piece, whole pieces, a part of a piece, more pieces than are in flight at once (256 KB each, four at once): equal to one copy into pinned memory."""
+    from wf_bitnet._lib import seq_check, seq_lib
+    from test_gpu_tutizen import attn, build, config, make_weights, with_ff, dense
+    cfg = config([with_ff(attn(), dense())], vocab=vocab)
+    m = build(cfg, make_weights(cfg, 3), "bfloat16", max_tokens=1024, slots=2, page_size=16, max_step_tokens=256)
+    rng = np.random.default_rng(vocab)
+    for n in wants:
+        toks = rng.integers(0, vocab, max(n, 2)).astype(np.int32)
+        rows = np.sort(rng.choice(toks.size, n, replace=False)).astype(np.int32)
+        slot = m.admit()
+        got = m.step([slot], [toks.size], toks, rows)
+        m.release(slot)
+        pinned = torch.full((n, vocab), float("nan")).pin_memory()
+        slot = m.admit()
+        s, c = np.array([slot], np.int32), np.array([toks.size], np.int32)
+        seq_check(seq_lib().wf_seq_step(m.engine._h, 1, s.ctypes.data, c.ctypes.data, toks.ctypes.data, n, rows.ctypes.data, pinned.data_ptr()))
+        m.release(slot)
+        assert np.isfinite(got).all() and np.array_equal(got, pinned.numpy()), n
+    m.close()

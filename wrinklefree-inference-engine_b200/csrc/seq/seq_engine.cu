@@ -19,6 +19,9 @@ using namespace wf::seq;
 
 namespace {
 
+constexpr int OUT_CHUNKS = 4;
+constexpr size_t OUT_CHUNK = 256 * 1024;
+
 struct TensorSlot {
     std::string name;
     void* dst = nullptr;      // where the elements go (device)
@@ -107,8 +110,13 @@ struct wf_seq_engine {
     size_t slot_stride = 0;           // floats per slot
     int32_t* d_block_table = nullptr;
     // step metadata
-    int32_t *h_meta = nullptr, *d_meta = nullptr;
+    int32_t *h_meta = nullptr, *d_meta = nullptr;   // the step's index arrays, and behind them the block table; pinned on the host
     size_t meta_ints = 0;
+    bool staged = false;              // a copy from h_meta may be under way: the step that issued it has not been waited for
+    // logits on their way to the caller's memory, and the tcgen05 kernels' error word: pinned, OUT_CHUNKS pieces in turn
+    unsigned char* h_out = nullptr;
+    cudaEvent_t out_ev[4] = {nullptr, nullptr, nullptr, nullptr};
+    int* h_err = nullptr;
     // workspace
     float *x = nullptr, *hn = nullptr, *y = nullptr, *proj = nullptr, *qr = nullptr, *qa = nullptr, *ov = nullptr, *qkvc = nullptr, *beta = nullptr,
           *decay = nullptr, *od = nullptr, *z = nullptr, *wts = nullptr, *gu = nullptr, *yexp = nullptr;
@@ -342,13 +350,46 @@ struct StepView {
     const int32_t* want;
 };
 
-// after a step's synchronisation: whether a bounded wait of the tcgen05 kernels ran out, and where
+// whether a bounded wait of the tcgen05 kernels ran out, and where, by the word that finish_step brought
 int check_waits(wf_seq_engine* e, const char* who) {
-    const int code = e->dt == WF_BF16 ? gemm_tc_error(e->stream) : 0;
+    const int code = *e->h_err;
     if (!code) return WF_OK;
-    if (code < 0) set_error("%s: the tcgen05 kernels' error word cannot be read", who);
-    else set_error("%s: a bounded wait of the tcgen05 %s ran out (%d)", who, code <= 3 ? "matrix product" : "attention", code);
+    set_error("%s: a bounded wait of the tcgen05 %s ran out (%d)", who, code <= 3 ? "matrix product" : "attention", code);
     return WF_ERR_CUDA;
+}
+
+// Waits for the step's kernels; count bytes at src come to host memory on the way, with the error word.  Pageable memory is filled through pinned pieces, the
+// next ones being copied meanwhile: 1 MB of logits in 55 us, 94 as one copy into pageable memory, and one wait in place of two.
+int finish_step(wf_seq_engine* e, const char* who, const void* src = nullptr, void* dst = nullptr, size_t count = 0) {
+    *e->h_err = 0;
+    if (int* word = e->dt == WF_BF16 ? tc_error_word(false) : nullptr)
+        if (cuda_check(cudaMemcpyAsync(e->h_err, word, 4, cudaMemcpyDeviceToHost, e->stream), who)) return WF_ERR_CUDA;
+    cudaPointerAttributes pa;
+    bool pageable = false;
+    if (count > 0) {
+        if (cudaPointerGetAttributes(&pa, dst) == cudaSuccess) pageable = pa.type == cudaMemoryTypeUnregistered;
+        else cudaGetLastError();
+    }
+    if (count > 0 && !pageable) {
+        if (cuda_check(cudaMemcpyAsync(dst, src, count, cudaMemcpyDeviceToHost, e->stream), who)) return WF_ERR_CUDA;
+    } else {
+        const size_t pieces = (count + OUT_CHUNK - 1) / OUT_CHUNK;
+        for (size_t i = 0; i < pieces + OUT_CHUNKS; ++i) {
+            if (i >= OUT_CHUNKS && i - OUT_CHUNKS < pieces) {           // piece i - OUT_CHUNKS leaves the slot that piece i is to have
+                const size_t j = i - OUT_CHUNKS, at = j * OUT_CHUNK;
+                if (cuda_check(cudaEventSynchronize(e->out_ev[j % OUT_CHUNKS]), who)) return WF_ERR_CUDA;
+                memcpy((unsigned char*)dst + at, e->h_out + j % OUT_CHUNKS * OUT_CHUNK, std::min(OUT_CHUNK, count - at));
+            }
+            if (i < pieces) {
+                const size_t at = i * OUT_CHUNK;
+                if (cuda_check(cudaMemcpyAsync(e->h_out + i % OUT_CHUNKS * OUT_CHUNK, (const unsigned char*)src + at, std::min(OUT_CHUNK, count - at), cudaMemcpyDeviceToHost, e->stream), who) ||
+                    cuda_check(cudaEventRecord(e->out_ev[i % OUT_CHUNKS], e->stream), who)) return WF_ERR_CUDA;
+            }
+        }
+    }
+    if (cuda_check(cudaStreamSynchronize(e->stream), who)) return WF_ERR_CUDA;
+    e->staged = false;
+    return check_waits(e, who);
 }
 
 // host bookkeeping + one H2D copy of a step's index arrays
@@ -380,6 +421,8 @@ int prepare_step(wf_seq_engine* e, int nseq, const int32_t* slots, const int32_t
             return WF_ERR_INVALID;
         }
     }
+    if (e->staged && cuda_check(cudaStreamSynchronize(e->stream), "sync")) return WF_ERR_CUDA;      // a step that failed behind its copies
+    e->staged = false;
     int32_t* m = e->h_meta;
     const size_t T = c.max_step_tokens, S = c.slots;
     int32_t *m_tok = m, *m_tseq = m + T, *m_tpos = m + 2 * T, *m_start = m + 3 * T, *m_len = m_start + S, *m_pos0 = m_len + S, *m_slot = m_pos0 + S,
@@ -399,14 +442,13 @@ int prepare_step(wf_seq_engine* e, int nseq, const int32_t* slots, const int32_t
         ctx += m_pos0[i] + counts[i];
     }
     v->b.ctx_total = (int)ctx;                      // at most the pool's tokens
-    if (cuda_check(cudaMemcpyAsync(e->d_meta, m, e->meta_ints * 4, cudaMemcpyHostToDevice, e->stream), "step metadata H2D")) return WF_ERR_CUDA;
-    if (e->pt.dirty) {
-        std::vector<int32_t> tmp(e->pt.table);
-        for (auto& p : tmp) if (p < 0) p = 0;      // a stale lookup can never leave the pool
-        if (cuda_check(cudaMemcpyAsync(e->d_block_table, tmp.data(), tmp.size() * 4, cudaMemcpyHostToDevice, e->stream), "block table H2D")) return WF_ERR_CUDA;
-        if (cuda_check(cudaStreamSynchronize(e->stream), "sync")) return WF_ERR_CUDA;   // tmp is pageable
+    size_t ints = e->meta_ints;
+    if (e->pt.dirty) {                              // the block table goes with them
+        for (int32_t p : e->pt.table) m[ints++] = p < 0 ? 0 : p;      // a stale lookup can never leave the pool
         e->pt.dirty = false;
     }
+    e->staged = true;
+    if (cuda_check(cudaMemcpyAsync(e->d_meta, m, ints * 4, cudaMemcpyHostToDevice, e->stream), "step metadata H2D")) { e->pt.dirty = true; return WF_ERR_CUDA; }
     int32_t* d = e->d_meta;
     v->tokens = d;
     v->b.n = n; v->b.nseq = nseq;
@@ -1520,10 +1562,15 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     const int max_blocks = c.max_pages;        // one sequence may hold the whole pool
     e->pt.init(c.max_pages, c.page_size, c.slots, max_blocks);
     e->h_len.assign(c.slots, 0);
-    TRY(dalloc_n(e, &e->d_block_table, (size_t)c.slots * max_blocks));
     e->meta_ints = (size_t)4 * T + (size_t)5 * c.slots;
-    TRY(dalloc_n(e, &e->d_meta, e->meta_ints));
-    if (cuda_check(cudaMallocHost((void**)&e->h_meta, e->meta_ints * 4), "pinned metadata")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
+    const size_t with_table = e->meta_ints + (size_t)c.slots * max_blocks;
+    TRY(dalloc_n(e, &e->d_meta, with_table));
+    e->d_block_table = e->d_meta + e->meta_ints;
+    if (cuda_check(cudaMallocHost((void**)&e->h_meta, with_table * 4), "pinned metadata")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
+    if (cuda_check(cudaMallocHost((void**)&e->h_out, OUT_CHUNKS * OUT_CHUNK + 64), "pinned results")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
+    e->h_err = (int*)(e->h_out + OUT_CHUNKS * OUT_CHUNK);
+    for (auto& ev : e->out_ev)
+        if (cuda_check(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
     // workspaces
     TRY(dalloc_n(e, &e->row_inv, (size_t)T * c.norm_groups));
     TRY(dalloc_n(e, &e->x, (size_t)T * W)); TRY(dalloc_n(e, &e->hn, (size_t)T * W)); TRY(dalloc_n(e, &e->y, (size_t)T * W));
@@ -1600,6 +1647,8 @@ extern "C" void wf_seq_destroy(wf_seq_engine* e) {
     if (e->d_uniform) cudaFree(e->d_uniform);
     if (e->d_next) cudaFree(e->d_next);
     if (e->h_meta) cudaFreeHost(e->h_meta);
+    if (e->h_out) cudaFreeHost(e->h_out);
+    for (auto& ev : e->out_ev) if (ev) cudaEventDestroy(ev);
     if (e->stream) cudaStreamDestroy(e->stream);
     delete e;
 }
@@ -1756,10 +1805,7 @@ extern "C" int wf_seq_step(wf_seq_engine* e, int nseq, const int32_t* slots, con
     const long long l0 = launch_count();
     if ((rc = run_model(e, v, nwant))) return rc;
     if (launch_count() > l0) e->launches = (int)(launch_count() - l0);     // a graph replay launches what its capture counted
-    if (logits_host && nwant > 0)
-        if (cuda_check(cudaMemcpyAsync(logits_host, e->logits, (size_t)nwant * e->cfg.vocab * 4, cudaMemcpyDeviceToHost, e->stream), "logits D2H")) return WF_ERR_CUDA;
-    if (cuda_check(cudaStreamSynchronize(e->stream), "wf_seq_step")) return WF_ERR_CUDA;
-    if ((rc = check_waits(e, "wf_seq_step"))) return rc;
+    if ((rc = finish_step(e, "wf_seq_step", e->logits, logits_host, logits_host && nwant > 0 ? (size_t)nwant * e->cfg.vocab * 4 : 0))) return rc;
     commit_lengths(e, nseq, slots, counts);
     return WF_OK;
 }
@@ -1841,9 +1887,7 @@ extern "C" int wf_seq_run_part(wf_seq_engine* e, int layer, int part, int nseq, 
         if (!rc && part == 2 && L.ob && norm_takes_bias(e, L)) rc = launch_add_bias(e->dt, e->y, W, L.ob, n, W, s);
     } else { set_error("wf_seq_run_part: unknown part %d", part); return WF_ERR_INVALID; }
     if (rc) return rc;
-    if (cuda_check(cudaMemcpyAsync(out_host, result, bytes, cudaMemcpyDeviceToHost, s), "out")) return WF_ERR_CUDA;
-    if (cuda_check(cudaStreamSynchronize(s), "wf_seq_run_part")) return WF_ERR_CUDA;
-    if ((rc = check_waits(e, "wf_seq_run_part"))) return rc;
+    if ((rc = finish_step(e, "wf_seq_run_part", result, out_host, bytes))) return rc;
     commit_lengths(e, nseq, slots, counts);
     return WF_OK;
 }
@@ -1913,13 +1957,14 @@ extern "C" int wf_seq_time_step(wf_seq_engine* e, int nseq, const int32_t* slots
     }
     cudaEventRecord(e1, e->stream);
     const cudaError_t ce = cudaStreamSynchronize(e->stream);
+    e->staged = false;
     float ms = 0.f;
     if (!rc && ce == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0); cudaEventDestroy(e1);
     for (int i = 0; i < nseq; ++i) e->pt.truncate(slots[i], e->h_len[slots[i]]);   // the timed tokens are not kept
     if (rc) return rc;
     if (cuda_check(ce, "wf_seq_time_step")) return WF_ERR_CUDA;
-    if ((rc = check_waits(e, "wf_seq_time_step"))) return rc;
+    if ((rc = finish_step(e, "wf_seq_time_step"))) return rc;
     *ms_out = ms / iters;
     return WF_OK;
 }

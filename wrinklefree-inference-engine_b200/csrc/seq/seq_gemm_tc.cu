@@ -319,11 +319,11 @@ void* tensor_map_encoder() {
     return (void*)g_encode;
 }
 
-int* tc_error_word() {
+int* tc_error_word(bool make) {
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev > 63) dev = 0;
-    if (!g_err_dev[dev]) {
+    if (!g_err_dev[dev] && make) {
         if (cuda_check(cudaMalloc((void**)&g_err_dev[dev], 4), "cudaMalloc")) { g_err_dev[dev] = nullptr; return nullptr; }
         if (cuda_check(cudaMemset(g_err_dev[dev], 0, 4), "memset")) return nullptr;
     }

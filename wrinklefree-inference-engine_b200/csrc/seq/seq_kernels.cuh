@@ -124,7 +124,7 @@ bool gemm_tc_usable(const GemmArgs& g);
 int launch_gemm_tc(const GemmArgs& g, int n_groups, cudaStream_t s);
 // shared by the tcgen05 kernels: the driver's tensor-map encoder (null: unavailable) and the current device's error word (null: no memory)
 void* tensor_map_encoder();
-int* tc_error_word();
+int* tc_error_word(bool make = true);       // the device's word (make: allocated where there is none yet)
 int gemm_tc_error(cudaStream_t s);           // 0 = no bounded wait of the tcgen05 kernel ever ran out on this device
 // dst T [P, W] = src T [rows[i], :] (zero rows where rows[i] < 0)
 int launch_gather_rows(int dt, const void* src, int ld, const int32_t* rows, int P, int W, void* dst, cudaStream_t s);
