@@ -126,6 +126,106 @@ __global__ void __launch_bounds__(GP_MAXW * 32) gqa_prep_kernel(Batch b, GqaDims
     }
 }
 
+// The same for head sizes that are multiples of 4 up to 128 (no norm over the whole projection; pairs side by side, or half the rotated entries apart with
+// that half a multiple of 4): a head vector lies in the lanes of a warp four entries each, a warp's GQ vectors are requested before the cosines are formed,
+// and a pair's other entry comes from its lane.  2048 tokens, 20 + 5 + 5 heads of 128 with a gate per element (88 MB): 62 us one entry at a time, 24 so.
+constexpr int GQ = 4;
+template <typename T>
+__global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D, const float* __restrict__ proj, int ld, int k_off, int v_off, int g_off, const T* __restrict__ qb,
+                                                           const T* __restrict__ kb, const T* __restrict__ vb, float eps, PagedCache pc, T* __restrict__ qn,
+                                                           float* __restrict__ gate) {
+    pdl_enter();
+    __shared__ float rot_c[64], rot_s[64];
+    const int i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = 4 * lane;
+    const int sq = b.tok_seq[i], pos = b.tok_pos[i];
+    const float* row = proj + (size_t)i * ld;
+    const int units = D.H + (k_off >= 0 ? (D.v_is_k ? D.G : 2 * D.G) : 0);
+    T* page = nullptr;
+    if (k_off >= 0) {
+        const int pg = pc.block_table[(size_t)b.seq_slot[sq] * pc.max_blocks + pos / pc.page_size];
+        page = (T*)pc.pool + (size_t)pg * pc.page_stride + pc.layer_off;
+    }
+    const int slot = pos % pc.page_size, half = D.rope_dims / 2;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u0 = warp; u0 == warp || u0 < units; u0 += 8 * GQ) {         // every warp comes by the barrier
+        float4 x[GQ], bi[GQ];
+#pragma unroll
+        for (int k = 0; k < GQ; ++k) {
+            const int u = u0 + 8 * k, g = u - D.H - (u >= D.H + D.G ? D.G : 0);
+            const bool isq = u < D.H, isk = !isq && u < D.H + D.G;
+            const int dim = isq || isk ? D.d : D.dv;
+            const bool in = u < units && c < dim;
+            const T* bias = isq ? qb : isk ? kb : vb;
+            const int at = (isq ? u : g) * dim + c;
+            x[k] = in ? load4(row + (isq ? 0 : isk ? k_off : v_off) + at) : zero;
+            bi[k] = in && bias ? load4(bias + at) : zero;
+        }
+        if (u0 == warp) {
+            const int table = (half + 31) & ~31, t = (int)threadIdx.x - table;       // the other warps form the gates meanwhile
+            if ((int)threadIdx.x < half) {
+                const double a = (double)pos * (D.freq ? D.freq[threadIdx.x] : exp2(-2.0 * (double)threadIdx.x / (double)D.rope_dims * log2((double)D.rope_base)));
+                double sn, cs;
+                sincos(a, &sn, &cs);
+                rot_c[threadIdx.x] = (float)cs * D.mscale; rot_s[threadIdx.x] = (float)sn * D.mscale;
+            } else if (gate && t >= 0) {
+                const int ng = D.gate_elem ? D.H * D.dv : D.H, nt = 256 - table;
+                if (ng % 4 == 0 && g_off % 4 == 0 && g_off >= 0) {
+                    for (int h = t * 4; h < ng; h += nt * 4) {
+                        const float4 z = load4(row + g_off + h);
+                        const float o[4] = {sigmoid_f(z.x), sigmoid_f(z.y), sigmoid_f(z.z), sigmoid_f(z.w)};
+                        store4(gate + (size_t)i * ng + h, o);
+                    }
+                } else {
+                    for (int h = t; h < ng; h += nt) gate[(size_t)i * ng + h] = g_off >= 0 ? sigmoid_f(row[g_off + h]) : 1.f;
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int k = 0; k < GQ; ++k) {
+            const int u = u0 + 8 * k;
+            if (u >= units) break;
+            const bool isq = u < D.H, isk = !isq && u < D.H + D.G;
+            const int g = isq ? u : u - D.H - (isk ? 0 : D.G), dim = isq || isk ? D.d : D.dv;
+            const int norm = isq || isk ? D.qk_norm : (D.v_norm ? 1 : 0);
+            float v[4] = {x[k].x + bi[k].x, x[k].y + bi[k].y, x[k].z + bi[k].z, x[k].w + bi[k].w};
+            if (norm) {
+                const float ss = warp_sum(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]);
+                const float inv = 1.f / sqrtf(ss / (float)dim + eps);
+                const T* nw = norm == 2 ? (const T*)(isq ? D.q_norm_w : D.k_norm_w) : nullptr;
+                const float4 m = nw && c < dim ? load4(nw + c) : make_float4(1.f, 1.f, 1.f, 1.f);
+                v[0] = v[0] * inv * m.x; v[1] = v[1] * inv * m.y; v[2] = v[2] * inv * m.z; v[3] = v[3] * inv * m.w;
+            }
+            if (half > 0 && (isq || isk)) {
+                if (D.rope_interleaved) {
+                    if (c < D.rope_dims) {
+#pragma unroll
+                        for (int e = 0; e < 4; e += 2) {
+                            if (c + e >= D.rope_dims) break;
+                            const int p = (c + e) >> 1;
+                            const float f = v[e], s = v[e + 1];
+                            v[e] = f * rot_c[p] - s * rot_s[p];
+                            v[e + 1] = s * rot_c[p] + f * rot_s[p];
+                        }
+                    }
+                } else {
+                    const bool in = c < D.rope_dims, first = c < half;
+                    const int from = in ? (first ? lane + half / 4 : lane - half / 4) : lane;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float o = __shfl_sync(0xffffffffu, v[e], from);
+                        if (in) { const int p = first ? c + e : c + e - half; v[e] = first ? v[e] * rot_c[p] - o * rot_s[p] : v[e] * rot_c[p] + o * rot_s[p]; }
+                    }
+                }
+            }
+            if (c >= dim) continue;
+            T* dst = isq ? qn + ((size_t)i * D.H + u) * D.d
+                         : isk ? page + ((size_t)g * pc.page_size + slot) * D.d : page + (size_t)D.G * pc.page_size * D.d + ((size_t)g * pc.page_size + slot) * D.dv;
+            store4(dst + c, v);
+        }
+    }
+}
+
 // One block per (token, head).  Its warps take the visible keys (the kept first ones, then the window) round-robin, a warp one key at a time
 // with its lanes over the dimensions; running max / sum / weighted value sum per warp, merged through shared memory.
 template <typename T>
@@ -313,6 +413,13 @@ int launch_gqa_prep(int dt, const Batch& b, const GqaDims& D, const float* proj,
     if (int rc = check_dims(D)) return rc;
     if (!D.v_is_k && (k_off >= 0) != (v_off >= 0)) { set_error("attention: keys and values are projected together or not at all"); return WF_ERR_INVALID; }
     const bool small = D.d <= 128 && D.dv <= 128;
+    if (small && D.d % 4 == 0 && D.dv % 4 == 0 && D.qk_norm < 3 && (D.rope_interleaved || D.rope_dims % 8 == 0) && ld % 4 == 0 && (k_off < 0 || (k_off % 4 == 0 && (D.v_is_k || v_off % 4 == 0))) &&
+        (k_off < 0 || (pc.layer_off % 4 == 0 && pc.page_stride % 4 == 0 && vec_ok(pc.pool, 16))) && vec_ok(proj, 16) && vec_ok(qb, 16) && vec_ok(kb, 16) && vec_ok(vb, 16) && vec_ok(qn, 16) && vec_ok(gate, 16) &&
+        vec_ok(D.q_norm_w, 16) && vec_ok(D.k_norm_w, 16)) {
+        if (dt == WF_BF16) launch_pdl(gqa_prep_vec_kernel<__nv_bfloat16>, b.n, 256, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const __nv_bfloat16*)qb, (const __nv_bfloat16*)kb, (const __nv_bfloat16*)vb, eps, pc, (__nv_bfloat16*)qn, gate);
+        else launch_pdl(gqa_prep_vec_kernel<float>, b.n, 256, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const float*)qb, (const float*)kb, (const float*)vb, eps, pc, (float*)qn, gate);
+        return launch_check(cudaGetLastError(), "gqa_prep_vec");
+    }
     const int threads = 32 * (b.n <= sm_count() ? GP_MAXW : GA_WARPS);
 #define GP_LAUNCH(T, MD) launch_pdl(gqa_prep_kernel<T, MD>, b.n, threads, (size_t)threads * MD * sizeof(float), s, b, D, proj, ld, k_off, v_off, g_off, (const T*)qb, (const T*)kb, (const T*)vb, eps, pc, (T*)qn, gate)
     if (dt == WF_BF16) { if (small) GP_LAUNCH(__nv_bfloat16, 4); else GP_LAUNCH(__nv_bfloat16, GA_MAXD); }

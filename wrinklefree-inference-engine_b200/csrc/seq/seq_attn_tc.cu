@@ -169,7 +169,7 @@ __device__ __noinline__ void at_row(const Batch& b, const AtParams& p, int head,
 template <bool SPLIT>
 __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ Batch b,
                                                                 const __grid_constant__ AtParams p) {
-    pdl_enter();
+    pdl_wait_prior();
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t q_full[2], k_full[2], k_empty[2], v_full[2], v_empty[2], v_fixed, s_full[2], p_full[2], o_full[2], drained;
     __shared__ uint32_t tmem_base_s;

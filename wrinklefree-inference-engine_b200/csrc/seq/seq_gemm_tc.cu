@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_s;
-    pdl_enter();                                       // barriers, TMEM and the pair's meeting above overlap the kernel before
+    pdl_wait_prior();                                  // barriers, TMEM and the pair's meeting above overlap the kernel before
 
     // every role of both CTAs walks the same list of tiles and skips the same ones; `it` counts ring items, `done` counts tiles that were computed
     if (warp == TC_EPW) {

@@ -5,14 +5,22 @@
 namespace wf {
 namespace seq {
 
-template <typename T>
+// VEC = 4: W a multiple of 4, everything aligned (2048 x 2560 bf16: 13 us one element at a time, 7 so)
+template <typename T, int VEC>
 __global__ void embed_f32_kernel(const T* __restrict__ table, const int32_t* __restrict__ tokens, int W, float* __restrict__ x, float scale, T* __restrict__ x_t,
                                  const T* __restrict__ pos_table, const int32_t* __restrict__ tok_pos) {
     pdl_enter();
     const int i = blockIdx.x;
     const T* row = table + (size_t)tokens[i] * W;
     const T* prow = pos_table ? pos_table + (size_t)tok_pos[i] * W : nullptr;
-    for (int c = threadIdx.x; c < W; c += blockDim.x) {
+    for (int c = threadIdx.x * VEC; c < W; c += blockDim.x * VEC) {
+        if (VEC == 4) {
+            const float4 a = load4(row + c), q = prow ? load4(prow + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float v[4] = {a.x * scale + q.x, a.y * scale + q.y, a.z * scale + q.z, a.w * scale + q.w};
+            store4(x + (size_t)i * W + c, v);
+            if (x_t) store4(x_t + (size_t)i * W + c, v);
+            continue;
+        }
         float v = to_f(row[c]) * scale;
         if (prow) v += to_f(prow[c]);
         x[(size_t)i * W + c] = v;
@@ -23,8 +31,11 @@ __global__ void embed_f32_kernel(const T* __restrict__ table, const int32_t* __r
 int launch_embed_f32(int dt, const void* table, const int32_t* tokens, int n, int W, float* x, cudaStream_t s, float scale, void* x_t,
                      const void* pos_table, const int32_t* tok_pos) {
     if (n <= 0) return WF_OK;
-    if (dt == WF_BF16) launch_pdl(embed_f32_kernel<__nv_bfloat16>, n, 256, 0, s, (const __nv_bfloat16*)table, tokens, W, x, scale, (__nv_bfloat16*)x_t, (const __nv_bfloat16*)pos_table, tok_pos);
-    else launch_pdl(embed_f32_kernel<float>, n, 256, 0, s, (const float*)table, tokens, W, x, scale, (float*)x_t, (const float*)pos_table, tok_pos);
+    const bool vec = W % 4 == 0 && vec_ok(table, 16) && vec_ok(x, 16) && vec_ok(x_t, 16) && vec_ok(pos_table, 16);
+#define EMB_LAUNCH(T, V) launch_pdl(embed_f32_kernel<T, V>, n, 256, 0, s, (const T*)table, tokens, W, x, scale, (T*)x_t, (const T*)pos_table, tok_pos)
+    if (dt == WF_BF16) { if (vec) EMB_LAUNCH(__nv_bfloat16, 4); else EMB_LAUNCH(__nv_bfloat16, 1); }
+    else { if (vec) EMB_LAUNCH(float, 4); else EMB_LAUNCH(float, 1); }
+#undef EMB_LAUNCH
     return launch_check(cudaGetLastError(), "embed_f32");
 }
 
@@ -167,11 +178,65 @@ __global__ void group_rmsnorm_kernel(const float* __restrict__ x, int ldx, const
     }
 }
 
+// The same with four consecutive elements per load and every input of a row requested before the first is used; a thread owns NV groups of four,
+// blockDim.x * NV * 4 >= gw.  What bounds it is the bytes: 2048 rows of 2560 from two inputs and a residual, 94 MB: 30 us one element at a time, 17 so.
+template <typename T, int NV>
+__global__ void __launch_bounds__(1024) group_rmsnorm_vec_kernel(const float* x, int ldx, const T* __restrict__ w, int gw, float eps, const float* res, float* y, int ldy,
+                                                                 T* __restrict__ y_t, int ldt, const int32_t* __restrict__ rows, const float* x2, float a, float b,
+                                                                 float w_offset) {
+    pdl_enter();
+    __shared__ float scratch[33];
+    const int i = blockIdx.x, g = blockIdx.y;
+    const int src = rows ? rows[i] : i;
+    const size_t at = (size_t)src * ldx + (size_t)g * gw;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[NV], v2[NV], rv[NV], wv[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int c = (threadIdx.x + k * blockDim.x) * 4;
+        const bool in = c < gw;
+        v[k] = in ? load4(x + at + c) : zero;
+        v2[k] = in && x2 ? load4(x2 + at + c) : zero;
+        rv[k] = in && res ? load4(res + (size_t)src * ldy + (size_t)g * gw + c) : zero;
+        wv[k] = in ? load4(w + (size_t)g * gw + c) : zero;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        if (x2) v[k] = make_float4(a * v[k].x + b * v2[k].x, a * v[k].y + b * v2[k].y, a * v[k].z + b * v2[k].z, a * v[k].w + b * v2[k].w);
+        ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+    }
+    ss = block_sum(ss, scratch);
+    const float inv = 1.f / sqrtf(ss / (float)gw + eps);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int c = (threadIdx.x + k * blockDim.x) * 4;
+        if (c >= gw) continue;
+        float o[4] = {v[k].x * inv * (w_offset + wv[k].x), v[k].y * inv * (w_offset + wv[k].y), v[k].z * inv * (w_offset + wv[k].z), v[k].w * inv * (w_offset + wv[k].w)};
+        if (res) { o[0] += rv[k].x; o[1] += rv[k].y; o[2] += rv[k].z; o[3] += rv[k].w; }
+        if (y) store4(y + (size_t)i * ldy + (size_t)g * gw + c, o);
+        if (y_t) store4(y_t + (size_t)i * ldt + (size_t)g * gw + c, o);
+    }
+}
+
+// rows of four-element groups in registers: groups per thread and threads
+inline int vec_groups(int W) { return W <= 1024 ? 1 : 2; }
+inline int vec_threads(int W) { const int nv = vec_groups(W); return (W / 4 + nv * 32 - 1) / (nv * 32) * 32; }
+
 int launch_group_rmsnorm(int dt, const float* x, int ldx, const void* w, int groups, float eps, int n, int W, const float* res, float* y,
                          int ldy, void* y_t, int ldt, const int32_t* rows, cudaStream_t s, const float* x2, float a, float b, float w_offset) {
     if (n <= 0) return WF_OK;
     if (groups <= 0 || W % groups) { set_error("group_rmsnorm: width %d not divisible into %d groups", W, groups); return WF_ERR_INVALID; }
     if (res && rows && y == res) { set_error("group_rmsnorm: gathered rows cannot be added in place"); return WF_ERR_INVALID; }
+    if (W / groups % 4 == 0 && W / groups <= 8192 && ldx % 4 == 0 && ldy % 4 == 0 && ldt % 4 == 0 && vec_ok(x, 16) && vec_ok(x2, 16) && vec_ok(res, 16) && vec_ok(y, 16) &&
+        vec_ok(w, 16) && vec_ok(y_t, 16)) {
+        const int wide = W / groups;
+#define GR_LAUNCH(T, NV) launch_pdl(group_rmsnorm_vec_kernel<T, NV>, dim3(n, groups), vec_threads(wide), 0, s, x, ldx, (const T*)w, wide, eps, res, y, ldy, (T*)y_t, ldt, rows, x2, a, b, w_offset)
+        if (dt == WF_BF16) { if (vec_groups(wide) == 1) GR_LAUNCH(__nv_bfloat16, 1); else GR_LAUNCH(__nv_bfloat16, 2); }
+        else { if (vec_groups(wide) == 1) GR_LAUNCH(float, 1); else GR_LAUNCH(float, 2); }
+#undef GR_LAUNCH
+        return launch_check(cudaGetLastError(), "group_rmsnorm_vec");
+    }
     const int gw = W / groups;
     const int threads = gw >= 2048 ? 512 : (gw >= 1024 ? 256 : (gw >= 256 ? 128 : 64));
     dim3 grid(n, groups);
@@ -218,9 +283,71 @@ __global__ void __launch_bounds__(AD_THREADS) add_dual_norm_kernel(float* __rest
     }
 }
 
+// Four consecutive elements per load, everything requested before the first is used (rows of up to 8192; see group_rmsnorm_vec_kernel).
+template <typename T, int NV>
+__global__ void __launch_bounds__(1024) add_dual_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ y1, float a1, const float* __restrict__ y2, float a2,
+                                                                 const float* __restrict__ y3, const T* __restrict__ w1, const T* __restrict__ w2, float w_offset, float eps,
+                                                                 int W, T* __restrict__ h1, T* __restrict__ h2) {
+    pdl_enter();
+    __shared__ float scratch[33];
+    const size_t base = (size_t)blockIdx.x * W;
+    const bool adds = y1 || y2 || y3;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[NV], p1[NV], p2[NV], p3[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int c = (threadIdx.x + k * blockDim.x) * 4;
+        const bool in = c < W;
+        v[k] = in ? load4(x + base + c) : zero;
+        p1[k] = in && y1 ? load4(y1 + base + c) : zero;
+        p2[k] = in && y2 ? load4(y2 + base + c) : zero;
+        p3[k] = in && y3 ? load4(y3 + base + c) : zero;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int c = (threadIdx.x + k * blockDim.x) * 4;
+        if (adds && c < W) {
+            auto add = [&](float o, float q1, float q2, float q3) {
+                float t = 0.f;
+                if (y1) t = a1 * q1;
+                if (y2) t = fmaf(a2, q2, t);
+                if (y3) t += q3;
+                return o + t;
+            };
+            const float o[4] = {add(v[k].x, p1[k].x, p2[k].x, p3[k].x), add(v[k].y, p1[k].y, p2[k].y, p3[k].y), add(v[k].z, p1[k].z, p2[k].z, p3[k].z), add(v[k].w, p1[k].w, p2[k].w, p3[k].w)};
+            store4(x + base + c, o);
+            v[k] = make_float4(o[0], o[1], o[2], o[3]);
+        }
+        ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+    }
+    if (!w1 && !w2) return;
+    ss = block_sum(ss, scratch);
+    const float inv = 1.f / sqrtf(ss / (float)W + eps);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int c = (threadIdx.x + k * blockDim.x) * 4;
+        if (c >= W) continue;
+        auto scaled = [&](const T* w, T* h) {
+            const float4 m = load4(w + c);
+            const float o[4] = {v[k].x * inv * (w_offset + m.x), v[k].y * inv * (w_offset + m.y), v[k].z * inv * (w_offset + m.z), v[k].w * inv * (w_offset + m.w)};
+            store4(h + base + c, o);
+        };
+        if (w1) scaled(w1, h1);
+        if (w2) scaled(w2, h2);
+    }
+}
+
 int launch_add_dual_norm(int dt, float* x, const float* y1, float a1, const float* y2, float a2, const float* y3, const void* w1, const void* w2,
                          float w_offset, float eps, int n, int W, void* h1, void* h2, cudaStream_t s) {
     if (n <= 0) return WF_OK;
+    if (W % 4 == 0 && W <= 8192 && vec_ok(x, 16) && vec_ok(y1, 16) && vec_ok(y2, 16) && vec_ok(y3, 16) && vec_ok(w1, 16) && vec_ok(w2, 16) && vec_ok(h1, 16) && vec_ok(h2, 16)) {
+#define AD_LAUNCH(T, NV) launch_pdl(add_dual_norm_vec_kernel<T, NV>, n, vec_threads(W), 0, s, x, y1, a1, y2, a2, y3, (const T*)w1, (const T*)w2, w_offset, eps, W, (T*)h1, (T*)h2)
+        if (dt == WF_BF16) { if (vec_groups(W) == 1) AD_LAUNCH(__nv_bfloat16, 1); else AD_LAUNCH(__nv_bfloat16, 2); }
+        else { if (vec_groups(W) == 1) AD_LAUNCH(float, 1); else AD_LAUNCH(float, 2); }
+#undef AD_LAUNCH
+        return launch_check(cudaGetLastError(), "add_dual_norm_vec");
+    }
     if (dt == WF_BF16) launch_pdl(add_dual_norm_kernel<__nv_bfloat16>, n, AD_THREADS, 0, s, x, y1, a1, y2, a2, y3, (const __nv_bfloat16*)w1, (const __nv_bfloat16*)w2, w_offset, eps, W, (__nv_bfloat16*)h1, (__nv_bfloat16*)h2);
     else launch_pdl(add_dual_norm_kernel<float>, n, AD_THREADS, 0, s, x, y1, a1, y2, a2, y3, (const float*)w1, (const float*)w2, w_offset, eps, W, (float*)h1, (float*)h2);
     return launch_check(cudaGetLastError(), "add_dual_norm");
@@ -342,18 +469,6 @@ __global__ void __launch_bounds__(512) branch_add_norm_kernel(float* __restrict_
     }
     for (int c = threadIdx.x + LN_PER * blockDim.x; c < W; c += blockDim.x)
         h[base + c] = from_f<T>((row[c] - mean) * inv * (w_offset + to_f(w[c])) + (b ? to_f(b[c]) : 0.f));
-}
-
-template <typename T> __device__ __forceinline__ float4 load4(const T* p);
-template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *reinterpret_cast<const float4*>(p); }
-template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
-    const uint2 v = *reinterpret_cast<const uint2*>(p);
-    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
-}
-__device__ __forceinline__ void store4(float* p, const float (&v)[4]) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
-__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
-    const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
-    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
 // The same with four consecutive elements per load, every input of a row requested before the first is used; a thread owns NV groups of four,
@@ -595,10 +710,70 @@ __global__ void causal_taps_kernel(Batch b, const float* __restrict__ in, int ld
     }
 }
 
+// Many tokens: a thread takes four channels of TR tokens one after another, so an input is read once instead of once per tap, all of the run's inputs are
+// requested before the first is used, and the weights are read once a run.  1801 tokens x 5120 channels, four taps (74 MB): 72 us a channel and token per
+// thread, 17 so.  Sums in the same order as above.
+constexpr int TR = 8;
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(128) causal_taps_run_kernel(Batch b, const float* __restrict__ in, int ld_in, const T* __restrict__ w, int C, const float* __restrict__ state,
+                                                              size_t slot_stride, int identity, int silu, T* __restrict__ out_t, int ld_t, float* __restrict__ out_f, int ld_f,
+                                                              const T* __restrict__ bias) {
+    pdl_enter();
+    const int c = (blockIdx.y * 128 + threadIdx.x) * 4, i0 = blockIdx.x * TR;
+    if (c >= C) return;
+    float4 cur[TR];
+#pragma unroll
+    for (int t = 0; t < TR; ++t)
+        if (i0 + t < b.n) cur[t] = load4(in + (size_t)(i0 + t) * ld_in + c);
+    float4 wt[TAPS], win[TAPS];
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j)
+        wt[j] = make_float4(to_f(w[(size_t)c * TAPS + j]), to_f(w[(size_t)(c + 1) * TAPS + j]), to_f(w[(size_t)(c + 2) * TAPS + j]), to_f(w[(size_t)(c + 3) * TAPS + j]));
+    const float4 bs = bias ? load4(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < TR; ++t) {
+        const int i = i0 + t;
+        if (i >= b.n) break;
+        const int sq = b.tok_seq[i], li = i - b.seq_start[sq];             // li: index inside this step's portion
+        if (t == 0 || li == 0) {
+            const float* st = state + (size_t)b.seq_slot[sq] * slot_stride + c;
+#pragma unroll
+            for (int j = 0; j < TAPS - 1; ++j) {
+                const int src = li - (TAPS - 1) + j;
+                win[j] = src >= 0 ? load4(in + (size_t)(i - li + src) * ld_in + c) : load4(st + (size_t)(src + TAPS - 1) * C);
+            }
+        }
+        win[TAPS - 1] = cur[t];
+        float4 acc = identity ? cur[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            acc.x = fmaf(wt[j].x, win[j].x, acc.x); acc.y = fmaf(wt[j].y, win[j].y, acc.y);
+            acc.z = fmaf(wt[j].z, win[j].z, acc.z); acc.w = fmaf(wt[j].w, win[j].w, acc.w);
+        }
+        float o[4] = {acc.x, acc.y, acc.z, acc.w};
+        if (bias) { o[0] += bs.x; o[1] += bs.y; o[2] += bs.z; o[3] += bs.w; }
+        if (silu) { o[0] = silu_f(o[0]); o[1] = silu_f(o[1]); o[2] = silu_f(o[2]); o[3] = silu_f(o[3]); }
+        if (out_t) store4(out_t + (size_t)i * ld_t + c, o);
+        if (out_f) store4(out_f + (size_t)i * ld_f + c, o);
+#pragma unroll
+        for (int j = 0; j + 1 < TAPS; ++j) win[j] = win[j + 1];
+    }
+}
+
 int launch_causal_taps(int dt, const Batch& b, const float* in, int ld_in, const void* w, int taps, int C, const float* state,
                        size_t slot_stride, int identity, int silu, void* out_t, int ld_t, float* out_f, int ld_f, cudaStream_t s, const void* bias) {
     if (b.n <= 0) return WF_OK;
     if (taps < 1) { set_error("causal_taps: taps %d", taps); return WF_ERR_INVALID; }
+    // runs of tokens where they fill the SMs twice: below, a thread's eight tokens in a row are the longer way
+    const int runs = (b.n + TR - 1) / TR, cblocks = (C / 4 + 127) / 128;
+    if (taps >= 2 && taps <= 4 && C % 4 == 0 && (long long)runs * cblocks >= 2 * sm_count() && ld_in % 4 == 0 && ld_t % 4 == 0 && ld_f % 4 == 0 && slot_stride % 4 == 0 &&
+        vec_ok(in, 16) && vec_ok(state, 16) && vec_ok(out_t, 16) && vec_ok(out_f, 16) && vec_ok(bias, 16)) {
+#define CT_LAUNCH(T, N) launch_pdl(causal_taps_run_kernel<T, N>, dim3(runs, cblocks), 128, 0, s, b, in, ld_in, (const T*)w, C, state, slot_stride, identity, silu, (T*)out_t, ld_t, out_f, ld_f, (const T*)bias)
+        if (dt == WF_BF16) { if (taps == 2) CT_LAUNCH(__nv_bfloat16, 2); else if (taps == 3) CT_LAUNCH(__nv_bfloat16, 3); else CT_LAUNCH(__nv_bfloat16, 4); }
+        else { if (taps == 2) CT_LAUNCH(float, 2); else if (taps == 3) CT_LAUNCH(float, 3); else CT_LAUNCH(float, 4); }
+#undef CT_LAUNCH
+        return launch_check(cudaGetLastError(), "causal_taps_run");
+    }
     dim3 grid(b.n, (C + 255) / 256 > 8 ? 8 : (C + 255) / 256);
     if (dt == WF_BF16) launch_pdl(causal_taps_kernel<__nv_bfloat16>, grid, 256, 0, s, b, in, ld_in, (const __nv_bfloat16*)w, taps, C, state, slot_stride, identity, silu, (__nv_bfloat16*)out_t, ld_t, out_f, ld_f, (const __nv_bfloat16*)bias);
     else launch_pdl(causal_taps_kernel<float>, grid, 256, 0, s, b, in, ld_in, (const float*)w, taps, C, state, slot_stride, identity, silu, (float*)out_t, ld_t, out_f, ld_f, (const float*)bias);
