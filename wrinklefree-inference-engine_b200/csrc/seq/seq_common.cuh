@@ -97,6 +97,15 @@ __device__ __forceinline__ float epilogue_f(int ep, float v) {        // GemmArg
 }
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
+// gated activations (launch_silu_mul's act): silu(g) u; 1: clamped, with u + 1; 2: tanh-gelu(g) u
+__device__ __forceinline__ float glu_f(int act, float g, float u, float limit) {
+    if (act == 1) {
+        const float gg = fminf(g, limit), uu = fminf(fmaxf(u, -limit), limit);
+        return gg * sigmoid_f(1.702f * gg) * (uu + 1.f);
+    }
+    if (act == 2) return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
+    return silu_f(g) * u;
+}
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 }  // namespace seq

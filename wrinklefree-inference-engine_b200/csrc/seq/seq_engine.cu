@@ -825,6 +825,16 @@ int run_unit(wf_seq_engine* e, LayerState& L, const Batch& b, float* out, const 
         if ((rc = launch_gemm(e->dt, g, s))) return rc;
         mark(e, "unit.up");
     } else {
+        // prompts: the activation where the product stores its results, so that [gate | up] (113 MB at 2048 x 6912) is neither written nor read
+        GemmArgs g = lin(in, 0, W, L.ugu, W, e->uhmid, 0, ff, n, 2 * ff, W);
+        g.glu = 1 + L.c.ff_act; g.limit = L.ulimit;
+        if (L.c.ff_act <= 2 && gemm_glu_usable(e->dt, g)) {
+            if ((rc = launch_gemm(e->dt, g, s))) return rc;
+            mark(e, "unit.gate_up");
+            rc = launch_gemm(e->dt, lin(e->uhmid, 0, ff, L.ud, ff, out, 1, W, n, W, ff), s);
+            mark(e, "unit.down");
+            return rc;
+        }
         if ((rc = launch_gemm(e->dt, lin(in, 0, W, L.ugu, W, e->ugu, 1, 2 * ff, n, 2 * ff, W), s))) return rc;
         mark(e, "unit.gate_up");
         if ((rc = launch_silu_mul(e->dt, e->ugu, n, ff, nullptr, e->uhmid, s, L.c.ff_act, L.ulimit))) return rc;

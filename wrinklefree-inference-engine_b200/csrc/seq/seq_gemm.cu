@@ -455,11 +455,21 @@ int g_force_simt = -1, g_tc_min = -1;
 
 }  // namespace
 
-int launch_gemm(int dt, const GemmArgs& g, cudaStream_t s) {
-    if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return WF_OK;
-    if (g.K <= 0 || !g.A || !g.B || !g.C) { set_error("gemm: bad arguments (M %d N %d K %d)", g.M, g.N, g.K); return WF_ERR_INVALID; }
+static void read_env() {
     if (g_tc_min < 0) { const char* e = getenv("WF_SEQ_TC_MIN"); g_tc_min = e ? atoi(e) : 17; }
     if (g_force_simt < 0) { const char* e = getenv("WF_SEQ_GEMM_SIMT"); g_force_simt = (e && atoi(e)) ? 1 : 0; }
+}
+// the rows that launch_gemm gives to the tcgen05 form by itself
+bool gemm_glu_usable(int dt, const GemmArgs& g) {
+    read_env();
+    return dt == WF_BF16 && g.algo == 0 && !g_force_simt && g.M >= g_tc_min && g.M > 8 && gemm_tc_usable(g);
+}
+
+int launch_gemm(int dt, const GemmArgs& g, cudaStream_t s) {
+    if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return WF_OK;
+    if (g.glu && !gemm_glu_usable(dt, g)) { set_error("gemm: no gated form takes this shape"); return WF_ERR_UNSUPPORTED; }
+    if (g.K <= 0 || !g.A || !g.B || !g.C) { set_error("gemm: bad arguments (M %d N %d K %d)", g.M, g.N, g.K); return WF_ERR_INVALID; }
+    read_env();
     const bool few = g.batch == 1 && !g.tile_group && !g.a_rows && g.M <= 8;
     // (9 to 16 rows go to the tcgen05 form where WF_SEQ_TC_MIN asks for it)
     const bool few_mma = g.algo == 5 || (g.algo == 0 && !g_force_simt && (g.M <= 8 || g.M < g_tc_min || !gemm_tc_usable(g)));

@@ -38,6 +38,7 @@ struct TcParams {
     int tn;                        // tokens per tile
     int n_tiles, tiles;            // tiles of 256 weight rows; all tiles
     void* C; int ldc, c_f32, ep;
+    int glu; float limit;          // > 0: rows [gate | up] (N = 2 ff), stored as activation glu - 1 of the pair in bf16 [M, ff]; its clamp
     const int32_t* tile_group;     // per 128-token tile: expert, or < 0 = skip (null: dense)
     int group_w_rows;              // weight rows between consecutive experts in the stacked tensor
     int* err;
@@ -99,6 +100,9 @@ __device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity) {
                    "=r"(v[30]), "=r"(v[31])                                                                             \
                  : "r"(taddr) : "memory")
 
+// GLU: a CTA's 128 weight rows are four blocks of 16 gate rows and the 16 up rows that belong to them (one box of a four-dimensional map), so that a pair
+// meets in the lanes of one warp and only the activation's result is stored.  A form of its own: the plain form's epilogue keeps its registers.
+template <bool GLU>
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_a,
                                                                 const TcParams p) {
     extern __shared__ unsigned char smem_raw[];
@@ -151,8 +155,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
                     const int s = it % TC_STAGES;
                     if (it >= TC_STAGES && !wait_bounded(smem_u32(&empty_bar[s]), (uint32_t)(((it / TC_STAGES) & 1) ^ 1))) { ok = false; break; }
                     if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * (TC_W_BYTES + half * 128));      // both CTAs' loads report here
-                    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                                 ::"r"(ring + s * TC_STAGE_BYTES), "l"(&tmap_w), "r"(kc * TC_KC), "r"(w_row), "r"(full0 + s * 8) : "memory");
+                    if (GLU)
+                        asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                                     ::"r"(ring + s * TC_STAGE_BYTES), "l"(&tmap_w), "r"(kc * TC_KC), "r"(0), "r"(0), "r"(w_row / 32), "r"(full0 + s * 8) : "memory");
+                    else
+                        asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                                     ::"r"(ring + s * TC_STAGE_BYTES), "l"(&tmap_w), "r"(kc * TC_KC), "r"(w_row), "r"(full0 + s * 8) : "memory");
                     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                                  ::"r"(ring + s * TC_STAGE_BYTES + TC_W_BYTES), "l"(&tmap_a), "r"(kc * TC_KC), "r"(mt * p.tn + rank * half), "r"(full0 + s * 8) : "memory");
                 }
@@ -231,6 +239,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const __grid_con
                 const int m0 = mt * p.tn + c * 32;
                 int mcnt = p.M - m0 < 32 ? p.M - m0 : 32;                  // tokens of this chunk that exist and belong to this tile (warp-uniform)
                 if (p.tn - c * 32 < mcnt) mcnt = p.tn - c * 32;
+                if (GLU) {
+                    // lanes 0 .. 15 hold gate rows and keep the chunk's tokens 0 .. 15, lanes 16 .. 31 the up rows and keep the others; they swap the rest
+                    const bool up = lane >= 16;
+                    __nv_bfloat16* dst = (__nv_bfloat16*)p.C + (size_t)(m0 + (up ? 16 : 0)) * p.ldc + (n >> 5) * 16 + (n & 15);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(up ? r[j] : r[16 + j]), 16), mine = __uint_as_float(up ? r[16 + j] : r[j]);
+                        const float a = glu_f(p.glu - 1, up ? got : mine, up ? mine : got, p.limit);
+                        if (n_ok && (up ? 16 : 0) + j < mcnt) *dst = __float2bfloat16_rn(a);
+                        dst += p.ldc;
+                    }
+                    __syncwarp();
+                    continue;
+                }
                 if (p.ep != EP_NONE) {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(epilogue_f(p.ep, __uint_as_float(r[j])));
@@ -306,6 +328,7 @@ bool gemm_tc_usable(const GemmArgs& g) {
     if (g.a_f32 || g.batch != 1 || g.a_rows) return false;
     if (g.lda % 8 || g.ldb % 8 || ((uintptr_t)g.A & 15) || ((uintptr_t)g.B & 15) || g.K < 8 || g.lda < g.K || g.ldb < g.K) return false;
     if (g.tile_group && (g.group_stride % g.ldb)) return false;
+    if (g.glu && (g.tile_group || g.c_f32 || g.ep != EP_NONE || g.N % 32)) return false;
     return true;
 }
 
@@ -342,14 +365,23 @@ int gemm_tc_error(cudaStream_t s) {
 
 // n_groups: number of stacked weight matrices (1 when dense)
 int launch_gemm_tc(const GemmArgs& g, int n_groups, cudaStream_t s) {
-    if (g_attr.need()) cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
+    if (g_attr.need()) {
+        cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
+        cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
+    }
     if (!tensor_map_encoder()) { set_error("gemm_tc: cuTensorMapEncodeTiled unavailable"); return WF_ERR_CUDA; }
     int* err = tc_error_word();
     if (!err) return WF_ERR_CUDA;
     CUtensorMap tw, ta;
     const int group_w_rows = g.tile_group ? (int)(g.group_stride / g.ldb) : 0;
     const uint64_t w_rows = g.tile_group ? (uint64_t)(n_groups - 1) * group_w_rows + g.N : (uint64_t)g.N;
-    if (int rc = encode_2d(&tw, g.B, w_rows, g.K, g.ldb, TC_ROWS)) return rc;
+    if (g.glu) {
+        const cuuint64_t dim[4] = {(cuuint64_t)g.K, 16, 2, (cuuint64_t)(g.N / 32)}, row = (cuuint64_t)g.ldb * 2, stride[3] = {row, row * (g.N / 2), row * 16};
+        const cuuint32_t box[4] = {TC_KC, 16, 2, TC_ROWS / 32}, one[4] = {1, 1, 1, 1};
+        const CUresult cr = g_encode(&tw, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)g.B, dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (cr != CUDA_SUCCESS) { set_error("gemm_tc: tensor map failed (%d)", (int)cr); return WF_ERR_CUDA; }
+    } else if (int rc = encode_2d(&tw, g.B, w_rows, g.K, g.ldb, TC_ROWS)) return rc;
     const int sms = sm_count(), pairs = sms / 2;
     const int tn = g.tile_group ? GEMM_BM : tokens_per_tile(g.M, g.N, g.K, pairs);
     if (int rc = encode_2d(&ta, g.A, g.M, g.K, g.lda, tn / 2)) return rc;
@@ -359,6 +391,7 @@ int launch_gemm_tc(const GemmArgs& g, int n_groups, cudaStream_t s) {
     p.n_tiles = (g.N + 2 * TC_ROWS - 1) / (2 * TC_ROWS);
     p.tiles = p.n_tiles * ((g.M + tn - 1) / tn);
     p.C = g.C; p.ldc = g.ldc; p.c_f32 = g.c_f32; p.ep = g.ep;
+    p.glu = g.glu; p.limit = g.limit;
     p.tile_group = g.tile_group; p.group_w_rows = group_w_rows;
     p.err = err;
     cudaLaunchConfig_t cfg = {};
@@ -373,7 +406,7 @@ int launch_gemm_tc(const GemmArgs& g, int n_groups, cudaStream_t s) {
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 2;
-    return launch_check(cudaLaunchKernelEx(&cfg, gemm_tc_kernel, tw, ta, p), "gemm_tc");
+    return launch_check(g.glu ? cudaLaunchKernelEx(&cfg, gemm_tc_kernel<true>, tw, ta, p) : cudaLaunchKernelEx(&cfg, gemm_tc_kernel<false>, tw, ta, p), "gemm_tc");
 }
 
 }  // namespace seq

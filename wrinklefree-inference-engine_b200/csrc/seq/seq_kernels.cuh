@@ -115,12 +115,16 @@ struct GemmArgs {
     const int32_t* a_rows = nullptr;
     int n_groups = 1;                        // weight matrices stacked behind B (grouped form)
     int ep = EP_NONE;
+    // gated activation where the product stores its results (tcgen05 form only, gemm_glu_usable): B's rows are [gate | up], N = 2 ff, C is T [M, ff] =
+    // activation glu - 1 (launch_silu_mul's act) of the two floats
+    int glu = 0; float limit = 0.f;
     int algo = 0;                            // 0 = choose; 1 plain FMA, 2 mma.sync, 3 tcgen05, 4 few-row streaming, 5 few rows on mma.sync (tests and measurements)
 };
 constexpr int GEMM_BM = 128;                 // row granule of the grouped form (the token tile of the tcgen05 kernel)
 int launch_gemm(int dt, const GemmArgs& g, cudaStream_t s);
 // tcgen05 form (seq_gemm_tc.cu): bf16 operands, dense A rows; launch_gemm picks it from WF_SEQ_TC_MIN (17) rows up
 bool gemm_tc_usable(const GemmArgs& g);
+bool gemm_glu_usable(int dt, const GemmArgs& g);   // whether launch_gemm takes g with its glu
 int launch_gemm_tc(const GemmArgs& g, int n_groups, cudaStream_t s);
 // shared by the tcgen05 kernels: the driver's tensor-map encoder (null: unavailable) and the current device's error word (null: no memory)
 void* tensor_map_encoder();
