@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32, I8 ? 3 : 2) paged_decode_attn_k
     const bool tr = FUSED && !I8 && p.trace && bid == 0 && threadIdx.x == 0;
     if (tr) p.trace[0] = gtimer();
     if (FUSED) pdl_launch_dependents();
+    else { pdl_wait_prior(); pdl_launch_dependents(); }   // queries, lengths, table and cache may all be the work of the kernel before
 
     // ---- work decomposition.
     // Legacy form (p.even == 0): CTA = (chunk, kv head, sequence), one segment.
@@ -784,7 +785,6 @@ __global__ void __launch_bounds__(AT_WARPS * 32, I8 ? 3 : 2) paged_decode_attn_k
         }
     }
     if (FUSED && p.signal_flag >= 0) tp_signal_grid_done(p.tp, p.signal_flag, nctas);
-    if (!FUSED) pdl_launch_dependents();
 }
 
 struct MergeParams {
@@ -1281,7 +1281,7 @@ extern "C" int wf_paged_decode_attn(const void* q, const wf_kv_layout* kv, int l
     if (out_dtype != WF_BF16 && out_dtype != WF_F32) { set_error("wf_paged_decode_attn: out dtype"); return WF_ERR_INVALID; }
     if (B <= 0) return WF_OK;
     return attn_decode(q, kv->pool, kv->layers, layer, kv->kv_heads, kv->page_size, block_table, max_blocks, seq_lens, B, H, scale, out,
-                       out_dtype, max_blocks * kv->page_size, workspace, workspace_bytes, (cudaStream_t)stream, false, kv_scales_of(kv));
+                       out_dtype, max_blocks * kv->page_size, workspace, workspace_bytes, (cudaStream_t)stream, true, kv_scales_of(kv));
 }
 
 namespace wf {

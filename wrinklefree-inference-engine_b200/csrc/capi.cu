@@ -105,7 +105,7 @@ static int ternary_linear(const wf_linear_args* a, const float* w_scales_host, v
         else algo = tc_is_faster(a->M, a->N, a->K) ? 3 : 2;
     }
     switch (algo) {
-        case 1: return launch_gemv_stream(a, ep, s, false);
+        case 1: return launch_gemv_stream(a, ep, s, true, true);
         case 2: return launch_gemm_mma(a, ep, s);
         case 3: return launch_gemm_tc(a, ep, s);
     }

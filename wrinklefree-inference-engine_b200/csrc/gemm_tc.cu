@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
         m_blk = ct / p.tiles_n;
         n_blk = ct - m_blk * p.tiles_n;
     };
-    pdl_launch_dependents();   // no-op unless launched with programmatic stream serialisation (decode step)
+    if (p.red_acc) pdl_launch_dependents();   // decode step: the next phase's weights are on their way while this one runs
 
     if (tid == 0) {
         for (int s = 0; s < TC_STAGES; ++s) { mbar_init(&full_bar[s], 5); mbar_init(&empty_bar[s], 1); }
@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(tc_threads(NU), 1) ternary_gemm_tc_kernel(cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
+    if (!p.red_acc) pdl_wait_prior();   // elsewhere the weights, too, may be the work of the kernel before
 
     if (warp == W_TMA) {
         // ------------------------------------------------------------ TMA producer: int8 activations
@@ -509,12 +510,7 @@ static int launch_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t 
     p.ep = ep;
     p.splitk = 1; p.KBs = p.KB; p.ksplit = 1; p.red_acc = nullptr; p.red_ld = 0; p.l2_ahead = 0;
     const int total = p.tiles_n * p.tiles_m, sms = sm_count();
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(total < sms ? total : sms);
-    cfg.blockDim = dim3(tc_threads(NU));
-    cfg.dynamicSmemBytes = TC_SMEM;
-    cfg.stream = s;
-    return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<NU>, tmap, p), "ternary_gemm_tc");
+    return launch_check(launch_pdl(ternary_gemm_tc_kernel<NU>, dim3(total < sms ? total : sms), dim3(tc_threads(NU)), TC_SMEM, s, tmap, p), "ternary_gemm_tc");
 }
 
 // Batched-decode form (the engine's phase kernels, 32 < M <= 128): S[m][n] += sum over this launch's K columns, added into the
@@ -590,11 +586,13 @@ static int launch_tc_split(const wf_linear_args* a, const EpiParams& ep, int ksp
     cfg.blockDim = dim3(tc_threads(NU));
     cfg.dynamicSmemBytes = TC_SMEM;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = ksplit; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<NU, true>, tmap, p), "ternary_gemm_tc(split)");
 }
 

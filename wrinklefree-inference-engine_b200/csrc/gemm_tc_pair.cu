@@ -200,6 +200,7 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
+    pdl_wait_prior();                                       // barriers, TMEM and the pair's meeting above overlap the kernel before
 
     if (warp == W_ACT) {
         // ------------------------------------------------------------ activations: this CTA's half of the tile's tokens
@@ -496,11 +497,13 @@ int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream
     cfg.blockDim = dim3(tp_threads(NU));
     cfg.dynamicSmemBytes = TP_SMEM;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return launch_check(p.tn > 192 ? cudaLaunchKernelEx(&cfg, ternary_gemm_pair_kernel<NU, 1>, tq, tw, p) : cudaLaunchKernelEx(&cfg, ternary_gemm_pair_kernel<NU, 2>, tq, tw, p), "ternary_gemm_pair");
 }
 

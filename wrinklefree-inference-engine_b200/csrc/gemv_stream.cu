@@ -48,6 +48,7 @@ struct StreamParams {
     int* ws_cnt;
     int aligned;          // 1: CTA slabs are whole finalisation groups (no split-K, no workspace traffic)
     int stages;           // ring depth (<= SV_MAX_STAGES)
+    int wait_first;       // the weights wait for the prior grid too
     int l2_ahead;         // producer prefetches this many stages beyond the ring into L2 (0 = off)
     int debug;            // bit0: stream-only (wf_bench_gemv: the ceiling of the TMA ring without the math)
     EpiParams ep;
@@ -102,8 +103,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, CW <= 8 ? 2 : 1) ternary_gemv_s
     __syncthreads();
 
     if (warp == CW) {
-        // ------------------------------------------------ producer warp (one elected lane); never waits on the prior grid
+        // ------------------------------------------------ producer warp (one elected lane); waits for the prior grid only where that may have made the weights
         if (lane == 0) {
+            if (p.wait_first) pdl_wait_prior();
             int s = 0, ph = 1;
             for (int it = 0; it < nstages; ++it) {
                 if (p.l2_ahead > 0) {
@@ -400,7 +402,7 @@ bool gemv_stream_fits(int M, int K) {
     return act_bytes + 3 * (size_t)SV_TPW * SV_CW * WF_TILE_BYTES + 24 * 1024 <= 220 * 1024;
 }
 
-int launch_gemv_stream(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s, bool pdl) {
+int launch_gemv_stream(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s, bool pdl, bool wait_first) {
     if (a->w_layout != WF_W_TILE) { set_error("gemv_stream: needs the b200_tile_v1 layout"); return WF_ERR_UNSUPPORTED; }
     if (a->M < 1 || a->M > 8) { set_error("gemv_stream: M=%d outside 1..8", a->M); return WF_ERR_UNSUPPORTED; }
     StreamParams p;
@@ -414,6 +416,7 @@ int launch_gemv_stream(const wf_linear_args* a, const EpiParams& ep, cudaStream_
     p.ep = ep;
     p.debug = g_gemv_debug;
     p.l2_ahead = g_gemv_l2_ahead;
+    p.wait_first = wait_first;
     // Grid: two CTAs per SM (two independent TMA streams per SM: +15 % stream rate, measured) once every CTA still gets a few
     // stages and both fit in shared memory; one per SM otherwise.  Slabs: whole row-block groups per CTA when there are
     // enough of them and the matrix is small (no split-K: saves three dependent L2 round trips), an even tile split else.

@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(QT) act_quant_rows_kernel(const T* __restrict_
     __shared__ int is[33];
     const int m = blockIdx.x;
     const T* row = x + (size_t)m * ldx;
+    pdl_wait_prior();
+    pdl_launch_dependents();
     const float amax = block_max<QT>(row_absmax(row, K), fs);
     const float scale = act_scale_from_absmax(amax);
     const int total = block_sum_i<QT>(row_quant(row, K, scale, q + (size_t)m * K), is);
@@ -112,6 +114,8 @@ __global__ void __launch_bounds__(QT) act_quant_rows_kernel(const T* __restrict_
 template <typename T>
 __global__ void __launch_bounds__(QT) act_absmax_kernel(const T* __restrict__ x, int M, int K, int ldx,
                                                         unsigned int* __restrict__ amax_bits) {
+    pdl_wait_prior();
+    pdl_launch_dependents();
     float amax = 0.f;
     for (int m = blockIdx.x; m < M; m += gridDim.x) amax = fmaxf(amax, row_absmax(x + (size_t)m * ldx, K));
     amax = warp_max(amax);
@@ -125,6 +129,8 @@ __global__ void __launch_bounds__(QT) act_quant_tensor_kernel(const T* __restric
                                                               int8_t* __restrict__ q, float* __restrict__ scale_out,
                                                               int32_t* __restrict__ rowsum) {
     __shared__ int is[QT / 32];
+    pdl_wait_prior();
+    pdl_launch_dependents();
     const int m = gridDim.x - 1 - blockIdx.x;
     const float scale = act_scale_from_absmax(__uint_as_float(*amax_bits));
     const int part = warp_sum_i(row_quant(x + (size_t)m * ldx, K, scale, q + (size_t)m * K));
@@ -200,12 +206,12 @@ template <typename T>
 static int launch_act_quant(const T* x, int M, int K, int ldx, int per_token, int8_t* q, float* scale_out, int32_t* rowsum,
                             void* workspace, cudaStream_t s) {
     if (per_token) {
-        act_quant_rows_kernel<T><<<M, QT, 0, s>>>(x, K, ldx, q, scale_out, rowsum);
+        launch_pdl(act_quant_rows_kernel<T>, M, QT, 0, s, x, K, ldx, q, scale_out, rowsum);
     } else {
         if (cuda_check(cudaMemsetAsync(workspace, 0, 4, s), "memset absmax")) return WF_ERR_CUDA;
         int g = M < sm_count() * 4 ? M : sm_count() * 4;
-        act_absmax_kernel<T><<<g, QT, 0, s>>>(x, M, K, ldx, (unsigned int*)workspace);
-        act_quant_tensor_kernel<T><<<M, QT, 0, s>>>(x, K, ldx, (const unsigned int*)workspace, q, scale_out, rowsum);
+        launch_pdl(act_absmax_kernel<T>, g, QT, 0, s, x, M, K, ldx, (unsigned int*)workspace);
+        launch_pdl(act_quant_tensor_kernel<T>, M, QT, 0, s, x, K, ldx, (const unsigned int*)workspace, q, scale_out, rowsum);
     }
     return launch_check(cudaGetLastError(), "wf_act_quant_i8");
 }
@@ -254,7 +260,7 @@ extern "C" int wf_rmsnorm_quant(const void* x, const void* gamma, float eps, int
     if (!x || !gamma || !q || !scale_out) { set_error("wf_rmsnorm_quant: null pointer"); return WF_ERR_INVALID; }
     if (M <= 0 || K <= 0 || K % 8 != 0) { set_error("wf_rmsnorm_quant: bad shape M=%d K=%d (K %% 8 == 0)", M, K); return WF_ERR_INVALID; }
     if ((size_t)K * 2 > 128 * 1024) { set_error("wf_rmsnorm_quant: K=%d exceeds the 64K-element row limit", K); return WF_ERR_UNSUPPORTED; }
-    return launch_rmsnorm_quant(x, gamma, eps, M, K, y_out, q, scale_out, rowsum_out, (cudaStream_t)stream, false);
+    return launch_rmsnorm_quant(x, gamma, eps, M, K, y_out, q, scale_out, rowsum_out, (cudaStream_t)stream, true);
 }
 
 namespace wf {

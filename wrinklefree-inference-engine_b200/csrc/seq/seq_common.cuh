@@ -3,7 +3,6 @@
 // stream, norms, softmax, rotary angles, routers and recurrent state are float in both.
 #pragma once
 #include "../common.cuh"
-#include <utility>
 
 namespace wf {
 namespace seq {
@@ -50,20 +49,6 @@ struct Batch {
 // kernels of 2 to 6 us, a prompt layer one of 15 to 25, at about 1 us of launch each.  Measured without / with: a decode step of 8 sequences, four layers
 // 182 / 159 us (221 where a kernel lets the next one in before its own wait: the CTAs of several waiting kernels then hold slots); layers 524 / 491, 940 / 918, 1060 / 1019 us.
 __device__ __forceinline__ void pdl_enter() { pdl_wait_prior(); pdl_launch_dependents(); }
-template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
-}
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
