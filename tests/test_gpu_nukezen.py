@@ -417,6 +417,21 @@ def test_tensor_core_attention_with_key_splits_in_a_ragged_batch():
         m.close()
 
 
+def test_low_rank_products_of_long_portions():
+    """Gate and decay logits of many tokens come from the product on CTA pairs, those of short portions from the other one: the same mixer over one portion
+    and over portions of 100.  Tolerance: both round the low-rank columns to the same bf16 numbers, so only the order of float sums and what bf16 results
+    make of it (2^-9) is left; 5e-3 of a row's size covers two such roundings."""
+    cfg = config([cdelta(heads=8, kv=4, dim=64, vdim=64, conv=4)], width=64, vocab=40)
+    w = make_weights((cfg, {0: {"rank_a": 128, "rank_g": 96}}), 7)
+    m = build(cfg, w, "bfloat16", max_tokens=2600, page_size=16, max_step_tokens=1700)
+    rows = _rows(1700, 64, 8, 1.0)
+    whole = part_alone(m, 0, 2, rows, [1700])
+    cut = part_alone(m, 0, 2, rows, [100] * 17)
+    err = np.linalg.norm(whole - cut, axis=1) / np.linalg.norm(cut, axis=1)
+    assert np.median(err) < 5e-3 and err.max() < 3e-2, (np.median(err), err.max())
+    m.close()
+
+
 # ------------------------------------------------------------------------------------------------- scheduler and command line
 def _greedy_matches(cfg, w, prompt, output):
     seq = list(prompt)

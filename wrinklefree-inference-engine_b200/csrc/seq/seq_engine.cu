@@ -583,6 +583,18 @@ int run_latent(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
     return rc;
 }
 
+// out float [n, nout] = columns src (float, ld) x w T [nout, rank].  Prompts: the columns as bf16 first (in og, whose last reader is done; what the product
+// rounds them to in any case), and the product on CTA pairs: 1801 x 2560, rank 128 27.5 -> 8.7 + 2.5 us, 256 tokens 8.7 -> 4.9 + 2.5, but 1024 x 1801, rank 64 only
+// 8.4 -> 5.7 + 2.5, which is where the line lies.
+int low_rank(wf_seq_engine* e, const float* src, int ld, const void* w, int rank, float* out, int nout, int n, int og_cols) {
+    const GemmArgs g = lin(e->og, 0, rank, w, rank, out, 1, nout, n, nout, rank);
+    if (e->dt == WF_BF16 && rank <= og_cols && (long long)n * nout * rank >= 80000000ll && gemm_tc_usable(g)) {
+        if (int rc = launch_gate_mul(e->dt, src, ld, src, ld, 2, n, rank, e->og, rank, e->stream)) return rc;
+        return launch_gemm(e->dt, g, e->stream);
+    }
+    return launch_gemm(e->dt, lin(src, 1, ld, w, rank, out, 1, nout, n, nout, rank), e->stream);
+}
+
 int run_delta(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
     const wf_seq_layer& c = L.c;
     const int W = e->cfg.width, n = b.n, H = c.heads, nv = H * c.vdim, C = L.C;
@@ -596,13 +608,13 @@ int run_delta(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
     const float* g_raw = e->proj + L.g_col;
     int ldg = L.np;
     if (c.gate_rank > 0) {
-        if ((rc = launch_gemm(e->dt, lin(e->proj + L.g_col, 1, L.np, L.g2, c.gate_rank, e->gfull, 1, nv, n, nv, c.gate_rank), s))) return rc;
+        if ((rc = low_rank(e, e->proj + L.g_col, L.np, L.g2, c.gate_rank, e->gfull, nv, n, nv))) return rc;
         g_raw = e->gfull; ldg = nv;
     }
     const float* a_raw = e->proj + L.a_col;
     int lda = L.np;
     if (c.decay_rank > 0) {
-        if ((rc = launch_gemm(e->dt, lin(e->proj + L.a_col, 1, L.np, L.a2, c.decay_rank, e->afull, 1, L.n_decay, n, L.n_decay, c.decay_rank), s))) return rc;
+        if ((rc = low_rank(e, e->proj + L.a_col, L.np, L.a2, c.decay_rank, e->afull, L.n_decay, n, nv))) return rc;
         a_raw = e->afull; lda = L.n_decay;
     }
     if (c.gate_rank > 0 || c.decay_rank > 0) mark(e, "delta.lowrank_gemm");
