@@ -219,15 +219,18 @@ template <int DS, bool VEC, bool DELTA> struct CrStage {
 };
 constexpr int CR_RS = 24;                                 // row stride of the partial sums [16 columns][16 tokens]
 
-template <int DS, bool VEC, bool DELTA>
+// CT: tiles of 16 columns that a block takes.  The key and query rows that the products need as sums of two numbers are split once for all of them; without the
+// correction that splitting was the larger part of the work.
+template <int DS, bool VEC, bool DELTA, int CT>
 __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
     pdl_enter();
     using L = CrStage<DS, VEC, DELTA>;
     constexpr int REC = cr_rec_floats(DS, VEC), NT = DS / (8 * CR_WARPS), STEP = CR_THREADS / (DS / 4);
+    static_assert(CT == 1 || (CT == 2 && !DELTA), "the partial sums hold two tiles");
     extern __shared__ __align__(16) float sm[];
-    float* red = sm + 2 * L::FLOATS;                      // [4 warps][S^T q | R][16 columns][CR_RS]
+    float* red = sm + 2 * L::FLOATS;                      // [4 warps][S^T q | R, or S^T q of each column tile][16 columns][CR_RS]
     const int sq = blockIdx.x / sg.n, seg = blockIdx.x - sq * sg.n, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    const int col0 = blockIdx.z * CR_COLS, dvs = D.dv + D.ones_col, kh = h / (D.H / D.Hk);
+    const int col0 = blockIdx.z * CR_COLS * CT, dvs = D.dv + D.ones_col, kh = h / (D.H / D.Hk);
     const int first = seg * SCAN_CHUNK, seq0 = b.seq_start[sq], start = seq0 + first;
     const int len = sg.pass ? min(SCAN_CHUNK, b.seq_len[sq] - first) : b.seq_len[sq], nch = (len + CR - 1) / CR;
     if (len <= 0) return;                                 // this sequence has fewer segments
@@ -236,17 +239,19 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
     const float* rec0 = w.rec + ((size_t)(seq0 / CR + sq + first / CR) * D.H + h) * REC;
     float prod = 1.f;
     const int row0 = warp * 8 * NT;                       // this warp's key rows
-    // s[nt]: columns col0 + g (0, 1) and col0 + g + 8 (2, 3), rows row0 + 8 nt + 2 t (0, 2) and + 1 (1, 3)
-    float s[NT][4];
-    auto at_state = [&](int nt, int e, bool& ok) -> size_t {
-        const int r = row0 + 8 * nt + 2 * t + (e & 1), c = col0 + g + 8 * (e >> 1);
+    // s[ct][nt]: columns col0 + 16 ct + g (0, 1) and + 8 (2, 3), rows row0 + 8 nt + 2 t (0, 2) and + 1 (1, 3)
+    float s[CT][NT][4];
+    auto at_state = [&](int ct, int nt, int e, bool& ok) -> size_t {
+        const int r = row0 + 8 * nt + 2 * t + (e & 1), c = col0 + 16 * ct + g + 8 * (e >> 1);
         ok = r < D.d && c < dvs;
         return (size_t)r * dvs + c;
     };
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+    for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) { bool ok; const size_t i = at_state(nt, e, ok); s[nt][e] = ok && sg.pass != 1 ? S0[i] : 0.f; }
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { bool ok; const size_t i = at_state(ct, nt, e, ok); s[ct][nt][e] = ok && sg.pass != 1 ? S0[i] : 0.f; }
     auto stage = [&](int ch) {
         float* dst = sm + (ch & 1) * L::FLOATS;
         const float* src = rec0 + (size_t)ch * D.H * REC;
@@ -287,14 +292,18 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
         cp_async_commit();
     };
     // a chunk's values (times beta without the correction), in accumulator layout: columns g and g + 8, tokens 8 n + 2 t and + 1
-    float vn[2][4], bn[2][2];
+    float vn[CT][2][4], bn[2][2];
     auto values = [&](int tok0) {
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int tk = tok0 + 8 * n + 2 * t + (e & 1), c = col0 + g + 8 * (e >> 1);
-                vn[n][e] = tk >= len || c >= dvs ? 0.f : c == D.dv ? 1.f : w.qkv[(size_t)(start + tk) * w.ld + w.v_off + h * D.dv + c];
+                const int tk = tok0 + 8 * n + 2 * t + (e & 1);
+#pragma unroll
+                for (int ct = 0; ct < CT; ++ct) {
+                    const int c = col0 + 16 * ct + g + 8 * (e >> 1);
+                    vn[ct][n][e] = tk >= len || c >= dvs ? 0.f : c == D.dv ? 1.f : w.qkv[(size_t)(start + tk) * w.ld + w.v_off + h * D.dv + c];
+                }
                 if (!DELTA && e < 2) bn[n][e] = w.beta && tk < len ? w.beta[(size_t)(start + tk) * D.H + h] : 1.f;
             }
     };
@@ -303,25 +312,30 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
     values(0);
     for (int ch = 0; ch < nch; ++ch) {
         const int tok0 = ch * CR;
-        float v[2][4];
+        float v[CT][2][4];
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[n][e] = DELTA ? vn[n][e] : vn[n][e] * bn[n][e & 1];
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[ct][n][e] = DELTA ? vn[ct][n][e] : vn[ct][n][e] * bn[n][e & 1];
         cp_async_wait<0>();
         __syncthreads();                                  // chunk ch has landed; everyone is done with the other half and the partial sums
         if (ch + 1 < nch) { stage(ch + 1); values(tok0 + CR); }
         const float* st = sm + (ch & 1) * L::FLOATS;
         if (DELTA || sg.pass != 1) {
         // ---- this warp's rows' share of S^T q and R; the small terms in accumulators of their own, so that no product waits for the one before it
-        float oq[2][4], rk[2][4], oql[2][4], rkl[2][4];
+        float oq[CT][2][4], rk[2][4], oql[CT][2][4], rkl[2][4];
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) oq[n][e] = rk[n][e] = oql[n][e] = rkl[n][e] = 0.f;
+            for (int e = 0; e < 4; ++e) {
+                rk[n][e] = rkl[n][e] = 0.f;
+#pragma unroll
+                for (int ct = 0; ct < CT; ++ct) oq[ct][n][e] = oql[ct][n][e] = 0.f;
+            }
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-            const CrA a = cr_a(s[nt]);
             const int r = row0 + 8 * nt + 2 * t;
             CrB q[2], k[2];
 #pragma unroll
@@ -330,23 +344,26 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
                 if (DELTA) k[n] = cr_b2(st + L::K + (8 * n + g) * L::QS + r);
             }
 #pragma unroll
-            for (int n = 0; n < 2; ++n) { cr_mma(oql[n], a.l, q[n].h); if (DELTA) cr_mma(rkl[n], a.l, k[n].h); }
+            for (int ct = 0; ct < CT; ++ct) {
+                const CrA a = cr_a(s[ct][nt]);
 #pragma unroll
-            for (int n = 0; n < 2; ++n) { cr_mma(oq[n], a.h, q[n].h); if (DELTA) cr_mma(rk[n], a.h, k[n].h); }
+                for (int n = 0; n < 2; ++n) { cr_mma(oql[ct][n], a.l, q[n].h); if (DELTA) cr_mma(rkl[n], a.l, k[n].h); }
 #pragma unroll
-            for (int n = 0; n < 2; ++n) { cr_mma(oql[n], a.h, q[n].l); if (DELTA) cr_mma(rkl[n], a.h, k[n].l); }
+                for (int n = 0; n < 2; ++n) { cr_mma(oq[ct][n], a.h, q[n].h); if (DELTA) cr_mma(rk[n], a.h, k[n].h); }
+#pragma unroll
+                for (int n = 0; n < 2; ++n) { cr_mma(oql[ct][n], a.h, q[n].l); if (DELTA) cr_mma(rkl[n], a.h, k[n].l); }
+            }
         }
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) { oq[n][e] += oql[n][e]; if (DELTA) rk[n][e] += rkl[n][e]; }
         float* mine = red + warp * 2 * CR_COLS * CR_RS;
 #pragma unroll
         for (int n = 0; n < 2; ++n)
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                *reinterpret_cast<float2*>(mine + (g + 8 * c) * CR_RS + 8 * n + 2 * t) = make_float2(oq[n][2 * c], oq[n][2 * c + 1]);
-                if (DELTA) *reinterpret_cast<float2*>(mine + (CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t) = make_float2(rk[n][2 * c], rk[n][2 * c + 1]);
+#pragma unroll
+                for (int ct = 0; ct < CT; ++ct)
+                    *reinterpret_cast<float2*>(mine + (ct * CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t) =
+                        make_float2(oq[ct][n][2 * c] + oql[ct][n][2 * c], oq[ct][n][2 * c + 1] + oql[ct][n][2 * c + 1]);
+                if (DELTA) *reinterpret_cast<float2*>(mine + (CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t) = make_float2(rk[n][2 * c] + rkl[n][2 * c], rk[n][2 * c + 1] + rkl[n][2 * c + 1]);
             }
         }
         if (DELTA || sg.pass != 1) __syncthreads();
@@ -357,7 +374,7 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
             for (int k = 1; k < CR_WARPS; ++k) { const float2 y = *reinterpret_cast<const float2*>(p + k * 2 * CR_COLS * CR_RS); x.x += y.x; x.y += y.y; }
             return x;
         };
-        float u[2][4];
+        float u[CT][2][4];
         if (DELTA) {                                      // every warp forms all of U: it is the update's operand
 #pragma unroll
             for (int n = 0; n < 2; ++n)
@@ -365,97 +382,116 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
                 for (int c = 0; c < 2; ++c) {
                     float2 r = total(1, n, c);
                     if (!VEC) { r.x *= st[L::G + 8 * n + 2 * t]; r.y *= st[L::G + 8 * n + 2 * t + 1]; }
-                    v[n][2 * c] -= r.x; v[n][2 * c + 1] -= r.y;
+                    v[0][n][2 * c] -= r.x; v[0][n][2 * c + 1] -= r.y;
                 }
-            const CrA w0 = cr_a(v[0]), w1 = cr_a(v[1]);
+            const CrA w0 = cr_a(v[0][0]), w1 = cr_a(v[0][1]);
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
-                u[n][0] = u[n][1] = u[n][2] = u[n][3] = 0.f;
+                u[0][n][0] = u[0][n][1] = u[0][n][2] = u[0][n][3] = 0.f;
                 const float* row = st + L::T + (8 * n + g) * L::TS + 2 * t;
-                cr_mma3(u[n], w0, cr_b2(row));
-                if (n) cr_mma3(u[n], w1, cr_b2(row + 8));   // T is lower triangular
+                cr_mma3(u[0][n], w0, cr_b2(row));
+                if (n) cr_mma3(u[0][n], w1, cr_b2(row + 8));   // T is lower triangular
             }
         } else {
 #pragma unroll
-            for (int n = 0; n < 2; ++n)
+            for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) u[n][e] = v[n][e];
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) u[ct][n][e] = v[ct][n][e];
         }
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) cr_watch(watch[2 * n + (e & 1)], u[n][e]);
-        if (warp < 2 && sg.pass != 1) {                                   // the read-out of 8 tokens each
-            const int n = warp;
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) cr_watch(watch[2 * n + (e & 1)], u[ct][n][e]);
+        if (warp < 2 * CT && sg.pass != 1) {                              // the read-out of 8 tokens of a column tile each
+            const int n = warp & 1, ct = warp >> 1;
             float out[4], add[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                float2 x = total(0, n, c);
+                float2 x = total(ct, n, c);
                 if (!VEC) { x.x *= st[L::G + 8 * n + 2 * t]; x.y *= st[L::G + 8 * n + 2 * t + 1]; }
                 out[2 * c] = x.x; out[2 * c + 1] = x.y;
             }
+            float ua[2][4];                               // this tile's values: a choice of registers, not an indexed array
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) ua[m][e] = CT == 2 && ct ? u[CT - 1][m][e] : u[0][m][e];
             const float* row = st + L::B + (8 * n + g) * L::TS + 2 * t;
-            cr_mma3(add, cr_a(u[0]), cr_b2(row));
-            if (n) cr_mma3(add, cr_a(u[1]), cr_b2(row + 8));
+            cr_mma3(add, cr_a(ua[0]), cr_b2(row));
+            if (n) cr_mma3(add, cr_a(ua[1]), cr_b2(row + 8));
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const int tk = tok0 + 8 * n + 2 * t + (e & 1), c = col0 + g + 8 * (e >> 1);
+                const int tk = tok0 + 8 * n + 2 * t + (e & 1), c = col0 + 16 * ct + g + 8 * (e >> 1);
                 if (tk < len && c < dvs) o[((size_t)(start + tk) * D.H + h) * dvs + c] = (out[e] + add[e]) * D.o_scale;
             }
         }
         if (!VEC) prod *= st[L::G + 32];
         // ---- state update: the chunk's own sum from zero, so that the state itself is only ever rounded to nearest (the matrix unit's sums are cut off)
-        if (!VEC) {
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                const float d0 = st[L::G + 16 + 8 * n + 2 * t], d1 = st[L::G + 16 + 8 * n + 2 * t + 1];
-                u[n][0] *= d0; u[n][1] *= d1; u[n][2] *= d0; u[n][3] *= d1;
-            }
-        }
-        const CrA u0 = cr_a(u[0]), u1 = cr_a(u[1]);
         CrB k0[NT], k1[NT];
-        float ds[NT][4];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             const float* kr = st + L::N + 2 * t * L::KS + row0 + 8 * nt + g;
             k0[nt] = cr_b(kr[0], kr[L::KS]); k1[nt] = cr_b(kr[8 * L::KS], kr[9 * L::KS]);
-            ds[nt][0] = ds[nt][1] = ds[nt][2] = ds[nt][3] = 0.f;
         }
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u0.l, k0[nt].h);
+        for (int ct = 0; ct < CT; ++ct) {
+            if (!VEC) {
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u0.h, k0[nt].l);
+                for (int n = 0; n < 2; ++n) {
+                    const float d0 = st[L::G + 16 + 8 * n + 2 * t], d1 = st[L::G + 16 + 8 * n + 2 * t + 1];
+                    u[ct][n][0] *= d0; u[ct][n][1] *= d1; u[ct][n][2] *= d0; u[ct][n][3] *= d1;
+                }
+            }
+            const CrA u0 = cr_a(u[ct][0]), u1 = cr_a(u[ct][1]);
+            float ds[NT][4];
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u1.l, k1[nt].h);
+            for (int nt = 0; nt < NT; ++nt) ds[nt][0] = ds[nt][1] = ds[nt][2] = ds[nt][3] = 0.f;
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u1.h, k1[nt].l);
+            for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u0.l, k0[nt].h);
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u0.h, k0[nt].h);
+            for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u0.h, k0[nt].l);
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u1.h, k1[nt].h);
+            for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u1.l, k1[nt].h);
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-            float2 ge;
-            if (VEC) ge = *reinterpret_cast<const float2*>(st + L::G + row0 + 8 * nt + 2 * t);
-            else ge.x = ge.y = st[L::G + 32];
-            s[nt][0] = fmaf(s[nt][0], ge.x, ds[nt][0]); s[nt][1] = fmaf(s[nt][1], ge.y, ds[nt][1]);
-            s[nt][2] = fmaf(s[nt][2], ge.x, ds[nt][2]); s[nt][3] = fmaf(s[nt][3], ge.y, ds[nt][3]);
+            for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u1.h, k1[nt].l);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u0.h, k0[nt].h);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) cr_mma(ds[nt], u1.h, k1[nt].h);
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                float2 ge;
+                if (VEC) ge = *reinterpret_cast<const float2*>(st + L::G + row0 + 8 * nt + 2 * t);
+                else ge.x = ge.y = st[L::G + 32];
+                s[ct][nt][0] = fmaf(s[ct][nt][0], ge.x, ds[nt][0]); s[ct][nt][1] = fmaf(s[ct][nt][1], ge.y, ds[nt][1]);
+                s[ct][nt][2] = fmaf(s[ct][nt][2], ge.x, ds[nt][2]); s[ct][nt][3] = fmaf(s[ct][nt][3], ge.y, ds[nt][3]);
+            }
         }
     }
     // a state that has left the finite numbers does not come back: looked at once
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+    for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) cr_watch(watch[e], s[nt][e]);
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) cr_watch(watch[e], s[ct][nt][e]);
     const int lost = __syncthreads_or(!((watch[0] + watch[1]) + (watch[2] + watch[3]) == 0.f));
-    if (lost && tid == 0) w.redo[((size_t)sq * D.H + h) * w.cols + blockIdx.z] = 1;
+    int* mark = w.redo + ((size_t)sq * D.H + h) * w.cols + blockIdx.z * CT;      // the preparation marks all of a head's tiles
+    const int tiles = min(CT, w.cols - (int)blockIdx.z * CT);
+    if (lost && tid < tiles) mark[tid] = 1;
     if (sg.pass == 3) return;                             // scan_prefix_kernel has left the end states
-    if (sg.pass == 0 && (lost || w.redo[((size_t)sq * D.H + h) * w.cols + blockIdx.z])) return;      // the slot keeps the start state for chunk_redo_kernel
+    if (sg.pass == 0 && (lost || *mark)) return;          // the slot keeps the start state for chunk_redo_kernel
     float* S1 = sg.pass ? sg.local + entry : state + (size_t)b.seq_slot[sq] * slot_stride + (size_t)h * D.d * dvs;
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+    for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) { bool ok; const size_t i = at_state(nt, e, ok); if (ok) S1[i] = s[nt][e]; }
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { bool ok; const size_t i = at_state(ct, nt, e, ok); if (ok) S1[i] = s[ct][nt][e]; }
     if (!VEC && sg.pass && blockIdx.z == 0 && tid == 0) sg.prod[(size_t)(seq0 / SCAN_CHUNK + sq + seg) * D.H + h] = prod;
 }
 
@@ -544,7 +580,8 @@ int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const floa
     if (int rc = launch_check(cudaGetLastError(), "chunk_prep")) return rc;
     constexpr size_t smem = (size_t)(2 * CrStage<DS, VEC, DELTA>::FLOATS + CR_WARPS * 2 * CR_COLS * CR_RS) * sizeof(float);
     static DevOnce once;
-    if (once.need() && cuda_check(cudaFuncSetAttribute(chunk_scan_kernel<DS, VEC, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "chunk shared memory")) return WF_ERR_CUDA;
+    constexpr int CT = DELTA ? 1 : 2;                      // column tiles per block
+    if (once.need() && cuda_check(cudaFuncSetAttribute(chunk_scan_kernel<DS, VEC, DELTA, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "chunk shared memory")) return WF_ERR_CUDA;
     Segments sg;
     const int cols = w.cols;
     auto redo = [&]() {
@@ -553,7 +590,7 @@ int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const floa
     };
     auto scan_pass = [&](int pass) {
         sg.pass = pass;
-        launch_pdl(chunk_scan_kernel<DS, VEC, DELTA>, dim3(b.nseq * sg.n, D.H, cols), CR_THREADS, smem, s, b, D, w, state, slot_stride, o, sg);
+        launch_pdl(chunk_scan_kernel<DS, VEC, DELTA, CT>, dim3(b.nseq * sg.n, D.H, (cols + CT - 1) / CT), CR_THREADS, smem, s, b, D, w, state, slot_stride, o, sg);
         return launch_check(cudaGetLastError(), "chunk_scan");
     };
     // Segments in parallel where the recurrence is linear in the state, one portion is long and the chains of whole portions leave the machine idle: the two
