@@ -11,7 +11,7 @@
 //     shared memory once per chunk.
 // What bounded the forms before: token by token, a chain of multiply-adds, shuffles and shared-memory reads of about 1000 clk per token; chunks on
 // the multiply-add units, shared-memory bandwidth (every thread of a column reads every key: 5 wavefronts per request, 450 us for the case below).
-// Measured: delta rule (20 heads, 128 x 128, two sequences, 1801 tokens) 569 -> 236 us, state space (40 heads, 128 x 64, one sequence, 2048 tokens) 307 -> 213 us;
+// Measured: delta rule (20 heads, 128 x 128, two sequences, 1801 tokens) 569 -> 236 us, state space (40 heads, 128 x 64, one sequence, 2048 tokens) 307 -> 179 us;
 // with eight warps of half the rows each 287 and 257 us (both in one pass).  Left: the chain of a chunk, about 3000 clk of products, one exchange of partial
 // sums and two barriers.  Error against 64 bits (2-norm of a mixer's output, up to 2048 tokens): in float32 engines 4.47e-7 against 4.36e-7 token by token (delta rule),
 // 3.35e-7 / 3.33e-7 (state space), 4.82e-7 / 4.94e-7 (matrix memory); float32 engines keep the token form all the same.  In bf16 engines both 2.05e-3, 1.67e-3, 1.66e-3.
@@ -220,15 +220,15 @@ template <int DS, bool VEC, bool DELTA> struct CrStage {
 constexpr int CR_RS = 24;                                 // row stride of the partial sums [16 columns][16 tokens]
 
 // CT: tiles of 16 columns that a block takes.  The key and query rows that the products need as sums of two numbers are split once for all of them; without the
-// correction that splitting was the larger part of the work.
+// correction that splitting was the larger part of the work (the two passes over 40 heads of 128 x 64, 2048 tokens: 63 + 97 us with one, 48 + 78 with two).
 template <int DS, bool VEC, bool DELTA, int CT>
 __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
     pdl_enter();
     using L = CrStage<DS, VEC, DELTA>;
     constexpr int REC = cr_rec_floats(DS, VEC), NT = DS / (8 * CR_WARPS), STEP = CR_THREADS / (DS / 4);
-    static_assert(CT == 1 || (CT == 2 && !DELTA), "the partial sums hold two tiles");
+    constexpr int PARTS = DELTA ? 2 * CT : 2;              // partial sums of a warp: S^T q of each column tile, then R of each
     extern __shared__ __align__(16) float sm[];
-    float* red = sm + 2 * L::FLOATS;                      // [4 warps][S^T q | R, or S^T q of each column tile][16 columns][CR_RS]
+    float* red = sm + 2 * L::FLOATS;                      // [4 warps][PARTS][16 columns][CR_RS]
     const int sq = blockIdx.x / sg.n, seg = blockIdx.x - sq * sg.n, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int col0 = blockIdx.z * CR_COLS * CT, dvs = D.dv + D.ones_col, kh = h / (D.H / D.Hk);
     const int first = seg * SCAN_CHUNK, seq0 = b.seq_start[sq], start = seq0 + first;
@@ -325,15 +325,13 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
         const float* st = sm + (ch & 1) * L::FLOATS;
         if (DELTA || sg.pass != 1) {
         // ---- this warp's rows' share of S^T q and R; the small terms in accumulators of their own, so that no product waits for the one before it
-        float oq[CT][2][4], rk[2][4], oql[CT][2][4], rkl[2][4];
+        float oq[CT][2][4], rk[CT][2][4], oql[CT][2][4], rkl[CT][2][4];
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                rk[n][e] = rkl[n][e] = 0.f;
+            for (int n = 0; n < 2; ++n)
 #pragma unroll
-                for (int ct = 0; ct < CT; ++ct) oq[ct][n][e] = oql[ct][n][e] = 0.f;
-            }
+                for (int e = 0; e < 4; ++e) oq[ct][n][e] = oql[ct][n][e] = rk[ct][n][e] = rkl[ct][n][e] = 0.f;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             const int r = row0 + 8 * nt + 2 * t;
@@ -347,50 +345,54 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
             for (int ct = 0; ct < CT; ++ct) {
                 const CrA a = cr_a(s[ct][nt]);
 #pragma unroll
-                for (int n = 0; n < 2; ++n) { cr_mma(oql[ct][n], a.l, q[n].h); if (DELTA) cr_mma(rkl[n], a.l, k[n].h); }
+                for (int n = 0; n < 2; ++n) { cr_mma(oql[ct][n], a.l, q[n].h); if (DELTA) cr_mma(rkl[ct][n], a.l, k[n].h); }
 #pragma unroll
-                for (int n = 0; n < 2; ++n) { cr_mma(oq[ct][n], a.h, q[n].h); if (DELTA) cr_mma(rk[n], a.h, k[n].h); }
+                for (int n = 0; n < 2; ++n) { cr_mma(oq[ct][n], a.h, q[n].h); if (DELTA) cr_mma(rk[ct][n], a.h, k[n].h); }
 #pragma unroll
-                for (int n = 0; n < 2; ++n) { cr_mma(oql[ct][n], a.h, q[n].l); if (DELTA) cr_mma(rkl[n], a.h, k[n].l); }
+                for (int n = 0; n < 2; ++n) { cr_mma(oql[ct][n], a.h, q[n].l); if (DELTA) cr_mma(rkl[ct][n], a.h, k[n].l); }
             }
         }
-        float* mine = red + warp * 2 * CR_COLS * CR_RS;
+        float* mine = red + warp * PARTS * CR_COLS * CR_RS;
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int ct = 0; ct < CT; ++ct)
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (int n = 0; n < 2; ++n)
 #pragma unroll
-                for (int ct = 0; ct < CT; ++ct)
-                    *reinterpret_cast<float2*>(mine + (ct * CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t) =
-                        make_float2(oq[ct][n][2 * c] + oql[ct][n][2 * c], oq[ct][n][2 * c + 1] + oql[ct][n][2 * c + 1]);
-                if (DELTA) *reinterpret_cast<float2*>(mine + (CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t) = make_float2(rk[n][2 * c] + rkl[n][2 * c], rk[n][2 * c + 1] + rkl[n][2 * c + 1]);
-            }
+                for (int c = 0; c < 2; ++c) {
+                    float* to = mine + (ct * CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t;
+                    *reinterpret_cast<float2*>(to) = make_float2(oq[ct][n][2 * c] + oql[ct][n][2 * c], oq[ct][n][2 * c + 1] + oql[ct][n][2 * c + 1]);
+                    if (DELTA) *reinterpret_cast<float2*>(to + CT * CR_COLS * CR_RS) = make_float2(rk[ct][n][2 * c] + rkl[ct][n][2 * c], rk[ct][n][2 * c + 1] + rkl[ct][n][2 * c + 1]);
+                }
         }
         if (DELTA || sg.pass != 1) __syncthreads();
         auto total = [&](int part, int n, int c) {
             const float* p = red + (part * CR_COLS + g + 8 * c) * CR_RS + 8 * n + 2 * t;
             float2 x = *reinterpret_cast<const float2*>(p);
 #pragma unroll
-            for (int k = 1; k < CR_WARPS; ++k) { const float2 y = *reinterpret_cast<const float2*>(p + k * 2 * CR_COLS * CR_RS); x.x += y.x; x.y += y.y; }
+            for (int k = 1; k < CR_WARPS; ++k) { const float2 y = *reinterpret_cast<const float2*>(p + k * PARTS * CR_COLS * CR_RS); x.x += y.x; x.y += y.y; }
             return x;
         };
         float u[CT][2][4];
         if (DELTA) {                                      // every warp forms all of U: it is the update's operand
+            CrB tb[3];                                    // T is lower triangular
+            tb[0] = cr_b2(st + L::T + g * L::TS + 2 * t); tb[1] = cr_b2(st + L::T + (8 + g) * L::TS + 2 * t); tb[2] = cr_b2(st + L::T + (8 + g) * L::TS + 2 * t + 8);
 #pragma unroll
-            for (int n = 0; n < 2; ++n)
+            for (int ct = 0; ct < CT; ++ct) {
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    float2 r = total(1, n, c);
-                    if (!VEC) { r.x *= st[L::G + 8 * n + 2 * t]; r.y *= st[L::G + 8 * n + 2 * t + 1]; }
-                    v[0][n][2 * c] -= r.x; v[0][n][2 * c + 1] -= r.y;
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        float2 r = total(CT + ct, n, c);
+                        if (!VEC) { r.x *= st[L::G + 8 * n + 2 * t]; r.y *= st[L::G + 8 * n + 2 * t + 1]; }
+                        v[ct][n][2 * c] -= r.x; v[ct][n][2 * c + 1] -= r.y;
+                    }
+                const CrA w0 = cr_a(v[ct][0]), w1 = cr_a(v[ct][1]);
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    u[ct][n][0] = u[ct][n][1] = u[ct][n][2] = u[ct][n][3] = 0.f;
+                    cr_mma3(u[ct][n], w0, tb[n]);
+                    if (n) cr_mma3(u[ct][n], w1, tb[2]);
                 }
-            const CrA w0 = cr_a(v[0][0]), w1 = cr_a(v[0][1]);
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                u[0][n][0] = u[0][n][1] = u[0][n][2] = u[0][n][3] = 0.f;
-                const float* row = st + L::T + (8 * n + g) * L::TS + 2 * t;
-                cr_mma3(u[0][n], w0, cr_b2(row));
-                if (n) cr_mma3(u[0][n], w1, cr_b2(row + 8));   // T is lower triangular
             }
         } else {
 #pragma unroll
@@ -574,13 +576,12 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_redo_kernel(Batch b, DeltaDi
     if (tid == 0) *mark = 0;
 }
 
-template <int DS, bool VEC, bool DELTA>
+template <int DS, bool VEC, bool DELTA, int CT>
 int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const float* decay, float* state, size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan) {
     launch_pdl(chunk_prep_kernel<DS, VEC, DELTA>, dim3(b.nseq * w.nchunks, D.H), CR_THREADS, 0, s, b, D, w);
     if (int rc = launch_check(cudaGetLastError(), "chunk_prep")) return rc;
-    constexpr size_t smem = (size_t)(2 * CrStage<DS, VEC, DELTA>::FLOATS + CR_WARPS * 2 * CR_COLS * CR_RS) * sizeof(float);
+    constexpr size_t smem = (size_t)(2 * CrStage<DS, VEC, DELTA>::FLOATS + CR_WARPS * (DELTA ? 2 * CT : 2) * CR_COLS * CR_RS) * sizeof(float);
     static DevOnce once;
-    constexpr int CT = DELTA ? 1 : 2;                      // column tiles per block
     if (once.need() && cuda_check(cudaFuncSetAttribute(chunk_scan_kernel<DS, VEC, DELTA, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "chunk shared memory")) return WF_ERR_CUDA;
     Segments sg;
     const int cols = w.cols;
@@ -632,9 +633,12 @@ int launch_chunk_recurrence(const Batch& b, const DeltaDims& D, const float* qkv
     w.q_off = D.q_off >= 0 ? D.q_off : 0; w.k_off = D.k_off >= 0 ? D.k_off : D.Hk * D.d; w.v_off = D.v_off >= 0 ? D.v_off : 2 * D.Hk * D.d;
     w.redo = scan->redo; w.cols = (D.dv + D.ones_col + CR_COLS - 1) / CR_COLS;
     w.rec = scan->rec; w.nchunks = (b.max_len + CR - 1) / CR;
-#define CR_PICK(vec, delta) (D.d <= 64 ? cr_launch<64, vec, delta>(b, D, w, decay, state, slot_stride, o, s, scan) : cr_launch<128, vec, delta>(b, D, w, decay, state, slot_stride, o, s, scan))
-    if (D.no_delta) return D.vec_decay ? CR_PICK(true, false) : CR_PICK(false, false);
-    return D.vec_decay ? CR_PICK(true, true) : CR_PICK(false, true);
+#define CR_PICK(vec, delta, ct) (D.d <= 64 ? cr_launch<64, vec, delta, ct>(b, D, w, decay, state, slot_stride, o, s, scan) : cr_launch<128, vec, delta, ct>(b, D, w, decay, state, slot_stride, o, s, scan))
+    if (D.no_delta) return D.vec_decay ? CR_PICK(true, false, 2) : CR_PICK(false, false, 2);
+    // With the correction two column tiles a block are the longer chain and the lesser work: us with one / two, 20 heads of 128 x 128 in 1 sequence (160 blocks
+    // of one) 351 / 387, 2 (320) 192 / 208, 4 (640) 186 / 171.
+    if ((long long)b.nseq * D.H * w.cols > 4LL * sm_count()) return D.vec_decay ? CR_PICK(true, true, 2) : CR_PICK(false, true, 2);
+    return D.vec_decay ? CR_PICK(true, true, 1) : CR_PICK(false, true, 1);
 #undef CR_PICK
 }
 
