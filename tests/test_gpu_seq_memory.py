@@ -46,9 +46,9 @@ def test_the_workspaces_of_the_faster_forms_are_not_required(monkeypatch):
     assert size == small and np.array_equal(tight, plain)
 
 
-@pytest.mark.parametrize("vocab,wants", [(4099, (1, 64, 65, 130)), (65536, (1, 4, 5, 9))])
+@pytest.mark.parametrize("vocab,wants", [(4099, (1, 64, 65, 180)), (65536, (1, 2, 8, 11))])
 def test_logits_reach_pageable_memory_as_they_reach_pinned(vocab, wants):
-    """One piece, whole pieces, a part of a piece, more pieces than are in flight at once (256 KB each, four at once): equal to one copy into pinned memory."""
+    """One piece, whole pieces, a part of a piece, more pieces than are in flight at once (512 KB each, four at once): equal to one copy into pinned memory."""
     from wf_bitnet._lib import seq_check, seq_lib
     from test_gpu_tutizen import attn, build, config, make_weights, with_ff, dense
     cfg = config([with_ff(attn(), dense())], vocab=vocab)

@@ -372,22 +372,41 @@ __global__ void __launch_bounds__(AM_THREADS, 3) gqa_attn_mma_kernel(Batch b, Gq
     }
 }
 
-// one warp per (token, head): merge the key splits' partial results (maxima in units of log 2), apply the gate
+// one warp per (token, head): merge the key splits' partial results (maxima in units of log 2), apply the gate.  A lane a split for the maxima and sums, then the
+// splits' values side by side: two memory latencies, where one split after the other took one each (a merge of a decode step 4.3 -> 2.4 us).
 __global__ void gqa_attn_merge_kernel(GqaDims D, int rows, int splits, const float* __restrict__ part, const float* __restrict__ gate, __nv_bfloat16* __restrict__ out) {
     pdl_enter();
-    const int dv = D.dv, gate_elem = D.gate_elem;
+    const int dv = D.dv, gate_elem = D.gate_elem, stride = dv + 2;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
-    const float* p = part + (size_t)row * splits * (dv + 2);
+    const float* p = part + (size_t)row * splits * stride;
+    auto peak = [&](int z) { return z < splits ? p[(size_t)z * stride + dv] : -INFINITY; };
     float mg = -INFINITY;
-    for (int z = 0; z < splits; ++z) mg = fmaxf(mg, p[(size_t)z * (dv + 2) + dv]);
+    for (int z = lane; z < splits; z += 32) mg = fmaxf(mg, peak(z));
+    mg = warp_max(mg);
     float lg = 0.f;
-    for (int z = 0; z < splits; ++z) { const float m = p[(size_t)z * (dv + 2) + dv]; lg += m == -INFINITY ? 0.f : p[(size_t)z * (dv + 2) + dv + 1] * exp2f(m - mg); }
+    for (int z = lane; z < splits; z += 32) { const float m = peak(z); lg += m == -INFINITY ? 0.f : p[(size_t)z * stride + dv + 1] * exp2f(m - mg); }
+    lg = warp_sum(lg);
     const float mul = (gate && !gate_elem ? gate[row] : 1.f) * am_inv_sum(D, row % D.H, mg, lg);
-    for (int c = lane; c < dv; c += 32) {
-        float v = 0.f;
-        for (int z = 0; z < splits; ++z) { const float m = p[(size_t)z * (dv + 2) + dv]; if (m != -INFINITY) v += p[(size_t)z * (dv + 2) + c] * exp2f(m - mg); }
-        out[(size_t)row * dv + c] = __float2bfloat16_rn(v * mul * (gate && gate_elem ? gate[(size_t)row * dv + c] : 1.f));
+    float v[4] = {0.f, 0.f, 0.f, 0.f};                     // channels lane + 32 k (at most 128 of them)
+    for (int z0 = 0; z0 < splits; z0 += 32) {
+        const float m = peak(z0 + lane), w = m == -INFINITY ? 0.f : exp2f(m - mg);
+        const unsigned live = __ballot_sync(0xffffffffu, m != -INFINITY);        // a split without keys has written no values
+        const int n = min(32, splits - z0);
+#pragma unroll 4
+        for (int z = 0; z < n; ++z) {
+            const float wz = __shfl_sync(0xffffffffu, w, z);
+            const float* q = p + (size_t)(z0 + z) * stride;
+            if (live >> z & 1) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) if (lane + 32 * k < dv) v[k] += q[lane + 32 * k] * wz;
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int c = lane + 32 * k;
+        if (c < dv) out[(size_t)row * dv + c] = __float2bfloat16_rn(v[k] * mul * (gate && gate_elem ? gate[(size_t)row * dv + c] : 1.f));
     }
 }
 

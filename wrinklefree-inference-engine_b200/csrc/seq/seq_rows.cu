@@ -57,21 +57,28 @@ template <typename T>
 __global__ void embed_pos_kernel(const T* __restrict__ table, const int32_t* __restrict__ tokens, const int32_t* __restrict__ tok_pos, int W, float base,
                                  float* __restrict__ x, T* __restrict__ x_t) {
     pdl_enter();
-    const int i = blockIdx.x;
+    // a thread per pair of channels, which share an angle: the double precision sine and cosine are what this kernel costs (8 tokens x 1024: 5.9 us with four
+    // angles a thread one after the other, 3.6 so)
+    const int i = blockIdx.x, c = 2 * (blockIdx.y * blockDim.x + threadIdx.x);
+    if (c >= W) return;
     const T* row = table + (size_t)tokens[i] * W;
-    const double pos = (double)tok_pos[i], lb = log2((double)base);
-    for (int c = threadIdx.x; c < W; c += blockDim.x) {
-        const double a = pos * exp2(-2.0 * (double)(c >> 1) / (double)W * lb);
-        const float v = to_f(row[c]) + (float)((c & 1) ? cos(a) : sin(a));
-        x[(size_t)i * W + c] = v;
-        if (x_t) x_t[(size_t)i * W + c] = from_f<T>(v);
+    const double a = (double)tok_pos[i] * exp2(-2.0 * (double)(c >> 1) / (double)W * log2((double)base));
+    double sn, cs;
+    sincos(a, &sn, &cs);
+    const float v[2] = {to_f(row[c]) + (float)sn, c + 1 < W ? to_f(row[c + 1]) + (float)cs : 0.f};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if (c + k >= W) break;
+        x[(size_t)i * W + c + k] = v[k];
+        if (x_t) x_t[(size_t)i * W + c + k] = from_f<T>(v[k]);
     }
 }
 
 int launch_embed_pos(int dt, const void* table, const int32_t* tokens, const int32_t* tok_pos, int n, int W, float base, float* x, void* x_t, cudaStream_t s) {
     if (n <= 0) return WF_OK;
-    if (dt == WF_BF16) launch_pdl(embed_pos_kernel<__nv_bfloat16>, n, 256, 0, s, (const __nv_bfloat16*)table, tokens, tok_pos, W, base, x, (__nv_bfloat16*)x_t);
-    else launch_pdl(embed_pos_kernel<float>, n, 256, 0, s, (const float*)table, tokens, tok_pos, W, base, x, (float*)x_t);
+    const dim3 grid(n, ((W + 1) / 2 + 127) / 128);
+    if (dt == WF_BF16) launch_pdl(embed_pos_kernel<__nv_bfloat16>, grid, 128, 0, s, (const __nv_bfloat16*)table, tokens, tok_pos, W, base, x, (__nv_bfloat16*)x_t);
+    else launch_pdl(embed_pos_kernel<float>, grid, 128, 0, s, (const float*)table, tokens, tok_pos, W, base, x, (float*)x_t);
     return launch_check(cudaGetLastError(), "embed_pos");
 }
 
