@@ -76,11 +76,11 @@ def test_the_row_limit_of_the_tcgen05_form_holds_below_17(tmp_path):
         assert r.stdout.split("\n")[:2] == [want, want], r.stdout
 
 
-@pytest.mark.parametrize("ff", [16, 48, 144, 272])
+@pytest.mark.parametrize("ff", [16, 44, 48, 144, 272])
 @pytest.mark.parametrize("design", ["tutizen", "nukezen"])
 def test_gated_unit_in_the_product(design, ff):
-    """Feed-forwards of many tokens, whose activation is formed where the product stores its results: gate and up rows in blocks of 16, a CTA's last blocks
-    missing, token tiles that are not whole; both activations, against the sum in 64 bits on the same bf16 operands.
+    """Feed-forwards whose activation is formed where the product stores its results: few rows, gate and up rows in blocks of 8; many rows, blocks of 16, a CTA's
+    last blocks missing, token tiles that are not whole (44 has no such blocks and keeps the separate kernel there); both activations, against the sum in 64 bits on the same bf16 operands.
 
     Tolerance: the hidden values and the output's operands are rounded to bf16 (2^-9 each); 1e-2 of a row's size is two and a half times that."""
     import numpy as np
@@ -94,7 +94,7 @@ def test_gated_unit_in_the_product(design, ff):
     w = {k: torch.from_numpy(np.asarray(v, np.float32)).to(torch.bfloat16).float().numpy() for k, v in t.make_weights(cfg if design == "tutizen" else (cfg, {}), ff).items()}
     m = t.build(cfg, w, "bfloat16", max_tokens=512, max_step_tokens=384)
     g = {k[len("l0.mlp."):]: torch.from_numpy(v).double() for k, v in w.items() if k.startswith("l0.mlp.")}
-    for n in (17, 33, 300):
+    for n in (1, 7, 16, 17, 33, 300):
         x = torch.randn(n, W, generator=torch.Generator().manual_seed(n + ff)).to(torch.bfloat16).double() * 2
         gate, up = x @ g["gate"].T, x @ g["up"].T
         if design == "tutizen":

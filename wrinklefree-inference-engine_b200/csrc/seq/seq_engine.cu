@@ -475,6 +475,7 @@ int one_norm_rows(const wf_seq_layer& l) {
 GemmArgs lin(const void* A, int a_f32, int lda, const void* B, int ldb, void* C, int c_f32, int ldc, int M, int N, int K) {
     GemmArgs g;
     g.A = A; g.a_f32 = a_f32; g.lda = lda; g.B = B; g.ldb = ldb; g.C = C; g.c_f32 = c_f32; g.ldc = ldc; g.M = M; g.N = N; g.K = K;
+    g.b_const = 1;                                     // every B here is a weight, and loading waits for its copies
     return g;
 }
 
@@ -837,7 +838,7 @@ int run_unit(wf_seq_engine* e, LayerState& L, const Batch& b, float* out, const 
         if ((rc = launch_gemm(e->dt, g, s))) return rc;
         mark(e, "unit.up");
     } else {
-        // prompts: the activation where the product stores its results, so that [gate | up] (113 MB at 2048 x 6912) is neither written nor read
+        // the activation where the product stores its results: [gate | up] (113 MB at 2048 x 6912) is neither written nor read, and decoding has a kernel less
         GemmArgs g = lin(in, 0, W, L.ugu, W, e->uhmid, 0, ff, n, 2 * ff, W);
         g.glu = 1 + L.c.ff_act; g.limit = L.ulimit;
         if (L.c.ff_act <= 2 && gemm_glu_usable(e->dt, g)) {

@@ -339,9 +339,13 @@ void gemv_launch(const GemmArgs& g, const PairArgs& pa, int rows, int ny, cudaSt
 constexpr int FR_WARPS = 8;
 
 // U: 32-k blocks in flight per warp; OCC: blocks per SM
+// Weights that no kernel of the stream has written (b_const) are requested before the kernel waits for the one before it, as many as a warp has in flight: a
+// decode step of 8 sequences through four layers, 21 such products, 154 -> 146 us.
+// glu: a tile's rows 0 .. 7 are gate rows and 8 .. 15 the up rows of the same outputs, so that a pair meets where the tile's sums do.
 template <int NT, int WK, int U, int OCC, bool CF32>
 __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g) {
-    pdl_enter();
+    const bool early = OCC < 4 && g.b_const;              // (four blocks per SM have no registers for it, and one another's loads to wait under)
+    if (!early) pdl_enter();
     constexpr int TILES = FR_WARPS / WK;                  // 16-row tiles per block
     constexpr int C = NT == 1 ? 1 : 4;                    // running sums
     __shared__ float part[FR_WARPS][NT * 8][16 + 1];
@@ -349,7 +353,8 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
     const int tile = warp / WK, kw = warp % WK;
     const int n0 = (blockIdx.x * TILES + tile) * 16;
     const __nv_bfloat16 *B = (const __nv_bfloat16*)g.B, *A = (const __nv_bfloat16*)g.A;
-    const int ra = min(n0 + g4, g.N - 1), rb = min(n0 + g4 + 8, g.N - 1);          // rows past N repeat the last one; they are not stored
+    const int ff = g.N / 2, gr = min(n0 / 2 + g4, ff - 1);
+    const int ra = g.glu ? gr : min(n0 + g4, g.N - 1), rb = g.glu ? ff + gr : min(n0 + g4 + 8, g.N - 1);          // rows past N repeat the last one; they are not stored
     const __nv_bfloat16 *wa = B + (size_t)ra * g.ldb + 8 * t4, *wb = B + (size_t)rb * g.ldb + 8 * t4;
     const __nv_bfloat16* xa[NT];
     bool x_ok[NT];
@@ -362,16 +367,27 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
         for (int j = 0; j < NT; ++j) acc[c][j][0] = acc[c][j][1] = acc[c][j][2] = acc[c][j][3] = 0.f;
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     const int blocks = (g.K + 31) / 32;                   // block i of this warp: steps of 64 k (two blocks) dealt to the WK warps in turn
-    for (int i0 = 0; ; i0 += U) {
-        const int first = ((i0 >> 1) * WK + kw) * 2;
-        if (first >= blocks) break;
-        uint4 a[U], b[U], x[U][NT];
+    uint4 a[U], b[U];
+    auto weights = [&](int i0) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int blk = (((i0 + u) >> 1) * WK + kw) * 2 + ((i0 + u) & 1), k = blk * 32;
             const bool ok = blk < blocks && k + 8 * t4 + 8 <= g.K;
             a[u] = ok ? __ldg(reinterpret_cast<const uint4*>(wa + k)) : zero;
             b[u] = ok ? __ldg(reinterpret_cast<const uint4*>(wb + k)) : zero;
+        }
+    };
+    if (OCC < 4) weights(0);
+    if (early) pdl_enter();
+    for (int i0 = 0; ; i0 += U) {
+        const int first = ((i0 >> 1) * WK + kw) * 2;
+        if (first >= blocks) break;
+        if (OCC >= 4 || i0) weights(i0);
+        uint4 x[U][NT];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int blk = (((i0 + u) >> 1) * WK + kw) * 2 + ((i0 + u) & 1), k = blk * 32;
+            const bool ok = blk < blocks && k + 8 * t4 + 8 <= g.K;
 #pragma unroll
             for (int j = 0; j < NT; ++j) x[u][j] = ok && x_ok[j] ? *reinterpret_cast<const uint4*>(xa[j] + k) : zero;
         }
@@ -411,6 +427,18 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
 #pragma unroll
         for (int e = 0; e < 4; ++e) part[warp][j * 8 + 2 * t4 + (e & 1)][g4 + 8 * (e >> 1)] = C == 1 ? acc[0][j][e] : (acc[0][j][e] + acc[C / 2][j][e]) + (acc[C / 4][j][e] + acc[C - 1][j][e]);
     __syncthreads();
+    if (g.glu) {
+        for (int i = threadIdx.x; i < TILES * NT * 8 * 8; i += FR_WARPS * 32) {
+            const int r = i & 7, m = (i >> 3) % (NT * 8), t = (i >> 3) / (NT * 8);
+            const int n = (blockIdx.x * TILES + t) * 8 + r;
+            if (n >= ff || m >= g.M) continue;
+            double gate = 0., up = 0.;
+#pragma unroll
+            for (int w = 0; w < WK; ++w) { gate += part[t * WK + w][m][r]; up += part[t * WK + w][m][r + 8]; }
+            ((__nv_bfloat16*)g.C)[(size_t)m * g.ldc + n] = __float2bfloat16_rn(glu_f(g.glu - 1, (float)gate, (float)up, g.limit));
+        }
+        return;
+    }
     for (int i = threadIdx.x; i < TILES * NT * 8 * 16; i += FR_WARPS * 32) {
         const int r = i & 15, m = (i >> 4) % (NT * 8), t = (i >> 4) / (NT * 8);
         const int n = (blockIdx.x * TILES + t) * 16 + r;
@@ -426,7 +454,7 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
 
 template <int NT, int WK, int U, int OCC>
 void few_launch(const GemmArgs& g, cudaStream_t s) {
-    const int tiles = (g.N + 15) / 16, per = FR_WARPS / WK, blocks = (tiles + per - 1) / per;
+    const int tiles = g.glu ? (g.N / 2 + 7) / 8 : (g.N + 15) / 16, per = FR_WARPS / WK, blocks = (tiles + per - 1) / per;
     if (g.c_f32) launch_pdl(gemm_few_kernel<NT, WK, U, OCC, true>, blocks, FR_WARPS * 32, 0, s, g); else launch_pdl(gemm_few_kernel<NT, WK, U, OCC, false>, blocks, FR_WARPS * 32, 0, s, g);
 }
 // Which split: a warp wants many loads in flight while there are fewer row tiles than SMs (2560 x 6912: 14.4 us, 15.7 with half as many), blocks of two
@@ -459,10 +487,14 @@ static void read_env() {
     if (g_tc_min < 0) { const char* e = getenv("WF_SEQ_TC_MIN"); g_tc_min = e ? atoi(e) : 17; }
     if (g_force_simt < 0) { const char* e = getenv("WF_SEQ_GEMM_SIMT"); g_force_simt = (e && atoi(e)) ? 1 : 0; }
 }
-// the rows that launch_gemm gives to the tcgen05 form by itself
+// few rows on mma.sync, as launch_gemm chooses it by itself (9 to 16 rows go to the tcgen05 form where WF_SEQ_TC_MIN asks for it)
+static bool few_rows(int dt, const GemmArgs& g) {
+    return (g.M <= 8 || g.M < g_tc_min || !gemm_tc_usable(g)) && g.batch == 1 && !g.tile_group && !g.a_rows && g.M <= 16 && dt == WF_BF16 && !g.a_f32 && gemv_ok<__nv_bfloat16>(g);
+}
 bool gemm_glu_usable(int dt, const GemmArgs& g) {
     read_env();
-    return dt == WF_BF16 && g.algo == 0 && !g_force_simt && g.M >= g_tc_min && g.M > 8 && gemm_tc_usable(g);
+    if (dt != WF_BF16 || g.algo != 0 || g_force_simt || g.c_f32 || g.ep != EP_NONE || g.N % 2) return false;
+    return few_rows(dt, g) || (g.M >= g_tc_min && gemm_tc_usable(g));
 }
 
 int launch_gemm(int dt, const GemmArgs& g, cudaStream_t s) {
@@ -471,8 +503,7 @@ int launch_gemm(int dt, const GemmArgs& g, cudaStream_t s) {
     if (g.K <= 0 || !g.A || !g.B || !g.C) { set_error("gemm: bad arguments (M %d N %d K %d)", g.M, g.N, g.K); return WF_ERR_INVALID; }
     read_env();
     const bool few = g.batch == 1 && !g.tile_group && !g.a_rows && g.M <= 8;
-    // (9 to 16 rows go to the tcgen05 form where WF_SEQ_TC_MIN asks for it)
-    const bool few_mma = g.algo == 5 || (g.algo == 0 && !g_force_simt && (g.M <= 8 || g.M < g_tc_min || !gemm_tc_usable(g)));
+    const bool few_mma = g.algo == 5 || (g.algo == 0 && !g_force_simt && few_rows(dt, g));
     if (few_mma && g.batch == 1 && !g.tile_group && !g.a_rows && g.M <= 16 && dt == WF_BF16 && !g.a_f32 && gemv_ok<__nv_bfloat16>(g)) {
         if (g.M <= 8) few_dispatch<1>(g, s); else few_dispatch<2>(g, s);
         return launch_check(cudaGetLastError(), "gemm_few");

@@ -115,7 +115,8 @@ struct GemmArgs {
     const int32_t* a_rows = nullptr;
     int n_groups = 1;                        // weight matrices stacked behind B (grouped form)
     int ep = EP_NONE;
-    // gated activation where the product stores its results (tcgen05 form only, gemm_glu_usable): B's rows are [gate | up], N = 2 ff, C is T [M, ff] =
+    int b_const = 0;                         // B was complete before the stream's last kernel began (weights): it may be read ahead of that kernel's end
+    // gated activation where the product stores its results (tcgen05 and few-row forms, gemm_glu_usable): B's rows are [gate | up], N = 2 ff, C is T [M, ff] =
     // activation glu - 1 (launch_silu_mul's act) of the two floats
     int glu = 0; float limit = 0.f;
     int algo = 0;                            // 0 = choose; 1 plain FMA, 2 mma.sync, 3 tcgen05, 4 few-row streaming, 5 few rows on mma.sync (tests and measurements)
