@@ -145,3 +145,18 @@ def test_rmsnorm_quant_vs_oracle(M, K):
     # the quantiser applied to OUR normalised row must be bit-exact
     qo, so, ro = O.quantize_act_i8_rows(y.float().numpy())
     assert np.array_equal(q.cpu().numpy(), qo) and np.array_equal(s.cpu().numpy(), so) and np.array_equal(rs.cpu().numpy(), ro)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("at", ["first", "last", "middle"])
+def test_one_scale_for_many_rows(dtype, at):
+    """Enough rows that the maximum is taken over the tensor as one vector, whose length is no multiple of the grid's stride: the largest value at either end
+    and inside, bit-equal to the oracle."""
+    from wf_bitnet import ops
+    m, k = 4099, 2568
+    x = torch.randn(m, k, generator=torch.Generator().manual_seed(5)).to(dtype)
+    x.view(-1)[{"first": 0, "last": m * k - 1, "middle": 6543211}[at]] = -37.5
+    q, s, rs = ops.quantize_activations(x.cuda(), per_token=False)
+    qo, so = O.quantize_act_i8(x.float().numpy())
+    assert float(s.reshape(-1)[0]) == float(np.float32(so)) and np.array_equal(q.cpu().numpy(), np.asarray(qo).reshape(m, k))
+    assert np.array_equal(rs.cpu().numpy()[:m], np.asarray(qo).reshape(m, k).astype(np.int32).sum(1))

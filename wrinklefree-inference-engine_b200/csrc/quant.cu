@@ -121,8 +121,33 @@ __global__ void __launch_bounds__(QT) act_absmax_kernel(const T* __restrict__ x,
     amax = warp_max(amax);
     if ((threadIdx.x & 31) == 0 && amax > 0.f) atomicMax(amax_bits, __float_as_uint(amax));
 }
+// The same over rows that follow one another without a gap, as one vector: AU vectors of a thread in flight, whatever the row length leaves over (row by row
+// every row ends with a wait for its last loads).  16384 x 6912 bf16, 226 MB: 46 -> 38 us, 5.9 TB/s.
+constexpr int AU = 8;
+template <typename T>
+__global__ void __launch_bounds__(QT) act_absmax_flat_kernel(const T* __restrict__ x, size_t vectors, unsigned int* __restrict__ amax_bits) {
+    pdl_wait_prior();
+    pdl_launch_dependents();
+    const uint4* p = reinterpret_cast<const uint4*>(x);
+    const size_t step = (size_t)gridDim.x * QT;
+    float amax = 0.f;
+    for (size_t i = (size_t)blockIdx.x * QT + threadIdx.x; i < vectors; i += AU * step) {
+        uint4 raw[AU];
+#pragma unroll
+        for (int u = 0; u < AU; ++u) raw[u] = i + u * step < vectors ? __ldg(p + i + u * step) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int u = 0; u < AU; ++u) {
+            float v[8];
+            Vec<T>::unpack(raw[u], v);
+#pragma unroll
+            for (int k = 0; k < Vec<T>::N; ++k) amax = fmaxf(amax, fabsf(v[k]));
+        }
+    }
+    amax = warp_max(amax);
+    if ((threadIdx.x & 31) == 0 && amax > 0.f) atomicMax(amax_bits, __float_as_uint(amax));
+}
 // Per-tensor pass 2: grid = M, last rows first: pass 1 has left those in L2 (with quant_i8x4 79 -> 72 us at 16384 x 6912 bf16; the bytes
-// alone are 51).
+// alone are 51; a warp per row with three vectors in flight 91).
 template <typename T>
 __global__ void __launch_bounds__(QT) act_quant_tensor_kernel(const T* __restrict__ x, int K, int ldx,
                                                               const unsigned int* __restrict__ amax_bits,
@@ -209,8 +234,10 @@ static int launch_act_quant(const T* x, int M, int K, int ldx, int per_token, in
         launch_pdl(act_quant_rows_kernel<T>, M, QT, 0, s, x, K, ldx, q, scale_out, rowsum);
     } else {
         if (cuda_check(cudaMemsetAsync(workspace, 0, 4, s), "memset absmax")) return WF_ERR_CUDA;
-        int g = M < sm_count() * 4 ? M : sm_count() * 4;
-        launch_pdl(act_absmax_kernel<T>, g, QT, 0, s, x, M, K, ldx, (unsigned int*)workspace);
+        const int sms = sm_count();
+        const size_t vectors = (size_t)M * K / Vec<T>::N;
+        if (ldx == K && vectors >= (size_t)sms * 4 * QT * AU) launch_pdl(act_absmax_flat_kernel<T>, sms * 4, QT, 0, s, x, vectors, (unsigned int*)workspace);
+        else launch_pdl(act_absmax_kernel<T>, M < sms * 4 ? M : sms * 4, QT, 0, s, x, M, K, ldx, (unsigned int*)workspace);
         launch_pdl(act_quant_tensor_kernel<T>, M, QT, 0, s, x, K, ldx, (const unsigned int*)workspace, q, scale_out, rowsum);
     }
     return launch_check(cudaGetLastError(), "wf_act_quant_i8");

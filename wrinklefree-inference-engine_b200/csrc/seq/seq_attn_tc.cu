@@ -14,7 +14,7 @@
 // What bounds it: per pair of 128 x 128 tiles the tensor cores take 6 x 128^3 multiply-adds (about 3060 clk, 2040 without the split) and the eight
 // softmax warps about 5 instructions per score (1280 issue slots of each SM quarter's share), hence the packed float pairs and the scale folded
 // into the exponent's multiply-add.  Measured, 2048 tokens causal, 20 heads of 128: grouped-query attention 181 -> 67 us (mma.sync kernel before),
-// latent attention 895 -> 65 us (one CTA per token before; plus 24 us for the expansion).
+// latent attention 895 -> 49 us (one CTA per token before; plus 24 us for the expansion; 61 us with the heads' tiles handed out head after head).
 // Every wait is bounded: one that runs out records an error word that the host checks, and the CTA drains and leaves.
 // A value that is infinite or NaN meets the zero weights of the rows of its key tile that do not see it, too: a row whose sum of weights is finite and
 // whose output is not is taken again by its warp, over the keys that it sees (at_row).
@@ -116,7 +116,7 @@ __device__ __forceinline__ float at_ex2(float x) { float y; asm("ex2.approx.ftz.
 // registers would come out of the kernel's.
 __device__ __noinline__ void at_row(const Batch& b, const AtParams& p, int head, int tok) {
     const GqaDims& D = p.D;
-    const int kvh = blockIdx.y, sq = b.tok_seq[tok], pos = b.tok_pos[tok], row0 = p.key_row ? p.key_row[sq] : 0;
+    const int kvh = blockIdx.x % D.G, sq = b.tok_seq[tok], pos = b.tok_pos[tok], row0 = p.key_row ? p.key_row[sq] : 0;
     const int32_t* bt = p.key_row ? nullptr : p.block_table + (size_t)b.seq_slot[sq] * p.max_blocks;
     const int lane = threadIdx.x & 31;
     const __nv_bfloat16* q = p.qn + ((size_t)tok * D.H + head) * D.d;
@@ -175,11 +175,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     __shared__ uint32_t tmem_base_s;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const GqaDims& D = p.D;
-    const int kvh = blockIdx.y;
-    // ---- which sequence and which of its tokens: the last tiles of a sequence see the most keys and are handed out first
+    const int kvh = blockIdx.x % D.G;
+    // ---- which sequence and which of its tokens: the last tiles of a sequence see the most keys and are handed out first, those of all heads before the others
     int sq = -1, tok0 = 0, left = 0;
     {
-        int t = (int)(gridDim.x - 1 - blockIdx.x);
+        int t = (int)((gridDim.x - 1 - blockIdx.x) / D.G);
         for (int s = 0; s < b.nseq; ++s) {
             const int units = (b.seq_len[s] + 2 * p.tq - 1) / (2 * p.tq);
             if (t < units) { sq = s; tok0 = t * 2 * p.tq; left = b.seq_len[s] - tok0; break; }
@@ -502,7 +502,7 @@ int at_launch(const Batch& b, const AtParams& p, bool split, const CUtensorMap& 
     if (g_at_attr.need() && (cuda_check(cudaFuncSetAttribute(attn_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM), "attention shared memory") ||
                              cuda_check(cudaFuncSetAttribute(attn_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM), "attention shared memory"))) return WF_ERR_CUDA;
     // every sequence's tokens are cut into units of 2 tq; n / (2 tq) + nseq bounds their number (CTAs beyond the last unit return at once)
-    const dim3 grid(b.n / (2 * p.tq) + b.nseq, p.D.G);
+    const dim3 grid((b.n / (2 * p.tq) + b.nseq) * p.D.G);
     if (split) launch_pdl(attn_tc_kernel<true>, grid, AT_THREADS, AT_SMEM, s, tk, tv, b, p);
     else launch_pdl(attn_tc_kernel<false>, grid, AT_THREADS, AT_SMEM, s, tk, tv, b, p);
     return launch_check(cudaGetLastError(), "attn_tc");
