@@ -329,3 +329,27 @@ def test_streaming_gemm_accumulators_bit_exact(nk, m):
         got = acc.cpu()
         bad = (got != want).nonzero()
         assert bad.numel() == 0, (rep, bad[:8].tolist(), got[tuple(bad[0])].item(), want[tuple(bad[0])].item())
+
+
+@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("n,k", [(1, 128), (9, 2048), (2367, 2176), (4737, 640), (9475, 256), (129, 28672), (40, 24576)])
+def test_packed_weights_of_one_and_two_tokens(m, n, k):
+    """One, two and four rows per warp, the last warps' rows missing, fewer pieces than lanes and several rounds of them, sizes on both sides of what the
+    shared memory takes: accumulators equal to the oracle's, every other kind of output to the mma.sync kernel's."""
+    from wf_bitnet import ops
+    rng = np.random.default_rng(n + k + m)
+    code = rng.integers(0, 3, size=(n, k // 128, 4, 32)).astype(np.uint8)
+    packed = (code[:, :, 0] << 6 | code[:, :, 1] << 4 | code[:, :, 2] << 2 | code[:, :, 3]).reshape(n, k // 4)
+    q = rng.integers(-128, 128, size=(m, k)).astype(np.int8)
+    pi, qd = cu(packed), cu(q)
+    want = O.gemm_i32_fast(packed, q, 0)
+    assert np.array_equal(ops.ternary_linear(pi, n, k, qd, layout="i2s", mode="i32_plus1").cpu().numpy(), want)
+    rs, sc, ws = qd.int().sum(1).int(), torch.rand(m, device="cuda") + 0.5, torch.tensor([0.3, 0.2], device="cuda")
+    res = torch.randn(m, n, device="cuda").to(torch.bfloat16)
+    lin = dict(mode="linear", rowsum=rs, act_scale=sc, layout="i2s")
+    for f in (dict(mode="i32", rowsum=rs, layout="i2s"), dict(lin, w_scale=ws[:1], out_dtype=torch.bfloat16), dict(lin, w_scale=ws[:1], residual=res, out_dtype=torch.bfloat16),
+              dict(lin, w_scale=ws, seg_end=[(n + 1) // 2, n], out_dtype=torch.float32)):
+        a, b = (ops.ternary_linear(pi, n, k, qd, algo=x, **f) for x in (0, 2))
+        assert torch.equal(a, b), list(f)
+    y = ops.bitnet_gemv(pi, qd[0], 0.0123) if m == 1 else ops.bitnet_gemm(pi, qd, 0.0123)
+    assert np.array_equal(y.cpu().numpy().reshape(m, n), want.astype(np.float32) * np.float32(0.0123))

@@ -102,6 +102,8 @@ static int ternary_linear(const wf_linear_args* a, const float* w_scales_host, v
     int algo = a->algo;
     if (algo == 0) {
         if (a->M <= 8 && a->w_layout == WF_W_TILE && a->workspace && gemv_stream_fits(a->M, a->K)) algo = 1;   // else (70B down at M = 8: 8 x 28672 int8 rows) the tiled GEMM
+        // (one or two tokens on packed weights, us mma.sync / dp4a: 2560 x 2560 4.9 / 2.4, 8192 x 8192 10.5 / 4.9; two tokens 5.1 / 2.8, 10.3 / 6.9)
+        else if (gemv_packed_usable(a)) return launch_gemv_packed(a, ep, s);
         else algo = tc_is_faster(a->M, a->N, a->K) ? 3 : 2;
     }
     switch (algo) {

@@ -96,6 +96,8 @@ int fill_epi(const wf_linear_args* a, EpiParams* p, const float* w_scales_host =
 int launch_gemm_mma(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s);
 int launch_gemv_stream(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s, bool pdl, bool wait_first = false);   // wait_first: the weights, too, may be the work of the kernel before
 bool gemv_stream_fits(int M, int K);
+bool gemv_packed_usable(const wf_linear_args* a);
+int launch_gemv_packed(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s);
 int launch_gemm_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s);
 size_t gemm_mma_workspace_bytes(int M, int N, int K);
 
