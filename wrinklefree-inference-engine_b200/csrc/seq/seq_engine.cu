@@ -1589,8 +1589,9 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     const size_t with_table = e->meta_ints + (size_t)c.slots * max_blocks;
     TRY(dalloc_n(e, &e->d_meta, with_table));
     e->d_block_table = e->d_meta + e->meta_ints;
-    if (cuda_check(cudaMallocHost((void**)&e->h_meta, with_table * 4), "pinned metadata")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
-    if (cuda_check(cudaMallocHost((void**)&e->h_out, OUT_CHUNKS * OUT_CHUNK + 64), "pinned results")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
+    const size_t meta_bytes = (with_table * 4 + 63) / 64 * 64;         // one pinned allocation (2 to 3 ms each): arrays and table, pieces of results, error word
+    if (cuda_check(cudaMallocHost((void**)&e->h_meta, meta_bytes + OUT_CHUNKS * OUT_CHUNK + 64), "pinned step memory")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
+    e->h_out = (unsigned char*)e->h_meta + meta_bytes;
     e->h_err = (int*)(e->h_out + OUT_CHUNKS * OUT_CHUNK);
     for (auto& ev : e->out_ev)
         if (cuda_check(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
@@ -1670,7 +1671,6 @@ extern "C" void wf_seq_destroy(wf_seq_engine* e) {
     if (e->d_uniform) cudaFree(e->d_uniform);
     if (e->d_next) cudaFree(e->d_next);
     if (e->h_meta) cudaFreeHost(e->h_meta);
-    if (e->h_out) cudaFreeHost(e->h_out);
     for (auto& ev : e->out_ev) if (ev) cudaEventDestroy(ev);
     if (e->stream) cudaStreamDestroy(e->stream);
     delete e;
