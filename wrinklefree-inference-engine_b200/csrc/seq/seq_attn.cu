@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(GP_MAXW * 32) gqa_prep_kernel(Batch b, GqaDims
 
 // The same for head sizes that are multiples of 4 up to 128 (no norm over the whole projection; pairs side by side, or half the rotated entries apart with
 // that half a multiple of 4): a head vector lies in the lanes of a warp four entries each, a warp's GQ vectors are requested before the cosines are formed,
-// and a pair's other entry comes from its lane.  2048 tokens, 20 + 5 + 5 heads of 128 with a gate per element (88 MB): 62 us one entry at a time, 24 so.
+// and a pair's other entry comes from its lane.  2048 tokens, 20 + 5 + 5 heads of 128 with a gate per element (88 MB): 62 us one entry at a time, 33 so.
 constexpr int GQ = 4;
 template <typename T>
 __global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D, const float* __restrict__ proj, int ld, int k_off, int v_off, int g_off, const T* __restrict__ qb,

@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(AM_THREADS, 3) gqa_attn_mma_kernel(Batch b, Gq
 }
 
 // one warp per (token, head): merge the key splits' partial results (maxima in units of log 2), apply the gate.  A lane a split for the maxima and sums, then the
-// splits' values side by side: two memory latencies, where one split after the other took one each (a merge of a decode step 4.3 -> 2.4 us).
+// splits' values side by side: two memory latencies, where one split after the other took one each (a merge of a decode step 4.2 -> 3.2 us).
 __global__ void gqa_attn_merge_kernel(GqaDims D, int rows, int splits, const float* __restrict__ part, const float* __restrict__ gate, __nv_bfloat16* __restrict__ out) {
     pdl_enter();
     const int dv = D.dv, gate_elem = D.gate_elem, stride = dv + 2;

@@ -115,7 +115,7 @@ __global__ void ssd_post_kernel(int H, int dv, int groups, const float* __restri
 }
 
 // The same with a group's values in registers between the two passes, four consecutive elements per load: gw a multiple of 4 up to 2048, dv one of 4.
-// 2048 tokens x 2560 channels in 5 groups (73 MB): 35 us with every input read twice, 14 so.
+// 2048 tokens x 2560 channels in 5 groups (73 MB): 35 us with every input read twice, 16 so.
 template <typename T>
 __global__ void __launch_bounds__(512) ssd_post_vec_kernel(int H, int dv, int groups, const float* __restrict__ o, const float* __restrict__ x, int ldx, const float* __restrict__ z, int ldz,
                                                            const T* __restrict__ Dskip, const T* __restrict__ w, float eps, T* __restrict__ y) {

@@ -1589,7 +1589,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     const size_t with_table = e->meta_ints + (size_t)c.slots * max_blocks;
     TRY(dalloc_n(e, &e->d_meta, with_table));
     e->d_block_table = e->d_meta + e->meta_ints;
-    const size_t meta_bytes = (with_table * 4 + 63) / 64 * 64;         // one pinned allocation (2 to 3 ms each): arrays and table, pieces of results, error word
+    const size_t meta_bytes = (with_table * 4 + 63) / 64 * 64;         // one pinned allocation (three made a state 2 ms slower to create): arrays and table, pieces of results, error word
     if (cuda_check(cudaMallocHost((void**)&e->h_meta, meta_bytes + OUT_CHUNKS * OUT_CHUNK + 64), "pinned step memory")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
     e->h_out = (unsigned char*)e->h_meta + meta_bytes;
     e->h_err = (int*)(e->h_out + OUT_CHUNKS * OUT_CHUNK);

@@ -61,7 +61,7 @@ __global__ void latent_q_prep_kernel(Batch b, LatentDims L, const float* __restr
 }
 
 // The same, four consecutive elements per load: d, r and the rotated entries multiples of 4 (of 8 where pairs lie half the rotated entries apart).
-// 2048 tokens, 20 heads of 96 + 32 (31 MB): 19 us one element at a time, 10 so.
+// 2048 tokens, 20 heads of 96 + 32 (31 MB): 19 us one element at a time, 9 so.
 template <typename T>
 __global__ void __launch_bounds__(256) latent_q_prep_vec_kernel(Batch b, LatentDims L, const float* __restrict__ q, int ldq, T* __restrict__ qn, float* __restrict__ qr) {
     pdl_enter();

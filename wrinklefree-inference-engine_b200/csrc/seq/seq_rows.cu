@@ -58,7 +58,7 @@ __global__ void embed_pos_kernel(const T* __restrict__ table, const int32_t* __r
                                  float* __restrict__ x, T* __restrict__ x_t) {
     pdl_enter();
     // a thread per pair of channels, which share an angle: the double precision sine and cosine are what this kernel costs (8 tokens x 1024: 5.9 us with four
-    // angles a thread one after the other, 3.6 so)
+    // angles a thread one after the other, 2.5 so)
     const int i = blockIdx.x, c = 2 * (blockIdx.y * blockDim.x + threadIdx.x);
     if (c >= W) return;
     const T* row = table + (size_t)tokens[i] * W;
@@ -186,7 +186,7 @@ __global__ void group_rmsnorm_kernel(const float* __restrict__ x, int ldx, const
 }
 
 // The same with four consecutive elements per load and every input of a row requested before the first is used; a thread owns NV groups of four,
-// blockDim.x * NV * 4 >= gw.  What bounds it is the bytes: 2048 rows of 2560 from two inputs and a residual, 94 MB: 30 us one element at a time, 17 so.
+// blockDim.x * NV * 4 >= gw.  What bounds it is the bytes: 2048 rows of 2560 from two inputs and a residual, 94 MB: 30 us one element at a time, 15 so.
 template <typename T, int NV>
 __global__ void __launch_bounds__(1024) group_rmsnorm_vec_kernel(const float* x, int ldx, const T* __restrict__ w, int gw, float eps, const float* res, float* y, int ldy,
                                                                  T* __restrict__ y_t, int ldt, const int32_t* __restrict__ rows, const float* x2, float a, float b,
@@ -718,8 +718,8 @@ __global__ void causal_taps_kernel(Batch b, const float* __restrict__ in, int ld
 }
 
 // Many tokens: a thread takes four channels of TR tokens one after another, so an input is read once instead of once per tap, all of the run's inputs are
-// requested before the first is used, and the weights are read once a run.  1801 tokens x 5120 channels, four taps (74 MB): 72 us a channel and token per
-// thread, 17 so.  Sums in the same order as above.
+// requested before the first is used, and the weights are read once a run.  1801 tokens x 5120 channels, four taps (74 MB): 63 to 72 us a channel and
+// token per thread, 21 so.  Sums in the same order as above.
 constexpr int TR = 8;
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128) causal_taps_run_kernel(Batch b, const float* __restrict__ in, int ld_in, const T* __restrict__ w, int C, const float* __restrict__ state,
