@@ -15,6 +15,7 @@
 // tokens 43 / 24; 14336 x 4096, 48 tokens 17.4 / 13.1.
 // Every wait is bounded: one that runs out sets pair_error, and the CTAs wait for their own copies and products and leave.
 #include "gemm_tc_common.cuh"
+#include "gemm_tc_pair_walk.h"
 #include "kernels.cuh"
 #include <string.h>
 
@@ -26,8 +27,6 @@ constexpr int TP_ROWS = 128;                        // weight rows per CTA
 constexpr int TP_MAX_TOK = 256;                     // most tokens per tile (UMMA N)
 constexpr int TP_BK = 128;                          // k per stage
 constexpr int TP_AS_MAX = 16;                       // most activation loads in flight
-constexpr int TP_WKB = 4;                           // k-blocks per weight load
-constexpr int TP_WS = 3;                            // weight stages
 constexpr int TP_W_BYTES = TP_ROWS * TP_WKB * 32;
 constexpr int TP_A_COLS = TP_BK / 4;
 constexpr int TP_EPW = 8;
@@ -185,7 +184,7 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
     if (tid == 0) {
         for (int s = 0; s < AS; ++s) { mbar_init(&act_full[s], 1); mbar_init(&act_empty[s], 1); }
         for (int s = 0; s < TP_TS; ++s) { mbar_init(&a_full[s], 8); mbar_init(&a_empty[s], 1); }
-        for (int s = 0; s < TP_WS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 4 * TP_WKB); }
+        for (int s = 0; s < TP_WS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 4 * NU); }
         for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * TP_EPW); }
         mbar_init(&drained, 1);
         fence_mbar_init();
@@ -325,13 +324,17 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
         const uint32_t rx = p.i2s ? (uint32_t)(row & 7) : (uint32_t)((row & 7) >> 1);
         const bool odd = (row >> 3) & 1;
         const bool i2s = p.i2s != 0;
-        int kb = grp, l0 = 0;                         // k-block in its tile, first weight load of the tile (counted over all tiles)
-        while (kb >= KB) { kb -= KB; l0 += wloads; }
+        PairWeightWalk walk(grp, NU, KB);
         bool ok = true;
-        uint32_t pk[8], empty = 0, count = 0;          // an item's packed codes, and the hand-back of their buffer
+        uint32_t pk[8];                               // an item's packed codes
+        auto landed = [&](int load) { return __all_sync(0xffffffffu, wait_bounded(smem_u32(&w_full[load % TP_WS]), (uint32_t)((load / TP_WS) & 1))) != 0; };
+        auto hand_back = [&](int load) {              // every lane has its codes
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&w_empty[load % TP_WS]);
+        };
         auto fetch = [&]() -> bool {
-            const int load = l0 + kb / TP_WKB, ws = load % TP_WS, j = kb % TP_WKB;
-            if (!__all_sync(0xffffffffu, wait_bounded(smem_u32(&w_full[ws]), (uint32_t)((load / TP_WS) & 1)))) return false;
+            if (!walk.next(landed, hand_back)) return false;
+            const int ws = walk.load % TP_WS, j = walk.part;
             const uint32_t src = wring + ws * TP_W_BYTES + rbase;
             if (i2s) {
 #pragma unroll
@@ -347,10 +350,6 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
                     pk[4 + c] = odd ? e : d;
                 }
             }
-            empty = smem_u32(&w_empty[ws]);
-            count = kb == KB - 1 ? (uint32_t)(1 + TP_WKB * wloads - KB) : 1u;   // the item that ends a tile's last, partial load stands for the missing ones
-            kb += NU;
-            while (kb >= KB) { kb -= KB; l0 += wloads; }
             return true;
         };
         if (grp < n_items) ok = fetch();
@@ -360,8 +359,6 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
             for (int g = 0; g < 4; ++g)
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[8 * g + i] = (pk[i] >> (6 - 2 * g)) & 0x03030303u;   // k = 32g + 4i .. +3
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty), "r"(count) : "memory");
             if (it + NU < n_items && !fetch()) { ok = false; break; }       // the next item's codes arrive while this one waits for its TMEM stage
             const int ts = it % TP_TS;
             if (it >= TP_TS && !__all_sync(0xffffffffu, wait_bounded(smem_u32(&a_empty[ts]), (uint32_t)((it / TP_TS - 1) & 1)))) { ok = false; break; }   // its last MMAs are done
