@@ -128,6 +128,10 @@ size_t wf_linear_workspace_bytes(int M, int N, int K);
 int wf_ternary_linear(const wf_linear_args* args, void* stream);
 /* The same with the weight scales by value: w_scales points at args->nseg (1..4) host floats and args->w_scale is not read. */
 int wf_ternary_linear_scales(const wf_linear_args* args, const float* w_scales, void* stream);
+/* A ternary product on CTA pairs bounds its waits (one second).  One that runs out leaves its output incomplete and a nonzero code in the current device's word,
+ * whose host address this is (null where there is no device or no such word).  The next ternary product on the device, and the engine's waits, clear the word
+ * and return WF_ERR_CUDA; a caller that replays a graph of such products can look at the word itself once the replay has ended. */
+int* wf_wait_word(void);
 /* What wf_bitnet_gemv / wf_bitnet_gemm (and wf_ternary_linear with algo 0 beyond 8 rows) can use of a workspace for this shape: at most
  * wf_linear_workspace_bytes, 0 where the kernel they choose needs none. */
 size_t wf_bitnet_gemm_workspace_bytes(int M, int N, int K);

@@ -177,3 +177,62 @@ def test_tc_pairs(nkm):
             a, b = (ops.ternary_linear(wt, n, k, q, layout=layout, algo=x, **f) for x in (3, 2))
             assert torch.equal(a, b), (layout, list(f))
     assert torch.equal(ops.bitnet_gemm(pi, q, 0.0123).cpu()[rows], torch.from_numpy(want.astype(np.float32) * np.float32(0.0123)))
+
+
+def test_a_wait_that_ran_out_is_reported_once():
+    """The word that a product leaves behind when one of its waits ran out, set from the host: the next call on the device raises, whichever way it comes,
+    and the one after that is an ordinary call again."""
+    from sgl_kernel.quantization import bitnet_gemm, bitnet_gemv
+    from test_gpu_engine import small_cfg
+    from wf_bitnet import ops
+    from wf_bitnet._lib import WfError, lib
+    from wf_bitnet.engine import Engine
+    from wf_bitnet.synth import make_weights
+    word = lib().wf_wait_word()
+    assert word and word[0] == 0
+    n, k, m = 512, 640, 48
+    rng = np.random.default_rng(4)
+    code = rng.integers(0, 3, size=(n, k // 128, 4, 32)).astype(np.uint8)
+    pi = cu((code[:, :, 0] << 6 | code[:, :, 1] << 4 | code[:, :, 2] << 2 | code[:, :, 3]).reshape(n, k // 4))
+    q = torch.from_numpy(rng.integers(-128, 128, size=(m, k)).astype(np.int8)).cuda()
+    x = torch.randn(m, k, device="cuda").to(torch.bfloat16)
+    g, f = torch.ones(n, device="cuda", dtype=torch.bfloat16), cu(np.full((k, n // 4), 0x55, np.uint8))
+    cfg = small_cfg()
+    engine = Engine(cfg)
+    engine.load_weights(make_weights(cfg, seed=1234))
+    calls = [lambda: bitnet_gemm(pi, q, 0.5), lambda: bitnet_gemv(pi, q[0], 0.5), lambda: ops.ternary_linear(pi, n, k, q, layout="i2s", mode="i32_plus1"),
+             lambda: torch.ops.sgl_kernel.bitnet_mlp_forward_cpu(x, pi, pi, f, 0.1, 0.1, 0.1, g, 1e-5), lambda: engine.decode([5])]
+    for i, call in enumerate(calls):
+        call()
+        torch.cuda.synchronize()
+        word[0] = 4
+        with pytest.raises(WfError, match="ran out"):
+            call()
+        assert word[0] == 0, i
+        call()
+    torch.cuda.synchronize()
+    assert torch.equal(calls[0]().cpu(), torch.from_numpy(O.gemm_i32_fast(pi.cpu().numpy(), q.cpu().numpy(), 0).astype(np.float32) * np.float32(0.5)))
+    engine.close()
+
+
+def test_the_first_product_of_a_process_may_be_captured():
+    """A process whose first product, one on CTA pairs, lies in a graph capture that allows nothing unsafe to any thread."""
+    import subprocess
+    import sys
+    code = """
+import torch, sgl_kernel
+from sgl_kernel.quantization import bitnet_gemm
+w = torch.randint(0, 256, (14336, 1024), device="cuda", dtype=torch.uint8) & 0xAA
+x = torch.randint(-127, 128, (48, 4096), device="cuda", dtype=torch.int8)
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g, capture_error_mode="global"):
+    y = bitnet_gemm(w, x, 0.5)
+g.replay()
+torch.cuda.synchronize()
+assert torch.equal(y, bitnet_gemm(w, x, 0.5)) and float(y.abs().sum()) > 0
+print("equal")
+"""
+    from conftest import PKG
+    r = subprocess.run([sys.executable, "-c", code], cwd=str(PKG), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "equal", r.stderr[-2000:]

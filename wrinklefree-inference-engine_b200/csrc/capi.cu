@@ -98,6 +98,7 @@ static int ternary_linear(const wf_linear_args* a, const float* w_scales_host, v
     int rc = fill_epi(a, &ep, w_scales_host);
     if (rc) return rc;
     if (a->M == 0) return WF_OK;
+    if ((rc = check_wait_word("wf_ternary_linear"))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     int algo = a->algo;
     if (algo == 0) {
@@ -114,6 +115,8 @@ static int ternary_linear(const wf_linear_args* a, const float* w_scales_host, v
     set_error("wf_ternary_linear: unknown algo %d", a->algo);
     return WF_ERR_INVALID;
 }
+
+extern "C" int* wf_wait_word(void) { return tc_wait_word(); }
 
 extern "C" int wf_ternary_linear(const wf_linear_args* a, void* stream) { return ternary_linear(a, nullptr, stream); }
 

@@ -816,7 +816,7 @@ static int check_device_error(wf_engine* e) {
                   "the engine state is undefined, destroy it", code, code >= 1000 ? "TP exchange flag" : "grid barrier");
         return WF_ERR_CUDA;
     }
-    return WF_OK;
+    return check_wait_word("engine");
 }
 extern "C" int wf_engine_sync(wf_engine* e) { return e ? check_device_error(e) : WF_ERR_INVALID; }
 

@@ -616,7 +616,8 @@ int launch_gemm_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s)
     int ksplit = 1;
     while (ksplit < 8 && tiles * ksplit * 2 <= sms && a->K / WF_QK >= ksplit * 2 * 4) ksplit *= 2;
     const bool relu2 = ep.out_mode == WF_OUT_LINEAR && (ep.epi_flags & WF_EPI_RELU2_MUL);
-    if (gemm_tc_pair_time(a->M, a->N, a->K) < tile_time(a->M, a->K / WF_QK, tiles, ksplit, sms, relu2)) return launch_gemm_tc_pair(a, ep, s);
+    // (where the host memory that pairs report to cannot be had, the forms of this file, whose waits have no limit)
+    if (gemm_tc_pair_time(a->M, a->N, a->K) < tile_time(a->M, a->K / WF_QK, tiles, ksplit, sms, relu2) && tc_wait_word()) return launch_gemm_tc_pair(a, ep, s);
     if (ksplit > 1) return launch_tc_split(a, ep, ksplit, s);
     if (g_tc_nu == 1) return launch_tc<1>(a, ep, s);
     return g_tc_nu == 2 ? launch_tc<2>(a, ep, s) : launch_tc<3>(a, ep, s);

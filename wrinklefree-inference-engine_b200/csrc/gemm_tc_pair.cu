@@ -13,11 +13,14 @@
 // Roles of a CTA: 8 epilogue warps, 4 * NU unpack warps, one warp loading activations, one loading weights, one issuing MMAs (first CTA of the pair).
 // Measured without / with it (us): 6912 x 2560, 1987 tokens 44.8 / 34.8; 2560 x 6912, 16384 tokens 246 / 177 (3.3 PTOP/s); gate | up of 13824 x 2560, 512
 // tokens 43 / 24; 14336 x 4096, 48 tokens 17.4 / 13.1.
-// Every wait is bounded: one that runs out sets pair_error, and the CTAs wait for their own copies and products and leave.
+// Every wait is bounded: one that runs out leaves a code in the device's wait word (tc_wait_word), and the CTAs wait for their own copies and products and
+// leave.  The word is host memory, so that the next ternary call on the device and the engine's waits see it without a copy: they fail with WF_ERR_CUDA once.
 #include "gemm_tc_common.cuh"
 #include "gemm_tc_pair_walk.h"
 #include "kernels.cuh"
 #include <string.h>
+#include <atomic>
+#include <mutex>
 
 namespace wf {
 
@@ -42,11 +45,14 @@ struct TpParams {
     int tn, n_tiles, tiles;
     int i2s;
     int akb, as;         // k-blocks per activation load, loads in flight
+    int* err;            // the wait word
     EpiParams ep;
 };
 
-__device__ int pair_error;
-
+__device__ __forceinline__ void gave_up(const TpParams& p, int role) {
+    *(volatile int*)p.err = role;
+    __threadfence_system();
+}
 __device__ __forceinline__ uint32_t of_first_cta(uint32_t saddr) {        // the pair's first CTA's copy of a shared-memory address
     uint32_t ra;
     asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(ra) : "r"(saddr));
@@ -65,7 +71,7 @@ __device__ __noinline__ bool wait_long(uint32_t bar, uint32_t parity) {
         if (try_wait_cluster(bar, parity)) return true;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
     } while (t1 - t0 < TP_LIMIT_NS);
-    return false;
+    return try_wait_cluster(bar, parity);              // the time may have passed between the look and the clock, with the SM in other hands
 }
 // (one look inline and the rest out of line: the issuing thread's loop paces a stage when it is long)
 __device__ __forceinline__ bool wait_bounded(uint32_t bar, uint32_t parity) { return try_wait_cluster(bar, parity) || wait_long(bar, parity); }
@@ -223,7 +229,7 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
             // the last stages' hand-backs come from the first CTA: none may be under way when this CTA leaves
             for (int j = it > AS ? it - AS : 0; ok && j < it; ++j) ok = wait_bounded(smem_u32(&act_empty[j % AS]), (uint32_t)((j / AS) & 1));
             if (!ok) {                                                     // leaves early, but not before the pair's copies have landed
-                atomicExch(&pair_error, 1);
+                gave_up(p, 1);
                 for (int j = it > AS ? it - AS : 0; rank == 0 && j < it; ++j) wait_bounded(smem_u32(&act_full[j % AS]), (uint32_t)((j / AS) & 1));
             }
         }
@@ -250,7 +256,7 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
                 }
             }
             if (!ok) {
-                atomicExch(&pair_error, 2);
+                gave_up(p, 2);
                 for (int j = c > TP_WS ? c - TP_WS : 0; j < c; ++j) wait_bounded(smem_u32(&w_full[j % TP_WS]), (uint32_t)((j / TP_WS) & 1));
             }
         }
@@ -306,7 +312,7 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
                 return true;
             };
             if (!stream()) {                                               // not while a product still reads shared memory
-                atomicExch(&pair_error, 3);
+                gave_up(p, 3);
                 commit_pair(smem_u32(&drained));
                 wait_bounded(smem_u32(&drained), 0);
             }
@@ -369,7 +375,7 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
             __syncwarp();
             if (lane == 0) arrive_remote(afull0 + ts * 8);
         }
-        if (!ok && lane == 0) atomicExch(&pair_error, 4);
+        if (!ok && lane == 0) gave_up(p, 4);
     } else {
         // ------------------------------------------------------------ epilogue warps: TMEM -> registers -> global
         const int q = warp & 3, part = warp >> 2;                          // lane quarter; its two warps take alternate 32-token chunks
@@ -413,7 +419,7 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
             __syncwarp();
             if (lane == 0) arrive_remote(tempty0 + buf * 8);
         }
-        if (!ok && lane == 0) atomicExch(&pair_error, 5);
+        if (!ok && lane == 0) gave_up(p, 5);
     }
     tc_fence_before();
     __syncthreads();
@@ -441,7 +447,46 @@ int tokens_per_tile(int M, int N, int KB, int pairs) {
 
 DevOnce g_attr;
 
+// The wait words: a page of the library's own memory that every device may write.  Nothing is allocated; locking the page is also allowed to a call that is
+// being captured.
+constexpr int WAIT_WORDS = 64;
+alignas(4096) int g_wait_page[4096 / sizeof(int)];
+std::atomic<int> g_wait_state{0};                      // 1: usable; -1: the page cannot be locked
+
+bool wait_page_usable() {
+    if (const int st = g_wait_state.load(std::memory_order_acquire)) return st > 0;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    if (const int st = g_wait_state.load(std::memory_order_acquire)) return st > 0;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    const bool swapped = cudaThreadExchangeStreamCaptureMode(&mode) == cudaSuccess;
+    void* dev = nullptr;
+    const bool ok = cudaHostRegister(g_wait_page, sizeof g_wait_page, cudaHostRegisterPortable | cudaHostRegisterMapped) == cudaSuccess &&
+                    cudaHostGetDevicePointer(&dev, g_wait_page, 0) == cudaSuccess && dev == (void*)g_wait_page;
+    if (!ok) cudaGetLastError();
+    if (swapped) cudaThreadExchangeStreamCaptureMode(&mode);
+    g_wait_state.store(ok ? 1 : -1, std::memory_order_release);
+    return ok;
+}
+
 }  // namespace
+
+int* tc_wait_word() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= WAIT_WORDS || !wait_page_usable()) return nullptr;
+    return g_wait_page + dev;
+}
+
+int check_wait_word(const char* who) {
+    if (g_wait_state.load(std::memory_order_acquire) <= 0) return WF_OK;
+    int* word = tc_wait_word();
+    if (!word || !*(volatile int*)word) return WF_OK;
+    if (const int role = __atomic_exchange_n(word, 0, __ATOMIC_ACQ_REL)) {
+        set_error("%s: a bounded wait of an earlier ternary product on this device ran out (%d); that product's output is not complete", who, role);
+        return WF_ERR_CUDA;
+    }
+    return WF_OK;
+}
 
 double gemm_tc_pair_time(int M, int N, int K) {
     const int pairs = sm_count() / 2;
@@ -465,6 +510,8 @@ int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream
     p.akb = p.tn <= 128 ? 4 : 2;
     p.as = TP_ACT_RING / (p.akb * p.tn / 2 * TP_BK);
     if (p.as > TP_AS_MAX) p.as = TP_AS_MAX;
+    p.err = tc_wait_word();
+    if (!p.err) { set_error("gemm_tc_pair: no wait word"); return WF_ERR_CUDA; }
     p.ep = ep;
     CUtensorMap tq, tw;
     const cuuint32_t one[4] = {1, 1, 1, 1};

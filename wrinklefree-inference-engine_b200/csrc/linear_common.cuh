@@ -100,5 +100,9 @@ bool gemv_packed_usable(const wf_linear_args* a);
 int launch_gemv_packed(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s);
 int launch_gemm_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s);
 size_t gemm_mma_workspace_bytes(int M, int N, int K);
+// what a bounded wait of the CTA-pair product that ran out leaves behind (gemm_tc_pair.cu): the current device's word in host memory, or null where there is
+// none; and the check of it, WF_ERR_CUDA once for each time
+int* tc_wait_word();
+int check_wait_word(const char* who);
 
 }  // namespace wf
