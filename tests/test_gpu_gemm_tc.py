@@ -236,3 +236,16 @@ print("equal")
     from conftest import PKG
     r = subprocess.run([sys.executable, "-c", code], cwd=str(PKG), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "equal", r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("nkm", [(256, 128, 40), (6912, 2560, 300)])
+def test_tc_pairs_subtract_whole_sums(nkm):
+    """Sums of activations beyond 2^24, which K above 131072 or a caller's own sums bring: subtracted as the whole numbers that they are."""
+    from wf_bitnet import ops
+    n, k, m = nkm
+    rng = np.random.default_rng(k)
+    q = torch.from_numpy(rng.integers(-128, 128, size=(m, k)).astype(np.int8)).cuda()
+    w = cu(rng.integers(0, 256, size=(n, k // 4)).astype(np.uint8) & 0xAA)
+    rs = torch.from_numpy(rng.integers(-(1 << 30), 1 << 30, size=m).astype(np.int32) | 1).cuda()
+    a, b = (ops.ternary_linear(w, n, k, q, layout="i2s", mode="i32", rowsum=rs, algo=x) for x in (3, 2))
+    assert torch.equal(a, b)

@@ -90,7 +90,7 @@ __device__ __forceinline__ void commit_pair(uint32_t bar) {
 }
 
 // The linear epilogue of 32 tokens (m0 ..) of one weight row per lane: the rounding sequence of linear_value (linear_common.cuh).
-// tk[j]: {fl(w_s * Sigma a) where one scale serves the matrix, else (float) Sigma a; activation scale} of token m0 + j.
+// tk[j]: {fl(w_s * Sigma a) where one scale serves the matrix, the bits of Sigma a for whole-number results, else (float) Sigma a; activation scale} of token m0 + j.
 struct PairEp {
     int mode;
     bool relu2, resid, obf16, fold;
@@ -150,7 +150,7 @@ __device__ __forceinline__ void pair_store(const EpiParams& ep, const PairEp& e,
     __nv_bfloat16* const ob = reinterpret_cast<__nv_bfloat16*>(ep.out);
     if (e.mode == WF_OUT_COMPAT_F32) each(of, [&](int j) { return __fmul_rn((float)(int)v[j], ep.host_scale); });
     else if (e.mode == WF_OUT_I32_PLUS1) each(reinterpret_cast<int32_t*>(ep.out), [&](int j) { return (int32_t)v[j]; });
-    else if (e.mode == WF_OUT_I32) each(reinterpret_cast<int32_t*>(ep.out), [&](int j) { return (int32_t)v[j] - (int32_t)tk[j].x; });
+    else if (e.mode == WF_OUT_I32) each(reinterpret_cast<int32_t*>(ep.out), [&](int j) { return (int32_t)v[j] - __float_as_int(tk[j].x); });
     else if (e.resid) {
         const __nv_bfloat16* rp = ep.residual + (size_t)m0 * ldo + n;
         auto added = [&](int j) { return __bfloat162float(rp[(size_t)j * ldo]) + bf16_round(plain(j)); };
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
                     const int m = min(mt * p.tn + c * 32 + lane, p.M - 1);
                     const int rs = p.ep.rowsum ? p.ep.rowsum[m] : 0;
                     const float sa = e.mode == WF_OUT_LINEAR ? p.ep.act_scale[p.ep.act_scale_per_token ? m : 0] : 1.f;
-                    tok[i * 32 + lane] = make_float2(e.fold ? __fmul_rn(ws_all, (float)rs) : (float)rs, sa);      // |Sigma a| <= 127 K < 2^24: exact
+                    tok[i * 32 + lane] = make_float2(e.mode == WF_OUT_I32 ? __int_as_float(rs) : e.fold ? __fmul_rn(ws_all, (float)rs) : (float)rs, sa);
                 }
                 __syncwarp();
             }
