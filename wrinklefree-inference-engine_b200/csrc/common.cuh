@@ -115,7 +115,8 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* gsrc, uint32_t byte
 __device__ __forceinline__ void pdl_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // A launch that may overlap the end of the kernel before it in the stream.  For kernels that wait (pdl_wait_prior) before their first read of memory that the
-// stream's earlier work may have written and before their first write.
+// stream's earlier work may have written and before their first write.  Such memory changes while they are resident: it is read by ordinary loads, never by
+// non-coherent ones (__ldg, const __restrict__ parameters), which are for weights alone.
 template <typename... P, typename... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
     cudaLaunchConfig_t cfg = {};

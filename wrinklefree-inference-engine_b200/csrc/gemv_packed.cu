@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(GP_WARPS * 32) ternary_gemv_packed_kernel(cons
     // byte j of a 32-byte block holds the codes of k = j, j + 32, j + 64, j + 96 from its high bits down: group g of piece c starts at k = c / 2 * 128 + 32 g + c % 2 * 16
     for (int i = tid; i < M * 4 * pieces; i += GP_WARPS * 32) {
         const int m = i / (4 * pieces), s = i - m * 4 * pieces, blk = s >> 3, g = (s >> 1) & 3, half = s & 1;
-        xs[(m * 4 + g) * pieces + blk * 2 + half] = __ldg(reinterpret_cast<const uint4*>(p.q + (size_t)m * p.ldq) + s);
+        xs[(m * 4 + g) * pieces + blk * 2 + half] = reinterpret_cast<const uint4*>(p.q + (size_t)m * p.ldq)[s];
     }
     __syncthreads();
     int acc[M][R];

@@ -93,7 +93,7 @@ __device__ __forceinline__ int row_quant(const T* row, int K, float scale, int8_
 
 // per-token: grid = M
 template <typename T>
-__global__ void __launch_bounds__(QT) act_quant_rows_kernel(const T* __restrict__ x, int K, int ldx, int8_t* __restrict__ q,
+__global__ void __launch_bounds__(QT) act_quant_rows_kernel(const T* x, int K, int ldx, int8_t* __restrict__ q,
                                                             float* __restrict__ scale_out, int32_t* __restrict__ rowsum) {
     __shared__ float fs[33];
     __shared__ int is[33];
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(QT) act_quant_rows_kernel(const T* __restrict_
 
 // per-tensor pass 1: grid-stride absmax -> atomicMax on the float bit pattern (values are >= 0)
 template <typename T>
-__global__ void __launch_bounds__(QT) act_absmax_kernel(const T* __restrict__ x, int M, int K, int ldx,
+__global__ void __launch_bounds__(QT) act_absmax_kernel(const T* x, int M, int K, int ldx,
                                                         unsigned int* __restrict__ amax_bits) {
     pdl_wait_prior();
     pdl_launch_dependents();
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(QT) act_absmax_kernel(const T* __restrict__ x,
 // every row ends with a wait for its last loads).  16384 x 6912 bf16, 226 MB: 46 -> 38 us, 5.9 TB/s.
 constexpr int AU = 8;
 template <typename T>
-__global__ void __launch_bounds__(QT) act_absmax_flat_kernel(const T* __restrict__ x, size_t vectors, unsigned int* __restrict__ amax_bits) {
+__global__ void __launch_bounds__(QT) act_absmax_flat_kernel(const T* x, size_t vectors, unsigned int* __restrict__ amax_bits) {
     pdl_wait_prior();
     pdl_launch_dependents();
     const uint4* p = reinterpret_cast<const uint4*>(x);
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(QT) act_absmax_flat_kernel(const T* __restrict
     for (size_t i = (size_t)blockIdx.x * QT + threadIdx.x; i < vectors; i += AU * step) {
         uint4 raw[AU];
 #pragma unroll
-        for (int u = 0; u < AU; ++u) raw[u] = i + u * step < vectors ? __ldg(p + i + u * step) : make_uint4(0u, 0u, 0u, 0u);
+        for (int u = 0; u < AU; ++u) raw[u] = i + u * step < vectors ? p[i + u * step] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
         for (int u = 0; u < AU; ++u) {
             float v[8];
@@ -149,8 +149,8 @@ __global__ void __launch_bounds__(QT) act_absmax_flat_kernel(const T* __restrict
 // Per-tensor pass 2: grid = M, last rows first: pass 1 has left those in L2 (with quant_i8x4 79 -> 72 us at 16384 x 6912 bf16; the bytes
 // alone are 51; a warp per row with three vectors in flight 91).
 template <typename T>
-__global__ void __launch_bounds__(QT) act_quant_tensor_kernel(const T* __restrict__ x, int K, int ldx,
-                                                              const unsigned int* __restrict__ amax_bits,
+__global__ void __launch_bounds__(QT) act_quant_tensor_kernel(const T* x, int K, int ldx,
+                                                              const unsigned int* amax_bits,
                                                               int8_t* __restrict__ q, float* __restrict__ scale_out,
                                                               int32_t* __restrict__ rowsum) {
     __shared__ int is[QT / 32];
@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(QT) act_quant_tensor_kernel(const T* __restric
 //   y        = bf16( bf16(x * r) * gamma )              (two bf16 multiplies)
 //   q        = quantize_activations_i8(float(y))        (per token)
 // The normalised row is kept in shared memory as bf16 (K*2 bytes, dynamic).
-__global__ void __launch_bounds__(QT) rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x,
-                                                           const __nv_bfloat16* __restrict__ gamma, float eps, int K,
+__global__ void __launch_bounds__(QT) rmsnorm_quant_kernel(const __nv_bfloat16* x,
+                                                           const __nv_bfloat16* gamma, float eps, int K,
                                                            __nv_bfloat16* __restrict__ y_out, int8_t* __restrict__ q,
                                                            float* __restrict__ scale_out, int32_t* __restrict__ rowsum) {
     extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -28,8 +28,8 @@ constexpr int GP_MAXW = 16;     // most warps of a gqa_prep_kernel block
 // angles are formed once per block in double, so that the float values are the correctly rounded ones at any position.
 // MAXD: values a lane holds of one head vector (head sizes up to 32 * MAXD).
 template <typename T, int MAXD>
-__global__ void __launch_bounds__(GP_MAXW * 32) gqa_prep_kernel(Batch b, GqaDims D, const float* __restrict__ proj, int ld, int k_off, int v_off, int g_off,
-                                                                   const T* __restrict__ qb, const T* __restrict__ kb, const T* __restrict__ vb, float eps,
+__global__ void __launch_bounds__(GP_MAXW * 32) gqa_prep_kernel(Batch b, GqaDims D, const float* proj, int ld, int k_off, int v_off, int g_off,
+                                                                   const T* qb, const T* kb, const T* vb, float eps,
                                                                    PagedCache pc, T* __restrict__ qn, float* __restrict__ gate) {
     pdl_enter();
     __shared__ float rot_c[GA_MAXROT], rot_s[GA_MAXROT];
@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(GP_MAXW * 32) gqa_prep_kernel(Batch b, GqaDims
 // and a pair's other entry comes from its lane.  2048 tokens, 20 + 5 + 5 heads of 128 with a gate per element (88 MB): 62 us one entry at a time, 33 so.
 constexpr int GQ = 4;
 template <typename T>
-__global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D, const float* __restrict__ proj, int ld, int k_off, int v_off, int g_off, const T* __restrict__ qb,
-                                                           const T* __restrict__ kb, const T* __restrict__ vb, float eps, PagedCache pc, T* __restrict__ qn,
+__global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D, const float* proj, int ld, int k_off, int v_off, int g_off, const T* qb,
+                                                           const T* kb, const T* vb, float eps, PagedCache pc, T* __restrict__ qn,
                                                            float* __restrict__ gate) {
     pdl_enter();
     __shared__ float rot_c[64], rot_s[64];
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D
 // One block per (token, head).  Its warps take the visible keys (the kept first ones, then the window) round-robin, a warp one key at a time
 // with its lanes over the dimensions; running max / sum / weighted value sum per warp, merged through shared memory.
 template <typename T>
-__global__ void __launch_bounds__(GA_WARPS * 32) gqa_attn_kernel(Batch b, GqaDims D, const T* __restrict__ qn, const float* __restrict__ gate, PagedCache pc,
+__global__ void __launch_bounds__(GA_WARPS * 32) gqa_attn_kernel(Batch b, GqaDims D, const T* qn, const float* gate, PagedCache pc,
                                                                    T* __restrict__ out) {
     pdl_enter();
     extern __shared__ float sm[];   // [GA_WARPS][dv] partial sums, [GA_WARPS] m, [GA_WARPS] l
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(GA_WARPS * 32) gqa_attn_kernel(Batch b, GqaDim
 // accumulators [H][dv] too (any sizes that fit: the launcher checks).
 constexpr int GT_KEYS = 32, GT_THREADS = 256;
 template <typename T>
-__global__ void __launch_bounds__(GT_THREADS) gqa_talk_attn_kernel(Batch b, GqaDims D, const T* __restrict__ qn, const float* __restrict__ gate, PagedCache pc,
+__global__ void __launch_bounds__(GT_THREADS) gqa_talk_attn_kernel(Batch b, GqaDims D, const T* qn, const float* gate, PagedCache pc,
                                                                    T* __restrict__ out) {
     pdl_enter();
     extern __shared__ float sm[];

@@ -36,7 +36,7 @@ struct AmParams {
 // EXT: the score of an element is formed in full (scale, tanh cap, bias by distance, distance penalty) instead of by the one-FMA form
 // that scale and penalty alone allow.
 template <int DKP, int DVP, bool DECODE, int NSTAGE, bool EXT>
-__global__ void __launch_bounds__(AM_THREADS, 3) gqa_attn_mma_kernel(Batch b, GqaDims D, const __nv_bfloat16* __restrict__ qn, const float* __restrict__ gate,
+__global__ void __launch_bounds__(AM_THREADS, 3) gqa_attn_mma_kernel(Batch b, GqaDims D, const __nv_bfloat16* qn, const float* gate,
                                                                     PagedCache pc, __nv_bfloat16* __restrict__ out, AmParams ap) {
     pdl_enter();
     constexpr int KS = DKP + 8, VS = DVP + 8;              // shared-memory row strides in elements
@@ -374,7 +374,7 @@ __global__ void __launch_bounds__(AM_THREADS, 3) gqa_attn_mma_kernel(Batch b, Gq
 
 // one warp per (token, head): merge the key splits' partial results (maxima in units of log 2), apply the gate.  A lane a split for the maxima and sums, then the
 // splits' values side by side: two memory latencies, where one split after the other took one each (a merge of a decode step 4.2 -> 3.2 us).
-__global__ void gqa_attn_merge_kernel(GqaDims D, int rows, int splits, const float* __restrict__ part, const float* __restrict__ gate, __nv_bfloat16* __restrict__ out) {
+__global__ void gqa_attn_merge_kernel(GqaDims D, int rows, int splits, const float* part, const float* gate, __nv_bfloat16* __restrict__ out) {
     pdl_enter();
     const int dv = D.dv, gate_elem = D.gate_elem, stride = dv + 2;
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;

@@ -95,7 +95,7 @@ struct TalkPromptShared {
 
 template <int DKP, int DVP, int KT>
 __global__ void __launch_bounds__(TP_THREADS, 1) __cluster_dims__(TP_CLUSTER, 1, 1)
-    talk_prompt_kernel(Batch b, GqaDims D, const __nv_bfloat16* __restrict__ qn, PagedCache pc, __nv_bfloat16* __restrict__ out, TalkParams tp) {
+    talk_prompt_kernel(Batch b, GqaDims D, const __nv_bfloat16* qn, PagedCache pc, __nv_bfloat16* __restrict__ out, TalkParams tp) {
     pdl_enter();
     using SH = TalkPromptShared<DKP, DVP, KT>;
     constexpr int KS = SH::KS, VS = SH::VS, PS = SH::PS, WS = SH::WS, NKS = DKP / 16, NVT = DVP / 8, NST = KT / 8;
@@ -372,7 +372,7 @@ struct TalkDecodeShared {
 
 // MT: 16-row tiles of heads; IT: (key/value head, 16 value columns) items per warp
 template <int MT, int IT>
-__global__ void __launch_bounds__(TK_THREADS, MT * IT <= 10 ? 2 : 1) talk_decode_kernel(Batch b, GqaDims D, const __nv_bfloat16* __restrict__ qn, PagedCache pc, TalkParams tp) {
+__global__ void __launch_bounds__(TK_THREADS, MT * IT <= 10 ? 2 : 1) talk_decode_kernel(Batch b, GqaDims D, const __nv_bfloat16* qn, PagedCache pc, TalkParams tp) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
     const TalkDecodeShared sh(D, tp.kt);
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(TK_THREADS, MT * IT <= 10 ? 2 : 1) talk_decode
 // block per (token, key/value head, four of its query heads): normalise the source heads over the splits, mix, write; every partial result is
 // read once.  blockDim = (values rounded up to 32, slices of the sum)
 constexpr int TM_HEADS = 4;
-__global__ void talk_merge_kernel(Batch b, GqaDims D, int splits, const float* __restrict__ parts, __nv_bfloat16* __restrict__ out) {
+__global__ void talk_merge_kernel(Batch b, GqaDims D, int splits, const float* parts, __nv_bfloat16* __restrict__ out) {
     pdl_enter();
     extern __shared__ __align__(16) float cf[];            // [splits][H][TM_HEADS] factors, then [slices][TM_HEADS][dv] partial sums
     const int sq = blockIdx.x, kv = blockIdx.y, rep = D.H / D.G, h0 = kv * rep + blockIdx.z * TM_HEADS, tok = b.seq_start[sq];

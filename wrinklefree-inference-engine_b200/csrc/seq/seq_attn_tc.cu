@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
             const int chunks = D.d > 64 ? 16 : 8;
             for (int c = 0; c < chunks; ++c) {
                 uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (r_ok && c * 8 < D.d) v = __ldg(src + c);
+                if (r_ok && c * 8 < D.d) v = src[c];
                 asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(qrow + (c >> 3) * AT_HALF + (((c & 7) ^ (row & 7)) << 4)), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
             }
             fence_proxy_async();

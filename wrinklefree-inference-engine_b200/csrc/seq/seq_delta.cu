@@ -12,8 +12,8 @@ namespace {
 
 // one block per token: unit-normalise the q and k heads in place, compute the write strength and the decay of every head
 template <typename T>
-__global__ void delta_prep_kernel(DeltaDims D, float* __restrict__ qkv, int ld, const float* __restrict__ a_raw, int lda, const float* __restrict__ b_raw,
-                                  int ldb, const T* __restrict__ A_log, const T* __restrict__ dt_bias, float* __restrict__ beta, float* __restrict__ decay) {
+__global__ void delta_prep_kernel(DeltaDims D, float* __restrict__ qkv, int ld, const float* a_raw, int lda, const float* b_raw,
+                                  int ldb, const T* A_log, const T* dt_bias, float* __restrict__ beta, float* __restrict__ decay) {
     pdl_enter();
     const int i = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -39,8 +39,8 @@ __global__ void delta_prep_kernel(DeltaDims D, float* __restrict__ qkv, int ld, 
 // The same, four consecutive elements per load, a head vector in the lanes of one warp (d a multiple of 4 up to 128).  1801 tokens, 20 heads of 128 with a
 // decay per channel (74 MB): 32 us one element at a time, 18 so.
 template <typename T>
-__global__ void __launch_bounds__(256) delta_prep_vec_kernel(DeltaDims D, float* __restrict__ qkv, int ld, const float* __restrict__ a_raw, int lda, const float* __restrict__ b_raw,
-                                                             int ldb, const T* __restrict__ A_log, const T* __restrict__ dt_bias, float* __restrict__ beta,
+__global__ void __launch_bounds__(256) delta_prep_vec_kernel(DeltaDims D, float* __restrict__ qkv, int ld, const float* a_raw, int lda, const float* b_raw,
+                                                             int ldb, const T* A_log, const T* dt_bias, float* __restrict__ beta,
                                                              float* __restrict__ decay) {
     pdl_enter();
     const int i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(256) delta_prep_vec_kernel(DeltaDims D, float*
 
 // state-space recurrence: the step size and the decay of every head
 template <typename T>
-__global__ void ssd_prep_kernel(int n, int H, const float* __restrict__ dt_raw, int ld, const T* __restrict__ A_log, const T* __restrict__ dt_bias,
+__global__ void ssd_prep_kernel(int n, int H, const float* dt_raw, int ld, const T* A_log, const T* dt_bias,
                                 float* __restrict__ step, float* __restrict__ decay) {
     pdl_enter();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -93,8 +93,8 @@ __global__ void ssd_prep_kernel(int n, int H, const float* __restrict__ dt_raw, 
 
 // one block per (token, norm group): v = (o + D_h x) * silu(z), divided by the root mean square of the group, times the weight
 template <typename T>
-__global__ void ssd_post_kernel(int H, int dv, int groups, const float* __restrict__ o, const float* __restrict__ x, int ldx, const float* __restrict__ z, int ldz,
-                                const T* __restrict__ Dskip, const T* __restrict__ w, float eps, T* __restrict__ y) {
+__global__ void ssd_post_kernel(int H, int dv, int groups, const float* o, const float* x, int ldx, const float* z, int ldz,
+                                const T* Dskip, const T* w, float eps, T* __restrict__ y) {
     pdl_enter();
     __shared__ float scratch[33];
     const int i = blockIdx.x, g = blockIdx.y;
@@ -117,8 +117,8 @@ __global__ void ssd_post_kernel(int H, int dv, int groups, const float* __restri
 // The same with a group's values in registers between the two passes, four consecutive elements per load: gw a multiple of 4 up to 2048, dv one of 4.
 // 2048 tokens x 2560 channels in 5 groups (73 MB): 35 us with every input read twice, 16 so.
 template <typename T>
-__global__ void __launch_bounds__(512) ssd_post_vec_kernel(int H, int dv, int groups, const float* __restrict__ o, const float* __restrict__ x, int ldx, const float* __restrict__ z, int ldz,
-                                                           const T* __restrict__ Dskip, const T* __restrict__ w, float eps, T* __restrict__ y) {
+__global__ void __launch_bounds__(512) ssd_post_vec_kernel(int H, int dv, int groups, const float* o, const float* x, int ldx, const float* z, int ldz,
+                                                           const T* Dskip, const T* w, float eps, T* __restrict__ y) {
     pdl_enter();
     __shared__ float scratch[33];
     const int i = blockIdx.x, g = blockIdx.y;
@@ -164,8 +164,8 @@ __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gsrc) {
 // DELTA: the write is corrected by what the state already holds along the key (the delta rule); without it u = beta v.
 // NC: columns per thread (consecutive ones; 2 halves the shared-memory reads per multiply-add where there are columns and rows enough).
 template <int DPT, int DR_PARTS, bool VEC, bool DELTA, int NC>
-__global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(Batch b, DeltaDims D, const float* __restrict__ qkv, int ld,
-                                                                         const float* __restrict__ beta, const float* __restrict__ decay,
+__global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(Batch b, DeltaDims D, const float* qkv, int ld,
+                                                                         const float* beta, const float* decay,
                                                                          float* __restrict__ state, size_t slot_stride, float* __restrict__ o, ScanArgs sa) {
     pdl_enter();
     constexpr int DR_COLS = DR_THREADS / DR_PARTS * NC;
@@ -361,8 +361,8 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(Batch b, DeltaDi
 
 // thread per (sequence, head, state element): chains the chunks' start states from the slot's state and leaves the end state in the slot.
 // prod has one entry per (chunk, head), or (d > 0) one per (chunk, head, key row) of dd / d state columns each
-__global__ void scan_prefix_kernel(Batch b, int H, int dd, int chunk, float* __restrict__ state, size_t slot_stride, const float* __restrict__ local,
-                                   float* __restrict__ startws, const float* __restrict__ prod, int d) {
+__global__ void scan_prefix_kernel(Batch b, int H, int dd, int chunk, float* __restrict__ state, size_t slot_stride, const float* local,
+                                   float* __restrict__ startws, const float* prod, int d) {
     pdl_enter();
     const int sq = blockIdx.x, h = blockIdx.y, e = blockIdx.z * blockDim.x + threadIdx.x;
     if (e >= dd) return;
@@ -378,7 +378,7 @@ __global__ void scan_prefix_kernel(Batch b, int H, int dd, int chunk, float* __r
 }
 
 // thread per (sequence and chunk, head and key row): the product of the chunk's decays
-__global__ void scan_decay_prod_kernel(Batch b, int nd, int chunk, int nchunks, const float* __restrict__ decay, float* __restrict__ prod) {
+__global__ void scan_decay_prod_kernel(Batch b, int nd, int chunk, int nchunks, const float* decay, float* __restrict__ prod) {
     pdl_enter();
     const int sq = blockIdx.x / nchunks, c = blockIdx.x - sq * nchunks, k = blockIdx.y * blockDim.x + threadIdx.x;
     const int len = b.seq_len[sq], start = b.seq_start[sq];
@@ -398,8 +398,8 @@ __device__ __forceinline__ float gla_decay_of(float z, float inv_tau) {        /
 // The same on tensor cores (bf16 storage): 64 tokens x 64 channels per block, a warp per 16 tokens.  The float low-rank rows enter as a
 // two-term bf16 split, so that the product sees them to 2^-17; a2 is bf16 as stored.  rp: rank rounded up to 16.
 constexpr int GM_TOK = 64, GM_CH = 64;
-__global__ void __launch_bounds__(128) gla_decay_mma_kernel(int n, int rank, int rp, int nout, const float* __restrict__ a1, int ld, const __nv_bfloat16* __restrict__ a2,
-                                                            const __nv_bfloat16* __restrict__ bias, float inv_tau, float* __restrict__ decay) {
+__global__ void __launch_bounds__(128) gla_decay_mma_kernel(int n, int rank, int rp, int nout, const float* a1, int ld, const __nv_bfloat16* a2,
+                                                            const __nv_bfloat16* bias, float inv_tau, float* __restrict__ decay) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char gm_raw[];
     __shared__ float zb[GM_CH];
@@ -471,8 +471,8 @@ __global__ void __launch_bounds__(128) gla_decay_mma_kernel(int n, int rank, int
 // decay of gated linear attention: a thread owns one output channel and GD_TOK tokens; the tokens' low-rank rows lie in shared memory
 constexpr int GD_TOK = 8, GD_THREADS = 128;
 template <typename T>
-__global__ void __launch_bounds__(GD_THREADS) gla_decay_kernel(int n, int rank, int nout, const float* __restrict__ a1, int ld, const T* __restrict__ a2,
-                                                               const T* __restrict__ bias, float inv_tau, float* __restrict__ decay) {
+__global__ void __launch_bounds__(GD_THREADS) gla_decay_kernel(int n, int rank, int nout, const float* a1, int ld, const T* a2,
+                                                               const T* bias, float inv_tau, float* __restrict__ decay) {
     pdl_enter();
     extern __shared__ float rows[];                  // [rank][GD_TOK]
     const int i0 = blockIdx.x * GD_TOK, c = blockIdx.y * GD_THREADS + threadIdx.x;
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(GD_THREADS) gla_decay_kernel(int n, int rank, 
 }
 
 template <typename T>
-__global__ void delta_post_kernel(DeltaDims D, const float* __restrict__ o, const T* __restrict__ w, float eps, const float* __restrict__ g, int ldg,
+__global__ void delta_post_kernel(DeltaDims D, const float* o, const T* w, float eps, const float* g, int ldg,
                                   T* __restrict__ y, int act) {
     pdl_enter();
     const int i = blockIdx.x;
@@ -519,7 +519,7 @@ __global__ void delta_post_kernel(DeltaDims D, const float* __restrict__ o, cons
 
 // a warp per (token, head), four consecutive elements per load (dv a multiple of 4 up to 128): 1801 tokens, 20 heads of 128 (46 MB) 30 -> 12 us
 template <typename T>
-__global__ void __launch_bounds__(128) delta_post_vec_kernel(DeltaDims D, const float* __restrict__ o, const T* __restrict__ w, float eps, const float* __restrict__ g, int ldg,
+__global__ void __launch_bounds__(128) delta_post_vec_kernel(DeltaDims D, const float* o, const T* w, float eps, const float* g, int ldg,
                                                              T* __restrict__ y, int act) {
     pdl_enter();
     const int i = blockIdx.x, lane = threadIdx.x & 31, h = blockIdx.y * 4 + (threadIdx.x >> 5), c = 4 * lane;

@@ -23,8 +23,8 @@ constexpr int MG_UN = 8;        // tokens whose inputs are loaded before any of 
 // ch: channels of a block (a power of two up to 32); a warp holds 32 / ch time slices of them.  Few channels per block make more blocks
 // and more slices when one long portion has to fill the machine; 8 floats are still a whole 32-byte sector of a row.
 template <typename T>
-__global__ void __launch_bounds__(32 * MG_MAXW) mingru_kernel(Batch b, int C, int ch, const float* __restrict__ proj, int ld, int z_off, int x_off, int g_off,
-                                                                const T* __restrict__ zb, const T* __restrict__ xb, float* __restrict__ state,
+__global__ void __launch_bounds__(32 * MG_MAXW) mingru_kernel(Batch b, int C, int ch, const float* proj, int ld, int z_off, int x_off, int g_off,
+                                                                const T* zb, const T* xb, float* __restrict__ state,
                                                                 size_t slot_stride, T* __restrict__ out) {
     pdl_enter();
     __shared__ float sA[32 * MG_MAXW], sB[32 * MG_MAXW];       // [slice][ch]
@@ -90,8 +90,8 @@ constexpr int ML_MAXW = 32;
 // I = log input gate); maps compose as (F1, I1) then (F2, I2) = (F1 + F2, max(F2 + I1, I2)).  Each warp scans its 32 maps with shuffles,
 // the warps' totals are chained through shared memory, and the block walks the portion in passes of 32 tokens per warp.
 template <typename T>
-__global__ void __launch_bounds__(32 * ML_MAXW) mlstm_gates_kernel(Batch b, int H, const float* __restrict__ proj, int ld, int i_off, int f_off,
-                                                                     const T* __restrict__ ib, const T* __restrict__ fb, float cap, float* __restrict__ mstate,
+__global__ void __launch_bounds__(32 * ML_MAXW) mlstm_gates_kernel(Batch b, int H, const float* proj, int ld, int i_off, int f_off,
+                                                                     const T* ib, const T* fb, float cap, float* __restrict__ mstate,
                                                                      size_t slot_stride, float* __restrict__ keep, float* __restrict__ put, float* __restrict__ mrun) {
     pdl_enter();
     __shared__ float totF[ML_MAXW], totI[ML_MAXW];
@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(32 * ML_MAXW) mlstm_gates_kernel(Batch b, int 
 
 // one warp per (token, head)
 template <typename T>
-__global__ void mlstm_post_kernel(int n, int H, int dv, const float* __restrict__ o, const float* __restrict__ mrun, float qscale, const T* __restrict__ w,
-                                  float eps, const float* __restrict__ g, int ldg, T* __restrict__ y) {
+__global__ void mlstm_post_kernel(int n, int H, int dv, const float* o, const float* mrun, float qscale, const T* w,
+                                  float eps, const float* g, int ldg, T* __restrict__ y) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const long long unit = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);

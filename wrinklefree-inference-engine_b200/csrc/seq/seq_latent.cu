@@ -32,7 +32,7 @@ __device__ __forceinline__ void rope_table(const LatentDims& L, int pos, float* 
     }
 }
 // entry e of a rotated part `src` (r entries, the first rope_dims of them in pairs) after the rotation
-__device__ __forceinline__ float rope_entry(const LatentDims& L, const float* __restrict__ src, int e, const float* cs, const float* sn) {
+__device__ __forceinline__ float rope_entry(const LatentDims& L, const float* src, int e, const float* cs, const float* sn) {
     if (e >= L.rope_dims) return src[e];
     const int half = L.rope_dims / 2;
     int p, other; bool first;
@@ -42,7 +42,7 @@ __device__ __forceinline__ float rope_entry(const LatentDims& L, const float* __
 }
 
 template <typename T>
-__global__ void latent_q_prep_kernel(Batch b, LatentDims L, const float* __restrict__ q, int ldq, T* __restrict__ qn, float* __restrict__ qr) {
+__global__ void latent_q_prep_kernel(Batch b, LatentDims L, const float* q, int ldq, T* __restrict__ qn, float* __restrict__ qr) {
     pdl_enter();
     __shared__ float cs[LA_MAXPAIRS], sn[LA_MAXPAIRS];
     const int i = blockIdx.x;
@@ -63,7 +63,7 @@ __global__ void latent_q_prep_kernel(Batch b, LatentDims L, const float* __restr
 // The same, four consecutive elements per load: d, r and the rotated entries multiples of 4 (of 8 where pairs lie half the rotated entries apart).
 // 2048 tokens, 20 heads of 96 + 32 (31 MB): 19 us one element at a time, 9 so.
 template <typename T>
-__global__ void __launch_bounds__(256) latent_q_prep_vec_kernel(Batch b, LatentDims L, const float* __restrict__ q, int ldq, T* __restrict__ qn, float* __restrict__ qr) {
+__global__ void __launch_bounds__(256) latent_q_prep_vec_kernel(Batch b, LatentDims L, const float* q, int ldq, T* __restrict__ qn, float* __restrict__ qr) {
     pdl_enter();
     __shared__ float cs[LA_MAXPAIRS], sn[LA_MAXPAIRS];
     const int i = blockIdx.x, per = L.d + L.r, total = L.H * per, half = L.rope_dims / 2, step = gridDim.y * 1024;
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(256) latent_q_prep_vec_kernel(Batch b, LatentD
 
 // one block per token: latent RMS norm + rotary of the shared key part, stored as T in the token's cache row
 template <typename T>
-__global__ void latent_kv_write_kernel(Batch b, LatentDims L, const float* __restrict__ dkv, int ld, const T* __restrict__ w, float eps, PagedCache pc) {
+__global__ void latent_kv_write_kernel(Batch b, LatentDims L, const float* dkv, int ld, const T* w, float eps, PagedCache pc) {
     pdl_enter();
     __shared__ float scratch[33];
     __shared__ float cs[LA_MAXPAIRS], sn[LA_MAXPAIRS];
@@ -125,7 +125,7 @@ constexpr int LA_MAXr = 8;     // rotated size up to 32 * 8
 // over the dimensions (coalesced reads of the cache row), keeps a running max / sum / weighted latent sum, and the warps' partial results
 // are merged through shared memory at the end.
 template <typename T>
-__global__ void __launch_bounds__(LA_WARPS * 32) latent_attn_kernel(Batch b, LatentDims L, const float* __restrict__ qa, const float* __restrict__ qr,
+__global__ void __launch_bounds__(LA_WARPS * 32) latent_attn_kernel(Batch b, LatentDims L, const float* qa, const float* qr,
                                                                       PagedCache pc, T* __restrict__ out) {
     pdl_enter();
     extern __shared__ float sm[];   // [LA_WARPS][R] partial sums, then [LA_WARPS] m, [LA_WARPS] l
@@ -200,7 +200,7 @@ int check_dims(const LatentDims& L) {
 
 // rows of every head's key [W_uk | 0] and [0 | unit rows], then of every head's value [W_uv | 0]
 template <typename T>
-__global__ void latent_expand_weight_kernel(LatentDims L, const T* __restrict__ uk, const T* __restrict__ uv, T* __restrict__ out) {
+__global__ void latent_expand_weight_kernel(LatentDims L, const T* uk, const T* uv, T* __restrict__ out) {
     pdl_enter();
     const int width = L.R + L.r, per = L.d + L.r, row = blockIdx.x;
     for (int c = threadIdx.x; c < width; c += blockDim.x) {
@@ -215,7 +215,7 @@ __global__ void latent_expand_weight_kernel(LatentDims L, const T* __restrict__ 
 }
 
 // a warp per cached row, 16 bytes per lane and copy
-__global__ void latent_gather_kernel(Batch b, LatentDims L, PagedCache pc, const int32_t* __restrict__ key_row, int rows, __nv_bfloat16* __restrict__ out) {
+__global__ void latent_gather_kernel(Batch b, LatentDims L, PagedCache pc, const int32_t* key_row, int rows, __nv_bfloat16* __restrict__ out) {
     pdl_enter();
     const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;

@@ -41,7 +41,7 @@ struct MmaParams {
 
 // NT = R / 32: n-tiles (8 latent dimensions each) per warp in the value product
 template <int NT>
-__global__ void latent_attn_mma_kernel(Batch b, LatentDims L, const float* __restrict__ qa, const float* __restrict__ qr, PagedCache pc,
+__global__ void latent_attn_mma_kernel(Batch b, LatentDims L, const float* qa, const float* qr, PagedCache pc,
                                        __nv_bfloat16* __restrict__ out, MmaParams mp) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -218,7 +218,7 @@ __global__ void latent_attn_mma_kernel(Batch b, LatentDims L, const float* __res
 }
 
 // one block per (token, head): out = sum_s exp(m_s - m) O_s / sum_s exp(m_s - m) l_s
-__global__ void latent_attn_merge_kernel(int H, int R, int splits, const float* __restrict__ part, __nv_bfloat16* __restrict__ out, const float* __restrict__ sink) {
+__global__ void latent_attn_merge_kernel(int H, int R, int splits, const float* part, __nv_bfloat16* __restrict__ out, const float* sink) {
     pdl_enter();
     const int i = blockIdx.x, h = blockIdx.y;
     const float* p0 = part + (((size_t)i * splits) * H + h) * (R + 2);
@@ -259,7 +259,7 @@ __device__ __forceinline__ void ldsm_x2_trans_a(uint32_t (&r)[2], uint32_t addr)
 __host__ __device__ constexpr int kt_pt_stride(int NH) { return (NH & 1) ? NH * 8 + 16 : NH * 8 + 8; }   // 16-byte units per row odd: conflict-free ldmatrix
 
 template <int NH, int MTW>
-__global__ void __launch_bounds__(256) latent_attn_kt_kernel(Batch b, LatentDims L, const float* __restrict__ qa, const float* __restrict__ qr, PagedCache pc,
+__global__ void __launch_bounds__(256) latent_attn_kt_kernel(Batch b, LatentDims L, const float* qa, const float* qr, PagedCache pc,
                                                              __nv_bfloat16* __restrict__ out, MmaParams mp) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];

@@ -21,7 +21,7 @@ __device__ __forceinline__ void warp_argmax(float& v, int& idx) {   // largest v
 // The choice of one token by one warp.  zr: the token's logits (global or shared); sm: 2 N + groups floats of shared memory
 // (s[N] scores, ch[N] choice scores, gs[G] group scores).
 template <typename T>
-__device__ void route_token(const RouterDims& R, const float* zr, const T* __restrict__ correction, int32_t* __restrict__ ids, float* __restrict__ wts,
+__device__ void route_token(const RouterDims& R, const float* zr, const T* correction, int32_t* __restrict__ ids, float* __restrict__ wts,
                             int32_t* __restrict__ counts, float* sm, int i, int lane) {
     const int N = R.E + R.I, gsz = N / R.groups;
     float* sc = sm;
@@ -95,7 +95,7 @@ __device__ void route_token(const RouterDims& R, const float* zr, const T* __res
 
 // one warp per token
 template <typename T>
-__global__ void moe_route_kernel(RouterDims R, const float* __restrict__ z, int ldz, const T* __restrict__ correction, int32_t* __restrict__ ids,
+__global__ void moe_route_kernel(RouterDims R, const float* z, int ldz, const T* correction, int32_t* __restrict__ ids,
                                  float* __restrict__ wts, int32_t* __restrict__ counts) {
     pdl_enter();
     extern __shared__ float sm[];
@@ -111,8 +111,8 @@ __global__ void moe_route_kernel(RouterDims R, const float* __restrict__ z, int 
 // NT: threads of a block — one warp per router row when the tokens do not fill the machine by themselves.
 constexpr int RF_THREADS = 256, RF_THREADS_FEW = 1024, RF_TB = 1;
 template <typename T, bool VEC, int NT>
-__global__ void __launch_bounds__(NT) router_fused_kernel(RouterDims R, int n, int tb, const float* __restrict__ x, int ldx, const T* __restrict__ w, int NZ, int W,
-                                                                  float* __restrict__ z, int ldz, const T* __restrict__ correction, int32_t* __restrict__ ids,
+__global__ void __launch_bounds__(NT) router_fused_kernel(RouterDims R, int n, int tb, const float* x, int ldx, const T* w, int NZ, int W,
+                                                                  float* __restrict__ z, int ldz, const T* correction, int32_t* __restrict__ ids,
                                                                   float* __restrict__ wts, int32_t* __restrict__ counts) {
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(NT) router_fused_kernel(RouterDims R, int n, i
 }
 
 // single block.  scratch: off[E + 1], cursor[E]
-__global__ void moe_plan_kernel(RouterDims R, int n, const int32_t* __restrict__ ids, const int32_t* __restrict__ counts, int32_t* __restrict__ scratch,
+__global__ void moe_plan_kernel(RouterDims R, int n, const int32_t* ids, const int32_t* counts, int32_t* __restrict__ scratch,
                                 int32_t* __restrict__ sorted_rows, int32_t* __restrict__ pair_row, int32_t* __restrict__ tile_group, int P) {
     pdl_enter();
     int32_t* off = scratch;
@@ -195,7 +195,7 @@ __global__ void moe_plan_kernel(RouterDims R, int n, const int32_t* __restrict__
 
 // VEC = 4: ff a multiple of 4 (16-byte loads of the gate and up halves)
 template <typename T, int VEC>
-__global__ void silu_mul_kernel(const float* __restrict__ gu, int ff, const int32_t* __restrict__ tile_group, T* __restrict__ hmid, int act, float limit) {
+__global__ void silu_mul_kernel(const float* gu, int ff, const int32_t* tile_group, T* __restrict__ hmid, int act, float limit) {
     pdl_enter();
     const int r = blockIdx.x;
     if (tile_group && tile_group[r / GEMM_BM] < 0) return;
@@ -222,9 +222,9 @@ __global__ void silu_mul_kernel(const float* __restrict__ gu, int ff, const int3
 
 // VEC = 4: W a multiple of 4
 template <typename T, int VEC>
-__global__ void moe_combine_kernel(RouterDims R, int W, const int32_t* __restrict__ ids, const float* __restrict__ wts, const int32_t* __restrict__ pair_row,
-                                   const float* __restrict__ y, const T* __restrict__ h, float* __restrict__ out, const float* __restrict__ shared_y,
-                                   const float* __restrict__ shared_gate, int ld_gate) {
+__global__ void moe_combine_kernel(RouterDims R, int W, const int32_t* ids, const float* wts, const int32_t* pair_row,
+                                   const float* y, const T* h, float* __restrict__ out, const float* shared_y,
+                                   const float* shared_gate, int ld_gate) {
     pdl_enter();
     const int i = blockIdx.x;
     const float sg = shared_y ? (shared_gate ? sigmoid_f(shared_gate[(size_t)i * ld_gate]) : 1.f) : 0.f;
@@ -345,8 +345,8 @@ __device__ float block_reduce_sum(float v, float* scratch) { return block_sum(v,
 // One block per row.  Greedy: argmax, lowest index among equals.  Otherwise p = softmax(logits / temperature); the kept set is
 // {p >= tau} with tau found by bisection so that it holds at most top_k entries and is the smallest such set whose mass reaches top_p;
 // the draw walks the kept entries in index order.
-__global__ void __launch_bounds__(SM_THREADS) sample_kernel(const float* __restrict__ logits, int V, float temperature, int top_k, float top_p,
-                                                             const float* __restrict__ u, int32_t* __restrict__ next) {
+__global__ void __launch_bounds__(SM_THREADS) sample_kernel(const float* logits, int V, float temperature, int top_k, float top_p,
+                                                             const float* u, int32_t* __restrict__ next) {
     pdl_enter();
     __shared__ float scratch[33];
     __shared__ float sv[SM_THREADS / 32];

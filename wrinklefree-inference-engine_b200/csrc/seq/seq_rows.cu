@@ -7,8 +7,8 @@ namespace seq {
 
 // VEC = 4: W a multiple of 4, everything aligned (2048 x 2560 bf16: 13 us one element at a time, 7 so)
 template <typename T, int VEC>
-__global__ void embed_f32_kernel(const T* __restrict__ table, const int32_t* __restrict__ tokens, int W, float* __restrict__ x, float scale, T* __restrict__ x_t,
-                                 const T* __restrict__ pos_table, const int32_t* __restrict__ tok_pos) {
+__global__ void embed_f32_kernel(const T* table, const int32_t* tokens, int W, float* __restrict__ x, float scale, T* __restrict__ x_t,
+                                 const T* pos_table, const int32_t* tok_pos) {
     pdl_enter();
     const int i = blockIdx.x;
     const T* row = table + (size_t)tokens[i] * W;
@@ -39,7 +39,7 @@ int launch_embed_f32(int dt, const void* table, const int32_t* tokens, int n, in
     return launch_check(cudaGetLastError(), "embed_f32");
 }
 
-__global__ void axpby_kernel(float* __restrict__ y, float a, const float* __restrict__ y2, float b, size_t count) {
+__global__ void axpby_kernel(float* __restrict__ y, float a, const float* y2, float b, size_t count) {
     pdl_enter();
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x) y[k] = a * y[k] + b * y2[k];
 }
@@ -54,7 +54,7 @@ int launch_axpby(float* y, float a, const float* y2, float b, size_t count, cuda
 // x[i, :] = table[tokens[i], :] + position vector of tok_pos[i]: entry 2k = sin(a), entry 2k + 1 = cos(a), a = pos * base^(-2k / W).
 // The frequency and the angle are formed in double so that the float result is the correctly rounded one also at large positions.
 template <typename T>
-__global__ void embed_pos_kernel(const T* __restrict__ table, const int32_t* __restrict__ tokens, const int32_t* __restrict__ tok_pos, int W, float base,
+__global__ void embed_pos_kernel(const T* table, const int32_t* tokens, const int32_t* tok_pos, int W, float base,
                                  float* __restrict__ x, T* __restrict__ x_t) {
     pdl_enter();
     // a thread per pair of channels, which share an angle: the double precision sine and cosine are what this kernel costs (8 tokens x 1024: 5.9 us with four
@@ -84,7 +84,7 @@ int launch_embed_pos(int dt, const void* table, const int32_t* tokens, const int
 
 // x_t[i, :] = T(x[i, :])
 template <typename T>
-__global__ void round_rows_kernel(const float* __restrict__ x, size_t count, T* __restrict__ x_t) {
+__global__ void round_rows_kernel(const float* x, size_t count, T* __restrict__ x_t) {
     pdl_enter();
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < count; k += (size_t)gridDim.x * blockDim.x) x_t[k] = from_f<T>(x[k]);
 }
@@ -102,9 +102,9 @@ int launch_round_rows(int dt, const float* x, int n, int W, void* x_t, cudaStrea
 // registers between the two passes (up to SN_PER values per thread, re-read beyond that).
 constexpr int SN_THREADS = 256, SN_PER = 8;
 template <typename T>
-__global__ void __launch_bounds__(SN_THREADS) scalar_rmsnorm_kernel(const float* __restrict__ y, int ldy, const T* __restrict__ bias, const T* __restrict__ gain, float mult,
+__global__ void __launch_bounds__(SN_THREADS) scalar_rmsnorm_kernel(const float* y, int ldy, const T* bias, const T* gain, float mult,
                                                                     float eps, int W, const float* res, float* out, int ldo, T* __restrict__ out_t, int ldt,
-                                                                    const int32_t* __restrict__ rows) {
+                                                                    const int32_t* rows) {
     pdl_enter();
     __shared__ float scratch[33];
     const int i = blockIdx.x;
@@ -150,7 +150,7 @@ int launch_scalar_rmsnorm(int dt, const float* y, int ldy, const void* bias, con
 
 // y[i, :] += bias
 template <typename T>
-__global__ void add_bias_kernel(float* __restrict__ y, int ld, const T* __restrict__ bias, int W) {
+__global__ void add_bias_kernel(float* __restrict__ y, int ld, const T* bias, int W) {
     pdl_enter();
     for (int c = threadIdx.x; c < W; c += blockDim.x) y[(size_t)blockIdx.x * ld + c] += to_f(bias[c]);
 }
@@ -164,8 +164,8 @@ int launch_add_bias(int dt, float* y, int ld, const void* bias, int n, int W, cu
 
 // one block per (row, group).  x2 (optional): the normalised quantity is a * x + b * x2 (two mixers' outputs combined on the way in)
 template <typename T>
-__global__ void group_rmsnorm_kernel(const float* __restrict__ x, int ldx, const T* __restrict__ w, int gw, float eps, const float* res,
-                                     float* y, int ldy, T* __restrict__ y_t, int ldt, const int32_t* __restrict__ rows, const float* __restrict__ x2, float a,
+__global__ void group_rmsnorm_kernel(const float* x, int ldx, const T* w, int gw, float eps, const float* res,
+                                     float* y, int ldy, T* __restrict__ y_t, int ldt, const int32_t* rows, const float* x2, float a,
                                      float b, float w_offset) {
     pdl_enter();
     __shared__ float scratch[33];
@@ -188,8 +188,8 @@ __global__ void group_rmsnorm_kernel(const float* __restrict__ x, int ldx, const
 // The same with four consecutive elements per load and every input of a row requested before the first is used; a thread owns NV groups of four,
 // blockDim.x * NV * 4 >= gw.  What bounds it is the bytes: 2048 rows of 2560 from two inputs and a residual, 94 MB: 30 us one element at a time, 15 so.
 template <typename T, int NV>
-__global__ void __launch_bounds__(1024) group_rmsnorm_vec_kernel(const float* x, int ldx, const T* __restrict__ w, int gw, float eps, const float* res, float* y, int ldy,
-                                                                 T* __restrict__ y_t, int ldt, const int32_t* __restrict__ rows, const float* x2, float a, float b,
+__global__ void __launch_bounds__(1024) group_rmsnorm_vec_kernel(const float* x, int ldx, const T* w, int gw, float eps, const float* res, float* y, int ldy,
+                                                                 T* __restrict__ y_t, int ldt, const int32_t* rows, const float* x2, float a, float b,
                                                                  float w_offset) {
     pdl_enter();
     __shared__ float scratch[33];
@@ -256,8 +256,8 @@ int launch_group_rmsnorm(int dt, const float* x, int ldx, const void* w, int gro
 // thread; wider rows are re-read from x, which the same thread has just written).
 constexpr int AD_THREADS = 256, AD_PER = 8;
 template <typename T>
-__global__ void __launch_bounds__(AD_THREADS) add_dual_norm_kernel(float* __restrict__ x, const float* __restrict__ y1, float a1, const float* __restrict__ y2, float a2,
-                                                                     const float* __restrict__ y3, const T* __restrict__ w1, const T* __restrict__ w2, float w_offset,
+__global__ void __launch_bounds__(AD_THREADS) add_dual_norm_kernel(float* __restrict__ x, const float* y1, float a1, const float* y2, float a2,
+                                                                     const float* y3, const T* w1, const T* w2, float w_offset,
                                                                      float eps, int W, T* __restrict__ h1, T* __restrict__ h2) {
     pdl_enter();
     __shared__ float scratch[33];
@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(AD_THREADS) add_dual_norm_kernel(float* __rest
 
 // Four consecutive elements per load, everything requested before the first is used (rows of up to 8192; see group_rmsnorm_vec_kernel).
 template <typename T, int NV>
-__global__ void __launch_bounds__(1024) add_dual_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ y1, float a1, const float* __restrict__ y2, float a2,
-                                                                 const float* __restrict__ y3, const T* __restrict__ w1, const T* __restrict__ w2, float w_offset, float eps,
+__global__ void __launch_bounds__(1024) add_dual_norm_vec_kernel(float* __restrict__ x, const float* y1, float a1, const float* y2, float a2,
+                                                                 const float* y3, const T* w1, const T* w2, float w_offset, float eps,
                                                                  int W, T* __restrict__ h1, T* __restrict__ h2) {
     pdl_enter();
     __shared__ float scratch[33];
@@ -376,8 +376,8 @@ __device__ __forceinline__ float block_sq_dev(const float (&keep)[PER], const fl
 // one block per row; the row stays in registers between the two statistics and the store (re-read beyond LN_PER values per thread)
 constexpr int LN_PER = 8;
 template <typename T>
-__global__ void __launch_bounds__(512) layer_norm_kernel(const float* __restrict__ x, int ldx, const T* __restrict__ w, const T* __restrict__ b, float eps, int W,
-                                                         float* __restrict__ y, int ldy, T* __restrict__ y_t, int ldt, const int32_t* __restrict__ rows) {
+__global__ void __launch_bounds__(512) layer_norm_kernel(const float* x, int ldx, const T* w, const T* b, float eps, int W,
+                                                         float* __restrict__ y, int ldy, T* __restrict__ y_t, int ldt, const int32_t* rows) {
     pdl_enter();
     __shared__ float scratch[33];
     const int i = blockIdx.x;
@@ -419,7 +419,7 @@ int launch_layer_norm(int dt, const float* x, int ldx, const void* w, const void
 
 // one block per row (launch_branch_add_norm)
 template <typename T>
-__global__ void __launch_bounds__(512) branch_add_norm_kernel(float* __restrict__ x, BranchSum bs, const T* __restrict__ w, const T* __restrict__ b, float w_offset, float eps,
+__global__ void __launch_bounds__(512) branch_add_norm_kernel(float* __restrict__ x, BranchSum bs, const T* w, const T* b, float w_offset, float eps,
                                                               int W, T* __restrict__ h) {
     pdl_enter();
     __shared__ float scratch[33];
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(512) branch_add_norm_kernel(float* __restrict_
 // The same with four consecutive elements per load, every input of a row requested before the first is used; a thread owns NV groups of four,
 // blockDim.x * NV * 4 >= W.
 template <typename T, int NV>
-__global__ void __launch_bounds__(1024) branch_add_norm_vec_kernel(float* __restrict__ x, BranchSum bs, const T* __restrict__ w, const T* __restrict__ b, float w_offset, float eps,
+__global__ void __launch_bounds__(1024) branch_add_norm_vec_kernel(float* __restrict__ x, BranchSum bs, const T* w, const T* b, float w_offset, float eps,
                                                                    int W, T* __restrict__ h) {
     pdl_enter();
     __shared__ float scratch[33];
@@ -573,8 +573,8 @@ int launch_branch_add_norm(int dt, float* x, const BranchSum& bs, const void* w,
 
 // ---- element-wise norms (tanh(alpha x) w + b): no row statistics, so everything between two sublayers is one pass over the row ----------
 template <typename T>
-__global__ void dyn_tanh_kernel(const float* __restrict__ x, int ldx, const T* __restrict__ w, const T* __restrict__ b, const T* __restrict__ alpha, int W,
-                                float* __restrict__ y, T* __restrict__ y_t, const int32_t* __restrict__ rows) {
+__global__ void dyn_tanh_kernel(const float* x, int ldx, const T* w, const T* b, const T* alpha, int W,
+                                float* __restrict__ y, T* __restrict__ y_t, const int32_t* rows) {
     pdl_enter();
     const int i = blockIdx.x;
     const float* xr = x + (size_t)(rows ? rows[i] : i) * ldx;
@@ -695,9 +695,9 @@ int launch_softcap(float* z, size_t count, float cap, cudaStream_t s) {
 
 // thread per (token, channel)
 template <typename T>
-__global__ void causal_taps_kernel(Batch b, const float* __restrict__ in, int ld_in, const T* __restrict__ w, int taps, int C,
-                                   const float* __restrict__ state, size_t slot_stride, int identity, int silu, T* __restrict__ out_t, int ld_t,
-                                   float* __restrict__ out_f, int ld_f, const T* __restrict__ bias) {
+__global__ void causal_taps_kernel(Batch b, const float* in, int ld_in, const T* w, int taps, int C,
+                                   const float* state, size_t slot_stride, int identity, int silu, T* __restrict__ out_t, int ld_t,
+                                   float* __restrict__ out_f, int ld_f, const T* bias) {
     pdl_enter();
     const int i = blockIdx.x;
     const int sq = b.tok_seq[i];
@@ -722,9 +722,9 @@ __global__ void causal_taps_kernel(Batch b, const float* __restrict__ in, int ld
 // token per thread, 21 so.  Sums in the same order as above.
 constexpr int TR = 8;
 template <typename T, int TAPS>
-__global__ void __launch_bounds__(128) causal_taps_run_kernel(Batch b, const float* __restrict__ in, int ld_in, const T* __restrict__ w, int C, const float* __restrict__ state,
+__global__ void __launch_bounds__(128) causal_taps_run_kernel(Batch b, const float* in, int ld_in, const T* w, int C, const float* state,
                                                               size_t slot_stride, int identity, int silu, T* __restrict__ out_t, int ld_t, float* __restrict__ out_f, int ld_f,
-                                                              const T* __restrict__ bias) {
+                                                              const T* bias) {
     pdl_enter();
     const int c = (blockIdx.y * 128 + threadIdx.x) * 4, i0 = blockIdx.x * TR;
     if (c >= C) return;
@@ -789,7 +789,7 @@ int launch_causal_taps(int dt, const Batch& b, const float* in, int ld_in, const
 
 // thread per (sequence, channel): state[k] <- input at portion index len - (taps - 1) + k, taken from the old state when that is negative.
 // Ascending k is safe in place: entry k reads old entry len + k > k.
-__global__ void taps_state_kernel(Batch b, const float* __restrict__ in, int ld_in, int taps, int C, float* __restrict__ state, size_t slot_stride,
+__global__ void taps_state_kernel(Batch b, const float* in, int ld_in, int taps, int C, float* __restrict__ state, size_t slot_stride,
                                   int skip_single) {
     pdl_enter();
     const int sq = blockIdx.x;
@@ -818,7 +818,7 @@ int launch_taps_state(const Batch& b, const float* in, int ld_in, int taps, int 
 constexpr int NTAPS_MAX = 8;
 
 template <typename T>
-__global__ void norm_taps_kernel(Batch b, const float* __restrict__ x, int ldx, const T* __restrict__ nw, int groups, float eps, const T* __restrict__ cw,
+__global__ void norm_taps_kernel(Batch b, const float* x, int ldx, const T* nw, int groups, float eps, const T* cw,
                                  int taps, int W, float* __restrict__ state, size_t slot_stride, T* __restrict__ out_t, int ld_t, float* __restrict__ hn) {
     pdl_enter();
     __shared__ float red[NTAPS_MAX][33];
@@ -890,7 +890,7 @@ int launch_norm_taps(int dt, const Batch& b, const float* x, int ldx, const void
 
 // ---- the same for many tokens: statistics once per row, then a fully parallel apply ------------------------------------------------
 // inv[row][group] = 1 / sqrt(mean_group(x^2) + eps): one warp per (row, group)
-__global__ void row_group_inv_rms_kernel(const float* __restrict__ x, int ldx, int n, int groups, int gw, float eps, float* __restrict__ inv) {
+__global__ void row_group_inv_rms_kernel(const float* x, int ldx, int n, int groups, int gw, float eps, float* __restrict__ inv) {
     pdl_enter();
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (wid >= n * groups) return;
@@ -905,8 +905,8 @@ __global__ void row_group_inv_rms_kernel(const float* __restrict__ x, int ldx, i
 // thread per (token, 4 channels): the taps over rows normalised with the precomputed statistics (or taken from the carried state).
 // VEC = 4 needs W, the group width and the row strides to be multiples of 4 (one group per thread, 16-byte loads); VEC = 1 takes anything.
 template <typename T, int VEC>
-__global__ void norm_taps_apply_kernel(Batch b, const float* __restrict__ x, int ldx, const float* __restrict__ inv, const T* __restrict__ nw, int groups,
-                                       const T* __restrict__ cw, int taps, int W, const float* __restrict__ state, size_t slot_stride, T* __restrict__ out_t,
+__global__ void norm_taps_apply_kernel(Batch b, const float* x, int ldx, const float* inv, const T* nw, int groups,
+                                       const T* cw, int taps, int W, const float* state, size_t slot_stride, T* __restrict__ out_t,
                                        int ld_t, float* __restrict__ hn) {
     pdl_enter();
     const int i = blockIdx.x;
@@ -966,7 +966,7 @@ int launch_norm_taps_rows(int dt, const Batch& b, const float* x, int ldx, const
 }
 
 template <typename T>
-__global__ void gate_mul_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ g, int ldg, int act, int C, T* __restrict__ y, int ldy) {
+__global__ void gate_mul_kernel(const float* x, int ldx, const float* g, int ldg, int act, int C, T* __restrict__ y, int ldy) {
     pdl_enter();
     const int i = blockIdx.x;
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < C; c += gridDim.y * blockDim.x) {
@@ -984,7 +984,7 @@ int launch_gate_mul(int dt, const float* x, int ldx, const float* g, int ldg, in
 }
 
 template <typename T>
-__global__ void gather_rows_kernel(const T* __restrict__ src, int ld, const int32_t* __restrict__ rows, int W, T* __restrict__ dst) {
+__global__ void gather_rows_kernel(const T* src, int ld, const int32_t* rows, int W, T* __restrict__ dst) {
     pdl_enter();
     const int i = blockIdx.x, r = rows[i];
     for (int c = threadIdx.x; c < W; c += blockDim.x) dst[(size_t)i * W + c] = r >= 0 ? src[(size_t)r * ld + c] : from_f<T>(0.f);
@@ -998,7 +998,7 @@ int launch_gather_rows(int dt, const void* src, int ld, const int32_t* rows, int
 }
 
 template <typename T>
-__global__ void transpose_heads_kernel(const T* __restrict__ in, int R, int C, T* __restrict__ out) {
+__global__ void transpose_heads_kernel(const T* in, int R, int C, T* __restrict__ out) {
     pdl_enter();
     const size_t h = blockIdx.y;
     for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < R * C; idx += gridDim.x * blockDim.x) {
