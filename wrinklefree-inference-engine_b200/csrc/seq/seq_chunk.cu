@@ -591,7 +591,10 @@ int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const floa
     };
     auto scan_pass = [&](int pass) {
         sg.pass = pass;
-        launch_pdl(chunk_scan_kernel<DS, VEC, DELTA, CT>, dim3(b.nseq * sg.n, D.H, (cols + CT - 1) / CT), CR_THREADS, smem, s, b, D, w, state, slot_stride, o, sg);
+        // Behind the end of the kernel before, not by launch_pdl: blocks that come while that kernel still holds most SMs gather on the few that are free, several
+        // to one, and a scan is as slow as its fullest SM.  us by launch_pdl / so: delta rule, 8 heads of 64 x 128, one sequence of 2048 tokens (64 blocks) 300 / 146,
+        // 20 heads of 128 x 128 (160 blocks) 395 / 313; state space, 80 heads of 64 x 64 (160 blocks) 383 / 241, 16 heads, 4 sequences (128 blocks) 104 / 57.
+        chunk_scan_kernel<DS, VEC, DELTA, CT><<<dim3(b.nseq * sg.n, D.H, (cols + CT - 1) / CT), CR_THREADS, smem, s>>>(b, D, w, state, slot_stride, o, sg);
         return launch_check(cudaGetLastError(), "chunk_scan");
     };
     // Segments in parallel where the recurrence is linear in the state, one portion is long and the chains of whole portions leave the machine idle: the two

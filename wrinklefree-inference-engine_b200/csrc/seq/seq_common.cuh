@@ -44,7 +44,7 @@ struct Batch {
     int ctx_total = 0;         // those rows: the sum over sequences of the positions behind the step (known on the host)
 };
 
-// Every kernel of the engine is launched by launch_pdl and begins with pdl_enter (the CTA pairs' product: behind its set-up): its launch overlaps the kernel
+// Every kernel of the engine but the scans of the recurrences is launched by launch_pdl and begins with pdl_enter (the CTA pairs' product: behind its set-up): its launch overlaps the kernel
 // before it in the stream, whose results, and whose reads of what this one overwrites, are complete behind pdl_enter.  A decode step is a chain of some 40
 // kernels of 2 to 6 us, a prompt layer one of 15 to 25, at about 1 us of launch each.  Measured without / with: a decode step of 8 sequences, four layers
 // 182 / 159 us (221 where a kernel lets the next one in before its own wait: the CTAs of several waiting kernels then hold slots); layers 524 / 491, 940 / 918, 1060 / 1019 us.
