@@ -80,7 +80,7 @@ def test_state_space(heads, groups, state, vdim, lens, cuts):
 
 
 @pytest.mark.parametrize("lens,cuts", CUTS)
-@pytest.mark.parametrize("heads,dim,vdim", [(4, 128, 128), (3, 24, 15)])
+@pytest.mark.parametrize("heads,dim,vdim", [(4, 128, 128), (3, 24, 15), (150, 20, 36)])
 def test_matrix_memory(heads, dim, vdim, lens, cuts):
     W = 40
     left = {"heads": 2, "kv_heads": 1, "dim": 8, "vdim": 8, "scale": 0.3, "mask": {"size": 8}, "bias_max": 16}

@@ -221,6 +221,7 @@ constexpr int CR_RS = 24;                                 // row stride of the p
 
 // CT: tiles of 16 columns that a block takes.  The key and query rows that the products need as sums of two numbers are split once for all of them; without the
 // correction that splitting was the larger part of the work (the two passes over 40 heads of 128 x 64, 2048 tokens: 63 + 97 us with one, 48 + 78 with two).
+// Which one: two_tiles.
 template <int DS, bool VEC, bool DELTA, int CT>
 __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
     pdl_enter();
@@ -576,13 +577,32 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_redo_kernel(Batch b, DeltaDi
     if (tid == 0) *mark = 0;
 }
 
+// Whether a recurrence without the correction takes two column tiles a block, where tiles is the number of 16-column tiles and pairs that of blocks of two.  A scan
+// takes as long as its fullest SM.  us a chunk with n blocks there, 128-row states: one tile a block 1.2, 1.7, 2.5, 3.3, 4.4 (n = 1 .. 5), two tiles 1.5, 2.6, 3.9.
+// So 16 heads of 128 x 64 (64 tiles), one sequence of 256 tokens 36 / 41 us, 40 heads, 2 sequences of 2048 (320 tiles) 317 / 338, but 4 of 1024 (640) 287 / 259;
+// an odd tile is a block of its own: matrix memory, 16 heads of 64 x 129, 4 of 1024 (576 tiles, 320 pairs) 147 / 163.
+bool two_tiles(long long tiles, long long pairs) {
+    const long long sms = sm_count(), one = (tiles + sms - 1) / sms, two = (pairs + sms - 1) / sms;
+    return 3 * two < 2 * one;
+}
+
 template <int DS, bool VEC, bool DELTA, int CT>
-int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const float* decay, float* state, size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan) {
-    launch_pdl(chunk_prep_kernel<DS, VEC, DELTA>, dim3(b.nseq * w.nchunks, D.H), CR_THREADS, 0, s, b, D, w);
-    if (int rc = launch_check(cudaGetLastError(), "chunk_prep")) return rc;
+int cr_scan(const Batch& b, const DeltaDims& D, const ChunkView& w, float* state, size_t slot_stride, float* o, const Segments& sg, cudaStream_t s) {
+    const int cols = w.cols;
     constexpr size_t smem = (size_t)(2 * CrStage<DS, VEC, DELTA>::FLOATS + CR_WARPS * (DELTA ? 2 * CT : 2) * CR_COLS * CR_RS) * sizeof(float);
     static DevOnce once;
     if (once.need() && cuda_check(cudaFuncSetAttribute(chunk_scan_kernel<DS, VEC, DELTA, CT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "chunk shared memory")) return WF_ERR_CUDA;
+    // Behind the end of the kernel before, not by launch_pdl: blocks that come while that kernel still holds most SMs gather on the few that are free, several
+    // to one, and a scan is as slow as its fullest SM.  us by launch_pdl / so: delta rule, 8 heads of 64 x 128, one sequence of 2048 tokens (64 blocks) 300 / 146,
+    // 20 heads of 128 x 128 (160 blocks) 395 / 313; state space, 80 heads of 64 x 64 (160 blocks) 383 / 241, 16 heads, 4 sequences (128 blocks) 104 / 57.
+    chunk_scan_kernel<DS, VEC, DELTA, CT><<<dim3(b.nseq * sg.n, D.H, (cols + CT - 1) / CT), CR_THREADS, smem, s>>>(b, D, w, state, slot_stride, o, sg);
+    return launch_check(cudaGetLastError(), "chunk_scan");
+}
+
+template <int DS, bool VEC, bool DELTA>
+int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const float* decay, float* state, size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan) {
+    launch_pdl(chunk_prep_kernel<DS, VEC, DELTA>, dim3(b.nseq * w.nchunks, D.H), CR_THREADS, 0, s, b, D, w);
+    if (int rc = launch_check(cudaGetLastError(), "chunk_prep")) return rc;
     Segments sg;
     const int cols = w.cols;
     auto redo = [&]() {
@@ -591,15 +611,16 @@ int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const floa
     };
     auto scan_pass = [&](int pass) {
         sg.pass = pass;
-        // Behind the end of the kernel before, not by launch_pdl: blocks that come while that kernel still holds most SMs gather on the few that are free, several
-        // to one, and a scan is as slow as its fullest SM.  us by launch_pdl / so: delta rule, 8 heads of 64 x 128, one sequence of 2048 tokens (64 blocks) 300 / 146,
-        // 20 heads of 128 x 128 (160 blocks) 395 / 313; state space, 80 heads of 64 x 64 (160 blocks) 383 / 241, 16 heads, 4 sequences (128 blocks) 104 / 57.
-        chunk_scan_kernel<DS, VEC, DELTA, CT><<<dim3(b.nseq * sg.n, D.H, (cols + CT - 1) / CT), CR_THREADS, smem, s>>>(b, D, w, state, slot_stride, o, sg);
-        return launch_check(cudaGetLastError(), "chunk_scan");
+        const long long chains = (long long)b.nseq * sg.n * D.H, tiles = chains * cols;
+        // With the correction two column tiles a block are the longer chain and the lesser work from four blocks an SM on: us with one / two, 20 heads of 128 x 128
+        // in one sequence (160 tiles) 351 / 387, 2 (320) 192 / 208, 4 (640) 186 / 171.
+        const bool two = DELTA ? tiles > 4LL * sm_count() : two_tiles(tiles, chains * ((cols + 1) / 2));
+        return two ? cr_scan<DS, VEC, DELTA, 2>(b, D, w, state, slot_stride, o, sg, s) : cr_scan<DS, VEC, DELTA, 1>(b, D, w, state, slot_stride, o, sg, s);
     };
     // Segments in parallel where the recurrence is linear in the state, one portion is long and the chains of whole portions leave the machine idle: the two
-    // passes cost half as much work again.  us, whole -> segments: 4 heads 128 x 64, 1024 tokens 87 -> 40, 300 tokens 35 -> 36; 16 heads, 2048 tokens 168 -> 95;
-    // 40 heads (160 blocks) 224 -> 202; two sequences of 841 and 1207, 16 heads (128 blocks) 109 -> 102, 40 heads (320 blocks) 185 -> 206.
+    // passes cost half as much work again.  us, whole -> segments, each with the better number of tiles a block: 4 heads of 128 x 64, 1024 tokens 88 -> 40, 600 tokens
+    // 59 -> 39; 16 heads, 2048 tokens 171 -> 93; 40 heads (160 tiles) 230 -> 175; 24 heads, 2 sequences of 1024 (192 tiles) 126 -> 121, 16 heads, 4 sequences of
+    // 1024 (256 tiles) 131 -> 147.
     if (DELTA || !scan->local || b.max_len < 4 * SCAN_CHUNK || b.n / SCAN_CHUNK + b.nseq + 1 > scan->chunks || 2LL * b.nseq * D.H * cols >= 3LL * sm_count())
     {
         if (int rc = scan_pass(0)) return rc;
@@ -636,12 +657,9 @@ int launch_chunk_recurrence(const Batch& b, const DeltaDims& D, const float* qkv
     w.q_off = D.q_off >= 0 ? D.q_off : 0; w.k_off = D.k_off >= 0 ? D.k_off : D.Hk * D.d; w.v_off = D.v_off >= 0 ? D.v_off : 2 * D.Hk * D.d;
     w.redo = scan->redo; w.cols = (D.dv + D.ones_col + CR_COLS - 1) / CR_COLS;
     w.rec = scan->rec; w.nchunks = (b.max_len + CR - 1) / CR;
-#define CR_PICK(vec, delta, ct) (D.d <= 64 ? cr_launch<64, vec, delta, ct>(b, D, w, decay, state, slot_stride, o, s, scan) : cr_launch<128, vec, delta, ct>(b, D, w, decay, state, slot_stride, o, s, scan))
-    if (D.no_delta) return D.vec_decay ? CR_PICK(true, false, 2) : CR_PICK(false, false, 2);
-    // With the correction two column tiles a block are the longer chain and the lesser work: us with one / two, 20 heads of 128 x 128 in 1 sequence (160 blocks
-    // of one) 351 / 387, 2 (320) 192 / 208, 4 (640) 186 / 171.
-    if ((long long)b.nseq * D.H * w.cols > 4LL * sm_count()) return D.vec_decay ? CR_PICK(true, true, 2) : CR_PICK(false, true, 2);
-    return D.vec_decay ? CR_PICK(true, true, 1) : CR_PICK(false, true, 1);
+#define CR_PICK(vec, delta) (D.d <= 64 ? cr_launch<64, vec, delta>(b, D, w, decay, state, slot_stride, o, s, scan) : cr_launch<128, vec, delta>(b, D, w, decay, state, slot_stride, o, s, scan))
+    if (D.no_delta) return D.vec_decay ? CR_PICK(true, false) : CR_PICK(false, false);
+    return D.vec_decay ? CR_PICK(true, true) : CR_PICK(false, true);
 #undef CR_PICK
 }
 
