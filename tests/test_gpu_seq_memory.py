@@ -67,3 +67,25 @@ def test_logits_reach_pageable_memory_as_they_reach_pinned(vocab, wants):
         m.release(slot)
         assert np.isfinite(got).all() and np.array_equal(got, pinned.numpy()), n
     m.close()
+
+
+def test_a_large_block_table_is_not_page_locked():
+    """32 slots x 16,384 pages, a table of 2 MB: the same tokens as with a small table, over steps that add pages and that do not."""
+    from test_gpu_tutizen import attn, build, config, make_weights, with_ff, dense
+    cfg = config([with_ff(attn(), dense())], vocab=70)
+    w = make_weights(cfg, 3)
+    outs = []
+    for pages in (64, 16384):
+        m = build(cfg, w, "bfloat16", max_tokens=pages * 4, slots=32, page_size=4, max_step_tokens=64)
+        assert m.engine.free_pages() == pages
+        a, b = m.admit(), m.admit()
+        rng = np.random.default_rng(1)
+        got = []
+        for counts in ([13, 5], [1, 1], [2, 1], [1, 1], [30, 9]):
+            got.append(m.step([a, b], counts, rng.integers(0, 70, sum(counts)).astype(np.int32), np.arange(sum(counts), dtype=np.int32)))
+        m.release(a)
+        c = m.admit()
+        got.append(m.step([b, c], [3, 20], rng.integers(0, 70, 23).astype(np.int32), np.arange(23, dtype=np.int32)))
+        outs.append(np.concatenate(got))
+        m.close()
+    assert np.isfinite(outs[0]).all() and np.array_equal(outs[0], outs[1])

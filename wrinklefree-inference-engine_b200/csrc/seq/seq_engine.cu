@@ -19,6 +19,7 @@ using namespace wf::seq;
 
 namespace {
 
+constexpr size_t TABLE_PINNED = 1024 * 1024;      // block tables up to this size travel with the step's index arrays, from page-locked memory
 constexpr int OUT_CHUNKS = 4;
 constexpr size_t OUT_CHUNK = 512 * 1024;
 
@@ -110,8 +111,9 @@ struct wf_seq_engine {
     size_t slot_stride = 0;           // floats per slot
     int32_t* d_block_table = nullptr;
     // step metadata
-    int32_t *h_meta = nullptr, *d_meta = nullptr;   // the step's index arrays, and behind them the block table; pinned on the host
+    int32_t *h_meta = nullptr, *d_meta = nullptr;   // the step's index arrays, and behind them the block table; pinned on the host (a large table is not)
     size_t meta_ints = 0;
+    bool table_pinned = false;
     bool staged = false;              // a copy from h_meta may be under way: the step that issued it has not been waited for
     // logits on their way to the caller's memory, and the tcgen05 kernels' error word: pinned, OUT_CHUNKS pieces in turn
     unsigned char* h_out = nullptr;
@@ -443,12 +445,19 @@ int prepare_step(wf_seq_engine* e, int nseq, const int32_t* slots, const int32_t
     }
     v->b.ctx_total = (int)ctx;                      // at most the pool's tokens
     size_t ints = e->meta_ints;
-    if (e->pt.dirty) {                              // the block table goes with them
+    if (e->pt.dirty && e->table_pinned) {           // the block table goes with them
         for (int32_t p : e->pt.table) m[ints++] = p < 0 ? 0 : p;      // a stale lookup can never leave the pool
         e->pt.dirty = false;
     }
     e->staged = true;
     if (cuda_check(cudaMemcpyAsync(e->d_meta, m, ints * 4, cudaMemcpyHostToDevice, e->stream), "step metadata H2D")) { e->pt.dirty = true; return WF_ERR_CUDA; }
+    if (e->pt.dirty) {                              // a table that would hold too much of the host's memory locked: through a copy that ends here
+        std::vector<int32_t> tmp(e->pt.table);
+        for (auto& p : tmp) if (p < 0) p = 0;
+        if (cuda_check(cudaMemcpyAsync(e->d_block_table, tmp.data(), tmp.size() * 4, cudaMemcpyHostToDevice, e->stream), "block table H2D") ||
+            cuda_check(cudaStreamSynchronize(e->stream), "sync")) return WF_ERR_CUDA;
+        e->pt.dirty = false;
+    }
     int32_t* d = e->d_meta;
     v->tokens = d;
     v->b.n = n; v->b.nseq = nseq;
@@ -1589,7 +1598,8 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     const size_t with_table = e->meta_ints + (size_t)c.slots * max_blocks;
     TRY(dalloc_n(e, &e->d_meta, with_table));
     e->d_block_table = e->d_meta + e->meta_ints;
-    const size_t meta_bytes = (with_table * 4 + 63) / 64 * 64;         // one pinned allocation (three made a state 2 ms slower to create): arrays and table, pieces of results, error word
+    e->table_pinned = (with_table - e->meta_ints) * 4 <= TABLE_PINNED;
+    const size_t meta_bytes = ((e->table_pinned ? with_table : e->meta_ints) * 4 + 63) / 64 * 64;         // one pinned allocation (three made a state 2 ms slower to create): arrays and table, pieces of results, error word
     if (cuda_check(cudaMallocHost((void**)&e->h_meta, meta_bytes + OUT_CHUNKS * OUT_CHUNK + 64), "pinned step memory")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
     e->h_out = (unsigned char*)e->h_meta + meta_bytes;
     e->h_err = (int*)(e->h_out + OUT_CHUNKS * OUT_CHUNK);
