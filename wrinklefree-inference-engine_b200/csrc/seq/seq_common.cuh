@@ -49,6 +49,15 @@ struct Batch {
 // kernels of 2 to 6 us, a prompt layer one of 15 to 25, at about 1 us of launch each.  Measured without / with: a decode step of 8 sequences, four layers
 // 182 / 159 us (221 where a kernel lets the next one in before its own wait: the CTAs of several waiting kernels then hold slots); layers 524 / 491, 940 / 918, 1060 / 1019 us.
 __device__ __forceinline__ void pdl_enter() { pdl_wait_prior(); pdl_launch_dependents(); }
+// Kernels of one short block a row do so (their last argument) up to eight blocks an SM: the two instructions cost a block some 0.5 us, which beyond that is more than
+// the overlap gives.  16128 padded rows of a routed feed-forward: their activation (384 wide) 22.5 us with them, 16 without; plan and gathering (2560 wide) 28.5 / 23.
+inline bool few_blocks(dim3 grid) { return (long long)grid.x * grid.y * grid.z <= 8LL * sm_count(); }
+template <typename... P, typename... A>
+inline cudaError_t launch_rows(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+    if (few_blocks(grid)) return launch_pdl(kernel, grid, block, smem, s, std::forward<A>(args)..., true);
+    kernel<<<grid, block, smem, s>>>(std::forward<A>(args)..., false);
+    return cudaPeekAtLastError();
+}
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

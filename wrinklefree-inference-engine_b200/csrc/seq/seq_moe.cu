@@ -195,8 +195,8 @@ __global__ void moe_plan_kernel(RouterDims R, int n, const int32_t* ids, const i
 
 // VEC = 4: ff a multiple of 4 (16-byte loads of the gate and up halves)
 template <typename T, int VEC>
-__global__ void silu_mul_kernel(const float* gu, int ff, const int32_t* tile_group, T* __restrict__ hmid, int act, float limit) {
-    pdl_enter();
+__global__ void silu_mul_kernel(const float* gu, int ff, const int32_t* tile_group, T* __restrict__ hmid, int act, float limit, bool overlap) {
+    if (overlap) pdl_enter();
     const int r = blockIdx.x;
     if (tile_group && tile_group[r / GEMM_BM] < 0) return;
     const float* row = gu + (size_t)r * (act == 3 ? 1 : 2) * ff;
@@ -319,8 +319,8 @@ int launch_silu_mul(int dt, const float* gu, int P, int ff, const int32_t* tile_
     const bool vec = ff % 4 == 0 && (((uintptr_t)gu) & 15) == 0;
     const int per = 128 * (vec ? 4 : 1);
     const dim3 grid(P, P < 256 ? (ff + per - 1) / per : 1);
-    if (dt == WF_BF16) { if (vec) launch_pdl(silu_mul_kernel<__nv_bfloat16, 4>, grid, 128, 0, s, gu, ff, tile_group, (__nv_bfloat16*)hmid, act, limit); else launch_pdl(silu_mul_kernel<__nv_bfloat16, 1>, grid, 128, 0, s, gu, ff, tile_group, (__nv_bfloat16*)hmid, act, limit); }
-    else { if (vec) launch_pdl(silu_mul_kernel<float, 4>, grid, 128, 0, s, gu, ff, tile_group, (float*)hmid, act, limit); else launch_pdl(silu_mul_kernel<float, 1>, grid, 128, 0, s, gu, ff, tile_group, (float*)hmid, act, limit); }
+    if (dt == WF_BF16) { if (vec) launch_rows(silu_mul_kernel<__nv_bfloat16, 4>, grid, 128, 0, s, gu, ff, tile_group, (__nv_bfloat16*)hmid, act, limit); else launch_rows(silu_mul_kernel<__nv_bfloat16, 1>, grid, 128, 0, s, gu, ff, tile_group, (__nv_bfloat16*)hmid, act, limit); }
+    else { if (vec) launch_rows(silu_mul_kernel<float, 4>, grid, 128, 0, s, gu, ff, tile_group, (float*)hmid, act, limit); else launch_rows(silu_mul_kernel<float, 1>, grid, 128, 0, s, gu, ff, tile_group, (float*)hmid, act, limit); }
     return launch_check(cudaGetLastError(), "silu_mul");
 }
 

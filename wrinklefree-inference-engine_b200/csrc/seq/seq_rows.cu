@@ -984,16 +984,16 @@ int launch_gate_mul(int dt, const float* x, int ldx, const float* g, int ldg, in
 }
 
 template <typename T>
-__global__ void gather_rows_kernel(const T* src, int ld, const int32_t* rows, int W, T* __restrict__ dst) {
-    pdl_enter();
+__global__ void gather_rows_kernel(const T* src, int ld, const int32_t* rows, int W, T* __restrict__ dst, bool overlap) {
+    if (overlap) pdl_enter();
     const int i = blockIdx.x, r = rows[i];
     for (int c = threadIdx.x; c < W; c += blockDim.x) dst[(size_t)i * W + c] = r >= 0 ? src[(size_t)r * ld + c] : from_f<T>(0.f);
 }
 
 int launch_gather_rows(int dt, const void* src, int ld, const int32_t* rows, int P, int W, void* dst, cudaStream_t s) {
     if (P <= 0) return WF_OK;
-    if (dt == WF_BF16) launch_pdl(gather_rows_kernel<__nv_bfloat16>, P, 256, 0, s, (const __nv_bfloat16*)src, ld, rows, W, (__nv_bfloat16*)dst);
-    else launch_pdl(gather_rows_kernel<float>, P, 256, 0, s, (const float*)src, ld, rows, W, (float*)dst);
+    if (dt == WF_BF16) launch_rows(gather_rows_kernel<__nv_bfloat16>, P, 256, 0, s, (const __nv_bfloat16*)src, ld, rows, W, (__nv_bfloat16*)dst);
+    else launch_rows(gather_rows_kernel<float>, P, 256, 0, s, (const float*)src, ld, rows, W, (float*)dst);
     return launch_check(cudaGetLastError(), "gather_rows");
 }
 
