@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D
                                                            float* __restrict__ gate) {
     pdl_enter();
     __shared__ float rot_c[64], rot_s[64];
-    const int i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = 4 * lane;
+    const int i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, c = 4 * lane;
     const int sq = b.tok_seq[i], pos = b.tok_pos[i];
     const float* row = proj + (size_t)i * ld;
     const int units = D.H + (k_off >= 0 ? (D.v_is_k ? D.G : 2 * D.G) : 0);
@@ -147,11 +147,11 @@ __global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D
     }
     const int slot = pos % pc.page_size, half = D.rope_dims / 2;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int u0 = warp; u0 == warp || u0 < units; u0 += 8 * GQ) {         // every warp comes by the barrier
+    for (int u0 = warp; u0 == warp || u0 < units; u0 += nw * GQ) {         // every warp comes by the barrier
         float4 x[GQ], bi[GQ];
 #pragma unroll
         for (int k = 0; k < GQ; ++k) {
-            const int u = u0 + 8 * k, g = u - D.H - (u >= D.H + D.G ? D.G : 0);
+            const int u = u0 + nw * k, g = u - D.H - (u >= D.H + D.G ? D.G : 0);
             const bool isq = u < D.H, isk = !isq && u < D.H + D.G;
             const int dim = isq || isk ? D.d : D.dv;
             const bool in = u < units && c < dim;
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D
                 sincos(a, &sn, &cs);
                 rot_c[threadIdx.x] = (float)cs * D.mscale; rot_s[threadIdx.x] = (float)sn * D.mscale;
             } else if (gate && t >= 0) {
-                const int ng = D.gate_elem ? D.H * D.dv : D.H, nt = 256 - table;
+                const int ng = D.gate_elem ? D.H * D.dv : D.H, nt = (int)blockDim.x - table;
                 if (ng % 4 == 0 && g_off % 4 == 0 && g_off >= 0) {
                     for (int h = t * 4; h < ng; h += nt * 4) {
                         const float4 z = load4(row + g_off + h);
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D
         }
 #pragma unroll
         for (int k = 0; k < GQ; ++k) {
-            const int u = u0 + 8 * k;
+            const int u = u0 + nw * k;
             if (u >= units) break;
             const bool isq = u < D.H, isk = !isq && u < D.H + D.G;
             const int g = isq ? u : u - D.H - (isk ? 0 : D.G), dim = isq || isk ? D.d : D.dv;
@@ -416,8 +416,13 @@ int launch_gqa_prep(int dt, const Batch& b, const GqaDims& D, const float* proj,
     if (small && D.d % 4 == 0 && D.dv % 4 == 0 && D.qk_norm < 3 && (D.rope_interleaved || D.rope_dims % 8 == 0) && ld % 4 == 0 && (k_off < 0 || (k_off % 4 == 0 && (D.v_is_k || v_off % 4 == 0))) &&
         (k_off < 0 || (pc.layer_off % 4 == 0 && pc.page_stride % 4 == 0 && vec_ok(pc.pool, 16))) && vec_ok(proj, 16) && vec_ok(qb, 16) && vec_ok(kb, 16) && vec_ok(vb, 16) && vec_ok(qn, 16) && vec_ok(gate, 16) &&
         vec_ok(D.q_norm_w, 16) && vec_ok(D.k_norm_w, 16)) {
-        if (dt == WF_BF16) launch_pdl(gqa_prep_vec_kernel<__nv_bfloat16>, b.n, 256, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const __nv_bfloat16*)qb, (const __nv_bfloat16*)kb, (const __nv_bfloat16*)vb, eps, pc, (__nv_bfloat16*)qn, gate);
-        else launch_pdl(gqa_prep_vec_kernel<float>, b.n, 256, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const float*)qb, (const float*)kb, (const float*)vb, eps, pc, (float*)qn, gate);
+        // Warps a token: eight while the tokens' latency counts (300 tokens, 8 + 2 heads of 64: 10.5 us, 10.6 with four) or there are vectors for them (4096 tokens, 20 + 5
+        // heads of 128 72, 77 with four); else fewer, so that more tokens are resident while their double-precision cosines are formed: 4096 tokens, 8 + 2 heads of 64
+        // 34.7 / 26.9 with four, 4 + 1 heads 28.9 / 20.7 and 18.9 with three (the cosines of 64 pairs take two, the gates the third).
+        const int units = D.H + (k_off >= 0 ? (D.v_is_k ? 1 : 2) * D.G : 0);
+        const int threads = b.n <= 4 * sm_count() || units > 24 ? 256 : units > 8 ? 128 : 96;
+        if (dt == WF_BF16) launch_pdl(gqa_prep_vec_kernel<__nv_bfloat16>, b.n, threads, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const __nv_bfloat16*)qb, (const __nv_bfloat16*)kb, (const __nv_bfloat16*)vb, eps, pc, (__nv_bfloat16*)qn, gate);
+        else launch_pdl(gqa_prep_vec_kernel<float>, b.n, threads, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const float*)qb, (const float*)kb, (const float*)vb, eps, pc, (float*)qn, gate);
         return launch_check(cudaGetLastError(), "gqa_prep_vec");
     }
     const int threads = 32 * (b.n <= sm_count() ? GP_MAXW : GA_WARPS);
