@@ -596,28 +596,35 @@ static int launch_tc_split(const wf_linear_args* a, const EpiParams& ep, int ksp
     return launch_check(cudaLaunchKernelEx(&cfg, ternary_gemm_tc_kernel<NU, true>, tmap, p), "ternary_gemm_tc(split)");
 }
 
-// This file's forms against CTA pairs (gemm_tc_pair.cu), by what each is expected to take.  Measured over N 2560 .. 14336, K 2560 .. 14336, 20 .. 4000 tokens
-// (us, this file / pairs):
-//   * K shared by a cluster: 0.25 us a k-block, 0.1 us per token that a CTA finishes: 4096 x 14336, 48 tokens 15.7 / 27.8; 2560 x 6912, 128 tokens 13.6 / 17.1;
-//     but 6912 x 2560, 48 tokens 12.3 / 10.6;
-//   * one CTA a tile: 0.26 us a k-block and round of tiles, and 4.5 us for an epilogue with missing tokens: 2560 x 2560, 512 tokens 10.4 / 11.4;
-//     14336 x 4096, 128 tokens 13.3 / 13.9, 96 tokens 17.1 / 13.3; 2560 x 6912, 1024 tokens 31.2 / 20.9.
-// relu^2 * up without a cluster: its epilogue here takes 14 us a tile (13824 x 2560, 512 tokens 43 / 24).
-static double tile_time(int M, int KB, int tiles, int ksplit, int sms, bool relu2) {
-    if (ksplit > 1) return 6.7 + 0.25 * ((KB + ksplit - 1) / ksplit) + 0.1 * (M < TC_BN ? M : TC_BN) / ksplit;
+// This file's forms against CTA pairs (gemm_tc_pair.cu), by what each is expected to take: fitted to both, measured back to back over 17 matrices of N 256 .. 28672 and
+// K 128 .. 28672 with 17 .. 4096 tokens, packed and tile layout, float, bf16 and gated results (1008 products).  The rule takes the faster form, or one within
+// 3 % of it, for all but 18 of them.  us, this file / pairs:
+//   * K shared by a cluster: 0.28 us a k-block, 0.11 us per token that a CTA finishes (0.05 where the results are gated, whole numbers or scaled by one factor): 4096 x 14336, 64 tokens 15.6 / 30.8; 2560 x 6912, 128 tokens
+//     13.2 / 18.2, gated 192 tokens 16.1 / 18.8; but 6912 x 2560, 64 tokens 11.8 / 10.5; 16 clusters of 8 and more take a second round: 1024 x 4096, 256 tokens 19.1 / 13.2;
+//   * one CTA a tile: 0.263 us a k-block and round of tiles, 2.9 us (1.4) for an epilogue with missing tokens: 2560 x 6912, 512 tokens 17.3 / 19.4; 13824 x 2560, 128 tokens
+//     10.3 / 11.7, 96 tokens 13.9 / 11.3; 2560 x 6912, 1024 tokens 31.2 / 20.9; gated, 10 us a tile more: 13824 x 2560, 512 tokens 42 / 24.
+static double tile_time(int M, int KB, int tiles, int ksplit, int sms, bool relu2, bool linear) {
+    if (ksplit > 1) return 5.9 + 0.28 * ((KB + ksplit - 1) / ksplit) + (relu2 || !linear ? 0.05 : 0.11) * (M < TC_BN ? M : TC_BN) / ksplit + (ksplit == 8 && tiles >= 16 ? 8. : 0.);
     const int rounds = (tiles + sms - 1) / sms;
-    return 4.7 + 0.26 * rounds * KB + (M % TC_EP_TOKS ? 4.5 : 0.) + (relu2 ? 10. * rounds : 0.);
+    return 4.6 + 0.263 * rounds * KB + (M % TC_BN ? (linear ? 2.9 : 1.4) : 0.) + (relu2 ? 10. * rounds : 0.);
+}
+
+// tokens a tile on CTA pairs, 0: this file's forms, sharing K over clusters of *ksplit
+static int choose_form(int M, int N, int K, int out_mode, int epi_flags, int* ksplit) {
+    const bool linear = out_mode == WF_OUT_LINEAR, relu2 = linear && (epi_flags & WF_EPI_RELU2_MUL);
+    const int tiles = ((N + TC_BM - 1) / TC_BM) * ((M + TC_BN - 1) / TC_BN), sms = sm_count();
+    int ks = 1;
+    while (ks < 8 && tiles * ks * 2 <= sms && K / WF_QK >= ks * 2 * 4) ks *= 2;
+    *ksplit = ks;
+    return gemm_tc_pair_time(M, N, K, relu2) < tile_time(M, K / WF_QK, tiles, ks, sms, relu2, linear) ? gemm_tc_pair_tokens(M, N, K) : 0;
 }
 
 int launch_gemm_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s) {
     gemm_tc_init_attrs();
     if (!g_encode) { set_error("gemm_tc: tcgen05 path unavailable (driver entry point / smem attribute)"); return WF_ERR_CUDA; }
-    const int tiles = ((a->N + TC_BM - 1) / TC_BM) * ((a->M + TC_BN - 1) / TC_BN), sms = sm_count();
-    int ksplit = 1;
-    while (ksplit < 8 && tiles * ksplit * 2 <= sms && a->K / WF_QK >= ksplit * 2 * 4) ksplit *= 2;
-    const bool relu2 = ep.out_mode == WF_OUT_LINEAR && (ep.epi_flags & WF_EPI_RELU2_MUL);
+    int ksplit;
     // (where the host memory that pairs report to cannot be had, the forms of this file, whose waits have no limit)
-    if (gemm_tc_pair_time(a->M, a->N, a->K) < tile_time(a->M, a->K / WF_QK, tiles, ksplit, sms, relu2) && tc_wait_word()) return launch_gemm_tc_pair(a, ep, s);
+    if (choose_form(a->M, a->N, a->K, ep.out_mode, ep.epi_flags, &ksplit) && tc_wait_word()) return launch_gemm_tc_pair(a, ep, s);
     if (ksplit > 1) return launch_tc_split(a, ep, ksplit, s);
     if (g_tc_nu == 1) return launch_tc<1>(a, ep, s);
     return g_tc_nu == 2 ? launch_tc<2>(a, ep, s) : launch_tc<3>(a, ep, s);

@@ -53,8 +53,9 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn tc_encoder();   // cuTensorMapEncodeTiled, or null where the driver has none
 
-// CTA-pair form (gemm_tc_pair.cu) and the time (us) that it is expected to take
-double gemm_tc_pair_time(int M, int N, int K);
+// CTA-pair form (gemm_tc_pair.cu), the tokens of its tiles and the time (us) that it is expected to take
+int gemm_tc_pair_tokens(int M, int N, int K);
+double gemm_tc_pair_time(int M, int N, int K, bool relu2);
 int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s);
 
 }  // namespace wf

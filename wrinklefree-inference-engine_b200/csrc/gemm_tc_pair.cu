@@ -488,9 +488,12 @@ int check_wait_word(const char* who) {
     return WF_OK;
 }
 
-double gemm_tc_pair_time(int M, int N, int K) {
-    const int pairs = sm_count() / 2;
-    return pair_time(M, N, K / WF_QK, tokens_per_tile(M, N, K / WF_QK, pairs), pairs);
+int gemm_tc_pair_tokens(int M, int N, int K) { return tokens_per_tile(M, N, K / WF_QK, sm_count() / 2); }
+
+double gemm_tc_pair_time(int M, int N, int K, bool relu2) {
+    const int pairs = sm_count() / 2, tn = gemm_tc_pair_tokens(M, N, K);
+    const long long tiles = (long long)((N + 2 * TP_ROWS - 1) / (2 * TP_ROWS)) * ((M + tn - 1) / tn);
+    return pair_time(M, N, K / WF_QK, tn, pairs) + (relu2 ? 0.4 * (double)((tiles + pairs - 1) / pairs) : 0.);      // the pairs' exchange of gate and up
 }
 
 int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s) {
