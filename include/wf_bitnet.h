@@ -132,6 +132,8 @@ int wf_ternary_linear_scales(const wf_linear_args* args, const float* w_scales, 
  * whose host address this is (null where there is no device or no such word).  The next ternary product on the device, and the engine's waits, clear the word
  * and return WF_ERR_CUDA; a caller that replays a graph of such products can look at the word itself once the replay has ended. */
 int* wf_wait_word(void);
+/* How algo 3 takes a product (out_mode, epi_flags as in wf_linear_args): the tokens of a tile on CTA pairs, 0 for one CTA a tile. */
+int wf_gemm_tc_pair_tokens(int M, int N, int K, int out_mode, int epi_flags);
 /* What wf_bitnet_gemv / wf_bitnet_gemm (and wf_ternary_linear with algo 0 beyond 8 rows) can use of a workspace for this shape: at most
  * wf_linear_workspace_bytes, 0 where the kernel they choose needs none. */
 size_t wf_bitnet_gemm_workspace_bytes(int M, int N, int K);

@@ -67,6 +67,17 @@ def test_delta_rule_of_many_heads(heads, kv_heads, dim, vdim):
     check(cfg, w, {"l0.mix.a1": (8, W), "l0.mix.g1": (8, W)}, lambda x: NO.channel_delta(x, d64(w, "l0.mix."), "", m, EPS), [90, 64], [[32, 17], [15, 47], [43, 0]], W)
 
 
+@pytest.mark.parametrize("conv", [2, 3])
+def test_convolutions_of_two_and_three_taps_over_many_tokens(conv):
+    """Enough tokens x channels (6400) that a thread of the convolution takes eight tokens one after another: portions that begin and end inside such a run, behind a carried
+    state of one and two inputs, and a portion of one token."""
+    W = 40
+    m = {"heads": 40, "kv_heads": 20, "dim": 64, "vdim": 96, "conv": conv}
+    cfg = {"architecture": "Nukezen", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": EPS}, "layers": [{"type": "channel_delta", "mixer": m, "mlp": None}]}
+    w = NO.random_weights(cfg, 1, {0: {"rank_a": 8, "rank_g": 8}})
+    check(cfg, w, {"l0.mix.a1": (8, W), "l0.mix.g1": (8, W)}, lambda x: NO.channel_delta(x, d64(w, "l0.mix."), "", m, EPS), [391, 203], [[190, 1], [1, 199], [200, 3]], W)
+
+
 @pytest.mark.parametrize("lens,cuts", CUTS)
 @pytest.mark.parametrize("heads,groups,state,vdim", [(4, 2, 128, 64), (6, 3, 20, 12), (80, 5, 64, 64)])
 def test_state_space(heads, groups, state, vdim, lens, cuts):

@@ -144,16 +144,20 @@ def test_tc_shared_k_range(m, nk):
         assert torch.equal(got, torch.relu(g).square() * u)
 
 
-# 32 .. 256 tokens per tile of CTA pairs: one k-block, partial loads of four k-blocks, one and several rounds of tiles, rows and tokens that end inside a tile
-PAIR_SHAPES = [(256, 128, 40), (272, 640, 33), (131, 384, 190), (2560, 2560, 200), (6912, 2560, 75), (4090, 1152, 777), (6905, 2560, 1987), (2560, 6912, 1500),
-               (13824, 2560, 300)]
+# (N, K, tokens, tokens per tile of CTA pairs): every width; one k-block, a last weight load of one, two, three and four k-blocks; one round of tiles and several, at both depths of
+# the operand ring (192 tokens and 256); rows and tokens that end inside a tile
+PAIR_SHAPES = [(256, 128, 40, 32), (272, 640, 33, 32), (131, 384, 190, 32), (2560, 2560, 200, 32), (6912, 2560, 75, 64), (4090, 1152, 777, 96), (6912, 1152, 500, 128),
+               (6905, 2560, 1987, 160), (13824, 2560, 300, 160), (8192, 896, 2500, 160), (6912, 128, 4000, 192), (6912, 640, 4000, 192), (2560, 6912, 1500, 256),
+               (2560, 6912, 2700, 256)]
 
 
 @pytest.mark.parametrize("nkm", PAIR_SHAPES)
 def test_tc_pairs(nkm):
     """Every kind of output on CTA pairs, both weight layouts, bit-equal to the mma.sync kernel; accumulators of a sample of rows equal to the oracle's."""
     from wf_bitnet import ops
-    n, k, m = nkm
+    from wf_bitnet._lib import lib
+    n, k, m, tokens = nkm
+    assert lib().wf_gemm_tc_pair_tokens(m, n, k, 3, 0) == tokens              # linear results
     rng = np.random.default_rng(n + k + m)
     q = torch.from_numpy(rng.integers(-128, 128, size=(m, k)).astype(np.int8)).cuda()
     code = rng.integers(0, 3, size=(n, k // 128, 4, 32)).astype(np.uint8)

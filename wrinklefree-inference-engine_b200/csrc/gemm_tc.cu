@@ -631,3 +631,8 @@ int launch_gemm_tc(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s)
 }
 
 }  // namespace wf
+
+extern "C" int wf_gemm_tc_pair_tokens(int M, int N, int K, int out_mode, int epi_flags) {
+    int ksplit;
+    return M > 0 && N > 0 && K >= WF_QK ? wf::choose_form(M, N, K, out_mode, epi_flags, &ksplit) : 0;
+}

@@ -72,6 +72,7 @@ SYMBOLS = {
     "wf_ternary_linear": (_i, [C.POINTER(LinearArgs), _vp]),
     "wf_ternary_linear_scales": (_i, [C.POINTER(LinearArgs), _vp, _vp]),
     "wf_bitnet_gemm_workspace_bytes": (_sz, [_i, _i, _i]),
+    "wf_gemm_tc_pair_tokens": (_i, [_i, _i, _i, _i, _i]),
     "wf_wait_word": (C.POINTER(_i), []),
     "wf_bitnet_gemv": (_i, [_vp, _vp, _f, _i, _i, _vp, _vp, _sz, _vp]),
     "wf_bitnet_gemm": (_i, [_vp, _vp, _f, _i, _i, _i, _vp, _vp, _sz, _vp]),
