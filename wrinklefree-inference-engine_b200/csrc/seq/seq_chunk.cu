@@ -577,10 +577,12 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_redo_kernel(Batch b, DeltaDi
     if (tid == 0) *mark = 0;
 }
 
-// Whether a recurrence without the correction takes two column tiles a block, where tiles is the number of 16-column tiles and pairs that of blocks of two.  A scan
+// Whether a recurrence takes two column tiles a block, where tiles is the number of 16-column tiles and pairs that of blocks of two.  A scan
 // takes as long as its fullest SM.  us a chunk with n blocks there, 128-row states: one tile a block 1.2, 1.7, 2.5, 3.3, 4.4 (n = 1 .. 5), two tiles 1.5, 2.6, 3.9.
 // So 16 heads of 128 x 64 (64 tiles), one sequence of 256 tokens 36 / 41 us, 40 heads, 2 sequences of 2048 (320 tiles) 317 / 338, but 4 of 1024 (640) 287 / 259;
 // an odd tile is a block of its own: matrix memory, 16 heads of 64 x 129, 4 of 1024 (576 tiles, 320 pairs) 147 / 163.
+// The same with the correction: 20 heads of 128 x 128, 1801 tokens in 1 sequence (160 tiles) 280 / 259, 2 (320) 209 / 224, 3 (480) 203 / 169, 4 (640) 190 / 192;
+// 20 heads of 64 x 64 in 1 (80 tiles) 142 / 190.
 bool two_tiles(long long tiles, long long pairs) {
     const long long sms = sm_count(), one = (tiles + sms - 1) / sms, two = (pairs + sms - 1) / sms;
     return 3 * two < 2 * one;
@@ -612,10 +614,7 @@ int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const floa
     auto scan_pass = [&](int pass) {
         sg.pass = pass;
         const long long chains = (long long)b.nseq * sg.n * D.H, tiles = chains * cols;
-        // With the correction two column tiles a block are the longer chain and the lesser work from four blocks an SM on: us with one / two, 20 heads of 128 x 128
-        // in one sequence (160 tiles) 351 / 387, 2 (320) 192 / 208, 4 (640) 186 / 171.
-        const bool two = DELTA ? tiles > 4LL * sm_count() : two_tiles(tiles, chains * ((cols + 1) / 2));
-        return two ? cr_scan<DS, VEC, DELTA, 2>(b, D, w, state, slot_stride, o, sg, s) : cr_scan<DS, VEC, DELTA, 1>(b, D, w, state, slot_stride, o, sg, s);
+        return two_tiles(tiles, chains * ((cols + 1) / 2)) ? cr_scan<DS, VEC, DELTA, 2>(b, D, w, state, slot_stride, o, sg, s) : cr_scan<DS, VEC, DELTA, 1>(b, D, w, state, slot_stride, o, sg, s);
     };
     // Segments in parallel where the recurrence is linear in the state, one portion is long and the chains of whole portions leave the machine idle: the two
     // passes cost half as much work again.  us, whole -> segments, each with the better number of tiles a block: 4 heads of 128 x 64, 1024 tokens 88 -> 40, 600 tokens
