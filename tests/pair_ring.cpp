@@ -38,7 +38,7 @@ int main(int argc, char** argv) {
         std::mt19937 rng(seed);
         Bar full[TP_WS], empty[TP_WS], a_full[16], a_empty[16];
         int content[TP_WS];
-        for (int s = 0; s < TP_WS; ++s) { full[s].init(1); empty[s].init(form ? TP_WKB : NU); content[s] = -1; }
+        for (int s = 0; s < TP_WS; ++s) { full[s].init(1); empty[s].init(TP_WKB); content[s] = -1; }
         for (int s = 0; s < TS; ++s) { a_full[s].init(1); a_empty[s].init(1); }
         std::vector<int> flying;
         std::vector<Task> tasks(NU + 2);
@@ -60,7 +60,8 @@ int main(int argc, char** argv) {
         };
         for (int g = 0; g < NU; ++g)
             tasks[2 + g].body = [&, g] {
-                PairWeightWalk walk(g, NU, KB);
+                PairWeightWalk<true> ragged(g, NU, KB);
+                PairWeightWalk<false> even(g, NU, KB);
                 int kb = g, first = 0, load = 0;
                 auto wait = [&](int l) { until([&, l] { return full[l % TP_WS].passed((l / TP_WS) & 1); }); return true; };
                 auto back = [&](int l) { empty[l % TP_WS].arrive(); };
@@ -74,8 +75,8 @@ int main(int argc, char** argv) {
                         kb += NU;
                         while (kb >= KB) { kb -= KB; first += per; }
                     } else {
-                        walk.next(wait, back);
-                        load = walk.load;
+                        if (pair_ragged(KB, NU)) ragged.next(wait, back), load = ragged.load, back_n = ragged.count;
+                        else even.next(wait, back), load = even.load, back_n = even.count;
                     }
                     stale += content[load % TP_WS] != load;
                     return back_n;
@@ -83,7 +84,7 @@ int main(int argc, char** argv) {
                 int n = 0;
                 if (g < items) n = fetch();
                 for (int it = g; it < items; it += NU) {
-                    if (form) empty[load % TP_WS].arrive(n);
+                    empty[load % TP_WS].arrive(n);
                     if (it + NU < items) n = fetch();
                     if (it >= TS) until([&, it] { return a_empty[it % TS].passed((it / TS - 1) & 1); });
                     until([] { return true; });

@@ -163,7 +163,7 @@ __device__ __forceinline__ void pair_store(const EpiParams& ep, const PairEp& e,
     else each(of, plain);
 }
 
-template <int NU, int NBUF>
+template <int NU, int NBUF, bool RAGGED>
 __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_w,
                                                                               const TpParams p) {
     extern __shared__ unsigned char smem_raw[];
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
     if (tid == 0) {
         for (int s = 0; s < AS; ++s) { mbar_init(&act_full[s], 1); mbar_init(&act_empty[s], 1); }
         for (int s = 0; s < TP_TS; ++s) { mbar_init(&a_full[s], 8); mbar_init(&a_empty[s], 1); }
-        for (int s = 0; s < TP_WS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 4 * NU); }
+        for (int s = 0; s < TP_WS; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 4 * TP_WKB); }
         for (int b = 0; b < 2; ++b) { mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * TP_EPW); }
         mbar_init(&drained, 1);
         fence_mbar_init();
@@ -330,17 +330,15 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
         const uint32_t rx = p.i2s ? (uint32_t)(row & 7) : (uint32_t)((row & 7) >> 1);
         const bool odd = (row >> 3) & 1;
         const bool i2s = p.i2s != 0;
-        PairWeightWalk walk(grp, NU, KB);
+        PairWeightWalk<RAGGED> walk(grp, NU, KB);
         bool ok = true;
-        uint32_t pk[8];                               // an item's packed codes
+        uint32_t pk[8], empty = 0;                    // an item's packed codes, and the hand-back barrier of their buffer
         auto landed = [&](int load) { return __all_sync(0xffffffffu, wait_bounded(smem_u32(&w_full[load % TP_WS]), (uint32_t)((load / TP_WS) & 1))) != 0; };
-        auto hand_back = [&](int load) {              // every lane has its codes
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&w_empty[load % TP_WS]);
-        };
+        auto pass_by = [&](int load) { if (lane == 0) mbar_arrive(&w_empty[load % TP_WS]); };
         auto fetch = [&]() -> bool {
-            if (!walk.next(landed, hand_back)) return false;
+            if (!walk.next(landed, pass_by)) return false;
             const int ws = walk.load % TP_WS, j = walk.part;
+            empty = smem_u32(&w_empty[ws]);
             const uint32_t src = wring + ws * TP_W_BYTES + rbase;
             if (i2s) {
 #pragma unroll
@@ -365,6 +363,8 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
             for (int g = 0; g < 4; ++g)
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[8 * g + i] = (pk[i] >> (6 - 2 * g)) & 0x03030303u;   // k = 32g + 4i .. +3
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty), "r"((uint32_t)walk.count) : "memory");
             if (it + NU < n_items && !fetch()) { ok = false; break; }       // the next item's codes arrive while this one waits for its TMEM stage
             const int ts = it % TP_TS;
             if (it >= TP_TS && !__all_sync(0xffffffffu, wait_bounded(smem_u32(&a_empty[ts]), (uint32_t)((it / TP_TS - 1) & 1)))) { ok = false; break; }   // its last MMAs are done
@@ -500,8 +500,14 @@ int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream
     constexpr int NU = 3;
     EncodeTiledFn enc = tc_encoder();
     if (!enc) { set_error("gemm_tc_pair: cuTensorMapEncodeTiled unavailable"); return WF_ERR_CUDA; }
-    if (g_attr.need() && (cuda_check(cudaFuncSetAttribute(ternary_gemm_pair_kernel<NU, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM), "gemm_tc_pair attribute") ||
-                          cuda_check(cudaFuncSetAttribute(ternary_gemm_pair_kernel<NU, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM), "gemm_tc_pair attribute"))) return WF_ERR_CUDA;
+    typedef void (*Kernel)(CUtensorMap, CUtensorMap, TpParams);
+    static const Kernel kernels[2][2] = {{ternary_gemm_pair_kernel<NU, 2, false>, ternary_gemm_pair_kernel<NU, 2, true>},       // [one accumulator][ragged]
+                                         {ternary_gemm_pair_kernel<NU, 1, false>, ternary_gemm_pair_kernel<NU, 1, true>}};
+    if (g_attr.need()) {
+        for (const auto& row : kernels)
+            for (Kernel k : row)
+                if (cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TP_SMEM), "gemm_tc_pair attribute")) return WF_ERR_CUDA;
+    }
     TpParams p;
     memset(&p, 0, sizeof p);
     p.M = a->M; p.N = a->N; p.K = a->K; p.KB = a->K / WF_QK;
@@ -551,7 +557,7 @@ int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 2;
-    return launch_check(p.tn > 192 ? cudaLaunchKernelEx(&cfg, ternary_gemm_pair_kernel<NU, 1>, tq, tw, p) : cudaLaunchKernelEx(&cfg, ternary_gemm_pair_kernel<NU, 2>, tq, tw, p), "ternary_gemm_pair");
+    return launch_check(cudaLaunchKernelEx(&cfg, kernels[p.tn > 192][pair_ragged(p.KB, NU)], tq, tw, p), "ternary_gemm_pair");
 }
 
 }  // namespace wf
