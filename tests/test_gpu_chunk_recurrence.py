@@ -57,9 +57,9 @@ def test_delta_rule_with_a_decay_per_row(heads, kv_heads, dim, vdim, lens, cuts)
     check(cfg, w, {"l0.mix.a1": (8, W), "l0.mix.g1": (8, W)}, lambda x: NO.channel_delta(x, d64(w, "l0.mix."), "", m, EPS), lens, cuts, W)
 
 
-@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(60, 20, 64, 97), (40, 20, 100, 130), (160, 20, 36, 20)])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(60, 20, 64, 97), (64, 16, 64, 97), (40, 20, 100, 130), (160, 20, 36, 20)])
 def test_delta_rule_of_many_heads(heads, kv_heads, dim, vdim):
-    """Enough (sequence, head, 16 columns) blocks that each takes two column tiles, the last one of an odd count alone."""
+    """Enough (sequence, head, 16 columns) tiles that a block takes two of them (not with 60 heads), the last one of an odd count alone."""
     W = 40
     m = {"heads": heads, "kv_heads": kv_heads, "dim": dim, "vdim": vdim, "conv": 4}
     cfg = {"architecture": "Nukezen", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": EPS}, "layers": [{"type": "channel_delta", "mixer": m, "mlp": None}]}
