@@ -22,11 +22,11 @@ CUTS = [([70], [[70]]), ([33, 100], [[33, 100]]), ([90, 64], [[32, 0], [15, 47],
 EPS = 1e-5
 
 
-def check(cfg, weights, shapes, wants, lens, cuts, W):
+def check(cfg, weights, shapes, wants, lens, cuts, W, max_tokens=800, step=672):
     from wf_bitnet import registry
     cls = registry.resolve(cfg)
     extra = {"shapes": shapes} if getattr(cls, "reads_shapes", False) else {}
-    m = cls(cfg, dtype="float32", max_tokens=800, slots=4, page_size=16, max_step_tokens=672, **extra)
+    m = cls(cfg, dtype="float32", max_tokens=max_tokens, slots=4, page_size=16, max_step_tokens=step, **extra)
     m.load_weights((k, v.numpy(), "F32") for k, v in weights.items())
     g = np.random.default_rng(sum(lens))
     rows = [g.standard_normal((n, W)).astype(np.float32) for n in lens]
@@ -100,6 +100,26 @@ def test_matrix_memory(heads, dim, vdim, lens, cuts):
            "layers": [{"type": "parallel", "mixer": {"left": left, "left_scale": 0.0, "right": right, "right_scale": 1.0}, "mlp": None}]}
     w = FO.random_weights(cfg, 3)
     check(cfg, w, {"l0.mix.left.rel": (8, 2)}, lambda x: FO.matrix_memory(x, d64(w, "l0.mix.right."), "", right, EPS), lens, cuts, W)
+
+
+# long portions: segments of 128 tokens all at once.  Whole segments, a last one of one token and of one less than a whole one, a carried state, two sequences of unequal
+# segments; key sizes that leave rows of a warp over, value sizes below, at and beyond 64 columns
+@pytest.mark.parametrize("lens,cuts", [([512], [[512]]), ([670, 513], [[30, 513], [640, 0]]), ([639], [[639]])])
+@pytest.mark.parametrize("kind,heads,groups,dim,vdim", [("ssd", 4, 2, 128, 64), ("ssd", 6, 3, 20, 12), ("ssd", 8, 1, 64, 68), ("memory", 2, 2, 128, 128), ("memory", 3, 3, 24, 15)])
+def test_segments(kind, heads, groups, dim, vdim, lens, cuts):
+    W = 40
+    left = {"heads": 2, "kv_heads": 1, "dim": 8, "vdim": 8, "scale": 0.3, "mask": {"size": 8}}
+    if kind == "ssd":
+        left["rot"] = {"dims": 8, "base": 10000.0}
+        right = {"heads": heads, "vdim": vdim, "state": dim, "groups": groups, "conv": 4, "norm_groups": groups}
+    else:
+        left["bias_max"] = 16
+        right = {"heads": heads, "dim": dim, "vdim": vdim, "gate_cap": 15.0}
+    cfg = {"architecture": "Nukezen" if kind == "ssd" else "Fivedra", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": EPS},
+           "layers": [{"type": "parallel", "mixer": {"left": left, "left_scale": 0.0, "right": right, "right_scale": 1.0}, "mlp": None}]}
+    w = (NO if kind == "ssd" else FO).random_weights(cfg, 4)
+    oracle = (lambda x: NO.state_space(x, d64(w, "l0.mix.right."), "", right, EPS)) if kind == "ssd" else (lambda x: FO.matrix_memory(x, d64(w, "l0.mix.right."), "", right, EPS))
+    check(cfg, w, {} if kind == "ssd" else {"l0.mix.left.rel": (8, 2)}, oracle, lens, cuts, W, 1400, 1184)
 
 
 # ---- numbers that are not finite: long portions (the 16-token form, and its parallel segments where the recurrence is plain) against the same rows in portions of 31 tokens (token by token)

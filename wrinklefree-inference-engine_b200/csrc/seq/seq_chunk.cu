@@ -20,29 +20,19 @@
 // anything that it reads or forms is not finite, the scan those in which U or the state is not, and chunk_redo_kernel takes the marked portions again from
 // their start, token by token as the recurrence is stated: a launch of blocks that leave at once where nothing is marked (about 2 us; deciding chunk by
 // chunk inside the scan cost it 15 to 30 %).
-#include "seq_kernels.cuh"
+#include "seq_chunk.cuh"
 
 namespace wf {
 namespace seq {
 
 namespace {
 
-constexpr int CR = CHUNK_TOKENS, CR_WARPS = 4, CR_THREADS = 32 * CR_WARPS, CR_COLS = 16;
+constexpr int CR = CHUNK_TOKENS, CR_WARPS = 4, CR_THREADS = 32 * CR_WARPS;
 static_assert(CR == 16, "a chunk is two 8-token tiles");
 
 __device__ __forceinline__ void cr_cp16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-
-struct ChunkView {
-    const float *qkv, *beta, *decay; int ld, q_off, k_off, v_off;
-    float* rec;
-    int nchunks;
-    int *redo, cols;               // [sequence][head][CR_COLS columns]: marked; zero between launches
-};
-
-// x * 0 summed up: zero while everything is finite, NaN from the first infinity or NaN on
-__device__ __forceinline__ void cr_watch(float& w, float x) { w = fmaf(x, 0.f, w); }
 
 // one of the two passes over segments of SCAN_CHUNK tokens in parallel (recurrences linear in the state): pass 1 leaves each segment's own end state (from a
 // zero one) and, with one decay per head, the product of its decays; pass 3 reads the segments' start states, chained by scan_prefix_kernel; 0: whole portions
@@ -185,31 +175,6 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_prep_kernel(Batch b, DeltaDi
     if (!(watch == 0.f))
         for (int z = 0; z < w.cols; ++z) w.redo[((size_t)sq * D.H + h) * w.cols + z] = 1;
 }
-
-__device__ __forceinline__ void cr_split(float x, uint32_t& hi, uint32_t& lo) {
-    // round to 10 stored bits by integer arithmetic (the conversion instruction runs at a fraction of its rate); the instruction drops the low 13 bits of lo
-    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
-}
-__device__ __forceinline__ void cr_mma(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-struct CrA { uint32_t h[4], l[4]; };
-struct CrB { uint32_t h[2], l[2]; };
-// an accumulator tile as the A operand: columns 2 t and 2 t + 1 become k = t and t + 4
-__device__ __forceinline__ CrA cr_a(const float (&c)[4]) {
-    CrA a;
-    cr_split(c[0], a.h[0], a.l[0]); cr_split(c[2], a.h[1], a.l[1]); cr_split(c[1], a.h[2], a.l[2]); cr_split(c[3], a.h[3], a.l[3]);
-    return a;
-}
-__device__ __forceinline__ CrB cr_b(float x, float y) {
-    CrB b;
-    cr_split(x, b.h[0], b.l[0]); cr_split(y, b.h[1], b.l[1]);
-    return b;
-}
-__device__ __forceinline__ CrB cr_b2(const float* p) { const float2 v = *reinterpret_cast<const float2*>(p); return cr_b(v.x, v.y); }
-__device__ __forceinline__ void cr_mma3(float (&d)[4], const CrA& a, const CrB& b) { cr_mma(d, a.l, b.h); cr_mma(d, a.h, b.l); cr_mma(d, a.h, b.h); }
 
 template <int DS, bool VEC, bool DELTA> struct CrStage {
     static constexpr int QS = DS + 8, KS = DS + 4;        // row strides: pairs of rows 8 tokens apart, single rows 2 tokens apart, each without bank conflicts
@@ -603,20 +568,25 @@ int cr_scan(const Batch& b, const DeltaDims& D, const ChunkView& w, float* state
 
 template <int DS, bool VEC, bool DELTA>
 int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const float* decay, float* state, size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan) {
-    launch_pdl(chunk_prep_kernel<DS, VEC, DELTA>, dim3(b.nseq * w.nchunks, D.H), CR_THREADS, 0, s, b, D, w);
-    if (int rc = launch_check(cudaGetLastError(), "chunk_prep")) return rc;
     Segments sg;
     const int cols = w.cols;
     auto redo = [&]() {
         launch_pdl(chunk_redo_kernel<DS, VEC, DELTA>, dim3(b.nseq, D.H, cols), CR_THREADS, 0, s, b, D, w, state, slot_stride, o, sg);
         return launch_check(cudaGetLastError(), "chunk_redo");
     };
+    if (!VEC && !DELTA && segments_usable(b, D, scan)) {
+        if (int rc = launch_segments(b, D, w, decay, state, slot_stride, o, s, scan)) return rc;
+        sg.start = scan->start;
+        return redo();
+    }
+    launch_pdl(chunk_prep_kernel<DS, VEC, DELTA>, dim3(b.nseq * w.nchunks, D.H), CR_THREADS, 0, s, b, D, w);
+    if (int rc = launch_check(cudaGetLastError(), "chunk_prep")) return rc;
     auto scan_pass = [&](int pass) {
         sg.pass = pass;
         const long long chains = (long long)b.nseq * sg.n * D.H, tiles = chains * cols;
         return two_tiles(tiles, chains * ((cols + 1) / 2)) ? cr_scan<DS, VEC, DELTA, 2>(b, D, w, state, slot_stride, o, sg, s) : cr_scan<DS, VEC, DELTA, 1>(b, D, w, state, slot_stride, o, sg, s);
     };
-    // Segments in parallel where the recurrence is linear in the state, one portion is long and the chains of whole portions leave the machine idle: the two
+    // (Portions that launch_segments leaves.)  Segments in parallel where the recurrence is linear in the state, one portion is long and the chains of whole portions leave the machine idle: the two
     // passes cost half as much work again.  us, whole -> segments, each with the better number of tiles a block: 4 heads of 128 x 64, 1024 tokens 88 -> 40, 600 tokens
     // 59 -> 39; 16 heads, 2048 tokens 171 -> 93; 40 heads (160 tiles) 230 -> 175; 24 heads, 2 sequences of 1024 (192 tiles) 126 -> 121, 16 heads, 4 sequences of
     // 1024 (256 tiles) 131 -> 147.

@@ -361,18 +361,29 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(Batch b, DeltaDi
 
 // thread per (sequence, head, state element): chains the chunks' start states from the slot's state and leaves the end state in the slot.
 // prod has one entry per (chunk, head), or (d > 0) one per (chunk, head, key row) of dd / d state columns each
-__global__ void scan_prefix_kernel(Batch b, int H, int dd, int chunk, float* __restrict__ state, size_t slot_stride, const float* local,
-                                   float* __restrict__ startws, const float* prod, int d) {
+__global__ void scan_prefix_kernel(Batch b, int H, int dd, int chunk, float* __restrict__ state, size_t slot_stride, const float* __restrict__ local,
+                                   float* __restrict__ startws, const float* __restrict__ prod, int d) {
     pdl_enter();
     const int sq = blockIdx.x, h = blockIdx.y, e = blockIdx.z * blockDim.x + threadIdx.x;
     if (e >= dd) return;
-    const int len = b.seq_len[sq], nc = (len + chunk - 1) / chunk, base = b.seq_start[sq] / chunk + sq;
+    const int len = b.seq_len[sq], nc = (len + chunk - 1) / chunk, base = b.seq_start[sq] / chunk + sq, row = d > 0 ? e / (dd / d) : 0;
     float* Sp = state + (size_t)b.seq_slot[sq] * slot_stride + (size_t)h * dd + e;
     float S = *Sp;
-    for (int c = 0; c < nc; ++c) {
-        const size_t entry = (size_t)(base + c) * H + h;
-        startws[entry * dd + e] = S;
-        S = fmaf(d > 0 ? prod[entry * d + e / (dd / d)] : prod[entry], S, local[entry * dd + e]);
+    // SP chunks requested at once: only the additions wait for one another (16 chunks of 40 heads of 128 x 64: 26 -> 14 us)
+    constexpr int SP = 8;
+    for (int c0 = 0; c0 < nc; c0 += SP) {
+        float x[SP], p[SP];
+#pragma unroll
+        for (int k = 0; k < SP; ++k) {
+            const size_t entry = (size_t)(base + c0 + k) * H + h;
+            if (c0 + k < nc) { x[k] = __ldcg(local + entry * dd + e); p[k] = __ldcg(prod + (d > 0 ? entry * d + row : entry)); }
+        }
+#pragma unroll
+        for (int k = 0; k < SP; ++k) {
+            if (c0 + k >= nc) break;
+            startws[((size_t)(base + c0 + k) * H + h) * dd + e] = S;
+            S = fmaf(p[k], S, x[k]);
+        }
     }
     *Sp = S;
 }

@@ -1266,7 +1266,11 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
     size_t max_talk_ws = 0;          // mixed heads: one unsplit partial result for every sequence, and room for one per SM
     bool any_mlstm = false;
     size_t max_redo = 0;
-    auto rec_for = [&](const DeltaDims& D) { max_rec = std::max(max_rec, chunk_workspace_floats(D, T, c.slots)); max_redo = std::max(max_redo, chunk_redo_words(D, c.slots)); };
+    size_t max_segment = 0;
+    auto rec_for = [&](const DeltaDims& D) {
+        max_rec = std::max(max_rec, chunk_workspace_floats(D, T, c.slots)); max_redo = std::max(max_redo, chunk_redo_words(D, c.slots));
+        max_segment = std::max(max_segment, segment_workspace_floats(D, T, c.slots));
+    };
     bool own = true;                 // false while a tied layer is laid out: it allocates and names nothing, its weights are its source's
     auto walloc = [&](void** ptr, size_t count) -> int { return own ? dalloc_t(e, ptr, count) : WF_OK; };
     auto name = [&](const std::string& n, void* dst, size_t count) { if (own) add_tensor(e, n, dst, count); };
@@ -1405,7 +1409,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             L.st_S = st; st += (size_t)l.heads * l.dim * (l.vdim + 1);
             L.st_m = st; st += l.heads;
             max_scan = std::max(max_scan, (size_t)l.heads * l.dim * (l.vdim + 1));
-            rec_for(DeltaDims{l.heads, l.heads, l.dim, l.vdim});
+            rec_for(DeltaDims{l.heads, l.heads, l.dim, l.vdim, 0, 1});
             max_hv = std::max(max_hv, (size_t)l.heads * (l.vdim + 1));
             any_mlstm = true;
         } else if (l.type == WF_SEQ_GLA) {
@@ -1426,7 +1430,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             L.st_S = st; st += nk * l.vdim;
             max_decay = std::max(max_decay, nk);
             max_scan = std::max(max_scan, nk * l.vdim);
-            rec_for(DeltaDims{l.heads, l.heads, l.dim, l.vdim, 1});
+            rec_for(DeltaDims{l.heads, l.heads, l.dim, l.vdim, 1, 1});
         } else if (l.type == WF_SEQ_SSD) {
             // [z | x | B | C | dt]: x, B and C are the convolved channels
             const size_t GN = (size_t)l.kv_heads * l.dim;
@@ -1443,7 +1447,7 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
             L.st_S = st; st += (size_t)l.heads * l.dim * l.vdim;
             max_C = std::max(max_C, (size_t)L.C);
             max_scan = std::max(max_scan, (size_t)l.heads * l.dim * l.vdim);
-            rec_for(DeltaDims{l.heads, l.kv_heads, l.dim, l.vdim});
+            rec_for(DeltaDims{l.heads, l.kv_heads, l.dim, l.vdim, 0, 1});
         } else {
             // [q | k | v | gate (or its first factor) | write strength | decay (or its first factor)]
             const size_t nqk = (size_t)l.kv_heads * l.dim;
@@ -1643,10 +1647,17 @@ extern "C" int wf_seq_create(const wf_seq_config* cfg, const wf_seq_layer* layer
 #undef TRY
     // What only the faster forms of prompt portions need comes last, each form's part as a whole, and only where that leaves three quarters of what is free
     // by then: an engine that fits without them still fits, and takes the forms that need none.
-    if (e->chunk_rec && max_rec && T >= 2 * CHUNK_TOKENS && dalloc_spare(e, (void**)&e->scan.rec, (max_rec + max_redo) * sizeof(float))) {
-        e->scan.rec_floats = max_rec;
-        e->scan.redo = (int*)(e->scan.rec + max_rec); e->scan.redo_words = max_redo;
-        if (cuda_check(cudaMemsetAsync(e->scan.redo, 0, max_redo * 4, e->stream), "marks")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
+    if (e->chunk_rec && max_rec && T >= 2 * CHUNK_TOKENS) {
+        size_t recs = std::max(max_rec, max_segment);
+        if (!dalloc_spare(e, (void**)&e->scan.rec, (recs + max_redo) * sizeof(float))) {
+            const bool less = recs > max_rec;      // segments want more of it than records
+            recs = less && dalloc_spare(e, (void**)&e->scan.rec, (max_rec + max_redo) * sizeof(float)) ? max_rec : 0;
+        }
+        if (recs) {
+            e->scan.rec_floats = recs;
+            e->scan.redo = (int*)(e->scan.rec + recs); e->scan.redo_words = max_redo;
+            if (cuda_check(cudaMemsetAsync(e->scan.redo, 0, max_redo * 4, e->stream), "marks")) { wf_seq_destroy(e); return WF_ERR_CUDA; }
+        }
     }
     if (max_kvx) {                             // enough positions for sequences of several full steps; longer ones keep the form that reads the latents
         const size_t rows = (size_t)std::min<long long>((long long)c.max_pages * c.page_size, 4LL * T);

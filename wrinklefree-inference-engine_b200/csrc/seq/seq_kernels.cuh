@@ -269,6 +269,7 @@ int launch_scan_prefix(const Batch& b, const DeltaDims& D, const float* decay, f
 constexpr int CHUNK_TOKENS = 16;
 size_t chunk_workspace_floats(const DeltaDims& D, int max_step_tokens, int slots);
 size_t chunk_redo_words(const DeltaDims& D, int slots);
+size_t segment_workspace_floats(const DeltaDims& D, int max_step_tokens, int slots);      // the same of its form in segments (seq_segment.cu), which is left out where rec holds less
 bool chunk_usable(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const ScanWorkspace* scan);
 int launch_chunk_recurrence(const Batch& b, const DeltaDims& D, const float* qkv, int ld, const float* beta, const float* decay, float* state, size_t slot_stride,
                             float* o, cudaStream_t s, const ScanWorkspace* scan);
