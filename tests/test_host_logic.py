@@ -182,3 +182,17 @@ def test_which_product_kernel_a_shape_takes(m, n, k, tcgen05):
     """Either side of the lines between the mma.sync and the tcgen05 ternary product (148 SMs); only the former asks for a workspace."""
     from wf_bitnet import _lib
     assert (_lib.lib().wf_bitnet_gemm_workspace_bytes(m, n, k) == 0) == tcgen05
+
+
+@pytest.mark.parametrize("entries", [[0] * 31, list(range(-20, 20)), [-2 ** 31, 2 ** 31 - 1] * 20, [1] * 40 + [2 ** 31], [1] * 40 + [-2 ** 31 - 1], [True] * 40, [1.5] * 40,
+                                     [np.int64(3)] * 40, ["a"] * 40, [[1]] * 40, (7,) * 40, range(50), np.arange(40), []])
+def test_lists_of_token_ids_become_arrays_as_numpy_makes_them(entries):
+    from wf_bitnet.seq_engine import _i32
+    try:
+        want = np.ascontiguousarray(entries, dtype=np.int32)
+    except Exception as e:
+        with pytest.raises(type(e)):
+            _i32(entries)
+        return
+    got = _i32(entries)
+    assert got.dtype == want.dtype and got.shape == want.shape and np.array_equal(got, want)

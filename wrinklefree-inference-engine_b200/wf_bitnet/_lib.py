@@ -201,6 +201,20 @@ SEQ_SYMBOLS = {
 _seq_lib = None
 
 
+def _load_py_i32():
+    """wf_py_i32 of libwf_py.so (csrc/py_host.c), or None where it has not been built or is another interpreter's."""
+    try:
+        fn = C.PyDLL(str(_PKG_ROOT / "libwf_py.so")).wf_py_i32
+    except (OSError, AttributeError):
+        return None
+    fn.restype = C.c_int
+    fn.argtypes = [C.py_object, C.c_void_p, C.c_ssize_t]
+    return fn
+
+
+py_i32 = _load_py_i32()
+
+
 def build_seq_lib() -> None:
     """Compile libwf_seq.so in-tree (make target `seq`: the sequence-model sources only)."""
     import subprocess
