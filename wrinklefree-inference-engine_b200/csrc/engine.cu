@@ -953,12 +953,9 @@ extern "C" int wf_engine_set_context(wf_engine* e, int slot, int len, int fill_r
     if (!e->pt.ensure(slot, len)) { set_error("KV pool exhausted"); return WF_ERR_INVALID; }
     e->pt.dirty = true;
     e->h_pos[slot] = len;
-    // on the engine stream (it is cudaStreamNonBlocking: a default-stream copy could race an in-flight asynchronous step, whose
-    // advance kernel updates the same words)
-    const int32_t pl[2] = {len, len + 1};
-    if (cuda_check(cudaMemcpyAsync(e->d_pos + slot, &pl[0], 4, cudaMemcpyHostToDevice, e->stream), "ctx pos")) return WF_ERR_CUDA;
-    if (cuda_check(cudaMemcpyAsync(e->d_len + slot, &pl[1], 4, cudaMemcpyHostToDevice, e->stream), "ctx len")) return WF_ERR_CUDA;
-    if (cuda_check(cudaStreamSynchronize(e->stream), "ctx sync")) return WF_ERR_CUDA;
+    // on the engine stream (an in-flight asynchronous step's advance kernel updates the same words); one launch with the length by value in place of two copies from the
+    // stack and the wait for them: 6 us less of the caller's time (64 sequences set back between four steps: 20039 -> 19640 us in all)
+    if (int rc = launch_set_context(e->d_pos + slot, e->d_len + slot, len, e->stream)) return rc;
     if (fill_random) {
         // a page is one contiguous run of layers*2*Hkv*page_size*D elements
         const size_t page_elems = (size_t)e->cfg.layers * 2 * e->Hkv * ps * e->D;

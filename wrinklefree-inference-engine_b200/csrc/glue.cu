@@ -240,6 +240,12 @@ __global__ void advance_kernel(int32_t* positions, int32_t* seq_lens, int32_t* t
     if (threadIdx.x == 0 && step) *step += 1;
 }
 
+__global__ void set_context_kernel(int32_t* position, int32_t* seq_len, int len) { *position = len; *seq_len = len + 1; }
+int launch_set_context(int32_t* position, int32_t* seq_len, int len, cudaStream_t s) {
+    set_context_kernel<<<1, 1, 0, s>>>(position, seq_len, len);
+    return launch_check(cudaGetLastError(), "set_context");
+}
+
 // ---------------------------------------------------------------------------------------------
 // synthetic data (bench / smoke only): splitmix64 counter hash
 __device__ __forceinline__ uint64_t mix64(uint64_t x) {

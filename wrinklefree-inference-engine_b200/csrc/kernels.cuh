@@ -23,6 +23,7 @@ int attn_decode(const void* q, const void* pool, int layers, int layer, int Hkv,
                 void* ws, size_t ws_bytes, cudaStream_t s, bool pdl, float* kv_scales = nullptr);
 int launch_gemm_tc_red(const uint8_t* w_tile, int N, int K, const int8_t* q, int M, int ldq, int k_off, float* acc, int acc_ld,
                        cudaStream_t s, bool pdl);
+int launch_set_context(int32_t* position, int32_t* seq_len, int len, cudaStream_t s);
 int launch_embed(const void* table, const int32_t* tokens, int B, int H, void* out, cudaStream_t s);
 int launch_advance(int32_t* positions, int32_t* seq_lens, int32_t* tokens, const int32_t* next, int B, int feed_back, cudaStream_t s);
 int launch_fill_ternary(void* out, size_t bytes, uint64_t seed, cudaStream_t s);
