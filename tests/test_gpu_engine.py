@@ -1,5 +1,7 @@
 """GPU parity: the whole decode step (wf_engine) vs the oracle forward (scripts/direct_inference_full.py
 restated in oracle/model.py) on identical synthetic random-init ternary weights."""
+import dataclasses
+
 import numpy as np
 import pytest
 import torch
@@ -268,7 +270,6 @@ def test_layer_tail_handoff_forms_equal_phase_kernels(shape, monkeypatch):
     """Batch 1 at the real layer widths: the persistent tail kernel with flag-in-data hand-offs (default at the 2B shape; the 8B ffn row
     is too long for the register glue, so there the default IS the grid-barrier form), the same kernel with grid barriers (WF_TAIL_LAM=0) and the
     per-phase kernels (WF_TAIL=0) must produce identical logits over a run of steps — a lost or early hand-off would flip bits."""
-    import dataclasses
     from wf_bitnet.engine import EngineConfig
     mk = EngineConfig.bitnet_2b if shape == "2b" else EngineConfig.llama3_8b
     cfg = dataclasses.replace(mk(max_seq=1024, max_batch=1), layers=3, vocab=4096)
@@ -321,6 +322,21 @@ def test_tcgen05_decode_linears_equal_per_op_kernels(B, ctx, monkeypatch):
         assert (na == nb).all() and (nc == nb).all()
 
 
+@pytest.mark.parametrize("shape", ["2b", "8b"])
+def test_batches_of_changing_size_equal_per_op_kernels(shape, monkeypatch):
+    """Steps that change between the forms of gate|up (activation where CTA pairs store it from 33 rows on, sums in a cleared buffer below): nothing of one is left for the other."""
+    from wf_bitnet.engine import EngineConfig
+    make = EngineConfig.bitnet_2b if shape == "2b" else EngineConfig.llama3_8b
+    cfg = dataclasses.replace(make(max_seq=512, max_batch=64, vocab=4096), layers=2)
+    rng = np.random.default_rng(5)
+    steps = [list(map(int, rng.integers(0, cfg.vocab, B))) for B in (64, 12, 33, 40, 20, 64)]
+    a = _run_tokens(cfg, None, True, steps, monkeypatch, ctx=100, synthetic=5)
+    b = _run_tokens(cfg, None, False, steps, monkeypatch, ctx=100, synthetic=5)
+    for i, ((la, na, _), (lb, nb, _)) in enumerate(zip(a, b)):
+        assert torch.equal(la, lb), (i, (la - lb).abs().max().item())
+        assert (na == nb).all()
+
+
 @pytest.mark.parametrize("shape,B,ctx", [("2b", 2, 80), ("2b", 13, 200), ("2b", 32, 120), ("8b", 1, 90), ("8b", 5, 90), ("8b", 16, 150), ("8b", 32, 60)])
 def test_streaming_decode_gemm_equals_default_kernels(shape, B, ctx, monkeypatch):
     """WF_DECODE_STREAM=2: every decode linear of 2..32 rows on the streaming batched GEMM (gemm_stream.cu: K windows, TMA ring, masked
@@ -328,7 +344,6 @@ def test_streaming_decode_gemm_equals_default_kernels(shape, B, ctx, monkeypatch
     tcgen05 forms; those are held against the one-kernel-per-op path by the tests above).  Both runs share the attention kernel and its
     chunking, so any difference is the GEMM's.  2B widths: one window (K = 2560) and two windows of 27 k-blocks (K = 6912); 8B widths:
     one window of 32 and four of 28."""
-    import dataclasses
     from wf_bitnet.engine import EngineConfig
     mk = EngineConfig.bitnet_2b if shape == "2b" else EngineConfig.llama3_8b
     cfg = dataclasses.replace(mk(max_seq=1024, max_batch=B), layers=2, vocab=4096)
@@ -386,7 +401,6 @@ def cfg0_weights():
 
 
 def _sliced(cfg, w, layers):
-    import dataclasses
     c = dataclasses.replace(cfg, layers=layers)
     ww = dict(w)
     ww["layers"] = w["layers"][:layers]

@@ -56,6 +56,6 @@ EncodeTiledFn tc_encoder();   // cuTensorMapEncodeTiled, or null where the drive
 // CTA-pair form (gemm_tc_pair.cu), the tokens of its tiles and the time (us) that it is expected to take
 int gemm_tc_pair_tokens(int M, int N, int K);
 double gemm_tc_pair_time(int M, int N, int K, bool relu2);
-int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s);
+int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s, bool ahead = false);   // ahead: the weights are not the work of the kernel before
 
 }  // namespace wf

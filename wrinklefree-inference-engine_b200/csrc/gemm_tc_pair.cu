@@ -45,6 +45,7 @@ struct TpParams {
     int tn, n_tiles, tiles;
     int i2s;
     int akb, as;         // k-blocks per activation load, loads in flight
+    int ahead;           // the weights were complete long before: their loads and expansion do not wait for the kernel before, and the next one may come early
     int* err;            // the wait word
     EpiParams ep;
 };
@@ -205,7 +206,8 @@ __global__ void __launch_bounds__(tp_threads(NU), 1) ternary_gemm_pair_kernel(co
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
-    pdl_wait_prior();                                       // barriers, TMEM and the pair's meeting above overlap the kernel before
+    if (p.ahead) pdl_launch_dependents();
+    if (!p.ahead || warp < TP_EPW || warp == W_ACT) pdl_wait_prior();   // barriers, TMEM and the pair's meeting above overlap the kernel before
 
     if (warp == W_ACT) {
         // ------------------------------------------------------------ activations: this CTA's half of the tile's tokens
@@ -496,7 +498,7 @@ double gemm_tc_pair_time(int M, int N, int K, bool relu2) {
     return pair_time(M, N, K / WF_QK, tn, pairs) + (relu2 ? 0.4 * (double)((tiles + pairs - 1) / pairs) : 0.);      // the pairs' exchange of gate and up
 }
 
-int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s) {
+int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream_t s, bool ahead) {
     constexpr int NU = 3;
     EncodeTiledFn enc = tc_encoder();
     if (!enc) { set_error("gemm_tc_pair: cuTensorMapEncodeTiled unavailable"); return WF_ERR_CUDA; }
@@ -522,6 +524,7 @@ int launch_gemm_tc_pair(const wf_linear_args* a, const EpiParams& ep, cudaStream
     p.err = tc_wait_word();
     if (!p.err) { set_error("gemm_tc_pair: no wait word"); return WF_ERR_CUDA; }
     p.ep = ep;
+    p.ahead = ahead;
     CUtensorMap tq, tw;
     const cuuint32_t one[4] = {1, 1, 1, 1};
     {
