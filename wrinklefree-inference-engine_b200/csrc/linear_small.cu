@@ -257,21 +257,30 @@ __global__ void __launch_bounds__(LS_THREADS, 2) linear_small_kernel(const Small
 // ---------------------------------------------------------------------------------------------------------------
 // Standalone glue for large batch: grid = M rows, 256 threads; int8 codes / scale / rowsum go to global.
 constexpr int GR_T = 512;   // one pass iteration for K <= 4096, two for the 2B ffn width
+// IT > 0: the row stays in registers, IT vectors of eight a thread (K <= 4096 IT; sums of this GPU alone), the norm's weights requested ahead of the wait on the kernel
+// before; the same sums in the same order.  IT 0: through shared memory.  Batches above GLUE_LATE rows let the next kernel in behind their own wait: ahead of it a chain of
+// waiting kernels takes the SMs that the present one still needs (2B, 64 sequences 2.04 -> 1.97 ms a step, 8B 3.10 -> 3.05); up to there the next product's weights come early
+// (8B, 16 sequences 2.39 ms, 2.53 so).  Which form: launch_glue_rows.
+constexpr int GLUE_LATE = 32;
+template <int IT>
 __global__ void __launch_bounds__(GR_T) glue_rows_kernel(const GlueParams p) {
     extern __shared__ __align__(16) unsigned char gsm[];
     __nv_bfloat16* ys = reinterpret_cast<__nv_bfloat16*>(gsm);
     __shared__ float fs[32];
     __shared__ int is[32];
-    pdl_launch_dependents();
+    if (p.M <= GLUE_LATE) pdl_launch_dependents();
+    if (IT > 0) glue_prefetch_gamma<GR_T>(p);
     pdl_wait_prior();
     if (p.wait_flag >= 0) {
         if (threadIdx.x < 32) tp_wait_flags_warp(p.tp, p.wait_flag);
         __syncthreads();
     }
-    glue_zero_duty<GR_T>(p);
+    if (p.M > GLUE_LATE) pdl_launch_dependents();
     const int m = blockIdx.x;
     float sc; int rsum;
-    glue_row<1, GR_T>(p, m, ys, p.q_out + (size_t)m * p.K, fs, is, true, sc, rsum);
+    glue_zero_duty<GR_T>(p);
+    if (IT > 0) glue_row_regs<1, GR_T, IT ? IT : 1>(p, m, p.q_out + (size_t)m * p.K, fs, is, true, sc, rsum, QMAP_PLAIN);
+    else glue_row<1, GR_T>(p, m, ys, p.q_out + (size_t)m * p.K, fs, is, true, sc, rsum);
     if (threadIdx.x == 0) {
         if (p.scale_out) p.scale_out[m] = sc;
         if (p.rowsum_out) p.rowsum_out[m] = rsum;
@@ -384,6 +393,10 @@ int launch_glue_rows(const GlueParams& g, cudaStream_t s, bool pdl) {
         cfg.numAttrs = pdl ? 2 : 1;
         return launch_check(cudaLaunchKernelEx(&cfg, glue_rows_cluster_kernel, g), "glue_rows_cluster");
     }
+    // In registers: ms a step, through shared memory / so: 2B (rows of 2560 and 6912), 2 sequences 1.33 / 1.24, 16 1.58 / 1.53, 24 1.98 / 1.86, 48 1.71 / 1.67, 64 1.97 / 1.96;
+    // 8B (4096) 16 sequences 2.39 / 2.34, 24 3.13 / 3.03, but 8 2.01 / 2.04 and 64 3.05 / 3.14.
+    const bool odd = g.K > 3072 && g.K <= 8 * GR_T && (g.M <= 8 || g.M > GLUE_LATE);
+    const int it = g.mode == GL_RELU2 || g.acc_own_cols > 0 || odd || g.K > 2 * 8 * GR_T ? 0 : g.K > 8 * GR_T ? 2 : 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g.M);
     cfg.blockDim = dim3(GR_T);
@@ -391,7 +404,7 @@ int launch_glue_rows(const GlueParams& g, cudaStream_t s, bool pdl) {
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     set_pdl(cfg, at, pdl);
-    return launch_check(cudaLaunchKernelEx(&cfg, glue_rows_kernel, g), "glue_rows");
+    return launch_check(cudaLaunchKernelEx(&cfg, it == 1 ? glue_rows_kernel<1> : it == 2 ? glue_rows_kernel<2> : glue_rows_kernel<0>, g), "glue_rows");
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -439,7 +452,7 @@ int launch_h_exchange(const HExchangeArgs& a, cudaStream_t s, bool pdl) {
 void linear_small_init_attrs() {
     cudaFuncSetAttribute(linear_small_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     cudaFuncSetAttribute(linear_small_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    cudaFuncSetAttribute(glue_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
+    cudaFuncSetAttribute(glue_rows_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
 }
 
 }  // namespace wf
