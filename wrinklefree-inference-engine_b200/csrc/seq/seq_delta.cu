@@ -361,8 +361,8 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(Batch b, DeltaDi
 
 // thread per (sequence, head, state element): chains the chunks' start states from the slot's state and leaves the end state in the slot.
 // prod has one entry per (chunk, head), or (d > 0) one per (chunk, head, key row) of dd / d state columns each
-__global__ void scan_prefix_kernel(Batch b, int H, int dd, int chunk, float* __restrict__ state, size_t slot_stride, const float* __restrict__ local,
-                                   float* __restrict__ startws, const float* __restrict__ prod, int d) {
+__global__ void scan_prefix_kernel(Batch b, int H, int dd, int chunk, float* __restrict__ state, size_t slot_stride, const float* local,
+                                   float* __restrict__ startws, const float* prod, int d) {
     pdl_enter();
     const int sq = blockIdx.x, h = blockIdx.y, e = blockIdx.z * blockDim.x + threadIdx.x;
     if (e >= dd) return;
