@@ -534,3 +534,15 @@ def test_command_line_trace_replay_and_generate(tmp_path):
             if top2[1] - top2[0] > 1e-3 * np.abs(lg).max():
                 assert int(np.argmax(lg)) == t
             seq.append(t)
+
+
+@pytest.mark.parametrize("width", [12, 1024, 1028, 1030, 8192, 8196])
+def test_one_gain_norms_of_row_widths_where_their_forms_change(width):
+    """Rows of less than a warp, one group of four a thread up to 1024 and two beyond, one element a thread where the width is no multiple of four or above 8192."""
+    cfg = config([with_ff(attn(heads=2, kv_heads=1, dim=8, vdim=8), dense(ff=8))], width=width, vocab=40)
+    w = make_weights(cfg, width)
+    m = build(cfg, w)
+    toks = tokens_for(cfg, 5, width)
+    got = m.step([m.admit()], [5], toks, range(5))
+    m.close()
+    assert_close(got, oracle_logits(cfg, w, toks), "float32", width)

@@ -69,20 +69,22 @@ __device__ __forceinline__ float warp_max(float v) {
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
 }
-// sum over a block of up to 1024 threads; every thread gets the result.  scratch: 33 floats of shared memory
+// sum over a block of up to 1024 threads; every thread gets the result (every warp adds the warps' sums for itself).  scratch: 33 floats of shared memory
 __device__ __forceinline__ float block_sum(float v, float* scratch) {
     v = warp_sum(v);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
     __syncthreads();
     if (lane == 0) scratch[w] = v;
     __syncthreads();
-    if (w == 0) {
-        float t = lane < nw ? scratch[lane] : 0.f;
-        t = warp_sum(t);
-        if (lane == 0) scratch[32] = t;
-    }
+    return warp_sum(lane < nw ? scratch[lane] : 0.f);
+}
+// the same where nothing else uses the scratch before
+__device__ __forceinline__ float block_sum_once(float v, float* scratch) {
+    v = warp_sum(v);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    if (lane == 0) scratch[w] = v;
     __syncthreads();
-    return scratch[32];
+    return warp_sum(lane < nw ? scratch[lane] : 0.f);
 }
 __device__ __forceinline__ float gelu_erf_f(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }
 __device__ __forceinline__ float epilogue_f(int ep, float v) {        // GemmArgs::ep

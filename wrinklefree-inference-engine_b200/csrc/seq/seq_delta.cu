@@ -124,15 +124,16 @@ __global__ void __launch_bounds__(512) ssd_post_vec_kernel(int H, int dv, int gr
     const int i = blockIdx.x, g = blockIdx.y;
     const int inner = H * dv, gw = inner / groups, e = threadIdx.x * 4, c = g * gw + e;
     float v[4] = {0.f, 0.f, 0.f, 0.f};
+    float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
     if (e < gw) {
+        m = load4(w + c);
         const float4 ov = load4(o + (size_t)i * inner + c), xv = load4(x + (size_t)i * ldx + c), zv = load4(z + (size_t)i * ldz + c);
         const float dk = to_f(Dskip[c / dv]);
         v[0] = (ov.x + dk * xv.x) * silu_f(zv.x); v[1] = (ov.y + dk * xv.y) * silu_f(zv.y); v[2] = (ov.z + dk * xv.z) * silu_f(zv.z); v[3] = (ov.w + dk * xv.w) * silu_f(zv.w);
     }
-    const float ss = block_sum(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3], scratch);
+    const float ss = block_sum_once(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3], scratch);
     const float inv = 1.f / sqrtf(ss / (float)gw + eps);
     if (e < gw) {
-        const float4 m = load4(w + c);
         const float r[4] = {v[0] * inv * m.x, v[1] * inv * m.y, v[2] * inv * m.z, v[3] * inv * m.w};
         store4(y + (size_t)i * inner + c, r);
     }

@@ -139,10 +139,62 @@ __global__ void __launch_bounds__(SN_THREADS) scalar_rmsnorm_kernel(const float*
     }
 }
 
+// rows of four-element groups in registers: groups per thread and threads
+inline int vec_groups(int W) { return W <= 1024 ? 1 : 2; }
+inline int vec_threads(int W) { const int nv = vec_groups(W); return (W / 4 + nv * 32 - 1) / (nv * 32) * 32; }
+
+// The same with four consecutive elements per load, rows of up to 8192: the weights are requested ahead of the wait on the kernel before, all of a row's inputs before the
+// first is used.  What bounds it is a latency (8 rows of 1024 in a decode step of the engine, behind products of few rows: 4.5 and 3.3 us one element at a time, 1.5 so).
+template <typename T, int NV>
+__global__ void __launch_bounds__(1024) scalar_rmsnorm_vec_kernel(const float* y, int ldy, const T* bias, const T* gain, float mult, float eps, int W, const float* res, float* out,
+                                                                  int ldo, T* __restrict__ out_t, int ldt, const int32_t* rows) {
+    __shared__ float scratch[33];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v[NV], bv[NV], rv[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int c = (threadIdx.x + k * blockDim.x) * 4;
+        bv[k] = bias && c < W ? load4(bias + c) : zero;
+    }
+    const float g = to_f(gain[0]);
+    pdl_enter();
+    const int i = blockIdx.x, src = rows ? rows[i] : i;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int c = (threadIdx.x + k * blockDim.x) * 4;
+        v[k] = c < W ? load4(y + (size_t)src * ldy + c) : zero;
+        rv[k] = c < W && res ? load4(res + (size_t)src * ldo + c) : zero;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        v[k] = make_float4(v[k].x + bv[k].x, v[k].y + bv[k].y, v[k].z + bv[k].z, v[k].w + bv[k].w);
+        ss = fmaf(v[k].x, v[k].x, fmaf(v[k].y, v[k].y, fmaf(v[k].z, v[k].z, fmaf(v[k].w, v[k].w, ss))));
+    }
+    ss = block_sum_once(ss, scratch);
+    const float f = mult * g / sqrtf(ss / (float)W + eps);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int c = (threadIdx.x + k * blockDim.x) * 4;
+        if (c >= W) continue;
+        float o[4] = {v[k].x * f, v[k].y * f, v[k].z * f, v[k].w * f};
+        if (res) { o[0] += rv[k].x; o[1] += rv[k].y; o[2] += rv[k].z; o[3] += rv[k].w; }
+        if (out) store4(out + (size_t)i * ldo + c, o);
+        if (out_t) store4(out_t + (size_t)i * ldt + c, o);
+    }
+}
+
 int launch_scalar_rmsnorm(int dt, const float* y, int ldy, const void* bias, const void* gain, float mult, float eps, int n, int W, const float* res, float* out,
                           int ldo, void* out_t, int ldt, const int32_t* rows, cudaStream_t s) {
     if (n <= 0) return WF_OK;
     if (res && rows && out == res) { set_error("scalar_rmsnorm: gathered rows cannot be added in place"); return WF_ERR_INVALID; }
+    if (W % 4 == 0 && W <= 8192 && ldy % 4 == 0 && ldo % 4 == 0 && ldt % 4 == 0 && vec_ok(y, 16) && vec_ok(res, 16) && vec_ok(out, 16) && vec_ok(bias, 16) && vec_ok(out_t, 16)) {
+#define SN_LAUNCH(T, NV) launch_pdl(scalar_rmsnorm_vec_kernel<T, NV>, n, vec_threads(W), 0, s, y, ldy, (const T*)bias, (const T*)gain, mult, eps, W, res, out, ldo, (T*)out_t, ldt, rows)
+        if (dt == WF_BF16) { if (vec_groups(W) == 1) SN_LAUNCH(__nv_bfloat16, 1); else SN_LAUNCH(__nv_bfloat16, 2); }
+        else { if (vec_groups(W) == 1) SN_LAUNCH(float, 1); else SN_LAUNCH(float, 2); }
+#undef SN_LAUNCH
+        return launch_check(cudaGetLastError(), "scalar_rmsnorm_vec");
+    }
     if (dt == WF_BF16) launch_pdl(scalar_rmsnorm_kernel<__nv_bfloat16>, n, SN_THREADS, 0, s, y, ldy, (const __nv_bfloat16*)bias, (const __nv_bfloat16*)gain, mult, eps, W, res, out, ldo, (__nv_bfloat16*)out_t, ldt, rows);
     else launch_pdl(scalar_rmsnorm_kernel<float>, n, SN_THREADS, 0, s, y, ldy, (const float*)bias, (const float*)gain, mult, eps, W, res, out, ldo, (float*)out_t, ldt, rows);
     return launch_check(cudaGetLastError(), "scalar_rmsnorm");
@@ -213,7 +265,7 @@ __global__ void __launch_bounds__(1024) group_rmsnorm_vec_kernel(const float* x,
         if (x2) v[k] = make_float4(a * v[k].x + b * v2[k].x, a * v[k].y + b * v2[k].y, a * v[k].z + b * v2[k].z, a * v[k].w + b * v2[k].w);
         ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
     }
-    ss = block_sum(ss, scratch);
+    ss = block_sum_once(ss, scratch);
     const float inv = 1.f / sqrtf(ss / (float)gw + eps);
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
@@ -225,10 +277,6 @@ __global__ void __launch_bounds__(1024) group_rmsnorm_vec_kernel(const float* x,
         if (y_t) store4(y_t + (size_t)i * ldt + (size_t)g * gw + c, o);
     }
 }
-
-// rows of four-element groups in registers: groups per thread and threads
-inline int vec_groups(int W) { return W <= 1024 ? 1 : 2; }
-inline int vec_threads(int W) { const int nv = vec_groups(W); return (W / 4 + nv * 32 - 1) / (nv * 32) * 32; }
 
 int launch_group_rmsnorm(int dt, const float* x, int ldx, const void* w, int groups, float eps, int n, int W, const float* res, float* y,
                          int ldy, void* y_t, int ldt, const int32_t* rows, cudaStream_t s, const float* x2, float a, float b, float w_offset) {
@@ -329,19 +377,25 @@ __global__ void __launch_bounds__(1024) add_dual_norm_vec_kernel(float* __restri
         ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
     }
     if (!w1 && !w2) return;
-    ss = block_sum(ss, scratch);
+    float4 m1[NV], m2[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int c = (threadIdx.x + k * blockDim.x) * 4;
+        m1[k] = w1 && c < W ? load4(w1 + c) : zero;
+        m2[k] = w2 && c < W ? load4(w2 + c) : zero;
+    }
+    ss = block_sum_once(ss, scratch);
     const float inv = 1.f / sqrtf(ss / (float)W + eps);
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
         const int c = (threadIdx.x + k * blockDim.x) * 4;
         if (c >= W) continue;
-        auto scaled = [&](const T* w, T* h) {
-            const float4 m = load4(w + c);
+        auto scaled = [&](const float4& m, T* h) {
             const float o[4] = {v[k].x * inv * (w_offset + m.x), v[k].y * inv * (w_offset + m.y), v[k].z * inv * (w_offset + m.z), v[k].w * inv * (w_offset + m.w)};
             store4(h + base + c, o);
         };
-        if (w1) scaled(w1, h1);
-        if (w2) scaled(w2, h2);
+        if (w1) scaled(m1[k], h1);
+        if (w2) scaled(m2[k], h2);
     }
 }
 
