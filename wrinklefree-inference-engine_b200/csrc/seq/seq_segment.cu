@@ -478,10 +478,11 @@ size_t segment_workspace_floats(const DeltaDims& D, int max_step_tokens, int slo
 // Long portions only: a segment moves its state five times through memory and its blocks cost their latencies however few the tokens.  us, 16 tokens at a time -> so:
 // 40 heads of 128 x 64, one portion of 256 tokens 38 / 48, of 512 67 / 67, 1024 104 / 88, 2048 173 / 131; 4 of 300 84 / 102, 4 of 512 134 / 132, 2 of 1024 162 / 130;
 // 16 heads of 64 x 64, one of 256 25 / 32, 512 35 / 34, 2048 63 / 46; 4 of 300 35 / 44, 4 of 512 53 / 46.
+// Three portions and more of about one length fill the machine 16 tokens at a time: 40 heads, 3 of 600 115 / 125, but one of 801, 600 and 400 141 / 129.
 bool segments_usable(const Batch& b, const DeltaDims& D, const ScanWorkspace* scan) {
-    const long long segs = b.n / SG + b.nseq + 1;
-    return D.no_delta && !D.vec_decay && b.max_len >= 4 * SG && b.n >= 3LL * SG * b.nseq && scan->local && segs <= scan->chunks &&
-           (size_t)segs * D.Hk * SG_G <= scan->rec_floats && D.H + D.Hk <= 65535;
+    const long long segs = b.n / SG + b.nseq + 1, tiles = (long long)b.nseq * D.H * ((D.dv + D.ones_col + CR_COLS - 1) / CR_COLS);
+    return D.no_delta && !D.vec_decay && b.max_len >= 4 * SG && b.n >= 3LL * SG * b.nseq && (tiles < 3 * sm_count() || 5LL * b.max_len > 2LL * b.n) && scan->local &&
+           segs <= scan->chunks && (size_t)segs * D.Hk * SG_G <= scan->rec_floats && D.H + D.Hk <= 65535;
 }
 
 int launch_segments(const Batch& b, const DeltaDims& D, const ChunkView& w, const float* decay, float* state, size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan) {
