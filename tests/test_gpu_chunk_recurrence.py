@@ -67,6 +67,17 @@ def test_delta_rule_of_many_heads(heads, kv_heads, dim, vdim):
     check(cfg, w, {"l0.mix.a1": (8, W), "l0.mix.g1": (8, W)}, lambda x: NO.channel_delta(x, d64(w, "l0.mix."), "", m, EPS), [90, 64], [[32, 17], [15, 47], [43, 0]], W)
 
 
+@pytest.mark.parametrize("lens", [[200, 330], [330, 200], [60, 400, 90]])
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(20, 10, 128, 128), (12, 12, 64, 97), (30, 10, 68, 33)])
+def test_delta_rule_of_portions_of_unequal_length(heads, kv_heads, dim, vdim, lens):
+    """The longest portion in blocks of one column tile, wherever it stands, and the others in blocks of two (an odd last one), each behind a carried state."""
+    W = 40
+    m = {"heads": heads, "kv_heads": kv_heads, "dim": dim, "vdim": vdim, "conv": 4}
+    cfg = {"architecture": "Nukezen", "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": EPS}, "layers": [{"type": "channel_delta", "mixer": m, "mlp": None}]}
+    w = NO.random_weights(cfg, 1, {0: {"rank_a": 8, "rank_g": 8}})
+    check(cfg, w, {"l0.mix.a1": (8, W), "l0.mix.g1": (8, W)}, lambda x: NO.channel_delta(x, d64(w, "l0.mix."), "", m, EPS), lens, [[3] * len(lens), [n - 3 for n in lens]], W, 1000)
+
+
 @pytest.mark.parametrize("conv", [2, 3])
 def test_convolutions_of_two_and_three_taps_over_many_tokens(conv):
     """Enough tokens x channels (6400) that a thread of the convolution takes eight tokens one after another: portions that begin and end inside such a run, behind a carried

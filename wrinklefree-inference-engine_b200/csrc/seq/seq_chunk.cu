@@ -56,8 +56,9 @@ __device__ __forceinline__ float cr_reduce(float (&v)[CR], int p) {
     return v[0];
 }
 
+// (128 registers in place of 167, a few of them spilled, where the correction takes most: four blocks an SM instead of three; 20 heads of 128 x 128, 1801 tokens 47 -> 40 us)
 template <int DS, bool VEC, bool DELTA>
-__global__ void __launch_bounds__(CR_THREADS) chunk_prep_kernel(Batch b, DeltaDims D, ChunkView w) {
+__global__ void __launch_bounds__(CR_THREADS, DS == 128 && DELTA ? 4 : 0) chunk_prep_kernel(Batch b, DeltaDims D, ChunkView w) {
     pdl_enter();
     constexpr int Q4 = DS / 64;             // float4 per lane part
     __shared__ __align__(16) float ks[CR][DS], qs[CR][DS], gs[VEC ? CR : 1][VEC ? DS : 4];
@@ -187,16 +188,17 @@ constexpr int CR_RS = 24;                                 // row stride of the p
 // CT: tiles of 16 columns that a block takes.  The key and query rows that the products need as sums of two numbers are split once for all of them; without the
 // correction that splitting was the larger part of the work (the two passes over 40 heads of 128 x 64, 2048 tokens: 63 + 97 us with one, 48 + 78 with two).
 // Which one: two_tiles.
+// sq, seg: the sequence and its segment; tile0: the first of the block's column tiles.
 template <int DS, bool VEC, bool DELTA, int CT>
-__global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
-    pdl_enter();
+__device__ __forceinline__ void chunk_scan(const Batch b, const DeltaDims D, const ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, const Segments sg,
+                                           const int sq, const int seg, const int h, const int tile0) {
     using L = CrStage<DS, VEC, DELTA>;
     constexpr int REC = cr_rec_floats(DS, VEC), NT = DS / (8 * CR_WARPS), STEP = CR_THREADS / (DS / 4);
     constexpr int PARTS = DELTA ? 2 * CT : 2;              // partial sums of a warp: S^T q of each column tile, then R of each
     extern __shared__ __align__(16) float sm[];
     float* red = sm + 2 * L::FLOATS;                      // [4 warps][PARTS][16 columns][CR_RS]
-    const int sq = blockIdx.x / sg.n, seg = blockIdx.x - sq * sg.n, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    const int col0 = blockIdx.z * CR_COLS * CT, dvs = D.dv + D.ones_col, kh = h / (D.H / D.Hk);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int col0 = tile0 * CR_COLS, dvs = D.dv + D.ones_col, kh = h / (D.H / D.Hk);
     const int first = seg * SCAN_CHUNK, seq0 = b.seq_start[sq], start = seq0 + first;
     const int len = sg.pass ? min(SCAN_CHUNK, b.seq_len[sq] - first) : b.seq_len[sq], nch = (len + CR - 1) / CR;
     if (len <= 0) return;                                 // this sequence has fewer segments
@@ -448,8 +450,8 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
 #pragma unroll
             for (int e = 0; e < 4; ++e) cr_watch(watch[e], s[ct][nt][e]);
     const int lost = __syncthreads_or(!((watch[0] + watch[1]) + (watch[2] + watch[3]) == 0.f));
-    int* mark = w.redo + ((size_t)sq * D.H + h) * w.cols + blockIdx.z * CT;      // the preparation marks all of a head's tiles
-    const int tiles = min(CT, w.cols - (int)blockIdx.z * CT);
+    int* mark = w.redo + ((size_t)sq * D.H + h) * w.cols + tile0;      // the preparation marks all of a head's tiles
+    const int tiles = min(CT, w.cols - tile0);
     if (lost && tid < tiles) mark[tid] = 1;
     if (sg.pass == 3) return;                             // scan_prefix_kernel has left the end states
     if (sg.pass == 0 && (lost || *mark)) return;          // the slot keeps the start state for chunk_redo_kernel
@@ -460,7 +462,37 @@ __global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDi
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
             for (int e = 0; e < 4; ++e) { bool ok; const size_t i = at_state(ct, nt, e, ok); if (ok) S1[i] = s[ct][nt][e]; }
-    if (!VEC && sg.pass && blockIdx.z == 0 && tid == 0) sg.prod[(size_t)(seq0 / SCAN_CHUNK + sq + seg) * D.H + h] = prod;
+    if (!VEC && sg.pass && tile0 == 0 && tid == 0) sg.prod[(size_t)(seq0 / SCAN_CHUNK + sq + seg) * D.H + h] = prod;
+}
+
+template <int DS, bool VEC, bool DELTA, int CT>
+__global__ void __launch_bounds__(CR_THREADS) chunk_scan_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o, Segments sg) {
+    pdl_enter();
+    const int sq = blockIdx.x / sg.n;
+    chunk_scan<DS, VEC, DELTA, CT>(b, D, w, state, slot_stride, o, sg, sq, blockIdx.x - sq * sg.n, blockIdx.y, blockIdx.z * CT);
+}
+
+// The longest portion in blocks of one column tile, handed out first, the others in blocks of two (mixed_tiles): the sequence that the scan waits for goes its chain with
+// less beside it, and two blocks fit every SM.
+template <int DS, bool VEC, bool DELTA>
+__global__ void __launch_bounds__(CR_THREADS, 2) chunk_scan_mixed_kernel(Batch b, DeltaDims D, ChunkView w, float* __restrict__ state, size_t slot_stride, float* __restrict__ o) {
+    pdl_enter();
+    int longest = 0;
+    for (int s = 1; s < b.nseq; ++s) if (b.seq_len[s] > b.seq_len[longest]) longest = s;
+    const Segments whole;
+    int i = blockIdx.x;
+    const int ones = D.H * w.cols, pairs = (w.cols + 1) / 2;
+    if (i < ones) {
+        const int h = i / w.cols;
+        chunk_scan<DS, VEC, DELTA, 1>(b, D, w, state, slot_stride, o, whole, longest, 0, h, i - h * w.cols);
+        return;
+    }
+    i -= ones;
+    int sq = i / (D.H * pairs);
+    i -= sq * D.H * pairs;
+    const int h = i / pairs;
+    if (sq >= longest) ++sq;
+    chunk_scan<DS, VEC, DELTA, 2>(b, D, w, state, slot_stride, o, whole, sq, 0, h, 2 * (i - h * pairs));
 }
 
 // The marked portions again, token by token (see above), a block per (sequence, head, 16 columns); their start state is still in the slot, or, with segments,
@@ -553,6 +585,19 @@ bool two_tiles(long long tiles, long long pairs) {
     return 3 * two < 2 * one;
 }
 
+// Whether the longest of a few portions is taken in blocks of one column tile and the others in blocks of two, by the same times: with 2.1 us a chunk where one of each share
+// an SM.  us, all blocks alike -> so: 20 heads of 128 x 128, 741 and 1060 tokens 231 / 191, 100 and 1700 336 / 272, 2 of 1024 228 / 213; 8 heads of 64 x 128, 400, 600 and
+// 801 tokens 89 / 68.
+bool mixed_tiles(const Batch& b, int H, int cols) {
+    const long long sms = sm_count(), ones = (long long)H * cols, pairs = (long long)H * ((cols + 1) / 2), blocks = ones + (b.nseq - 1) * pairs;
+    if (b.nseq < 2 || b.nseq > 16 || blocks > 2 * sms || b.max_len <= 0) return false;
+    const double rest = (double)(b.n - b.max_len) / (b.nseq - 1), len = b.max_len;
+    auto alone = [](double one, double two, double more, long long n) { return n <= 1 ? one : n == 2 ? two : more * n; };
+    const double t1 = len * alone(1.2, 1.7, 0.84, (b.nseq * ones + sms - 1) / sms), t2 = len * alone(1.5, 2.6, 1.3, (b.nseq * pairs + sms - 1) / sms);
+    const double shared = blocks > sms ? 2.1 * rest + 1.2 * (len - rest) : 1.5 * rest, own = len * (ones > sms ? 1.7 : 1.2);
+    return (shared > own ? shared : own) < 0.95 * (t1 < t2 ? t1 : t2);
+}
+
 template <int DS, bool VEC, bool DELTA, int CT>
 int cr_scan(const Batch& b, const DeltaDims& D, const ChunkView& w, float* state, size_t slot_stride, float* o, const Segments& sg, cudaStream_t s) {
     const int cols = w.cols;
@@ -581,6 +626,16 @@ int cr_launch(const Batch& b, const DeltaDims& D, const ChunkView& w, const floa
     }
     launch_pdl(chunk_prep_kernel<DS, VEC, DELTA>, dim3(b.nseq * w.nchunks, D.H), CR_THREADS, 0, s, b, D, w);
     if (int rc = launch_check(cudaGetLastError(), "chunk_prep")) return rc;
+    if constexpr (DELTA) {
+        if (mixed_tiles(b, D.H, cols)) {
+            constexpr size_t smem = (size_t)(2 * CrStage<DS, VEC, DELTA>::FLOATS + CR_WARPS * 4 * CR_COLS * CR_RS) * sizeof(float);
+            static DevOnce once;
+            if (once.need() && cuda_check(cudaFuncSetAttribute(chunk_scan_mixed_kernel<DS, VEC, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "chunk shared memory")) return WF_ERR_CUDA;
+            chunk_scan_mixed_kernel<DS, VEC, DELTA><<<D.H * cols + (b.nseq - 1) * D.H * ((cols + 1) / 2), CR_THREADS, smem, s>>>(b, D, w, state, slot_stride, o);
+            if (int rc = launch_check(cudaGetLastError(), "chunk_scan_mixed")) return rc;
+            return redo();
+        }
+    }
     auto scan_pass = [&](int pass) {
         sg.pass = pass;
         const long long chains = (long long)b.nseq * sg.n * D.H, tiles = chains * cols;
