@@ -80,7 +80,7 @@ def test_delta_rule_of_portions_of_unequal_length(heads, kv_heads, dim, vdim, le
 
 @pytest.mark.parametrize("conv", [2, 3])
 def test_convolutions_of_two_and_three_taps_over_many_tokens(conv):
-    """Enough tokens x channels (6400) that a thread of the convolution takes eight tokens one after another: portions that begin and end inside such a run, behind a carried
+    """Enough tokens x channels (6400) that a thread of the convolution takes four tokens one after another: portions that begin and end inside such a run, behind a carried
     state of one and two inputs, and a portion of one token."""
     W = 40
     m = {"heads": 40, "kv_heads": 20, "dim": 64, "vdim": 96, "conv": conv}

@@ -771,26 +771,56 @@ __global__ void causal_taps_kernel(Batch b, const float* in, int ld_in, const T*
     }
 }
 
-// Many tokens: a thread takes four channels of TR tokens one after another, so an input is read once instead of once per tap, all of the run's inputs are
-// requested before the first is used, and the weights are read once a run.  1801 tokens x 5120 channels, four taps (74 MB): 63 to 72 us a channel and
-// token per thread, 21 so.  Sums in the same order as above.
-constexpr int TR = 8;
+// Many tokens: a thread takes four channels of TR tokens one after another, so an input is read once instead of once per tap.  The weights are requested ahead of the
+// wait on the kernel before; the run's inputs and the TAPS - 1 before it all at once, whether or not its portion begins there: only a run in which one begins looks token
+// by token for where its window comes from.  Sums in the same order as above.  1801 tokens x 5120 channels, four taps (74 MB): 63 to 72 us a channel and token per
+// thread, 24 with eight tokens a run, the window asked for behind the token's sequence and the weights one by one, 21.6 so.
+constexpr int TR = 4;
 template <typename T, int TAPS>
 __global__ void __launch_bounds__(128) causal_taps_run_kernel(Batch b, const float* in, int ld_in, const T* w, int C, const float* state,
                                                               size_t slot_stride, int identity, int silu, T* __restrict__ out_t, int ld_t, float* __restrict__ out_f, int ld_f,
                                                               const T* bias) {
-    pdl_enter();
     const int c = (blockIdx.y * 128 + threadIdx.x) * 4, i0 = blockIdx.x * TR;
-    if (c >= C) return;
-    float4 cur[TR];
+    const bool mine = c < C;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float wf[4 * TAPS];                                   // four channels' taps lie side by side
 #pragma unroll
-    for (int t = 0; t < TR; ++t)
-        if (i0 + t < b.n) cur[t] = load4(in + (size_t)(i0 + t) * ld_in + c);
-    float4 wt[TAPS], win[TAPS];
+    for (int j = 0; j < TAPS; ++j) {
+        const float4 v = mine ? load4(w + (size_t)c * TAPS + 4 * j) : zero;
+        wf[4 * j] = v.x; wf[4 * j + 1] = v.y; wf[4 * j + 2] = v.z; wf[4 * j + 3] = v.w;
+    }
+    const float4 bs = mine && bias ? load4(bias + c) : zero;
+    pdl_enter();
+    if (!mine) return;
+    const int sq0 = b.tok_seq[i0];
+    float4 cur[TR], win[TAPS];
 #pragma unroll
-    for (int j = 0; j < TAPS; ++j)
-        wt[j] = make_float4(to_f(w[(size_t)c * TAPS + j]), to_f(w[(size_t)(c + 1) * TAPS + j]), to_f(w[(size_t)(c + 2) * TAPS + j]), to_f(w[(size_t)(c + 3) * TAPS + j]));
-    const float4 bs = bias ? load4(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < TAPS - 1; ++j) { const int i = i0 - (TAPS - 1) + j; win[j] = i >= 0 ? load4(in + (size_t)i * ld_in + c) : zero; }
+#pragma unroll
+    for (int t = 0; t < TR; ++t) cur[t] = i0 + t < b.n ? load4(in + (size_t)(i0 + t) * ld_in + c) : zero;
+    const int start0 = b.seq_start[sq0];
+    const bool plain = i0 - (TAPS - 1) >= start0 && min(i0 + TR, b.n) <= start0 + b.seq_len[sq0];       // the run and its window within one portion
+    auto put = [&](int i, const float4& x) {
+        win[TAPS - 1] = x;
+        float4 acc = identity ? x : zero;
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            acc.x = fmaf(wf[j], win[j].x, acc.x); acc.y = fmaf(wf[TAPS + j], win[j].y, acc.y);
+            acc.z = fmaf(wf[2 * TAPS + j], win[j].z, acc.z); acc.w = fmaf(wf[3 * TAPS + j], win[j].w, acc.w);
+        }
+        float o[4] = {acc.x, acc.y, acc.z, acc.w};
+        if (bias) { o[0] += bs.x; o[1] += bs.y; o[2] += bs.z; o[3] += bs.w; }
+        if (silu) { o[0] = silu_f(o[0]); o[1] = silu_f(o[1]); o[2] = silu_f(o[2]); o[3] = silu_f(o[3]); }
+        if (out_t) store4(out_t + (size_t)i * ld_t + c, o);
+        if (out_f) store4(out_f + (size_t)i * ld_f + c, o);
+#pragma unroll
+        for (int j = 0; j + 1 < TAPS; ++j) win[j] = win[j + 1];
+    };
+    if (plain) {
+#pragma unroll
+        for (int t = 0; t < TR; ++t) if (i0 + t < b.n) put(i0 + t, cur[t]);
+        return;
+    }
 #pragma unroll
     for (int t = 0; t < TR; ++t) {
         const int i = i0 + t;
@@ -804,20 +834,7 @@ __global__ void __launch_bounds__(128) causal_taps_run_kernel(Batch b, const flo
                 win[j] = src >= 0 ? load4(in + (size_t)(i - li + src) * ld_in + c) : load4(st + (size_t)(src + TAPS - 1) * C);
             }
         }
-        win[TAPS - 1] = cur[t];
-        float4 acc = identity ? cur[t] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < TAPS; ++j) {
-            acc.x = fmaf(wt[j].x, win[j].x, acc.x); acc.y = fmaf(wt[j].y, win[j].y, acc.y);
-            acc.z = fmaf(wt[j].z, win[j].z, acc.z); acc.w = fmaf(wt[j].w, win[j].w, acc.w);
-        }
-        float o[4] = {acc.x, acc.y, acc.z, acc.w};
-        if (bias) { o[0] += bs.x; o[1] += bs.y; o[2] += bs.z; o[3] += bs.w; }
-        if (silu) { o[0] = silu_f(o[0]); o[1] = silu_f(o[1]); o[2] = silu_f(o[2]); o[3] = silu_f(o[3]); }
-        if (out_t) store4(out_t + (size_t)i * ld_t + c, o);
-        if (out_f) store4(out_f + (size_t)i * ld_f + c, o);
-#pragma unroll
-        for (int j = 0; j + 1 < TAPS; ++j) win[j] = win[j + 1];
+        put(i, cur[t]);
     }
 }
 
@@ -825,10 +842,10 @@ int launch_causal_taps(int dt, const Batch& b, const float* in, int ld_in, const
                        size_t slot_stride, int identity, int silu, void* out_t, int ld_t, float* out_f, int ld_f, cudaStream_t s, const void* bias) {
     if (b.n <= 0) return WF_OK;
     if (taps < 1) { set_error("causal_taps: taps %d", taps); return WF_ERR_INVALID; }
-    // runs of tokens where they fill the SMs twice: below, a thread's eight tokens in a row are the longer way
+    // runs of tokens where they fill the SMs twice: below, a thread's tokens in a row are the longer way
     const int runs = (b.n + TR - 1) / TR, cblocks = (C / 4 + 127) / 128;
     if (taps >= 2 && taps <= 4 && C % 4 == 0 && (long long)runs * cblocks >= 2 * sm_count() && ld_in % 4 == 0 && ld_t % 4 == 0 && ld_f % 4 == 0 && slot_stride % 4 == 0 &&
-        vec_ok(in, 16) && vec_ok(state, 16) && vec_ok(out_t, 16) && vec_ok(out_f, 16) && vec_ok(bias, 16)) {
+        vec_ok(in, 16) && vec_ok(state, 16) && vec_ok(out_t, 16) && vec_ok(out_f, 16) && vec_ok(bias, 16) && vec_ok(w, 16)) {
 #define CT_LAUNCH(T, N) launch_pdl(causal_taps_run_kernel<T, N>, dim3(runs, cblocks), 128, 0, s, b, in, ld_in, (const T*)w, C, state, slot_stride, identity, silu, (T*)out_t, ld_t, out_f, ld_f, (const T*)bias)
         if (dt == WF_BF16) { if (taps == 2) CT_LAUNCH(__nv_bfloat16, 2); else if (taps == 3) CT_LAUNCH(__nv_bfloat16, 3); else CT_LAUNCH(__nv_bfloat16, 4); }
         else { if (taps == 2) CT_LAUNCH(float, 2); else if (taps == 3) CT_LAUNCH(float, 3); else CT_LAUNCH(float, 4); }
@@ -841,8 +858,9 @@ int launch_causal_taps(int dt, const Batch& b, const float* in, int ld_in, const
     return launch_check(cudaGetLastError(), "causal_taps");
 }
 
-// thread per (sequence, channel): state[k] <- input at portion index len - (taps - 1) + k, taken from the old state when that is negative.
-// Ascending k is safe in place: entry k reads old entry len + k > k.
+// thread per (sequence, channel): state[k] <- input at portion index len - (taps - 1) + k, taken from the old state when that is negative: all of a channel's entries are
+// read before the first is written, up to TS at a time (ascending k: entry k reads old entry len + k > k).
+constexpr int TS = 4;
 __global__ void taps_state_kernel(Batch b, const float* in, int ld_in, int taps, int C, float* __restrict__ state, size_t slot_stride,
                                   int skip_single) {
     pdl_enter();
@@ -851,16 +869,22 @@ __global__ void taps_state_kernel(Batch b, const float* in, int ld_in, int taps,
     if (skip_single && len == 1) return;                 // rolled by the fused norm + taps kernel
     float* st = state + (size_t)b.seq_slot[sq] * slot_stride;
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < C; c += gridDim.y * blockDim.x) {
-        for (int k = 0; k < taps - 1; ++k) {
-            const int src = len - (taps - 1) + k;
-            st[(size_t)k * C + c] = src >= 0 ? in[(size_t)(start + src) * ld_in + c] : st[(size_t)(src + taps - 1) * C + c];
+        for (int k0 = 0; k0 < taps - 1; k0 += TS) {
+            float v[TS];
+#pragma unroll
+            for (int k = 0; k < TS; ++k) {
+                const int src = len - (taps - 1) + k0 + k;
+                if (k0 + k < taps - 1) v[k] = src >= 0 ? in[(size_t)(start + src) * ld_in + c] : st[(size_t)(src + taps - 1) * C + c];
+            }
+#pragma unroll
+            for (int k = 0; k < TS; ++k) if (k0 + k < taps - 1) st[(size_t)(k0 + k) * C + c] = v[k];
         }
     }
 }
 
 int launch_taps_state(const Batch& b, const float* in, int ld_in, int taps, int C, float* state, size_t slot_stride, cudaStream_t s, int skip_single) {
     if (b.nseq <= 0 || taps <= 1) return WF_OK;
-    dim3 grid(b.nseq, (C + 255) / 256 > 8 ? 8 : (C + 255) / 256);
+    dim3 grid(b.nseq, (C + 255) / 256 > 64 ? 64 : (C + 255) / 256);
     launch_pdl(taps_state_kernel, grid, 256, 0, s, b, in, ld_in, taps, C, state, slot_stride, skip_single);
     return launch_check(cudaGetLastError(), "taps_state");
 }
