@@ -115,6 +115,29 @@ def test_paged_decode_attention(B, H, Hkv, ctx, page):
     assert torch.allclose(outb[b].float(), sd, atol=3e-2, rtol=3e-2)
 
 
+@pytest.mark.parametrize("lengths", [(300, 1), (2600, 257), (2304, 1100, 16), (23000, 9000, 100), (40000, 5)])
+def test_chunks_of_a_sequence_are_merged(lengths):
+    """Counts of chunks on both sides of what the merge requests ahead (8) and of a warp (32), with short sequences beside them; a
+    workspace full of NaN shows a value of a chunk that no block wrote."""
+    from wf_bitnet import ops
+    gen = torch.Generator().manual_seed(sum(lengths))
+    H, Hkv, D, page = 4, 1, 128, 16
+    B, blocks = len(lengths), (max(lengths) + 15) // 16
+    kv = ops.PagedKV(B * blocks, 1, Hkv, page, D)
+    kv.pool.copy_(torch.randn(kv.pool.shape, generator=gen).to(torch.bfloat16))
+    table = torch.randperm(B * blocks, generator=gen).reshape(B, blocks).to(torch.int32)
+    q = torch.randn(B, H, D, generator=gen).to(torch.bfloat16)
+    torch.full((1 << 24,), float("nan"), device="cuda")
+    out = ops.paged_decode_attn(q.cuda(), kv, 0, table.cuda(), torch.tensor(lengths, dtype=torch.int32).cuda(), out_dtype=torch.float32).cpu().double()
+    pool = kv.pool.cpu()
+    for b, n in enumerate(lengths):
+        pos = torch.arange(n)
+        k, v = (pool[table[b, pos // page].long(), 0, i, :, pos % page].reshape(n, D).double() for i in (0, 1))
+        p = torch.softmax(q[b].double() @ k.T / D ** 0.5, dim=-1)
+        # probabilities in bf16 ahead of P.V: half a unit of their eight bits each; as much again for the scores, exponentials and sums in 32 bits
+        assert ((out[b] - p @ v).abs() <= 2.0 ** -8 * (p @ v.abs())).all()
+
+
 def test_attention_ignores_garbage_beyond_seq_len():
     from wf_bitnet import ops
     kv = ops.PagedKV(8, 1, 5, 16, 128)

@@ -796,28 +796,51 @@ struct MergeParams {
     int out_dtype;
 };
 
-// grid = (H, B), block = 128 (one thread per d)
+// grid = (H, B), block = 128 (one thread per d).  A lane per chunk for the maxima and sums; the first chunks' values are requested together with them and with the
+// sequence's length, before it is known how many there are (every slot is memory of the workspace): one round of latency, where a loop over the chunks asked for the
+// length, then for each maximum, then for each value.  The call at 6 sequences of 8K tokens in int8 28.8 -> 25.9 us, at 64 of 4K in bf16 100.5 -> 99.4.  More chunks
+// than a warp has lanes (one or two sequences of more than 20K tokens) take the loop.
 __global__ void __launch_bounds__(AT_D) attn_merge_kernel(const MergeParams p) {
-    const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
+    constexpr int AHEAD = 8;
+    const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x, lane = threadIdx.x & 31;
+    const size_t base = ((size_t)b * p.H + h) * p.max_chunks;
     pdl_wait_prior();
+    pdl_launch_dependents();
+    float2 ml = make_float2(-INFINITY, 0.f);
+    if (lane < p.max_chunks) ml = make_float2(p.part_ml[(base + lane) * 2], p.part_ml[(base + lane) * 2 + 1]);
+    float o[AHEAD];
+#pragma unroll
+    for (int c = 0; c < AHEAD; ++c) o[c] = c < p.max_chunks ? p.part_o[(base + c) * AT_D + d] : 0.f;
     const int seq_len = p.seq_lens[b];
     const int nblocks = (seq_len + AT_BLK - 1) / AT_BLK;
     const int cbk = chunk_blocks_of(nblocks, p.chunk_blocks, p.max_chunks, p.min_cb);
     const int nch = (nblocks + cbk - 1) / cbk;
-    const size_t base = ((size_t)b * p.H + h) * p.max_chunks;
-    float M = -INFINITY;
-    for (int c = 0; c < nch; ++c) M = fmaxf(M, p.part_ml[(base + c) * 2]);
     float L = 0.f, O = 0.f;
-    for (int c = 0; c < nch; ++c) {
-        const float mc = p.part_ml[(base + c) * 2];
-        const float f = (mc == -INFINITY) ? 0.f : exp2f(mc - M);
-        L += p.part_ml[(base + c) * 2 + 1] * f;
-        O += p.part_o[(base + c) * AT_D + d] * f;
+    if (nch <= 32) {
+        const float m = lane < nch ? ml.x : -INFINITY, M = warp_max(m);
+        const float f = m == -INFINITY ? 0.f : exp2f(m - M);
+        L = warp_sum(lane < nch ? ml.y * f : 0.f);
+#pragma unroll
+        for (int c = 0; c < AHEAD; ++c) { const float fc = __shfl_sync(0xffffffffu, f, c); if (c < nch) O += o[c] * fc; }
+        for (int c0 = AHEAD; c0 < nch; c0 += AHEAD) {
+#pragma unroll
+            for (int c = 0; c < AHEAD; ++c) o[c] = c0 + c < nch ? p.part_o[(base + c0 + c) * AT_D + d] : 0.f;
+#pragma unroll
+            for (int c = 0; c < AHEAD; ++c) { const float fc = __shfl_sync(0xffffffffu, f, (c0 + c) & 31); if (c0 + c < nch) O += o[c] * fc; }
+        }
+    } else {
+        float M = -INFINITY;
+        for (int c = 0; c < nch; ++c) M = fmaxf(M, p.part_ml[(base + c) * 2]);
+        for (int c = 0; c < nch; ++c) {
+            const float mc = p.part_ml[(base + c) * 2];
+            const float f = (mc == -INFINITY) ? 0.f : exp2f(mc - M);
+            L += p.part_ml[(base + c) * 2 + 1] * f;
+            O += p.part_o[(base + c) * AT_D + d] * f;
+        }
     }
     const float v = (L > 0.f) ? O / L : 0.f;
     if (p.out_dtype == WF_BF16) reinterpret_cast<__nv_bfloat16*>(p.out)[((size_t)b * p.H + h) * AT_D + d] = __float2bfloat16_rn(v);
     else reinterpret_cast<float*>(p.out)[((size_t)b * p.H + h) * AT_D + d] = v;
-    pdl_launch_dependents();
 }
 
 // ---------------------------------------------------------------------------------------------
