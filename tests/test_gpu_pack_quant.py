@@ -147,6 +147,25 @@ def test_rmsnorm_quant_vs_oracle(M, K):
     assert np.array_equal(q.cpu().numpy(), qo) and np.array_equal(s.cpu().numpy(), so) and np.array_equal(rs.cpu().numpy(), ro)
 
 
+@pytest.mark.parametrize("K", [8, 248, 264, 4096, 4104, 6912, 8192, 8200, 65536])
+def test_rmsnorm_quant_of_row_widths_where_its_forms_change(K):
+    """Rows with their largest value at the end, one of zeros, one of tiny values.  The reciprocal root is a bf16, so a sum in another order gives it or, at a rounding
+    boundary, its neighbour: with one of them the two products are exact bit for bit, and so is the quantiser on them."""
+    from wf_bitnet import ops
+    gen = torch.Generator().manual_seed(K)
+    x = torch.randn(5, K, generator=gen) * torch.tensor([3.0, 0.0, 1e-30, 200.0, 1.0])[:, None]
+    x[3, K - 1], x[4, 0] = -777.0, 91.0
+    x, gamma = x.to(torch.bfloat16), (1 + 0.3 * torch.randn(K, generator=gen)).to(torch.bfloat16)
+    q, s, rs, y = ops.rmsnorm_quant(x.cuda(), gamma.cuda(), 1e-5, want_y=True)
+    y = y.cpu()
+    r = (1.0 / (x.double().pow(2).mean(1) + 1e-5).sqrt()).to(torch.bfloat16)
+    near = [r, *((r.view(torch.int16) + d).view(torch.bfloat16) for d in (1, -1))]
+    for i in range(5):
+        assert any(torch.equal(y[i], x[i] * n[i] * gamma) for n in near), i
+    qo, so, ro = O.quantize_act_i8_rows(y.float().numpy())
+    assert np.array_equal(q.cpu().numpy(), qo) and np.array_equal(s.cpu().numpy(), so) and np.array_equal(rs.cpu().numpy(), ro)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("at", ["first", "last", "middle"])
 def test_one_scale_for_many_rows(dtype, at):
