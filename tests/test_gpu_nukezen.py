@@ -364,6 +364,23 @@ def test_state_is_carried_over_hundreds_of_tokens():
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,kv,dim", [(3, 1, 8), (9, 3, 64), (28, 4, 128)])
+def test_attention_inputs_of_few_and_of_many_tokens(dtype, heads, kv, dim):
+    """Queries, keys and gates of a portion are formed by blocks that hold several vectors a warp up to four tokens per multiprocessor and one beyond it; gates by blocks of
+    their own, fewer than a block's threads, one round of them and more than one.  One long portion, and the lengths on both sides of the border, against the oracle."""
+    border = 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    cfg = config([par(heads=heads, kv=kv, dim=dim, vdim=dim, scale=dim ** -0.5, window=21, rot=(dim, 10000.0), ls=1.0, rs=0.0)], width=32)
+    w = make_weights((cfg, {}), 171)
+    m = build(cfg, w, dtype, max_tokens=4096, page_size=16, max_step_tokens=2048)
+    n = 2 * border + 5
+    rows = _rows(n, 32, 172)
+    want = oracle_mixer(cfg, w, 0, rows)
+    for cuts in ([n], [border, border + 1, 4]):
+        assert_close(part_alone(m, 0, 2, rows, cuts), want, dtype, cuts)
+    m.close()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_long_portions_of_the_state_space_recurrence(dtype):
     """Portions of several hundred tokens run the state-space recurrence in parallel chunks (every chunk from a zero state, the start
     states chained, every chunk again): a long portion after a short one, then a ragged batch of a long, a short and a chunk-sized

@@ -128,10 +128,13 @@ __global__ void __launch_bounds__(GP_MAXW * 32) gqa_prep_kernel(Batch b, GqaDims
 
 // The same for head sizes that are multiples of 4 up to 128 (no norm over the whole projection; pairs side by side, or half the rotated entries apart with
 // that half a multiple of 4): a head vector lies in the lanes of a warp four entries each, a warp's GQ vectors are requested before the cosines are formed,
-// and a pair's other entry comes from its lane.  2048 tokens, 20 + 5 + 5 heads of 128 with a gate per element (88 MB): 62 us one entry at a time, 33 so.
-constexpr int GQ = 4;
-template <typename T>
-__global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D, const float* proj, int ld, int k_off, int v_off, int g_off, const T* qb,
+// and a pair's other entry comes from its lane.  Gates of elements are blocks of their own (blockIdx.y = 1), a thread's values requested together: formed beside the cosines, one
+// after the other, they were the longest chain of a block.  Few tokens: GQ = 4 vectors of a warp in flight; where blocks wait for SMs, one vector a warp and with it six blocks
+// an SM hide more.  2048 tokens, 20 + 5 + 5 heads of 128 with a gate per element (88 MB): 62 us one entry at a time; 33.5 with the gates beside the cosines, 29.6 apart
+// (GQ = 4), 26.0 (GQ = 2, six blocks), 25.6 so; the cosines themselves cost nothing that shows.
+constexpr int GZ = 3;
+template <typename T, int GQ>
+__global__ void __launch_bounds__(256, GQ == 1 ? 6 : 4) gqa_prep_vec_kernel(Batch b, GqaDims D, const float* proj, int ld, int k_off, int v_off, int g_off, const T* qb,
                                                            const T* kb, const T* vb, float eps, PagedCache pc, T* __restrict__ qn,
                                                            float* __restrict__ gate) {
     pdl_enter();
@@ -139,6 +142,22 @@ __global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D
     const int i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, c = 4 * lane;
     const int sq = b.tok_seq[i], pos = b.tok_pos[i];
     const float* row = proj + (size_t)i * ld;
+    if (blockIdx.y) {
+        const int ng = D.H * D.dv;
+        float* out = gate + (size_t)i * ng;
+        const int step = 4 * (int)blockDim.x;
+        for (int h0 = threadIdx.x * 4; h0 < ng; h0 += GZ * step) {
+            float4 z[GZ];
+#pragma unroll
+            for (int k = 0; k < GZ; ++k) z[k] = h0 + k * step < ng ? load4(row + g_off + h0 + k * step) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < GZ; ++k) {
+                const float o[4] = {sigmoid_f(z[k].x), sigmoid_f(z[k].y), sigmoid_f(z[k].z), sigmoid_f(z[k].w)};
+                if (h0 + k * step < ng) store4(out + h0 + k * step, o);
+            }
+        }
+        return;
+    }
     const int units = D.H + (k_off >= 0 ? (D.v_is_k ? D.G : 2 * D.G) : 0);
     T* page = nullptr;
     if (k_off >= 0) {
@@ -161,23 +180,15 @@ __global__ void __launch_bounds__(256, 4) gqa_prep_vec_kernel(Batch b, GqaDims D
             bi[k] = in && bias ? load4(bias + at) : zero;
         }
         if (u0 == warp) {
-            const int table = (half + 31) & ~31, t = (int)threadIdx.x - table;       // the other warps form the gates meanwhile
+            const int table = (half + 31) & ~31, t = (int)threadIdx.x - table;       // the other warps form the gates of heads meanwhile
             if ((int)threadIdx.x < half) {
                 const double a = (double)pos * (D.freq ? D.freq[threadIdx.x] : exp2(-2.0 * (double)threadIdx.x / (double)D.rope_dims * log2((double)D.rope_base)));
                 double sn, cs;
                 sincos(a, &sn, &cs);
                 rot_c[threadIdx.x] = (float)cs * D.mscale; rot_s[threadIdx.x] = (float)sn * D.mscale;
-            } else if (gate && t >= 0) {
-                const int ng = D.gate_elem ? D.H * D.dv : D.H, nt = (int)blockDim.x - table;
-                if (ng % 4 == 0 && g_off % 4 == 0 && g_off >= 0) {
-                    for (int h = t * 4; h < ng; h += nt * 4) {
-                        const float4 z = load4(row + g_off + h);
-                        const float o[4] = {sigmoid_f(z.x), sigmoid_f(z.y), sigmoid_f(z.z), sigmoid_f(z.w)};
-                        store4(gate + (size_t)i * ng + h, o);
-                    }
-                } else {
-                    for (int h = t; h < ng; h += nt) gate[(size_t)i * ng + h] = g_off >= 0 ? sigmoid_f(row[g_off + h]) : 1.f;
-                }
+            } else if (gate && gridDim.y == 1 && t >= 0) {
+                const int ng = D.gate_elem ? D.H * D.dv : D.H;
+                for (int h = t; h < ng; h += (int)blockDim.x - table) gate[(size_t)i * ng + h] = g_off >= 0 ? sigmoid_f(row[g_off + h]) : 1.f;
             }
             __syncthreads();
         }
@@ -421,8 +432,14 @@ int launch_gqa_prep(int dt, const Batch& b, const GqaDims& D, const float* proj,
         // 34.7 / 26.9 with four, 4 + 1 heads 28.9 / 20.7 and 18.9 with three (the cosines of 64 pairs take two, the gates the third).
         const int units = D.H + (k_off >= 0 ? (D.v_is_k ? 1 : 2) * D.G : 0);
         const int threads = b.n <= 4 * sm_count() || units > 24 ? 256 : units > 8 ? 128 : 96;
-        if (dt == WF_BF16) launch_pdl(gqa_prep_vec_kernel<__nv_bfloat16>, b.n, threads, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const __nv_bfloat16*)qb, (const __nv_bfloat16*)kb, (const __nv_bfloat16*)vb, eps, pc, (__nv_bfloat16*)qn, gate);
-        else launch_pdl(gqa_prep_vec_kernel<float>, b.n, threads, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const float*)qb, (const float*)kb, (const float*)vb, eps, pc, (float*)qn, gate);
+        const dim3 grid(b.n, gate && D.gate_elem && g_off >= 0 && g_off % 4 == 0 ? 2 : 1);
+        auto go = [&](auto kernel, auto* t) {
+            using T = std::remove_pointer_t<decltype(t)>;
+            launch_pdl(kernel, grid, threads, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const T*)qb, (const T*)kb, (const T*)vb, eps, pc, (T*)qn, gate);
+        };
+        const bool few = b.n <= 4 * sm_count();
+        if (dt == WF_BF16) go(few ? gqa_prep_vec_kernel<__nv_bfloat16, 4> : gqa_prep_vec_kernel<__nv_bfloat16, 1>, (__nv_bfloat16*)nullptr);
+        else go(few ? gqa_prep_vec_kernel<float, 4> : gqa_prep_vec_kernel<float, 1>, (float*)nullptr);
         return launch_check(cudaGetLastError(), "gqa_prep_vec");
     }
     const int threads = 32 * (b.n <= sm_count() ? GP_MAXW : GA_WARPS);
