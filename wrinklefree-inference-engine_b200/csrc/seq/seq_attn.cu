@@ -433,13 +433,11 @@ int launch_gqa_prep(int dt, const Batch& b, const GqaDims& D, const float* proj,
         const int units = D.H + (k_off >= 0 ? (D.v_is_k ? 1 : 2) * D.G : 0);
         const int threads = b.n <= 4 * sm_count() || units > 24 ? 256 : units > 8 ? 128 : 96;
         const dim3 grid(b.n, gate && D.gate_elem && g_off >= 0 && g_off % 4 == 0 ? 2 : 1);
-        auto go = [&](auto kernel, auto* t) {
-            using T = std::remove_pointer_t<decltype(t)>;
-            launch_pdl(kernel, grid, threads, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const T*)qb, (const T*)kb, (const T*)vb, eps, pc, (T*)qn, gate);
-        };
         const bool few = b.n <= 4 * sm_count();
-        if (dt == WF_BF16) go(few ? gqa_prep_vec_kernel<__nv_bfloat16, 4> : gqa_prep_vec_kernel<__nv_bfloat16, 1>, (__nv_bfloat16*)nullptr);
-        else go(few ? gqa_prep_vec_kernel<float, 4> : gqa_prep_vec_kernel<float, 1>, (float*)nullptr);
+#define GPV_LAUNCH(T, GQ) launch_pdl(gqa_prep_vec_kernel<T, GQ>, grid, threads, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const T*)qb, (const T*)kb, (const T*)vb, eps, pc, (T*)qn, gate)
+        if (dt == WF_BF16) { if (few) GPV_LAUNCH(__nv_bfloat16, 4); else GPV_LAUNCH(__nv_bfloat16, 1); }
+        else { if (few) GPV_LAUNCH(float, 4); else GPV_LAUNCH(float, 1); }
+#undef GPV_LAUNCH
         return launch_check(cudaGetLastError(), "gqa_prep_vec");
     }
     const int threads = 32 * (b.n <= sm_count() ? GP_MAXW : GA_WARPS);
