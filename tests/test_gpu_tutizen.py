@@ -439,6 +439,26 @@ def test_attention_on_tensor_cores_prompts_decoding_and_key_splits(heads, kv_hea
     m.close()
 
 
+@pytest.mark.parametrize("splits", [2, 8, 9, 16])
+@pytest.mark.parametrize("vdim", [40, 128])
+def test_key_splits_of_one_long_sequence_beside_a_short_one(splits, vdim):
+    """Decoding with 2, 8, 9 and 16 key splits (one per 256 positions that the cache holds): as many as the merge requests ahead, one more, two rounds of them; most hold no key of the short
+    sequence."""
+    cfg = config([attn(heads=6, kv_heads=2, dim=64, vdim=vdim, scale=0.25)], width=64, vocab=20)
+    w = make_weights(cfg, 131)
+    P, mx = t64(O.sub(w, "l0.mix.")), cfg["layers"][0]["mixer"]
+    m = build(cfg, w, "bfloat16", max_tokens=256 * splits + 32, slots=2, page_size=16, max_step_tokens=8192)
+    lens = (256 * splits - 20, 9)
+    xs = [_rows(k + 2, 64, 132 + k) for k in lens]
+    want = [O.attention(torch.from_numpy(x).double(), P, mx, 2e-5)[0].numpy()[-2:] for x in xs]
+    slots = [m.admit() for _ in lens]
+    m.engine.run_part(0, 2, slots, lens, np.concatenate([x[:-2] for x in xs]))
+    got = [m.engine.run_part(0, 2, slots, [1, 1], np.stack([x[k] for x in xs])) for k in (-2, -1)]
+    for i in range(2):
+        assert rel_err(np.stack([g[i] for g in got]), want[i]).max() < 3e-2
+    m.close()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_long_decoding_over_page_borders(dtype):
     cfg = CONFIGS["thin"]
