@@ -11,7 +11,8 @@
 //     shared memory once per chunk.
 // What bounded the forms before: token by token, a chain of multiply-adds, shuffles and shared-memory reads of about 1000 clk per token; chunks on
 // the multiply-add units, shared-memory bandwidth (every thread of a column reads every key: 5 wavefronts per request, 450 us for the case below).
-// Measured: delta rule (20 heads, 128 x 128, two sequences, 1801 tokens) 569 -> 236 us, state space (40 heads, 128 x 64, one sequence, 2048 tokens) 307 -> 179 us;
+// Measured: delta rule (20 heads, 128 x 128, two sequences, 1801 tokens) 569 -> 236 us, since then 183 (the longer sequence in blocks of its own kind, four blocks an SM in the
+// preparation); state space (40 heads, 128 x 64, one sequence, 2048 tokens) 307 -> 179 us, 131 in segments, which it now takes (seq_segment.cu);
 // with eight warps of half the rows each 287 and 257 us (both in one pass).  Left: the chain of a chunk, about 3000 clk of products, one exchange of partial
 // sums and two barriers.  Error against 64 bits (2-norm of a mixer's output, up to 2048 tokens): in float32 engines 4.47e-7 against 4.36e-7 token by token (delta rule),
 // 3.35e-7 / 3.33e-7 (state space), 4.82e-7 / 4.94e-7 (matrix memory); float32 engines keep the token form all the same.  In bf16 engines both 2.05e-3, 1.67e-3, 1.66e-3.
