@@ -427,11 +427,11 @@ int launch_gqa_prep(int dt, const Batch& b, const GqaDims& D, const float* proj,
     if (small && D.d % 4 == 0 && D.dv % 4 == 0 && D.qk_norm < 3 && (D.rope_interleaved || D.rope_dims % 8 == 0) && ld % 4 == 0 && (k_off < 0 || (k_off % 4 == 0 && (D.v_is_k || v_off % 4 == 0))) &&
         (k_off < 0 || (pc.layer_off % 4 == 0 && pc.page_stride % 4 == 0 && vec_ok(pc.pool, 16))) && vec_ok(proj, 16) && vec_ok(qb, 16) && vec_ok(kb, 16) && vec_ok(vb, 16) && vec_ok(qn, 16) && vec_ok(gate, 16) &&
         vec_ok(D.q_norm_w, 16) && vec_ok(D.k_norm_w, 16)) {
-        // Warps a token: eight while the tokens' latency counts (300 tokens, 8 + 2 heads of 64: 10.5 us, 10.6 with four) or there are vectors for them (4096 tokens, 20 + 5
-        // heads of 128 72, 77 with four); else fewer, so that more tokens are resident while their double-precision cosines are formed: 4096 tokens, 8 + 2 heads of 64
-        // 34.7 / 26.9 with four, 4 + 1 heads 28.9 / 20.7 and 18.9 with three (the cosines of 64 pairs take two, the gates the third).
+        // Warps a token: eight while the tokens' latency counts (up to four blocks an SM) or there are vectors for them (600 tokens, 20 + 5 + 5 heads of 128 10.4 us, 13.1 with
+        // four; 2048 tokens without gates 20.6 / 21.6), but not where there are tokens enough either way (4096 tokens 53.4 / 47.4, without gates 38.1 / 35.8); else fewer, so that
+        // more tokens are resident while their double-precision cosines are formed: 4096 tokens, 8 + 2 + 2 heads of 128 29.3 / 22.4 with four, 8 + 2 heads 20.6 / 16.8.
         const int units = D.H + (k_off >= 0 ? (D.v_is_k ? 1 : 2) * D.G : 0);
-        const int threads = b.n <= 4 * sm_count() || units > 24 ? 256 : units > 8 ? 128 : 96;
+        const int threads = b.n <= 4 * sm_count() || (units > 24 && b.n <= 16 * sm_count()) ? 256 : units > 8 ? 128 : 96;
         const dim3 grid(b.n, gate && D.gate_elem && g_off >= 0 && g_off % 4 == 0 ? 2 : 1);
         const bool few = b.n <= 4 * sm_count();
 #define GPV_LAUNCH(T, GQ) launch_pdl(gqa_prep_vec_kernel<T, GQ>, grid, threads, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const T*)qb, (const T*)kb, (const T*)vb, eps, pc, (T*)qn, gate)
