@@ -43,6 +43,18 @@ def test_few_rows(M, N, K):
 
 
 @pytest.mark.parametrize("M", [1, 8])
+@pytest.mark.parametrize("K", [8, 520])
+@pytest.mark.parametrize("tiles", [(2, 1), (4, 0), (4, 1), (8, 1), (12, 0), (12, 1)])
+def test_few_rows_where_the_tiles_of_a_block_change(M, K, tiles):
+    """Blocks of one tile of 16 rows or of two, by the rounds that they make on four blocks an SM: widths on both sides of each change, the last tile short of 16."""
+    per_sm, more = tiles
+    N = 16 * per_sm * torch.cuda.get_device_properties(0).multi_processor_count + (3 if more else 0)
+    A, B = operands(M, N, K)
+    want = A.double() @ B.double().T
+    assert (product(A, B, 5).double() - want).abs().max() < 5e-6 * (1 + want.abs().max())
+
+
+@pytest.mark.parametrize("M", [1, 8])
 @pytest.mark.parametrize("K", [1024, 2560, 6912, 28672])
 def test_few_rows_are_as_close_as_multiply_adds(M, K):
     """Against 64 bits the matrix-unit form of up to 8 rows is no further off than the multiply-add form.  Four samples of 1024 sums or more leave each 2-norm

@@ -461,14 +461,19 @@ void few_launch(const GemmArgs& g, cudaStream_t s) {
 }
 // Which split: a warp wants many loads in flight while there are fewer row tiles than SMs (2560 x 6912: 14.4 us, 15.7 with half as many), blocks of two
 // tiles fit one wave up to two per SM (12.4 us), and beyond that resident blocks cover the latency (13824 x 2560: 14.6 us against 22.7 / 18.6 with
-// the first two; 128256 x 2560: 99 against 162 / 128).  With 9 to 16 rows the registers hold half as much in flight and a second block stays resident.
+// the first two; 128256 x 2560: 99 against 162 / 128).  There a block of one tile takes half the time of one of two, so the fuller rounds decide: us, two tiles / one:
+// one round of single tiles 4800 x 2560 11.3 / 9.0, 9472 x 6912 30.0 / 25.3; two rounds either way 13824 x 2560 16.1 / 17.1; three for four 20000 x 2560 25.1 / 22.8; as
+// many 32768 x 2560 30.7 / 32.3; seven for eight 65536 x 6912 147 / 141.  With 9 to 16 rows the registers hold half as much in flight and a second block stays resident.
 template <int NT>
 void few_dispatch(const GemmArgs& g, cudaStream_t s) {
     const int tiles = (g.N + 15) / 16, sms = sm_count();
     if (NT == 1) {
         if (tiles <= sms) few_launch<1, 8, 8, 1>(g, s);
         else if (tiles <= 2 * sms) few_launch<1, 4, 8, 1>(g, s);
-        else few_launch<1, 4, 4, 4>(g, s);
+        else {
+            const int slots = 4 * sms, tiles_a_block = (tiles + slots - 1) / slots, pairs_a_block = ((tiles + 1) / 2 + slots - 1) / slots;
+            if (tiles_a_block < 2 * pairs_a_block) few_launch<1, 8, 4, 4>(g, s); else few_launch<1, 4, 4, 4>(g, s);
+        }
     } else {
         if (tiles <= 4 * sms) few_launch<2, 8, 4, 1>(g, s);
         else few_launch<2, 2, 4, 2>(g, s);
