@@ -344,8 +344,8 @@ constexpr int FR_WARPS = 8;
 // glu: a tile's rows 0 .. 7 are gate rows and 8 .. 15 the up rows of the same outputs, so that a pair meets where the tile's sums do.
 template <int NT, int WK, int U, int OCC, bool CF32>
 __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g) {
-    // (with several blocks per SM there are no registers for it, and one another's loads to wait under: 16 rows x 13824 x 2560, gated, on two blocks 30 us, 25 without)
-    constexpr bool AHEAD = OCC == 1;
+    // (with more blocks per SM, or two of 9 to 16 rows, there are no registers for it, and one another's loads to wait under: 16 rows x 13824 x 2560, gated, on two blocks 30 us, 25 without)
+    constexpr bool AHEAD = OCC == 1 || (OCC == 2 && NT == 1);
     const bool early = AHEAD && g.b_const;
     if (!early) pdl_enter();
     constexpr int TILES = FR_WARPS / WK;                  // 16-row tiles per block
@@ -459,8 +459,9 @@ void few_launch(const GemmArgs& g, cudaStream_t s) {
     const int tiles = g.glu ? (g.N / 2 + 7) / 8 : (g.N + 15) / 16, per = FR_WARPS / WK, blocks = (tiles + per - 1) / per;
     if (g.c_f32) launch_pdl(gemm_few_kernel<NT, WK, U, OCC, true>, blocks, FR_WARPS * 32, 0, s, g); else launch_pdl(gemm_few_kernel<NT, WK, U, OCC, false>, blocks, FR_WARPS * 32, 0, s, g);
 }
-// Which split: a warp wants many loads in flight while there are fewer row tiles than SMs (2560 x 6912: 14.4 us, 15.7 with half as many), blocks of two
-// tiles fit one wave up to two per SM (12.4 us), and beyond that resident blocks cover the latency (13824 x 2560: 14.6 us against 22.7 / 18.6 with
+// Which split: a warp wants many loads in flight while there are fewer row tiles than SMs (2560 x 6912: 14.4 us, 15.7 with half as many); up to two tiles per SM a block
+// has one and two blocks share an SM, with half as many a warp under way (8 rows back to back, against blocks of two tiles with four warps each: 4608 x 2560 7.9 -> 7.2 us,
+// 4608 x 6912 16.1 -> 14.6, 2400 x 6912 13.8 -> 11.8; a decode step of four layers 2560 wide 283 -> 266); beyond that resident blocks cover the latency (13824 x 2560: 14.6 us against 22.7 / 18.6 with
 // the first two; 128256 x 2560: 99 against 162 / 128).  There a block of one tile takes half the time of one of two, so the fuller rounds decide: us, two tiles / one:
 // one round of single tiles 4800 x 2560 11.3 / 9.0, 9472 x 6912 30.0 / 25.3; two rounds either way 13824 x 2560 16.1 / 17.1; three for four 20000 x 2560 25.1 / 22.8; as
 // many 32768 x 2560 30.7 / 32.3; seven for eight 65536 x 6912 147 / 141.  With 9 to 16 rows the registers hold half as much in flight and a second block stays resident.
@@ -469,7 +470,7 @@ void few_dispatch(const GemmArgs& g, cudaStream_t s) {
     const int tiles = (g.N + 15) / 16, sms = sm_count();
     if (NT == 1) {
         if (tiles <= sms) few_launch<1, 8, 8, 1>(g, s);
-        else if (tiles <= 2 * sms) few_launch<1, 4, 8, 1>(g, s);
+        else if (tiles <= 2 * sms) few_launch<1, 8, 4, 2>(g, s);
         else {
             const int slots = 4 * sms, tiles_a_block = (tiles + slots - 1) / slots, pairs_a_block = ((tiles + 1) / 2 + slots - 1) / slots;
             if (tiles_a_block < 2 * pairs_a_block) few_launch<1, 8, 4, 4>(g, s); else few_launch<1, 4, 4, 4>(g, s);
