@@ -1,5 +1,7 @@
 """Host-side logic (no GPU): synthetic-weight packer, LSB<->I2_S re-blocking, page allocator,
 KV config arithmetic, sgl_kernel argument errors."""
+from pathlib import Path
+
 import numpy as np
 import pytest
 import torch
@@ -196,3 +198,27 @@ def test_lists_of_token_ids_become_arrays_as_numpy_makes_them(entries):
         return
     got = _i32(entries)
     assert got.dtype == want.dtype and got.shape == want.shape and np.array_equal(got, want)
+
+
+def _make_seq(tmp_path, *overrides):
+    """`make seq` with the CUDA library taken as built and the helper for token lists written to tmp_path."""
+    import shutil
+    import subprocess
+    import sys
+    if shutil.which("make") is None:
+        pytest.skip("no make")
+    csrc = Path(__file__).resolve().parents[1] / "wrinklefree-inference-engine_b200" / "csrc"
+    (tmp_path / "built.so").touch()
+    return subprocess.run(["make", "-C", str(csrc), "seq", f"SEQ_OUT={tmp_path / 'built.so'}", "SEQ_OBJS=", f"PY_OUT={tmp_path / 'libwf_py.so'}", f"PYTHON={sys.executable}",
+                           *overrides], capture_output=True, text=True, timeout=120)
+
+
+@pytest.mark.parametrize("headers", [True, False])
+def test_the_sequence_engine_is_built_with_and_without_the_interpreters_headers(headers, tmp_path):
+    """The helper that turns lists of token ids into arrays is an extra: numpy does it where the helper cannot be built."""
+    import sysconfig
+    if headers and not (Path(sysconfig.get_paths()["include"]) / "Python.h").exists():
+        pytest.skip("no Python.h here")
+    r = _make_seq(tmp_path, *(() if headers else (f"PY_INC={tmp_path / 'nothing'}",)))
+    assert r.returncode == 0, r.stderr
+    assert (tmp_path / "libwf_py.so").exists() == headers
