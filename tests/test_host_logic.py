@@ -188,8 +188,17 @@ def test_which_product_kernel_a_shape_takes(m, n, k, tcgen05):
 
 @pytest.mark.parametrize("entries", [[0] * 31, list(range(-20, 20)), [-2 ** 31, 2 ** 31 - 1] * 20, [1] * 40 + [2 ** 31], [1] * 40 + [-2 ** 31 - 1], [True] * 40, [1.5] * 40,
                                      [np.int64(3)] * 40, ["a"] * 40, [[1]] * 40, (7,) * 40, range(50), np.arange(40), []])
-def test_lists_of_token_ids_become_arrays_as_numpy_makes_them(entries):
+def test_lists_of_token_ids_become_arrays_as_numpy_makes_them(entries, monkeypatch):
+    """... and where the helper has been built, lists of 32 plain ints and more that fit go through it and no others."""
+    from wf_bitnet import _lib
     from wf_bitnet.seq_engine import _i32
+    helper, taken = _lib.py_i32(), []
+    assert (helper is not None) == py_library().exists()
+    if helper is not None:
+        def spy(a, to, n):
+            taken.append(helper(a, to, n))
+            return taken[-1]
+        monkeypatch.setattr(_lib, "_py_i32", spy)
     try:
         want = np.ascontiguousarray(entries, dtype=np.int32)
     except Exception as e:
@@ -198,6 +207,41 @@ def test_lists_of_token_ids_become_arrays_as_numpy_makes_them(entries):
         return
     got = _i32(entries)
     assert got.dtype == want.dtype and got.shape == want.shape and np.array_equal(got, want)
+    if helper is not None:
+        assert (taken == [1]) == (type(entries) is list and len(entries) >= 32 and all(type(x) is int for x in entries))
+
+
+def py_library():
+    import importlib.machinery
+    return Path(__file__).resolve().parents[1] / "wrinklefree-inference-engine_b200" / ("libwf_py" + importlib.machinery.EXTENSION_SUFFIXES[0])
+
+
+def test_the_helper_for_token_lists_is_this_interpreters_and_opened_on_use(tmp_path, monkeypatch):
+    """Its name carries the interpreter's ABI, so that one built for another (other object layouts) is not opened; a process that builds it finds it; importing the package opens
+    nothing."""
+    import shutil
+    import subprocess
+    import sys
+    if not py_library().exists():
+        pytest.skip("not built")
+    r = subprocess.run([sys.executable, "-c", "import sys; sys.path.insert(0, sys.argv[1]); from wf_bitnet import _lib; print('libwf_py' in open('/proc/self/maps').read())",
+                        str(py_library().parent)], capture_output=True, text=True, timeout=120)
+    assert r.stdout.strip() == "False", r.stdout + r.stderr
+    from wf_bitnet import _lib
+    from wf_bitnet.seq_engine import _i32
+    monkeypatch.setattr(_lib, "_PKG_ROOT", tmp_path)
+    monkeypatch.setattr(_lib, "_py_i32", None)
+    for other in ("libwf_py.so", "libwf_py.cpython-312d-x86_64-linux-gnu.so"):
+        shutil.copy(py_library(), tmp_path / other)
+    ids = list(range(40))
+    assert _lib.py_i32() is None and np.array_equal(_i32(ids), ids)
+
+    def make(cmd, **kw):
+        assert f"PYTHON={sys.executable}" in cmd
+        shutil.copy(py_library(), tmp_path / py_library().name)
+    monkeypatch.setattr(subprocess, "run", make)
+    _lib.build_seq_lib()
+    assert _lib.py_i32() is not None and np.array_equal(_i32(ids), ids)
 
 
 def _make_seq(tmp_path, *overrides):
@@ -209,7 +253,7 @@ def _make_seq(tmp_path, *overrides):
         pytest.skip("no make")
     csrc = Path(__file__).resolve().parents[1] / "wrinklefree-inference-engine_b200" / "csrc"
     (tmp_path / "built.so").touch()
-    return subprocess.run(["make", "-C", str(csrc), "seq", f"SEQ_OUT={tmp_path / 'built.so'}", "SEQ_OBJS=", f"PY_OUT={tmp_path / 'libwf_py.so'}", f"PYTHON={sys.executable}",
+    return subprocess.run(["make", "-C", str(csrc), "seq", f"SEQ_OUT={tmp_path / 'built.so'}", "SEQ_OBJS=", f"PY_OUT={tmp_path / py_library().name}", f"PYTHON={sys.executable}",
                            *overrides], capture_output=True, text=True, timeout=120)
 
 
@@ -221,4 +265,4 @@ def test_the_sequence_engine_is_built_with_and_without_the_interpreters_headers(
         pytest.skip("no Python.h here")
     r = _make_seq(tmp_path, *(() if headers else (f"PY_INC={tmp_path / 'nothing'}",)))
     assert r.returncode == 0, r.stderr
-    assert (tmp_path / "libwf_py.so").exists() == headers
+    assert (tmp_path / py_library().name).exists() == headers

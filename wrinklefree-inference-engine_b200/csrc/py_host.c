@@ -1,6 +1,9 @@
-/* Host helpers that need the interpreter's own view of an object (libwf_py.so, called through ctypes.PyDLL with the GIL held). */
+/* Host helpers that need the interpreter's own view of an object (libwf_py.<ABI>.so, called through ctypes.PyDLL with the GIL held). */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
+#ifdef Py_GIL_DISABLED
+#error "another thread may change the list meanwhile: left out, numpy does it"
+#endif
 #include <stdint.h>
 
 /* The n entries of a list as 32-bit integers; 0, and out in part written, when the object is not a list of n plain ints that fit.  A prompt of 2048 token ids: 5 us,

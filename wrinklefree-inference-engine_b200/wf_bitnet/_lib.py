@@ -201,27 +201,34 @@ SEQ_SYMBOLS = {
 _seq_lib = None
 
 
-def _load_py_i32():
-    """wf_py_i32 of libwf_py.so (csrc/py_host.c), or None where it has not been built or is another interpreter's."""
-    try:
-        fn = C.PyDLL(str(_PKG_ROOT / "libwf_py.so")).wf_py_i32
-    except (OSError, AttributeError):
-        return None
-    fn.restype = C.c_int
-    fn.argtypes = [C.py_object, C.c_void_p, C.c_ssize_t]
-    return fn
+_py_i32 = None          # False: looked for and not there
 
 
-py_i32 = _load_py_i32()
+def py_i32():
+    """wf_py_i32 of libwf_py.<this interpreter's ABI>.so (csrc/py_host.c), or None where it has not been built; opened when it is first asked for."""
+    global _py_i32
+    if _py_i32 is None:
+        import importlib.machinery
+        try:
+            fn = C.PyDLL(str(_PKG_ROOT / ("libwf_py" + importlib.machinery.EXTENSION_SUFFIXES[0]))).wf_py_i32
+            fn.restype = C.c_int
+            fn.argtypes = [C.py_object, C.c_void_p, C.c_ssize_t]
+            _py_i32 = fn
+        except (OSError, AttributeError):
+            _py_i32 = False
+    return _py_i32 or None
 
 
 def build_seq_lib() -> None:
     """Compile libwf_seq.so in-tree (make target `seq`: the sequence-model sources only)."""
+    global _py_i32
     import subprocess
+    import sys
     env = dict(os.environ)
     env.pop("CC", None)
     env.pop("CXX", None)
-    subprocess.run(["make", "-C", str(_PKG_ROOT / "csrc"), "seq", "-j8"], check=True, env=env, stdout=subprocess.DEVNULL)
+    subprocess.run(["make", "-C", str(_PKG_ROOT / "csrc"), "seq", "-j8", f"PYTHON={sys.executable}"], check=True, env=env, stdout=subprocess.DEVNULL)
+    _py_i32 = _py_i32 or None          # looked for again
 
 
 def seq_lib(build: bool = False) -> C.CDLL:

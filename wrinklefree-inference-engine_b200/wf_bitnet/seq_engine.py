@@ -12,9 +12,9 @@ from ._lib import SeqConfig, SeqLayer, seq_check, seq_lib
 
 
 def _i32(a) -> np.ndarray:
-    if type(a) is list and len(a) >= 32 and _lib.py_i32 is not None:      # token ids: numpy takes 28 ns an entry
+    if type(a) is list and len(a) >= 32 and (convert := _lib.py_i32()) is not None:      # token ids: numpy takes 28 ns an entry
         out = np.empty(len(a), dtype=np.int32)
-        if _lib.py_i32(a, out.ctypes.data, len(a)):
+        if convert(a, out.ctypes.data, len(a)):
             return out
     return np.ascontiguousarray(a, dtype=np.int32)
 
