@@ -218,6 +218,8 @@ int wf_seq_launches_last_step(const wf_seq_engine* e);
  * (WF_SEQ_BLOCK_PARALLEL with two norms, WF_SEQ_NORM_DYN_TANH), 6 and 7 the norms behind the mixer and the feed-forward (WF_SEQ_NORM_DYN_TANH).
  * Sequence lengths advance as in a step. */
 int wf_seq_set_layer_tap(wf_seq_engine* e, float* host);
+/* how many CTAs the key range of a token was cut over in the (latent or grouped-query) tensor-core attention launched last */
+int wf_seq_key_splits(const wf_seq_engine* e);
 int wf_seq_run_part(wf_seq_engine* e, int layer, int part, int nseq, const int32_t* slots, const int32_t* counts, const float* in_host,
                     float* out_host);
 /* mean device time of one step shape (measurement): runs the step `iters` times on synthetic tokens and returns milliseconds per step.

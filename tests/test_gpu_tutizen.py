@@ -454,6 +454,7 @@ def test_key_splits_of_one_long_sequence_beside_a_short_one(splits, vdim):
     slots = [m.admit() for _ in lens]
     m.engine.run_part(0, 2, slots, lens, np.concatenate([x[:-2] for x in xs]))
     got = [m.engine.run_part(0, 2, slots, [1, 1], np.stack([x[k] for x in xs])) for k in (-2, -1)]
+    assert m.engine.key_splits() == splits
     for i in range(2):
         assert rel_err(np.stack([g[i] for g in got]), want[i]).max() < 3e-2
     m.close()

@@ -373,42 +373,34 @@ __global__ void __launch_bounds__(AM_THREADS, 3) gqa_attn_mma_kernel(Batch b, Gq
 }
 
 // One block per (token, head), a thread per channel (at most 128): merge the key splits' partial results (maxima in units of log 2), apply the gate.  In every warp a lane holds a
-// split's maximum and sum, and the first splits' values and the gate are requested together with them, before it is known which splits have keys: one memory latency up to
-// eight splits, where one split after the other took one each (a merge of a decode step of 8 sequences, 20 heads 4.2 us) and maxima, sums and values behind one another three (3.4; 1.8 so).
+// split's maximum and sum (ATTN_MAX_SPLITS of them at most), and the first splits' values and the gate are requested together with them, before it is known which splits have keys:
+// one memory latency up to eight splits, where one split after the other took one each (a merge of a decode step of 8 sequences, 20 heads 4.2 us) and maxima, sums and values behind
+// one another three (3.4; 1.8 so).
 __global__ void __launch_bounds__(128) gqa_attn_merge_kernel(GqaDims D, int rows, int splits, const float* part, const float* gate, __nv_bfloat16* __restrict__ out) {
     pdl_enter();
     constexpr int AHEAD = 8;
+    static_assert(ATTN_MAX_SPLITS == 2 * AHEAD && ATTN_MAX_SPLITS <= 32, "two rounds of values, a lane per split");
     const int dv = D.dv, stride = dv + 2, row = blockIdx.x, c = threadIdx.x, lane = threadIdx.x & 31;
     const bool in = c < dv;
     const float* p = part + (size_t)row * splits * stride;
     const float gm = gate ? (D.gate_elem ? (in ? gate[(size_t)row * dv + c] : 0.f) : gate[row]) : 1.f;
-    float m = lane < splits ? p[(size_t)lane * stride + dv] : -INFINITY, l = lane < splits ? p[(size_t)lane * stride + dv + 1] : 0.f;
+    const float m = lane < splits ? p[(size_t)lane * stride + dv] : -INFINITY, l = lane < splits ? p[(size_t)lane * stride + dv + 1] : 0.f;
     float q[AHEAD];
 #pragma unroll
     for (int z = 0; z < AHEAD; ++z) q[z] = z < splits && in ? p[(size_t)z * stride + c] : 0.f;
-    float mg = m;
-    for (int z = lane + 32; z < splits; z += 32) mg = fmaxf(mg, p[(size_t)z * stride + dv]);
-    mg = warp_max(mg);
-    float lg = m == -INFINITY ? 0.f : l * exp2f(m - mg);
-    for (int z = lane + 32; z < splits; z += 32) { const float mz = p[(size_t)z * stride + dv]; lg += mz == -INFINITY ? 0.f : p[(size_t)z * stride + dv + 1] * exp2f(mz - mg); }
-    lg = warp_sum(lg);
+    const float mg = warp_max(m), w = m == -INFINITY ? 0.f : exp2f(m - mg), lg = warp_sum(m == -INFINITY ? 0.f : l * w);
     const float mul = (gate && !D.gate_elem ? gm : 1.f) * am_inv_sum(D, row % D.H, mg, lg);
+    const unsigned live = __ballot_sync(0xffffffffu, m != -INFINITY);        // a split without keys has written no values
     float v = 0.f;
-    for (int z0 = 0; z0 < splits; z0 += 32) {
-        if (z0) m = z0 + lane < splits ? p[(size_t)(z0 + lane) * stride + dv] : -INFINITY;
-        const float w = m == -INFINITY ? 0.f : exp2f(m - mg);
-        const unsigned live = __ballot_sync(0xffffffffu, m != -INFINITY);        // a split without keys has written no values
-        const int n = min(32, splits - z0);
-        for (int z1 = 0; z1 < n; z1 += AHEAD) {
-            if (z0 + z1) {
+    for (int z0 = 0; z0 < splits; z0 += AHEAD) {
+        if (z0) {
 #pragma unroll
-                for (int z = 0; z < AHEAD; ++z) q[z] = z1 + z < n && in ? p[(size_t)(z0 + z1 + z) * stride + c] : 0.f;
-            }
+            for (int z = 0; z < AHEAD; ++z) q[z] = z0 + z < splits && in ? p[(size_t)(z0 + z) * stride + c] : 0.f;
+        }
 #pragma unroll
-            for (int z = 0; z < AHEAD; ++z) {
-                const float wz = __shfl_sync(0xffffffffu, w, (z1 + z) & 31);
-                if (live >> ((z1 + z) & 31) & 1) v += q[z] * wz;
-            }
+        for (int z = 0; z < AHEAD; ++z) {
+            const float wz = __shfl_sync(0xffffffffu, w, z0 + z);
+            if (live >> (z0 + z) & 1) v += q[z] * wz;
         }
     }
     if (in) out[(size_t)row * dv + c] = __float2bfloat16_rn(v * mul * (gate && D.gate_elem ? gm : 1.f));
@@ -468,7 +460,7 @@ int launch_gqa_attn_mma(const Batch& b, const GqaDims& D, const void* qn, const 
     while (ap.rp2 < rep) { ap.rp2 <<= 1; ++ap.rp2_log; }
     const bool decode = b.n == b.nseq;
     ap.tq = (decode ? 16 : 64) / ap.rp2;
-    ap.splits = decode && workspace && splits > 1 ? splits : 1;
+    ap.splits = decode && workspace && splits > 1 ? (splits < ATTN_MAX_SPLITS ? splits : ATTN_MAX_SPLITS) : 1;
     ap.part = workspace;
     // every sequence's tokens are cut into tiles of tq; n / tq + nseq bounds their number (CTAs beyond the last tile return at once)
     const int tiles = decode ? b.n : b.n / ap.tq + b.nseq;

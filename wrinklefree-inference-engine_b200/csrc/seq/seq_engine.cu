@@ -147,6 +147,7 @@ struct wf_seq_engine {
     size_t gqa_ws_bytes = 0;
     float* attn_ws = nullptr;         // partial results of key-split attention
     int attn_ws_rows = 0;             // token-splits it holds
+    int key_splits = 0;               // of the tensor-core attention launched last (wf_seq_key_splits)
     int pair_path_max = 64;           // up to this many (token, expert) pairs the experts run as per-pair weight streams (WF_SEQ_PAIR_MAX)
     float* logits = nullptr;
     size_t logits_rows = 0;
@@ -572,9 +573,10 @@ int run_latent(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
             splits = resident / n;
             if (splits > span / 128) splits = span / 128;
             if (splits > e->attn_ws_rows / n) splits = e->attn_ws_rows / n;
-            if (splits > 16) splits = 16;
+            if (splits > ATTN_MAX_SPLITS) splits = ATTN_MAX_SPLITS;
             if (splits < 1) splits = 1;
         }
+        e->key_splits = splits;
         if (use_kt) { if ((rc = launch_latent_attn_kt(b, D, e->qa, e->qr, pc, e->olat, e->attn_ws, splits, s))) return rc; }
         else if ((rc = launch_latent_attn_mma(b, D, e->qa, e->qr, pc, e->olat, e->attn_ws, splits, s))) return rc;
     } else if ((rc = launch_latent_attn(e->dt, b, D, e->qa, e->qr, pc, e->olat, s))) return rc;
@@ -724,9 +726,10 @@ int run_gqa(wf_seq_engine* e, LayerState& L, const Batch& b, float* out) {
             splits = (e->attn_waves * resident + ctas - 1) / ctas;
             if (splits > span / 256) splits = (int)(span / 256);
             if (splits > e->gqa_ws_rows / (n * c.heads)) splits = e->gqa_ws_rows / (n * c.heads);
-            if (splits > 16) splits = 16;
+            if (splits > ATTN_MAX_SPLITS) splits = ATTN_MAX_SPLITS;
             if (splits < 1) splits = 1;
         }
+        e->key_splits = splits;
         if ((rc = launch_gqa_attn_mma(b, D, e->qn, gate, pc, e->og, e->gqa_ws, splits, s))) return rc;
     } else if ((rc = launch_gqa_attn(e->dt, b, D, e->qn, gate, pc, e->og, s))) return rc;
     mark(e, D.talk ? "attn.attention(mixed heads)" : D.softcap > 0.f || D.rel ? "attn.attention(cap+bias)" : D.keep_first > 0 ? "attn.attention(window+first)" : "attn.attention");
@@ -1937,6 +1940,8 @@ extern "C" int wf_seq_run_part(wf_seq_engine* e, int layer, int part, int nseq, 
 }
 
 extern "C" int wf_seq_time_step(wf_seq_engine* e, int nseq, const int32_t* slots, const int32_t* counts, int iters, float* ms_out);
+
+extern "C" int wf_seq_key_splits(const wf_seq_engine* e) { return e ? e->key_splits : 0; }
 
 extern "C" int wf_seq_set_length(wf_seq_engine* e, int slot, int len) {
     if (!e || slot < 0 || slot >= e->cfg.slots || !e->pt.live[slot] || len < 0) { set_error("wf_seq_set_length: bad slot / length"); return WF_ERR_INVALID; }

@@ -229,10 +229,11 @@ bool talk_attn_mma_usable(const GqaDims& D, const PagedCache& pc);
 size_t talk_attn_workspace(const GqaDims& D, int n, int splits);
 int launch_talk_attn_mma(const Batch& b, const GqaDims& D, const void* qn, const PagedCache& pc, void* out, float* workspace, int splits, cudaStream_t s);
 // the same on tensor cores (bf16 storage only; seq_attn_mma.cu): group sizes up to 16, per-head sizes multiples of 8 up to 128, cache rows
-// 16-byte aligned.  When every sequence brings one token the key range can be cut over `splits` CTAs; that needs a workspace of
+// 16-byte aligned.  When every sequence brings one token the key range can be cut over `splits` CTAs (up to ATTN_MAX_SPLITS); that needs a workspace of
 // gqa_attn_mma_workspace(n * H, splits, dv) bytes.
 bool gqa_attn_mma_usable(const GqaDims& D, const PagedCache& pc);
 bool gqa_attn_mma_takes(const GqaDims& D);      // the score and mask options of D that the tensor-core form implements
+constexpr int ATTN_MAX_SPLITS = 16;             // more are not taken: the merges have a lane per split
 size_t gqa_attn_mma_workspace(int rows, int splits, int dv);
 int launch_gqa_attn_mma(const Batch& b, const GqaDims& D, const void* qn, const float* gate, const PagedCache& pc, void* out, float* workspace, int splits,
                         cudaStream_t s);

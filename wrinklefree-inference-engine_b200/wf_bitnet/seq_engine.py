@@ -144,5 +144,9 @@ class SeqEngine:
         seq_check(seq_lib().wf_seq_profile_step(self._h, s.size, s.ctypes.data, c.ctypes.data, iters, buf, len(buf)))
         return {k: tuple(v) for k, v in json.loads(buf.value.decode()).items()}
 
+    def key_splits(self) -> int:
+        """How many CTAs the key range of a token was cut over in the tensor-core attention launched last."""
+        return int(seq_lib().wf_seq_key_splits(self._h))
+
     def set_length(self, slot: int, length: int) -> None:
         seq_check(seq_lib().wf_seq_set_length(self._h, slot, length))
