@@ -502,6 +502,25 @@ def test_latent_attention_on_tensor_cores_with_key_splits(heads, kv_rank, rot_di
     m.close()
 
 
+@pytest.mark.parametrize("heads,kv_rank,splits", [(5, 512, 16), (33, 512, 9), (20, 48, 16), (33, 64, 2)])
+def test_key_splits_of_latent_attention_beside_a_short_sequence(heads, kv_rank, splits):
+    """Decoding with 2, 9 and 16 key splits (one per 128 positions that the cache holds) in both tensor-core forms, the widest latent that either takes and blocks of less than two
+    warps; most splits hold no key of the short sequence."""
+    cfg = config([lat(heads=heads, dim=16, rot_dim=16, vdim=16, kv_rank=kv_rank, window=1 << 20, scale=0.5)], width=64, vocab=40, groups=1, taps=2)
+    w = make_weights(cfg, 63)
+    m = build(cfg, w, "bfloat16", max_tokens=128 * splits + 16, slots=2, page_size=16, max_step_tokens=4096)
+    P, lens = {k: torch.from_numpy(v).double() for k, v in O.sub(w, "l0.mix.").items()}, (128 * splits - 20, 9)
+    xs = [_rows(k + 2, 64, 64 + k) for k in lens]
+    want = [O.latent_attention(torch.from_numpy(x).double(), P, cfg["layers"][0]["mixer"], 1e-6).numpy()[-2:] for x in xs]
+    slots = [m.admit() for _ in lens]
+    m.engine.run_part(0, 2, slots, lens, np.concatenate([x[:-2] for x in xs]))
+    got = [m.engine.run_part(0, 2, slots, [1, 1], np.stack([x[k] for x in xs])) for k in (-2, -1)]
+    assert m.engine.key_splits() == splits
+    for i in range(2):
+        assert rel_err(np.stack([g[i] for g in got]), want[i]).max() < TOL["bfloat16"], i
+    m.close()
+
+
 def _write_model_dir(path, cfg, weights):
     import json
     import struct

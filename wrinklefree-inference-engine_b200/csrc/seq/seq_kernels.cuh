@@ -161,6 +161,7 @@ int launch_latent_kv_write(int dt, const Batch& b, const LatentDims& L, const fl
 // per (token, head): softmax over positions j in (pos - window, pos] of (qa . c_j + qr . kr_j) * scale; out T [n, H, R] = sum p_j c_j.
 // qa float [n, H, R] (the query carried through the key up-projection), qr float [n, H, r].
 int launch_latent_attn(int dt, const Batch& b, const LatentDims& L, const float* qa, const float* qr, const PagedCache& pc, void* out, cudaStream_t s);
+constexpr int ATTN_MAX_SPLITS = 16;             // of a token's keys; more are not taken: the merges have a lane per split and ask for all of them together
 // the same on tensor cores (bf16 storage only; seq_latent_mma.cu).  splits > 1 cuts every token's key range over that many CTAs and needs
 // workspace for n * splits partial results (latent_attn_mma_workspace(n * splits, H, R) bytes).  The cache rows must start 16-byte aligned.
 bool latent_attn_mma_usable(const LatentDims& L);
@@ -233,7 +234,6 @@ int launch_talk_attn_mma(const Batch& b, const GqaDims& D, const void* qn, const
 // gqa_attn_mma_workspace(n * H, splits, dv) bytes.
 bool gqa_attn_mma_usable(const GqaDims& D, const PagedCache& pc);
 bool gqa_attn_mma_takes(const GqaDims& D);      // the score and mask options of D that the tensor-core form implements
-constexpr int ATTN_MAX_SPLITS = 16;             // more are not taken: the merges have a lane per split
 size_t gqa_attn_mma_workspace(int rows, int splits, int dv);
 int launch_gqa_attn_mma(const Batch& b, const GqaDims& D, const void* qn, const float* gate, const PagedCache& pc, void* out, float* workspace, int splits,
                         cudaStream_t s);

@@ -217,41 +217,32 @@ __global__ void latent_attn_mma_kernel(Batch b, LatentDims L, const float* qa, c
     }
 }
 
-// One block per (token, head), a thread per channel up to 512: out = sum_s exp(m_s - m) O_s / sum_s exp(m_s - m) l_s.  A lane per split for maxima and sums; a thread's
-// values of the splits (at most 16) are requested with them, before it is known which splits have keys.  Bound by latency: 20 heads of rank 512, 1 / 8 sequences 8.8 / 9.0 us
+// One block per (token, head), a thread per channel (both forms take latents of up to 512): out = sum_s exp(m_s - m) O_s / sum_s exp(m_s - m) l_s.  A lane per split for maxima and
+// sums; a thread's values of all splits are requested with them, before it is known which splits have keys.  Bound by latency: 20 heads of rank 512, 1 / 8 sequences 8.8 / 9.0 us
 // with 128 threads and maxima, sums and values one split after the other; 5.6 / 6.1 with the loads together; 2.4 / 3.3 with a thread per channel (8 ahead: 2.7 / 3.6).
 __global__ void __launch_bounds__(512) latent_attn_merge_kernel(int H, int R, int splits, const float* part, __nv_bfloat16* __restrict__ out, const float* sink) {
     pdl_enter();
-    constexpr int AHEAD = 16;
-    const int i = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31;
+    static_assert(ATTN_MAX_SPLITS <= 32, "a lane per split");
+    const int i = blockIdx.x, h = blockIdx.y, c = threadIdx.x, lane = threadIdx.x & 31;
     const float* p0 = part + (((size_t)i * splits) * H + h) * (R + 2);
     const size_t sstride = (size_t)H * (R + 2);
-    const bool mine = lane < splits;                       // (at most 16 splits)
+    const bool mine = lane < splits;
     const float ms = mine ? p0[lane * sstride + R] : -INFINITY, ls = mine ? p0[lane * sstride + R + 1] : 0.f;
-    float q[AHEAD];
+    float q[ATTN_MAX_SPLITS];
 #pragma unroll
-    for (int s = 0; s < AHEAD; ++s) q[s] = s < splits && (int)threadIdx.x < R ? p0[s * sstride + threadIdx.x] : 0.f;
+    for (int s = 0; s < ATTN_MAX_SPLITS; ++s) q[s] = s < splits && c < R ? p0[s * sstride + c] : 0.f;
     const float m = warp_max(ms), w = ms == -INFINITY ? 0.f : expf(ms - m);
     float l = warp_sum(ms == -INFINITY ? 0.f : w * ls);
     if (sink) l += expf(sink[h] - m);
     const float inv = 1.f / l;
     const unsigned live = __ballot_sync(0xffffffffu, ms != -INFINITY);
-    for (int c0 = 0; c0 < R; c0 += blockDim.x) {
-        const int c = c0 + threadIdx.x;
-        float v = 0.f;
-        for (int s0 = 0; s0 < splits; s0 += AHEAD) {
-            if (c0 + s0) {
+    float v = 0.f;
 #pragma unroll
-                for (int s = 0; s < AHEAD; ++s) q[s] = s0 + s < splits && c < R ? p0[(s0 + s) * sstride + c] : 0.f;
-            }
-#pragma unroll
-            for (int s = 0; s < AHEAD; ++s) {
-                const float ws = __shfl_sync(0xffffffffu, w, (s0 + s) & 31);
-                if (live >> ((s0 + s) & 31) & 1) v += ws * q[s];
-            }
-        }
-        if (c < R) out[((size_t)i * H + h) * R + c] = __float2bfloat16_rn(v * inv);
+    for (int s = 0; s < ATTN_MAX_SPLITS; ++s) {
+        const float ws = __shfl_sync(0xffffffffu, w, s);
+        if (live >> s & 1) v += ws * q[s];
     }
+    if (c < R) out[((size_t)i * H + h) * R + c] = __float2bfloat16_rn(v * inv);
 }
 
 
@@ -533,7 +524,7 @@ int launch_latent_attn_kt(const Batch& b, const LatentDims& L, const float* qa, 
                           int splits, cudaStream_t s) {
     if (b.n <= 0) return WF_OK;
     MmaParams mp;
-    mp.splits = splits < 1 ? 1 : (splits > 16 ? 16 : splits);
+    mp.splits = splits < 1 ? 1 : (splits > ATTN_MAX_SPLITS ? ATTN_MAX_SPLITS : splits);
     mp.part = workspace;
     mp.dkp = (L.R + L.r + 15) / 16 * 16;
     mp.stride = mp.dkp + 8;
@@ -550,7 +541,7 @@ int launch_latent_attn_kt(const Batch& b, const LatentDims& L, const float* qa, 
     if (rc) return rc;
     if (mp.splits > 1) {
         dim3 grid(b.n, L.H);
-        launch_pdl(latent_attn_merge_kernel, grid, L.R < 512 ? (L.R + 31) & ~31 : 512, 0, s, L.H, L.R, mp.splits, workspace, (__nv_bfloat16*)out, L.sink);
+        launch_pdl(latent_attn_merge_kernel, grid, (L.R + 31) & ~31, 0, s, L.H, L.R, mp.splits, workspace, (__nv_bfloat16*)out, L.sink);
         return launch_check(cudaGetLastError(), "latent_attn_merge");
     }
     return WF_OK;
@@ -578,7 +569,7 @@ int launch_latent_attn_mma(const Batch& b, const LatentDims& L, const float* qa,
                            int splits, cudaStream_t s) {
     if (b.n <= 0) return WF_OK;
     MmaParams mp;
-    mp.splits = splits < 1 ? 1 : (splits > 16 ? 16 : splits);
+    mp.splits = splits < 1 ? 1 : (splits > ATTN_MAX_SPLITS ? ATTN_MAX_SPLITS : splits);
     mp.part = workspace;
     mp.dkp = (L.R + L.r + 15) / 16 * 16;
     mp.stride = mp.dkp + 8;
@@ -600,7 +591,7 @@ int launch_latent_attn_mma(const Batch& b, const LatentDims& L, const float* qa,
     if (rc) return rc;
     if (mp.splits > 1) {
         dim3 grid(b.n, L.H);
-        launch_pdl(latent_attn_merge_kernel, grid, L.R < 512 ? (L.R + 31) & ~31 : 512, 0, s, L.H, L.R, mp.splits, workspace, (__nv_bfloat16*)out, L.sink);
+        launch_pdl(latent_attn_merge_kernel, grid, (L.R + 31) & ~31, 0, s, L.H, L.R, mp.splits, workspace, (__nv_bfloat16*)out, L.sink);
         return launch_check(cudaGetLastError(), "latent_attn_merge");
     }
     return WF_OK;
