@@ -252,7 +252,9 @@ int wf_engine_finalize_weights(wf_engine* e);
 /* Sequence slots: block tables are managed by the engine (free-list page allocator with the
  * KVCacheManager semantics, tests/test_kv_cache_cpp.py:44-70). */
 int wf_engine_reset(wf_engine* e);
-/* mark slot b as holding `len` tokens of (synthetic/garbage) context: allocates pages only (bench); in order on the engine's stream */
+/* mark slot b as holding `len` tokens of (synthetic/garbage) context: allocates pages only (bench).  With fill_random it returns when the pages are filled; without, it is
+ * asynchronous: position and length are set in order on the engine's stream, behind steps in flight and ahead of later ones, and a reader of wf_engine_buffer's pointers on
+ * another stream waits for wf_engine_sync first. */
 int wf_engine_set_context(wf_engine* e, int slot, int len, int fill_random);
 
 /* One decode step for B sequences (slots 0..B-1): HOST token ids in, HOST next-token ids out

@@ -322,6 +322,47 @@ def test_tcgen05_decode_linears_equal_per_op_kernels(B, ctx, monkeypatch):
         assert (na == nb).all() and (nc == nb).all()
 
 
+def _set_back(waiting, slots=(0, 2, 3, 5), device=0, caller=0):
+    """Thirty fed-back steps, some slots set back behind them, two more steps: positions, lengths, next tokens and logits of the last."""
+    from wf_bitnet.engine import Engine, EngineConfig
+    cfg = EngineConfig(hidden=256, layers=2, heads=2, kv_heads=1, ffn=384, vocab=512, max_seq=256, max_batch=6)
+    wait = (lambda: eng.sync()) if waiting else (lambda: None)
+    with torch.cuda.device(device):
+        eng = Engine(cfg)
+        eng.init_synthetic(3)
+        for slot in range(6):
+            eng.set_context(slot, 40 + slot, fill_random=True)
+        eng.decode([1, 2, 3, 4, 5, 6])
+        for _ in range(30):
+            eng.decode_device(6)
+    wait()
+    with torch.cuda.device(caller):
+        for slot in slots:
+            eng.set_context(slot, 20 + slot)
+        assert torch.cuda.current_device() == caller
+    wait()
+    with torch.cuda.device(device):
+        for _ in range(2):
+            eng.decode_device(6)
+            wait()
+        out = [eng.buffer(n, (6,), torch.int32).cpu() for n in ("positions", "seq_lens", "next")] + [eng.buffer("logits", (6, cfg.vocab), torch.float32).cpu()]
+        eng.close()
+    assert out[0].tolist() == [(20 + s if s in slots else 71 + s) + 2 for s in range(6)] and torch.equal(out[1], out[0] + 1)
+    return out
+
+
+def test_contexts_set_behind_steps_in_flight_take_effect_with_the_next_step():
+    """Without fill_random a slot's context is set in order on the engine's stream, with no wait on either side: the same as with one before and behind it."""
+    for a, b in zip(_set_back(False), _set_back(True)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="two GPUs")
+def test_a_context_is_set_whichever_device_is_current():
+    for a, b in zip(_set_back(False, device=1, caller=0), _set_back(True, device=1, caller=1)):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("shape", ["2b", "8b"])
 def test_batches_of_changing_size_equal_per_op_kernels(shape, monkeypatch):
     """Steps that change between the forms of gate|up (activation where CTA pairs store it from 33 rows on, sums in a cleared buffer below): nothing of one is left for the other."""

@@ -36,6 +36,7 @@ const char* kLinNames[7] = {"q", "k", "v", "o", "gate", "up", "down"};
 struct wf_engine {
     wf_model_config cfg;
     cudaStream_t stream = nullptr;
+    int device = 0;                          // the stream's
     std::vector<LayerW> layers;
     __nv_bfloat16 *embed = nullptr, *final_norm = nullptr, *cos_tab = nullptr, *sin_tab = nullptr;
     // local (per TP rank) dims: H / Hkv heads, ffn rows, attn_dim = H*D of THIS rank; *_full = the whole model's
@@ -669,7 +670,7 @@ extern "C" int wf_engine_create(const wf_model_config* cfg, wf_engine** out) {
     }
     int rc = WF_OK;
     auto fail = [&](int r) { wf_engine_destroy(e); return r; };
-    if (cuda_check(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking), "stream create")) return fail(WF_ERR_CUDA);
+    if (cuda_check(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking), "stream create") || cuda_check(cudaGetDevice(&e->device), "device")) return fail(WF_ERR_CUDA);
     init_all_kernel_attrs();
     fused_init_attrs();
     cudaGetLastError();
@@ -970,8 +971,14 @@ extern "C" int wf_engine_set_context(wf_engine* e, int slot, int len, int fill_r
     e->pt.dirty = true;
     e->h_pos[slot] = len;
     // on the engine stream (an in-flight asynchronous step's advance kernel updates the same words); one launch with the length by value in place of two copies from the
-    // stack and the wait for them: 6 us less of the caller's time (64 sequences set back between four steps: 20039 -> 19640 us in all)
-    if (int rc = launch_set_context(e->d_pos + slot, e->d_len + slot, len, e->stream)) return rc;
+    // stack and a wait for them: 64 slots in a row, with a wait for the last, 519 -> 214 us (one launch each and a wait each 546).  A launch, unlike a copy, wants its
+    // stream's device to be the caller's current one.
+    int current = e->device;
+    if (cuda_check(cudaGetDevice(&current), "set_context device")) return WF_ERR_CUDA;
+    if (current != e->device && cuda_check(cudaSetDevice(e->device), "set_context device")) return WF_ERR_CUDA;
+    const int rc_words = launch_set_context(e->d_pos + slot, e->d_len + slot, len, e->stream);
+    if (current != e->device && cuda_check(cudaSetDevice(current), "set_context device")) return WF_ERR_CUDA;
+    if (rc_words) return rc_words;
     if (fill_random) {
         // a page is one contiguous run of layers*2*Hkv*page_size*D elements
         const size_t page_elems = (size_t)e->cfg.layers * 2 * e->Hkv * ps * e->D;

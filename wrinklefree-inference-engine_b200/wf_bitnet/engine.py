@@ -119,6 +119,7 @@ class Engine:
         check(lib().wf_engine_reset(self._h))
 
     def set_context(self, slot: int, length: int, fill_random: bool = False) -> None:
+        """Slot `slot` holds `length` tokens of context from here on.  Without fill_random asynchronous, in order on the engine's stream."""
         check(lib().wf_engine_set_context(self._h, slot, length, 1 if fill_random else 0))
 
     def device_bytes(self) -> int:
