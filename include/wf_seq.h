@@ -237,6 +237,10 @@ int wf_seq_set_length(wf_seq_engine* e, int slot, int len);
 int wf_seq_op_gemm(int dtype, const void* A, int a_f32, int lda, const void* B, int ldb, void* C, int c_f32, int ldc, int M, int N, int K,
                    const int32_t* tile_group, long long group_stride, int n_groups, int algo, void* stream);
 
+/* whether a recurrence with one decay per head and no correction (state space; normaliser: matrix memory) takes nseq prompt portions of `tokens` tokens in all, the longest of
+ * `longest`, in segments of 128 tokens that run at once, where the engine has the workspace for it (csrc/seq/seq_segment.cu) */
+int wf_seq_in_segments(int heads, int key_heads, int dim, int vdim, int normaliser, int nseq, int tokens, int longest);
+
 #ifdef __cplusplus
 }
 #endif

@@ -113,11 +113,26 @@ def test_matrix_memory(heads, dim, vdim, lens, cuts):
     check(cfg, w, {"l0.mix.left.rel": (8, 2)}, lambda x: FO.matrix_memory(x, d64(w, "l0.mix.right."), "", right, EPS), lens, cuts, W)
 
 
-# long portions: segments of 128 tokens all at once.  Whole segments, a last one of one token and of one less than a whole one, a carried state, two sequences of unequal
-# segments; key sizes that leave rows of a warp over, value sizes below, at and beyond 64 columns
+# long portions, of which some sizes of heads take some in segments of 128 tokens all at once
 @pytest.mark.parametrize("lens,cuts", [([512], [[512]]), ([670, 513], [[30, 513], [640, 0]]), ([639], [[639]])])
 @pytest.mark.parametrize("kind,heads,groups,dim,vdim", [("ssd", 4, 2, 128, 64), ("ssd", 6, 3, 20, 12), ("ssd", 8, 1, 64, 68), ("memory", 2, 2, 128, 128), ("memory", 3, 3, 24, 15)])
 def test_segments(kind, heads, groups, dim, vdim, lens, cuts):
+    check_plain(kind, heads, groups, dim, vdim, lens, cuts)
+
+
+# Whole segments, a last one of one token and of one less than a whole one, a carried state, a sequence of less than a segment beside them; key sizes that leave rows of a warp over,
+# value sizes below, at and beyond 64 columns, several heads on a key head and one
+@pytest.mark.parametrize("kind,heads,groups,dim,vdim,lens,cuts", [
+    *((*k, *c) for k in (("ssd", 8, 2, 128, 64), ("ssd", 6, 3, 20, 12), ("ssd", 8, 1, 64, 68), ("memory", 3, 3, 24, 15), ("memory", 14, 14, 128, 128))
+      for c in (([799, 70], [[30, 0], [769, 70]]), ([767, 31], [[767, 31]]), ([768, 1], [[768, 1]]))),
+    ("ssd", 32, 1, 64, 68, [512], [[512]]), ("ssd", 24, 2, 68, 33, [640, 513], [[640, 513]]), ("ssd", 32, 1, 64, 68, [540, 639], [[28, 0], [512, 639]])])
+def test_portions_taken_in_segments(kind, heads, groups, dim, vdim, lens, cuts):
+    from wf_bitnet import _lib
+    assert _lib.seq_lib().wf_seq_in_segments(heads, groups, dim, vdim, kind == "memory", sum(c > 0 for c in cuts[-1]), sum(cuts[-1]), max(cuts[-1]))
+    check_plain(kind, heads, groups, dim, vdim, lens, cuts)
+
+
+def check_plain(kind, heads, groups, dim, vdim, lens, cuts):
     W = 40
     left = {"heads": 2, "kv_heads": 1, "dim": 8, "vdim": 8, "scale": 0.3, "mask": {"size": 8}}
     if kind == "ssd":
@@ -152,6 +167,39 @@ def nonfinite_layer(kind):
     cfg = {"architecture": arch, "vocab": 31, "width": W, "embedding": {"scale": 1.0}, "norm": {"eps": EPS},
            "layers": [{"type": "parallel", "mixer": {"left": left, "left_scale": 0.0, "right": right, "right_scale": 1.0}, "mlp": None}]}
     return cfg, make(cfg), shapes, W
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), 3e38, 1e13])
+@pytest.mark.parametrize("at", [0, 37, 530, 745])
+@pytest.mark.parametrize("kind", ["state_space", "memory"])
+def test_numbers_that_are_not_finite_in_segments(kind, at, bad, monkeypatch):
+    """The same for a long portion and a short one beside it in segments: such a number in one of them (from row 740 on the short one's) leaves the other as it is."""
+    from wf_bitnet import _lib, registry
+    assert _lib.seq_lib().wf_seq_in_segments(4, 2 if kind == "state_space" else 4, 64, 32, kind == "memory", 2, 800, 740)
+    monkeypatch.setenv("WF_SEQ_ATTN_MMA", "0")
+    cfg, weights, shapes, W = nonfinite_layer(kind)
+    cls = registry.resolve(cfg)
+    extra = {"shapes": shapes} if getattr(cls, "reads_shapes", False) else {}
+    m = cls(cfg, dtype="bfloat16", max_tokens=2000, slots=4, page_size=16, max_step_tokens=800, **extra)
+    m.load_weights((k, v.numpy(), "F32") for k, v in weights.items())
+    g = np.random.default_rng(8)
+    rows = torch.from_numpy(g.standard_normal((900, W)).astype(np.float32)).to(torch.bfloat16).float().numpy()
+    rows[at, 3] = bad
+    first, second = np.r_[0:740, 800:850], np.r_[740:800, 850:900]         # what each sequence is fed: a portion of the first step, then 50 rows
+    a, b, c, d = (m.admit() for _ in range(4))
+    whole = np.empty((900, W), np.float32)
+    whole[:800], whole[800:] = m.engine.run_part(0, 2, [a, b], [740, 60], rows[:800]), m.engine.run_part(0, 2, [a, b], [50, 50], rows[800:])
+    pieces = np.empty_like(whole)
+    for slot, idx in ((c, first), (d, second)):
+        pieces[idx] = np.concatenate([m.engine.run_part(0, 2, [slot], [len(idx[t:t + 31])], rows[idx[t:t + 31]]) for t in range(0, len(idx), 31)])
+    m.close()
+    ok, want = np.isfinite(whole).all(-1), np.isfinite(pieces).all(-1)
+    assert np.array_equal(ok, want), (np.flatnonzero(ok != want), ok.sum(), want.sum())
+    hit = first if at < 740 else second
+    clean = np.r_[second if at < 740 else first, hit[hit < at]]
+    assert want[clean].all()
+    x, y = whole[clean], pieces[clean]
+    assert (np.sqrt(((x - y) ** 2).mean(-1)) / np.sqrt((y ** 2).mean(-1))).max() < 2e-2          # two bf16 roundings of the same float values, and the products around them
 
 
 @pytest.mark.parametrize("bad", [float("nan"), float("inf"), 3e38, 1e13])

@@ -244,6 +244,18 @@ def test_the_helper_for_token_lists_is_this_interpreters_and_opened_on_use(tmp_p
     assert _lib.py_i32() is not None and np.array_equal(_i32(ids), ids)
 
 
+@pytest.mark.parametrize("heads,key_heads,dim,vdim,memory,lens,so", [
+    (40, 5, 128, 64, 0, [2048], 1), (40, 5, 128, 64, 0, [512], 1), (40, 5, 128, 64, 0, [511], 0), (40, 5, 128, 64, 0, [600] * 3, 0), (40, 5, 128, 64, 0, [1024] * 2, 1),
+    (40, 5, 128, 64, 0, [1700, 100], 1), (8, 1, 128, 64, 0, [1024], 0), (8, 1, 128, 64, 0, [4096], 1), (16, 2, 128, 128, 0, [512] * 4, 0), (16, 2, 128, 128, 0, [600] * 3, 0),
+    (16, 2, 128, 128, 0, [801, 600, 400], 1), (16, 2, 64, 64, 0, [600] * 3, 1),
+    (16, 16, 128, 128, 1, [512] * 2, 0), (16, 16, 128, 128, 1, [2048], 0), (16, 16, 128, 128, 1, [1500, 400, 100], 1), (4, 4, 128, 128, 1, [900, 300, 300, 300], 0),
+    (4, 4, 64, 128, 1, [1200, 400, 400], 1), (40, 40, 128, 64, 0, [1024] * 2, 0), (40, 40, 128, 64, 0, [1700, 100], 1)])
+def test_which_portions_a_recurrence_takes_in_segments(heads, key_heads, dim, vdim, memory, lens, so):
+    """Both sides of the lines between the two forms, each as measured on 148 SMs."""
+    from wf_bitnet import _lib
+    assert _lib.seq_lib().wf_seq_in_segments(heads, key_heads, dim, vdim, memory, len(lens), sum(lens), max(lens)) == so
+
+
 def _make_seq(tmp_path, *overrides):
     """`make seq` with the CUDA library taken as built and the helper for token lists written to tmp_path."""
     import shutil

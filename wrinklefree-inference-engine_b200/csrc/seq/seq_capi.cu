@@ -1,5 +1,5 @@
 // Per-op C entry points of the sequence-model kernels (tests and measurements call the launchers the engine uses).
-#include "seq_kernels.cuh"
+#include "seq_chunk.cuh"
 #include "wf_seq.h"
 
 using namespace wf;
@@ -17,4 +17,11 @@ extern "C" int wf_seq_op_gemm(int dtype, const void* A, int a_f32, int lda, cons
         if (dtype != WF_SEQ_F32 && gemm_tc_error((cudaStream_t)stream)) { set_error("wf_seq_op_gemm: a bounded wait of the tcgen05 kernel ran out"); return WF_ERR_CUDA; }
     }
     return WF_OK;
+}
+
+extern "C" int wf_seq_in_segments(int heads, int key_heads, int dim, int vdim, int normaliser, int nseq, int tokens, int longest) {
+    if (key_heads < 1 || heads < key_heads || heads % key_heads || dim < 1 || dim > 128 || vdim < 1) return 0;
+    DeltaDims D{heads, key_heads, dim, vdim, 0, 1};
+    D.ones_col = normaliser != 0;
+    return segments_faster(D, nseq, tokens, longest);
 }

@@ -20,6 +20,7 @@ __device__ __forceinline__ void cr_watch(float& w, float x) { w = fmaf(x, 0.f, w
 
 // Recurrences with one decay per head and no correction, in segments of SCAN_CHUNK tokens (seq_segment.cu): the segments' own end states and products q k in w.rec,
 // the chain between them, the outputs.  What it marks is left to chunk_redo_kernel.
+bool segments_faster(const DeltaDims& D, int nseq, int n, int max_len);          // n tokens in nseq portions
 bool segments_usable(const Batch& b, const DeltaDims& D, const ScanWorkspace* scan);
 int launch_segments(const Batch& b, const DeltaDims& D, const ChunkView& w, const float* decay, float* state, size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan);
 

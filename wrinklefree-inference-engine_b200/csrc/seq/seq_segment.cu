@@ -14,6 +14,7 @@
 // overlap taken off: 173 us 16 tokens at a time (records 30, two passes 48 + 76, their chain 26), 131 so (sums 46, chain 14, outputs 65).
 // Numbers that are not finite: everything read and formed is watched, and what is marked is taken again by chunk_redo_kernel, as in seq_chunk.cu.
 #include "seq_chunk.cuh"
+#include <math.h>
 
 namespace wf {
 namespace seq {
@@ -475,14 +476,43 @@ size_t segment_workspace_floats(const DeltaDims& D, int max_step_tokens, int slo
     return D.no_delta && !D.vec_decay && max_step_tokens >= 4 * SG ? (size_t)scan_chunks_needed(max_step_tokens, slots) * D.Hk * SG_G : 0;
 }
 
-// Long portions only: a segment moves its state five times through memory and its blocks cost their latencies however few the tokens.  us, 16 tokens at a time -> so:
-// 40 heads of 128 x 64, one portion of 256 tokens 38 / 48, of 512 67 / 67, 1024 104 / 88, 2048 173 / 131; 4 of 300 84 / 102, 4 of 512 134 / 132, 2 of 1024 162 / 130;
-// 16 heads of 64 x 64, one of 256 25 / 32, 512 35 / 34, 2048 63 / 46; 4 of 300 35 / 44, 4 of 512 53 / 46.
-// Three portions and more of about one length fill the machine 16 tokens at a time: 40 heads, 3 of 600 115 / 125, but one of 801, 600 and 400 141 / 129.
+// Whether portions are taken in segments, by what 22 sets of portions of 19 sizes of heads took in both forms (us, 16 tokens at a time / so).  Long portions only: a segment moves
+// its state five times through memory and its blocks cost their latencies however few the tokens; 40 heads of 128 x 64 over 5, one portion of 256 tokens 38 / 48.
+//   * The longest well beyond the average: the other form waits for it with SMs idle.  40 heads over 5, 1700 and 100 tokens 1.9 times as fast so; matrix memory, 16 heads of
+//     64 x 128, 1500, 400 and 100 tokens 1.35.  Not where heads have keys of their own, 128 wide, and the other form cuts its portions, too (other_in_passes): matrix memory, 4
+//     heads of 128 x 128, 900 and 3 x 300 tokens 0.86.
+//   * About one length: only where several heads share a key head's products q k.  With keys of their own segments lose more often than they gain (matrix memory, whose normaliser
+//     column takes 64 columns for itself besides: 16 heads of 128 x 128, 2 of 512 tokens 0.68, 2 of 2048 0.79; at best 32 heads of 64 x 64, 1024 tokens 1.14).  Shared, by the
+//     times of both: rounds of blocks over the SMs, each kernel to about 15 %.  40 heads of 128 x 64 over 5, 512 tokens 1.09, 2048 1.32; 16 of 128 x 128 over 2, 1024 1.23; but 8 of
+//     128 x 64 over 1, 1024 tokens 0.79, 16 of 128 x 128 over 2, 4 of 512 0.81.
+// Of those 418 sets five are slower so than the other form by more than 2 %, the worst by 10 (16 heads of 128 x 128 over 2, one portion of 512).
+bool segments_faster(const DeltaDims& D, int nseq, int n, int max_len) {
+    const long long sms = sm_count();
+    const int dvs = D.dv + D.ones_col, cols = (dvs + CR_COLS - 1) / CR_COLS, z = (dvs + SG_COLS - 1) / SG_COLS;
+    if (!D.no_delta || D.vec_decay || nseq < 1 || max_len < 4 * SG || n < 3LL * SG * nseq) return false;
+    const long long tiles = (long long)nseq * D.H * cols, pairs = (long long)nseq * D.H * ((cols + 1) / 2);
+    const bool big = D.d > 64, shared = D.H >= 4 * D.Hk, other_in_passes = 2 * tiles < 3 * sms;
+    if (5LL * max_len * nseq > 7LL * n) return shared || !big || !other_in_passes;
+    if (!shared) return false;
+    auto rounds = [&](double blocks) { return ceil(blocks / (double)sms); };
+    const double segs = n / (double)SG + 0.5 * nseq, heads = segs * D.H;
+    double so = big ? 21. + 17. * rounds(heads * z) + 12. * segs * D.Hk / sms : 15. + 12. * rounds(heads * z) + 7. * segs * D.Hk / sms;
+    double other = 4. + (big ? 5e-3 : 3.7e-3) * n / CHUNK_TOKENS * D.H;          // the preparation, then the scan
+    if (other_in_passes) {
+        const double one = 0.84 * heads * cols / sms, two = 1.3 * heads * ((cols + 1) / 2) / sms, chunks = SG / CHUNK_TOKENS * (one < two ? one : two);
+        other += big ? 19. + 1.3 * chunks : 17. + 0.85 * chunks;                  // (the chain of the passes is the same kernel as here)
+    } else {
+        auto chunk = [&](long long blocks, double one, double two, double more) { const long long k = (blocks + sms - 1) / sms; return k <= 1 ? one : k == 2 ? two : more * (double)k; };
+        const double one = chunk(tiles, 1.2, 1.7, 0.84), two = chunk(pairs, 1.5, 2.6, 1.3);
+        other += 8. + (big ? 0.91 : 0.67) * max_len / CHUNK_TOKENS * (one < two ? one : two);
+        so += 3. + 2.2e-6 * heads * D.d * dvs;
+    }
+    return so < 0.95 * other;
+}
+
 bool segments_usable(const Batch& b, const DeltaDims& D, const ScanWorkspace* scan) {
-    const long long segs = b.n / SG + b.nseq + 1, tiles = (long long)b.nseq * D.H * ((D.dv + D.ones_col + CR_COLS - 1) / CR_COLS);
-    return D.no_delta && !D.vec_decay && b.max_len >= 4 * SG && b.n >= 3LL * SG * b.nseq && (tiles < 3 * sm_count() || 5LL * b.max_len > 2LL * b.n) && scan->local &&
-           segs <= scan->chunks && (size_t)segs * D.Hk * SG_G <= scan->rec_floats && D.H + D.Hk <= 65535;
+    const long long segs = b.n / SG + b.nseq + 1;
+    return segments_faster(D, b.nseq, b.n, b.max_len) && scan->local && segs <= scan->chunks && (size_t)segs * D.Hk * SG_G <= scan->rec_floats && D.H + D.Hk <= 65535;
 }
 
 int launch_segments(const Batch& b, const DeltaDims& D, const ChunkView& w, const float* decay, float* state, size_t slot_stride, float* o, cudaStream_t s, const ScanWorkspace* scan) {

@@ -197,6 +197,7 @@ SEQ_SYMBOLS = {
     "wf_seq_profile_step": (_i, [_vp, _i, _vp, _vp, _i, C.c_char_p, _sz]),
     "wf_seq_set_length": (_i, [_vp, _i, _i]),
     "wf_seq_key_splits": (_i, [_vp]),
+    "wf_seq_in_segments": (_i, [_i] * 8),
     "wf_seq_op_gemm": (_i, [_i, _vp, _i, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _vp, C.c_longlong, _i, _i, _vp]),
 }
 _seq_lib = None
