@@ -378,6 +378,20 @@ def test_batches_of_changing_size_equal_per_op_kernels(shape, monkeypatch):
         assert (na == nb).all()
 
 
+@pytest.mark.parametrize("hidden", [3968, 4096])
+def test_row_kernels_equal_per_op_kernels_where_their_forms_change(hidden, monkeypatch):
+    """Rows of 4096 leave the registers above 24 sequences, narrower ones do not; both sides of it, and a few sequences, in steps that follow one another."""
+    from wf_bitnet.engine import EngineConfig
+    cfg = EngineConfig(hidden=hidden, layers=1, heads=hidden // 128, kv_heads=hidden // 128, ffn=512, vocab=4096, max_seq=128, max_batch=33)
+    rng = np.random.default_rng(hidden)
+    steps = [list(map(int, rng.integers(0, cfg.vocab, B))) for B in (33, 2, 8, 9, 24, 25, 32)]
+    a = _run_tokens(cfg, None, True, steps, monkeypatch, ctx=20, synthetic=6)
+    b = _run_tokens(cfg, None, False, steps, monkeypatch, ctx=20, synthetic=6)
+    for i, ((la, na, _), (lb, nb, _)) in enumerate(zip(a, b)):
+        assert torch.equal(la, lb), (i, (la - lb).abs().max().item())
+        assert (na == nb).all()
+
+
 @pytest.mark.parametrize("shape,B,ctx", [("2b", 2, 80), ("2b", 13, 200), ("2b", 32, 120), ("8b", 1, 90), ("8b", 5, 90), ("8b", 16, 150), ("8b", 32, 60)])
 def test_streaming_decode_gemm_equals_default_kernels(shape, B, ctx, monkeypatch):
     """WF_DECODE_STREAM=2: every decode linear of 2..32 rows on the streaming batched GEMM (gemm_stream.cu: K windows, TMA ring, masked

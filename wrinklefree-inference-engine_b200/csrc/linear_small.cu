@@ -393,14 +393,16 @@ int launch_glue_rows(const GlueParams& g, cudaStream_t s, bool pdl) {
         cfg.numAttrs = pdl ? 2 : 1;
         return launch_check(cudaLaunchKernelEx(&cfg, glue_rows_cluster_kernel, g), "glue_rows_cluster");
     }
-    // In registers: ms a step, through shared memory / so: 2B (rows of 2560 and 6912), 2 sequences 1.33 / 1.24, 16 1.58 / 1.53, 24 1.98 / 1.86, 48 1.71 / 1.67, 64 1.97 / 1.96;
-    // 8B (4096) 16 sequences 2.39 / 2.34, 24 3.13 / 3.03, but 8 2.01 / 2.04 and 64 3.05 / 3.14.
-    const bool odd = g.K > 3072 && g.K <= 8 * GR_T && (g.M <= 8 || g.M > GLUE_LATE);
-    const int it = g.mode == GL_RELU2 || g.acc_own_cols > 0 || odd || g.K > 2 * 8 * GR_T ? 0 : g.K > 8 * GR_T ? 2 : 1;
+    // In registers, and without the shared memory that the other form needs: us a layer of the engine at 60 tokens, through shared memory / so, 2, 8, 24 and 64 sequences: 2B widths
+    // (rows of 2560 and 6912) 42.3 / 39.4, 46.4 / 44.2, 63.5 / 59.4, 55.0 / 55.7; 3584 wide 53.4 / 51.4, 55.7 / 53.9, 76.2 / 72.5, 68.3 / 69.0; 8192 wide 107.7 / 104.4, 106.3 / 104.2,
+    // 204 / 202, 189 / 187.  Only rows that give each of the block's threads one vector, 4096 wide, lose from some size on (8B 58.4 / 55.4, 61.6 / 58.7, 94.8 / 92.0, but 32 sequences
+    // 88.5 / 91.2 and 64 81.6 / 85.3; with ffn rows of 11008 even at 26, 2 % at 32 and 64), for a reason not found: 3968 wide the two are within 2 % from 20 sequences on.
+    const bool full = g.K == 8 * GR_T && g.M > 24;
+    const int it = g.mode == GL_RELU2 || g.acc_own_cols > 0 || full || g.K > 2 * 8 * GR_T ? 0 : g.K > 8 * GR_T ? 2 : 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(g.M);
     cfg.blockDim = dim3(GR_T);
-    cfg.dynamicSmemBytes = (size_t)g.K * 2;
+    cfg.dynamicSmemBytes = it ? 0 : (size_t)g.K * 2;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     set_pdl(cfg, at, pdl);
