@@ -366,8 +366,8 @@ def test_state_is_carried_over_hundreds_of_tokens():
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("heads,kv,dim", [(3, 1, 8), (9, 3, 64), (28, 4, 128)])
 def test_attention_inputs_of_few_and_of_many_tokens(dtype, heads, kv, dim):
-    """Queries, keys and gates of a portion are formed by blocks that hold several vectors a warp up to four tokens per multiprocessor and one beyond it; gates by blocks of
-    their own, fewer than a block's threads, one round of them and more than one.  One long portion, and the lengths on both sides of the border, against the oracle."""
+    """Queries, keys and gates of a portion are formed by blocks that hold several vectors a warp up to four tokens per multiprocessor and one beyond it, where gates have blocks of
+    their own: fewer than a block's threads, one round of them and more than one.  One long portion, and the lengths on both sides of the border, against the oracle."""
     border = 4 * torch.cuda.get_device_properties(0).multi_processor_count
     cfg = config([par(heads=heads, kv=kv, dim=dim, vdim=dim, scale=dim ** -0.5, window=21, rot=(dim, 10000.0), ls=1.0, rs=0.0)], width=32)
     w = make_weights((cfg, {}), 171)

@@ -128,10 +128,12 @@ __global__ void __launch_bounds__(GP_MAXW * 32) gqa_prep_kernel(Batch b, GqaDims
 
 // The same for head sizes that are multiples of 4 up to 128 (no norm over the whole projection; pairs side by side, or half the rotated entries apart with
 // that half a multiple of 4): a head vector lies in the lanes of a warp four entries each, a warp's GQ vectors are requested before the cosines are formed,
-// and a pair's other entry comes from its lane.  Gates of elements are blocks of their own (blockIdx.y = 1), a thread's values requested together: formed beside the cosines, one
-// after the other, they were the longest chain of a block.  Few tokens: GQ = 4 vectors of a warp in flight; where blocks wait for SMs, one vector a warp and with it six blocks
-// an SM hide more.  2048 tokens, 20 + 5 + 5 heads of 128 with a gate per element (88 MB): 62 us one entry at a time; 33.5 with the gates beside the cosines, 29.6 apart
-// (GQ = 4), 26.0 (GQ = 2, six blocks), 25.6 so; the cosines themselves cost nothing that shows.
+// and a pair's other entry comes from its lane.  Few tokens: GQ = 4 vectors of a warp in flight, the gates formed beside the cosines.  Where blocks wait for SMs, one vector a warp
+// and with it six blocks an SM hide more, and gates of elements are blocks of their own (blockIdx.y = 1), a thread's values requested together: beside the cosines, one after the
+// other, they were the longest chain of a block.  2048 tokens, 20 + 5 + 5 heads of 128 with a gate per element (88 MB): 62 us one entry at a time; 33.5 with the gates beside the
+// cosines, 29.6 apart (GQ = 4), 26.0 (GQ = 2, six blocks), 25.6 so; the cosines themselves cost nothing that shows.  Few tokens' gate blocks save up to 1 us here, but the attention
+// behind starts when the last of them lets it in: both kernels, beside / apart, 8 + 2 + 2 heads: 80 tokens of four sequences 21.9 / 23.2, 300 28.0 / 27.0, one of 590 tokens
+// 37.4 / 42.2; 20 + 5 + 5 heads, one of 80 tokens 26.5 / 31.0.
 constexpr int GZ = 3;
 template <typename T, int GQ>
 __global__ void __launch_bounds__(256, GQ == 1 ? 6 : 4) gqa_prep_vec_kernel(Batch b, GqaDims D, const float* proj, int ld, int k_off, int v_off, int g_off, const T* qb,
@@ -180,15 +182,23 @@ __global__ void __launch_bounds__(256, GQ == 1 ? 6 : 4) gqa_prep_vec_kernel(Batc
             bi[k] = in && bias ? load4(bias + at) : zero;
         }
         if (u0 == warp) {
-            const int table = (half + 31) & ~31, t = (int)threadIdx.x - table;       // the other warps form the gates of heads meanwhile
+            const int table = (half + 31) & ~31, t = (int)threadIdx.x - table;       // the other warps form the gates meanwhile
             if ((int)threadIdx.x < half) {
                 const double a = (double)pos * (D.freq ? D.freq[threadIdx.x] : exp2(-2.0 * (double)threadIdx.x / (double)D.rope_dims * log2((double)D.rope_base)));
                 double sn, cs;
                 sincos(a, &sn, &cs);
                 rot_c[threadIdx.x] = (float)cs * D.mscale; rot_s[threadIdx.x] = (float)sn * D.mscale;
             } else if (gate && gridDim.y == 1 && t >= 0) {
-                const int ng = D.gate_elem ? D.H * D.dv : D.H;
-                for (int h = t; h < ng; h += (int)blockDim.x - table) gate[(size_t)i * ng + h] = g_off >= 0 ? sigmoid_f(row[g_off + h]) : 1.f;
+                const int ng = D.gate_elem ? D.H * D.dv : D.H, nt = (int)blockDim.x - table;
+                if (ng % 4 == 0 && g_off % 4 == 0 && g_off >= 0) {
+                    for (int h = t * 4; h < ng; h += nt * 4) {
+                        const float4 z = load4(row + g_off + h);
+                        const float o[4] = {sigmoid_f(z.x), sigmoid_f(z.y), sigmoid_f(z.z), sigmoid_f(z.w)};
+                        store4(gate + (size_t)i * ng + h, o);
+                    }
+                } else {
+                    for (int h = t; h < ng; h += nt) gate[(size_t)i * ng + h] = g_off >= 0 ? sigmoid_f(row[g_off + h]) : 1.f;
+                }
             }
             __syncthreads();
         }
@@ -432,8 +442,8 @@ int launch_gqa_prep(int dt, const Batch& b, const GqaDims& D, const float* proj,
         // more tokens are resident while their double-precision cosines are formed: 4096 tokens, 8 + 2 + 2 heads of 128 29.3 / 22.4 with four, 8 + 2 heads 20.6 / 16.8.
         const int units = D.H + (k_off >= 0 ? (D.v_is_k ? 1 : 2) * D.G : 0);
         const int threads = b.n <= 4 * sm_count() || (units > 24 && b.n <= 16 * sm_count()) ? 256 : units > 8 ? 128 : 96;
-        const dim3 grid(b.n, gate && D.gate_elem && g_off >= 0 && g_off % 4 == 0 ? 2 : 1);
         const bool few = b.n <= 4 * sm_count();
+        const dim3 grid(b.n, !few && gate && D.gate_elem && g_off >= 0 && g_off % 4 == 0 ? 2 : 1);
 #define GPV_LAUNCH(T, GQ) launch_pdl(gqa_prep_vec_kernel<T, GQ>, grid, threads, 0, s, b, D, proj, ld, k_off, v_off, g_off, (const T*)qb, (const T*)kb, (const T*)vb, eps, pc, (T*)qn, gate)
         if (dt == WF_BF16) { if (few) GPV_LAUNCH(__nv_bfloat16, 4); else GPV_LAUNCH(__nv_bfloat16, 1); }
         else { if (few) GPV_LAUNCH(float, 4); else GPV_LAUNCH(float, 1); }
