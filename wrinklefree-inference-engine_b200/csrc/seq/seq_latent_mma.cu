@@ -220,6 +220,9 @@ __global__ void latent_attn_mma_kernel(Batch b, LatentDims L, const float* qa, c
 // One block per (token, head), a thread per channel (both forms take latents of up to 512): out = sum_s exp(m_s - m) O_s / sum_s exp(m_s - m) l_s.  A lane per split for maxima and
 // sums; a thread's values of all splits are requested with them, before it is known which splits have keys.  Bound by latency: 20 heads of rank 512, 1 / 8 sequences 8.8 / 9.0 us
 // with 128 threads and maxima, sums and values one split after the other; 5.6 / 6.1 with the loads together; 2.4 / 3.3 with a thread per channel (8 ahead: 2.7 / 3.6).
+// S: as many as there are splits, or the next power of two.  Many rows have few splits and are bound by instructions: 130 and 148
+// tokens, two splits, 8.4 and 9.3 us, 15.2 and 16.9 with 16 whatever the splits (9.6 and 10.5 with 128 threads); 64 of rank 256, nine splits, 3.4.
+template <int S>
 __global__ void __launch_bounds__(512) latent_attn_merge_kernel(int H, int R, int splits, const float* part, __nv_bfloat16* __restrict__ out, const float* sink) {
     pdl_enter();
     static_assert(ATTN_MAX_SPLITS <= 32, "a lane per split");
@@ -228,9 +231,9 @@ __global__ void __launch_bounds__(512) latent_attn_merge_kernel(int H, int R, in
     const size_t sstride = (size_t)H * (R + 2);
     const bool mine = lane < splits;
     const float ms = mine ? p0[lane * sstride + R] : -INFINITY, ls = mine ? p0[lane * sstride + R + 1] : 0.f;
-    float q[ATTN_MAX_SPLITS];
+    float q[S];
 #pragma unroll
-    for (int s = 0; s < ATTN_MAX_SPLITS; ++s) q[s] = s < splits && c < R ? p0[s * sstride + c] : 0.f;
+    for (int s = 0; s < S; ++s) q[s] = s < splits && c < R ? p0[s * sstride + c] : 0.f;
     const float m = warp_max(ms), w = ms == -INFINITY ? 0.f : expf(ms - m);
     float l = warp_sum(ms == -INFINITY ? 0.f : w * ls);
     if (sink) l += expf(sink[h] - m);
@@ -238,11 +241,19 @@ __global__ void __launch_bounds__(512) latent_attn_merge_kernel(int H, int R, in
     const unsigned live = __ballot_sync(0xffffffffu, ms != -INFINITY);
     float v = 0.f;
 #pragma unroll
-    for (int s = 0; s < ATTN_MAX_SPLITS; ++s) {
+    for (int s = 0; s < S; ++s) {
         const float ws = __shfl_sync(0xffffffffu, w, s);
         if (live >> s & 1) v += ws * q[s];
     }
     if (c < R) out[((size_t)i * H + h) * R + c] = __float2bfloat16_rn(v * inv);
+}
+
+int launch_merge(const Batch& b, const LatentDims& L, int splits, const float* workspace, void* out, cudaStream_t s) {
+    const dim3 grid(b.n, L.H);
+#define LM_LAUNCH(S) launch_pdl(latent_attn_merge_kernel<S>, grid, (L.R + 31) & ~31, 0, s, L.H, L.R, splits, workspace, (__nv_bfloat16*)out, L.sink)
+    if (splits <= 2) LM_LAUNCH(2); else if (splits <= 4) LM_LAUNCH(4); else if (splits <= 8) LM_LAUNCH(8); else LM_LAUNCH(ATTN_MAX_SPLITS);
+#undef LM_LAUNCH
+    return launch_check(cudaGetLastError(), "latent_attn_merge");
 }
 
 
@@ -539,12 +550,7 @@ int launch_latent_attn_kt(const Batch& b, const LatentDims& L, const float* qa, 
 #undef KT_CASE
     if (rc == WF_ERR_UNSUPPORTED) set_error("latent_attn_kt: unsupported sizes (heads %d, latent %d)", L.H, L.R);
     if (rc) return rc;
-    if (mp.splits > 1) {
-        dim3 grid(b.n, L.H);
-        launch_pdl(latent_attn_merge_kernel, grid, (L.R + 31) & ~31, 0, s, L.H, L.R, mp.splits, workspace, (__nv_bfloat16*)out, L.sink);
-        return launch_check(cudaGetLastError(), "latent_attn_merge");
-    }
-    return WF_OK;
+    return mp.splits > 1 ? launch_merge(b, L, mp.splits, workspace, out, s) : WF_OK;
 }
 
 int latent_attn_mma_ctas_per_sm(const LatentDims& L) {
@@ -589,12 +595,7 @@ int launch_latent_attn_mma(const Batch& b, const LatentDims& L, const float* qa,
         default: set_error("latent_attn_mma: unsupported latent size %d", L.R); return WF_ERR_UNSUPPORTED;
     }
     if (rc) return rc;
-    if (mp.splits > 1) {
-        dim3 grid(b.n, L.H);
-        launch_pdl(latent_attn_merge_kernel, grid, (L.R + 31) & ~31, 0, s, L.H, L.R, mp.splits, workspace, (__nv_bfloat16*)out, L.sink);
-        return launch_check(cudaGetLastError(), "latent_attn_merge");
-    }
-    return WF_OK;
+    return mp.splits > 1 ? launch_merge(b, L, mp.splits, workspace, out, s) : WF_OK;
 }
 
 }  // namespace seq
