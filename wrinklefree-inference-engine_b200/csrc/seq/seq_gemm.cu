@@ -337,6 +337,7 @@ void gemv_launch(const GemmArgs& g, const PairArgs& pa, int rows, int ny, cudaSt
 // Bound: the weight stream, by latency on small matrices.  Measured with 8 rows against gemv_rows_kernel: 1024 x 2304 23.1 -> 9.3 us, 2560 x 6912
 // 64.6 -> 12.5, 13824 x 2560 43.7 -> 14.8, 128256 x 2560 298 -> 102; with 16 rows against gemm_mma_kernel: 2560 x 6912 131 -> 12.6.
 constexpr int FR_WARPS = 8;
+constexpr int FR_CARVEOUT = 14;                           // per cent of an SM's memory: four blocks' sums (0, which leaves room for less, takes twice as long)
 
 // U: 32-k blocks in flight per warp; OCC: blocks per SM
 // Weights that no kernel of the stream has written (b_const) are requested before the kernel waits for the one before it, as many as a warp has in flight: a
@@ -457,6 +458,13 @@ __global__ void __launch_bounds__(FR_WARPS * 32, OCC) gemm_few_kernel(GemmArgs g
 template <int NT, int WK, int U, int OCC>
 void few_launch(const GemmArgs& g, cudaStream_t s) {
     const int tiles = g.glu ? (g.N / 2 + 7) / 8 : (g.N + 15) / 16, per = FR_WARPS / WK, blocks = (tiles + per - 1) / per;
+    // An SM that kernels overlap on keeps the split between cache and shared memory that the first of them had.  Behind an attention its cache would be what 200 KB of shared
+    // memory leave, too little for the loads of four blocks under way: a decode step of 8 sequences, 6440 x 2560 behind the attention's output product 18.4 us, 9.7 with a split stated.
+    static DevOnce once;
+    if (once.need()) {
+        if (cudaFuncSetAttribute(gemm_few_kernel<NT, WK, U, OCC, true>, cudaFuncAttributePreferredSharedMemoryCarveout, FR_CARVEOUT) != cudaSuccess ||
+            cudaFuncSetAttribute(gemm_few_kernel<NT, WK, U, OCC, false>, cudaFuncAttributePreferredSharedMemoryCarveout, FR_CARVEOUT) != cudaSuccess) cudaGetLastError();      // a preference only
+    }
     if (g.c_f32) launch_pdl(gemm_few_kernel<NT, WK, U, OCC, true>, blocks, FR_WARPS * 32, 0, s, g); else launch_pdl(gemm_few_kernel<NT, WK, U, OCC, false>, blocks, FR_WARPS * 32, 0, s, g);
 }
 // Which split: a warp wants many loads in flight while there are fewer row tiles than SMs (2560 x 6912: 14.4 us, 15.7 with half as many); up to two tiles per SM a block
