@@ -133,7 +133,8 @@ __global__ void __launch_bounds__(GP_MAXW * 32) gqa_prep_kernel(Batch b, GqaDims
 // other, they were the longest chain of a block.  2048 tokens, 20 + 5 + 5 heads of 128 with a gate per element (88 MB): 62 us one entry at a time; 33.5 with the gates beside the
 // cosines, 29.6 apart (GQ = 4), 26.0 (GQ = 2, six blocks), 25.6 so; the cosines themselves cost nothing that shows.  Few tokens' gate blocks save up to 1 us here, but the attention
 // behind starts when the last of them lets it in: both kernels, beside / apart, 8 + 2 + 2 heads: 80 tokens of four sequences 21.9 / 23.2, 300 28.0 / 27.0, one of 590 tokens
-// 37.4 / 42.2; 20 + 5 + 5 heads, one of 80 tokens 26.5 / 31.0.
+// 37.4 / 42.2; 20 + 5 + 5 heads, one of 80 tokens 26.5 / 31.0.  Their form is compiled without the gates' blocks: with that branch it spills, and a decode step of 64 sequences
+// through four layers, three of them with attention, takes 396 us, 379 without.
 constexpr int GZ = 3;
 template <typename T, int GQ>
 __global__ void __launch_bounds__(256, GQ == 1 ? 6 : 4) gqa_prep_vec_kernel(Batch b, GqaDims D, const float* proj, int ld, int k_off, int v_off, int g_off, const T* qb,
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(256, GQ == 1 ? 6 : 4) gqa_prep_vec_kernel(Batc
     const int i = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, c = 4 * lane;
     const int sq = b.tok_seq[i], pos = b.tok_pos[i];
     const float* row = proj + (size_t)i * ld;
-    if (blockIdx.y) {
+    if (GQ == 1 && blockIdx.y) {
         const int ng = D.H * D.dv;
         float* out = gate + (size_t)i * ng;
         const int step = 4 * (int)blockDim.x;
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(256, GQ == 1 ? 6 : 4) gqa_prep_vec_kernel(Batc
                 double sn, cs;
                 sincos(a, &sn, &cs);
                 rot_c[threadIdx.x] = (float)cs * D.mscale; rot_s[threadIdx.x] = (float)sn * D.mscale;
-            } else if (gate && gridDim.y == 1 && t >= 0) {
+            } else if (gate && (GQ > 1 || gridDim.y == 1) && t >= 0) {
                 const int ng = D.gate_elem ? D.H * D.dv : D.H, nt = (int)blockDim.x - table;
                 if (ng % 4 == 0 && g_off % 4 == 0 && g_off >= 0) {
                     for (int h = t * 4; h < ng; h += nt * 4) {
