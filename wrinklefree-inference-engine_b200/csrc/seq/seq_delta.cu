@@ -367,24 +367,15 @@ __global__ void scan_prefix_kernel(Batch b, int H, int dd, int chunk, float* __r
     pdl_enter();
     const int sq = blockIdx.x, h = blockIdx.y, e = blockIdx.z * blockDim.x + threadIdx.x;
     if (e >= dd) return;
-    const int len = b.seq_len[sq], nc = (len + chunk - 1) / chunk, base = b.seq_start[sq] / chunk + sq, row = d > 0 ? e / (dd / d) : 0;
+    const int len = b.seq_len[sq], nc = (len + chunk - 1) / chunk, base = b.seq_start[sq] / chunk + sq;
     float* Sp = state + (size_t)b.seq_slot[sq] * slot_stride + (size_t)h * dd + e;
     float S = *Sp;
-    // SP chunks requested at once: only the additions wait for one another (16 chunks of 40 heads of 128 x 64: 26 -> 14 us)
-    constexpr int SP = 8;
-    for (int c0 = 0; c0 < nc; c0 += SP) {
-        float x[SP], p[SP];
-#pragma unroll
-        for (int k = 0; k < SP; ++k) {
-            const size_t entry = (size_t)(base + c0 + k) * H + h;
-            if (c0 + k < nc) { x[k] = __ldcg(local + entry * dd + e); p[k] = __ldcg(prod + (d > 0 ? entry * d + row : entry)); }
-        }
-#pragma unroll
-        for (int k = 0; k < SP; ++k) {
-            if (c0 + k >= nc) break;
-            startws[((size_t)(base + c0 + k) * H + h) * dd + e] = S;
-            S = fmaf(p[k], S, x[k]);
-        }
+    // One chunk after another by plain loads, a full SM of threads: what hides the latency.  us alone, chunks in L2, so / four at a time / eight at a time / eight and __ldcg: 40 heads of
+    // 128 x 64, 16 chunks 12.3 / 12.3 / 14.3 / 18.5; 20 of 128 x 129, 4 chunks 8.2 / 9.0 / 10.4 / 16.4, 16 12.3 / 13.2 / 15.2 / 27.5; but 8 of 128 x 129, 16 chunks 10.2 / 8.2 / 10.3 / 18.5.
+    for (int c = 0; c < nc; ++c) {
+        const size_t entry = (size_t)(base + c) * H + h;
+        startws[entry * dd + e] = S;
+        S = fmaf(d > 0 ? prod[entry * d + e / (dd / d)] : prod[entry], S, local[entry * dd + e]);
     }
     *Sp = S;
 }
