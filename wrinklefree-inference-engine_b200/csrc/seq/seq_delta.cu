@@ -115,9 +115,10 @@ __global__ void ssd_post_kernel(int H, int dv, int groups, const float* o, const
 }
 
 // The same with a group's values in registers between the two passes, four consecutive elements per load: gw a multiple of 4 up to 2048, dv one of 4.
-// 2048 tokens x 2560 channels in 5 groups (73 MB): 35 us with every input read twice, 16 so.
+// 2048 tokens x 2560 channels in 5 groups (73 MB): 35 us with every input read twice, 16 so.  The weights are requested with the inputs (300 tokens x 1024 3.1 -> 2.8 us), in
+// the 32 registers that a full SM allows: with the 34 that it takes otherwise 4000 tokens x 2560 27 -> 30 us.
 template <typename T>
-__global__ void __launch_bounds__(512) ssd_post_vec_kernel(int H, int dv, int groups, const float* o, const float* x, int ldx, const float* z, int ldz,
+__global__ void __launch_bounds__(512, 4) ssd_post_vec_kernel(int H, int dv, int groups, const float* o, const float* x, int ldx, const float* z, int ldz,
                                                            const T* Dskip, const T* w, float eps, T* __restrict__ y) {
     pdl_enter();
     __shared__ float scratch[33];
