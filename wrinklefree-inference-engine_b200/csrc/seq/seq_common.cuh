@@ -78,12 +78,21 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     __syncthreads();
     return warp_sum(lane < nw ? scratch[lane] : 0.f);
 }
-// the same where nothing else uses the scratch before
-__device__ __forceinline__ float block_sum_once(float v, float* scratch) {
+// the same where nothing else uses the scratch before.  many: of more blocks than SMs hold, where instructions count and not a block's latency, one warp adds for all (rows of 1024,
+// 4000 of them 12.4 -> 11.6 us; 300 2.4 / 2.6)
+__device__ __forceinline__ float block_sum_once(float v, float* scratch, bool many = false) {
     v = warp_sum(v);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
     if (lane == 0) scratch[w] = v;
     __syncthreads();
+    if (many) {
+        if (w == 0) {
+            v = warp_sum(lane < nw ? scratch[lane] : 0.f);
+            if (lane == 0) scratch[32] = v;
+        }
+        __syncthreads();
+        return scratch[32];
+    }
     return warp_sum(lane < nw ? scratch[lane] : 0.f);
 }
 __device__ __forceinline__ float gelu_erf_f(float z) { return 0.5f * z * (1.f + erff(z * 0.70710678118654752f)); }

@@ -242,7 +242,7 @@ __global__ void group_rmsnorm_kernel(const float* x, int ldx, const T* w, int gw
 template <typename T, int NV>
 __global__ void __launch_bounds__(1024) group_rmsnorm_vec_kernel(const float* x, int ldx, const T* w, int gw, float eps, const float* res, float* y, int ldy,
                                                                  T* __restrict__ y_t, int ldt, const int32_t* rows, const float* x2, float a, float b,
-                                                                 float w_offset) {
+                                                                 float w_offset, bool many) {
     pdl_enter();
     __shared__ float scratch[33];
     const int i = blockIdx.x, g = blockIdx.y;
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(1024) group_rmsnorm_vec_kernel(const float* x,
         if (x2) v[k] = make_float4(a * v[k].x + b * v2[k].x, a * v[k].y + b * v2[k].y, a * v[k].z + b * v2[k].z, a * v[k].w + b * v2[k].w);
         ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
     }
-    ss = block_sum_once(ss, scratch);
+    ss = block_sum_once(ss, scratch, many);
     const float inv = 1.f / sqrtf(ss / (float)gw + eps);
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
@@ -286,7 +286,7 @@ int launch_group_rmsnorm(int dt, const float* x, int ldx, const void* w, int gro
     if (W / groups % 4 == 0 && W / groups <= 8192 && ldx % 4 == 0 && ldy % 4 == 0 && ldt % 4 == 0 && vec_ok(x, 16) && vec_ok(x2, 16) && vec_ok(res, 16) && vec_ok(y, 16) &&
         vec_ok(w, 16) && vec_ok(y_t, 16)) {
         const int wide = W / groups;
-#define GR_LAUNCH(T, NV) launch_pdl(group_rmsnorm_vec_kernel<T, NV>, dim3(n, groups), vec_threads(wide), 0, s, x, ldx, (const T*)w, wide, eps, res, y, ldy, (T*)y_t, ldt, rows, x2, a, b, w_offset)
+#define GR_LAUNCH(T, NV) launch_pdl(group_rmsnorm_vec_kernel<T, NV>, dim3(n, groups), vec_threads(wide), 0, s, x, ldx, (const T*)w, wide, eps, res, y, ldy, (T*)y_t, ldt, rows, x2, a, b, w_offset, !few_blocks(dim3(n, groups)))
         if (dt == WF_BF16) { if (vec_groups(wide) == 1) GR_LAUNCH(__nv_bfloat16, 1); else GR_LAUNCH(__nv_bfloat16, 2); }
         else { if (vec_groups(wide) == 1) GR_LAUNCH(float, 1); else GR_LAUNCH(float, 2); }
 #undef GR_LAUNCH
