@@ -332,7 +332,7 @@ int run_step_tail(wf_engine* e, int B, int feed_back) {
 // The same step as phase kernels (fused_common.cuh): every linear leaves its raw accumulator in an fp32 buffer and the
 // NEXT phase applies scales / residual / relu^2*up / norm / re-quantisation in its prologue.
 //   B <= 8 : 5 launches per layer (qkv, attention, o, gate|up, down), each linear = glue prologue + TMA-streamed GEMV
-//   B  > 8 : 9 launches per layer (glue_rows + gemm_oneshot per linear, fused attention)
+//   B  > 8 : 10 launches per layer (glue_rows and a product per linear, relu^2(gate) * up, fused attention), 9 where gate|up stores the activation (from decode_tc_min rows on)
 // Tensor parallel (tp.size = T > 1): q|k|v and gate|up are split by output rows (whole heads), attention and
 // the KV pool by KV head, o and down by input columns.  The exchanges are fused into the producers (tp_comm.cuh):
 //   B  attention stores its heads into attn_full of every rank            (all-gather, flag 4l+0)
@@ -371,7 +371,8 @@ int run_step_fused(wf_engine* e, int B, int feed_back) {
         if (scatter) for (int r = 0; r < T; ++r) g.acc_peer[r] = reinterpret_cast<const float*>(e->tp.peer[r] + off);
     };
     // gate|up of batches that take the tcgen05 form: CTA pairs keep a tile's whole K and store relu^2(gate) * up themselves, instead of partial sums into a buffer that a
-    // kernel before has cleared and one behind reads.  ms a step at 200 tokens, 33 and 64 sequences: 2B 1.86 -> 1.76 and 2.18 -> 2.04, 8B 3.01 -> 2.64 and 3.50 -> 3.11
+    // kernel before has cleared and one behind reads.  ms a step at 200 tokens, 33 and 64 sequences: 2B 1.86 -> 1.76 and 2.18 -> 2.04, 8B 3.01 -> 2.64 and 3.50 -> 3.11.  Over widths of
+    // 1024 to 8192 with feed-forwards of 2816 to 28672, 33 to 64 sequences, a layer is 1.04 (1024) to 1.19 times as fast (4096 x 14336, 33 sequences 91.0 -> 76.7 us)
     const bool pair_gu = !tp && hx && e->decode_tc && B >= e->decode_tc_min && tc_wait_word();
     // one linear phase: prologue over the full activation vector of length Kfull, GEMV/GEMM over this rank's K columns
     auto phase = [&](GlueParams g, const uint8_t* w, int N, int Kfull, int K, int k_off, const TpDest& dest, int slot, bool first) -> int {

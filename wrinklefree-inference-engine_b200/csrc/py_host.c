@@ -6,8 +6,8 @@
 #endif
 #include <stdint.h>
 
-/* The n entries of a list as 32-bit integers; 0, and out in part written, when the object is not a list of n plain ints that fit.  A prompt of 2048 token ids: 5 us,
- * 58 as numpy.array(list). */
+/* The n entries of a list as 32-bit integers; 0, and out in part written, when the object is not a list of n plain ints that fit.  A prompt of 2048 token ids: 9 us,
+ * 54 as numpy.array(list). */
 int wf_py_i32(PyObject* list, int32_t* out, Py_ssize_t n) {
     if (!PyList_CheckExact(list) || PyList_GET_SIZE(list) != n) return 0;
     for (Py_ssize_t i = 0; i < n; ++i) {

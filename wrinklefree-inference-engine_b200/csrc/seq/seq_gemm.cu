@@ -467,12 +467,13 @@ void few_launch(const GemmArgs& g, cudaStream_t s) {
     }
     if (g.c_f32) launch_pdl(gemm_few_kernel<NT, WK, U, OCC, true>, blocks, FR_WARPS * 32, 0, s, g); else launch_pdl(gemm_few_kernel<NT, WK, U, OCC, false>, blocks, FR_WARPS * 32, 0, s, g);
 }
-// Which split: a warp wants many loads in flight while there are fewer row tiles than SMs (2560 x 6912: 14.4 us, 15.7 with half as many); up to two tiles per SM a block
-// has one and two blocks share an SM, with half as many a warp under way (8 rows back to back, against blocks of two tiles with four warps each: 4608 x 2560 7.9 -> 7.2 us,
-// 4608 x 6912 16.1 -> 14.6, 2400 x 6912 13.8 -> 11.8; a decode step of four layers 2560 wide 283 -> 266); beyond that resident blocks cover the latency (13824 x 2560: 14.6 us against 22.7 / 18.6 with
-// the first two; 128256 x 2560: 99 against 162 / 128).  There a block of one tile takes half the time of one of two, so the fuller rounds decide: us, two tiles / one:
-// one round of single tiles 4800 x 2560 11.3 / 9.0, 9472 x 6912 30.0 / 25.3; two rounds either way 13824 x 2560 16.1 / 17.1; three for four 20000 x 2560 25.1 / 22.8; as
-// many 32768 x 2560 30.7 / 32.3; seven for eight 65536 x 6912 147 / 141.  With 9 to 16 rows the registers hold half as much in flight and a second block stays resident.
+// Which split.  8 rows, weights from memory, back to back; us with blocks of one tile and eight warps: one block an SM with 8 loads a warp under way / two with 4 / four with 4; and four
+// blocks of two tiles with 4 warps each.  Up to a tile an SM a warp wants many loads under way: 1024 x 4096 4.3 / 5.6 / 7.7; 12.8, 2304 x 6912 8.3 / 9.7 / 12.8; 21.2.  Up to two
+// tiles two blocks share an SM: 2560 x 6912 14.8 / 10.5 / 13.1; 21.3, 4608 x 2560 8.2 / 5.7 / 7.0; 9.4 (a decode step of four layers 2560 wide 283 -> 266 us against blocks of two
+// tiles alone on an SM, 12.4 and 6.4 here).  Beyond, resident blocks cover the latency, and as a block of one tile takes half the time of one of two, the fuller rounds decide: one
+// round of single tiles 4800 x 2560 11.4 / 9.0 / 7.5; 9.5, 9472 x 6912 32.1 / 24.0 / 22.6; 27.7; two rounds either way 13824 x 2560 23.5 / 16.0 / 15.0; 13.5; three for four
+// 20000 x 2560 34.3 / 24.3 / 20.8; 22.9; as many 32768 x 2560 54.1 / 35.2 / 30.3; 28.4; seven for eight 65536 x 6912 205 / 154 / 139; 145; 128256 x 2560 204 / 134 / 106; 103.
+// With 9 to 16 rows the registers hold half as much in flight and a second block stays resident.
 template <int NT>
 void few_dispatch(const GemmArgs& g, cudaStream_t s) {
     const int tiles = (g.N + 15) / 16, sms = sm_count();
