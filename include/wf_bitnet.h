@@ -275,7 +275,7 @@ void* wf_engine_stream(wf_engine* e);
 size_t wf_engine_tp_handle_bytes(void);
 int wf_engine_tp_export(wf_engine* e, void* handle_out);
 int wf_engine_tp_attach(wf_engine* e, const void* handles);
-/* debug/parity taps (device pointers into engine state) */
+/* debug/parity taps (device pointers into engine state; acc_gu is not written by steps whose gate|up product stores the activation, 33 sequences and more) */
 void* wf_engine_buffer(wf_engine* e, const char* name);
 int wf_engine_launches_per_step(const wf_engine* e);
 int wf_engine_time_kernel(wf_engine* e, const char* which, int B, int iters, float* ms_out);
