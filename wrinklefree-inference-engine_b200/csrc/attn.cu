@@ -798,14 +798,15 @@ struct MergeParams {
 
 // grid = (H, B), block = 128 (one thread per d).  A lane per chunk for the maxima and sums; the first chunks' values are requested together with them and with the
 // sequence's length, before it is known how many there are (every slot is memory of the workspace): one round of latency, where a loop over the chunks asked for the
-// length, then for each maximum, then for each value.  The call at 6 sequences of 8K tokens in int8 28.8 -> 25.9 us, at 64 of 4K in bf16 100.5 -> 99.4.  More chunks
-// than a warp has lanes (one or two sequences of more than 20K tokens) take the loop.
+// length, then for each maximum, then for each value.  The call at 6 sequences of 8K tokens in int8 28.8 -> 26.6 us, at 64 of 4K in bf16 100.4 -> 99.3.  More chunks
+// than a warp has lanes (one or two sequences of more than 20K tokens) take the loop.  The next kernel starts when the blocks have ended: let in behind the wait, the next
+// call's attention finds some SMs taken and its blocks spread unevenly (64 query heads on 8 in bf16, 8 sequences of 12000 tokens 73.1 us a call and 81.2 so, 6 of 8192 38.3
+// and 42.4; elsewhere 1 to 3 % less).
 __global__ void __launch_bounds__(AT_D) attn_merge_kernel(const MergeParams p) {
     constexpr int AHEAD = 8;
     const int h = blockIdx.x, b = blockIdx.y, d = threadIdx.x, lane = threadIdx.x & 31;
     const size_t base = ((size_t)b * p.H + h) * p.max_chunks;
     pdl_wait_prior();
-    pdl_launch_dependents();
     float2 ml = make_float2(-INFINITY, 0.f);
     if (lane < p.max_chunks) ml = make_float2(p.part_ml[(base + lane) * 2], p.part_ml[(base + lane) * 2 + 1]);
     float o[AHEAD];
