@@ -380,11 +380,12 @@ def test_batches_of_changing_size_equal_per_op_kernels(shape, monkeypatch):
 
 @pytest.mark.parametrize("hidden", [3968, 4096])
 def test_row_kernels_equal_per_op_kernels_where_their_forms_change(hidden, monkeypatch):
-    """Rows of 4096 leave the registers above 24 sequences, narrower ones do not; both sides of it, and a few sequences, in steps that follow one another."""
+    """Rows of 4096 leave the registers above 24 sequences, narrower ones do not, and from there on (but at 32) the next kernel starts behind the row kernels' wait; both
+    sides of it, and a few sequences, in steps that follow one another."""
     from wf_bitnet.engine import EngineConfig
     cfg = EngineConfig(hidden=hidden, layers=1, heads=hidden // 128, kv_heads=hidden // 128, ffn=512, vocab=4096, max_seq=128, max_batch=33)
     rng = np.random.default_rng(hidden)
-    steps = [list(map(int, rng.integers(0, cfg.vocab, B))) for B in (33, 2, 8, 9, 24, 25, 32)]
+    steps = [list(map(int, rng.integers(0, cfg.vocab, B))) for B in (33, 2, 8, 9, 24, 25, 32, 31)]
     a = _run_tokens(cfg, None, True, steps, monkeypatch, ctx=20, synthetic=6)
     b = _run_tokens(cfg, None, False, steps, monkeypatch, ctx=20, synthetic=6)
     for i, ((la, na, _), (lb, nb, _)) in enumerate(zip(a, b)):

@@ -258,24 +258,25 @@ __global__ void __launch_bounds__(LS_THREADS, 2) linear_small_kernel(const Small
 // Standalone glue for large batch: grid = M rows, 256 threads; int8 codes / scale / rowsum go to global.
 constexpr int GR_T = 512;   // one pass iteration for K <= 4096, two for the 2B ffn width
 // IT > 0: the row stays in registers, IT vectors of eight a thread (K <= 4096 IT; sums of this GPU alone), the norm's weights requested ahead of the wait on the kernel
-// before; the same sums in the same order.  IT 0: through shared memory.  Batches above GLUE_LATE rows let the next kernel in behind their own wait: ahead of it a chain of
-// waiting kernels takes the SMs that the present one still needs (2B, 64 sequences 2.04 -> 1.97 ms a step, 8B 3.10 -> 3.05); up to there the next product's weights come early
-// (8B, 16 sequences 2.39 ms, 2.53 so).  Which form: launch_glue_rows.
-constexpr int GLUE_LATE = 32;
+// before; the same sums in the same order.  IT 0: through shared memory.  Which form: launch_glue_rows.  Larger batches let the next kernel in behind their own wait: ahead of
+// it a chain of waiting kernels takes the SMs that the present one still needs (2B, 64 sequences 2.04 -> 1.97 ms a step, 8B 3.10 -> 3.05; at 25 and 28 sequences of 60 tokens 2B
+// 2.06 -> 1.93 and 2.08 -> 1.98, 8B 3.40 -> 3.29 and 3.40 -> 3.27); in smaller ones the next product's weights come early (8B widths, 12 and 16 sequences 68.8 and 70.5 us a
+// layer, 71.1 and 74.6 so; at 17 to 24 2B, 8B and 70B are within 3 % either way).  So do they at 32, where the steps are shorter than at 31 (8B 2.77 ms, 2.81 so; 2B 5 % less so).
+__host__ __device__ constexpr bool glue_late(int M) { return M > 24 && M != 32; }
 template <int IT>
 __global__ void __launch_bounds__(GR_T) glue_rows_kernel(const GlueParams p) {
     extern __shared__ __align__(16) unsigned char gsm[];
     __nv_bfloat16* ys = reinterpret_cast<__nv_bfloat16*>(gsm);
     __shared__ float fs[32];
     __shared__ int is[32];
-    if (p.M <= GLUE_LATE) pdl_launch_dependents();
+    if (!glue_late(p.M)) pdl_launch_dependents();
     if (IT > 0) glue_prefetch_gamma<GR_T>(p);
     pdl_wait_prior();
     if (p.wait_flag >= 0) {
         if (threadIdx.x < 32) tp_wait_flags_warp(p.tp, p.wait_flag);
         __syncthreads();
     }
-    if (p.M > GLUE_LATE) pdl_launch_dependents();
+    if (glue_late(p.M)) pdl_launch_dependents();
     const int m = blockIdx.x;
     float sc; int rsum;
     glue_zero_duty<GR_T>(p);
